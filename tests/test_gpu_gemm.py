@@ -218,3 +218,39 @@ def test_gelu_forward_kernel():
         assert torch.allclose(y.float(), ref, rtol=tol, atol=tol), (shape, dt)
     edge = torch.tensor([-30.0, -8.0, -0.0, 0.0, 8.0, 30.0, float("inf")], device="cuda").repeat(4)[:24].contiguous()
     assert torch.allclose(gemm.gelu(edge), torch.nn.functional.gelu(edge), atol=1e-5)
+
+
+@pytest.mark.parametrize("M,N,K,bias", [(256, 256, 64, True), (300, 520, 136, True), (384, 264, 72, False), (3072, 1000, 200, True)])
+def test_gelu_epilogue_equals_product_then_gelu(M, N, K, bias):
+    """One kernel that writes z and gelu(z): the same bits as the product followed by the elementwise pass (GELU of the
+    rounded z), tiles of 256 and of 192 columns, ragged edges."""
+    from torchmpi_b200.ops import gemm
+    torch.manual_seed(M + N)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    c = torch.randn(N, device="cuda").to(torch.bfloat16) if bias else None
+    z, y = gemm.matmul_nt_gelu(a, b, c)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    assert torch.equal(z, gemm.matmul_nt(a, b, c))
+    assert torch.equal(y, gemm.gelu(z))
+    ref = a.float() @ b.float().t() + (c.float() if bias else 0.0)
+    assert ((z.float() - ref).norm() / ref.norm()).item() < 4e-3          # one bf16 rounding: 2^-9 at most
+
+
+@pytest.mark.parametrize("M,N,K", [(3072, 1024, 200), (3072, 1000, 72), (8192, 384, 136)])
+def test_pair_gemm_narrow_tiles(M, N, K):
+    """Shapes whose tiles are 192 columns wide (they fill the SMs better than 256), all operand layouts, a bias."""
+    from torchmpi_b200.ops import gemm
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    c = torch.randn(N, device="cuda").to(torch.bfloat16)
+    ref = a.float() @ b.float().t()
+    rel = lambda got, want: ((got.float() - want).norm() / want.norm()).item()
+    assert rel(gemm.matmul_nt(a, b, c), ref + c.float()) < 4e-3
+    assert rel(gemm.matmul_nn(a, b.t().contiguous()), ref) < 4e-3
+    assert rel(gemm.matmul_tn(a.t().contiguous(), b.t().contiguous()), ref) < 4e-3
+    odd = torch.randn(N + 1, device="cuda").to(torch.bfloat16)[1:]         # a bias that 16-byte loads cannot read
+    assert rel(gemm.matmul_nt(a, b, odd), ref + odd.float()) < 4e-3
+    gemm.check_status()

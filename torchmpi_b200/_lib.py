@@ -195,9 +195,14 @@ _CUDA_PROTOS = {
     "tmpi_bn_relu_pool_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp]),
     "tmpi_stem_im2col": (_i, [_vp, _vp, _i, _i, _i, _i, _vp]),
     "tmpi_stem_patch_width": (_i, []),
+    "tmpi_stem_conv_supported": (_i, [_i, _i]),
+    "tmpi_stem_conv_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i64p, _vp]),
+    "tmpi_stem_conv_wgrad_workspace_bytes": (_sz, []),
+    "tmpi_stem_conv_wgrad": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i64p, _vp, _sz, _vp]),
     "tmpi_maxpool_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "tmpi_maxpool_bwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "tmpi_gemm_bf16_gelu": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_ex": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp]),
     "tmpi_gemm_status": (_i, []),
     "tmpi_conv_max_ctas": (_i, []),
@@ -212,7 +217,6 @@ _CUDA_PROTOS = {
     "tmpi_attention_bwd_set_trace": (None, [_vp]),
     "tmpi_attention_ctas_per_sm": (_i, []),
     "tmpi_attention_set_trace": (None, [_vp]),
-    "tmpi_attention_set_v_stages": (None, [_i]),
     "tmpi_attention_status": (_i, []),
     "tmpi_gemm_tn_splitk_workspace_bytes": (_sz, [_i, _i, _i64]),
     "tmpi_gemm_bf16_tn_splitk": (_i, [_vp, _vp, _vp, _i, _i, _i64, _i64, _i64, _vp, _sz, _i, _vp]),

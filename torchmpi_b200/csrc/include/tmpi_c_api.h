@@ -296,7 +296,6 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
 int tmpi_attention_bwd_status(void);
 void tmpi_attention_bwd_set_trace(void* device_buffer);   // tuning aid, as for the forward
 int tmpi_attention_ctas_per_sm(void);
-void tmpi_attention_set_v_stages(int n);              // tuning aid: 1 or 2 V buffers per CTA
 void tmpi_attention_set_trace(void* device_buffer);   // tuning aid: phase time stamps of one CTA
 int tmpi_attention_status(void);
 // C[M, N] (+)= A^T B for A [K, M], B [K, N] with a long K and a small output (split over K; same kernel family)
@@ -323,10 +322,20 @@ int tmpi_maxpool_bwd(const void* dy, const void* idx, void* dx, int N, int H, in
 int tmpi_stem_im2col(const void* x, void* col, int N, int H, int W, int dtype, void* stream);
 int tmpi_stem_patch_width(void);
 
+// The same convolution and its weight gradient as implicit GEMMs, for 64 output channels and W a multiple of 8 up to 256
+// (stem_conv.cu).  x [N, H, W, 3], y / dy [N, OH, OW, 64]; w_strides: the four strides of w / dw [64, 3, 7, 7], in elements.
+int tmpi_stem_conv_supported(int W, int cout);
+int tmpi_stem_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, int cout, const int64_t* w_strides, void* stream);
+size_t tmpi_stem_conv_wgrad_workspace_bytes(void);
+int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, int W, int cout, const int64_t* w_strides,
+                         void* workspace, size_t workspace_bytes, void* stream);
+
 // ---------------------------------------------------------------- tcgen05 GEMM family
 // C[M,N] = act(A[M,K] * B[N,K]^T (+ bias)), bf16 in, fp32 accumulate in TMEM.
 int tmpi_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                    int epilogue, void* stream);
+// Z = A B^T + bias and Y = gelu(Z) of the rounded Z in one kernel; M, N >= 256, N and K multiples of 8
+int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream);
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                       int64_t lda, int64_t ldb, int64_t ldc, int epilogue, void* stream);

@@ -6,6 +6,7 @@
 // 16-byte pack), two rows at a time per block; every thread keeps its eight column sums in
 // registers, blocks write partials and a second kernel adds them in block order (deterministic).
 // The GELU forward with the same approximation of the normal distribution lives here too.
+#include "gelu.cuh"
 #include "vec.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
@@ -16,32 +17,6 @@ namespace tmpi {
 constexpr int kBgThreads = 256, kBgCols = 128;      // 128 column groups x 2 rows per block
 constexpr int kBgMaxRowBlocks = 4 * 148;            // partial rows the scratch buffer holds
 constexpr int kBgFinCols = 32, kBgFinGroups = 32;   // finalize: 32 columns x 32 groups of partial rows per block
-
-// gelu(z) = z * Phi(z);  d/dz [z * Phi(z)] = Phi(z) + z * phi(z).  Phi through the rational erf approximation of Abramowitz and
-// Stegun 7.1.26 (absolute error 1.5e-7), which shares its exp(-z^2 / 2) with phi: one ex2, one rcp and a
-// dozen FMAs per element keep the kernel memory bound where erff() made it ALU bound.
-__device__ __forceinline__ void normal_parts(float z, float* cdf, float* e) {
-  *e = __expf(-0.5f * z * z);
-  const float t = __fdividef(1.f, fmaf(0.3275911f * 0.70710678118654752f, fabsf(z), 1.f));
-  float poly = fmaf(1.061405429f, t, -1.453152027f);
-  poly = fmaf(poly, t, 1.421413741f);
-  poly = fmaf(poly, t, -0.284496736f);
-  poly = fmaf(poly, t, 0.254829592f);
-  const float q = 0.5f * poly * t * *e;                 // 1 - Phi(|z|)
-  *cdf = z >= 0.f ? 1.f - q : q;
-}
-
-__device__ __forceinline__ float gelu_grad(float z) {
-  float cdf, e;
-  normal_parts(z, &cdf, &e);
-  return fmaf(z * 0.3989422804014327f, e, cdf);
-}
-
-__device__ __forceinline__ float gelu_value(float z) {
-  float cdf, e;
-  normal_parts(z, &cdf, &e);
-  return z * cdf;
-}
 
 // y = gelu(z), one 16-byte pack per thread and step, four steps in flight.
 template <typename T, int V>

@@ -26,17 +26,18 @@ __device__ __forceinline__ void band_order(int t, int tiles_m, int tiles_n, int*
   *n_blk = r / rows;
 }
 
-// p.tiles_m counts 256-row tiles here.
-__global__ void __launch_bounds__(THREADS, 1)
+// p.tiles_m counts 256-row tiles here.  TWO: gelu(C) goes to map_y beside C.
+template <bool TWO>
+__global__ void __launch_bounds__(GROUP_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                      const __grid_constant__ CUtensorMap map_c, const Problem p) {
+                      const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_y, const Problem p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char *tiles, *staging;
   Shared* sh;
   carve(smem_raw, &tiles, &sh, &staging);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = sm100::cluster_ctarank();
-  setup(sh, warp, &map_a, &map_b);
+  setup(sh, warp, &map_a, &map_b, 4 * GROUPS);
 
   const int total = p.tiles_m * p.tiles_n;
   const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
@@ -53,10 +54,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else if (warp == 1) {
     if (rank == 0 && sm100::elect_one()) mma_issuer(sh, tiles, p, order);
   } else {
-    epilogue(sh, staging, p, warp & 3, lane, order, [&](int m_blk, const CUtensorMap** m, int* row0) {
-      *row0 = m_blk * BM;
-      *m = *row0 < p.M ? &map_c : nullptr;
-    });
+    epilogue_groups<TWO>(sh, staging, p, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
   }
   __syncwarp();
   teardown(sh, warp);
@@ -67,18 +65,28 @@ static int max_clusters() {
   static int n = 0;
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(2 * (gemm_sm_count() / 2)); cfg.blockDim = dim3(THREADS);
+    cfg.gridDim = dim3(2 * (gemm_sm_count() / 2)); cfg.blockDim = dim3(GROUP_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES; cfg.attrs = at; cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, (void*)gemm_bf16_pair_kernel, &cfg) == cudaSuccess && c > 0) n = c;
+    if (cudaOccupancyMaxActiveClusters(&c, (void*)gemm_bf16_pair_kernel<false>, &cfg) == cudaSuccess && c > 0) n = c;
     else { cudaGetLastError(); n = gemm_sm_count() / 2; }
   });
   return n;
+}
+
+// Columns of a tile: 192 where that needs less time than 256.  A launch takes ceil(tiles / clusters) rounds of a tile
+// time that is proportional to its columns, so 48 tiles of 256 on 74 clusters (3072 x 1024: one round, 26 clusters
+// idle) lose to 72 tiles of 192 (one round of three quarters of the time).  Measured: 3072 x 1024, K = 8192: 55 -> 46 us;
+// 8192 x 3072, K = 1024: 51 -> 46.
+static int tile_columns(int tiles_m, int N, int clusters) {
+  auto cost = [&](int bn) { return (long long)((tiles_m * (long long)((N + bn - 1) / bn) + clusters - 1) / clusters) * bn; };
+  return 100 * cost(192) < 95 * cost(BN) ? 192 : BN;      // a narrower tile reads more of A per product: 5 % for that
 }
 
 }  // namespace gemm2
@@ -94,10 +102,14 @@ bool gemm_pair_applicable(const void* C, int M, int N, int K, int flags) {
 
 // lda / ldb / ldc: row pitch of A, B, C as stored, in elements (0: dense).  With explicit pitches the
 // extents themselves need not be multiples of 8 (a [T, 50257] matrix held in rows of 50264).
+// gelu_out (optional): a second [M, N] matrix with C's pitch that receives gelu(C).
 int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int epilogue,
-                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc) {
-  CUtensorMap ma, mb, mc;
+                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out) {
+  CUtensorMap ma, mb, mc, my;
   int st;
+  const int clusters = gemm2::max_clusters();
+  const int tiles_m = (M + 2 * gemm2::BM - 1) / (2 * gemm2::BM);
+  const int bn = gemm2::tile_columns(tiles_m, N, clusters);
   const bool a_km = (epilogue & gemm::A_IS_KM) != 0;       // A given as [K, M], M contiguous
   if (!lda) lda = a_km ? M : K;
   if (a_km) st = make_tmap_bf16(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, gemm2::BK);
@@ -106,14 +118,17 @@ int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, in
   const bool b_kn = (epilogue & gemm::B_IS_KN) != 0;       // B given as [K, N], N contiguous
   if (!ldb) ldb = b_kn ? N : K;
   if (b_kn) st = make_tmap_bf16(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, gemm2::BK);
-  else st = make_tmap_bf16(&mb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, gemm2::BN / 2);
+  else st = make_tmap_bf16(&mb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, bn / 2);
   if (st) return st;
   if (!ldc) ldc = N;
   if ((st = make_tmap_bf16(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, gemm2::BM))) return st;
+  my = mc;
+  if (gelu_out && (st = make_tmap_bf16(&my, gelu_out, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, gemm2::BM))) return st;
   gemm::Problem p{};
   p.M = M; p.N = N; p.K = K;
-  p.tiles_m = (M + 2 * gemm2::BM - 1) / (2 * gemm2::BM);
-  p.tiles_n = (N + gemm2::BN - 1) / gemm2::BN;
+  p.tiles_m = tiles_m;
+  p.tiles_n = (N + bn - 1) / bn;
+  p.pair_n = bn;
   p.k_blocks = (K + gemm2::BK - 1) / gemm2::BK;
   p.epilogue = epilogue & 3;
   p.b_mn = b_kn ? 1 : 0;
@@ -121,14 +136,15 @@ int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, in
   p.bias = (const __nv_bfloat16*)bias;
   p.tma_store = 1;
   p.status = status_word;
-  const int nclusters = std::min(p.tiles_m * p.tiles_n, gemm2::max_clusters());
+  const int nclusters = std::min(p.tiles_m * p.tiles_n, clusters);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(2 * nclusters); cfg.blockDim = dim3(gemm2::THREADS);
+  cfg.gridDim = dim3(2 * nclusters); cfg.blockDim = dim3(gemm2::GROUP_THREADS);
   cfg.dynamicSmemBytes = gemm2::SMEM_BYTES; cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel, ma, mb, mc, p);
+  cudaError_t e = gelu_out ? cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<true>, ma, mb, mc, my, p)
+                           : cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<false>, ma, mb, mc, my, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "pair gemm launch: %s", cudaGetErrorString(e));
 }
 

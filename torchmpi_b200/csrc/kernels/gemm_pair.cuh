@@ -12,10 +12,11 @@
 //   full[s]   lives in the even CTA; both producers' TMA loads count their bytes there
 //   empty[s]  one per CTA; the issuer commits to both after the MMAs of the stage
 //   acc_full  one per CTA; the issuer commits to both after the last K block of a tile
-//   acc_empty lives in the even CTA; the eight epilogue warps of the pair arrive there
+//   acc_empty lives in the even CTA; the epilogue warps of the pair (four or eight per CTA) arrive there
 // The roles take the same hooks as the single-CTA ones; m_blk counts 128-row blocks, so the hooks of
 // the fused kernels (rows-ready wait, destination map) apply per CTA.
 #pragma once
+#include "gelu.cuh"
 #include "gemm_core.cuh"
 
 namespace tmpi {
@@ -48,12 +49,12 @@ __device__ __forceinline__ void carve(unsigned char* raw, unsigned char** tiles,
 
 // All threads of both CTAs.  The dynamic shared memory has the same layout in both CTAs, so an
 // offset taken in one is valid in the other.
-__device__ __forceinline__ void setup(Shared* sh, int warp, const CUtensorMap* ma, const CUtensorMap* mb) {
+__device__ __forceinline__ void setup(Shared* sh, int warp, const CUtensorMap* ma, const CUtensorMap* mb, int epilogue_warps = 4) {
   if (warp == 0 && sm100::elect_one()) {
     sm100::tma_prefetch_desc(ma);
     sm100::tma_prefetch_desc(mb);
     for (int s = 0; s < STAGES; ++s) { sm100::mbar_init(&sh->full[s], 1); sm100::mbar_init(&sh->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { sm100::mbar_init(&sh->acc_full[a], 1); sm100::mbar_init(&sh->acc_empty[a], 8); }
+    for (int a = 0; a < 2; ++a) { sm100::mbar_init(&sh->acc_full[a], 1); sm100::mbar_init(&sh->acc_empty[a], 2 * epilogue_warps); }
     sh->error = 0;
     sm100::fence_barrier_init();
   }
@@ -71,6 +72,9 @@ __device__ __forceinline__ void setup(Shared* sh, int warp, const CUtensorMap* m
 template <typename TileOrder, typename ASource>
 __device__ __forceinline__ void producer(Shared* sh, unsigned char* tiles, const Problem& p, const CUtensorMap* ma,
                                          const CUtensorMap* mb, uint32_t rank, TileOrder order, ASource a_source) {
+  const int bn = p.pair_n ? p.pair_n : BN;
+  // bytes of B per stage and CTA: bn / 2 rows, or (MN-major) two whole 64-column boxes, of which bn / 2 columns are used
+  const uint32_t stage_tx = 2 * (A_BYTES + (p.b_mn ? B_BYTES : (bn / 2) * BK * 2));
   int stage = 0;
   uint32_t phase = 0;
   int m_blk, n_blk;
@@ -78,12 +82,12 @@ __device__ __forceinline__ void producer(Shared* sh, unsigned char* tiles, const
     const CUtensorMap* a_map = ma;
     int a_row0 = m_blk * BM;
     if (!a_source(m_blk, &a_map, &a_row0)) { gemm::fail(sh, p, 11); return; }
-    const int b_row0 = n_blk * BN + (int)rank * (BN / 2);
+    const int b_row0 = n_blk * bn + (int)rank * (bn / 2);
     for (int kb = 0; kb < p.k_blocks; ++kb) {
       if (!sm100::mbar_wait(&sh->empty[stage], phase ^ 1, kWaitBudgetNs) || sh->error) { gemm::fail(sh, p, 12); return; }
       unsigned char* a_dst = tiles + (size_t)stage * STAGE_BYTES;
       const uint32_t full0 = sm100::map_to_cta(&sh->full[stage], 0);
-      if (rank == 0) sm100::mbar_expect_tx(&sh->full[stage], 2 * STAGE_BYTES);   // both CTAs' bytes
+      if (rank == 0) sm100::mbar_expect_tx(&sh->full[stage], stage_tx);   // both CTAs' bytes
       if (!p.a_mn) {
         sm100::tma_load_2d_pair(a_dst, a_map, kb * BK, a_row0, full0);
       } else {   // A is [K, M]: two boxes of 64 rows of the product x 64 k-rows
@@ -104,7 +108,7 @@ __device__ __forceinline__ void producer(Shared* sh, unsigned char* tiles, const
 // One thread of the EVEN CTA only.
 template <typename TileOrder>
 __device__ __forceinline__ void mma_issuer(Shared* sh, unsigned char* tiles, const Problem& p, TileOrder order) {
-  const uint32_t idesc = sm100::make_idesc_f16(2 * BM, BN, true, p.b_mn != 0, p.a_mn != 0);
+  const uint32_t idesc = sm100::make_idesc_f16(2 * BM, p.pair_n ? p.pair_n : BN, true, p.b_mn != 0, p.a_mn != 0);
   int stage = 0;
   uint32_t phase = 0;
   int m_blk, n_blk;
@@ -144,6 +148,112 @@ __device__ __forceinline__ void epilogue(Shared* sh, unsigned char* staging, con
   gemm::epilogue_tma_impl(sh, staging, p, quarter, lane, order, dest, [sh](int acc) {
     sm100::mbar_arrive_cluster(sm100::map_to_cta(&sh->acc_empty[acc], 0));
   });
+}
+
+// The epilogue of the plain GEMM: two groups of four warps in EACH CTA take the 64-column slices of a tile in turn, each
+// through a staging tile of its own, so that one group converts while the other waits for its accumulator reads and its
+// staging tile.  With one group the four slices of a tile were a serial chain of about 1 us each that a product with a
+// short K (16 K blocks: 4.3 us of MMAs per tile) could not hide, and that every launch paid at its end.  The bias of a
+// slice is read as eight 16-byte loads (64 scalar loads before).  Measured, 8192 x 4096 x 1024 with a bias: 83 -> 52 us; without
+// one 59 -> 50; 8192 x 50264 x 1024: 694 -> 585; 1024^3, where the launch is one tile and its epilogue: 17 -> 15.
+// TWO: gelu(C) is written beside C (map2): GELU of the rounded bf16 value, which is what a separate pass over C computes,
+// without that pass's launch and its read of C.  The group's staging tile is reused for it; the GELU is evaluated in
+// registers while the TMA unit still reads C out of the tile.
+constexpr int GROUPS = 2, GROUP_THREADS = 64 + GROUPS * 128;
+
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
+template <bool TWO, typename TileOrder>
+__device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* staging, const Problem& p, int group, int quarter,
+                                                int lane, TileOrder order, const CUtensorMap* map_c, const CUtensorMap* map2) {
+  constexpr int SLICE = 64, SLICE_BYTES = BM * SLICE * 2;
+  static_assert(GROUPS * SLICE_BYTES <= gemm::EPI_STAGING_BYTES, "one staging tile per group");
+  const int row = quarter * 32 + lane;
+  const bool leader = quarter == 0 && lane == 0;
+  const int bn = p.pair_n ? p.pair_n : BN;
+  unsigned char* stg = staging + group * SLICE_BYTES;
+  unsigned char* stg_row = stg + row * 128;
+  const bool bias_vec = ((uintptr_t)p.bias & 15) == 0;
+  int m_blk, n_blk;
+  for (int it = 0; order(it, &m_blk, &n_blk); ++it) {
+    const int acc = it & 1;
+    const uint32_t ok = sm100::mbar_wait(&sh->acc_full[acc], (it >> 1) & 1, kWaitBudgetNs) && !sh->error;
+    uint32_t all_ok;                    // the group meets at named barriers below: it goes on, or leaves, together
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, 128, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(all_ok) : "r"(ok), "r"(1 + group) : "memory");
+    if (!all_ok) { gemm::fail(sh, p, 5); break; }
+    sm100::tc_fence_after();
+    const int row0 = m_blk * BM;
+    const bool store = leader && row0 < p.M;
+    const uint32_t t_base = sh->tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+#pragma unroll 1
+    for (int c0 = group * SLICE; c0 < bn; c0 += GROUPS * SLICE) {
+      const int col0 = n_blk * bn + c0;
+      if (col0 >= p.N) break;           // uniform over the group: the rest of the tile lies outside C
+      uint32_t r[2][32], w[32];
+      sm100::tmem_ld_32x32(t_base + c0, r[0]);
+      sm100::tmem_ld_32x32(t_base + c0 + 32, r[1]);
+      sm100::tmem_ld_wait();
+      if (p.epilogue & gemm::EPI_BIAS) {
+        if (bias_vec && col0 + SLICE <= p.N) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + j);
+            const uint32_t b[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint32_t* v = &r[j >> 2][(j & 3) * 8 + 2 * q];
+              v[0] = __float_as_uint(__uint_as_float(v[0]) + __uint_as_float(b[q] << 16));
+              v[1] = __float_as_uint(__uint_as_float(v[1]) + __uint_as_float(b[q] & 0xffff0000u));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 64; ++j)
+            if (col0 + j < p.N) r[j >> 5][j & 31] = __float_as_uint(__uint_as_float(r[j >> 5][j & 31]) + __bfloat162float(p.bias[col0 + j]));
+        }
+      }
+      if (p.epilogue & gemm::EPI_GELU) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) r[j >> 5][j & 31] = __float_as_uint(gemm::gelu_erf(__uint_as_float(r[j >> 5][j & 31])));
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[j >> 4][2 * (j & 15)]), __uint_as_float(r[j >> 4][2 * (j & 15) + 1]));
+        w[j] = *reinterpret_cast<uint32_t*>(&h);
+      }
+      auto put = [&](const CUtensorMap* map) {
+        // the store that used this staging tile before must have read it
+        if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        group_sync(group);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          *reinterpret_cast<uint4*>(stg_row + ((u ^ (row & 7)) << 4)) = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
+        sm100::fence_proxy_async_smem();       // generic-proxy writes to shared memory -> visible to the TMA unit
+        group_sync(group);
+        if (store) {
+          gemm::tma_store_2d(map, stg, col0, row0);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      };
+      put(map_c);
+      if (TWO) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {         // bf16 -> fp32 is a shift or a mask
+          __nv_bfloat162 h = __floats2bfloat162_rn(gelu_value(__uint_as_float(w[j] << 16)), gelu_value(__uint_as_float(w[j] & 0xffff0000u)));
+          w[j] = *reinterpret_cast<uint32_t*>(&h);
+        }
+        put(map2);
+      }
+    }
+    sm100::tc_fence_before();
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive_cluster(sm100::map_to_cta(&sh->acc_empty[acc], 0));
+  }
+  if (leader) {
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // all stores complete before exit
+    sm100::fence_proxy_async();
+  }
 }
 
 // All threads of both CTAs.  Neither CTA frees its tensor memory or exits while the other may still

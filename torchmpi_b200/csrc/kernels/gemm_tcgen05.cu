@@ -79,19 +79,41 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map of a row-major [rows, cols] bf16 matrix (cols contiguous, leading dimension ld elements)
-// with a box of box_rows x 64 columns and the 128-byte swizzle.
-int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+// Tensor map of a row-major [rows, cols] matrix (cols contiguous, leading dimension ld elements) with a box of box_rows
+// rows x 128 bytes and the 128-byte swizzle.
+static int make_tmap_2d(CUtensorMap* map, CUtensorMapDataType type, int bytes, const void* base, uint64_t rows, uint64_t cols,
+                        uint64_t ld, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(TMPI_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
-  if (((uintptr_t)base & 15) || (ld * 2) % 16) return fail(TMPI_ERR_INVALID, "TMA operand must be 16-byte aligned with a 16-byte multiple row pitch");
+  if (((uintptr_t)base & 15) || (ld * bytes) % 16) return fail(TMPI_ERR_INVALID, "TMA operand must be 16-byte aligned with a 16-byte multiple row pitch");
   cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)gemm::BK, box_rows};
+  cuuint64_t strides[1] = {ld * bytes};
+  cuuint32_t box[2] = {(cuuint32_t)(128 / bytes), box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(TMPI_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", (int)r);
+  return TMPI_OK;
+}
+
+int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+  return make_tmap_2d(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, ld, box_rows);
+}
+int make_tmap_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+  return make_tmap_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, ld, box_rows);
+}
+
+// Dense 4-D bf16 tensor (dims[0] contiguous), 128-byte swizzle; box[0] is 64 elements.
+int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(TMPI_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
+  if (((uintptr_t)base & 15) || (dims[0] * 2) % 16) return fail(TMPI_ERR_INVALID, "TMA operand must be 16-byte aligned with a 16-byte multiple row pitch");
+  cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]};
+  cuuint64_t strides[3] = {dims[0] * 2, dims[0] * dims[1] * 2, dims[0] * dims[1] * dims[2] * 2};
+  cuuint32_t b[4] = {box[0], box[1], box[2], box[3]};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), d, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TMPI_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", (int)r);
   return TMPI_OK;
 }
@@ -109,9 +131,9 @@ int gemm_sm_count() {
 
 bool gemm_pair_applicable(const void* C, int M, int N, int K, int flags);
 int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int epilogue,
-                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc);
+                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out);
 
-static int* gemm_status_word() {
+int* gemm_status_word() {
   static int* dev_ptr = nullptr;
   static int* host_ptr = nullptr;
   static std::once_flag once;
@@ -137,7 +159,7 @@ int tmpi_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int 
   if (k_rows && K % 8) return fail(TMPI_ERR_INVALID, "gemm: K must be a multiple of 8 (16-byte rows for TMA)");
   if ((epilogue & gemm::EPI_BIAS) && !bias) return fail(TMPI_ERR_INVALID, "gemm: bias epilogue without bias");
   if (tunable("gemm_pair") && gemm_pair_applicable(C, M, N, K, epilogue))
-    return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0);
+    return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, nullptr);
   if (epilogue & (gemm::B_IS_KN | gemm::A_IS_KM))
     return fail(TMPI_ERR_UNSUPPORTED, "gemm: operands given as [K, M] / [K, N] need the CTA-pair kernel (M, N >= 256, M, N %% 8 == 0)");
   CUtensorMap ma, mb;
@@ -180,7 +202,16 @@ int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, i
   if ((lda | ldb | ldc) % 8 || lda <= 0 || ldb <= 0 || ldc <= 0)
     return fail(TMPI_ERR_INVALID, "gemm_ex: row pitches must be positive multiples of 8 elements");
   if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return fail(TMPI_ERR_INVALID, "gemm_ex: operands must be 16-byte aligned");
-  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, lda, ldb, ldc);
+  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, lda, ldb, ldc, nullptr);
+}
+
+// Z = A B^T + bias and Y = gelu(Z) (of the rounded Z), both [M, N], in one kernel: the forward of a linear layer that is
+// followed by a GELU and keeps its pre-activation.  CTA-pair kernel only (M, N >= 256, N and K multiples of 8).
+int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream) {
+  if (M < 1 || N < 1 || K < 1 || K % 8) return fail(TMPI_ERR_INVALID, "gemm_gelu: needs a non-empty product with K a multiple of 8");
+  if (!tunable("gemm_pair") || !gemm_pair_applicable(Z, M, N, K, 0) || ((uintptr_t)Y & 15))
+    return fail(TMPI_ERR_UNSUPPORTED, "gemm_gelu: needs the CTA-pair kernel (M, N >= 256, N %% 8 == 0, 16-byte aligned outputs)");
+  return launch_gemm_pair(A, B, Z, bias, M, N, K, bias ? gemm::EPI_BIAS : 0, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, Y);
 }
 
 // Non-zero after a GEMM CTA gave up on a bounded wait (1000 + the point where it happened); clears it.

@@ -169,6 +169,26 @@ def gelu(z: torch.Tensor) -> torch.Tensor:
 
 
 _gelu_kernel = gelu          # `_LinearFn.forward` has a flag named `gelu`
+
+
+def matmul_nt_gelu(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor]):
+    """``(z, gelu(z))`` with ``z = a @ b.T + bias``: one kernel whose epilogue writes both where the CTA-pair kernel
+    applies, the product and a pass over it otherwise."""
+    global launch_count
+    a, b = a.contiguous(), b.contiguous()
+    M, K = a.shape
+    N = b.shape[0]
+    if not (supported(a, b) and has_symbol("tmpi_gemm_bf16_gelu") and pair_kernel_takes(M, N, K)):
+        z = matmul_nt(a, b, bias)
+        return z, _gelu_kernel(z)
+    z = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+    y = torch.empty_like(z)
+    check(lib.tmpi_gemm_bf16_gelu(a.data_ptr(), b.data_ptr(), z.data_ptr(), y.data_ptr(),
+                                  bias.contiguous().data_ptr() if bias is not None else None, M, N, K, stream_ptr()))
+    launch_count += 1
+    return z, y
+
+
 _bg_scratch = {}
 _bg_need = {}
 
@@ -211,8 +231,7 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, w, bias, gelu):
         x2 = x.reshape(-1, x.shape[-1])
         if gelu:
-            z = matmul_nt(x2, w, bias)                       # pre-activation is needed by backward
-            y = _gelu_kernel(z)
+            z, y = matmul_nt_gelu(x2, w, bias)               # the pre-activation is needed by backward
             ctx.save_for_backward(x2, w, z)
         else:
             y = matmul_nt(x2, w, bias)
