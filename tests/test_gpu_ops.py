@@ -243,3 +243,43 @@ def test_layernorm_matches_torch(dtype):
         for g, gr in ((x.grad, xr.grad), (ln.weight.grad, wr.grad), (ln.bias.grad, br.grad)):
             rel = (g.float() - gr).norm() / gr.norm()
             assert rel < (2e-2 if dtype == torch.bfloat16 else 1e-5), (rows, C, rel.item())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N,C,H,W", [(1, 8, 1, 1), (2, 64, 2, 3), (5, 128, 29, 30), (3, 16, 64, 5)])
+def test_bn_pool_stage_edges_and_ties(dtype, N, C, H, W):
+    """The pooling stage at single rows and columns, odd sizes and several strips, on values with many ties: the first
+    maximum of a window takes the gradient, a window that the ReLU closed passes none."""
+    from torchmpi_b200 import config
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLUMaxPool
+    torch.manual_seed(N * H + W)
+    x = torch.randint(-2, 3, (N, C, H, W), device="cuda").to(dtype).contiguous(memory_format=torch.channels_last)
+    m = FusedBatchNormReLUMaxPool(C).cuda().eval()                 # fixed statistics: (x - 0) / 1 exactly, ties stay ties
+    with torch.no_grad():
+        m.running_var.fill_(1.0 - m.eps)
+        m.weight[::2] *= -1
+    xg = x.clone().requires_grad_(True)
+    y = m(xg)
+    z = torch.relu(x.float() * m.weight.detach()[None, :, None, None]).to(dtype).float().requires_grad_(True)
+    ref = torch.nn.functional.max_pool2d(z, 3, 2, 1)
+    assert torch.allclose(y.float(), ref, rtol=1e-3, atol=1e-3)
+    # backward uses batch statistics in its formula; with both parameter sums removed it is the routed gradient, which the
+    # two-stage path (pool, then batch-norm) computes separately
+    dy = torch.randn_like(y)
+    got = {}
+    for fused in (1, 0):
+        config.set("bn_pool_fused_bwd", fused)
+        try:
+            xg.grad = m.weight.grad = m.bias.grad = None
+            m(xg).backward(dy)
+            got[fused] = (xg.grad.float().clone(), m.weight.grad.clone(), m.bias.grad.clone())
+        finally:
+            config.set("bn_pool_fused_bwd", 1)
+    ref.backward(dy.float())
+    # the bias gradient is the sum of the routed gradient over the positions that the ReLU lets through
+    routed = (z.grad * (z > 0)).sum((0, 2, 3))
+    scale = dy.float().abs().sum((0, 2, 3)).max().item() + 1e-6
+    assert (got[1][2] - routed).abs().max().item() <= 1e-5 * scale
+    tol = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}[dtype]      # two-stage rounds the routed gradient to dtype
+    for a, b in zip(got[1], got[0]):
+        assert (a - b).abs().max().item() <= tol * max(1.0, b.abs().max().item()) * 2, (dtype, (a - b).abs().max().item())

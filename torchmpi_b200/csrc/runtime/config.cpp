@@ -64,7 +64,7 @@ Tunable g_tunables[] = {
   {"heap_bytes", {int64_t(1) << 30}},      // symmetric heap per rank
   {"staging_bytes", {64 << 20}},           // bounce buffer inside the heap for foreign tensors
   {"use_nvls", {1}},
-  {"bn_pool_fused_bwd", {0}},              // stem batch-norm + pool backward as one stage (slower than pool, then batch-norm)
+  {"bn_pool_fused_bwd", {1}},              // stem batch-norm + pool backward as one stage (0: pool backward, then batch-norm backward)
   {"bn_reverse_stats", {1}},               // batch-norm statistics passes walk the tensor from its end (L2 reuse)
   {"grad_fork", {1}},                      // residual blocks sum the two gradients of their input inside a kernel
   {"conv_own_3x3", {0}},                   // 3x3 convolutions on the implicit-GEMM kernel (1x1 always are)

@@ -170,8 +170,8 @@ class _BnReluPoolFn(torch.autograd.Function):
                 _scratch_for(x.device, C).data_ptr(), stream_ptr()))
             launch_count += 3
         else:
-            # measured faster: route the gradient through the pool once, then the batch-norm backward with the
-            # ReLU mask rebuilt from x (the rectified activation itself was never stored)
+            # in two stages: route the gradient through the pool, then the batch-norm backward with the ReLU mask
+            # rebuilt from x (the rectified activation itself was never stored)
             OH, OW = dy.shape[2], dy.shape[3]
             da = torch.empty_like(x, memory_format=torch.channels_last)
             check(lib.tmpi_maxpool_bwd(dy.data_ptr(), idx.data_ptr(), da.data_ptr(), N, H, W, C, OH, OW, 3, 2, 1,
