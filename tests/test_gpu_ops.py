@@ -245,6 +245,32 @@ def test_layernorm_matches_torch(dtype):
             assert rel < (2e-2 if dtype == torch.bfloat16 else 1e-5), (rows, C, rel.item())
 
 
+@pytest.mark.parametrize("N,H,W,cl", [(1, 8, 8, True), (2, 17, 24, False), (3, 64, 256, True), (1, 224, 224, True), (150, 16, 40, False)])
+def test_stem_conv_implicit_gemm(N, H, W, cl):
+    """Forward and weight gradient of the implicit-GEMM stem against an fp32 convolution: the narrowest and widest rows, odd
+    heights, chunks cut by the image's end, more chunks than CTAs, both weight layouts."""
+    import torch.nn.functional as F
+    from torchmpi_b200.ops import stem_conv, gemm
+    torch.manual_seed(N + H + W)
+    conv = stem_conv.StemConv7x7(64).cuda().to(torch.bfloat16)
+    if cl:
+        conv = conv.to(memory_format=torch.channels_last)
+    x = torch.randn(N, 3, H, W, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    assert stem_conv.supported(x, conv.weight) and stem_conv.direct(x, conv.weight)
+    y = conv(x)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    gemm.check_status()
+    w = conv.weight.detach().float().requires_grad_(True)
+    ref = F.conv2d(x.float(), w, None, 2, 3)
+    ref.backward(dy.float())
+    assert y.shape == ref.shape and y.is_contiguous(memory_format=torch.channels_last)
+    rel = lambda a, b: ((a.float() - b).norm() / b.norm()).item()
+    # one bf16 rounding of an fp32 sum: 2^-9 at most, 2^-9 / sqrt(3) in the mean
+    assert rel(y, ref.detach()) < 4e-3, rel(y, ref.detach())
+    assert rel(conv.weight.grad, w.grad) < 4e-3, rel(conv.weight.grad, w.grad)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("N,C,H,W", [(1, 8, 1, 1), (2, 64, 2, 3), (5, 128, 29, 30), (3, 16, 64, 5)])
 def test_bn_pool_stage_edges_and_ties(dtype, N, C, H, W):

@@ -1,0 +1,433 @@
+// The ResNet stem convolution (7 x 7, stride 2, pad 3, 3 input channels, 64 output channels) as an implicit GEMM on the
+// tcgen05 tensor cores: forward and weight gradient, without a patch matrix.
+//
+// The input goes to shared memory as rows of 16-byte units, one per pair of pixels (2p, 2p + 1), each pixel padded to four
+// channels.  The window of output pixel ow covers the four pairs ow - 2 .. ow + 1 (one padded tap on the left), so
+// neighbouring output pixels read neighbouring units, and a row of units IS the operand in the unswizzled core-matrix
+// layout of the tensor core: eight consecutive output pixels x 8 values are 128 contiguous bytes, the next tap pair is the
+// same 128 bytes moved by one unit.  Overlapping core matrices cost nothing, so nothing is copied per window.
+//
+//   forward          Y[ow, co] += X[ow, (pair, channel)] W[co, (pair, channel)] for each of the seven input rows of a window:
+//                    14 MMAs of 128 x 64 x 16 per output row (K = 7 rows x 4 pairs x 8 = 224 for 147 weights)
+//   weight gradient  the output pixels are the K dimension.  Two output rows share an operand: M = 128 = dY rows (i, i + 1)
+//                    of 64 channels, N = 80 = ten input rows x 8 values of one tap pair (the rows are a constant stride
+//                    apart), four MMAs per 16 pixels; input row r meets kernel row r of dY row i and r - 2 of row i + 1.
+//                    Partial sums per CTA, added in CTA order by a second kernel (deterministic).
+//
+// What bounds it: forward the 411 MB of output (62 us at the copy rate, 256 images of 224 x 224) and, about as much, the
+// MMAs (448 cycles per output row); the weight gradient the reads of dY, the same bytes, and the MMAs (their 128-row dY
+// operand comes out of shared memory once per tap pair).  The patch matrix that both products read before was 1.03 GB,
+// written once and read twice.  Measured, 256 x 224 x 224: forward 138 us
+// (patch matrix 354 + product 262 + weight layout 9), weight gradient 147 us (split-K product 221).
+//
+// The reference has no convolution of its own (it trains Torch7 modules).  One persistent CTA per SM, work in chunks of
+// eight output rows, double-buffered; every wait is bounded.
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <cuda_bf16.h>
+#include <algorithm>
+#include <mutex>
+#include "sm100_ptx.cuh"
+#include "../include/tmpi_c_api.h"
+#include "../runtime/common.h"
+
+namespace tmpi {
+
+int gemm_sm_count();
+int* gemm_status_word();
+int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]);
+
+namespace stem {
+
+constexpr int COUT = 64, TAPS = 4, KROWS = 7, R = 8, IN_ROWS = 2 * R + 6;      // chunk: R output rows, 2 R + 5 input rows (+ 1: N = 80)
+constexpr int MAX_OW = 128;
+constexpr int LOADERS = 256, THREADS = 512;        // warp 0 issues MMAs, warps 4-7 drain, warps 8-15 load x; wgrad: warp 1 loads dY
+constexpr int STAGING = 4096;                      // 32 pixels x 64 channels
+constexpr int W_BYTES = KROWS * TAPS * 8 * COUT * 2;
+constexpr int ACCS = 4, DY_STAGES = 3, WG_N = 80;
+constexpr unsigned long long kWaitBudgetNs = 4000000000ull;
+
+struct Shared {
+  uint64_t x_full[2], x_empty[2], acc_full[ACCS], acc_empty[ACCS], dy_full[DY_STAGES], dy_empty[DY_STAGES];
+  uint32_t tmem_base;
+  int error;
+};
+
+struct Params {
+  int N, H, W, OH, OW, ow16, units, chunks_per_image, chunks;
+  int row_bytes;               // shared-memory bytes of one input row: units * 16
+  int64_t ws_co, ws_c, ws_h, ws_w;      // strides of the weight (and its gradient), elements
+  const __nv_bfloat16* x;
+  const __nv_bfloat16* w;
+  float* partial;              // weight gradient: [gridDim.x][128][TAPS * WG_N]
+  int* status;
+};
+
+__device__ __forceinline__ void fail(Shared* sh, const Params& p, int where) {
+  atomicExch(&sh->error, where);
+  if (p.status) atomicCAS(p.status, 0, 1000 + where);
+}
+#define STEM_WAIT(bar, parity, where) \
+  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
+
+// Unswizzled operand: core matrices of 8 rows x 16 bytes, 128 contiguous bytes each.  K-major: `lead` between the two
+// core matrices along K, `stride` between groups of eight rows.  MN-major: `stride` between core matrices along M / N,
+// `lead` between groups of eight along K.
+__device__ __forceinline__ uint64_t desc_plain(uint32_t addr, uint32_t lead, uint32_t stride) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)(lead >> 4) << 16 | (uint64_t)(stride >> 4) << 32 | (uint64_t)1 << 46;
+}
+
+__device__ __forceinline__ bool chunk(const Params& p, int it, int* n, int* oh0) {
+  const int c = blockIdx.x + it * gridDim.x;
+  if (c >= p.chunks) return false;
+  *n = c / p.chunks_per_image;
+  *oh0 = (c - *n * p.chunks_per_image) * R;
+  return true;
+}
+
+// Warps 8-15: the input rows of a chunk as units.  A unit is 12 contiguous bytes of the image (W is even: a pair is inside
+// or outside as a whole).  Four units per thread are in flight; the loads of a chunk's first four start before the buffer
+// is free.
+__device__ void load_rows(Shared* sh, unsigned char* rows, const Params& p, int tid) {
+  const int total = IN_ROWS * p.units, pairs = p.W / 2;
+  int n, oh0;
+  for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
+    const int b = it & 1;
+    unsigned char* dst = rows + b * IN_ROWS * p.row_bytes;
+    const uint32_t* img = reinterpret_cast<const uint32_t*>(p.x) + (size_t)n * p.H * (p.W * 3 / 2);
+    bool free = it < 2;
+    for (int t0 = tid; t0 < total; t0 += 4 * LOADERS) {
+      uint32_t w[4][3];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = t0 + q * LOADERS;
+        const int row = t / p.units, pr = t - row * p.units - 2, ih = 2 * oh0 - 3 + row;
+        w[q][0] = w[q][1] = w[q][2] = 0u;
+        if (t < total && ih >= 0 && ih < p.H && pr >= 0 && pr < pairs) {
+          const uint32_t* s = img + (size_t)ih * (p.W * 3 / 2) + pr * 3;
+          w[q][0] = __ldg(s); w[q][1] = __ldg(s + 1); w[q][2] = __ldg(s + 2);
+        }
+      }
+      if (!free) { STEM_WAIT(&sh->x_empty[b], ((it >> 1) - 1) & 1, 61); free = true; }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = t0 + q * LOADERS;
+        if (t < total)
+          *reinterpret_cast<uint4*>(dst + (size_t)t * 16) =
+              make_uint4(w[q][0], w[q][1] & 0xffffu, (w[q][1] >> 16) | (w[q][2] << 16), w[q][2] >> 16);
+      }
+    }
+    sm100::fence_proxy_async_smem();
+    __syncwarp();
+    if ((tid & 31) == 0) sm100::mbar_arrive(&sh->x_full[b]);
+  }
+}
+
+__device__ __forceinline__ void setup(Shared* sh, int warp) {
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < 2; ++b) { sm100::mbar_init(&sh->x_full[b], LOADERS / 32); sm100::mbar_init(&sh->x_empty[b], 1); }
+    for (int a = 0; a < ACCS; ++a) { sm100::mbar_init(&sh->acc_full[a], 1); sm100::mbar_init(&sh->acc_empty[a], 4); }
+    for (int s = 0; s < DY_STAGES; ++s) { sm100::mbar_init(&sh->dy_full[s], 1); sm100::mbar_init(&sh->dy_empty[s], 1); }
+    sh->error = 0;
+    sm100::fence_barrier_init();
+  }
+  if (warp == 0) {
+    sm100::tmem_alloc(&sh->tmem_base, 512);
+    sm100::tmem_relinquish();
+  }
+}
+__device__ __forceinline__ void teardown(Shared* sh, int warp) {
+  __syncwarp();
+  sm100::tc_fence_before();
+  __syncthreads();
+  if (sh->error && threadIdx.x == 0) {
+    const unsigned long long t0 = sm100::now_ns();
+    while (sm100::now_ns() - t0 < 200000000ull) { __nanosleep(1000); }   // copies in flight land within microseconds
+  }
+  __syncthreads();
+  if (warp == 0) {
+    sm100::tc_fence_after();
+    sm100::tmem_dealloc(sh->tmem_base, 512);
+  }
+}
+
+// ---------------------------------------------------------------- forward
+__device__ void fwd_mma(Shared* sh, unsigned char* rows, unsigned char* weights, const Params& p) {
+  constexpr uint32_t idesc = sm100::make_idesc_f16(128, COUT, true);
+  const uint32_t x0 = sm100::smem_u32(rows), w0 = sm100::smem_u32(weights);
+  int n, oh0, count = 0;
+  for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
+    const int b = it & 1;
+    STEM_WAIT(&sh->x_full[b], (it >> 1) & 1, 62);
+    const int lines = min(R, p.OH - oh0);
+    for (int i = 0; i < lines; ++i, ++count) {
+      const int acc = count % ACCS;
+      if (count >= ACCS) STEM_WAIT(&sh->acc_empty[acc], (count / ACCS - 1) & 1, 63);
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < 2 * KROWS; ++k) {                  // kernel row k / 2, tap pairs 2 (k % 2) and the next
+        const uint32_t a = x0 + (uint32_t)(b * IN_ROWS + 2 * i + (k >> 1)) * p.row_bytes + (k & 1) * 32;
+        sm100::umma_f16(sh->tmem_base + acc * COUT, desc_plain(a, 16, 128), desc_plain(w0 + k * 2 * COUT * 16, COUT * 16, 128), idesc,
+                        k > 0 ? 1u : 0u);
+      }
+      sm100::umma_commit(&sh->acc_full[acc]);
+    }
+    sm100::umma_commit(&sh->x_empty[b]);
+  }
+}
+
+__device__ void fwd_drain(Shared* sh, unsigned char* staging, const Params& p, const CUtensorMap* my, int quarter, int lane) {
+  const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
+  int n, oh0, count = 0;
+  for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
+    const int lines = min(R, p.OH - oh0);
+    for (int i = 0; i < lines; ++i, ++count) {
+      const int acc = count % ACCS;
+      STEM_WAIT(&sh->acc_full[acc], (count / ACCS) & 1, 64);
+      sm100::tc_fence_after();
+      uint32_t r[2][32];
+      sm100::tmem_ld_32x32(tm + acc * COUT, r[0]);
+      sm100::tmem_ld_32x32(tm + acc * COUT + 32, r[1]);
+      sm100::tmem_ld_wait();
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        sm100::mbar_arrive(&sh->acc_empty[acc]);
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the store two rows ago has read its tile
+      }
+      __syncwarp();
+      if (quarter * 32 < p.OW) {
+        unsigned char* stg = staging + (quarter * 2 + (count & 1)) * STAGING;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = (u & 3) * 8 + 2 * e;
+            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[u >> 2][j]), __uint_as_float(r[u >> 2][j + 1]));
+            w[e] = *reinterpret_cast<uint32_t*>(&h);
+          }
+          *reinterpret_cast<uint4*>(stg + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        sm100::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) sm100::tma_store_4d(my, stg, 0, quarter * 32, oh0 + i, n);      // pixels beyond the row are clipped
+      }
+      if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_constant__ CUtensorMap map_y, const Params p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  unsigned char* staging = smem;                              // 4 warps x 2 tiles
+  unsigned char* weights = smem + 8 * STAGING;
+  unsigned char* rows = weights + W_BYTES;
+  // the 128-row operand of the last input row runs on past it by up to MAX_OW units, into the tail that follows the rows
+  Shared* sh = (Shared*)(rows + 2 * IN_ROWS * p.row_bytes + (MAX_OW + 4) * 16);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  setup(sh, warp);
+  // weights: K chunk k (kernel row k / 2, tap pairs 2 (k % 2) ..), its halves, groups of eight output channels
+  for (int t = threadIdx.x; t < KROWS * TAPS * COUT; t += THREADS) {
+    const int co = t % COUT, unit = t / COUT, kh = unit / TAPS, tap = unit % TAPS;
+    unsigned short v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int kw = 2 * tap + (e >> 2) - 1, c = e & 3;
+      v[e] = 0;
+      if (kw >= 0 && kw < 7 && c < 3)
+        v[e] = *reinterpret_cast<const unsigned short*>(p.w + co * p.ws_co + c * p.ws_c + kh * p.ws_h + kw * p.ws_w);
+    }
+    *reinterpret_cast<uint4*>(weights + (size_t)t * 16) = make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16,
+                                                                     v[4] | (uint32_t)v[5] << 16, v[6] | (uint32_t)v[7] << 16);
+  }
+  sm100::fence_proxy_async_smem();
+  sm100::tc_fence_before();
+  __syncthreads();
+  sm100::tc_fence_after();
+  if (warp == 0) {
+    if (sm100::elect_one()) fwd_mma(sh, rows, weights, p);
+  } else if (warp >= 8) {
+    load_rows(sh, rows, p, threadIdx.x - 256);
+  } else if (warp >= 4) {
+    fwd_drain(sh, staging, p, &map_y, warp & 3, lane);
+  }
+  teardown(sh, warp);
+}
+
+// ---------------------------------------------------------------- weight gradient
+__global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const Params p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int dy_row = p.ow16 * 128, dy_stage = 2 * dy_row;     // a pair of dY rows of 64 channels, 128-byte swizzle
+  unsigned char* dys = smem;
+  unsigned char* rows = smem + DY_STAGES * dy_stage;
+  Shared* sh = (Shared*)(rows + 2 * IN_ROWS * p.row_bytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  setup(sh, warp);
+  sm100::tc_fence_before();
+  __syncthreads();
+  sm100::tc_fence_after();
+  int n, oh0;
+  if (warp >= 8) {
+    load_rows(sh, rows, p, threadIdx.x - 256);
+  } else if (warp == 1) {
+    if (sm100::elect_one()) [&]() {
+      int count = 0;
+      for (int it = 0; chunk(p, it, &n, &oh0); ++it)
+        for (int i = 0; i < R && oh0 + i < p.OH; i += 2, ++count) {
+          const int s = count % DY_STAGES;
+          if (count >= DY_STAGES) STEM_WAIT(&sh->dy_empty[s], (count / DY_STAGES - 1) & 1, 65);
+          sm100::mbar_expect_tx(&sh->dy_full[s], dy_stage);
+          // rows beyond the image and pixels beyond the row are zeros
+          sm100::tma_load_4d(dys + s * dy_stage, &map_dy, 0, 0, oh0 + i, n, &sh->dy_full[s]);
+          sm100::tma_load_4d(dys + s * dy_stage + dy_row, &map_dy, 0, 0, oh0 + i + 1, n, &sh->dy_full[s]);
+        }
+    }();
+  } else if (warp == 0) {
+    if (sm100::elect_one()) [&]() {
+      constexpr uint32_t idesc = sm100::make_idesc_f16(128, WG_N, true, true, true);      // both operands MN-major (pixels are K)
+      const uint32_t x0 = sm100::smem_u32(rows);
+      int count = 0;
+      for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
+        const int b = it & 1;
+        STEM_WAIT(&sh->x_full[b], (it >> 1) & 1, 66);
+        for (int i = 0; i < R && oh0 + i < p.OH; i += 2, ++count) {
+          const int s = count % DY_STAGES;
+          STEM_WAIT(&sh->dy_full[s], (count / DY_STAGES) & 1, 67);
+          sm100::tc_fence_after();
+          const uint64_t a = sm100::make_desc_sw128_mn(sm100::smem_u32(dys + s * dy_stage), dy_row, 1024);
+          const uint32_t x_row = x0 + (uint32_t)(b * IN_ROWS + 2 * i) * p.row_bytes;
+          for (int k = 0; k < p.ow16 / 16; ++k)
+#pragma unroll
+            for (int t = 0; t < TAPS; ++t)
+              sm100::umma_f16(sh->tmem_base + t * WG_N, a + (uint64_t)((k * 16 * 128) >> 4), desc_plain(x_row + (k * 16 + t) * 16, 128, p.row_bytes),
+                              idesc, (count | k) ? 1u : 0u);
+          sm100::umma_commit(&sh->dy_empty[s]);
+        }
+        sm100::umma_commit(&sh->x_empty[b]);
+      }
+      sm100::umma_commit(&sh->acc_full[0]);
+    }();
+  } else if (warp >= 4) {
+    [&]() {
+      STEM_WAIT(&sh->acc_full[0], 0, 68);
+      sm100::tc_fence_after();
+      const int row = (warp & 3) * 32 + lane;
+      float* out = p.partial + ((size_t)blockIdx.x * 128 + row) * (TAPS * WG_N);
+      for (int c = 0; c < TAPS * WG_N; c += 32) {
+        uint32_t r[32];
+        sm100::tmem_ld_32x32(sh->tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c, r);
+        sm100::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(out + c + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                                                __uint_as_float(r[j + 3]));
+      }
+      sm100::tc_fence_before();
+    }();
+  }
+  teardown(sh, warp);
+}
+
+// One block per output channel: ten groups of threads add the partial rows of a contiguous range of CTAs (dY row i and, ten
+// input rows being shared by two dY rows, row i + 1 two input rows further on), the groups' sums are added in order.
+constexpr int RED_COLS = TAPS * WG_N / 4, RED_GROUPS = 10;
+__global__ void __launch_bounds__(RED_COLS * RED_GROUPS)
+stem_wgrad_reduce_kernel(const float* __restrict__ partial, int ctas, __nv_bfloat16* __restrict__ dw, int64_t s_co, int64_t s_c, int64_t s_h,
+                         int64_t s_w) {
+  __shared__ float4 sum[RED_GROUPS][2][RED_COLS];
+  const int col = threadIdx.x % RED_COLS, grp = threadIdx.x / RED_COLS, co = blockIdx.x;
+  const int per = (ctas + RED_GROUPS - 1) / RED_GROUPS;
+  float4 a[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll 4
+  for (int c = grp * per; c < min(ctas, (grp + 1) * per); ++c)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(partial + ((size_t)c * 128 + h * 64 + co) * (TAPS * WG_N)) + col);
+      a[h].x += v.x; a[h].y += v.y; a[h].z += v.z; a[h].w += v.w;
+    }
+  sum[grp][0][col] = a[0];
+  sum[grp][1][col] = a[1];
+  __syncthreads();
+  for (int o = threadIdx.x; o < 147; o += blockDim.x) {
+    const int kh = o / 21, kw = o % 21 / 3, c = o % 3;
+    const int tap = (kw + 1) >> 1, e = (kw + 1) & 1;
+    const int at0 = tap * WG_N + kh * 8 + e * 4 + c, at1 = at0 + 16;
+    float t = 0.f;
+    for (int g = 0; g < RED_GROUPS; ++g)
+      t += reinterpret_cast<const float*>(sum[g][0])[at0] + reinterpret_cast<const float*>(sum[g][1])[at1];
+    dw[co * s_co + c * s_c + kh * s_h + kw * s_w] = __float2bfloat16_rn(t);
+  }
+}
+
+static int fill(Params* p, const void* x, int N, int H, int W, int cout, const int64_t* strides) {
+  if (N < 1 || H < 1 || W < 8) return tmpi::fail(TMPI_ERR_INVALID, "stem convolution: empty input");
+  const int OH = (H - 1) / 2 + 1, OW = (W - 1) / 2 + 1;
+  if (cout != COUT || W % 8 || OW > MAX_OW || ((uintptr_t)x & 15))
+    return tmpi::fail(TMPI_ERR_UNSUPPORTED, "stem convolution: needs %d output channels, W a multiple of 8 up to %d and a 16-byte aligned input", COUT, 2 * MAX_OW);
+  p->N = N; p->H = H; p->W = W; p->OH = OH; p->OW = OW;
+  p->ow16 = (OW + 15) / 16 * 16;
+  p->units = p->ow16 + 4;
+  p->row_bytes = p->units * 16;
+  p->chunks_per_image = (OH + R - 1) / R;
+  if ((int64_t)N * p->chunks_per_image > 0x7fffffffLL) return tmpi::fail(TMPI_ERR_UNSUPPORTED, "stem convolution: too many images");
+  p->chunks = N * p->chunks_per_image;
+  p->x = (const __nv_bfloat16*)x;
+  p->ws_co = strides[0]; p->ws_c = strides[1]; p->ws_h = strides[2]; p->ws_w = strides[3];
+  p->status = gemm_status_word();
+  return TMPI_OK;
+}
+
+}  // namespace stem
+}  // namespace tmpi
+
+using namespace tmpi;
+
+extern "C" {
+
+// 1 if tmpi_stem_conv_fwd / _wgrad take an image width and a number of output channels
+int tmpi_stem_conv_supported(int W, int cout) { return cout == stem::COUT && W >= 8 && W % 8 == 0 && (W - 1) / 2 + 1 <= stem::MAX_OW; }
+
+// y[N, OH, OW, 64] (channels-last) = convolution of x [N, H, W, 3] (channels-last) with w [64, 3, 7, 7] (any strides, given in
+// elements), stride 2, pad 3.  bf16, fp32 accumulation.
+int tmpi_stem_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, int cout, const int64_t* w_strides, void* stream) {
+  stem::Params p{};
+  int st = stem::fill(&p, x, N, H, W, cout, w_strides);
+  if (st) return st;
+  p.w = (const __nv_bfloat16*)w;
+  CUtensorMap my;
+  if ((st = make_tmap_bf16_4d(&my, y, {(uint64_t)stem::COUT, (uint64_t)p.OW, (uint64_t)p.OH, (uint64_t)N}, {64, 32, 1, 1}))) return st;
+  const int smem = 8 * stem::STAGING + stem::W_BYTES + 2 * stem::IN_ROWS * p.row_bytes + (stem::MAX_OW + 4) * 16 + (int)sizeof(stem::Shared);
+  cudaError_t e = cudaFuncSetAttribute(stem::stem_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "stem convolution: shared memory attribute: %s", cudaGetErrorString(e));
+  stem::stem_fwd_kernel<<<std::min(p.chunks, gemm_sm_count()), stem::THREADS, smem, (cudaStream_t)stream>>>(my, p);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "stem convolution launch: %s", cudaGetErrorString(e));
+}
+
+size_t tmpi_stem_conv_wgrad_workspace_bytes(void) { return (size_t)gemm_sm_count() * 128 * stem::TAPS * stem::WG_N * sizeof(float); }
+
+// dw [64, 3, 7, 7] (strides as given) from dy [N, OH, OW, 64] and x; workspace: tmpi_stem_conv_wgrad_workspace_bytes.
+int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, int W, int cout, const int64_t* w_strides,
+                         void* workspace, size_t workspace_bytes, void* stream) {
+  stem::Params p{};
+  int st = stem::fill(&p, x, N, H, W, cout, w_strides);
+  if (st) return st;
+  const int grid = std::min(p.chunks, gemm_sm_count());
+  if (workspace_bytes < (size_t)grid * 128 * stem::TAPS * stem::WG_N * sizeof(float))
+    return fail(TMPI_ERR_INVALID, "stem convolution: the workspace is too small");
+  p.partial = (float*)workspace;
+  CUtensorMap mdy;
+  if ((st = make_tmap_bf16_4d(&mdy, dy, {(uint64_t)stem::COUT, (uint64_t)p.OW, (uint64_t)p.OH, (uint64_t)N}, {64, (uint32_t)p.ow16, 1, 1}))) return st;
+  const int smem = stem::DY_STAGES * 2 * p.ow16 * 128 + 2 * stem::IN_ROWS * p.row_bytes + (int)sizeof(stem::Shared);
+  cudaError_t e = cudaFuncSetAttribute(stem::stem_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "stem weight gradient: shared memory attribute: %s", cudaGetErrorString(e));
+  stem::stem_wgrad_kernel<<<grid, stem::THREADS, smem, (cudaStream_t)stream>>>(mdy, p);
+  stem::stem_wgrad_reduce_kernel<<<stem::COUT, stem::RED_COLS * stem::RED_GROUPS, 0, (cudaStream_t)stream>>>(
+      (const float*)workspace, grid, (__nv_bfloat16*)dw, p.ws_co, p.ws_c, p.ws_h, p.ws_w);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "stem weight gradient launch: %s", cudaGetErrorString(e));
+}
+
+}  // extern "C"

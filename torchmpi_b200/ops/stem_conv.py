@@ -1,15 +1,16 @@
-"""The ResNet stem (7x7, stride 2, pad 3, 3 input channels) as im2col + tcgen05 GEMM.
+"""The ResNet stem (7x7, stride 2, pad 3, 3 input channels) on the tensor cores.
 
 ``StemConv7x7`` is an ``nn.Conv2d(3, C, 7, stride=2, padding=3, bias=False)`` with the same parameter
 (``weight [C, 3, 7, 7]``), so checkpoints and parameter counts do not change.  On a channels-last
-bf16 CUDA input, forward writes the patch matrix ``col [N*OH*OW, 160]`` with one kernel
-(csrc/kernels/im2col.cu) and multiplies it with the ``[C, 160]`` weight matrix on the tensor cores;
-the result is the channels-last output as it lies.  Backward needs only the weight gradient (the
-image has none): ``dW = dY^T col``, a split-K product on the same tensor-core kernel family over the saved
-patch matrix.  Other inputs take
-``F.conv2d``.
+bf16 CUDA input with 64 output channels and rows of up to 256 pixels, forward and weight gradient (the image
+has none) are implicit GEMMs that read the image itself (csrc/kernels/stem_conv.cu).  Other widths and channel
+counts go through the patch matrix ``col [N*OH*OW, 160]``, written by one kernel (csrc/kernels/im2col.cu) and
+multiplied with the ``[C, 160]`` weight matrix; their weight gradient is the split-K product ``dY^T col`` over the
+saved patch matrix.  Inputs that neither takes go to ``F.conv2d``.
 """
 from __future__ import annotations
+
+import ctypes
 
 import torch
 import torch.nn as nn
@@ -20,6 +21,54 @@ from . import gemm
 
 launch_count = 0
 PATCH = 147
+_ws = {}
+
+
+def _workspace(dev: torch.device) -> torch.Tensor:
+    """Per (device, stream) buffer for the partial sums of the weight gradient (one row of CTAs: 24 MB)."""
+    key = (dev.index, stream_ptr())
+    buf = _ws.get(key)
+    if buf is None:
+        buf = _ws[key] = torch.empty(lib.tmpi_stem_conv_wgrad_workspace_bytes(), dtype=torch.uint8, device=dev)
+    return buf
+
+
+class _StemDirectFn(torch.autograd.Function):
+    """The implicit GEMMs: nothing but the image is kept for backward."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        global launch_count
+        N, _, H, W = x.shape
+        y = torch.empty((N, w.shape[0], (H - 1) // 2 + 1, (W - 1) // 2 + 1), dtype=x.dtype, device=x.device,
+                        memory_format=torch.channels_last)
+        check(lib.tmpi_stem_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, w.shape[0],
+                                     (ctypes.c_int64 * 4)(*w.stride()), stream_ptr()))
+        launch_count += 1
+        ctx.save_for_backward(x)
+        ctx.wshape, ctx.wstride = tuple(w.shape), w.stride()
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        global launch_count
+        (x,) = ctx.saved_tensors
+        N, _, H, W = x.shape
+        dy = dy.contiguous(memory_format=torch.channels_last)
+        if dy.data_ptr() % 16:                                               # a view into a larger buffer
+            dy = dy.clone(memory_format=torch.channels_last)
+        dw = torch.empty_strided(ctx.wshape, ctx.wstride, dtype=x.dtype, device=x.device)
+        ws = _workspace(x.device)
+        check(lib.tmpi_stem_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, H, W, ctx.wshape[0],
+                                       (ctypes.c_int64 * 4)(*dw.stride()), ws.data_ptr(), ws.numel(), stream_ptr()))
+        launch_count += 2
+        return None, dw
+
+
+def direct(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a supported input takes the implicit GEMMs (every TMA row and the image itself 16-byte aligned)."""
+    return (has_symbol("tmpi_stem_conv_fwd") and x.data_ptr() % 16 == 0 and x.numel() > 0
+            and bool(lib.tmpi_stem_conv_supported(x.shape[3], w.shape[0])))
 
 
 def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -65,5 +114,7 @@ class StemConv7x7(nn.Conv2d):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if supported(x, self.weight):
+            if direct(x, self.weight):
+                return _StemDirectFn.apply(x, self.weight)
             return _StemConvFn.apply(x, self.weight)
         return F.conv2d(x, self.weight, None, self.stride, self.padding)
