@@ -142,3 +142,29 @@ def test_attention_backward_matches_fp32(B, T, H):
     dqkv2 = attention.attention_backward(qkv, out, lse, dout, H)
     assert torch.equal(dqkv[:, :, C:], dqkv2[:, :, C:])
     assert torch.allclose(dqkv[:, :, :C].float(), dqkv2[:, :, :C].float(), atol=1e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("B,T,H", [(5, 384, 24), (40, 128, 16), (1, 640, 1)])
+def test_attention_several_items_per_team_and_growing_maxima(B, T, H):
+    """More (block, head) items than persistent teams (rings and accumulators reused across items), and keys that grow
+    along the sequence, so that the running maximum of most rows moves in every block and O is rescaled."""
+    from torchmpi_b200.ops import attention
+    torch.manual_seed(B * T + H)
+    C = H * 64
+    qkv = torch.randn(B, T, 3 * C, device="cuda")
+    qkv[:, :, C:2 * C] *= torch.linspace(0.2, 2.5, T, device="cuda")[None, :, None]
+    qkv = qkv.to(torch.bfloat16)
+    leaf = qkv.detach().float().requires_grad_(True)
+    ref, ref_lse = _ref(leaf, H)
+    out, lse = attention.attention_forward(qkv, H)
+    dout = torch.randn_like(out)
+    dqkv = attention.attention_backward(qkv, out, lse, dout, H)
+    torch.cuda.synchronize()
+    attention.check_status()
+    ref.backward(dout.float())
+    assert torch.allclose(lse, ref_lse, atol=2e-3, rtol=1e-4), (lse - ref_lse).abs().max().item()
+    rel = lambda a, b: ((a.float() - b).norm() / b.norm()).item()
+    # bf16 P and outputs: 2^-9 relative rounding each; the gradients go through two more roundings (dS, the result)
+    assert rel(out, ref.detach()) < 6e-3, rel(out, ref.detach())
+    for name, sl in (("dq", slice(0, C)), ("dk", slice(C, 2 * C)), ("dv", slice(2 * C, 3 * C))):
+        assert rel(dqkv[:, :, sl], leaf.grad[:, :, sl]) < 1.5e-2, (name, rel(dqkv[:, :, sl], leaf.grad[:, :, sl]))

@@ -1,29 +1,43 @@
 // Causal self-attention forward (softmax(Q K^T / sqrt(d)) V, head size 64) as one tcgen05 kernel.
 //
 // The reference has no attention (its models are MNIST networks, examples/mnist/*.lua); the GPT-2 configuration
-// of this package needs one, and it is a contraction, so it belongs on the tensor cores.  One CTA handles one
-// block of 128 queries of one (batch, head) and walks the key / value blocks up to its diagonal:
+// of this package needs one, and it is a contraction, so it belongs on the tensor cores.  Work items are blocks of
+// 128 queries of one (batch, head); a CTA walks the key / value blocks of an item up to its diagonal:
 //
-//   warp 0     TMA producer: the Q tile once, then K tiles of 128 keys through a two-stage ring and V tiles through
-//              one buffer (V of the next block is fetched while its scores are exponentiated)
-//   warp 1     MMA issuer:   S = Q K^T (128 x 128, fp32, tensor memory), then O_j = P V (128 x 64, tensor memory)
-//   warps 2-9  softmax:      two threads per query row (tcgen05.ld 32x32b gives a thread its own row, so there are no
-//                            shuffles; both read the whole row for its maximum, each exponentiates 64 of the 128
-//                            scores): running maximum, P = exp2(scaled S - max) written as bf16 into shared memory
-//                            in the K-major 128-byte-swizzled layout that the second MMA reads, then the running
-//                            output acc = acc * alpha + O_j in registers (32 of the 64 columns per thread)
+//   one warp    TMA producer: Q tiles through two buffers (the next item's Q is fetched under the current one), K and V
+//               tiles of 128 keys through two-stage rings
+//   one warp    MMA issuer:   S = Q K^T (128 x 128, fp32, tensor memory), then O += P V (128 x 64) with P read from
+//               tensor memory and O accumulated there over all key blocks
+//   eight warps softmax:     two threads per query row, 64 scores each (tcgen05.ld 32x32b gives a thread its own row, so
+//                            there are no shuffles; the halves exchange their maxima through shared memory): the scores
+//                            go into registers at once, which frees S for the next block's MMA; maximum, P = exp2(scaled
+//                            S - m) as bf16 into tensor memory
 //
-// S for block j + 1 is issued as soon as the softmax warps have read S of block j, so the tensor core works on it
-// while they exponentiate, and the row maximum of block j + 1 is found while the tensor core multiplies P_j by V; a
-// quarter of the exponentials run as a cubic on the FMA pipe because the special-function unit (which also packs
-// fp32 pairs into bf16) is the busiest pipe of this kernel.  Two CTAs fit on an SM (256 tensor-memory columns and 96 KB of shared memory each), so
-// one CTA's softmax overlaps the other's MMAs.  Q, K and V are read where the fused QKV projection left them
-// ([B * T, 3 C], one tensor map per operand) and the output is written as [B * T, C]: no transposes around the
-// kernel.  Every wait is bounded; a CTA that gives up records where in the status word and frees its tensor memory.
+// What bounds it: neither the special-function unit (16 exp2 per cycle and SM, 1024 cycles per 128 x 128 block; a quarter of
+// them run as a cubic on the FMA pipe) nor the MMAs (512 cycles per block), but the latency of a team's chain S -> maximum
+// -> P -> P V, about 1.9 us per key block.  Everything that is not needed per score is therefore kept off the softmax
+// warps: P goes to tensor memory (no shared-memory stores, swizzle arithmetic or proxy fence), and O stays in tensor
+// memory: only where a row's maximum grew do its threads scale O there by exp2(old max - new max), instead of reading every
+// O_j back.  Tried and taken back: moving the maximum only when it grows by more than 2^8 (the largest P of a row is then
+// no longer exactly 1, and its bf16 rounding showed in the output); one thread per row (63 us in place of 56); all
+// exponentials before the wait for the previous product (61); descriptors in uniform registers (no difference).
+//
+// A CTA (one per SM) runs two such teams, each with its own items, rings, barriers and 256 tensor-memory columns, so that
+// one exponentiates while the other waits.  Teams are persistent and take items longest-first in snake order (item
+// r * G + i, then r * G + G - 1 - i), which leaves the key blocks per team within one of each other at 8 x 16 x 1024; the
+// next item's loads and first S run under the end of the current one.
+//
+// Measured on a B200, back to back: 8 x 16 heads x 1024 x 64 64.2 -> 55.7 us, 1 x 16 x 2048 36.5 -> 32.7; before, P went
+// through shared memory and O through registers for each block, and every thread read the whole row for its maximum.
+//
+// Q, K and V are read where the fused QKV projection left them ([B * T, 3 C], one tensor map per operand) and the
+// output is written as [B * T, C]: no transposes around the kernel.  Every wait is bounded; a CTA that gives up records
+// where in the status word and frees its tensor memory.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <algorithm>
 #include <mutex>
 #include "sm100_ptx.cuh"
 #include "attn_util.cuh"
@@ -34,31 +48,32 @@ using namespace tmpi;
 
 namespace tmpi {
 int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+int gemm_sm_count();
 }
 
 namespace attn {
 using namespace attn_util;
 
-constexpr int BQ = 128, BKV = 128, D = 64, THREADS = 320, UMMA_K = 16;
+constexpr int BQ = 128, BKV = 128, D = 64, TEAMS = 2, SOFTMAX_WARPS = 8, UMMA_K = 16;
+constexpr int THREADS = 32 * TEAMS * (2 + SOFTMAX_WARPS);
 constexpr int TILE_BYTES = 128 * D * 2;                       // a 128 x 64 bf16 tile: 16 KB
-constexpr int P_BYTES = BQ * BKV * 2;                         // 32 KB: two K-major chunks of 64 keys
-constexpr int SMEM_TILES = TILE_BYTES * 4 + P_BYTES;          // Q, K x 2, V, P
-constexpr int V_OFF = TILE_BYTES * 3;                          // P follows the one or two V buffers
-constexpr int SMEM_SHARED = 256;                              // the barrier block follows the tiles
-constexpr int TMEM_COLS = 256;                                // S: columns 0-127, O_j: columns 128-191
+constexpr int Q_OFF = 0, K_OFF = 2 * TILE_BYTES, V_OFF = 4 * TILE_BYTES, SMEM_TILES = 6 * TILE_BYTES;
+constexpr int SMEM_SHARED = 256;                              // the teams' barrier blocks follow their tiles
+constexpr int XCH_BYTES = 2 * 2 * BQ * 4;                     // two phases x two halves of the rows: values the halves exchange
+constexpr int SMEM_BYTES = TEAMS * (SMEM_TILES + SMEM_SHARED + XCH_BYTES);
+constexpr int TMEM_COLS = 256, TMEM_P = 128, TMEM_O = 192;    // S: columns 0-127 of a team, P (bf16 pairs): 128-191, O: 192-255
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_full, o_full;
-  uint64_t pair[4];            // the 64 threads that share 32 rows meet here (bounded, unlike a named barrier)
+  uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_full, pv_done, o_empty;
+  uint64_t pair[4];            // the two warps that share 32 rows meet here (bounded, unlike a named barrier)
   uint32_t tmem_base;
   int error;
 };
 static_assert(sizeof(Shared) <= SMEM_SHARED, "barrier block");
 
 struct Params {
-  int B, T, H, q_blocks;
-  int v_stages;                // 1 or 2 V buffers (2 prefetches V a block ahead and costs 16 KB of shared memory)
+  int B, T, H, q_blocks, items;
   float scale_log2;            // softmax scale times log2(e)
   __nv_bfloat16* out;          // [B * T, ld_out], head h at columns h * 64
   int ld_out;
@@ -72,315 +87,342 @@ __device__ __forceinline__ void fail(Shared* sh, const Params& p, int where) {
   if (p.status) atomicCAS(p.status, 0, 3000 + where);
 }
 
-// Phase time stamps of one CTA for tuning: slot = (block * 16 + event), written by one thread per role.
-__device__ __forceinline__ void stamp(const Params& p, int j, int ev) {
-  if (p.trace && blockIdx.x == 0) p.trace[j * 16 + ev] = sm100::now_ns();
+// Warps 0-1 are the producers of the two teams, 2-3 the MMA issuers, 4-11 and 12-19 the softmax warps.
+__device__ __forceinline__ int team() {
+  const int warp = threadIdx.x >> 5;
+  return warp < 4 ? warp & 1 : (warp - 4) / SOFTMAX_WARPS;
+}
+
+// Phase time stamps of one team's first item for tuning: slot = (block * 16 + event), written by one thread per role.
+__device__ __forceinline__ void stamp(const Params& p, int round, int j, int ev) {
+  if (p.trace && blockIdx.x == 0 && round == 0 && team() == 0) p.trace[j * 16 + ev] = sm100::now_ns();
+}
+
+// The item of this team in a round: (batch, head) and query block, long ones (late query blocks) first, every other
+// round in reverse so that a team that got a long item gets a short one next.
+__device__ __forceinline__ bool item(const Params& p, int round, int* bh, int* qblk) {
+  const int g = TEAMS * (int)gridDim.x, i = (int)blockIdx.x + team() * (int)gridDim.x;
+  const long long t = (long long)round * g + ((round & 1) ? g - 1 - i : i);
+  if (t >= p.items) return false;
+  const int n = p.B * p.H;
+  *qblk = p.q_blocks - 1 - (int)(t / n);
+  *bh = (int)(t % n);
+  return true;
 }
 
 #define ATTN_WAIT(bar, parity, where) \
   do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
 
 __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
-                         const CUtensorMap* mv, int b, int h, int qblk) {
-  const int row0 = b * p.T;
-  sm100::mbar_expect_tx(&sh->q_full, TILE_BYTES);
-  sm100::tma_load_2d(tiles, mq, h * D, row0 + qblk * BQ, &sh->q_full);
-  auto load_k = [&](int j) {
-    sm100::mbar_expect_tx(&sh->k_full[j & 1], TILE_BYTES);
-    sm100::tma_load_2d(tiles + TILE_BYTES * (1 + (j & 1)), mk, h * D, row0 + j * BKV, &sh->k_full[j & 1]);
-  };
-  load_k(0);
-  for (int j = 0; j <= qblk; ++j) {
-    if (j < qblk) {                                                        // K runs one block ahead of V
-      if (j + 1 >= 2) ATTN_WAIT(&sh->k_empty[(j + 1) & 1], (((j + 1) >> 1) - 1) & 1, 1);   // S of block j - 1 has read this stage
-      load_k(j + 1);
+                         const CUtensorMap* mv) {
+  int kc = 0, vc = 0, bh, qblk;                            // K and V tiles loaded so far, over all items
+  for (int r = 0; item(p, r, &bh, &qblk); ++r) {
+    const int b = bh / p.H, h = bh - b * p.H, row0 = b * p.T;
+    auto load_k = [&](int j) -> bool {
+      const int st = kc & 1;
+      if (kc >= 2 && (!sm100::mbar_wait(&sh->k_empty[st], ((kc >> 1) - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
+      sm100::mbar_expect_tx(&sh->k_full[st], TILE_BYTES);
+      sm100::tma_load_2d(tiles + K_OFF + st * TILE_BYTES, mk, h * D, row0 + j * BKV, &sh->k_full[st]);
+      ++kc;
+      return true;
+    };
+    if (r >= 2) ATTN_WAIT(&sh->q_empty[r & 1], ((r >> 1) - 1) & 1, 12);
+    sm100::mbar_expect_tx(&sh->q_full[r & 1], TILE_BYTES);
+    sm100::tma_load_2d(tiles + Q_OFF + (r & 1) * TILE_BYTES, mq, h * D, row0 + qblk * BQ, &sh->q_full[r & 1]);
+    if (!load_k(0)) { fail(sh, p, 1); return; }
+    for (int j = 0; j <= qblk; ++j) {
+      if (j < qblk && !load_k(j + 1)) { fail(sh, p, 1); return; }          // K runs one block ahead of V
+      const int st = vc & 1;
+      if (vc >= 2) ATTN_WAIT(&sh->v_empty[st], ((vc >> 1) - 1) & 1, 13);
+      sm100::mbar_expect_tx(&sh->v_full[st], TILE_BYTES);
+      sm100::tma_load_2d(tiles + V_OFF + st * TILE_BYTES, mv, h * D, row0 + j * BKV, &sh->v_full[st]);
+      ++vc;
     }
-    const int vs = p.v_stages == 2 ? (j & 1) : 0, vuse = p.v_stages == 2 ? (j >> 1) : j;
-    if (vuse >= 1) ATTN_WAIT(&sh->v_empty[vs], (vuse - 1) & 1, 13);        // the P V that read this buffer is done
-    sm100::mbar_expect_tx(&sh->v_full[vs], TILE_BYTES);
-    sm100::tma_load_2d(tiles + V_OFF + vs * TILE_BYTES, mv, h * D, row0 + j * BKV, &sh->v_full[vs]);
   }
 }
 
-__device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p, int qblk) {
-  const uint32_t tmem_s = sh->tmem_base, tmem_o = sh->tmem_base + 128;
-  const uint32_t q_addr = sm100::smem_u32(tiles), p_addr = sm100::smem_u32(tiles + V_OFF + p.v_stages * TILE_BYTES);
+__device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
+  const uint32_t tmem_s = sh->tmem_base, tmem_p = sh->tmem_base + TMEM_P, tmem_o = sh->tmem_base + TMEM_O;
   constexpr uint32_t idesc_s = sm100::make_idesc_f16(BQ, BKV, true);            // Q and K both K-major
-  constexpr uint32_t idesc_o = sm100::make_idesc_f16(BQ, D, true, true);        // P K-major, V MN-major (d contiguous)
-  // descriptors of every operand slice, built once
-  uint64_t dq[D / UMMA_K], dk[2][D / UMMA_K], dp[BKV / UMMA_K], dv[2][BKV / UMMA_K];
-  const uint32_t v_addr = sm100::smem_u32(tiles + V_OFF);
-#pragma unroll
-  for (int k = 0; k < D / UMMA_K; ++k) {
-    dq[k] = sm100::make_desc_sw128(q_addr + k * UMMA_K * 2);
-    dk[0][k] = sm100::make_desc_sw128(sm100::smem_u32(tiles + TILE_BYTES) + k * UMMA_K * 2);
-    dk[1][k] = sm100::make_desc_sw128(sm100::smem_u32(tiles + 2 * TILE_BYTES) + k * UMMA_K * 2);
-  }
-#pragma unroll
-  for (int k = 0; k < BKV / UMMA_K; ++k) {
-    dp[k] = sm100::make_desc_sw128(p_addr + (k >> 2) * TILE_BYTES + (k & 3) * UMMA_K * 2);
-    dv[0][k] = sm100::make_desc_sw128_mn(v_addr + k * UMMA_K * 128, TILE_BYTES, 1024);
-    dv[1][k] = sm100::make_desc_sw128_mn(v_addr + TILE_BYTES + k * UMMA_K * 128, TILE_BYTES, 1024);
-  }
-  auto issue_s = [&](int j) {
-    if (j & 1) {
-#pragma unroll
-      for (int k = 0; k < D / UMMA_K; ++k) sm100::umma_f16(tmem_s, dq[k], dk[1][k], idesc_s, k > 0 ? 1u : 0u);
-    } else {
-#pragma unroll
-      for (int k = 0; k < D / UMMA_K; ++k) sm100::umma_f16(tmem_s, dq[k], dk[0][k], idesc_s, k > 0 ? 1u : 0u);
-    }
-    sm100::umma_commit(&sh->s_full);
-    sm100::umma_commit(&sh->k_empty[j & 1]);
-  };
-  ATTN_WAIT(&sh->q_full, 0, 2);
-  ATTN_WAIT(&sh->k_full[0], 0, 3);
-  sm100::tc_fence_after();
-  issue_s(0);
-  for (int j = 0; j <= qblk; ++j) {
-    if (j < qblk) {                      // S of the next block, as soon as this block's S has been read
-      ATTN_WAIT(&sh->s_empty, j & 1, 4);
-      stamp(p, j, 8);
-      ATTN_WAIT(&sh->k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, 5);
-      sm100::tc_fence_after();
-      issue_s(j + 1);
-      stamp(p, j, 9);
-    }
-    ATTN_WAIT(&sh->p_full, j & 1, 6);
-    stamp(p, j, 10);
-    const int vs = p.v_stages == 2 ? (j & 1) : 0, vuse = p.v_stages == 2 ? (j >> 1) : j;
-    ATTN_WAIT(&sh->v_full[vs], vuse & 1, 14);
-    stamp(p, j, 11);
+  constexpr uint32_t idesc_o = sm100::make_idesc_f16(BQ, D, true, true);        // P in tensor memory, V MN-major (d contiguous)
+  const uint64_t dq = sm100::make_desc_sw128(sm100::smem_u32(tiles + Q_OFF));
+  const uint64_t dk = sm100::make_desc_sw128(sm100::smem_u32(tiles + K_OFF));
+  const uint64_t dv = sm100::make_desc_sw128_mn(sm100::smem_u32(tiles + V_OFF), TILE_BYTES, 1024);
+  // a slice further into shared memory only adds to the address field (bytes / 16 in the low 14 bits)
+  auto at = [](uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); };
+  int g = 0;                                               // key blocks whose S has been issued, over all items
+  int bh, qblk;
+  // S of key block j of round r (block number g): waits for the softmax warps to have read the previous S
+  auto issue_s = [&](int r, int j, int last) -> bool {
+    if (j == 0 && (!sm100::mbar_wait(&sh->q_full[r & 1], (r >> 1) & 1, kWaitBudgetNs) || sh->error)) return false;
+    if (!sm100::mbar_wait(&sh->k_full[g & 1], (g >> 1) & 1, kWaitBudgetNs) || sh->error) return false;
+    if (g >= 1 && (!sm100::mbar_wait(&sh->s_empty, (g - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
     sm100::tc_fence_after();
-    if (vs) {
+    const uint64_t a = at(dq, (r & 1) * TILE_BYTES), b = at(dk, (g & 1) * TILE_BYTES);
 #pragma unroll
-      for (int k = 0; k < BKV / UMMA_K; ++k) sm100::umma_f16(tmem_o, dp[k], dv[1][k], idesc_o, k > 0 ? 1u : 0u);
-    } else {
+    for (int k = 0; k < D / UMMA_K; ++k)
+      sm100::umma_f16(tmem_s, at(a, k * UMMA_K * 2), at(b, k * UMMA_K * 2), idesc_s, k > 0 ? 1u : 0u);
+    sm100::umma_commit(&sh->s_full);
+    sm100::umma_commit(&sh->k_empty[g & 1]);
+    if (j == last) sm100::umma_commit(&sh->q_empty[r & 1]);
+    ++g;
+    return true;
+  };
+  bool more = item(p, 0, &bh, &qblk);
+  if (more && !issue_s(0, 0, qblk)) { fail(sh, p, 3); return; }
+  int v = 0;                                               // P V products issued so far
+  for (int r = 0; more; ++r) {
+    const int last = qblk;
+    more = item(p, r + 1, &bh, &qblk);                     // the next round's item: its first S runs before this one's last P V
+    for (int j = 0; j <= last; ++j) {
+      if (j < last) {
+        stamp(p, r, j, 8);
+        if (!issue_s(r, j + 1, last)) { fail(sh, p, 4); return; }
+        stamp(p, r, j, 9);
+      } else if (more) {
+        if (!issue_s(r + 1, 0, qblk)) { fail(sh, p, 5); return; }
+      }
+      if (j == 0 && r > 0) ATTN_WAIT(&sh->o_empty, (r - 1) & 1, 14);       // the previous item's output has been read
+      ATTN_WAIT(&sh->p_full, v & 1, 6);
+      stamp(p, r, j, 10);
+      ATTN_WAIT(&sh->v_full[v & 1], (v >> 1) & 1, 15);
+      stamp(p, r, j, 11);
+      sm100::tc_fence_after();
+      const uint64_t b = at(dv, (v & 1) * TILE_BYTES);
 #pragma unroll
-      for (int k = 0; k < BKV / UMMA_K; ++k) sm100::umma_f16(tmem_o, dp[k], dv[0][k], idesc_o, k > 0 ? 1u : 0u);
+      for (int k = 0; k < BKV / UMMA_K; ++k)               // 16 keys: eight columns of packed P, 16 rows of V
+        sm100::umma_f16_tmem_a(tmem_o, tmem_p + k * (UMMA_K / 2), at(b, k * UMMA_K * 128), idesc_o, (j | k) ? 1u : 0u);
+      sm100::umma_commit(&sh->pv_done);
+      sm100::umma_commit(&sh->v_empty[v & 1]);
+      stamp(p, r, j, 12);
+      ++v;
     }
-    sm100::umma_commit(&sh->o_full);
-    sm100::umma_commit(&sh->v_empty[vs]);
-    stamp(p, j, 12);
   }
 }
 
-// One thread's 64 scores of a block: P = exp2(S * c2 + nmc) as bf16 into the swizzled K-major tile; returns their sum.
-// DIAG: the block on the diagonal, where a key after the query gives 0 and whole chunks of 32 keys may be masked
-// for the warp (then there is nothing to load or exponentiate).
-template <bool DIAG>
-__device__ __forceinline__ float exp_pass(Shared* sh, uint32_t (&r)[32], uint32_t tmem_s, unsigned char* p_row, int row, int half,
-                                          int last_row, float c2, float nmc) {
+// Scores s[0, 32) of one row (a chunk of 32 keys) -> sixteen packed bf16 pairs of exp2(s * c2 + nmc), added to the row
+// sums.  A quarter of the exponentials run on the FMA pipe, the rest on the special-function unit; a masked score (-inf)
+// gives 0 there and 2^-120 here, which no sum that holds the row's maximum (1) can tell from 0.
+__device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint32_t (&w)[16], unsigned long long c2x2,
+                                          unsigned long long nmc2, unsigned long long& sum2) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    float a0, a1;
+    unpack2(fma2(pack2(s[2 * i], s[2 * i + 1]), c2x2, nmc2), a0, a1);
+    const bool fma_pipe = (i & 3) == 3;
+    const float e0 = fma_pipe ? ex2_fma(a0) : ex2(a0);
+    const float e1 = fma_pipe ? ex2_fma(a1) : ex2(a1);
+    sum2 = add2(sum2, pack2(__float_as_uint(e0), __float_as_uint(e1)));
+    w[i] = pack_bf16(__float_as_uint(e0), __float_as_uint(e1));
+  }
+}
+
+// Two threads per query row: `half` picks 64 of the 128 scores of a block and 32 of the 64 output columns.  The halves
+// exchange their maxima through shared memory, block by block, and their row sums at the end of an item.
+__device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarter, int half, int lane) {
+  const int row = quarter * 32 + lane;                     // the row of the tile; its tensor-memory lane
+  const uint32_t tmem = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
+  const uint32_t tmem_s = tmem + half * 64, tmem_p = tmem + TMEM_P + half * 32, tmem_o = tmem + TMEM_O + half * 32;
+  const float c2 = p.scale_log2;
   const unsigned long long c2x2 = pack2(__float_as_uint(c2), __float_as_uint(c2));
-  const unsigned long long nmc2 = pack2(__float_as_uint(nmc), __float_as_uint(nmc));
-  unsigned long long rs2 = 0ull;                          // two partial sums (0.f, 0.f)
-#pragma unroll 1
-  for (int c = 0; c < 2; ++c) {
-    const int key0 = half * 64 + c * 32;
-    const bool masked = DIAG && key0 > last_row;           // warp-uniform
-    if (!masked) {
-      sm100::tmem_ld_32x32(tmem_s + c * 32, r);
+  const bool tracer = row == 0 && half == 0;
+  int g = 0, met = 0, bh, qblk;                            // key blocks done and exchanges made so far, over all items
+  // this row's value of the other half
+  auto exchange = [&](float v, float* other) -> bool {
+    float* x = xch + (met & 1) * 2 * BQ;
+    x[half * BQ + row] = v;
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive(&sh->pair[quarter]);
+    if (!sm100::mbar_wait(&sh->pair[quarter], met & 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 11); return false; }
+    *other = x[(half ^ 1) * BQ + row];
+    ++met;
+    return true;
+  };
+  for (int r = 0; item(p, r, &bh, &qblk); ++r) {
+    float m = -INFINITY;                                   // the running maximum
+    unsigned long long sum2[2] = {0ull, 0ull};
+    for (int j = 0; j <= qblk; ++j, ++g) {
+      const bool diag = j == qblk;
+      uint32_t s[2][32];
+      if (tracer) stamp(p, r, j, 0);
+      ATTN_WAIT(&sh->s_full, g & 1, 7);
+      if (tracer) stamp(p, r, j, 1);
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) sm100::tmem_ld_32x32(tmem_s + c * 32, s[c]);
       sm100::tmem_ld_wait();
-    }
-    if (c == 1) {                                         // S is in registers: the next S may overwrite it
       sm100::tc_fence_before();
-      sm100::mbar_arrive(&sh->s_empty);
-    }
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->s_empty);     // S is in registers: the next S may overwrite it
+      if (diag) {                                          // keys after the query
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {                          // eight keys = one 16-byte unit of the swizzled row
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
-      if (!masked) {
+        for (int c = 0; c < 2; ++c) {
+          const int chunk = half * 2 + c;
+          if (chunk >= quarter) {                          // warp-uniform
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = u * 8 + 2 * q;
-          float a0, a1;
-          unpack2(fma2(pack2(r[i], r[i + 1]), c2x2, nmc2), a0, a1);
-          // a quarter of the exponentials on the FMA pipe, the rest on the special-function unit
-          float e0 = q == 3 ? ex2_fma(a0) : ex2(a0);
-          float e1 = q == 3 ? ex2_fma(a1) : ex2(a1);
-          if (DIAG) {
-            if (key0 + i > row) e0 = 0.f;
-            if (key0 + i + 1 > row) e1 = 0.f;
+            for (int i = 0; i < 32; ++i)
+              if (chunk > quarter || i > lane) s[c][i] = 0xff800000u;
           }
-          rs2 = add2(rs2, pack2(__float_as_uint(e0), __float_as_uint(e1)));
-          __nv_bfloat162 hh = __floats2bfloat162_rn(e0, e1);
-          w[q] = *reinterpret_cast<uint32_t*>(&hh);
         }
       }
-      const int unit = c * 4 + u;
-      *reinterpret_cast<uint4*>(p_row + ((unit ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-  }
-  float rs0, rs1;
-  unpack2(rs2, rs0, rs1);
-  return rs0 + rs1;
-}
-
-// Two threads per query row: the warps with the same (warp & 3) read the same 32 tensor-memory lanes; `half` picks
-// which 64 of the 128 score columns a thread exponentiates (and which 32 of the 64 output columns it accumulates).
-// Both read the whole row for its maximum (tensor-memory reads are cheap and this needs no exchange); each keeps
-// the partial row sum of its own columns, and the two are added once at the end through shared memory.
-__device__ void softmax_rows(Shared* sh, unsigned char* tiles, const Params& p, int b, int h, int qblk, int quarter, int half,
-                             int lane) {
-  const int row = quarter * 32 + lane;
-  const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-  const uint32_t tmem_row = sh->tmem_base + lane_base, tmem_s = tmem_row + half * 64;
-  const uint32_t tmem_o = sh->tmem_base + 128 + lane_base + half * 32;
-  unsigned char* p_tile = tiles + V_OFF + p.v_stages * TILE_BYTES;
-  unsigned char* p_row = p_tile + half * TILE_BYTES + row * 128;      // chunk `half`: keys 64 half ...
-  float* xch = reinterpret_cast<float*>(p_tile);     // the P tile, once the last MMA has read it
-  const float c2 = p.scale_log2;
-  float m = -INFINITY, l = 0.f;
-  unsigned long long acc2[D / 4];                         // this thread's 32 output columns, two per register pair
+      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;      // four chains
 #pragma unroll
-  for (int i = 0; i < D / 4; ++i) acc2[i] = 0ull;
-  uint32_t r[32];
-  const int last_row = quarter * 32 + 31;                 // a chunk of keys beyond it is masked for the whole warp
-  // the maximum of the row over block j (on the diagonal block a key after the query is masked)
-  auto row_max = [&](int j, float mx) {
-    const bool diag = j == qblk;
-#pragma unroll 1
-    for (int c = 0; c < BKV / 32; ++c) {
-      if (diag && c * 32 > last_row) break;
-      sm100::tmem_ld_32x32(tmem_row + c * 32, r);
-      sm100::tmem_ld_wait();
-      if (!diag) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (c * 32 + i <= row) mx = fmaxf(mx, __uint_as_float(r[i]));
+      for (int i = 0; i < 32; i += 4) {
+        mx0 = max3(mx0, __uint_as_float(s[0][i]), __uint_as_float(s[0][i + 1]));
+        mx1 = max3(mx1, __uint_as_float(s[0][i + 2]), __uint_as_float(s[0][i + 3]));
+        mx2 = max3(mx2, __uint_as_float(s[1][i]), __uint_as_float(s[1][i + 1]));
+        mx3 = max3(mx3, __uint_as_float(s[1][i + 2]), __uint_as_float(s[1][i + 3]));
       }
+      float mx = fmaxf(max3(mx0, mx1, mx2), mx3), mx_other;
+      if (!exchange(mx, &mx_other)) return;
+      mx = fmaxf(mx, mx_other);
+      if (tracer) stamp(p, r, j, 2);
+      // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
+      const float next = fmaxf(m, mx);
+      const bool grew = j > 0 && __any_sync(~0u, next > m);
+      const float alpha = ex2((m - next) * c2);
+      const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
+      m = next;
+      if (grew) { sum2[0] = mul2(sum2[0], al2); sum2[1] = mul2(sum2[1], al2); }
+      const float nmc = -m * c2;
+      const unsigned long long nmc2 = pack2(__float_as_uint(nmc), __float_as_uint(nmc));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t w[16], o[2][16];
+        if (diag && half * 2 + c > quarter) {              // every key of the chunk is after every query of the warp
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = 0u;
+        } else {
+          exp_chunk(s[c], w, c2x2, nmc2, sum2[c]);
+        }
+        if (c == 0 && g > 0) {     // the previous block's product has read its P and added to O
+          ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 8);
+          if (tracer && j > 0) { stamp(p, r, j - 1, 5); stamp(p, r, j - 1, 6); }
+          sm100::tc_fence_after();
+        }
+        sm100::tmem_st_32x16(tmem_p + c * 16, w);
+        if (c == 1 && grew) {                              // the scores are spent: their registers hold O
+          sm100::tmem_ld_32x16(tmem_o, o[0]);
+          sm100::tmem_ld_32x16(tmem_o + 16, o[1]);
+          sm100::tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float a0, a1;
+              unpack2(mul2(pack2(o[q][i], o[q][i + 1]), al2), a0, a1);
+              o[q][i] = __float_as_uint(a0); o[q][i + 1] = __float_as_uint(a1);
+            }
+            sm100::tmem_st_32x16(tmem_o + q * 16, o[q]);
+          }
+        }
+      }
+      sm100::tmem_st_wait();
+      if (tracer) stamp(p, r, j, 3);
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->p_full);
+      if (tracer) stamp(p, r, j, 4);
     }
-    return mx;
-  };
-  const bool tracer = row == 0 && half == 0;
-  if (tracer) stamp(p, 0, 0);
-  ATTN_WAIT(&sh->s_full, 0, 7);
-  if (tracer) stamp(p, 0, 1);
-  sm100::tc_fence_after();
-  float mx = row_max(0, m);
-  for (int j = 0; j <= qblk; ++j) {
-    const bool diag = j == qblk;
-    if (tracer) stamp(p, j, 2);
-    const float alpha = ex2((m - mx) * c2);             // 0 for the first block (m = -inf)
-    const float nmc = -mx * c2;
-    // second pass: P = exp2(S * c2 - max * c2) as bf16 into the swizzled K-major tile
-    const float rs = diag ? exp_pass<true>(sh, r, tmem_s, p_row, row, half, last_row, c2, nmc)
-                          : exp_pass<false>(sh, r, tmem_s, p_row, row, half, last_row, c2, nmc);
-    l = l * alpha + rs;
-    m = mx;
-    if (tracer) stamp(p, j, 3);
-    sm100::fence_proxy_async_smem();                      // the MMA reads P through the async proxy
-    sm100::mbar_arrive(&sh->p_full);
-    if (tracer) stamp(p, j, 4);
-    // while the tensor core multiplies P by V: the maximum of the next block's scores, which are already there
-    if (j < qblk) {
-      ATTN_WAIT(&sh->s_full, (j + 1) & 1, 7);
-      if (tracer) stamp(p, j + 1, 1);
-      sm100::tc_fence_after();
-      mx = row_max(j + 1, m);
-    }
-    // running output: this thread's 32 columns
-    ATTN_WAIT(&sh->o_full, j & 1, 8);
-    if (tracer) stamp(p, j, 5);
+    // the item's output: O / l
+    float l0, l1, l_other;
+    unpack2(add2(sum2[0], sum2[1]), l0, l1);
+    if (!exchange(l0 + l1, &l_other)) return;
+    const float l = half ? l_other + (l0 + l1) : (l0 + l1) + l_other, inv = 1.f / l;
+    ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
+    if (tracer) stamp(p, r, qblk, 5);
     sm100::tc_fence_after();
-    sm100::tmem_ld_32x32(tmem_o, r);
+    uint32_t o[32];
+    sm100::tmem_ld_32x32(tmem_o, o);
     sm100::tmem_ld_wait();
-    const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) acc2[i] = fma2(acc2[i], al2, pack2(r[2 * i], r[2 * i + 1]));
-    if (tracer) stamp(p, j, 6);
     sm100::tc_fence_before();
-  }
-  // the row sum is the sum of the two halves' partial sums (the last o_full says that the MMAs are done with P)
-  xch[half * 128 + row] = l;
-  sm100::mbar_arrive(&sh->pair[quarter]);
-  ATTN_WAIT(&sh->pair[quarter], 0, 11);
-  l += xch[(half ^ 1) * 128 + row];
-  const float inv = 1.f / l;
-  const size_t grow = (size_t)b * p.T + (size_t)qblk * BQ + row;
-  __nv_bfloat16* o = p.out + grow * p.ld_out + h * D + half * 32;
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive(&sh->o_empty);
+    const int b = bh / p.H, h = bh - b * p.H;
+    const size_t t = (size_t)qblk * BQ + row;
+    __nv_bfloat16* out = p.out + ((size_t)b * p.T + t) * p.ld_out + h * D + half * 32;
 #pragma unroll
-  for (int u = 0; u < D / 16; ++u) {
-    uint32_t w[4];
+    for (int u = 0; u < 4; ++u) {
+      uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float a0, a1;
-      unpack2(acc2[u * 4 + i], a0, a1);
-      __nv_bfloat162 hh = __floats2bfloat162_rn(a0 * inv, a1 * inv);
-      w[i] = *reinterpret_cast<uint32_t*>(&hh);
+      for (int i = 0; i < 4; ++i)
+        w[i] = pack_bf16(__float_as_uint(__uint_as_float(o[u * 8 + 2 * i]) * inv), __float_as_uint(__uint_as_float(o[u * 8 + 2 * i + 1]) * inv));
+      *reinterpret_cast<uint4*>(out + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    *reinterpret_cast<uint4*>(o + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (p.lse && half == 0) p.lse[(size_t)bh * p.T + t] = m * c2 * 0.6931471805599453f + __logf(l);
+    if (tracer) stamp(p, r, qblk, 6);
   }
-  if (p.lse && half == 0) p.lse[((size_t)b * p.H + h) * p.T + (size_t)qblk * BQ + row] = m * c2 * 0.6931471805599453f + __logf(l);
 }
 
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(THREADS, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const Params p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];   // no static shared memory: the tiles start aligned
-  unsigned char* tiles = smem_raw;
-  Shared* sh = (Shared*)(smem_raw + SMEM_TILES + (p.v_stages - 1) * TILE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the longest rows of blocks (near the end of the sequence) start first
-  const int bh = blockIdx.x % (p.B * p.H);
-  const int qblk = p.q_blocks - 1 - blockIdx.x / (p.B * p.H);
-  const int b = bh / p.H, h = bh - b * p.H;
-  if (warp == 0 && sm100::elect_one()) {
+  unsigned char* tiles = smem_raw + team() * SMEM_TILES;
+  Shared* sh = (Shared*)(smem_raw + TEAMS * SMEM_TILES + team() * SMEM_SHARED);
+  if (warp < 2 && sm100::elect_one()) {
     sm100::tma_prefetch_desc(&map_q);
     sm100::tma_prefetch_desc(&map_k);
     sm100::tma_prefetch_desc(&map_v);
-    sm100::mbar_init(&sh->q_full, 1);
-    for (int s = 0; s < 2; ++s) { sm100::mbar_init(&sh->k_full[s], 1); sm100::mbar_init(&sh->k_empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { sm100::mbar_init(&sh->v_full[s], 1); sm100::mbar_init(&sh->v_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) {
+      sm100::mbar_init(&sh->q_full[s], 1); sm100::mbar_init(&sh->q_empty[s], 1);
+      sm100::mbar_init(&sh->k_full[s], 1); sm100::mbar_init(&sh->k_empty[s], 1);
+      sm100::mbar_init(&sh->v_full[s], 1); sm100::mbar_init(&sh->v_empty[s], 1);
+    }
     sm100::mbar_init(&sh->s_full, 1);
-    sm100::mbar_init(&sh->s_empty, 256);
-    sm100::mbar_init(&sh->p_full, 256);
-    sm100::mbar_init(&sh->o_full, 1);
-    for (int q = 0; q < 4; ++q) sm100::mbar_init(&sh->pair[q], 64);
+    sm100::mbar_init(&sh->s_empty, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->p_full, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->pv_done, 1);
+    sm100::mbar_init(&sh->o_empty, SOFTMAX_WARPS);
+    for (int q = 0; q < 4; ++q) sm100::mbar_init(&sh->pair[q], 2);
     sh->error = 0;
     sm100::fence_barrier_init();
   }
-  if (warp == 1) {
-    sm100::tmem_alloc(&sh->tmem_base, TMEM_COLS);
+  Shared* sh0 = (Shared*)(smem_raw + TEAMS * SMEM_TILES);
+  if (warp == 2) {
+    sm100::tmem_alloc(&sh0->tmem_base, TEAMS * TMEM_COLS);
     sm100::tmem_relinquish();
   }
   sm100::tc_fence_before();
   __syncthreads();
   sm100::tc_fence_after();
+  if (threadIdx.x == 0) ((Shared*)((unsigned char*)sh0 + SMEM_SHARED))->tmem_base = sh0->tmem_base + TMEM_COLS;
+  __syncthreads();
 
   // the swizzled tiles need a 1024-byte aligned base
   const bool fits = (sm100::smem_u32(tiles) & 1023u) == 0;
   if (!fits) {
-    if (threadIdx.x == 0) fail(sh, p, 9);
-  } else if (warp == 0) {
-    if (sm100::elect_one()) producer(sh, tiles, p, &map_q, &map_k, &map_v, b, h, qblk);
-  } else if (warp == 1) {
-    if (sm100::elect_one()) mma_issuer(sh, tiles, p, qblk);
+    if (lane == 0) fail(sh, p, 9);
+  } else if (warp < 4) {                                   // registers per four warps: 56 + 4 * 104 of the launch's 5 * 96
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp < 2) {
+      if (sm100::elect_one()) producer(sh, tiles, p, &map_q, &map_k, &map_v);
+    } else {
+      if (sm100::elect_one()) mma_issuer(sh, tiles, p);
+    }
   } else {
-    softmax_rows(sh, tiles, p, b, h, qblk, warp & 3, (warp - 2) >> 2, lane);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    float* xch = (float*)(smem_raw + TEAMS * (SMEM_TILES + SMEM_SHARED) + team() * XCH_BYTES);
+    softmax_rows(sh, xch, p, warp & 3, ((warp - 4) >> 2) & 1, lane);
   }
   __syncwarp();
   sm100::tc_fence_before();
   __syncthreads();
-  if (sh->error && warp == 0 && sm100::elect_one()) {
+  if (sh->error && warp < 2 && sm100::elect_one()) {
     const unsigned long long t0 = sm100::now_ns();
     while (sm100::now_ns() - t0 < 200000000ull) { __nanosleep(1000); }   // copies in flight land within microseconds
   }
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 2) {
     sm100::tc_fence_after();
-    sm100::tmem_dealloc(sh->tmem_base, TMEM_COLS);
+    sm100::tmem_dealloc(sh0->tmem_base, TEAMS * TMEM_COLS);
   }
 }
 
 }  // namespace attn
 
 static unsigned long long* g_attn_trace = nullptr;
-static int g_attn_v_stages = 1;
-static int attn_smem_bytes() { return attn::SMEM_TILES + (g_attn_v_stages - 1) * attn::TILE_BYTES + attn::SMEM_SHARED; }
 
 static int* attn_status_word(int** host_out = nullptr) {
   static int* dev_ptr = nullptr;
@@ -412,9 +454,7 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   if ((st = make_tmap_bf16(&mq, q, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mk, k, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mv, v, rows, cols, (uint64_t)ld_qkv, 128))) return st;
-  cudaError_t ae = cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes());
-  if (ae == cudaSuccess)          // two CTAs per SM need the largest shared-memory carve-out
-    ae = cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  cudaError_t ae = cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
   attn::Params p;
   p.B = B; p.T = T; p.H = H; p.q_blocks = T / attn::BQ;
@@ -422,28 +462,27 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.out = (__nv_bfloat16*)out; p.ld_out = (int)ld_out; p.lse = lse;
   p.status = attn_status_word();
   p.trace = g_attn_trace;
-  const int grid = B * H * p.q_blocks;
-  p.v_stages = g_attn_v_stages;
-  attn::attention_fwd_kernel<<<grid, attn::THREADS, attn_smem_bytes(), (cudaStream_t)stream>>>(mq, mk, mv, p);
+  p.items = B * H * p.q_blocks;
+  // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
+  const int grid = std::min(p.items, gemm_sm_count());
+  attn::attention_fwd_kernel<<<grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream>>>(mq, mk, mv, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));
 }
 
-// Resident CTAs of the attention kernel per SM (2 when shared memory and registers allow the intended overlap).
+// Resident CTAs of the attention kernel per SM (1: a CTA holds two teams that overlap each other).
 int tmpi_attention_ctas_per_sm(void) {
   int n = 0;
-  cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes());
-  cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn::attention_fwd_kernel, attn::THREADS, attn_smem_bytes()) != cudaSuccess) return -1;
+  cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn::attention_fwd_kernel, attn::THREADS, attn::SMEM_BYTES) != cudaSuccess) return -1;
   return n;
 }
 
-// Tuning aid: with a device buffer of (T / 128) * 16 64-bit words, CTA 0 of every later launch (the last query block
-// of the first batch and head) records the time of each phase of each key block (ns): 0 waits for S, 1 has S, 2 row
-// maximum known, 3 P written, 4 P announced, 5 has O_j, 6 output updated; MMA thread: 8 S was read, 9 next S issued,
-// 10 has P, 11 has V, 12 P V issued.  nullptr switches it off.
-// Tuning aid: one or two V buffers per CTA (see Params::v_stages).
-void tmpi_attention_set_v_stages(int n) { g_attn_v_stages = n == 2 ? 2 : 1; }
+// Tuning aid: with a device buffer of (T / 128) * 16 64-bit words, team 0 of CTA 0 in every later launch (the last query block
+// of the first batch and head) records the time of each phase of each key block of its first item (ns): 0 waits for S,
+// 1 has S, 2 row maximum known, 3 P written, 4 P announced, 5 knows that P V is done, 6 the same (last block: output
+// written); MMA thread: 8 waits to issue the next S, 9 next S issued, 10 has P, 11 has V, 12 P V issued.  nullptr
+// switches it off.
 
 void tmpi_attention_set_trace(void* device_buffer) { g_attn_trace = (unsigned long long*)device_buffer; }
 

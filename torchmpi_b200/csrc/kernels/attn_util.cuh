@@ -1,6 +1,7 @@
-// Small arithmetic helpers shared by the attention kernels: exp2 on the special-function unit and on the FMA pipe,
+// Small arithmetic helpers shared by the attention kernels and the GELU: reciprocal, exp2 on the special-function unit and on the FMA pipe,
 // three-input maximum, and the packed two-lane fp32 operations of sm_100.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -9,6 +10,12 @@ namespace attn_util {
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -23,6 +30,12 @@ __device__ __forceinline__ float ex2_fma(float a) {
   q = fmaf(q, f, 0.6932610273361206f);
   q = fmaf(q, f, 0.9999280571937561f);
   return __uint_as_float(__float_as_uint(q) + (__float_as_uint(t) << 23));
+}
+
+// two fp32 values as packed bf16
+__device__ __forceinline__ uint32_t pack_bf16(uint32_t lo, uint32_t hi) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
+  return *reinterpret_cast<uint32_t*>(&h);
 }
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -48,6 +61,15 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
   unsigned long long r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  const unsigned long long m1 = pack2(0xbf800000u, 0xbf800000u);
+  return fma2(b, m1, a);                                   // a - b, rounded once
 }
 
 }  // namespace attn_util
