@@ -1,27 +1,41 @@
 // Causal self-attention backward (head size 64) as one tcgen05 kernel: dQ, dK, dV from Q, K, V, dO, the forward's
 // log-sum-exp and delta = rowsum(dO * O).
 //
-// One CTA owns one block of 128 keys of one (batch, head) and walks the query blocks from its diagonal to the end
-// of the sequence.  Per pair (query block i, key block j), five MMAs with fp32 accumulators in tensor memory:
+// A work item is one block of 128 keys of one (batch, head); a persistent CTA per SM walks the query blocks of an item
+// from its diagonal to the end of the sequence.  Scores are computed transposed, [key][query], so that P and dS are born
+// in the layout in which the tensor core takes its first operand out of tensor memory.  Per pair (query block i, key
+// block j), five MMAs with fp32 accumulators in tensor memory:
 //
-//   S  = Q_i K_j^T            dP = dO_i V_j^T                       (128 x 128 each; read by the softmax warps)
-//   dV += P^T dO_i            dK += dS^T Q_i                        (128 keys x 64, accumulated over i, read once)
-//   dQ_ij = dS K_j                                                  (128 queries x 64, added to a fp32 dQ buffer)
+//   S^T  = K_j Q_i^T          dP^T = V_j dO_i^T                     (128 keys x 128 queries each)
+//   dV  += P^T dO_i           dK  += dS^T Q_i                       (P^T, dS^T read from tensor memory; 128 x 64)
+//   dQ_ij = dS K_j                                                  (dS^T read MN-major out of shared memory; 128 x 64)
 //
-// with P = exp(scale S - lse) and dS = scale P (dP - delta) computed by sixteen warps (four threads per query row, 32
-// keys each) and written as bf16 into two shared-memory tiles laid out [query][key] with the 128-byte swizzle: the
-// tensor core reads them K-major for dS K_j and MN-major (transposed) for P^T dO_i and dS^T Q_i, so nothing is
-// transposed by hand.  Q_i and dO_i arrive by TMA through a two-stage ring, K_j and V_j once.  S and dP of the next
-// pair are issued as soon as the softmax warps have read the current ones, and P and dS are double-buffered, so the
-// softmax of pair n + 1 runs while the tensor core works on the three products of pair n.
+// with P = exp(scale S - lse) and dS = P (dP - delta); the softmax scale is applied to dK and dQ at the end.
 //
-// dQ receives contributions from every key block: each CTA adds its 128 x 64 tile to a fp32 buffer with vector
-// reductions (red.global.add.v4.f32), so the low bits of dQ depend on the order in which CTAs arrive; dK and dV are
-// bit-reproducible.  Every wait is bounded; a CTA that gives up records where and frees its tensor memory.
+//   warp 0      TMA producer: K_j and V_j through two buffers (the next item's arrive under the current one), Q_i, dO_i
+//               and the block's 128 lse / delta values through a three-stage ring
+//   warp 1      MMA issuer; order per pair n: S(n+1), dV(n), dK(n), dQ(n), dP(n+1), so that the exponentials of pair
+//               n + 1 run under the products of pair n
+//   warps 4-7   drain dQ_ij (every pair) and dK, dV (every item): one thread per row; dQ goes through a swizzled staging
+//               tile and is added to the fp32 buffer by the TMA unit (cp.reduce, whole 128-byte rows)
+//   warps 8-23  four threads per key row: P^T as bf16 into its own tensor-memory columns, then dS^T over the dP^T columns
+//               that the thread itself has read, and into shared memory for dQ
+//
+// What bounds it: not the MMAs (1280 cycles per pair, about 1700 with their shared-memory operands) nor the 16384
+// exponentials (1024 cycles), but the chain dP -> dS -> dK, dQ -> dP of a pair, about 4000 cycles: tensor-memory and
+// shared-memory latencies of warps that work on the same pair.  So nothing but two packed operations per pair of scores, the
+// rounding and the stores lies on it, and sixteen softmax warps share it (eight: 105 us in place of 97).  The version before
+// kept P and dS in shared memory (2400 cycles of operand traffic per pair), was not persistent, and added dQ with
+// red.global.v4 from the accumulator layout (32 different lines per instruction).  Measured on a B200, 8 x 16 heads x
+// 1024 x 64, this kernel: 122 -> 97 us.
+//
+// The order in which CTAs add to dQ is not fixed, so its low bits vary; dK and dV are bit-reproducible.  Every wait is
+// bounded; a CTA that gives up records where and frees its tensor memory.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <algorithm>
 #include <mutex>
 #include "sm100_ptx.cuh"
 #include "attn_util.cuh"
@@ -32,32 +46,40 @@ using namespace tmpi;
 
 namespace tmpi {
 int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+int make_tmap_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+int gemm_sm_count();
 }
 
 namespace attnb {
 using namespace attn_util;
 
-constexpr int BLK = 128, D = 64, SOFTMAX_WARPS = 16, THREADS = 64 + SOFTMAX_WARPS * 32, UMMA_K = 16;
+constexpr int BLK = 128, D = 64, UMMA_K = 16, DRAIN_WARPS = 4, SOFTMAX_WARPS = 16;
+constexpr int THREADS = 32 * (4 + DRAIN_WARPS + SOFTMAX_WARPS);
+constexpr int QD_STAGES = 3;
 constexpr int TILE = BLK * D * 2;                             // a 128 x 64 bf16 tile: 16 KB
-constexpr int K_OFF = 0, V_OFF = TILE, Q_OFF = 2 * TILE, DO_OFF = 4 * TILE, P_OFF = 6 * TILE, DS_OFF = 10 * TILE;
-constexpr int SMEM_TILES = 14 * TILE;                         // K, V, Q x 2, dO x 2, P x 2 (32 KB each), dS x 2: 224 KB
-constexpr int SMEM_SHARED = 256;
-constexpr int TMEM_COLS = 512;                                // S 0, dP 128, dV 256, dK 320, dQ 384
+constexpr int K_OFF = 0, V_OFF = 2 * TILE, Q_OFF = 4 * TILE, DO_OFF = Q_OFF + QD_STAGES * TILE,
+              DS_OFF = DO_OFF + QD_STAGES * TILE, DQ_OFF = DS_OFF + 2 * TILE;
+constexpr int SMEM_TILES = DQ_OFF + TILE;                     // 208 KB; the dQ staging is 4 KB (32 rows x 32 columns) per warp
+constexpr int STAT_BYTES = BLK * 4;                           // lse or delta of a query block
+constexpr int STAT_OFF = SMEM_TILES, SHARED_OFF = STAT_OFF + QD_STAGES * 2 * STAT_BYTES;
+constexpr int SMEM_SHARED = 512, SMEM_BYTES = SHARED_OFF + SMEM_SHARED;
+static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
+constexpr int TMEM_COLS = 512, T_S = 0, T_DP = 128, T_DV = 256, T_DK = 320, T_DQ = 384, T_P = 448;
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
-  uint64_t kv_full, qd_full[2], qd_empty[2], sdp_full, sdp_empty, pds_full[2], dq_full, dq_empty, all_done;
+  uint64_t kv_full[2], kv_empty[2], qd_full[QD_STAGES], qd_empty[QD_STAGES], s_full, s_empty, p_full, dv_done, dp_full, ds_full,
+      dk_done, dq_full, dq_empty, acc_full, acc_empty;
   uint32_t tmem_base;
   int error;
 };
 static_assert(sizeof(Shared) <= SMEM_SHARED, "barrier block");
 
 struct Params {
-  int B, T, H, blocks;
+  int B, T, H, blocks, items;
   float scale, scale_log2;
   const float* lse;            // [B, H, T], natural log
   const float* delta;          // [B, H, T]
-  float* dq_acc;               // [B * T, H * 64] fp32, cleared by the delta kernel
   __nv_bfloat16* dk;           // [B * T, ld_dkv], head h at columns h * 64
   __nv_bfloat16* dv;
   int ld_dkv;
@@ -70,253 +92,355 @@ __device__ __forceinline__ void fail(Shared* sh, const Params& p, int where) {
   if (p.status) atomicCAS(p.status, 0, 3100 + where);
 }
 
-// Phase time stamps of one CTA for tuning: slot = (pair * 16 + event), written by one thread per role.
-__device__ __forceinline__ void stamp(const Params& p, int n, int ev) {
-  if (p.trace && blockIdx.x == 0) p.trace[n * 16 + ev] = sm100::now_ns();
+// Phase time stamps of one CTA's first item for tuning: slot = (pair * 16 + event), written by one thread per role.
+__device__ __forceinline__ void stamp(const Params& p, int round, int n, int ev) {
+  if (p.trace && blockIdx.x == 0 && round == 0) p.trace[n * 16 + ev] = sm100::now_ns();
 }
+
+// The item of this CTA in a round: key blocks near the start of the sequence meet the most query blocks and come first,
+// every other round in reverse, so that a CTA that got a long item gets a short one next.
+__device__ __forceinline__ bool item(const Params& p, int round, int* bh, int* jblk) {
+  const int g = (int)gridDim.x, i = (int)blockIdx.x;
+  const long long t = (long long)round * g + ((round & 1) ? g - 1 - i : i);
+  if (t >= p.items) return false;
+  const int n = p.B * p.H;
+  *jblk = (int)(t / n);
+  *bh = (int)(t % n);
+  return true;
+}
+
+// Position in a ring of N stages after every step over all items: stage index and the parity of its current use.
+template <int N>
+struct Ring {
+  int stage = 0, use = 0;
+  __device__ __forceinline__ void next() { if (++stage == N) { stage = 0; ++use; } }
+};
 
 #define ATTNB_WAIT(bar, parity, where) \
   do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
 
-__device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
-                         const CUtensorMap* mv, const CUtensorMap* mdo, int b, int h, int jblk) {
-  const int row0 = b * p.T;
-  sm100::mbar_expect_tx(&sh->kv_full, 2 * TILE);
-  sm100::tma_load_2d(tiles + K_OFF, mk, h * D, row0 + jblk * BLK, &sh->kv_full);
-  sm100::tma_load_2d(tiles + V_OFF, mv, h * D, row0 + jblk * BLK, &sh->kv_full);
-  int n = 0;
-  for (int i = jblk; i < p.blocks; ++i, ++n) {
-    const int st = n & 1;
-    if (n >= 2) ATTNB_WAIT(&sh->qd_empty[st], ((n >> 1) - 1) & 1, 1);
-    sm100::mbar_expect_tx(&sh->qd_full[st], 2 * TILE);
-    sm100::tma_load_2d(tiles + Q_OFF + st * TILE, mq, h * D, row0 + i * BLK, &sh->qd_full[st]);
-    sm100::tma_load_2d(tiles + DO_OFF + st * TILE, mdo, h * D, row0 + i * BLK, &sh->qd_full[st]);
+__device__ void producer(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
+                         const CUtensorMap* mv, const CUtensorMap* mdo) {
+  Ring<QD_STAGES> q;
+  int bh, jblk;
+  for (int r = 0; item(p, r, &bh, &jblk); ++r) {
+    const int b = bh / p.H, h = bh - b * p.H, row0 = b * p.T, kv = r & 1;
+    if (r >= 2) ATTNB_WAIT(&sh->kv_empty[kv], ((r >> 1) - 1) & 1, 1);
+    sm100::mbar_expect_tx(&sh->kv_full[kv], 2 * TILE);
+    sm100::tma_load_2d(smem + K_OFF + kv * TILE, mk, h * D, row0 + jblk * BLK, &sh->kv_full[kv]);
+    sm100::tma_load_2d(smem + V_OFF + kv * TILE, mv, h * D, row0 + jblk * BLK, &sh->kv_full[kv]);
+    for (int i = jblk; i < p.blocks; ++i, q.next()) {
+      const int st = q.stage;
+      if (q.use >= 1) ATTNB_WAIT(&sh->qd_empty[st], (q.use - 1) & 1, 2);
+      unsigned char* stat = smem + STAT_OFF + st * 2 * STAT_BYTES;
+      const size_t at = (size_t)bh * p.T + (size_t)i * BLK;
+      sm100::mbar_expect_tx(&sh->qd_full[st], 2 * TILE + 2 * STAT_BYTES);
+      sm100::tma_load_2d(smem + Q_OFF + st * TILE, mq, h * D, row0 + i * BLK, &sh->qd_full[st]);
+      sm100::bulk_load(stat, p.lse + at, STAT_BYTES, &sh->qd_full[st]);
+      sm100::tma_load_2d(smem + DO_OFF + st * TILE, mdo, h * D, row0 + i * BLK, &sh->qd_full[st]);
+      sm100::bulk_load(stat + STAT_BYTES, p.delta + at, STAT_BYTES, &sh->qd_full[st]);
+    }
   }
 }
 
-__device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p, int jblk) {
-  const uint32_t t_s = sh->tmem_base, t_dp = t_s + 128, t_dv = t_s + 256, t_dk = t_s + 320, t_dq = t_s + 384;
-  const uint32_t k_addr = sm100::smem_u32(tiles + K_OFF), v_addr = sm100::smem_u32(tiles + V_OFF);
+__device__ void mma_issuer(Shared* sh, unsigned char* smem, const Params& p) {
+  const uint32_t tm = sh->tmem_base;
   constexpr uint32_t idesc_s = sm100::make_idesc_f16(BLK, BLK, true);                 // both operands K-major
-  constexpr uint32_t idesc_t = sm100::make_idesc_f16(BLK, D, true, true, true);       // A and B MN-major (transposed reads)
-  constexpr uint32_t idesc_q = sm100::make_idesc_f16(BLK, D, true, true, false);      // A K-major, B MN-major
-  const int pairs = p.blocks - jblk;
-  // Descriptors: one per operand tile, built once; a slice further into the tile only adds to the address field
-  // (bytes / 16 in the low 14 bits; shared memory is far smaller than the field, so nothing carries out of it).
+  constexpr uint32_t idesc_a = sm100::make_idesc_f16(BLK, D, true, true, false);      // A in tensor memory, B MN-major
+  constexpr uint32_t idesc_q = sm100::make_idesc_f16(BLK, D, true, true, true);       // A and B MN-major
+  // Descriptors: one per operand, built once; a slice or a stage further on only adds to the address field (bytes / 16 in
+  // the low 14 bits; shared memory is far smaller than the field, so nothing carries out of it).
   auto at = [](uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); };
-  const uint64_t k_kmaj = sm100::make_desc_sw128(k_addr), v_kmaj = sm100::make_desc_sw128(v_addr);
-  const uint64_t k_mn = sm100::make_desc_sw128_mn(k_addr, TILE, 1024);
-  uint64_t q_kmaj[2], do_kmaj[2], q_mn[2], do_mn[2], p_mn[2], ds_mn[2], ds_kmaj[2];
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const uint32_t q_addr = sm100::smem_u32(tiles + Q_OFF + s * TILE), do_addr = sm100::smem_u32(tiles + DO_OFF + s * TILE);
-    const uint32_t p_addr = sm100::smem_u32(tiles + P_OFF + s * 2 * TILE), ds_addr = sm100::smem_u32(tiles + DS_OFF + s * 2 * TILE);
-    q_kmaj[s] = sm100::make_desc_sw128(q_addr);
-    do_kmaj[s] = sm100::make_desc_sw128(do_addr);
-    q_mn[s] = sm100::make_desc_sw128_mn(q_addr, TILE, 1024);
-    do_mn[s] = sm100::make_desc_sw128_mn(do_addr, TILE, 1024);
-    p_mn[s] = sm100::make_desc_sw128_mn(p_addr, TILE, 1024);
-    ds_mn[s] = sm100::make_desc_sw128_mn(ds_addr, TILE, 1024);
-    ds_kmaj[s] = sm100::make_desc_sw128(ds_addr);
-  }
-  auto issue_sdp = [&](int n) {
-    const uint64_t dq = (n & 1) ? q_kmaj[1] : q_kmaj[0], dd = (n & 1) ? do_kmaj[1] : do_kmaj[0];
+  const uint64_t k_k = sm100::make_desc_sw128(sm100::smem_u32(smem + K_OFF)), v_k = sm100::make_desc_sw128(sm100::smem_u32(smem + V_OFF));
+  const uint64_t q_k = sm100::make_desc_sw128(sm100::smem_u32(smem + Q_OFF)), do_k = sm100::make_desc_sw128(sm100::smem_u32(smem + DO_OFF));
+  const uint64_t k_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + K_OFF), TILE, 1024);
+  const uint64_t q_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + Q_OFF), TILE, 1024);
+  const uint64_t do_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + DO_OFF), TILE, 1024);
+  const uint64_t ds_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + DS_OFF), TILE, 1024);
+  auto ready = [&](uint64_t* bar, int parity, int where) -> bool {
+    if (sm100::mbar_wait(bar, parity & 1, kWaitBudgetNs) && !sh->error) return true;
+    fail(sh, p, where);
+    return false;
+  };
+  auto product_128 = [&](uint32_t d, uint64_t a, uint64_t b) {            // 128 x 128 over the 64 head columns
 #pragma unroll
     for (int k = 0; k < D / UMMA_K; ++k)
-      sm100::umma_f16(t_s, at(dq, k * UMMA_K * 2), at(k_kmaj, k * UMMA_K * 2), idesc_s, k > 0 ? 1u : 0u);
-#pragma unroll
-    for (int k = 0; k < D / UMMA_K; ++k)
-      sm100::umma_f16(t_dp, at(dd, k * UMMA_K * 2), at(v_kmaj, k * UMMA_K * 2), idesc_s, k > 0 ? 1u : 0u);
-    sm100::umma_commit(&sh->sdp_full);
+      sm100::umma_f16(tm + d, at(a, k * UMMA_K * 2), at(b, k * UMMA_K * 2), idesc_s, k > 0 ? 1u : 0u);
   };
-  auto issue_products = [&](int n) {
-    const int s = n & 1;
-    const uint64_t a_p = s ? p_mn[1] : p_mn[0], a_ds = s ? ds_mn[1] : ds_mn[0], a_dsk = s ? ds_kmaj[1] : ds_kmaj[0];
-    const uint64_t b_do = s ? do_mn[1] : do_mn[0], b_q = s ? q_mn[1] : q_mn[0];
-    const uint32_t acc = n > 0 ? 1u : 0u;
-    // K dimension = the 128 queries of the block: 16 rows of 128 bytes per step in every [query][...] tile
-#pragma unroll
-    for (int k = 0; k < BLK / UMMA_K; ++k)      // dV += P^T dO
-      sm100::umma_f16(t_dv, at(a_p, k * UMMA_K * 128), at(b_do, k * UMMA_K * 128), idesc_t, k > 0 ? 1u : acc);
-#pragma unroll
-    for (int k = 0; k < BLK / UMMA_K; ++k)      // dK += dS^T Q
-      sm100::umma_f16(t_dk, at(a_ds, k * UMMA_K * 128), at(b_q, k * UMMA_K * 128), idesc_t, k > 0 ? 1u : acc);
-    // K dimension = the 128 keys: dS read K-major (two chunks of 64 keys), K_j read MN-major
-#pragma unroll
-    for (int k = 0; k < BLK / UMMA_K; ++k)      // dQ_ij = dS K_j
-      sm100::umma_f16(t_dq, at(a_dsk, (k >> 2) * TILE + (k & 3) * UMMA_K * 2), at(k_mn, k * UMMA_K * 128), idesc_q, k > 0 ? 1u : 0u);
-    sm100::umma_commit(&sh->dq_full);                // also: these P / dS buffers and this stage of Q / dO are free again
-    sm100::umma_commit(&sh->qd_empty[s]);
-  };
-  ATTNB_WAIT(&sh->kv_full, 0, 2);
-  ATTNB_WAIT(&sh->qd_full[0], 0, 3);
+  int bh, jblk;
+  if (!item(p, 0, &bh, &jblk)) return;
+  if (!ready(&sh->kv_full[0], 0, 3) || !ready(&sh->qd_full[0], 0, 3)) return;
   sm100::tc_fence_after();
-  issue_sdp(0);
-  int next_sdp = 1;                                  // the next pair whose S and dP are to be issued
-  for (int n = 0; n < pairs; ++n) {
-    // Two things may become possible, in either order: S and dP of pair n + 1 (its Q and dO have landed and the
-    // softmax warps have read pair n's), and the three products of pair n (its P and dS are written and the previous
-    // dQ tile has been collected).  Whichever is ready goes first, so a late TMA load does not hold up the products.
-    const unsigned long long t0 = sm100::now_ns();
-    bool products_done = false;
-    unsigned spins = 0;
-    while (!products_done || (next_sdp == n + 1 && n + 1 < pairs)) {
-      if (next_sdp == n + 1 && n + 1 < pairs && sm100::mbar_try_wait(&sh->sdp_empty, n & 1) &&
-          sm100::mbar_try_wait(&sh->qd_full[(n + 1) & 1], ((n + 1) >> 1) & 1)) {
-        if (!products_done) stamp(p, n, 8);
+  product_128(T_S, k_k, q_k);
+  sm100::umma_commit(&sh->s_full);
+  product_128(T_DP, v_k, do_k);
+  sm100::umma_commit(&sh->dp_full);
+  Ring<QD_STAGES> q;                                       // the stage of the pair in work
+  int g = 0;                                               // pairs done, over all items
+  bool more = true;
+  for (int r = 0; more; ++r) {
+    const int pairs = p.blocks - jblk, kv = r & 1;
+    more = item(p, r + 1, &bh, &jblk);
+    for (int n = 0; n < pairs; ++n, ++g) {
+      const bool last = n + 1 == pairs, next = !last || more;
+      Ring<QD_STAGES> qn = q;
+      qn.next();
+      const int kvn = last ? (kv ^ 1) : kv;                // buffer of the next pair's K and V
+      if (next) {                                          // S of the next pair, once this pair's has been read
+        if (last && !ready(&sh->kv_full[kvn], (r + 1) >> 1, 3)) return;
+        if (!ready(&sh->qd_full[qn.stage], qn.use, 4) || !ready(&sh->s_empty, g, 5)) return;
+        stamp(p, r, n, 8);
         sm100::tc_fence_after();
-        issue_sdp(n + 1);
-        ++next_sdp;
-        stamp(p, n, 9);
-      } else if (!products_done && sm100::mbar_try_wait(&sh->pds_full[n & 1], (n >> 1) & 1) &&
-                 (n == 0 || sm100::mbar_try_wait(&sh->dq_empty, (n - 1) & 1))) {
-        stamp(p, n, 10);
-        sm100::tc_fence_after();
-        issue_products(n);
-        products_done = true;
-        stamp(p, n, 12);
-      } else if ((++spins & 255u) == 0 && (sm100::now_ns() - t0 > kWaitBudgetNs || sh->error)) {
-        fail(sh, p, 6);
-        return;
+        product_128(T_S, at(k_k, kvn * TILE), at(q_k, qn.stage * TILE));
+        sm100::umma_commit(&sh->s_full);
+        stamp(p, r, n, 9);
       }
+      if (n == 0 && r > 0 && !ready(&sh->acc_empty, r - 1, 6)) return;    // the previous item's dK and dV have been read
+      if (!ready(&sh->p_full, g, 7)) return;
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < BLK / UMMA_K; ++k)               // dV += P^T dO: 16 queries = eight columns of packed P, 16 rows of dO
+        sm100::umma_f16_tmem_a(tm + T_DV, tm + T_P + k * 8, at(do_mn, q.stage * TILE + k * UMMA_K * 128), idesc_a, (n | k) ? 1u : 0u);
+      sm100::umma_commit(&sh->dv_done);
+      if (!ready(&sh->ds_full, g, 8)) return;
+      stamp(p, r, n, 10);
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < BLK / UMMA_K; ++k)               // dK += dS^T Q: dS^T sits in the first half of each 32 columns of dP^T
+        sm100::umma_f16_tmem_a(tm + T_DK, tm + T_DP + (k >> 1) * 32 + (k & 1) * 8, at(q_mn, q.stage * TILE + k * UMMA_K * 128), idesc_a,
+                               (n | k) ? 1u : 0u);
+      sm100::umma_commit(&sh->dk_done);
+      sm100::umma_commit(&sh->qd_empty[q.stage]);          // both products that read this stage are done
+      if (last) sm100::umma_commit(&sh->acc_full);
+      if (g > 0 && !ready(&sh->dq_empty, g - 1, 9)) return;
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < BLK / UMMA_K; ++k)               // dQ_ij = dS K_j: 16 keys = 16 rows of dS^T and of K
+        sm100::umma_f16(tm + T_DQ, at(ds_mn, k * UMMA_K * 128), at(k_mn, kv * TILE + k * UMMA_K * 128), idesc_q, k > 0 ? 1u : 0u);
+      sm100::umma_commit(&sh->dq_full);                    // also: dS in shared memory is free again
+      if (last) sm100::umma_commit(&sh->kv_empty[kv]);
+      stamp(p, r, n, 12);
+      if (next) {                                          // dP of the next pair, once dK has read dS out of these columns
+        if (!ready(&sh->dk_done, g, 10)) return;
+        sm100::tc_fence_after();
+        product_128(T_DP, at(v_k, kvn * TILE), at(do_k, qn.stage * TILE));
+        sm100::umma_commit(&sh->dp_full);
+      }
+      q = qn;
     }
   }
-  sm100::umma_commit(&sh->all_done);
 }
 
-// Four threads per query row (warps with the same warp & 3 share 32 tensor-memory lanes); `part` picks 32 of the 128
-// keys of the pair and 16 of the 64 columns of dQ (and, at the end, of dK / dV, where the rows are keys).
-__device__ void softmax_rows(Shared* sh, unsigned char* tiles, const Params& p, int b, int h, int jblk, int quarter, int part,
-                             int lane) {
-  const int row = quarter * 32 + lane;
-  const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-  const uint32_t t_s = sh->tmem_base + lane_base + part * 32, t_dp = t_s + 128;
-  const uint32_t t_dv = sh->tmem_base + lane_base + 256 + part * 16, t_dk = t_dv + 64, t_dq = t_dv + 128;
-  const float c2 = p.scale_log2, scale = p.scale;
-  const int key0 = part * 32;
-  const int tile_off = (part >> 1) * TILE + row * 128;    // which 64-key chunk of the [query][key] tiles
-  const int unit0 = (part & 1) * 4;                       // first 16-byte unit of this thread's keys in the row
-  const bool masked_diag = key0 > quarter * 32 + 31;      // on the diagonal block: every key of the chunk is after the query
-  uint32_t rs[32], rp[32];
-  const int pairs = p.blocks - jblk;
+// Four threads per key row (`part` picks 32 of the 128 queries of a pair).
+__device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, int quarter, int part, int lane) {
+  const int row = quarter * 32 + lane;                     // key inside the block; tensor-memory lane
+  const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
+  const uint32_t t_s = tm + T_S + part * 32, t_dp = tm + T_DP + part * 32, t_p = tm + T_P + part * 16;
+  unsigned char* ds_row = smem + DS_OFF + (part >> 1) * TILE + row * 128;
+  const int unit0 = (part & 1) * 4;                        // first 16-byte unit of this thread's queries in the row
+  const unsigned long long c2x2 = pack2(__float_as_uint(p.scale_log2), __float_as_uint(p.scale_log2));
+  const unsigned long long nl2e = pack2(__float_as_uint(-1.4426950408889634f), __float_as_uint(-1.4426950408889634f));
   const bool tracer = row == 0 && part == 0;
-  // P and dS of pair n (query block jblk + n) into the buffers n & 1
-  auto softmax_pair = [&](int n) -> bool {
-    const int i = jblk + n;
-    const bool diag = n == 0;
-    unsigned char* p_row = tiles + P_OFF + (n & 1) * 2 * TILE + tile_off;
-    unsigned char* ds_row = tiles + DS_OFF + (n & 1) * 2 * TILE + tile_off;
-    const size_t stat = ((size_t)b * p.H + h) * p.T + (size_t)i * BLK + row;
-    const float nl2 = -p.lse[stat] * 1.4426950408889634f, delta = p.delta[stat];
-    if (tracer) stamp(p, n, 0);
-    if (!sm100::mbar_wait(&sh->sdp_full, n & 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 8); return false; }
-    if (tracer) stamp(p, n, 1);
-    sm100::tc_fence_after();
-    const bool masked = diag && masked_diag;               // warp-uniform: nothing to load or exponentiate
-    if (!masked) {
-      sm100::tmem_ld_32x32(t_s, rs);
-      sm100::tmem_ld_32x32(t_dp, rp);
+  Ring<QD_STAGES> q;
+  int g = 0, bh, jblk;
+  for (int r = 0; item(p, r, &bh, &jblk); ++r) {
+    const int pairs = p.blocks - jblk;
+    for (int n = 0; n < pairs; ++n, ++g, q.next()) {
+      const float4* lse = reinterpret_cast<const float4*>(smem + STAT_OFF + q.stage * 2 * STAT_BYTES) + part * 8;
+      const float4* delta = lse + STAT_BYTES / 16;
+      const bool diag = n == 0, masked = diag && part < quarter;               // masked: every query of the thread is before its key
+      if (tracer) stamp(p, r, n, 0);
+      ATTNB_WAIT(&sh->qd_full[q.stage], q.use & 1, 11);    // lse and delta (the MMA waits for the tiles itself)
+      ATTNB_WAIT(&sh->s_full, g & 1, 12);
+      if (tracer) stamp(p, r, n, 1);
+      sm100::tc_fence_after();
+      uint32_t s[32], w[16];
+      sm100::tmem_ld_32x32(t_s, s);
       sm100::tmem_ld_wait();
-    }
-    sm100::tc_fence_before();                              // S and dP are in registers: the next pair may overwrite them
-    sm100::mbar_arrive(&sh->sdp_empty);
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->s_empty);     // S is in registers: the next pair's may overwrite it
+      if (masked) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      uint32_t wp[4] = {0u, 0u, 0u, 0u}, wd[4] = {0u, 0u, 0u, 0u};
-      if (!masked) {
+        for (int e = 0; e < 32; ++e) s[e] = 0u;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int e = u * 8 + 2 * q;
-          float p0 = ex2(fmaf(__uint_as_float(rs[e]), c2, nl2)), p1 = ex2(fmaf(__uint_as_float(rs[e + 1]), c2, nl2));
-          if (diag) {
-            if (key0 + e > row) p0 = 0.f;
-            if (key0 + e + 1 > row) p1 = 0.f;
+        for (int e = 0; e < 16; ++e) w[e] = 0u;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {                      // P = exp2(S * scale * log2(e) - lse * log2(e)) over S in place
+          const float4 l = lse[u];                         // the same four values for all lanes
+          const unsigned long long l01 = mul2(pack2(__float_as_uint(l.x), __float_as_uint(l.y)), nl2e);
+          const unsigned long long l23 = mul2(pack2(__float_as_uint(l.z), __float_as_uint(l.w)), nl2e);
+          float a[4];
+          unpack2(fma2(pack2(s[4 * u], s[4 * u + 1]), c2x2, l01), a[0], a[1]);
+          unpack2(fma2(pack2(s[4 * u + 2], s[4 * u + 3]), c2x2, l23), a[2], a[3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float v = ex2(a[e]);
+            if (diag && part * 32 + 4 * u + e < row) v = 0.f;                  // the diagonal block: a query before the key
+            s[4 * u + e] = __float_as_uint(v);
           }
-          const float d0 = p0 * (__uint_as_float(rp[e]) - delta) * scale, d1 = p1 * (__uint_as_float(rp[e + 1]) - delta) * scale;
-          __nv_bfloat162 hp = __floats2bfloat162_rn(p0, p1), hd = __floats2bfloat162_rn(d0, d1);
-          wp[q] = *reinterpret_cast<uint32_t*>(&hp);
-          wd[q] = *reinterpret_cast<uint32_t*>(&hd);
+          w[2 * u] = pack_bf16(s[4 * u], s[4 * u + 1]);
+          w[2 * u + 1] = pack_bf16(s[4 * u + 2], s[4 * u + 3]);
         }
       }
-      const int off = ((unit0 + u) ^ (row & 7)) << 4;
-      *reinterpret_cast<uint4*>(p_row + off) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
-      *reinterpret_cast<uint4*>(ds_row + off) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+      if (g > 0) {                                         // dV of the previous pair has read P
+        ATTNB_WAIT(&sh->dv_done, (g - 1) & 1, 13);
+        sm100::tc_fence_after();
+      }
+      sm100::tmem_st_32x16(t_p, w);
+      sm100::tmem_st_wait();
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->p_full);
+      if (g > 0) ATTNB_WAIT(&sh->dq_full, (g - 1) & 1, 14);                    // dQ of the previous pair has read dS
+      ATTNB_WAIT(&sh->dp_full, g & 1, 15);
+      sm100::tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {                        // dS = P (dP - delta), 16 queries at a time
+        uint32_t d[16], v[8];
+        sm100::tmem_ld_32x16(t_dp + c * 16, d);
+        sm100::tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 dl = delta[c * 4 + u];
+          const uint32_t* pv = &s[c * 16 + 4 * u];
+          float a[4];
+          unpack2(mul2(pack2(pv[0], pv[1]), sub2(pack2(d[4 * u], d[4 * u + 1]), pack2(__float_as_uint(dl.x), __float_as_uint(dl.y)))),
+                  a[0], a[1]);
+          unpack2(mul2(pack2(pv[2], pv[3]), sub2(pack2(d[4 * u + 2], d[4 * u + 3]), pack2(__float_as_uint(dl.z), __float_as_uint(dl.w)))),
+                  a[2], a[3]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            __nv_bfloat162 hh = __floats2bfloat162_rn(a[2 * e], a[2 * e + 1]);
+            v[2 * u + e] = masked ? 0u : *reinterpret_cast<uint32_t*>(&hh);
+          }
+        }
+        sm100::tmem_st_32x8(t_dp + c * 8, v);              // columns that this thread has read already
+#pragma unroll
+        for (int u = 0; u < 2; ++u)                        // eight queries = one 16-byte unit of the swizzled row
+          *reinterpret_cast<uint4*>(ds_row + (((unit0 + c * 2 + u) ^ (row & 7)) << 4)) =
+              make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+      }
+      sm100::tmem_st_wait();
+      sm100::fence_proxy_async_smem();                     // the MMA reads dS through the async proxy
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        sm100::mbar_arrive(&sh->ds_full);
+        sm100::mbar_arrive(&sh->qd_empty[q.stage]);        // lse and delta have been read
+      }
+      if (tracer) stamp(p, r, n, 2);
     }
-    sm100::fence_proxy_async_smem();                      // the MMAs read P and dS through the async proxy
-    sm100::mbar_arrive(&sh->pds_full[n & 1]);
-    if (tracer) stamp(p, n, 2);
-    return true;
+  }
+}
+
+// Reads dQ of every pair and dK, dV of every item; one thread per row of the tile.
+__device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mdq, int quarter, int lane) {
+  const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
+  unsigned char* staging = smem + DQ_OFF + quarter * (TILE / DRAIN_WARPS);      // 32 rows of 128 bytes
+  const unsigned long long scale2 = pack2(__float_as_uint(p.scale), __float_as_uint(p.scale));
+  const bool tracer = quarter == 0 && lane == 0;
+  auto scaled = [&](uint32_t (&v)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      float a0, a1;
+      unpack2(mul2(pack2(v[i], v[i + 1]), scale2), a0, a1);
+      v[i] = __float_as_uint(a0); v[i + 1] = __float_as_uint(a1);
+    }
   };
-  if (!softmax_pair(0)) return;
-  uint32_t rq[16];
-  for (int n = 0; n < pairs; ++n) {
-    // the next pair's P and dS while the tensor core multiplies this pair's (its buffers were freed by the MMAs of
-    // pair n - 1, whose dQ this thread has already collected)
-    if (n + 1 < pairs && !softmax_pair(n + 1)) return;
-    // this pair's share of dQ: 16 columns of this thread's query row, added to the fp32 buffer
-    if (tracer) stamp(p, n, 3);
-    ATTNB_WAIT(&sh->dq_full, n & 1, 9);
-    if (tracer) stamp(p, n, 4);
+  int g = 0, bh, jblk;
+  for (int r = 0; item(p, r, &bh, &jblk); ++r) {
+    const int pairs = p.blocks - jblk, b = bh / p.H, h = bh - b * p.H;
+    uint32_t v[2][32];
+    for (int n = 0; n < pairs; ++n, ++g) {
+      if (tracer) stamp(p, r, n, 3);
+      ATTNB_WAIT(&sh->dq_full, g & 1, 16);
+      if (tracer) stamp(p, r, n, 4);
+      sm100::tc_fence_after();
+      sm100::tmem_ld_32x32(tm + T_DQ, v[0]);
+      sm100::tmem_ld_32x32(tm + T_DQ + 32, v[1]);
+      sm100::tmem_ld_wait();
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->dq_empty);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        scaled(v[c]);
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the staging tile has been read
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          *reinterpret_cast<uint4*>(staging + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+              make_uint4(v[c][4 * u], v[c][4 * u + 1], v[c][4 * u + 2], v[c][4 * u + 3]);
+        sm100::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          sm100::tma_reduce_add_2d(mdq, staging, h * D + c * 32, b * p.T + (jblk + n) * BLK + quarter * 32);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+      if (tracer) stamp(p, r, n, 5);
+    }
+    ATTNB_WAIT(&sh->acc_full, r & 1, 17);
     sm100::tc_fence_after();
-    sm100::tmem_ld_32x16(t_dq, rq);
+    const size_t at = ((size_t)b * p.T + (size_t)jblk * BLK + quarter * 32 + lane) * p.ld_dkv + h * D;
+    auto store = [&](__nv_bfloat16* o) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = (u & 3) * 8 + 2 * e;
+          __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(v[u >> 2][i]), __uint_as_float(v[u >> 2][i + 1]));
+          w[e] = *reinterpret_cast<uint32_t*>(&hh);
+        }
+        *reinterpret_cast<uint4*>(o + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    };
+    sm100::tmem_ld_32x32(tm + T_DV, v[0]);
+    sm100::tmem_ld_32x32(tm + T_DV + 32, v[1]);
+    sm100::tmem_ld_wait();
+    store(p.dv + at);
+    sm100::tmem_ld_32x32(tm + T_DK, v[0]);
+    sm100::tmem_ld_32x32(tm + T_DK + 32, v[1]);
     sm100::tmem_ld_wait();
     sm100::tc_fence_before();
-    sm100::mbar_arrive(&sh->dq_empty);
-    float* dq = p.dq_acc + ((size_t)b * p.T + (size_t)(jblk + n) * BLK + row) * (p.H * D) + h * D + part * 16;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dq + 4 * u), "f"(__uint_as_float(rq[4 * u])),
-                   "f"(__uint_as_float(rq[4 * u + 1])), "f"(__uint_as_float(rq[4 * u + 2])), "f"(__uint_as_float(rq[4 * u + 3]))
-                   : "memory");
-    if (tracer) stamp(p, n, 5);
+    __syncwarp();
+    if (lane == 0) sm100::mbar_arrive(&sh->acc_empty);
+    scaled(v[0]);
+    scaled(v[1]);
+    store(p.dk + at);
   }
-  // dV and dK of this key block: the accumulator rows are keys now
-  ATTNB_WAIT(&sh->all_done, 0, 10);
-  sm100::tc_fence_after();
-  const size_t grow = (size_t)b * p.T + (size_t)jblk * BLK + row;
-  auto store = [&](uint32_t taddr, __nv_bfloat16* base) {
-    sm100::tmem_ld_32x16(taddr, rq);
-    sm100::tmem_ld_wait();
-    __nv_bfloat16* o = base + grow * p.ld_dkv + h * D + part * 16;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      uint32_t w[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(rq[u * 8 + 2 * e]), __uint_as_float(rq[u * 8 + 2 * e + 1]));
-        w[e] = *reinterpret_cast<uint32_t*>(&hh);
-      }
-      *reinterpret_cast<uint4*>(o + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-  };
-  store(t_dv, p.dv);
-  store(t_dk, p.dk);
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");     // every addition is done before the kernel ends
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do, const Params p) {
+                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
+                     const __grid_constant__ CUtensorMap map_dq, const Params p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* tiles = smem_raw;
-  Shared* sh = (Shared*)(smem_raw + SMEM_TILES);
+  Shared* sh = (Shared*)(smem_raw + SHARED_OFF);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // key blocks near the start of the sequence meet the most query blocks: they start first
-  const int bh = blockIdx.x % (p.B * p.H);
-  const int jblk = blockIdx.x / (p.B * p.H);
-  const int b = bh / p.H, h = bh - b * p.H;
   if (warp == 0 && sm100::elect_one()) {
     sm100::tma_prefetch_desc(&map_q);
     sm100::tma_prefetch_desc(&map_k);
     sm100::tma_prefetch_desc(&map_v);
     sm100::tma_prefetch_desc(&map_do);
-    sm100::mbar_init(&sh->kv_full, 1);
-    for (int s = 0; s < 2; ++s) { sm100::mbar_init(&sh->qd_full[s], 1); sm100::mbar_init(&sh->qd_empty[s], 1); }
-    sm100::mbar_init(&sh->sdp_full, 1);
-    sm100::mbar_init(&sh->sdp_empty, SOFTMAX_WARPS * 32);
-    for (int s = 0; s < 2; ++s) sm100::mbar_init(&sh->pds_full[s], SOFTMAX_WARPS * 32);
+    sm100::tma_prefetch_desc(&map_dq);
+    for (int s = 0; s < 2; ++s) { sm100::mbar_init(&sh->kv_full[s], 1); sm100::mbar_init(&sh->kv_empty[s], 1); }
+    for (int s = 0; s < QD_STAGES; ++s) { sm100::mbar_init(&sh->qd_full[s], 1); sm100::mbar_init(&sh->qd_empty[s], 1 + SOFTMAX_WARPS); }
+    sm100::mbar_init(&sh->s_full, 1);
+    sm100::mbar_init(&sh->s_empty, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->p_full, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->dv_done, 1);
+    sm100::mbar_init(&sh->dp_full, 1);
+    sm100::mbar_init(&sh->ds_full, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->dk_done, 1);
     sm100::mbar_init(&sh->dq_full, 1);
-    sm100::mbar_init(&sh->dq_empty, SOFTMAX_WARPS * 32);
-    sm100::mbar_init(&sh->all_done, 1);
+    sm100::mbar_init(&sh->dq_empty, DRAIN_WARPS);
+    sm100::mbar_init(&sh->acc_full, 1);
+    sm100::mbar_init(&sh->acc_empty, DRAIN_WARPS);
     sh->error = 0;
     sm100::fence_barrier_init();
   }
@@ -328,15 +452,22 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __syncthreads();
   sm100::tc_fence_after();
 
-  const bool aligned = (sm100::smem_u32(tiles) & 1023u) == 0;     // the swizzled tiles need a 1024-byte aligned base
+  const bool aligned = (sm100::smem_u32(smem_raw) & 1023u) == 0;     // the swizzled tiles need a 1024-byte aligned base
   if (!aligned) {
-    if (threadIdx.x == 0) fail(sh, p, 11);
-  } else if (warp == 0) {
-    if (sm100::elect_one()) producer(sh, tiles, p, &map_q, &map_k, &map_v, &map_do, b, h, jblk);
-  } else if (warp == 1) {
-    if (sm100::elect_one()) mma_issuer(sh, tiles, p, jblk);
+    if (threadIdx.x == 0) fail(sh, p, 18);
+  } else if (warp < 4) {                                   // registers per four warps: 56 + 72 + 4 * 88 = the launch's 6 * 80
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0) {
+      if (sm100::elect_one()) producer(sh, smem_raw, p, &map_q, &map_k, &map_v, &map_do);
+    } else if (warp == 1) {
+      if (sm100::elect_one()) mma_issuer(sh, smem_raw, p);
+    }
+  } else if (warp < 4 + DRAIN_WARPS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    drain(sh, smem_raw, p, &map_dq, warp & 3, lane);
   } else {
-    softmax_rows(sh, tiles, p, b, h, jblk, warp & 3, (warp - 2) >> 2, lane);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    softmax_rows(sh, smem_raw, p, warp & 3, (warp - 4 - DRAIN_WARPS) >> 2, lane);
   }
   __syncwarp();
   sm100::tc_fence_before();
@@ -435,31 +566,33 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
                        void* dv, int64_t ld_dkv, int B, int T, int H, float scale, void* stream) {
   if (B < 1 || H < 1 || T < 128 || T % 128) return fail(TMPI_ERR_UNSUPPORTED, "attention backward: T=%d must be a positive multiple of 128", T);
   if (ld_dkv % 8 || ((uintptr_t)dk & 15) || ((uintptr_t)dv & 15) || ((uintptr_t)dq_acc & 15) || ld_o % 8 || ld_do % 8 ||
-      ((uintptr_t)o & 15) || ((uintptr_t)dout & 15))
+      ((uintptr_t)o & 15) || ((uintptr_t)dout & 15) || ((uintptr_t)lse & 15) || ((uintptr_t)delta & 15))
     return fail(TMPI_ERR_INVALID, "attention backward: operands must be 16-byte aligned with pitches that are multiples of 8");
   if ((int64_t)B * H * (T / 128) > 0x7fffffffLL) return fail(TMPI_ERR_INVALID, "attention backward: too many blocks");
   cudaStream_t s = (cudaStream_t)stream;
   const long long rows_heads = (long long)B * T * H;
   const int dgrid = (int)std::min<long long>((rows_heads * 8 + 255) / 256, 148 * 8);
   attnb::attention_delta_kernel<<<dgrid, 256, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, ld_o, ld_do, delta, dq_acc, B, T, H);
-  CUtensorMap mq, mk, mv, mdo;
+  CUtensorMap mq, mk, mv, mdo, mdq;
   int st;
   const uint64_t rows = (uint64_t)B * T, cols = (uint64_t)H * attnb::D;
   if ((st = make_tmap_bf16(&mq, q, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mk, k, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mv, v, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mdo, dout, rows, cols, (uint64_t)ld_do, 128))) return st;
-  const int smem = attnb::SMEM_TILES + attnb::SMEM_SHARED;
+  if ((st = make_tmap_f32(&mdq, dq_acc, rows, cols, cols, 32))) return st;
+  const int smem = attnb::SMEM_BYTES;
   cudaError_t ae = cudaFuncSetAttribute(attnb::attention_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention backward: shared memory attribute: %s", cudaGetErrorString(ae));
   attnb::Params p;
   p.B = B; p.T = T; p.H = H; p.blocks = T / attnb::BLK;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
-  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc;
+  p.lse = lse; p.delta = delta;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.ld_dkv = (int)ld_dkv;
   p.status = attnb_status_word();
   p.trace = g_attnb_trace;
-  attnb::attention_bwd_kernel<<<B * H * p.blocks, attnb::THREADS, smem, s>>>(mq, mk, mv, mdo, p);
+  p.items = B * H * p.blocks;
+  attnb::attention_bwd_kernel<<<std::min(p.items, gemm_sm_count()), attnb::THREADS, smem, s>>>(mq, mk, mv, mdo, mdq, p);
   if (dq) {
     if ((uintptr_t)dq & 15) return fail(TMPI_ERR_INVALID, "attention backward: dq must be 16-byte aligned");
     const long long groups = (long long)rows * (cols / 8);
@@ -472,8 +605,8 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
 
 // Tuning aid: with a device buffer of (T / 128) * 16 64-bit words, CTA 0 of every later launch (the first key block of
 // the first batch and head, which meets every query block) records the time of each phase of each pair (ns):
-// 0 waits for S and dP, 1 has them, 2 P and dS announced, 3 waits for dQ, 4 has it, 5 reductions issued; MMA thread:
-// 8 S and dP were read, 9 next S and dP issued, 10 has P and dS, 11 dQ tile free, 12 three products issued.
+// 0 waits for S, 1 has it, 2 dS announced, 3 waits for dQ, 4 has it, 5 additions issued; MMA thread: 8 S was read and the
+// next tiles are there, 9 next S issued, 10 has dS, 12 three products issued.
 void tmpi_attention_bwd_set_trace(void* device_buffer) { g_attnb_trace = (unsigned long long*)device_buffer; }
 
 // Non-zero after a CTA of the attention backward gave up on a bounded wait (3100 + the point where); clears it.
