@@ -32,14 +32,22 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const T* __restrict__ z, 
     for (int u = 0; u < U; ++u) {
       Pack<T, V> o;
 #pragma unroll
-      for (int k = 0; k < V; ++k) o.v[k] = from_acc<T>((typename AccOf<T>::type)gelu_value((float)to_acc<T>(a[u].v[k])));
+      for (int k = 0; k < V; k += 2) {
+        float y0, y1;
+        gelu_value2((float)to_acc<T>(a[u].v[k]), (float)to_acc<T>(a[u].v[k + 1]), &y0, &y1);
+        o.v[k] = from_acc<T>((typename AccOf<T>::type)y0); o.v[k + 1] = from_acc<T>((typename AccOf<T>::type)y1);
+      }
       st_pack<T, V>(y + (i + u * stride) * V, o);
     }
   }
   for (; i < npacks; i += stride) {
     Pack<T, V> a = ld_pack<T, V>(z + i * V), o;
 #pragma unroll
-    for (int k = 0; k < V; ++k) o.v[k] = from_acc<T>((typename AccOf<T>::type)gelu_value((float)to_acc<T>(a.v[k])));
+    for (int k = 0; k < V; k += 2) {
+      float y0, y1;
+      gelu_value2((float)to_acc<T>(a.v[k]), (float)to_acc<T>(a.v[k + 1]), &y0, &y1);
+      o.v[k] = from_acc<T>((typename AccOf<T>::type)y0); o.v[k + 1] = from_acc<T>((typename AccOf<T>::type)y1);
+    }
     st_pack<T, V>(y + i * V, o);
   }
 }
@@ -73,10 +81,14 @@ bias_grad_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __restric
     if (GELU) {
       Pack<T, V> o;
 #pragma unroll
-      for (int k = 0; k < V; ++k) {
-        const float v = (float)to_acc<T>(g.v[k]) * gelu_grad((float)to_acc<T>(a.v[k]));
-        o.v[k] = from_acc<T>((typename AccOf<T>::type)v);
-        acc[k] += (float)to_acc<T>(o.v[k]);             // the sum of what is stored
+      for (int k = 0; k < V; k += 2) {
+        float d[2];
+        gelu_grad2((float)to_acc<T>(a.v[k]), (float)to_acc<T>(a.v[k + 1]), &d[0], &d[1]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          o.v[k + e] = from_acc<T>((typename AccOf<T>::type)((float)to_acc<T>(g.v[k + e]) * d[e]));
+          acc[k + e] += (float)to_acc<T>(o.v[k + e]);   // the sum of what is stored
+        }
       }
       st_pack<T, V>(dz + at, o);
     } else {

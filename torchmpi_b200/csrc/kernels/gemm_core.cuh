@@ -48,7 +48,7 @@ struct Problem {
   int a_mn;                    // A is given as [K, M] with M contiguous (plain CTA-pair GEMM only)
   int mma_n;                   // single-CTA kernel, narrow outputs: rows of B staged per tile and N of the MMA
                                // (a multiple of 16 below BN); 0 = BN
-  int pair_n;                  // CTA-pair kernel: columns of a tile (BN, or 192 where that fills the SMs better); 0 = BN
+  int pair_n;                  // CTA-pair kernel: columns of a tile (BN, or 192 or 128 where that takes less time); 0 = BN
   int* status;                 // global error word (nullptr: none)
 };
 

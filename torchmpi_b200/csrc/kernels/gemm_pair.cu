@@ -34,7 +34,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   extern __shared__ unsigned char smem_raw[];
   unsigned char *tiles, *staging;
   Shared* sh;
-  carve(smem_raw, &tiles, &sh, &staging);
+  constexpr int NST = TWO ? STAGES - 1 : STAGES;
+  carve<NST>(smem_raw, &tiles, &sh, &staging);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = sm100::cluster_ctarank();
   setup(sh, warp, &map_a, &map_b, 4 * GROUPS);
@@ -50,9 +51,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     return true;
   };
   if (warp == 0) {
-    if (sm100::elect_one()) producer(sh, tiles, p, &map_a, &map_b, rank, order, [](int, const CUtensorMap**, int*) { return true; });
+    if (sm100::elect_one()) producer<NST>(sh, tiles, p, &map_a, &map_b, rank, order, [](int, const CUtensorMap**, int*) { return true; });
   } else if (warp == 1) {
-    if (rank == 0 && sm100::elect_one()) mma_issuer(sh, tiles, p, order);
+    if (rank == 0 && sm100::elect_one()) mma_issuer<NST>(sh, tiles, p, order);
   } else {
     epilogue_groups<TWO>(sh, staging, p, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
   }
@@ -80,13 +81,17 @@ static int max_clusters() {
   return n;
 }
 
-// Columns of a tile: 192 where that needs less time than 256.  A launch takes ceil(tiles / clusters) rounds of a tile
-// time that is proportional to its columns, so 48 tiles of 256 on 74 clusters (3072 x 1024: one round, 26 clusters
-// idle) lose to 72 tiles of 192 (one round of three quarters of the time).  Measured: 3072 x 1024, K = 8192: 55 -> 46 us;
-// 8192 x 3072, K = 1024: 51 -> 46.
+// Columns of a tile.  A launch takes ceil(tiles / clusters) rounds of a tile's time, which is its columns' MMAs or, for
+// narrow tiles, the operands' way out of L2: per 64-wide K block and CTA 32, 28 or 24 KB at about 64 bytes per cycle,
+// against 512, 384 or 256 cycles of MMAs.  So 48 tiles of 256 on 74 clusters (3072 x 1024: one round, 26 clusters idle)
+// lose to 72 tiles of 192, and 16 tiles of 256 (1024 x 1024) to 32 of 128, whose epilogue is half as long, too.
+// Measured: 3072 x 1024, K = 8192: 55 -> 46 us; 1024^3: 13.9 -> 10.2 (with the epilogue of
+// gemm_pair.cuh), 256 x 1000 x 2048: 14.4 -> 10.3.
 static int tile_columns(int tiles_m, int N, int clusters) {
-  auto cost = [&](int bn) { return (long long)((tiles_m * (long long)((N + bn - 1) / bn) + clusters - 1) / clusters) * bn; };
-  return 100 * cost(192) < 95 * cost(BN) ? 192 : BN;      // a narrower tile reads more of A per product: 5 % for that
+  auto cost = [&](int bn, int cycles) { return (long long)((tiles_m * (long long)((N + bn - 1) / bn) + clusters - 1) / clusters) * cycles; };
+  const long long c256 = cost(256, 512), c192 = cost(192, 448), c128 = cost(128, 384);
+  if (100 * c128 < 95 * std::min(c256, c192)) return 128;
+  return 100 * c192 < 95 * c256 ? 192 : 256;
 }
 
 }  // namespace gemm2

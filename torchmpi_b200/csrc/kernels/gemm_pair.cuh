@@ -40,10 +40,12 @@ struct Shared {
   int error;
 };
 
+// NST: stages of the operand ring in use; one fewer leaves its 32 KB to the epilogue's staging.
+template <int NST = STAGES>
 __device__ __forceinline__ void carve(unsigned char* raw, unsigned char** tiles, Shared** sh, unsigned char** staging) {
   uintptr_t base = ((uintptr_t)raw + 1023) & ~(uintptr_t)1023;
   *tiles = (unsigned char*)base;
-  *staging = (unsigned char*)(base + (size_t)STAGES * STAGE_BYTES);
+  *staging = (unsigned char*)(base + (size_t)NST * STAGE_BYTES);
   *sh = (Shared*)(base + (size_t)STAGES * STAGE_BYTES + gemm::EPI_STAGING_BYTES);
 }
 
@@ -69,12 +71,13 @@ __device__ __forceinline__ void setup(Shared* sh, int warp, const CUtensorMap* m
 }
 
 // One thread in EACH CTA.  order(it, &m_blk, &n_blk): m_blk is this CTA's 128-row block.
-template <typename TileOrder, typename ASource>
+template <int NST = STAGES, typename TileOrder, typename ASource>
 __device__ __forceinline__ void producer(Shared* sh, unsigned char* tiles, const Problem& p, const CUtensorMap* ma,
                                          const CUtensorMap* mb, uint32_t rank, TileOrder order, ASource a_source) {
   const int bn = p.pair_n ? p.pair_n : BN;
-  // bytes of B per stage and CTA: bn / 2 rows, or (MN-major) two whole 64-column boxes, of which bn / 2 columns are used
-  const uint32_t stage_tx = 2 * (A_BYTES + (p.b_mn ? B_BYTES : (bn / 2) * BK * 2));
+  // bytes of B per stage and CTA: bn / 2 rows, or (MN-major) whole 64-column boxes, of which bn / 2 columns are used
+  const bool two_boxes = bn / 2 > 64;
+  const uint32_t stage_tx = 2 * (A_BYTES + (p.b_mn ? (two_boxes ? B_BYTES : B_BYTES / 2) : (bn / 2) * BK * 2));
   int stage = 0;
   uint32_t phase = 0;
   int m_blk, n_blk;
@@ -98,15 +101,15 @@ __device__ __forceinline__ void producer(Shared* sh, unsigned char* tiles, const
         sm100::tma_load_2d_pair(a_dst + A_BYTES, mb, kb * BK, b_row0, full0);
       } else {   // B is [K, N]: two boxes of 64 columns x 64 k-rows, each a column of eight swizzle atoms
         sm100::tma_load_2d_pair(a_dst + A_BYTES, mb, b_row0, kb * BK, full0);
-        sm100::tma_load_2d_pair(a_dst + A_BYTES + B_BYTES / 2, mb, b_row0 + 64, kb * BK, full0);
+        if (two_boxes) sm100::tma_load_2d_pair(a_dst + A_BYTES + B_BYTES / 2, mb, b_row0 + 64, kb * BK, full0);
       }
-      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      if (++stage == NST) { stage = 0; phase ^= 1; }
     }
   }
 }
 
 // One thread of the EVEN CTA only.
-template <typename TileOrder>
+template <int NST = STAGES, typename TileOrder>
 __device__ __forceinline__ void mma_issuer(Shared* sh, unsigned char* tiles, const Problem& p, TileOrder order) {
   const uint32_t idesc = sm100::make_idesc_f16(2 * BM, p.pair_n ? p.pair_n : BN, true, p.b_mn != 0, p.a_mn != 0);
   int stage = 0;
@@ -133,7 +136,7 @@ __device__ __forceinline__ void mma_issuer(Shared* sh, unsigned char* tiles, con
       }
       sm100::umma_commit_pair(sm100::map_to_cta(&sh->empty[stage], 0));   // both producers may refill the stage
       sm100::umma_commit_pair(sm100::map_to_cta(&sh->empty[stage], 1));
-      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      if (++stage == NST) { stage = 0; phase ^= 1; }
     }
     sm100::umma_commit_pair(sm100::map_to_cta(&sh->acc_full[acc], 0));    // both epilogues may read
     sm100::umma_commit_pair(sm100::map_to_cta(&sh->acc_full[acc], 1));
@@ -157,8 +160,9 @@ __device__ __forceinline__ void epilogue(Shared* sh, unsigned char* staging, con
 // slice is read as eight 16-byte loads (64 scalar loads before).  Measured, 8192 x 4096 x 1024 with a bias: 83 -> 52 us; without
 // one 59 -> 50; 8192 x 50264 x 1024: 694 -> 585; 1024^3, where the launch is one tile and its epilogue: 17 -> 15.
 // TWO: gelu(C) is written beside C (map2): GELU of the rounded bf16 value, which is what a separate pass over C computes,
-// without that pass's launch and its read of C.  The group's staging tile is reused for it; the GELU is evaluated in
-// registers while the TMA unit still reads C out of the tile.
+// without that pass's launch and its read of C.  It has staging tiles of its own (the operand ring gives up a stage for
+// them), so a group never waits for the store it has just issued.  8192 x 4096 x 1024: product 83 and pass 36 us before, one
+// kernel of 69 now (82 with one staging tile per group).
 constexpr int GROUPS = 2, GROUP_THREADS = 64 + GROUPS * 128;
 
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
@@ -167,12 +171,11 @@ template <bool TWO, typename TileOrder>
 __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* staging, const Problem& p, int group, int quarter,
                                                 int lane, TileOrder order, const CUtensorMap* map_c, const CUtensorMap* map2) {
   constexpr int SLICE = 64, SLICE_BYTES = BM * SLICE * 2;
-  static_assert(GROUPS * SLICE_BYTES <= gemm::EPI_STAGING_BYTES, "one staging tile per group");
+  static_assert(GROUPS * SLICE_BYTES <= gemm::EPI_STAGING_BYTES && GROUPS * SLICE_BYTES <= STAGE_BYTES, "a staging tile per group and output");
   const int row = quarter * 32 + lane;
   const bool leader = quarter == 0 && lane == 0;
   const int bn = p.pair_n ? p.pair_n : BN;
-  unsigned char* stg = staging + group * SLICE_BYTES;
-  unsigned char* stg_row = stg + row * 128;
+  unsigned char* stg0 = staging + group * SLICE_BYTES;
   const bool bias_vec = ((uintptr_t)p.bias & 15) == 0;
   int m_blk, n_blk;
   for (int it = 0; order(it, &m_blk, &n_blk); ++it) {
@@ -222,28 +225,33 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
         __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[j >> 4][2 * (j & 15)]), __uint_as_float(r[j >> 4][2 * (j & 15) + 1]));
         w[j] = *reinterpret_cast<uint32_t*>(&h);
       }
-      auto put = [&](const CUtensorMap* map) {
-        // the store that used this staging tile before must have read it
-        if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      auto put = [&](const CUtensorMap* map, int which) {
+        unsigned char* stg = stg0 + which * GROUPS * SLICE_BYTES;
+        unsigned char* stg_row = stg + row * 128;
+        // the store that used this staging tile before must have read it (TWO: the other tile's may still be at it)
+        if (leader) {
+          if (TWO) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
         group_sync(group);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
           *reinterpret_cast<uint4*>(stg_row + ((u ^ (row & 7)) << 4)) = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
         sm100::fence_proxy_async_smem();       // generic-proxy writes to shared memory -> visible to the TMA unit
         group_sync(group);
-        if (store) {
-          gemm::tma_store_2d(map, stg, col0, row0);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
+        if (store) gemm::tma_store_2d(map, stg, col0, row0);
+        if (leader) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       };
-      put(map_c);
+      put(map_c, 0);
       if (TWO) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {         // bf16 -> fp32 is a shift or a mask
-          __nv_bfloat162 h = __floats2bfloat162_rn(gelu_value(__uint_as_float(w[j] << 16)), gelu_value(__uint_as_float(w[j] & 0xffff0000u)));
+          float y0, y1;
+          gelu_value2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u), &y0, &y1);
+          __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
           w[j] = *reinterpret_cast<uint32_t*>(&h);
         }
-        put(map2);
+        put(map2, 1);
       }
     }
     sm100::tc_fence_before();
@@ -251,8 +259,8 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
     if (lane == 0) sm100::mbar_arrive_cluster(sm100::map_to_cta(&sh->acc_empty[acc], 0));
   }
   if (leader) {
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // all stores complete before exit
-    sm100::fence_proxy_async();
+    // the tiles have been read before the CTA gives its shared memory back; the writes themselves complete with the kernel
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   }
 }
 
