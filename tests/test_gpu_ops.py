@@ -309,3 +309,70 @@ def test_bn_pool_stage_edges_and_ties(dtype, N, C, H, W):
     tol = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}[dtype]      # two-stage rounds the routed gradient to dtype
     for a, b in zip(got[1], got[0]):
         assert (a - b).abs().max().item() <= tol * max(1.0, b.abs().max().item()) * 2, (dtype, (a - b).abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 1, 0), (7, 33, 0), (336, 10, 0), (900, 128, 0), (300, 1000, 1008), (5, 1024, 0),
+                                             (3, 1025, 0), (700, 5003, 5008), (2, 60001, 0)])
+def test_cross_entropy_row_lengths(rows, cols, pitch, dtype):
+    """A warp per row, a block per row in shared memory (misaligned rows, a pitch) and the fallback for rows that do not fit
+    there: loss and gradient against fp64, labels outside the row included, padding columns cleared."""
+    from torchmpi_b200.ops import xent
+    torch.manual_seed(rows + cols)
+    buf = torch.randn(rows, pitch or cols, device="cuda").mul_(3.0).to(dtype)
+    x = buf[:, :cols].detach().requires_grad_(True)
+    labels = torch.randint(0, cols, (rows,), device="cuda")
+    loss = xent.cross_entropy(x, labels)
+    loss.backward()
+    ref_x = x.detach().double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(ref_x, labels)
+    ref.backward()
+    assert loss.shape == ref.shape
+    assert abs(loss.item() - ref.item()) <= 2e-6 * max(1.0, abs(ref.item()))
+    # exponentials from the special-function unit (2 ulp), fp16 between the passes of long 16-bit rows, one final rounding
+    unit = {torch.float32: 2e-6, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7.5}[dtype]
+    err = (x.grad.double() - ref_x.grad).abs()
+    # fp16 subnormals of the result; exponentials below 2^-14 kept as fp16 subnormals, and the label's p - 1, which cancels
+    floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / rows
+    assert bool((err <= unit * ref_x.grad.abs() + floor).all()), (err / (ref_x.grad.abs() + 1e-30)).max().item()
+
+
+def test_cross_entropy_infinities_and_bad_labels():
+    from torchmpi_b200.ops import xent
+    for cols in (40, 3000):
+        x = torch.randn(6, cols, device="cuda")
+        x[0, 1:] = float("-inf")                           # one class left
+        x[1, ::2] = float("-inf")
+        x[2, 3] = float("nan")
+        x[3] = torch.finfo(torch.float32).min              # a mask of the type's lowest value: uniform
+        xg = x.clone().requires_grad_(True)
+        labels = torch.zeros(6, dtype=torch.int64, device="cuda")
+        labels[1] = 1
+        loss = xent.cross_entropy(xg, labels)
+        loss.backward()
+        ref = x.clone().requires_grad_(True)
+        torch.nn.functional.cross_entropy(ref, labels).backward()
+        assert torch.isnan(loss)
+        for r in (0, 1, 3, 4, 5) if cols <= 1024 else (0, 1, 4, 5):     # the long-row kernel forms max * log2(e): NaN at the lowest value
+            assert torch.allclose(xg.grad[r], ref.grad[r], rtol=1e-5, atol=1e-8), (cols, r)
+        assert torch.isnan(xg.grad[2]).all()
+
+
+@pytest.mark.parametrize("n", [8, 4096, 511 * 8, 1_000_008])
+def test_elementwise_updates_at_block_edges(n):
+    """One pack per thread (SGD) and two (EASGD, Downpour): tensors of one pack, whole blocks, a cut last block."""
+    from torchmpi_b200.ops import elementwise as ew
+    torch.manual_seed(n)
+    for dtype in (torch.bfloat16, torch.float32):
+        local, center = torch.randn(n, device="cuda").to(dtype), torch.randn(n, device="cuda").to(dtype)
+        l0, delta = local.clone(), torch.full_like(local, 7.0)
+        ew.easgd_elastic(local, center, delta, 0.25)
+        d = center.float() - l0.float()
+        assert torch.equal(local, (l0.float() + 0.25 * d).to(dtype)) and torch.equal(delta, (-0.25 * d).to(dtype))
+        acc = l0.clone()
+        ew.downpour_accum(acc, center, scale=0.5)
+        assert torch.equal(acc, (l0.float() + 0.5 * center.float()).to(dtype))
+        w, m = l0.clone(), torch.zeros(n, device="cuda")
+        master = l0.float() if dtype != torch.float32 else None
+        ew.sgd_momentum_(w, center, lr=0.5, momentum=0.5, master=master, momentum_buf=m, first_step=True, zero_grad=False)
+        assert torch.equal(m, center.float()) and torch.equal(w, (l0.float() - 0.5 * center.float()).to(dtype))

@@ -171,6 +171,7 @@ _CUDA_PROTOS = {
     "tmpi_cuda_ps_pull": (_i, [_sz, _vp, _sz, _i, _gp, _vp]),
     "tmpi_sgd_momentum": (_i, [_vp, _i, _vp, _i, _vp, _vp, _sz, _f, _f, _f, _f, _f, _i, _i, _i, _vp]),
     "tmpi_xent_fwd_bwd": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _f, _vp, _vp]),
+    "tmpi_xent_mean_fwd_bwd_ld": (_i, [_vp, _i, _vp, _i, _i, _i, _vp, _vp, _f, _vp, _vp]),
     "tmpi_xent_fwd_bwd_ld": (_i, [_vp, _i, _vp, _i, _i, _i, _vp, _vp, _f, _vp, _vp]),
     "tmpi_xent_scratch_bytes": (_sz, [_i]),
     "tmpi_cuda_ps_push_async": (_u64, [_sz, _vp, _sz, _i, _i, _gp, _vp]),

@@ -229,6 +229,9 @@ int tmpi_xent_fwd_bwd(const void* logits, int dtype, const int64_t* labels, int 
 // the same with a row pitch `ld` (elements) for logits and dlogits; dlogits columns cols..ld-1 are zeroed
 int tmpi_xent_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld,
                       float* loss_sum, void* dlogits, float grad_scale, void* scratch, void* stream);
+// the mean of the row losses in place of their sum
+int tmpi_xent_mean_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld,
+                              float* loss_mean, void* dlogits, float grad_scale, void* scratch, void* stream);
 int tmpi_absmean_var(const void* x, int dtype, size_t n, double* out2, void* scratch, void* stream);
 size_t tmpi_absmean_var_scratch_bytes(void);
 int tmpi_easgd_elastic(void* local, const void* center, void* delta, size_t n, int dtype,

@@ -34,7 +34,7 @@ static int sm_count() {
 template <typename T>
 __global__ void __launch_bounds__(256) xent_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                                                    int rows, int cols, int ld, float* __restrict__ loss_out,
-                                                   T* __restrict__ dlogits, float gscale,
+                                                   T* __restrict__ dlogits, float gscale, float divisor,
                                                    float* __restrict__ row_loss, unsigned* __restrict__ counter) {
   __shared__ float s_red[32];
   __shared__ float s_bcast;
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) xent_kernel(const T* __restrict__ logits,
     if (threadIdx.x == 0) {
       float t = 0.f;
       for (int w = 0; w < nwarp; ++w) t += s_red[w];
-      loss_out[0] = t;
+      loss_out[0] = t / divisor;
       *counter = 0;
     }
   }
@@ -179,6 +179,74 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// What the kernel below ends with: the row's loss is published, and the block that arrives last adds all of them in a
+// fixed order and divides by `divisor`.
+template <int THREADS>
+__device__ __forceinline__ void xent_finish(int rows, const float* __restrict__ row_loss, unsigned* __restrict__ counter,
+                                            unsigned arrivals, float divisor, float* __restrict__ loss_out) {
+  __shared__ float s_fin[THREADS / 32];
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == arrivals - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  float v = 0.f;
+  for (int i = threadIdx.x; i < rows; i += THREADS) v += row_loss[i];   // fixed per-thread order
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+  if ((threadIdx.x & 31) == 0) s_fin[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int w = 0; w < THREADS / 32; ++w) t += s_fin[w];
+    loss_out[0] = t / divisor;
+    *counter = 0;
+  }
+}
+
+// Rows of up to 32 * PER elements: one warp per row, the row in registers (PER values per lane), no shared memory and no
+// barrier per row.  A block per row spends its time in three block reductions: 8192 x 1000 fp32 took 51 us, now 15.5;
+// 336 x 10 5.4, now 3.9.
+template <typename T, int PER>
+__global__ void __launch_bounds__(256) xent_warp_kernel(const T* __restrict__ logits, const long long* __restrict__ labels, int rows,
+                                                        int cols, int ld, float* __restrict__ loss_out, T* __restrict__ dlogits,
+                                                        float gscale, float divisor, float* __restrict__ row_loss,
+                                                        unsigned* __restrict__ counter) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  const int lane = threadIdx.x & 31;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
+    const T* x = logits + (size_t)r * ld;
+    const int label = (int)labels[r];
+    float v[PER], m = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) v[j] = lane + 32 * j < cols ? (float)to_acc<T>(x[lane + 32 * j]) : -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) m = fmaxf(m, v[j]);
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(~0u, m, o));
+    float xl = m;                                          // a label outside the row counts as the maximum
+    if (label >= 0 && label < cols) xl = (float)to_acc<T>(x[label]);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      v[j] = lane + 32 * j < cols ? ex2_approx((v[j] - m) * kLog2e) : 0.f;
+      sum += v[j];
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(~0u, sum, o);
+    if (lane == 0) row_loss[r] = __logf(sum) + m - xl;
+    if (dlogits) {
+      T* d = dlogits + (size_t)r * ld;
+      const float inv = 1.f / sum;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int c = lane + 32 * j;
+        if (c < cols) d[c] = from_acc<T>((typename AccOf<T>::type)((v[j] * inv - (c == label ? 1.f : 0.f)) * gscale));
+      }
+      for (int c = cols + lane; c < ld; c += 32) d[c] = from_acc<T>((typename AccOf<T>::type)0.f);      // pitch padding
+    }
+  }
+  xent_finish<256>(rows, row_loss, counter, gridDim.x, divisor, loss_out);
+}
+
 // One block per row with the row staged in shared memory: the logits are read from HBM once and the gradient is
 // written once.  The aligned body of the row travels as asynchronous 16-byte copies that are all in flight together
 // (the row keeps its global misalignment in shared memory, so aligned global packs land on aligned shared addresses;
@@ -189,7 +257,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS) xent_row_smem_kernel(
     const T* __restrict__ logits, const long long* __restrict__ labels, int rows, int cols, int ld,
-    float* __restrict__ loss_out, T* __restrict__ dlogits, float gscale, float* __restrict__ row_loss,
+    float* __restrict__ loss_out, T* __restrict__ dlogits, float gscale, float divisor, float* __restrict__ row_loss,
     unsigned* __restrict__ counter) {
   extern __shared__ __align__(16) unsigned char s_row_raw[];
   __shared__ float s_red[32];
@@ -310,7 +378,7 @@ __global__ void __launch_bounds__(THREADS) xent_row_smem_kernel(
     if (tid == 0) {
       float t = 0.f;
       for (int w = 0; w < nwarp; ++w) t += s_red[w];
-      loss_out[0] = t;
+      loss_out[0] = t / divisor;
       *counter = 0;
     }
   }
@@ -402,37 +470,53 @@ __global__ void __launch_bounds__(kStatThreads) absstat_kernel(const T* x, size_
 }
 
 // ------------------------------------------------------------------ EASGD / Downpour
+// Two packs per thread, no loop: every load of the block is in flight before the first use and the grid covers the tensor
+// (a capped grid that strode over it held half as many loads per SM).  Measured at 23.5 M bf16 parameters, easgd: 33.0 -> 29.7 us.
 template <typename T, int V>
 __global__ void __launch_bounds__(256) easgd_kernel(T* __restrict__ local, const T* __restrict__ center,
                                                     T* __restrict__ delta, size_t nv, float alpha) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x) {
-    Pack<T, V> x = ld_pack<T, V>(local + i * V), c = ld_pack<T, V>(center + i * V), d;
+  const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
+  Pack<T, V> x[2], c[2], d[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (i0 + 256 * u < nv) { x[u] = ld_pack<T, V>(local + (i0 + 256 * u) * V); c[u] = ld_pack<T, V>(center + (i0 + 256 * u) * V); }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (i0 + 256 * u >= nv) break;
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      float xv = (float)to_acc<T>(x.v[k]);
-      float dv = (float)to_acc<T>(c.v[k]) - xv;
-      x.v[k] = from_acc<T>((typename AccOf<T>::type)(xv + alpha * dv));
-      d.v[k] = from_acc<T>((typename AccOf<T>::type)(-alpha * dv));
+      float xv = (float)to_acc<T>(x[u].v[k]);
+      float dv = (float)to_acc<T>(c[u].v[k]) - xv;
+      x[u].v[k] = from_acc<T>((typename AccOf<T>::type)(xv + alpha * dv));
+      d[u].v[k] = from_acc<T>((typename AccOf<T>::type)(-alpha * dv));
     }
-    st_pack<T, V>(local + i * V, x);
-    st_pack<T, V>(delta + i * V, d);
+    st_pack<T, V>(local + (i0 + 256 * u) * V, x[u]);
+    st_pack<T, V>(delta + (i0 + 256 * u) * V, d[u]);
   }
 }
 
 template <typename T, int V>
 __global__ void __launch_bounds__(256) accum_kernel(T* __restrict__ acc, const T* __restrict__ g, size_t nv,
                                                     float scale, int zero_first) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x) {
-    Pack<T, V> a = ld_pack<T, V>(acc + i * V), x = ld_pack<T, V>(g + i * V);
+  const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
+  Pack<T, V> a[2], x[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (i0 + 256 * u < nv) { a[u] = ld_pack<T, V>(acc + (i0 + 256 * u) * V); x[u] = ld_pack<T, V>(g + (i0 + 256 * u) * V); }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (i0 + 256 * u >= nv) break;
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      float av = zero_first ? 0.f : (float)to_acc<T>(a.v[k]);
-      a.v[k] = from_acc<T>((typename AccOf<T>::type)(av + scale * (float)to_acc<T>(x.v[k])));
+      float av = zero_first ? 0.f : (float)to_acc<T>(a[u].v[k]);
+      a[u].v[k] = from_acc<T>((typename AccOf<T>::type)(av + scale * (float)to_acc<T>(x[u].v[k])));
     }
-    st_pack<T, V>(acc + i * V, a);
+    st_pack<T, V>(acc + (i0 + 256 * u) * V, a[u]);
   }
 }
 
+// blocks of 512 packs; a tensor of up to 2^40 packs
+static unsigned pack_blocks(size_t nv) { return (unsigned)std::max<size_t>(1, (nv + 511) / 512); }
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
@@ -449,9 +533,23 @@ using namespace tmpi;
     default: return fail(TMPI_ERR_UNSUPPORTED, "dtype %d not supported here", dtype); \
   }
 
+// Rows of up to 1024: a warp each.  Longer rows that fit in shared memory twice per SM: a block with the row staged there.
+// (One persistent block per SM with two row buffers, the next row on its way, was slower: 8192 x 50257 bf16 took 531 us with
+// 512 threads and 562 with 1024 in place of 450.)  The rest: a block per row that reads it three times.
 template <typename T>
 static cudaError_t launch_xent(const void* logits, const int64_t* labels, int rows, int cols, int ld, float* loss_sum, void* dlogits,
-                               float gscale, float* row_loss, unsigned* counter, cudaStream_t s) {
+                               float gscale, float divisor, float* row_loss, unsigned* counter, cudaStream_t s) {
+  const T* x = (const T*)logits;
+  T* d = (T*)dlogits;
+  const long long* lab = (const long long*)labels;
+  if (cols <= 1024) {
+    const int grid = std::min((rows + 7) / 8, sm_count() * 8);
+    if (cols <= 32) xent_warp_kernel<T, 1><<<grid, 256, 0, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
+    else if (cols <= 128) xent_warp_kernel<T, 4><<<grid, 256, 0, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
+    else if (cols <= 512) xent_warp_kernel<T, 16><<<grid, 256, 0, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
+    else xent_warp_kernel<T, 32><<<grid, 256, 0, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
+    return cudaGetLastError();
+  }
   // 512 threads measured faster than 1024 (0.37 against 0.39 ms for 8192 x 50257 bf16)
   constexpr int kThreads = 512;
   constexpr size_t kMaxRowBytes = 112 * 1024;          // two such blocks per SM
@@ -461,13 +559,69 @@ static cudaError_t launch_xent(const void* logits, const int64_t* labels, int ro
     cudaError_t ae = cudaFuncSetAttribute(xent_row_smem_kernel<T, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kMaxRowBytes);
     if (ae != cudaSuccess) return ae;
-    xent_row_smem_kernel<T, kThreads><<<rows, kThreads, row_bytes, s>>>((const T*)logits, (const long long*)labels, rows, cols, ld,
-                                                                        loss_sum, (T*)dlogits, gscale, row_loss, counter);
+    xent_row_smem_kernel<T, kThreads><<<rows, kThreads, row_bytes, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
   } else {
-    xent_kernel<T><<<rows, 256, 0, s>>>((const T*)logits, (const long long*)labels, rows, cols, ld, loss_sum, (T*)dlogits, gscale,
-                                        row_loss, counter);
+    xent_kernel<T><<<rows, 256, 0, s>>>(x, lab, rows, cols, ld, loss_sum, d, gscale, divisor, row_loss, counter);
   }
   return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ SGD on one rank
+// The step of ar_sgd.cu without peers: one 16-byte pack of the weight type per thread and no loop, so that the whole chip
+// has loads in flight and its 20 bytes per parameter (bf16 weights, fp32 master and momentum) move at the copy rate.  The
+// collective kernel's grid is capped by its flag table (256 blocks on 148 SMs, some with two, some with one): 25.6 M
+// parameters took 117 us, now 78.
+struct SgdStep { float lr, momentum, dampening, weight_decay, grad_scale; int nesterov, first_step, zero_grads; };
+
+template <typename T, int V>
+__global__ void __launch_bounds__(256) sgd_step_kernel(T* __restrict__ weight, T* __restrict__ grad, float* __restrict__ master,
+                                                       float* __restrict__ mom, size_t nv, SgdStep a) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= nv) return;
+  const Pack<T, V> gp = ld_pack<T, V>(grad + i * V);
+  float w[V], m[V];
+  if (master) {
+#pragma unroll
+    for (int k = 0; k < V; k += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(master + i * V + k);
+      w[k] = f.x; w[k + 1] = f.y; w[k + 2] = f.z; w[k + 3] = f.w;
+    }
+  } else {
+    const Pack<T, V> x = ld_pack<T, V>(weight + i * V);
+#pragma unroll
+    for (int k = 0; k < V; ++k) w[k] = (float)to_acc<T>(x.v[k]);
+  }
+  if (mom && !a.first_step) {
+#pragma unroll
+    for (int k = 0; k < V; k += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(mom + i * V + k);
+      m[k] = f.x; m[k + 1] = f.y; m[k + 2] = f.z; m[k + 3] = f.w;
+    }
+  }
+  Pack<T, V> out;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    float g = (float)to_acc<T>(gp.v[k]) * a.grad_scale;
+    if (a.weight_decay != 0.f) g += a.weight_decay * w[k];
+    if (mom) {
+      m[k] = a.first_step ? g : a.momentum * m[k] + (1.f - a.dampening) * g;
+      g = a.nesterov ? g + a.momentum * m[k] : m[k];
+    }
+    w[k] -= a.lr * g;
+    out.v[k] = from_acc<T>((typename AccOf<T>::type)w[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < V; k += 4) {
+    if (master) *reinterpret_cast<float4*>(master + i * V + k) = make_float4(w[k], w[k + 1], w[k + 2], w[k + 3]);
+    if (mom) *reinterpret_cast<float4*>(mom + i * V + k) = make_float4(m[k], m[k + 1], m[k + 2], m[k + 3]);
+  }
+  st_pack<T, V>(weight + i * V, out);
+  if (a.zero_grads) {
+    Pack<T, V> z;
+#pragma unroll
+    for (int k = 0; k < V; ++k) z.v[k] = from_acc<T>((typename AccOf<T>::type)0);
+    st_pack<T, V>(grad + i * V, z);
+  }
 }
 
 extern "C" {
@@ -479,16 +633,19 @@ int tmpi_sgd_momentum(void* weight, int wdt, const void* grad, int gdt, void* ma
   size_t es = dtype_size(wdt), V = 16 / es;
   if (n % V || !aligned16(weight) || !aligned16(grad) || !aligned16(master) || !aligned16(momentum))
     return fail(TMPI_ERR_INVALID, "sgd: buffers must be 16-byte aligned and hold a multiple of %zu elements", V);
-  SgdArgs a{};
-  a.P.n = 1; a.P.me = 0; a.P.base[0] = nullptr; a.P.status = nullptr;
-  // with a null heap base the "offsets" are the absolute addresses
-  a.grad_off = (size_t)grad; a.weight_off = (size_t)weight;
-  a.master = (float*)master; a.momentum = (float*)momentum; a.n = n;
-  a.lr = lr; a.momentum_coef = mc; a.dampening = damp; a.weight_decay = wd; a.grad_scale = gscale;
-  a.nesterov = nesterov; a.first_step = first_step; a.zero_grads = zero_grads; a.use_nvls = 0;
-  size_t nv = n / V;
-  int grid = (int)std::min<size_t>((nv + 511) / 512, (size_t)sm_count() * 2);
-  cudaError_t e = launch_allreduce_sgd(gdt, wdt, &a, 1, grid < 1 ? 1 : grid, 512, (cudaStream_t)stream);
+  const SgdStep a{lr, mc, damp, wd, gscale, nesterov, first_step, zero_grads};
+  const size_t nv = n / V, blocks = (nv + 255) / 256;
+  if (!nv) return TMPI_OK;
+  if (blocks > 0x7fffffffULL) return fail(TMPI_ERR_INVALID, "sgd: too many elements");
+  cudaStream_t s = (cudaStream_t)stream;
+  float *ms = (float*)master, *mo = (float*)momentum;
+  switch (wdt) {
+    case TMPI_BF16: sgd_step_kernel<__nv_bfloat16, 8><<<(unsigned)blocks, 256, 0, s>>>((__nv_bfloat16*)weight, (__nv_bfloat16*)const_cast<void*>(grad), ms, mo, nv, a); break;
+    case TMPI_F16: sgd_step_kernel<__half, 8><<<(unsigned)blocks, 256, 0, s>>>((__half*)weight, (__half*)const_cast<void*>(grad), ms, mo, nv, a); break;
+    case TMPI_F32: sgd_step_kernel<float, 4><<<(unsigned)blocks, 256, 0, s>>>((float*)weight, (float*)const_cast<void*>(grad), ms, mo, nv, a); break;
+    default: return cuda_fail(cudaErrorInvalidValue, "sgd_momentum launch");
+  }
+  cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : cuda_fail(e, "sgd_momentum launch");
 }
 
@@ -504,8 +661,8 @@ int tmpi_xent_fwd_bwd(const void* logits, int dtype, const int64_t* labels, int 
   return tmpi_xent_fwd_bwd_ld(logits, dtype, labels, rows, cols, cols, loss_sum, dlogits, gscale, scratch, stream);
 }
 
-int tmpi_xent_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld, float* loss_sum,
-                         void* dlogits, float gscale, void* scratch, void* stream) {
+static int xent_fwd_bwd(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld, float* loss, void* dlogits,
+                        float gscale, float divisor, void* scratch, void* stream) {
   if (rows < 1 || cols < 1) return fail(TMPI_ERR_INVALID, "xent: empty input");
   if (ld == 0) ld = cols;
   if (ld < cols) return fail(TMPI_ERR_INVALID, "xent: row pitch %d below the row length %d", ld, cols);
@@ -515,12 +672,23 @@ int tmpi_xent_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, i
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e;
   switch (dtype) {
-    case TMPI_F32: e = launch_xent<float>(logits, labels, rows, cols, ld, loss_sum, dlogits, gscale, row_loss, counter, s); break;
-    case TMPI_BF16: e = launch_xent<__nv_bfloat16>(logits, labels, rows, cols, ld, loss_sum, dlogits, gscale, row_loss, counter, s); break;
-    case TMPI_F16: e = launch_xent<__half>(logits, labels, rows, cols, ld, loss_sum, dlogits, gscale, row_loss, counter, s); break;
+    case TMPI_F32: e = launch_xent<float>(logits, labels, rows, cols, ld, loss, dlogits, gscale, divisor, row_loss, counter, s); break;
+    case TMPI_BF16: e = launch_xent<__nv_bfloat16>(logits, labels, rows, cols, ld, loss, dlogits, gscale, divisor, row_loss, counter, s); break;
+    case TMPI_F16: e = launch_xent<__half>(logits, labels, rows, cols, ld, loss, dlogits, gscale, divisor, row_loss, counter, s); break;
     default: return fail(TMPI_ERR_UNSUPPORTED, "xent: dtype %d", dtype);
   }
   return e == cudaSuccess ? TMPI_OK : cuda_fail(e, "xent launch");
+}
+
+int tmpi_xent_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld, float* loss_sum,
+                         void* dlogits, float gscale, void* scratch, void* stream) {
+  return xent_fwd_bwd(logits, dtype, labels, rows, cols, ld, loss_sum, dlogits, gscale, 1.f, scratch, stream);
+}
+
+// The mean of the row losses in place of their sum.
+int tmpi_xent_mean_fwd_bwd_ld(const void* logits, int dtype, const int64_t* labels, int rows, int cols, int ld, float* loss_mean,
+                              void* dlogits, float gscale, void* scratch, void* stream) {
+  return xent_fwd_bwd(logits, dtype, labels, rows, cols, ld, loss_mean, dlogits, gscale, (float)rows, scratch, stream);
 }
 
 size_t tmpi_absmean_var_scratch_bytes(void) { return 256 + (size_t)kStatBlocks * 2 * sizeof(double); }
@@ -550,11 +718,9 @@ int tmpi_easgd_elastic(void* local, const void* center, void* delta, size_t n, i
     constexpr int V = 16 / sizeof(T);
     if (vec && n % V == 0) {
       size_t nv = n / V;
-      int grid = (int)std::min<size_t>((nv + 255) / 256, (size_t)sm_count() * 8);
-      easgd_kernel<T, V><<<grid < 1 ? 1 : grid, 256, 0, s>>>((T*)local, (const T*)center, (T*)delta, nv, alpha);
+      easgd_kernel<T, V><<<pack_blocks(nv), 256, 0, s>>>((T*)local, (const T*)center, (T*)delta, nv, alpha);
     } else {
-      int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-      easgd_kernel<T, 1><<<grid < 1 ? 1 : grid, 256, 0, s>>>((T*)local, (const T*)center, (T*)delta, n, alpha);
+      easgd_kernel<T, 1><<<pack_blocks(n), 256, 0, s>>>((T*)local, (const T*)center, (T*)delta, n, alpha);
     }
   });
   cudaError_t e = cudaGetLastError();
@@ -568,11 +734,9 @@ int tmpi_downpour_accum(void* accum, const void* grad, size_t n, int dtype, floa
     constexpr int V = 16 / sizeof(T);
     if (vec && n % V == 0) {
       size_t nv = n / V;
-      int grid = (int)std::min<size_t>((nv + 255) / 256, (size_t)sm_count() * 8);
-      accum_kernel<T, V><<<grid < 1 ? 1 : grid, 256, 0, s>>>((T*)accum, (const T*)grad, nv, scale, zero_first);
+      accum_kernel<T, V><<<pack_blocks(nv), 256, 0, s>>>((T*)accum, (const T*)grad, nv, scale, zero_first);
     } else {
-      int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-      accum_kernel<T, 1><<<grid < 1 ? 1 : grid, 256, 0, s>>>((T*)accum, (const T*)grad, n, scale, zero_first);
+      accum_kernel<T, 1><<<pack_blocks(n), 256, 0, s>>>((T*)accum, (const T*)grad, n, scale, zero_first);
     }
   });
   cudaError_t e = cudaGetLastError();
