@@ -335,6 +335,8 @@ def test_cross_entropy_row_lengths(rows, cols, pitch, dtype):
     # fp16 subnormals of the result; exponentials below 2^-14 kept as fp16 subnormals, and the label's p - 1, which cancels
     floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / rows
     assert bool((err <= unit * ref_x.grad.abs() + floor).all()), (err / (ref_x.grad.abs() + 1e-30)).max().item()
+    with pytest.raises(RuntimeError):
+        loss.backward()                                    # the stored gradient has been handed out
 
 
 def test_cross_entropy_infinities_and_bad_labels():
@@ -376,3 +378,22 @@ def test_elementwise_updates_at_block_edges(n):
         master = l0.float() if dtype != torch.float32 else None
         ew.sgd_momentum_(w, center, lr=0.5, momentum=0.5, master=master, momentum_buf=m, first_step=True, zero_grad=False)
         assert torch.equal(m, center.float()) and torch.equal(w, (l0.float() - 0.5 * center.float()).to(dtype))
+
+
+def test_native_autograd_functions_save_through_hooks():
+    """The C++ functions keep their inputs as saved tensors: pack / unpack hooks see them, and the gradients are the same."""
+    from torchmpi_b200.ops import attention, gemm, layernorm
+    torch.manual_seed(0)
+    lin = gemm.Linear(128, 384, gelu=True).cuda().to(torch.bfloat16)
+    ln = layernorm.LayerNorm(256).cuda().to(torch.bfloat16)
+    cases = [(lambda t: lin(t), torch.randn(64, 128)), (lambda t: ln(t), torch.randn(40, 256)),
+             (lambda t: attention.causal_attention(t, 2), torch.randn(1, 128, 384))]
+    for fn, x in cases:
+        x = x.cuda().to(torch.bfloat16)
+        a, b = x.clone().requires_grad_(True), x.clone().requires_grad_(True)
+        fn(a).float().square().sum().backward()
+        seen = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.shape), t.cpu())[1], lambda t: t.cuda()):
+            fn(b).float().square().sum().backward()
+        assert seen
+        assert ((a.grad.float() - b.grad.float()).norm() / a.grad.float().norm()).item() < 1e-3

@@ -2,7 +2,7 @@
 
 ``python -m torchmpi_b200.build`` compiles every file under ``csrc/runtime``
 (host runtime) and ``csrc/kernels`` (CUDA) to an object under ``build/`` and
-links them into ``torchmpi_b200/lib/libtorchmpi_b200.so``.  Objects are rebuilt
+links them into ``torchmpi_b200/lib/libtorchmpi_b200.so``; g++ compiles ``csrc/bindings`` into ``lib/_autograd.so``.  Objects are rebuilt
 only when their source or a header is newer.  nvcc cross-compiles without a
 GPU, so this runs on a CPU-only machine too.
 
@@ -63,6 +63,55 @@ def is_current() -> bool:
     return LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == source_hash()
 
 
+# ---- C++ autograd functions: compiled against PyTorch's headers, resolved against the native library at load time
+BINDINGS_SRC = CSRC / "bindings" / "autograd.cpp"
+BINDINGS = PKG / "lib" / "_autograd.so"
+BINDINGS_STAMP = PKG / "lib" / "bindings.stamp"
+
+
+def bindings_hash() -> str:
+    import hashlib
+    import torch
+    h = hashlib.sha256(torch.__version__.encode() + sys.version.encode())
+    for f in (BINDINGS_SRC, CSRC / "include" / "tmpi_c_api.h"):
+        h.update(f.read_bytes())
+    return h.hexdigest()
+
+
+def bindings_current() -> bool:
+    return BINDINGS.exists() and BINDINGS_STAMP.exists() and BINDINGS_STAMP.read_text().strip() == bindings_hash()
+
+
+def build_bindings(force: bool = False) -> Path:
+    import sysconfig
+    import torch
+    cxx = shutil.which("g++")
+    if cxx is None:
+        raise RuntimeError("g++ not found; cannot build the C++ autograd functions")
+    root = Path(torch.__file__).resolve().parent
+    OBJ.mkdir(parents=True, exist_ok=True)
+    BINDINGS.parent.mkdir(parents=True, exist_ok=True)
+    import fcntl
+    with open(OBJ.parent / "lock_bindings", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)     # ranks importing at the same time build once
+        if not force and bindings_current():
+            return BINDINGS
+        cc = nvcc()
+        cuda = Path(cc).resolve().parent.parent / "include" if cc else Path("/usr/local/cuda/include")
+        tmp = BINDINGS.with_suffix(".tmp")
+        cmd = [cxx, "-O2", "-fPIC", "-shared", "-std=c++17", "-DTORCH_EXTENSION_NAME=_autograd", "-DTORCH_API_INCLUDE_EXTENSION_H",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", str(CSRC / "include"),
+               "-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda),
+               "-I", sysconfig.get_paths()["include"], str(BINDINGS_SRC), "-o", str(tmp), "-L", str(root / "lib"),
+               "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{root / 'lib'}"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed for {BINDINGS_SRC.name}:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+        tmp.replace(BINDINGS)
+        BINDINGS_STAMP.write_text(bindings_hash())
+    return BINDINGS
+
+
 def headers_mtime() -> float:
     hs = list(CSRC.rglob("*.h")) + list(CSRC.rglob("*.cuh"))
     return max((h.stat().st_mtime for h in hs), default=0.0)
@@ -120,3 +169,4 @@ def _build_locked(cc: str, force: bool, verbose: bool, ptxas_info: bool) -> Path
 if __name__ == "__main__":
     p = build(force="--force" in sys.argv, verbose="-v" in sys.argv, ptxas_info="--ptxas" in sys.argv)
     print(p)
+    print(build_bindings(force="--force" in sys.argv))

@@ -5,7 +5,8 @@
 the same buffer) and writes the heads side by side, so there is no transpose before or after it.  It also returns
 the row-wise log-sum-exp that a backward pass needs.
 
-Forward and backward are this package's kernels (csrc/kernels/attention.cu, attention_bwd.cu).  ``_BACKWARDS`` can
+Forward and backward are this package's kernels (csrc/kernels/attention.cu, attention_bwd.cu), tied together by the
+autograd function of csrc/bindings/autograd.cpp.  ``_BACKWARDS`` can
 put a library backward first instead, fed with this forward's output and log-sum-exp: cuDNN's attention backward (``aten._scaled_dot_product_cudnn_attention_backward``, 112 us for
 8 x 16 x 1024 x 64 on a B200), else PyTorch's flash-attention backward (246 us); if neither operator accepts the
 call, the backward recomputes the attention with ``F.scaled_dot_product_attention`` under autograd.
@@ -21,10 +22,19 @@ import os
 import torch
 import torch.nn.functional as F
 
+from .. import _native
 from .._lib import lib, check, has_symbol, stream_ptr, TorchMPIError
 
-launch_count = 0
+_launches = 0
 last_backward = ""
+
+
+def __getattr__(name: str):
+    if name == "launch_count":               # attention calls on this package's kernels, the C++ function's included
+        return _launches + _native.launches(_native.ATTENTION)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 HEAD = 64
 # backward kernels in order of preference: this package's, then the libraries'; TORCHMPI_ATTENTION_BACKWARD=cudnn
 # (or flash) puts a library first
@@ -50,7 +60,7 @@ def check_status() -> None:
 
 def attention_forward(qkv: torch.Tensor, n_head: int, need_lse: bool = True):
     """(out [B, T, C], lse [B, H, T] fp32 or None) of causal attention over the packed projection ``qkv``."""
-    global launch_count
+    global _launches
     B, T, C3 = qkv.shape
     C = C3 // 3
     out = torch.empty((B, T, C), dtype=qkv.dtype, device=qkv.device)
@@ -58,14 +68,14 @@ def attention_forward(qkv: torch.Tensor, n_head: int, need_lse: bool = True):
     base, es = qkv.data_ptr(), qkv.element_size()
     check(lib.tmpi_attention_fwd(base, base + C * es, base + 2 * C * es, C3, out.data_ptr(), C,
                                  lse.data_ptr() if need_lse else None, B, T, n_head, 1.0 / math.sqrt(HEAD), stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return out, lse
 
 
 def attention_backward(qkv: torch.Tensor, out: torch.Tensor, lse: torch.Tensor, dout: torch.Tensor, n_head: int) -> torch.Tensor:
     """Gradient of the packed projection ``[B, T, 3 C]`` on this package's backward kernel: dK and dV are written
     into their column blocks by the main kernel, dQ is accumulated in fp32 and rounded into its block by a last pass."""
-    global launch_count
+    global _launches
     B, T, C3 = qkv.shape
     C = C3 // 3
     dout = dout.contiguous()
@@ -76,7 +86,7 @@ def attention_backward(qkv: torch.Tensor, out: torch.Tensor, lse: torch.Tensor, 
     check(lib.tmpi_attention_bwd(base, base + C * es, base + 2 * C * es, C3, out.data_ptr(), C, dout.data_ptr(), C,
                                  lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), gbase, gbase + C * es, gbase + 2 * C * es,
                                  C3, B, T, n_head, 1.0 / math.sqrt(HEAD), stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return dqkv
 
 
@@ -88,6 +98,8 @@ def _reference(qkv: torch.Tensor, n_head: int) -> torch.Tensor:
 
 
 class _AttnFn(torch.autograd.Function):
+    """This package's forward with a library backward (see ``_BACKWARDS``)."""
+
     @staticmethod
     def forward(ctx, qkv, n_head):
         out, lse = attention_forward(qkv, n_head)
@@ -142,4 +154,9 @@ def causal_attention(qkv: torch.Tensor, n_head: int) -> torch.Tensor:
     """Causal multi-head attention over a packed ``[B, T, 3 C]`` projection; returns ``[B, T, C]``."""
     if not supported(qkv, n_head):
         return _reference(qkv, n_head)
+    if _BACKWARDS[0] == "own":
+        global last_backward
+        if qkv.requires_grad:
+            last_backward = "own"
+        return _native.ext().causal_attention(qkv, n_head)
     return _AttnFn.apply(qkv, n_head)

@@ -2,8 +2,8 @@
 
 ``matmul_nt(a, b)`` computes ``a @ b.T`` for row-major ``a [M, K]`` and ``b [N, K]`` (K contiguous,
 bf16), optionally with bias and GELU in the epilogue.  ``linear(x, w, bias, gelu)`` is the autograd
-version: ``dX = dY @ W`` (``matmul_nn``) and ``dW = dY.T @ X`` (``matmul_tn``) read their operands as they
-lie, through MN-major shared-memory descriptors, so backward makes no transposed copies.
+version (csrc/bindings/autograd.cpp): ``dX = dY @ W`` (as ``matmul_nn``) and ``dW = dY.T @ X`` (as ``matmul_tn``) read
+their operands as they lie, through MN-major shared-memory descriptors, so backward makes no transposed copies.
 """
 from __future__ import annotations
 
@@ -11,6 +11,7 @@ from typing import Optional
 
 import torch
 
+from .. import _native
 from .._lib import lib, check, dtype_code, has_symbol, stream_ptr, TorchMPIError
 
 EPI_NONE, EPI_BIAS, EPI_GELU = 0, 1, 2
@@ -21,7 +22,13 @@ A_IS_KM = 8          # the first operand is [K, M] with M contiguous
 def config_get(name: str) -> int:
     from .. import config
     return config.get(name)
-launch_count = 0
+_launches = 0
+
+
+def __getattr__(name: str):
+    if name == "launch_count":           # kernels launched by this module, the C++ functions included
+        return _launches + _native.launches(_native.LINEAR)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def supported(a: torch.Tensor, b: torch.Tensor) -> bool:
@@ -33,7 +40,7 @@ def supported(a: torch.Tensor, b: torch.Tensor) -> bool:
 def matmul_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, gelu: bool = False,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``act(a @ b.T + bias)`` with fp32 accumulation; a: [M, K], b: [N, K], both bf16 and contiguous."""
-    global launch_count
+    global _launches
     if not has_symbol("tmpi_gemm_bf16"):
         raise RuntimeError("torchmpi_b200: native kernel 'tmpi_gemm_bf16' is missing")
     if not supported(a, b):
@@ -46,7 +53,7 @@ def matmul_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = N
     epi = (EPI_BIAS if bias is not None else 0) | (EPI_GELU if gelu else 0)
     check(lib.tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(),
                              bias.contiguous().data_ptr() if bias is not None else None, M, N, K, epi, stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -60,7 +67,7 @@ def matmul_nn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     """``a @ b`` for row-major ``a [M, K]`` and ``b [K, N]`` (N contiguous): the kernel reads ``b`` as it
     lies, through an MN-major shared-memory descriptor, where ``matmul_nt`` would need a transposed
     copy.  Shapes the CTA-pair kernel does not take fall back to that copy."""
-    global launch_count
+    global _launches
     a, b = a.contiguous(), b.contiguous()
     M, K = a.shape
     N = b.shape[1]
@@ -69,7 +76,7 @@ def matmul_nn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     check(lib.tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), None, M, N, K, B_IS_KN, stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -77,7 +84,7 @@ def matmul_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     """``a.T @ b`` for row-major ``a [K, M]`` and ``b [K, N]``: both operands are read as they lie
     (MN-major descriptors), which is the layout of a weight gradient ``dY.T @ X``.  Shapes the CTA-pair
     kernel does not take fall back to transposed copies."""
-    global launch_count
+    global _launches
     a, b = a.contiguous(), b.contiguous()
     K, M = a.shape
     N = b.shape[1]
@@ -88,7 +95,7 @@ def matmul_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     check(lib.tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), None, M, N, K, A_IS_KM | B_IS_KN, stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return out
 
 
@@ -100,9 +107,9 @@ def check_status() -> None:
 
 
 def _gemm_ex(a, b, c, M, N, K, lda, ldb, ldc, flags):
-    global launch_count
+    global _launches
     check(lib.tmpi_gemm_bf16_ex(a.data_ptr(), b.data_ptr(), c.data_ptr(), None, M, N, K, lda, ldb, ldc, flags, stream_ptr()))
-    launch_count += 1
+    _launches += 1
 
 
 class _WideHeadFn(torch.autograd.Function):
@@ -156,7 +163,7 @@ def wide_head(x2: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 def gelu(z: torch.Tensor) -> torch.Tensor:
     """``gelu(z)`` (erf form, no autograd) through ``tmpi_gelu_fwd`` (csrc/kernels/bias_grad.cu: rational erf, so the pass
     is memory bound) where it applies; ``F.gelu`` otherwise.  ``bias_grad(dy, z)`` is its backward."""
-    global launch_count
+    global _launches
     if not (z.is_cuda and z.is_contiguous() and z.dtype in (torch.bfloat16, torch.float16, torch.float32)
             and (z.numel() * z.element_size()) % 16 == 0 and z.data_ptr() % 16 == 0 and has_symbol("tmpi_gelu_fwd")):
         return torch.nn.functional.gelu(z)
@@ -164,28 +171,25 @@ def gelu(z: torch.Tensor) -> torch.Tensor:
     st = lib.tmpi_gelu_fwd(z.data_ptr(), y.data_ptr(), z.numel(), dtype_code(z.dtype), stream_ptr())
     if st:
         check(st)
-    launch_count += 1
+    _launches += 1
     return y
-
-
-_gelu_kernel = gelu          # `_LinearFn.forward` has a flag named `gelu`
 
 
 def matmul_nt_gelu(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor]):
     """``(z, gelu(z))`` with ``z = a @ b.T + bias``: one kernel whose epilogue writes both where the CTA-pair kernel
     applies, the product and a pass over it otherwise."""
-    global launch_count
+    global _launches
     a, b = a.contiguous(), b.contiguous()
     M, K = a.shape
     N = b.shape[0]
     if not (supported(a, b) and has_symbol("tmpi_gemm_bf16_gelu") and pair_kernel_takes(M, N, K)):
         z = matmul_nt(a, b, bias)
-        return z, _gelu_kernel(z)
+        return z, gelu(z)
     z = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     y = torch.empty_like(z)
     check(lib.tmpi_gemm_bf16_gelu(a.data_ptr(), b.data_ptr(), z.data_ptr(), y.data_ptr(),
                                   bias.contiguous().data_ptr() if bias is not None else None, M, N, K, stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return z, y
 
 
@@ -196,7 +200,7 @@ _bg_need = {}
 def bias_grad(dy2: torch.Tensor, z: Optional[torch.Tensor] = None):
     """``(dz, db)`` with ``dz = dy2 * gelu'(z)`` (``dy2`` itself when ``z`` is None) and ``db = dz.sum(0)``, in one
     pass over ``dy2`` (and ``z``) where the kernel applies (csrc/kernels/bias_grad.cu); PyTorch ops otherwise."""
-    global launch_count
+    global _launches
     rows, C = dy2.shape
     per_slab = 128 * (16 // dy2.element_size())
     if not (dy2.is_cuda and dy2.is_contiguous() and C % per_slab == 0 and has_symbol("tmpi_bias_grad")
@@ -222,35 +226,8 @@ def bias_grad(dy2: torch.Tensor, z: Optional[torch.Tensor] = None):
                                 buf.data_ptr(), sp)
     if st:
         check(st)
-    launch_count += 2
+    _launches += 2
     return dz, db
-
-
-class _LinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, bias, gelu):
-        x2 = x.reshape(-1, x.shape[-1])
-        if gelu:
-            z, y = matmul_nt_gelu(x2, w, bias)               # the pre-activation is needed by backward
-            ctx.save_for_backward(x2, w, z)
-        else:
-            y = matmul_nt(x2, w, bias)
-            ctx.save_for_backward(x2, w, None)
-        ctx.has_bias, ctx.gelu, ctx.shape = bias is not None, gelu, x.shape
-        return y.reshape(*x.shape[:-1], w.shape[0])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w, z = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
-        db = None
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            dy2, db = bias_grad(dy2, z if ctx.gelu else None)       # GELU backward and the column sum in one pass
-        elif ctx.gelu:
-            dy2 = torch.ops.aten.gelu_backward(dy2, z)
-        dx = matmul_nn(dy2, w) if ctx.needs_input_grad[0] else None
-        dw = matmul_tn(dy2, x2) if ctx.needs_input_grad[1] else None
-        return (dx.reshape(ctx.shape) if dx is not None else None), dw, db, None
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, gelu: bool = False) -> torch.Tensor:
@@ -258,7 +235,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     rows = x.numel() // max(1, x.shape[-1])
     if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 \
             and w.shape[0] % 8 == 0 and rows % 8 == 0 and has_symbol("tmpi_gemm_bf16"):
-        return _LinearFn.apply(x, w, bias, gelu)
+        return _native.ext().linear(x, w, bias, gelu)
     y = torch.nn.functional.linear(x, w, bias)
     return torch.nn.functional.gelu(y) if gelu else y
 

@@ -83,7 +83,7 @@ def cases(small: bool):
     rows, cols = (8192, 50257) if not small else (2048, 50257)
     logits = torch.randn(rows, cols, device=dev).to(torch.bfloat16)
     labels = torch.randint(0, cols, (rows,), device=dev)
-    out["xent_fwd_bwd"] = (lambda: xent._XentFn.apply(logits, labels), rows * cols * 2 * 2)  # x once (the row is kept in shared memory), dx once
+    out["xent_fwd_bwd"] = (lambda: xent.cross_entropy(logits, labels), rows * cols * 2 * 2)  # x once (the row is kept in shared memory), dx once
 
     big = torch.randn((64 if small else 256) << 20, device=dev)
     stat_scratch = torch.zeros(lib.tmpi_absmean_var_scratch_bytes(), dtype=torch.uint8, device=dev)
@@ -135,7 +135,8 @@ def lazy_cases(small: bool) -> dict:
     """name -> builder; a builder allocates its inputs and returns ``(fn, bytes[, flops])``.  Built only when
     selected, so that a profiler capture of one kernel holds little memory."""
     import torch.nn.functional as F
-    from torchmpi_b200.ops import conv, layernorm, pool
+    from torchmpi_b200 import _native
+    from torchmpi_b200.ops import conv, pool
     from torchmpi_b200._lib import lib, dtype_code, stream_ptr, check
     dev = torch.device("cuda")
     B = 64 if small else 256
@@ -216,8 +217,8 @@ def lazy_cases(small: bool) -> dict:
             g = torch.ones(C, device=dev, dtype=torch.bfloat16, requires_grad=True)
             b = torch.zeros(C, device=dev, dtype=torch.bfloat16, requires_grad=True)
             if not backward:
-                return (lambda: layernorm._LayerNormFn.apply(x.detach(), g.detach(), b.detach(), 1e-5)), rows * C * 2 * 2
-            y = layernorm._LayerNormFn.apply(x, g, b, 1e-5)
+                return (lambda: _native.ext().layer_norm(x.detach(), g.detach(), b.detach(), 1e-5)), rows * C * 2 * 2
+            y = _native.ext().layer_norm(x, g, b, 1e-5)
             dy = torch.randn_like(y)
             return (lambda: torch.autograd.grad(y, (x, g, b), dy, retain_graph=True)), rows * C * 2 * 3
         return build
