@@ -254,3 +254,30 @@ def test_pair_gemm_narrow_tiles(M, N, K):
     odd = torch.randn(N + 1, device="cuda").to(torch.bfloat16)[1:]         # a bias that 16-byte loads cannot read
     assert rel(gemm.matmul_nt(a, b, odd), ref + odd.float()) < 4e-3
     gemm.check_status()
+
+
+@pytest.mark.parametrize("gelu", [False, True])
+@pytest.mark.parametrize("rows,n", [(8, 16), (264, 512)])
+@pytest.mark.parametrize("bias,frozen", [(False, ""), (False, "x"), (True, "w"), (True, "b"), (True, "xw")])
+def test_linear_without_bias_and_with_frozen_inputs(gelu, rows, n, bias, frozen):
+    """Every combination of a missing bias and inputs that want no gradient, with small operands and on the CTA-pair kernel."""
+    from torchmpi_b200.ops import gemm
+    torch.manual_seed(rows)
+    k = 256
+    t = {"x": torch.randn(2, rows, k), "w": torch.randn(n, k) / 16, "b": torch.randn(n)}
+    t = {a: v.cuda().to(torch.bfloat16).requires_grad_(a not in frozen) for a, v in t.items()}
+    r = {a: v.detach().float().requires_grad_(a not in frozen) for a, v in t.items()}
+    y = gemm.linear(t["x"], t["w"], t["b"] if bias else None, gelu=gelu)
+    z = torch.nn.functional.linear(r["x"], r["w"], r["b"] if bias else None)
+    ref = torch.nn.functional.gelu(z) if gelu else z
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    ref.backward(dy.float())
+    gemm.check_status()
+    # one rounding to bf16 (2^-9) of the result, and with GELU of z before it and of dz in front of the products
+    assert (y.float() - ref).norm() <= 2 ** -7 * ref.norm()
+    for a in "xwb":
+        if a in frozen or (a == "b" and not bias):
+            assert t[a].grad is None
+        else:
+            assert (t[a].grad.float() - r[a].grad).norm() <= 2 ** -7 * r[a].grad.norm(), a

@@ -116,7 +116,8 @@ std::pair<Tensor, Tensor> bias_grad(const Tensor& dy, const Tensor& z) {
 }
 
 struct LinearFn : public torch::autograd::Function<LinearFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& bias, bool with_gelu) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias_, bool with_gelu) {
+    const Tensor bias = bias_.has_value() ? *bias_ : Tensor();
     Tensor x2 = x.reshape({-1, x.size(-1)}), y, z;
     if (with_gelu) std::tie(z, y) = matmul_nt_gelu(x2, w, bias);          // the pre-activation is needed by backward
     else y = matmul_nt(x2, w, bias);
@@ -233,7 +234,7 @@ struct XentFn : public torch::autograd::Function<XentFn> {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, bool gelu) {
-    return LinearFn::apply(x, w, bias.has_value() ? *bias : Tensor(), gelu);
+    return LinearFn::apply(x, w, bias, gelu);      // an input without a tensor has to be a nullopt: apply asks every Tensor for its device
   });
   m.def("layer_norm", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormFn::apply(x, w, b, eps); });
   m.def("causal_attention", [](const Tensor& qkv, int64_t heads) { return AttentionFn::apply(qkv, heads); });
