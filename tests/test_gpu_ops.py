@@ -271,6 +271,30 @@ def test_stem_conv_implicit_gemm(N, H, W, cl):
     assert rel(conv.weight.grad, w.grad) < 4e-3, rel(conv.weight.grad, w.grad)
 
 
+@pytest.mark.parametrize("W", [8, 40, 256])
+def test_stem_conv_non_finite_pixels(W):
+    """A non-finite pixel reaches the windows that contain it and no other."""
+    import torch.nn.functional as F
+    from torchmpi_b200.ops import stem_conv, gemm
+    torch.manual_seed(W)
+    H = 21
+    conv = stem_conv.StemConv7x7(64).cuda().to(torch.bfloat16)
+    x = torch.randn(3, 3, H, W).to(torch.bfloat16)
+    x[0, 0, 0, 0], x[0, 1, 9, W - 2], x[0, 2, 20, 4], x[1, 1, 5, 2], x[1, 0, 12, 5] = (float(v) for v in ("inf", "-inf", "nan", "nan", "inf"))
+    xc = x.cuda().contiguous(memory_format=torch.channels_last)
+    assert stem_conv.direct(xc, conv.weight)
+    with torch.no_grad():
+        y = conv(xc).float().cpu()
+    gemm.check_status()
+    w = conv.weight.detach().double().cpu().reshape(64, 147)
+    ref = (w @ F.unfold(x.double(), 7, padding=3, stride=2)).reshape(y.shape)
+    assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+    assert torch.equal(y[ref.isinf()].double(), ref[ref.isinf()])
+    ok = ref.isfinite()
+    # 2^-9 for the rounding to bf16, 147 fp32 additions to sums below 4 (seven standard deviations)
+    assert ((y.double() - ref)[ok].abs() <= 2 ** -8 * ref[ok].abs() + 147 * 4 * 2 ** -23).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("N,C,H,W", [(1, 8, 1, 1), (2, 64, 2, 3), (5, 128, 29, 30), (3, 16, 64, 5)])
 def test_bn_pool_stage_edges_and_ties(dtype, N, C, H, W):

@@ -176,7 +176,38 @@ __device__ void fwd_mma(Shared* sh, unsigned char* rows, unsigned char* weights,
   }
 }
 
-__device__ void fwd_drain(Shared* sh, unsigned char* staging, const Params& p, const CUtensorMap* my, int quarter, int lane) {
+// The padded tap multiplies the pixel left of the window by a weight of zero, which is NaN in all channels when that pixel is
+// not finite.  A pixel whose first channel came out NaN is looked at again, and computed without that tap if it was the
+// reason: 147 x 64 multiply-adds on one thread, reached by non-finite images only.
+__device__ __noinline__ void redo_pixel(const __nv_bfloat16* img, int H, int W, const unsigned char* weights, unsigned char* out,
+                                        int swizzle, int oh, int ow) {
+  const int iw0 = 2 * ow - 3;
+  bool pad = false;
+  for (int kh = 0; kh < KROWS && iw0 > 0; ++kh) {
+    const int ih = 2 * oh - 3 + kh;
+    for (int c = 0; c < 3 && ih >= 0 && ih < H; ++c) pad |= !isfinite(__bfloat162float(img[((size_t)ih * W + iw0 - 1) * 3 + c]));
+  }
+  if (!pad) return;
+  const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(weights);
+#pragma unroll 1
+  for (int co = 0; co < COUT; ++co) {
+    float sum = 0.f;
+#pragma unroll 1
+    for (int kh = 0; kh < KROWS; ++kh) {
+      const int ih = 2 * oh - 3 + kh;
+      if (ih < 0 || ih >= H) continue;
+      for (int kw = 0; kw < 7; ++kw) {
+        if (iw0 + kw < 0 || iw0 + kw >= W) continue;
+        for (int c = 0; c < 3; ++c)
+          sum += __bfloat162float(img[((size_t)ih * W + iw0 + kw) * 3 + c]) *
+                 __bfloat162float(w[((kh * TAPS + (kw + 1) / 2) * COUT + co) * 8 + ((kw + 1) & 1) * 4 + c]);
+      }
+    }
+    *reinterpret_cast<__nv_bfloat16*>(out + (((co >> 3) ^ swizzle) << 4) + (co & 7) * 2) = __float2bfloat16(sum);
+  }
+}
+
+__device__ void fwd_drain(Shared* sh, unsigned char* staging, const unsigned char* weights, const Params& p, const CUtensorMap* my, int quarter, int lane) {
   const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
   int n, oh0, count = 0;
   for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
@@ -209,6 +240,8 @@ __device__ void fwd_drain(Shared* sh, unsigned char* staging, const Params& p, c
           }
           *reinterpret_cast<uint4*>(stg + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        if (isnan(__uint_as_float(r[0][0])) && quarter * 32 + lane < p.OW)
+          redo_pixel(p.x + (size_t)n * p.H * p.W * 3, p.H, p.W, weights, stg + lane * 128, lane & 7, oh0 + i, quarter * 32 + lane);
         sm100::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) sm100::tma_store_4d(my, stg, 0, quarter * 32, oh0 + i, n);      // pixels beyond the row are clipped
@@ -251,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_const
   } else if (warp >= 8) {
     load_rows(sh, rows, p, threadIdx.x - 256);
   } else if (warp >= 4) {
-    fwd_drain(sh, staging, p, &map_y, warp & 3, lane);
+    fwd_drain(sh, staging, weights, p, &map_y, warp & 3, lane);
   }
   teardown(sh, warp);
 }
