@@ -41,6 +41,7 @@
 #include <mutex>
 #include "sm100_ptx.cuh"
 #include "attn_util.cuh"
+#include "pdl.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
 
@@ -390,6 +391,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   if (threadIdx.x == 0) ((Shared*)((unsigned char*)sh0 + SMEM_SHARED))->tmem_base = sh0->tmem_base + TMEM_COLS;
   __syncthreads();
 
+  wait_previous();
   // the swizzled tiles need a 1024-byte aligned base
   const bool fits = (sm100::smem_u32(tiles) & 1023u) == 0;
   if (!fits) {
@@ -465,8 +467,7 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.items = B * H * p.q_blocks;
   // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
   const int grid = std::min(p.items, gemm_sm_count());
-  attn::attention_fwd_kernel<<<grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream>>>(mq, mk, mv, p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_overlapped(attn::attention_fwd_kernel, grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream, mq, mk, mv, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));
 }
 

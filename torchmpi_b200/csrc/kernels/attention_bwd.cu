@@ -39,6 +39,7 @@
 #include <mutex>
 #include "sm100_ptx.cuh"
 #include "attn_util.cuh"
+#include "pdl.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
 
@@ -452,6 +453,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __syncthreads();
   sm100::tc_fence_after();
 
+  wait_previous();
   const bool aligned = (sm100::smem_u32(smem_raw) & 1023u) == 0;     // the swizzled tiles need a 1024-byte aligned base
   if (!aligned) {
     if (threadIdx.x == 0) fail(sh, p, 18);
@@ -489,6 +491,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 __global__ void __launch_bounds__(256)
 attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, int64_t ld_o, int64_t ld_do,
                        float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int H) {
+  wait_previous(o, dout);
   const long long total = (long long)B * T * H;                  // (row, head) pairs; blockDim.x / 8 of them per block and step
   const int sub = threadIdx.x & 7;
   for (long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; idx < total;
@@ -521,6 +524,7 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
 // dq[r, c] = bf16(dq_acc[r, c]): the fp32 sums of the reductions rounded into the Q block of the packed gradient.
 __global__ void __launch_bounds__(256)
 attention_dq_round_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int64_t ld_dq, long long rows, int cols) {
+  wait_previous(acc);
   const int groups = cols / 8;
   const long long total = rows * groups;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
@@ -572,7 +576,9 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   cudaStream_t s = (cudaStream_t)stream;
   const long long rows_heads = (long long)B * T * H;
   const int dgrid = (int)std::min<long long>((rows_heads * 8 + 255) / 256, 148 * 8);
-  attnb::attention_delta_kernel<<<dgrid, 256, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, ld_o, ld_do, delta, dq_acc, B, T, H);
+  cudaError_t e = launch_overlapped(attnb::attention_delta_kernel, dgrid, 256, 0, s, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+                                    ld_o, ld_do, delta, dq_acc, B, T, H);
+  if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention backward launch: %s", cudaGetErrorString(e));
   CUtensorMap mq, mk, mv, mdo, mdq;
   int st;
   const uint64_t rows = (uint64_t)B * T, cols = (uint64_t)H * attnb::D;
@@ -592,14 +598,13 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.status = attnb_status_word();
   p.trace = g_attnb_trace;
   p.items = B * H * p.blocks;
-  attnb::attention_bwd_kernel<<<std::min(p.items, gemm_sm_count()), attnb::THREADS, smem, s>>>(mq, mk, mv, mdo, mdq, p);
-  if (dq) {
+  e = launch_overlapped(attnb::attention_bwd_kernel, std::min(p.items, gemm_sm_count()), attnb::THREADS, smem, s, mq, mk, mv, mdo, mdq, p);
+  if (dq && e == cudaSuccess) {
     if ((uintptr_t)dq & 15) return fail(TMPI_ERR_INVALID, "attention backward: dq must be 16-byte aligned");
     const long long groups = (long long)rows * (cols / 8);
     const int cgrid = (int)std::min<long long>((groups + 255) / 256, 148 * 8);
-    attnb::attention_dq_round_kernel<<<cgrid, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, ld_dkv, (long long)rows, (int)cols);
+    e = launch_overlapped(attnb::attention_dq_round_kernel, cgrid, 256, 0, s, dq_acc, (__nv_bfloat16*)dq, ld_dkv, (long long)rows, (int)cols);
   }
-  cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention backward launch: %s", cudaGetErrorString(e));
 }
 

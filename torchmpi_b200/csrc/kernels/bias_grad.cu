@@ -7,6 +7,7 @@
 // registers, blocks write partials and a second kernel adds them in block order (deterministic).
 // The GELU forward with the same approximation of the normal distribution lives here too.
 #include "gelu.cuh"
+#include "pdl.cuh"
 #include "vec.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
@@ -21,6 +22,7 @@ constexpr int kBgFinCols = 32, kBgFinGroups = 32;   // finalize: 32 columns x 32
 // y = gelu(z), one 16-byte pack per thread and step, four steps in flight.
 template <typename T, int V>
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const T* __restrict__ z, T* __restrict__ y, size_t npacks) {
+  wait_previous(z);
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   constexpr int U = 4;
@@ -60,8 +62,7 @@ static int gelu_fwd_t(const void* z, void* y, size_t n, cudaStream_t s) {
   const size_t npacks = n / V;
   if (!npacks) return TMPI_OK;
   const int blocks = (int)std::min<size_t>((npacks + 255) / 256, (size_t)148 * 8);
-  gelu_fwd_kernel<T, V><<<blocks, 256, 0, s>>>((const T*)z, (T*)y, npacks);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_overlapped(gelu_fwd_kernel<T, V>, blocks, 256, 0, s, (const T*)z, (T*)y, npacks);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "gelu_fwd launch: %s", cudaGetErrorString(e));
 }
 
@@ -70,6 +71,7 @@ template <typename T, int V, bool GELU>
 __global__ void __launch_bounds__(kBgThreads, 4)
 bias_grad_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __restrict__ dz, float* __restrict__ partial,
                  int rows, int C) {
+  wait_previous(dy, z);
   const int tx = threadIdx.x % kBgCols, ty = threadIdx.x / kBgCols;
   const int col = (blockIdx.x * kBgCols + tx) * V;
   float acc[V];
@@ -131,6 +133,7 @@ bias_grad_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __restric
 template <typename T>
 __global__ void __launch_bounds__(kBgFinCols * kBgFinGroups)
 bias_grad_finalize_kernel(const float* __restrict__ partial, int nblocks, int C, T* __restrict__ db) {
+  wait_previous(partial);
   const int cx = threadIdx.x % kBgFinCols, grp = threadIdx.x / kBgFinCols;
   const int c = blockIdx.x * kBgFinCols + cx;            // C is a multiple of 32
   const int per = (nblocks + kBgFinGroups - 1) / kBgFinGroups;
@@ -165,10 +168,12 @@ static int bias_grad_t(const void* dy, const void* z, void* dz, void* db, int ro
   const int per_sm = 4;                                  // resident blocks per SM
   const int rb = std::max(1, std::min((rows + 1) / 2, std::max(1, per_sm * 148 / slabs)));
   const dim3 grid(slabs, rb);
-  if (z) bias_grad_kernel<T, V, true><<<grid, kBgThreads, 0, s>>>((const T*)dy, (const T*)z, (T*)dz, (float*)scratch, rows, C);
-  else bias_grad_kernel<T, V, false><<<grid, kBgThreads, 0, s>>>((const T*)dy, nullptr, nullptr, (float*)scratch, rows, C);
-  bias_grad_finalize_kernel<T><<<C / kBgFinCols, kBgFinCols * kBgFinGroups, 0, s>>>((const float*)scratch, rb, C, (T*)db);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = z ? launch_overlapped(bias_grad_kernel<T, V, true>, grid, kBgThreads, 0, s, (const T*)dy, (const T*)z, (T*)dz,
+                                        (float*)scratch, rows, C)
+                    : launch_overlapped(bias_grad_kernel<T, V, false>, grid, kBgThreads, 0, s, (const T*)dy, (const T*)nullptr, (T*)nullptr,
+                                        (float*)scratch, rows, C);
+  if (e == cudaSuccess)
+    e = launch_overlapped(bias_grad_finalize_kernel<T>, C / kBgFinCols, kBgFinCols * kBgFinGroups, 0, s, (const float*)scratch, rb, C, (T*)db);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bias_grad launch: %s", cudaGetErrorString(e));
 }
 

@@ -2,6 +2,7 @@
 // two CTAs of a cluster (gemm_pair.cuh).  One cluster per TPC, persistent; tiles are visited in
 // bands of 8 tile-rows so that the clusters running at one time share B panels in L2.
 #include "gemm_pair.cuh"
+#include "pdl.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
 #include <algorithm>
@@ -39,6 +40,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = sm100::cluster_ctarank();
   setup(sh, warp, &map_a, &map_b, 4 * GROUPS);
+  wait_previous();
 
   const int total = p.tiles_m * p.tiles_n;
   const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
@@ -143,11 +145,13 @@ int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, in
   p.status = status_word;
   const int nclusters = std::min(p.tiles_m * p.tiles_n, clusters);
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see pdl.cuh
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(2 * nclusters); cfg.blockDim = dim3(gemm2::GROUP_THREADS);
-  cfg.dynamicSmemBytes = gemm2::SMEM_BYTES; cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = 1;
+  cfg.dynamicSmemBytes = gemm2::SMEM_BYTES; cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = 2;
   cudaError_t e = gelu_out ? cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<true>, ma, mb, mc, my, p)
                            : cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<false>, ma, mb, mc, my, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "pair gemm launch: %s", cudaGetErrorString(e));

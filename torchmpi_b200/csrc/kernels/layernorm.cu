@@ -7,6 +7,7 @@
 // per block and a second kernel adds the partials in block order (deterministic).  A framework
 // graph runs this as three kernels with three reads of dy and x (dx, then the two parameter
 // reductions).  The reference has no normalisation layer of its own (it trains Torch7 modules).
+#include "pdl.cuh"
 #include "vec.cuh"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
@@ -23,6 +24,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_fwd_kernel(const T* __restrict_
                                                             const T* __restrict__ beta, T* __restrict__ y,
                                                             float* __restrict__ mean, float* __restrict__ rstd, int rows, float eps) {
   constexpr int C = 32 * NP * V;
+  wait_previous(x, gamma, beta);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float g[NP][V], b[NP][V];
 #pragma unroll
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_bwd_kernel(const T* __restrict_
                                                             const float* __restrict__ rstd, T* __restrict__ dx,
                                                             float* __restrict__ partial, int rows) {
   constexpr int C = 32 * NP * V;
+  wait_previous(x, dy, gamma, mean, rstd);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float g[NP][V], db[NP][V], dg[NP][V];
 #pragma unroll
@@ -140,6 +143,7 @@ constexpr int kLnFinGroups = 32;
 template <typename T>
 __global__ void __launch_bounds__(32 * kLnFinGroups) ln_finalize_kernel(const float* __restrict__ partial, int nblocks, int C,
                                                                         T* __restrict__ dgamma, T* __restrict__ dbeta) {
+  wait_previous(partial);
   const int cx = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int o = blockIdx.x * 32 + cx;                       // (which, c); C is a multiple of 32
   const int which = o / C, c = o - which * C;
@@ -166,13 +170,13 @@ static cudaError_t ln_launch(bool fwd, const void* x, const void* a, const void*
   constexpr int V = 16 / sizeof(T);
   constexpr int C = 32 * NP * V;
   const int grid = fwd ? ln_grid(rows) : std::min(ln_grid(rows), kLnMaxGrid / 2);
-  if (fwd) {
-    ln_fwd_kernel<T, V, NP><<<grid, kLnThreads, 0, s>>>((const T*)x, (const T*)gamma, (const T*)beta, (T*)out, mean, rstd, rows, eps);
-  } else {
-    ln_bwd_kernel<T, V, NP><<<grid, kLnThreads, 0, s>>>((const T*)x, (const T*)a, (const T*)gamma, mean, rstd, (T*)out, partial, rows);
-    ln_finalize_kernel<T><<<2 * C / 32, 32 * kLnFinGroups, 0, s>>>(partial, grid, C, (T*)dgamma, (T*)dbeta);
-  }
-  return cudaGetLastError();
+  if (fwd)
+    return launch_overlapped(ln_fwd_kernel<T, V, NP>, grid, kLnThreads, 0, s, (const T*)x, (const T*)gamma, (const T*)beta, (T*)out, mean,
+                             rstd, rows, eps);
+  cudaError_t e = launch_overlapped(ln_bwd_kernel<T, V, NP>, grid, kLnThreads, 0, s, (const T*)x, (const T*)a, (const T*)gamma, mean, rstd,
+                                    (T*)out, partial, rows);
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(ln_finalize_kernel<T>, 2 * C / 32, 32 * kLnFinGroups, 0, s, partial, grid, C, (T*)dgamma, (T*)dbeta);
 }
 
 template <typename T>
