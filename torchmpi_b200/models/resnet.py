@@ -4,7 +4,7 @@ The reference ships no model beyond a logistic regressor
 (examples/mnist/mnist_allreduce.lua:31); this is the standard architecture
 (He et al. 2015, stride on the 3x3 convolution) written for channels_last bf16
 training.  With ``fused_bn=True`` batch-norm + ReLU (+ residual add) run as the fused kernels of
-``ops.bn_relu``, the max-pool as ``ops.pool`` and the stem convolution as im2col + tcgen05 GEMM
+``ops.bn_relu``, the max-pool as ``ops.pool`` and the stem convolution as an implicit tcgen05 GEMM
 (``ops.stem_conv``); the other convolutions run in cuDNN.
 """
 from __future__ import annotations
@@ -71,7 +71,7 @@ class ResNet(nn.Module):
         self.inplanes = width
         if fused_bn:
             from ..ops.stem_conv import StemConv7x7
-            self.conv1 = StemConv7x7(width)           # im2col + tensor-core GEMM; same parameter as the Conv2d
+            self.conv1 = StemConv7x7(width)           # tensor-core GEMM; same parameter as the Conv2d
         else:
             self.conv1 = nn.Conv2d(3, width, 7, stride=2, padding=3, bias=False)
         if fused_bn:
