@@ -281,3 +281,15 @@ def test_linear_without_bias_and_with_frozen_inputs(gelu, rows, n, bias, frozen)
             assert t[a].grad is None
         else:
             assert (t[a].grad.float() - r[a].grad).norm() <= 2 ** -7 * r[a].grad.norm(), a
+
+
+def test_refused_operands_of_linear_and_cross_entropy():
+    """Operands that do not fit each other and an empty batch raise before anything is launched."""
+    from torchmpi_b200.ops import gemm, xent
+    x = torch.zeros(16, 64, device="cuda", dtype=torch.bfloat16)
+    for w in (torch.zeros(32, 128, device="cuda"), torch.zeros(32, 56, device="cuda"), torch.zeros(32, 64), torch.zeros(32, device="cuda")):
+        for gelu in (False, True):
+            with pytest.raises(ValueError):
+                gemm.linear(x, w.to(torch.bfloat16), None, gelu=gelu)
+    with pytest.raises(ZeroDivisionError):
+        xent.cross_entropy(torch.zeros(0, 10, device="cuda"), torch.zeros(0, device="cuda", dtype=torch.int64))

@@ -119,6 +119,8 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias_, bool with_gelu) {
     const Tensor bias = bias_.has_value() ? *bias_ : Tensor();
     Tensor x2 = x.reshape({-1, x.size(-1)}), y, z;
+    if (!(w.dim() == 2 && w.is_cuda() && w.size(1) == x2.size(1)))
+      throw std::invalid_argument("matmul_nt expects bf16 CUDA matrices [M, K] and [N, K] with K a multiple of 8");
     if (with_gelu) std::tie(z, y) = matmul_nt_gelu(x2, w, bias);          // the pre-activation is needed by backward
     else y = matmul_nt(x2, w, bias);
     ctx->save_for_backward({x2, w, z});
@@ -207,6 +209,10 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
 struct XentFn : public torch::autograd::Function<XentFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& labels, const Tensor& scratch, bool unit_grad) {
     const int64_t rows = logits.size(0), cols = logits.size(1);
+    if (rows == 0) {                                            // the mean of no losses
+      PyErr_SetString(PyExc_ZeroDivisionError, "cross_entropy: no rows");
+      throw pybind11::error_already_set();
+    }
     // rows may sit in a wider buffer: the kernel takes the pitch, and the gradient keeps it
     const bool pitched = logits.stride(1) == 1 && logits.stride(0) >= cols && rows > 1;
     const Tensor x = pitched ? logits : logits.contiguous();
