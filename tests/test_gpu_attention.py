@@ -168,3 +168,24 @@ def test_attention_several_items_per_team_and_growing_maxima(B, T, H):
     assert rel(out, ref.detach()) < 6e-3, rel(out, ref.detach())
     for name, sl in (("dq", slice(0, C)), ("dk", slice(C, 2 * C)), ("dv", slice(2 * C, 3 * C))):
         assert rel(dqkv[:, :, sl], leaf.grad[:, :, sl]) < 1.5e-2, (name, rel(dqkv[:, :, sl], leaf.grad[:, :, sl]))
+
+
+@pytest.mark.parametrize("t0", [1, 6, 39, 70, 135, 200])
+def test_attention_later_tokens_leave_earlier_rows_alone(t0):
+    """Values of 1e38 behind the mask change no bit of the rows in front of them, and visible values of zero give zero:
+    a masked key has a probability of exactly 0."""
+    from torchmpi_b200.ops import attention
+    torch.manual_seed(t0)
+    B, T, H = 2, 256, 3
+    C = H * 64
+    qkv = torch.randn(B, T, 3 * C, device="cuda").to(torch.bfloat16)
+    out, lse = attention.attention_forward(qkv, H)
+    big = qkv.clone()
+    big[:, t0:, 2 * C:] = 1e38
+    out2, lse2 = attention.attention_forward(big, H)
+    big[:, :t0, 2 * C:] = 0.0
+    out3, _ = attention.attention_forward(big, H)
+    torch.cuda.synchronize()
+    attention.check_status()
+    assert torch.equal(out2[:, :t0], out[:, :t0]) and torch.equal(lse2, lse)
+    assert torch.count_nonzero(out3[:, :t0]) == 0

@@ -203,17 +203,17 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
 
 // Scores s[0, 32) of one row (a chunk of 32 keys) -> sixteen packed bf16 pairs of exp2(s * c2 + nmc), added to the row
 // sums.  A quarter of the exponentials run on the FMA pipe, the rest on the special-function unit; a masked score (-inf)
-// gives 0 there and 2^-120 here, which no sum that holds the row's maximum (1) can tell from 0.
+// gives exactly 0 on both.
 __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint32_t (&w)[16], unsigned long long c2x2,
                                           unsigned long long nmc2, unsigned long long& sum2) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     float a0, a1;
     unpack2(fma2(pack2(s[2 * i], s[2 * i + 1]), c2x2, nmc2), a0, a1);
-    const bool fma_pipe = (i & 3) == 3;
-    const float e0 = fma_pipe ? ex2_fma(a0) : ex2(a0);
-    const float e1 = fma_pipe ? ex2_fma(a1) : ex2(a1);
-    sum2 = add2(sum2, pack2(__float_as_uint(e0), __float_as_uint(e1)));
+    const unsigned long long e = (i & 3) == 3 ? ex2_fma2(a0, a1) : pack2(__float_as_uint(ex2(a0)), __float_as_uint(ex2(a1)));
+    sum2 = add2(sum2, e);
+    float e0, e1;
+    unpack2(e, e0, e1);
     w[i] = pack_bf16(__float_as_uint(e0), __float_as_uint(e1));
   }
 }

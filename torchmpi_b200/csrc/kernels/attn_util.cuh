@@ -19,19 +19,6 @@ __device__ __forceinline__ float rcp(float x) {
   return y;
 }
 
-// 2^a for a <= 0 on the FMA pipe (the special-function unit, 4 lanes per scheduler, is the bottleneck of the softmax:
-// a share of the exponentials goes here instead): round a to an integer n with the 1.5 * 2^23 trick, a cubic for
-// 2^(a - n) on [-0.5, 0.5] (relative error 7.5e-5, far below the bf16 rounding of P), and n added into the exponent.
-__device__ __forceinline__ float ex2_fma(float a) {
-  a = fmaxf(a, -120.f);
-  const float t = a + 12582912.f;
-  const float f = a - (t - 12582912.f);
-  float q = fmaf(0.05517157167196274f, f, 0.2426111102104187f);
-  q = fmaf(q, f, 0.6932610273361206f);
-  q = fmaf(q, f, 0.9999280571937561f);
-  return __uint_as_float(__float_as_uint(q) + (__float_as_uint(t) << 23));
-}
-
 // two fp32 values as packed bf16
 __device__ __forceinline__ uint32_t pack_bf16(uint32_t lo, uint32_t hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
@@ -70,6 +57,27 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
   const unsigned long long m1 = pack2(0xbf800000u, 0xbf800000u);
   return fma2(b, m1, a);                                   // a - b, rounded once
+}
+
+// 2^a, 2^b for a, b <= 0 on the FMA pipe (the special-function unit, 4 lanes per scheduler, is the bottleneck of the softmax:
+// a share of the exponentials goes here instead): round to an integer n with the 1.5 * 2^23 trick, a cubic for
+// 2^(a - n) on [-0.5, 0.5] (relative error 7.5e-5, far below the bf16 rounding of P), and times 2^n.  Like ex2 it flushes
+// subnormals: the last product does, so that an argument of -inf (a masked score, clamped to -126) gives exactly 0.
+__device__ __forceinline__ unsigned long long ex2_fma2(float a, float b) {
+  const float x[2] = {fmaxf(a, -126.f), fmaxf(b, -126.f)};
+  uint32_t q[2], p[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float t = x[i] + 12582912.f;
+    const float f = x[i] - (t - 12582912.f);
+    float c = fmaf(0.05517157167196274f, f, 0.2426111102104187f);
+    c = fmaf(c, f, 0.6932610273361206f);
+    q[i] = __float_as_uint(fmaf(c, f, 0.9999280571937561f));
+    p[i] = (__float_as_uint(t) << 23) + 0x3f800000u;
+  }
+  unsigned long long r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(q[0], q[1])), "l"(pack2(p[0], p[1])));
+  return r;
 }
 
 }  // namespace attn_util
