@@ -189,3 +189,29 @@ def test_attention_later_tokens_leave_earlier_rows_alone(t0):
     attention.check_status()
     assert torch.equal(out2[:, :t0], out[:, :t0]) and torch.equal(lse2, lse)
     assert torch.count_nonzero(out3[:, :t0]) == 0
+
+
+@pytest.mark.parametrize("key", [0, 5, 6, 7, 38, 63, 100, 134, 191])
+def test_attention_non_finite_scores(key):
+    """A score that is NaN or overflows to infinity makes its row NaN wherever its key lies; rows before the key and the
+    other head keep their bits."""
+    from torchmpi_b200.ops import attention
+    torch.manual_seed(key)
+    T, H, row = 256, 2, 250
+    C = H * 64
+    qkv = torch.randn(1, T, 3 * C, device="cuda").to(torch.bfloat16)
+    out, lse = attention.attention_forward(qkv, H)
+    bad = qkv.clone()
+    bad[0, key, C + 3] = float("nan")
+    out_nan, lse_nan = attention.attention_forward(bad, H)
+    huge = qkv.clone()
+    huge[0, row, :64] = 1e30
+    huge[0, key, C:C + 64] = 1e30
+    out_inf, lse_inf = attention.attention_forward(huge, H)
+    torch.cuda.synchronize()
+    attention.check_status()
+    for o, l in ((out_nan, lse_nan), (out_inf, lse_inf)):
+        assert torch.equal(o[:, :key], out[:, :key]) and torch.equal(o[:, :, 64:], out[:, :, 64:])
+        assert torch.equal(l[:, 0, :key], lse[:, 0, :key]) and torch.equal(l[:, 1], lse[:, 1])
+    assert out_nan[0, key:, :64].isnan().all() and lse_nan[0, 0, key:].isnan().all()
+    assert out_inf[0, row, :64].isnan().all() and lse_inf[0, 0, row].isnan()

@@ -269,23 +269,24 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;      // four chains
 #pragma unroll
       for (int i = 0; i < 32; i += 4) {
-        mx0 = max3(mx0, __uint_as_float(s[0][i]), __uint_as_float(s[0][i + 1]));
-        mx1 = max3(mx1, __uint_as_float(s[0][i + 2]), __uint_as_float(s[0][i + 3]));
-        mx2 = max3(mx2, __uint_as_float(s[1][i]), __uint_as_float(s[1][i + 1]));
-        mx3 = max3(mx3, __uint_as_float(s[1][i + 2]), __uint_as_float(s[1][i + 3]));
+        mx0 = max3_nan(mx0, __uint_as_float(s[0][i]), __uint_as_float(s[0][i + 1]));
+        mx1 = max3_nan(mx1, __uint_as_float(s[0][i + 2]), __uint_as_float(s[0][i + 3]));
+        mx2 = max3_nan(mx2, __uint_as_float(s[1][i]), __uint_as_float(s[1][i + 1]));
+        mx3 = max3_nan(mx3, __uint_as_float(s[1][i + 2]), __uint_as_float(s[1][i + 3]));
       }
-      float mx = fmaxf(max3(mx0, mx1, mx2), mx3), mx_other;
+      float mx = max_nan(max3_nan(mx0, mx1, mx2), mx3), mx_other;
       if (!exchange(mx, &mx_other)) return;
-      mx = fmaxf(mx, mx_other);
+      mx = max_nan(mx, mx_other);
       if (tracer) stamp(p, r, j, 2);
       // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
-      const float next = fmaxf(m, mx);
+      const float next = max_nan(m, mx);
       const bool grew = j > 0 && __any_sync(~0u, next > m);
       const float alpha = ex2((m - next) * c2);
       const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
       m = next;
       if (grew) { sum2[0] = mul2(sum2[0], al2); sum2[1] = mul2(sum2[1], al2); }
-      const float nmc = -m * c2;
+      // NaN where the maximum is NaN or infinite, and with it every P of the row: the polynomial's clamp alone would drop a NaN
+      const float nmc = fmaf(m, 0.f, -m * c2);
       const unsigned long long nmc2 = pack2(__float_as_uint(nmc), __float_as_uint(nmc));
 #pragma unroll
       for (int c = 0; c < 2; ++c) {

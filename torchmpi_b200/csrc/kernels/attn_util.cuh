@@ -25,9 +25,15 @@ __device__ __forceinline__ uint32_t pack_bf16(uint32_t lo, uint32_t hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-__device__ __forceinline__ float max3(float a, float b, float c) {
+// maxima that are NaN when an operand is
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
   float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
 // two fp32 lanes per instruction
