@@ -421,3 +421,35 @@ def test_native_autograd_functions_save_through_hooks():
             fn(b).float().square().sum().backward()
         assert seen
         assert ((a.grad.float() - b.grad.float()).norm() / a.grad.float().norm()).item() < 1e-3
+
+
+@pytest.mark.parametrize("dtype,C,H,W", [(torch.bfloat16, 64, 9, 219), (torch.bfloat16, 64, 8, 224), (torch.bfloat16, 64, 7, 256),
+                                         (torch.float32, 64, 9, 120), (torch.float32, 64, 6, 130), (torch.float16, 256, 5, 96)])
+@pytest.mark.parametrize("fused_bwd", [1, 0])
+def test_bn_pool_stage_long_rows(dtype, C, H, W, fused_bwd):
+    """Rows that would not fit in an SM's shared memory: forward and both backward routes against separate ops."""
+    from torchmpi_b200 import config
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLUMaxPool
+    torch.manual_seed(W)
+    x = torch.randn(2, C, H, W, device="cuda").to(dtype).contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    m = FusedBatchNormReLUMaxPool(C).cuda()
+    before = config.get("bn_pool_fused_bwd")
+    config.set("bn_pool_fused_bwd", fused_bwd)
+    try:
+        y = m(x)
+        dy = torch.randn_like(y)
+        y.backward(dy)
+    finally:
+        config.set("bn_pool_fused_bwd", before)
+    xr = x.detach().float().requires_grad_(True)
+    bn = torch.nn.BatchNorm2d(C).cuda()
+    z = torch.relu(bn(xr))
+    z = z + (z.to(dtype).float() - z).detach()              # the stage pools the rounded activation
+    yr = torch.nn.functional.max_pool2d(z, 3, 2, 1)
+    yr.backward(dy.float())
+    # one rounding of the result (2^-8 for bf16, 2^-11 for fp16), and a window whose two largest values round alike now and then
+    # sends its gradient to the other one
+    tol = {torch.bfloat16: 2e-2, torch.float16: 4e-3, torch.float32: 1e-4}[dtype]
+    assert torch.allclose(y.float(), yr, rtol=tol, atol=tol)
+    rel = lambda a, b: ((a.float() - b).norm() / b.norm()).item()
+    assert rel(x.grad, xr.grad) < tol and rel(m.weight.grad, bn.weight.grad) < tol and rel(m.bias.grad, bn.bias.grad) < tol

@@ -719,12 +719,14 @@ __global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_apply_kernel(
   });
 }
 
-// limits under which the two stages are offered (rows that an earlier shared-memory version of them could hold)
-template <typename T> static size_t bn_pool_fwd_smem(const BpDims& d) { return (size_t)3 * (d.W + 2) * d.C * sizeof(T); }
-template <typename T> static size_t bn_pool_bwd_smem(const BpDims& d) {
-  return (size_t)2 * (d.OW + 1) * d.C * (sizeof(T) + 1) + (size_t)2 * d.W * d.C * sizeof(T);
+// What both directions take, checked before anything is launched: the kernels stage nothing, so a row of any length that an
+// int can index.
+static int bn_pool_check(int64_t rows, const BpDims& d, int V) {
+  int st = bn_check(rows, d.C, V);
+  if (st) return st;
+  if ((int64_t)(d.W + 1) * d.C > 0x7fffffffLL) return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: rows of %d x %d are too long", d.W, d.C);
+  return TMPI_OK;
 }
-constexpr size_t kBpMaxSmem = 96 * 1024;
 
 template <typename T>
 static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, const float* beta, float* rmean, float* rvar,
@@ -732,9 +734,9 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, 
                          void* scratch, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   const int64_t rows = (int64_t)N * H * W;
-  int st = bn_check(rows, C, V);
-  if (st) return st;
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
+  int st = bn_pool_check(rows, d, V);
+  if (st) return st;
   if (training) {
     size_t nvec = (size_t)rows * (C / V);
     int grid = bn_grid(nvec);
@@ -744,8 +746,6 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, 
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
                                                            rows > 1 ? m / (m - 1.f) : 1.f, eps, momentum, smean, sinv, rmean, rvar);
   }
-  const size_t smem = bn_pool_fwd_smem<T>(d);
-  if (smem > kBpMaxSmem) return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: rows of %d x %d are too long", W, C);
   const BpWalk walk = bp_walk<V>(d);
   bn_pool_fwd_kernel<T, V><<<(unsigned)((walk.items + kBpThreads - 1) / kBpThreads), kBpThreads, 0, s>>>(
       (const T*)x, (T*)y, (unsigned char*)idx, gamma, beta, smean, sinv, d, walk);
@@ -774,10 +774,9 @@ static int bn_pool_bwd_t(const void* x, const void* dy, const void* idx, void* d
                          void* scratch, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   const int64_t rows = (int64_t)N * H * W;
-  int st = bn_check(rows, C, V);
-  if (st) return st;
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
-  if (bn_pool_bwd_smem<T>(d) > kBpMaxSmem) return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: rows of %d x %d are too long", W, C);
+  int st = bn_pool_check(rows, d, V);
+  if (st) return st;
   // 16-bit types: packs of four channels where their groups divide the block (up to 1024 channels).  They halve the
   // per-channel state, so that three blocks fit on an SM instead of two (256 x 112 x 112 x 64: statistics 150 -> 137 us, apply 254 -> 179).
   if constexpr (sizeof(T) == 2) {
