@@ -453,3 +453,55 @@ def test_bn_pool_stage_long_rows(dtype, C, H, W, fused_bwd):
     assert torch.allclose(y.float(), yr, rtol=tol, atol=tol)
     rel = lambda a, b: ((a.float() - b).norm() / b.norm()).item()
     assert rel(x.grad, xr.grad) < tol and rel(m.weight.grad, bn.weight.grad) < tol and rel(m.bias.grad, bn.bias.grad) < tol
+
+
+def test_cross_entropy_on_two_streams_at_once():
+    """Losses of equal row counts that run at the same time on two streams keep their own arrival counters and row losses."""
+    from torchmpi_b200 import _native
+    from torchmpi_b200.ops import xent
+    torch.manual_seed(3)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for rows, cols in ((8192, 1000), (600, 20000), (96, 10)):
+        x = [torch.randn(rows, cols, device="cuda") for _ in streams]
+        labels = [torch.randint(0, cols, (rows,), device="cuda") for _ in streams]
+        want = [xent.cross_entropy(a, b) for a, b in zip(x, labels)]
+        torch.cuda.synchronize()
+        got = [[], []]
+        for _ in range(20):
+            for k, s in enumerate(streams):
+                with torch.cuda.stream(s):
+                    got[k].append(xent.cross_entropy(x[k], labels[k]))
+        torch.cuda.synchronize()
+        for k in (0, 1):
+            assert all(torch.equal(v, want[k]) for v in got[k]), (rows, cols, k)
+    buffers = set()
+    for s in streams:
+        with torch.cuda.stream(s):
+            buffers.add(_native.ext().cross_entropy_scratch(x[0], 96).data_ptr())
+    assert len(buffers) == 2
+
+
+def test_cross_entropy_first_called_under_capture():
+    """A captured loss clears its own counter: right on every replay, and eager calls around it are right before the first."""
+    from torchmpi_b200.ops import xent
+    torch.manual_seed(4)
+    x = torch.randn(77, 300, device="cuda")
+    labels = torch.randint(0, 300, (77,), device="cuda")
+    want = xent.cross_entropy(x, labels)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        captured = xent.cross_entropy(x, labels)
+    with torch.cuda.stream(side):
+        eager = xent.cross_entropy(x, labels)
+    torch.cuda.synchronize()
+    assert torch.equal(eager, want)
+    for _ in range(3):
+        captured.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(captured, want)
+    torch.cuda.synchronize()
+    assert torch.equal(xent.cross_entropy(x, labels), want)

@@ -4,13 +4,16 @@
 // one layer took 100 - 160 us of Python (autograd.Function both ways, ctypes argument conversion, tensor bookkeeping)
 // around 10 - 50 us of kernels, and a transformer block about as long as its kernels.
 //
-// Scratch memory is allocated per call from PyTorch's caching allocator on the calling stream: nothing is shared between
-// threads or streams.  A non-zero status is raised through torchmpi_b200._lib.check, so callers see the usual exceptions.
+// Scratch memory is allocated per call from PyTorch's caching allocator on the calling stream; the one buffer that is kept
+// (cross-entropy, see xent_scratch) belongs to one stream.  A non-zero status is raised through torchmpi_b200._lib.check, so callers see the usual exceptions.
 // The reference has no counterpart (its layers are Torch7's).
 #include <torch/extension.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <atomic>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include "tmpi_c_api.h"
 
 namespace {
@@ -205,9 +208,38 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
 };
 
 // ---------------------------------------------------------------- cross-entropy
+// The arrival counter of the kernel's blocks (zero before and after every call) and the row losses.  Two calls may share a
+// buffer only if one ends before the other starts, so there is one per stream, grown to the next power of two.  A call that
+// is being captured gets its own, cleared inside the graph: the graph may be replayed on any stream, and has not run when the
+// next eager call comes.  So does a call of very many rows, where the clearing costs nothing beside the pass and the buffer
+// would be large to keep.  Buffers go back to the allocator, which hands them out on the stream they were used on.
+Tensor xent_scratch(const Tensor& x, int64_t rows) {
+  constexpr size_t KEEP_BYTES = size_t(1) << 20, KEEP_STREAMS = 64;
+  static std::mutex lock;
+  static auto& kept = *new std::map<std::pair<int, void*>, Tensor>();      // outlives the CUDA context: never destroyed
+  size_t need = tmpi_xent_scratch_bytes((int)rows);
+  const auto bytes = x.options().dtype(at::kByte);
+  if (need > KEEP_BYTES || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    return at::zeros({(int64_t)need}, bytes);
+  const std::pair<int, void*> key(x.get_device(), stream());
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    const auto found = kept.find(key);
+    if (found != kept.end() && (size_t)found->second.numel() >= need) return found->second;
+  }
+  size_t size = 4096;
+  while (size < need) size *= 2;
+  const Tensor fresh = at::zeros({(int64_t)size}, bytes);
+  std::map<std::pair<int, void*>, Tensor> old;                             // released outside the lock
+  std::lock_guard<std::mutex> hold(lock);
+  if (kept.size() >= KEEP_STREAMS) old.swap(kept);
+  kept[key] = fresh;
+  return fresh;
+}
+
 // The gradient is computed with the loss and scaled in place by the incoming gradient, so backward runs once.
 struct XentFn : public torch::autograd::Function<XentFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& labels, const Tensor& scratch, bool unit_grad) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logits, const Tensor& labels, bool unit_grad) {
     const int64_t rows = logits.size(0), cols = logits.size(1);
     if (rows == 0) {                                            // the mean of no losses
       PyErr_SetString(PyExc_ZeroDivisionError, "cross_entropy: no rows");
@@ -217,6 +249,7 @@ struct XentFn : public torch::autograd::Function<XentFn> {
     const bool pitched = logits.stride(1) == 1 && logits.stride(0) >= cols && rows > 1;
     const Tensor x = pitched ? logits : logits.contiguous();
     const int64_t ld = pitched ? logits.stride(0) : cols;
+    const Tensor scratch = xent_scratch(x, rows);
     Tensor buf = at::empty({rows, ld}, x.options()), loss = at::empty({}, x.options().dtype(at::kFloat));
     check(tmpi_xent_mean_fwd_bwd_ld(x.data_ptr(), dtype_code(x.scalar_type()), labels.data_ptr<int64_t>(), (int)rows, (int)cols, (int)ld,
                                     loss.data_ptr<float>(), buf.data_ptr(), (float)(1.0 / (double)rows), scratch.data_ptr(), stream()));
@@ -232,7 +265,7 @@ struct XentFn : public torch::autograd::Function<XentFn> {
     Tensor buf = kept.toTensor();
     kept = c10::IValue();
     if (!ctx->saved_data["unit"].toBool()) buf.mul_(grads[0].to(buf.scalar_type()));
-    return {buf.narrow(1, 0, ctx->saved_data["cols"].toInt()), Tensor(), Tensor(), Tensor()};
+    return {buf.narrow(1, 0, ctx->saved_data["cols"].toInt()), Tensor(), Tensor()};
   }
 };
 
@@ -244,8 +277,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("layer_norm", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormFn::apply(x, w, b, eps); });
   m.def("causal_attention", [](const Tensor& qkv, int64_t heads) { return AttentionFn::apply(qkv, heads); });
-  m.def("cross_entropy", [](const Tensor& logits, const Tensor& labels, const Tensor& scratch, bool unit_grad) {
-    return XentFn::apply(logits, labels, scratch, unit_grad);
+  m.def("cross_entropy", [](const Tensor& logits, const Tensor& labels, bool unit_grad) {
+    return XentFn::apply(logits, labels, unit_grad);
   });
+  m.def("cross_entropy_scratch", xent_scratch);
   m.def("launches", [](int what) { return g_launches[what].load(std::memory_order_relaxed); });
 }

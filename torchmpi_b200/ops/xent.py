@@ -10,22 +10,13 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from .._lib import lib, has_symbol
-
-_scratch = {}
+from .._lib import has_symbol
 
 
 def __getattr__(name: str):
     if name == "launch_count":               # kernels launched by this module (read by the benchmark)
         return _native.launches(_native.XENT)
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
-
-
-def _scratch_for(dev: torch.device, rows: int) -> torch.Tensor:
-    key = (dev.index, rows)
-    if key not in _scratch:
-        _scratch[key] = torch.zeros(lib.tmpi_xent_scratch_bytes(rows), dtype=torch.uint8, device=dev)
-    return _scratch[key]
 
 
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, unit_grad: bool = False) -> torch.Tensor:
@@ -37,7 +28,7 @@ def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, unit_grad: bool = 
             raise RuntimeError("torchmpi_b200: native kernel 'tmpi_xent_mean_fwd_bwd_ld' is missing")
         if logits.dim() != 2 or labels.dtype != torch.int64:
             raise ValueError("cross_entropy expects [rows, classes] logits and int64 labels")
-        return _native.ext().cross_entropy(logits, labels.contiguous(), _scratch_for(logits.device, logits.shape[0]), unit_grad)
+        return _native.ext().cross_entropy(logits, labels.contiguous(), unit_grad)
     return torch.nn.functional.cross_entropy(logits.float(), labels)
 
 
