@@ -340,7 +340,7 @@ def test_bn_pool_stage_edges_and_ties(dtype, N, C, H, W):
                                              (3, 1025, 0), (700, 5003, 5008), (2, 60001, 0)])
 def test_cross_entropy_row_lengths(rows, cols, pitch, dtype):
     """A warp per row, a block per row in shared memory (misaligned rows, a pitch) and the fallback for rows that do not fit
-    there: loss and gradient against fp64, labels outside the row included, padding columns cleared."""
+    there: loss and gradient against fp64, padding columns left out."""
     from torchmpi_b200.ops import xent
     torch.manual_seed(rows + cols)
     buf = torch.randn(rows, pitch or cols, device="cuda").mul_(3.0).to(dtype)
@@ -379,7 +379,7 @@ def test_cross_entropy_infinities_and_bad_labels():
         ref = x.clone().requires_grad_(True)
         torch.nn.functional.cross_entropy(ref, labels).backward()
         assert torch.isnan(loss)
-        for r in (0, 1, 3, 4, 5) if cols <= 1024 else (0, 1, 4, 5):     # the long-row kernel forms max * log2(e): NaN at the lowest value
+        for r in (0, 1, 3, 4, 5):
             assert torch.allclose(xg.grad[r], ref.grad[r], rtol=1e-5, atol=1e-8), (cols, r)
         assert torch.isnan(xg.grad[2]).all()
 
@@ -505,3 +505,27 @@ def test_cross_entropy_first_called_under_capture():
         assert torch.equal(captured, want)
     torch.cuda.synchronize()
     assert torch.equal(xent.cross_entropy(x, labels), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [40, 3000, 60001])
+def test_cross_entropy_rows_at_the_lowest_value(cols, dtype):
+    """A row filled with the type's lowest finite value is uniform, and so are two such logits beside -inf: the largest logit
+    times log2(e) overflows there and must not be formed."""
+    from torchmpi_b200.ops import xent
+    lowest = torch.finfo(dtype).min
+    x = torch.full((3, cols), lowest, device="cuda", dtype=dtype)
+    x[1, 2:] = float("-inf")
+    x[2] = -lowest                                         # the largest value
+    labels = torch.tensor([1, 0, cols - 1], device="cuda")
+    x.requires_grad_(True)
+    loss = xent.cross_entropy(x, labels)
+    loss.backward()
+    # logsumexp - x[label]: log(n) is lost beside 3e38 in 32 bits, and the loss is that of a uniform row without the cancellation
+    p = torch.zeros(3, cols, dtype=torch.double, device="cuda")
+    p[0], p[1, :2], p[2] = 1.0 / cols, 0.5, 1.0 / cols
+    p[torch.arange(3), labels] -= 1.0
+    unit = {torch.float32: 2e-6, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7.5}[dtype]
+    floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / 3
+    assert bool(((x.grad.double() - p / 3).abs() <= unit * p.abs() / 3 + floor).all())
+    assert torch.isfinite(loss)

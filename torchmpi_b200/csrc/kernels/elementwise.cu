@@ -303,12 +303,14 @@ __global__ void __launch_bounds__(THREADS) xent_row_smem_kernel(
   }
   __syncthreads();
   m = s_bcast;
-  const float mL = m * kLog2e;
+  // exponents as one multiply-add per logit.  From |m| = 2.3e38 on (a row at the type's lowest value) m * log2(e) overflows;
+  // such logits are equal or at least 2^103 apart, so the plain difference has the same exponential: 1 or 0
+  const float scale = fabsf(m * kLog2e) < INFINITY ? kLog2e : 1.f, mL = m * scale;
 
   // pass 2: exponentials, kept in shared memory in place of the logits, and their sum
   float sum0 = 0.f, sum1 = 0.f;
   auto scalar_exp = [&](int c) {
-    float e = ex2_approx(fmaf((float)to_acc<T>(srow[c]), kLog2e, -mL));
+    float e = ex2_approx(fmaf((float)to_acc<T>(srow[c]), scale, -mL));
     sum0 += e;
     reinterpret_cast<E*>(srow)[c] = from_acc<E>((typename AccOf<E>::type)e);
   };
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(THREADS) xent_row_smem_kernel(
     float f[V];
     RP::unpack(sx[i], f);
 #pragma unroll
-    for (int j = 0; j < V; ++j) f[j] = ex2_approx(fmaf(f[j], kLog2e, -mL));
+    for (int j = 0; j < V; ++j) f[j] = ex2_approx(fmaf(f[j], scale, -mL));
 #pragma unroll
     for (int j = 0; j < V; j += 2) { sum0 += f[j]; sum1 += f[j + 1]; }
     sx[i] = RP::pack_e(f);
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(THREADS) xent_row_smem_kernel(
     }
     __syncthreads();                                  // the label's entry is overwritten after every other store
     if (tid == 0 && label >= 0 && label < cols)
-      d[label] = from_acc<T>((typename AccOf<T>::type)((ex2_approx(fmaf(xl, kLog2e, -mL)) * inv - 1.f) * gscale));
+      d[label] = from_acc<T>((typename AccOf<T>::type)((ex2_approx(fmaf(xl, scale, -mL)) * inv - 1.f) * gscale));
   }
   if (tid == 0) {
     row_loss[r] = __logf(sum) + m - xl;
