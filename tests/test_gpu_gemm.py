@@ -293,3 +293,42 @@ def test_refused_operands_of_linear_and_cross_entropy():
                 gemm.linear(x, w.to(torch.bfloat16), None, gelu=gelu)
     with pytest.raises(ZeroDivisionError):
         xent.cross_entropy(torch.zeros(0, 10, device="cuda"), torch.zeros(0, device="cuda", dtype=torch.int64))
+
+
+def test_first_cuda_call_of_a_thread_encodes_a_tensor_map():
+    """A thread without a current context (the autograd thread of a process whose backward begins here) may call a kernel
+    that takes tensor maps before anything else has made the context current."""
+    import threading
+    from torchmpi_b200.ops import attention, conv, gemm, stem_conv
+    from torchmpi_b200._lib import lib, check, stream_ptr
+    a = torch.randn(256, 256, device="cuda").to(torch.bfloat16)
+    want, out = gemm.matmul_nt(a, a), torch.empty(256, 256, device="cuda", dtype=torch.bfloat16)
+    small, out_small = gemm.matmul_nt(a[:128], a), torch.empty(128, 256, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(2, 64, 8, 8, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    w = torch.randn(64, 64, 1, 1, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    y = torch.nn.functional.conv2d(x, w)
+    stem = stem_conv.StemConv7x7(64).cuda().to(torch.bfloat16)
+    img = torch.randn(1, 3, 16, 16, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    z = stem(img).detach()
+    qkv = torch.randn(1, 128, 192, device="cuda").to(torch.bfloat16)
+    o, _ = attention.attention_forward(qkv, 1)
+    torch.cuda.synchronize()
+    calls = {"pair": lambda: gemm.matmul_nt(a, a, out=out), "single": lambda: gemm.matmul_nt(a[:128], a, out=out_small),
+             "conv": lambda: got.update(conv=conv.conv2d(x, w)), "stem": lambda: got.update(stem=stem(img).detach()),
+             "attention": lambda: got.update(attention=attention.attention_forward(qkv, 1)[0])}
+    got, errors = {}, {}
+
+    def run(name, fn):
+        try:
+            with torch.no_grad():
+                fn()
+        except Exception as e:
+            errors[name] = repr(e)
+    for name, fn in calls.items():
+        t = threading.Thread(target=run, args=(name, fn))
+        t.start()
+        t.join()
+    assert not errors, errors
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and torch.equal(out_small, small) and torch.equal(got["stem"], z) and torch.equal(got["attention"], o)
+    assert ((got["conv"].float() - y.float()).norm() / y.float().norm()).item() < 1e-2

@@ -7,6 +7,7 @@
 // so that the CTAs running at one time share B panels in L2.  The reference has no GEMM
 // (its model-parallel example calls Torch's Linear, examples/mnist/mnist_modelparallel.lua:30-60).
 #include "gemm_core.cuh"
+#include "tmap_encode.h"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
 #include <cstring>
@@ -90,8 +91,10 @@ static int make_tmap_2d(CUtensorMap* map, CUtensorMapDataType type, int bytes, c
   cuuint64_t strides[1] = {ld * bytes};
   cuuint32_t box[2] = {(cuuint32_t)(128 / bytes), box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_in_context([&] {
+    return fn(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) return fail(TMPI_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", (int)r);
   return TMPI_OK;
 }
@@ -112,8 +115,10 @@ int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)
   cuuint64_t strides[3] = {dims[0] * 2, dims[0] * dims[1] * 2, dims[0] * dims[1] * dims[2] * 2};
   cuuint32_t b[4] = {box[0], box[1], box[2], box[3]};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), d, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = encode_in_context([&] {
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), d, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
   if (r != CUDA_SUCCESS) return fail(TMPI_ERR_CUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", (int)r);
   return TMPI_OK;
 }
