@@ -529,3 +529,35 @@ def test_cross_entropy_rows_at_the_lowest_value(cols, dtype):
     floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / 3
     assert bool(((x.grad.double() - p / 3).abs() <= unit * p.abs() / 3 + floor).all())
     assert torch.isfinite(loss)
+
+
+@pytest.mark.parametrize("H,W", [(21, 8), (24, 40), (22, 40), (21, 104), (50, 200), (23, 256), (5, 24), (2, 16)])
+def test_stem_weight_gradient_non_finite_pixels(H, W):
+    """A non-finite pixel reaches the taps that multiply it by an output gradient and no other: output widths that are not a
+    multiple of 16 and odd output heights, where the products run over padding."""
+    import torch.nn.functional as F
+    from torchmpi_b200.ops import stem_conv, gemm
+    torch.manual_seed(H * W)
+    conv = stem_conv.StemConv7x7(64).cuda().to(torch.bfloat16)
+    clean = torch.randn(4, 3, H, W).to(torch.bfloat16)
+    nan, inf = float("nan"), float("inf")
+    spots = [(0, 1, H - 1, W - 1, inf), (1, 0, H - 1, W // 2, nan), (2, 2, H // 2, W - 2, -inf), (3, 1, H - 2, W - 3, nan), (0, 2, 0, 0, inf)]
+    dy = None
+    for n, c, ih, iw, v in spots:
+        x = clean.clone()
+        x[n, c, ih, iw] = v
+        xc = x.cuda().contiguous(memory_format=torch.channels_last)
+        assert stem_conv.direct(xc, conv.weight)
+        conv.weight.grad = None
+        y = conv(xc)
+        dy = torch.randn_like(y) if dy is None else dy
+        y.backward(dy)
+        gemm.check_status()
+        got = conv.weight.grad.double().cpu()
+        col = F.unfold(x.double(), 7, padding=3, stride=2)                     # [N, 147, OH * OW]
+        ref = torch.einsum("nop,nkp->ok", dy.double().cpu().flatten(2), col).reshape(64, 3, 7, 7)
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf()), (n, c, ih, iw, v)
+        ok = ref.isfinite()
+        assert ok.any() or min(H, W) <= 8
+        # one rounding to bf16 (2^-9 at most) and fp32 sums
+        assert ((got - ref)[ok].norm() <= 4e-3 * ref[ok].norm()), (n, c, ih, iw, v)

@@ -13,6 +13,9 @@
 //                    of 64 channels, N = 80 = ten input rows x 8 values of one tap pair (the rows are a constant stride
 //                    apart), four MMAs per 16 pixels; input row r meets kernel row r of dY row i and r - 2 of row i + 1.
 //                    Partial sums per CTA, added in CTA order by a second kernel (deterministic).
+//                    Where K or M is padded (an output width that is not a multiple of 16, the last row of an odd height) dY is
+//                    zero and the image is not: the operands there are arranged so that a non-finite pixel meets no zero
+//                    that is not its own (tail units, the single row).
 //
 // What bounds it: forward the 411 MB of output (62 us at the copy rate, 256 images of 224 x 224) and, about as much, the
 // MMAs (448 cycles per output row); the weight gradient the reads of dY, the same bytes, and the MMAs (their 128-row dY
@@ -45,6 +48,8 @@ constexpr int LOADERS = 256, THREADS = 512;        // warp 0 issues MMAs, warps 
 constexpr int STAGING = 4096;                      // 32 pixels x 64 channels
 constexpr int W_BYTES = KROWS * TAPS * 8 * COUT * 2;
 constexpr int ACCS = 4, DY_STAGES = 3, WG_N = 80;
+constexpr int TAILS = 2;                           // tap pairs whose last 16 pixels are kept once more
+constexpr int SINGLE_N = 32, SINGLE_COL = TAPS * WG_N;      // accumulators of an odd height's last row: input rows 2..5 of each tap pair
 constexpr unsigned long long kWaitBudgetNs = 4000000000ull;
 
 struct Shared {
@@ -55,7 +60,7 @@ struct Shared {
 
 struct Params {
   int N, H, W, OH, OW, ow16, units, chunks_per_image, chunks;
-  int row_bytes;               // shared-memory bytes of one input row: units * 16
+  int row_bytes;               // shared-memory bytes of one input row: units * 16 (+ the tail units, see load_rows)
   int64_t ws_co, ws_c, ws_h, ws_w;      // strides of the weight (and its gradient), elements
   const __nv_bfloat16* x;
   const __nv_bfloat16* w;
@@ -88,6 +93,10 @@ __device__ __forceinline__ bool chunk(const Params& p, int it, int* n, int* oh0)
 // Warps 8-15: the input rows of a chunk as units.  A unit is 12 contiguous bytes of the image (W is even: a pair is inside
 // or outside as a whole).  Four units per thread are in flight; the loads of a chunk's first four start before the buffer
 // is free.
+// TAIL (weight gradient): where the output width is not a multiple of 16, the last 16 output pixels of a row are partly padding,
+// and under the first two tap pairs the padding's windows would reach into the image.  Each row carries those 16 units once
+// more per tap pair, zeros (written at the start) where the output pixel is padding.
+template <bool TAIL>
 __device__ void load_rows(Shared* sh, unsigned char* rows, const Params& p, int tid) {
   const int total = IN_ROWS * p.units, pairs = p.W / 2;
   int n, oh0;
@@ -112,9 +121,20 @@ __device__ void load_rows(Shared* sh, unsigned char* rows, const Params& p, int 
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int t = t0 + q * LOADERS;
-        if (t < total)
-          *reinterpret_cast<uint4*>(dst + (size_t)t * 16) =
-              make_uint4(w[q][0], w[q][1] & 0xffffu, (w[q][1] >> 16) | (w[q][2] << 16), w[q][2] >> 16);
+        if (t >= total) continue;
+        const uint4 unit = make_uint4(w[q][0], w[q][1] & 0xffffu, (w[q][1] >> 16) | (w[q][2] << 16), w[q][2] >> 16);
+        if constexpr (!TAIL) {
+          *reinterpret_cast<uint4*>(dst + (size_t)t * 16) = unit;
+        } else {
+          const int row = t / p.units, u = t - row * p.units, rest = p.OW & 15;
+          unsigned char* line = dst + (size_t)row * p.row_bytes;
+          *reinterpret_cast<uint4*>(line + u * 16) = unit;
+#pragma unroll
+          for (int tap = 0; tap < TAILS; ++tap) {
+            const int j = u - (p.OW - rest) - tap;               // pixel among the last 16
+            if (j >= 0 && j < rest) *reinterpret_cast<uint4*>(line + (p.units + tap * 16 + j) * 16) = unit;
+          }
+        }
       }
     }
     sm100::fence_proxy_async_smem();
@@ -282,7 +302,7 @@ __global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_const
   if (warp == 0) {
     if (sm100::elect_one()) fwd_mma(sh, rows, weights, p);
   } else if (warp >= 8) {
-    load_rows(sh, rows, p, threadIdx.x - 256);
+    load_rows<false>(sh, rows, p, threadIdx.x - 256);
   } else if (warp >= 4) {
     fwd_drain(sh, staging, weights, p, &map_y, warp & 3, lane);
   }
@@ -290,6 +310,10 @@ __global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_const
 }
 
 // ---------------------------------------------------------------- weight gradient
+// PADDED: an output width that is not a multiple of 16 or an odd output height (see load_rows and the row alone below).  The
+// other form stays as it is where nothing is padded: its code is shorter, and the thread that issues the MMAs is paced by it.
+// 256 x 200 x 200 135 us, 256 x 222 x 224 152 (136 and 148 without the precautions), 256 x 224 x 224, not padded, 148.
+template <bool PADDED>
 __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int dy_row = p.ow16 * 128, dy_stage = 2 * dy_row;     // a pair of dY rows of 64 channels, 128-byte swizzle
@@ -298,12 +322,27 @@ __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_con
   Shared* sh = (Shared*)(rows + 2 * IN_ROWS * p.row_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   setup(sh, warp);
+  if constexpr (PADDED) {
+    for (int t = threadIdx.x; t < 2 * IN_ROWS * TAILS * 16; t += THREADS)
+      *reinterpret_cast<uint4*>(rows + (t / (TAILS * 16)) * p.row_bytes + (p.units + t % (TAILS * 16)) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    sm100::fence_proxy_async_smem();
+  }
   sm100::tc_fence_before();
   __syncthreads();
   sm100::tc_fence_after();
+  if constexpr (PADDED) {                                     // two kinds of products, either may come first: all sums start at zero
+    if (warp >= 4 && warp < 8) {
+      const uint32_t zero[16] = {};
+      for (int c = 0; c < SINGLE_COL + TAPS * SINGLE_N; c += 16) sm100::tmem_st_32x16(sh->tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c, zero);
+      sm100::tmem_st_wait();
+    }
+    sm100::tc_fence_before();
+    __syncthreads();
+    sm100::tc_fence_after();
+  }
   int n, oh0;
   if (warp >= 8) {
-    load_rows(sh, rows, p, threadIdx.x - 256);
+    load_rows<PADDED>(sh, rows, p, threadIdx.x - 256);
   } else if (warp == 1) {
     if (sm100::elect_one()) [&]() {
       int count = 0;
@@ -320,6 +359,8 @@ __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_con
   } else if (warp == 0) {
     if (sm100::elect_one()) [&]() {
       constexpr uint32_t idesc = sm100::make_idesc_f16(128, WG_N, true, true, true);      // both operands MN-major (pixels are K)
+      constexpr uint32_t idesc_16 = sm100::make_idesc_f16(128, 16, true, true, true);
+      constexpr uint32_t idesc_single = sm100::make_idesc_f16(128, SINGLE_N, true, true, true);
       const uint32_t x0 = sm100::smem_u32(rows);
       int count = 0;
       for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
@@ -331,11 +372,39 @@ __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_con
           sm100::tc_fence_after();
           const uint64_t a = sm100::make_desc_sw128_mn(sm100::smem_u32(dys + s * dy_stage), dy_row, 1024);
           const uint32_t x_row = x0 + (uint32_t)(b * IN_ROWS + 2 * i) * p.row_bytes;
-          for (int k = 0; k < p.ow16 / 16; ++k)
+          if constexpr (!PADDED) {
+            for (int k = 0; k < p.ow16 / 16; ++k)
 #pragma unroll
-            for (int t = 0; t < TAPS; ++t)
-              sm100::umma_f16(sh->tmem_base + t * WG_N, a + (uint64_t)((k * 16 * 128) >> 4), desc_plain(x_row + (k * 16 + t) * 16, 128, p.row_bytes),
-                              idesc, (count | k) ? 1u : 0u);
+              for (int t = 0; t < TAPS; ++t)
+                sm100::umma_f16(sh->tmem_base + t * WG_N, a + (uint64_t)((k * 16 * 128) >> 4), desc_plain(x_row + (k * 16 + t) * 16, 128, p.row_bytes),
+                                idesc, (count | k) ? 1u : 0u);
+          } else {
+            // descriptors advance by units of 16 bytes in their address field
+            const uint64_t x = desc_plain(x_row, 128, p.row_bytes), x2 = desc_plain(x_row + 2 * p.row_bytes, 128, p.row_bytes);
+            const int blocks = p.OW / 16;                        // of 16 whole pixels
+            auto block = [&](int k, int (&at)[TAPS]) {
+              if (oh0 + i + 1 < p.OH) {
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t) sm100::umma_f16(sh->tmem_base + t * WG_N, a + (uint64_t)(k * 128), x + (uint64_t)at[t], idesc, 1u);
+              } else {
+                // Row i alone: dY row i + 1 is padding.  Its products land in the other 64 accumulator rows: input rows 0 and 1
+                // are none of its, input rows 2 - 5 go to columns of their own, later ones lie below the image.
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t) {
+                  sm100::umma_f16(sh->tmem_base + t * WG_N, a + (uint64_t)(k * 128), x + (uint64_t)at[t], idesc_16, 1u);
+                  sm100::umma_f16(sh->tmem_base + SINGLE_COL + t * SINGLE_N, a + (uint64_t)(k * 128), x2 + (uint64_t)at[t], idesc_single, 1u);
+                }
+              }
+            };
+            for (int k = 0; k < blocks; ++k) {
+              int at[TAPS] = {k * 16, k * 16 + 1, k * 16 + 2, k * 16 + 3};
+              block(k, at);
+            }
+            if (p.OW & 15) {                                     // the cut last block: tail units under the first tap pairs
+              int at[TAPS] = {p.units, p.units + 16, blocks * 16 + 2, blocks * 16 + 3};
+              block(blocks, at);
+            }
+          }
           sm100::umma_commit(&sh->dy_empty[s]);
         }
         sm100::umma_commit(&sh->x_empty[b]);
@@ -347,15 +416,30 @@ __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_con
       STEM_WAIT(&sh->acc_full[0], 0, 68);
       sm100::tc_fence_after();
       const int row = (warp & 3) * 32 + lane;
+      const uint32_t tm = sh->tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
       float* out = p.partial + ((size_t)blockIdx.x * 128 + row) * (TAPS * WG_N);
       for (int c = 0; c < TAPS * WG_N; c += 32) {
         uint32_t r[32];
-        sm100::tmem_ld_32x32(sh->tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + c, r);
+        sm100::tmem_ld_32x32(tm + c, r);
         sm100::tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           *reinterpret_cast<float4*>(out + c + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
                                                                 __uint_as_float(r[j + 3]));
+      }
+      if (PADDED && (warp & 3) < 2) {                           // the first 64 rows: the single rows' sums on top
+        for (int t = 0; t < TAPS; ++t) {
+          uint32_t r[32];
+          sm100::tmem_ld_32x32(tm + SINGLE_COL + t * SINGLE_N, r);
+          sm100::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            float4* o = reinterpret_cast<float4*>(out + t * WG_N + 16 + j);
+            const float4 v = *o;
+            *o = make_float4(v.x + __uint_as_float(r[j]), v.y + __uint_as_float(r[j + 1]), v.z + __uint_as_float(r[j + 2]),
+                             v.w + __uint_as_float(r[j + 3]));
+          }
+        }
       }
       sm100::tc_fence_before();
     }();
@@ -453,10 +537,13 @@ int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, 
   p.partial = (float*)workspace;
   CUtensorMap mdy;
   if ((st = make_tmap_bf16_4d(&mdy, dy, {(uint64_t)stem::COUT, (uint64_t)p.OW, (uint64_t)p.OH, (uint64_t)N}, {64, (uint32_t)p.ow16, 1, 1}))) return st;
+  const bool padded = p.OW % 16 != 0 || p.OH % 2 != 0;
+  if (padded) p.row_bytes += stem::TAILS * 16 * 16;
   const int smem = stem::DY_STAGES * 2 * p.ow16 * 128 + 2 * stem::IN_ROWS * p.row_bytes + (int)sizeof(stem::Shared);
-  cudaError_t e = cudaFuncSetAttribute(stem::stem_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const auto kernel = padded ? stem::stem_wgrad_kernel<true> : stem::stem_wgrad_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "stem weight gradient: shared memory attribute: %s", cudaGetErrorString(e));
-  stem::stem_wgrad_kernel<<<grid, stem::THREADS, smem, (cudaStream_t)stream>>>(mdy, p);
+  kernel<<<grid, stem::THREADS, smem, (cudaStream_t)stream>>>(mdy, p);
   stem::stem_wgrad_reduce_kernel<<<stem::COUT, stem::RED_COLS * stem::RED_GROUPS, 0, (cudaStream_t)stream>>>(
       (const float*)workspace, grid, (__nv_bfloat16*)dw, p.ws_co, p.ws_c, p.ws_h, p.ws_w);
   e = cudaGetLastError();
