@@ -215,3 +215,20 @@ def test_attention_non_finite_scores(key):
         assert torch.equal(l[:, 0, :key], lse[:, 0, :key]) and torch.equal(l[:, 1], lse[:, 1])
     assert out_nan[0, key:, :64].isnan().all() and lse_nan[0, 0, key:].isnan().all()
     assert out_inf[0, row, :64].isnan().all() and lse_inf[0, 0, row].isnan()
+
+
+def test_last_backward_names_a_backward_that_ran():
+    from torchmpi_b200.ops import attention
+    qkv = torch.randn(1, 128, 3 * 64, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    attention._BACKWARDS = ("none",)
+    try:
+        attention.causal_attention(qkv, 1).sum().backward()
+    finally:
+        attention._BACKWARDS = ("own", "cudnn", "flash")
+    assert attention.last_backward == "recompute"
+    out = attention.causal_attention(qkv, 1)
+    assert attention.last_backward == "recompute"          # a forward names nothing
+    out.sum().backward()
+    assert attention.last_backward == "own"
+    out, lse = attention.attention_forward(qkv.detach(), 1)
+    assert attention.last_backward == "own"

@@ -10,7 +10,7 @@ import importlib.util
 
 from . import _lib, build  # noqa: F401  (_lib loads the native library first)
 
-LINEAR, LAYERNORM, ATTENTION, XENT = range(4)      # counters of ``launches``
+LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD = range(5)      # counters of ``launches``; attention counts calls
 _ext = None
 
 
@@ -28,5 +28,6 @@ def ext():
 
 
 def launches(what: int) -> int:
-    """Kernels that the C++ functions of one kind have launched in this process (0 before the first use)."""
+    """Kernels (for attention: calls, both ways or backward alone) that the C++ functions of one kind have launched in this
+    process; 0 before the first use."""
     return _ext.launches(what) if _ext is not None else 0

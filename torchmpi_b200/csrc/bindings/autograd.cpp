@@ -22,8 +22,8 @@ using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-std::atomic<long long> g_launches[4];          // linear, layer norm, attention, cross-entropy
-enum { LINEAR = 0, LAYERNORM = 1, ATTENTION = 2, XENT = 3 };
+enum { LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD, KINDS };
+std::atomic<long long> g_launches[KINDS];      // attention: calls, and those of the backward alone
 enum { EPI_BIAS = 1, B_IS_KN = 4, A_IS_KM = 8 };
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
@@ -203,6 +203,7 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
                              delta.data_ptr<float>(), dq_acc.data_ptr<float>(), g, g + C * 2, g + 2 * C * 2, C3, (int)B, (int)T, (int)heads,
                              (float)(1.0 / std::sqrt((double)HEAD)), stream()));
     launched(ATTENTION, 1);
+    launched(ATTENTION_BACKWARD, 1);
     return {dqkv, Tensor()};
   }
 };

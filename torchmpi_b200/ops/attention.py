@@ -26,12 +26,14 @@ from .. import _native
 from .._lib import lib, check, has_symbol, stream_ptr, TorchMPIError
 
 _launches = 0
-last_backward = ""
+_last = ("", 0)      # the last backward that ran in Python, and how many had run in the C++ function by then
 
 
 def __getattr__(name: str):
     if name == "launch_count":               # attention calls on this package's kernels, the C++ function's included
         return _launches + _native.launches(_native.ATTENTION)
+    if name == "last_backward":              # the route of the last backward that ran ("" before the first)
+        return "own" if _native.launches(_native.ATTENTION_BACKWARD) > _last[1] else _last[0]
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
@@ -90,6 +92,11 @@ def attention_backward(qkv: torch.Tensor, out: torch.Tensor, lse: torch.Tensor, 
     return dqkv
 
 
+def _ran(route: str) -> None:
+    global _last
+    _last = (route, _native.launches(_native.ATTENTION_BACKWARD))
+
+
 def _reference(qkv: torch.Tensor, n_head: int) -> torch.Tensor:
     B, T, C3 = qkv.shape
     C = C3 // 3
@@ -109,7 +116,6 @@ class _AttnFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        global last_backward
         qkv, out, lse = ctx.saved_tensors
         H = ctx.n_head
         B, T, C3 = qkv.shape
@@ -122,7 +128,7 @@ class _AttnFn(torch.autograd.Function):
         grads = None
         for name in _BACKWARDS:
             if name == "own":              # this package's kernel: an error of it is raised, not routed around
-                last_backward = name
+                _ran(name)
                 return attention_backward(qkv, out, lse, dout, H), None
             try:
                 if name == "cudnn":
@@ -133,7 +139,7 @@ class _AttnFn(torch.autograd.Function):
                 else:
                     grads = torch.ops.aten._scaled_dot_product_flash_attention_backward(
                         go, q, k, v, o, lse, None, None, T, T, 0.0, True, zero, zero, scale=scale)
-                last_backward = name
+                _ran(name)
                 break
             except (RuntimeError, TypeError):
                 continue
@@ -141,7 +147,7 @@ class _AttnFn(torch.autograd.Function):
             with torch.enable_grad():
                 leaf = qkv.detach().requires_grad_(True)
                 (dqkv,) = torch.autograd.grad(_reference(leaf, H), leaf, dout)
-            last_backward = "recompute"
+            _ran("recompute")
             return dqkv, None
         dq, dk, dv = grads
         dqkv = torch.empty_like(qkv)
@@ -155,8 +161,5 @@ def causal_attention(qkv: torch.Tensor, n_head: int) -> torch.Tensor:
     if not supported(qkv, n_head):
         return _reference(qkv, n_head)
     if _BACKWARDS[0] == "own":
-        global last_backward
-        if qkv.requires_grad:
-            last_backward = "own"
         return _native.ext().causal_attention(qkv, n_head)
     return _AttnFn.apply(qkv, n_head)
