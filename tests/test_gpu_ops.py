@@ -561,3 +561,30 @@ def test_stem_weight_gradient_non_finite_pixels(H, W):
         assert ok.any() or min(H, W) <= 8
         # one rounding to bf16 (2^-9 at most) and fp32 sums
         assert ((got - ref)[ok].norm() <= 4e-3 * ref[ok].norm()), (n, c, ih, iw, v)
+
+
+def test_stem_weight_gradient_in_a_graph_beside_an_eager_one():
+    """A captured weight gradient, replayed while eager ones run on the stream it was captured on: each has its own partial
+    sums."""
+    from torchmpi_b200.ops.stem_conv import _StemDirectFn
+    torch.manual_seed(8)
+    w = torch.randn(64, 3, 7, 7, device="cuda").to(torch.bfloat16)
+    x = [torch.randn(64, 3, 64, 64, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last) for _ in range(2)]
+    dy = [torch.randn(64, 64, 32, 32, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last) for _ in range(2)]
+
+    def grad(k):
+        leaf = w.detach().requires_grad_(True)             # of the stream that this runs on
+        return torch.autograd.grad(_StemDirectFn.apply(x[k], leaf), leaf, dy[k])[0]
+
+    want = [grad(0), grad(1)]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        captured = grad(0)
+    for _ in range(10):
+        graph.replay()
+        with torch.cuda.stream(side):
+            eager = grad(1)
+        torch.cuda.synchronize()
+        assert torch.equal(captured, want[0]) and torch.equal(eager, want[1])

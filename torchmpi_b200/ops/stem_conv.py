@@ -3,7 +3,8 @@
 ``StemConv7x7`` is an ``nn.Conv2d(3, C, 7, stride=2, padding=3, bias=False)`` with the same parameter
 (``weight [C, 3, 7, 7]``), so checkpoints and parameter counts do not change.  On a channels-last
 bf16 CUDA input with 64 output channels and rows of up to 256 pixels, forward and weight gradient (the image
-has none) are implicit GEMMs that read the image itself (csrc/kernels/stem_conv.cu).  Other widths and channel
+has none) are implicit GEMMs that read the image itself (csrc/kernels/stem_conv.cu); backward reads it again, so as with
+``nn.Conv2d`` it must not be modified in between (autograd raises an error).  Other widths and channel
 counts go through the patch matrix ``col [N*OH*OW, 160]``, written by one kernel (csrc/kernels/im2col.cu) and
 multiplied with the ``[C, 160]`` weight matrix; their weight gradient is the split-K product ``dY^T col`` over the
 saved patch matrix.  Inputs that neither takes go to ``F.conv2d``.
@@ -21,16 +22,6 @@ from . import gemm
 
 launch_count = 0
 PATCH = 147
-_ws = {}
-
-
-def _workspace(dev: torch.device) -> torch.Tensor:
-    """Per (device, stream) buffer for the partial sums of the weight gradient (one row of CTAs: 24 MB)."""
-    key = (dev.index, stream_ptr())
-    buf = _ws.get(key)
-    if buf is None:
-        buf = _ws[key] = torch.empty(lib.tmpi_stem_conv_wgrad_workspace_bytes(), dtype=torch.uint8, device=dev)
-    return buf
 
 
 class _StemDirectFn(torch.autograd.Function):
@@ -58,7 +49,8 @@ class _StemDirectFn(torch.autograd.Function):
         if dy.data_ptr() % 16:                                               # a view into a larger buffer
             dy = dy.clone(memory_format=torch.channels_last)
         dw = torch.empty_strided(ctx.wshape, ctx.wstride, dtype=x.dtype, device=x.device)
-        ws = _workspace(x.device)
+        # partial sums of the CTAs (24 MB), from the allocator: calls on other streams, threads and in graphs have their own
+        ws = torch.empty(lib.tmpi_stem_conv_wgrad_workspace_bytes(), dtype=torch.uint8, device=x.device)
         check(lib.tmpi_stem_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, H, W, ctx.wshape[0],
                                        (ctypes.c_int64 * 4)(*dw.stride()), ws.data_ptr(), ws.numel(), stream_ptr()))
         launch_count += 2
