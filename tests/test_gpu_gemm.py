@@ -284,7 +284,8 @@ def test_linear_without_bias_and_with_frozen_inputs(gelu, rows, n, bias, frozen)
 
 
 def test_refused_operands_of_linear_and_cross_entropy():
-    """Operands that do not fit each other and an empty batch raise before anything is launched."""
+    """Operands that do not fit each other, an empty batch and types that no kernel takes raise before anything is launched."""
+    from torchmpi_b200._lib import TorchMPIError
     from torchmpi_b200.ops import gemm, xent
     x = torch.zeros(16, 64, device="cuda", dtype=torch.bfloat16)
     for w in (torch.zeros(32, 128, device="cuda"), torch.zeros(32, 56, device="cuda"), torch.zeros(32, 64), torch.zeros(32, device="cuda")):
@@ -293,6 +294,11 @@ def test_refused_operands_of_linear_and_cross_entropy():
                 gemm.linear(x, w.to(torch.bfloat16), None, gelu=gelu)
     with pytest.raises(ZeroDivisionError):
         xent.cross_entropy(torch.zeros(0, 10, device="cuda"), torch.zeros(0, device="cuda", dtype=torch.int64))
+    for dtype in (torch.float64, torch.int32, torch.int64):
+        with pytest.raises(TorchMPIError):
+            xent.cross_entropy(torch.zeros(4, 10, device="cuda", dtype=dtype), torch.zeros(4, device="cuda", dtype=torch.int64))
+    with pytest.raises(TypeError):
+        xent.cross_entropy(torch.zeros(4, 10, device="cuda", dtype=torch.complex64), torch.zeros(4, device="cuda", dtype=torch.int64))
 
 
 def test_first_cuda_call_of_a_thread_encodes_a_tensor_map():

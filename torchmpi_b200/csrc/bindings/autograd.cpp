@@ -14,6 +14,7 @@
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <string>
 #include "tmpi_c_api.h"
 
 namespace {
@@ -40,7 +41,13 @@ int dtype_code(at::ScalarType t) {
     case at::kHalf: return TMPI_F16;
     case at::kBFloat16: return TMPI_BF16;
     case at::kFloat: return TMPI_F32;
-    default: TORCH_CHECK(false, "torchmpi_b200: unsupported dtype ", t);
+    case at::kDouble: return TMPI_F64;                           // what a kernel does not take, its entry point refuses
+    case at::kByte: return TMPI_U8;
+    case at::kChar: return TMPI_I8;
+    case at::kShort: return TMPI_I16;
+    case at::kInt: return TMPI_I32;
+    case at::kLong: return TMPI_I64;
+    default: throw pybind11::type_error(std::string("torchmpi_b200: unsupported dtype ") + c10::toString(t));
   }
 }
 
