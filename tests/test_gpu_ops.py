@@ -588,3 +588,40 @@ def test_stem_weight_gradient_in_a_graph_beside_an_eager_one():
             eager = grad(1)
         torch.cuda.synchronize()
         assert torch.equal(captured, want[0]) and torch.equal(eager, want[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_operands_between_16_byte_boundaries(dtype):
+    """Views that start one element into a buffer, as inputs, parameters and incoming gradients: the bits of aligned operands."""
+    from torchmpi_b200.ops import gemm, layernorm
+    torch.manual_seed(6)
+
+    def shifted(t):
+        v = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape)
+        return v.copy_(t)
+
+    x, dy = torch.randn(37, 512, device="cuda").to(dtype), torch.randn(37, 512, device="cuda").to(dtype)
+    g, b = torch.randn(512, device="cuda").to(dtype), torch.randn(512, device="cuda").to(dtype)
+    out = []
+    for place in (torch.clone, shifted):
+        ln = layernorm.LayerNorm(512, device="cuda", dtype=dtype)
+        ln.weight, ln.bias = torch.nn.Parameter(place(g)), torch.nn.Parameter(place(b))
+        leaf = place(x).requires_grad_(True)
+        y = ln(leaf)
+        y.backward(place(dy))
+        out.append([y.detach(), leaf.grad, ln.weight.grad, ln.bias.grad])
+    assert all(torch.equal(a, c) for a, c in zip(*out))
+    rows, n = 64, 1024
+    dy, z = torch.randn(rows, n, device="cuda").to(dtype), torch.randn(rows, n, device="cuda").to(dtype)
+    (dz, db), (dz2, db2) = gemm.bias_grad(dy, z), gemm.bias_grad(shifted(dy), shifted(z))
+    unit = {torch.float32: 1e-5, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -6}[dtype]       # PyTorch's passes round once more
+    assert torch.allclose(dz, dz2, rtol=unit, atol=unit) and torch.allclose(db, db2, rtol=unit, atol=unit * rows ** 0.5)
+    if dtype == torch.bfloat16:
+        w, bias, xl = (torch.randn(*s, device="cuda").to(dtype) for s in ((n, 256), (n,), (rows, 256)))
+        for gelu in (False, True):
+            out = []
+            for place in (torch.clone, shifted):
+                leaves = [t.clone().requires_grad_(True) for t in (xl, w, bias)]
+                y = gemm.linear(*leaves, gelu=gelu)
+                out.append(torch.autograd.grad(y, leaves, place(dy)))
+            assert all(torch.equal(a, c) for a, c in zip(*out))

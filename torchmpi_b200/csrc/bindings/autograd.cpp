@@ -51,6 +51,13 @@ int dtype_code(at::ScalarType t) {
   }
 }
 
+// Contiguous and on a 16-byte boundary, which the elementwise kernels' loads need: a view into a larger buffer may start
+// anywhere.
+Tensor packed(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return (uintptr_t)c.data_ptr() % 16 ? c.clone() : c;
+}
+
 bool pair_enabled() {
   int64_t v = 0;
   check(tmpi_get_tunable("gemm_pair", &v));
@@ -144,7 +151,7 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2 = saved[0], &w = saved[1], &z = saved[2];
     const Tensor& dy = grads[0];
-    Tensor dy2 = dy.reshape({-1, dy.size(-1)}).contiguous(), db, dx, dw;
+    Tensor dy2 = packed(dy.reshape({-1, dy.size(-1)})), db, dx, dw;
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) std::tie(dy2, db) = bias_grad(dy2, z);
     else if (z.defined()) dy2 = at::gelu_backward(dy2, z);
     if (ctx->needs_input_grad(0)) dx = matmul_nn(dy2, w).reshape(ctx->saved_data["shape"].toIntVector());
@@ -157,14 +164,14 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
 struct LayerNormFn : public torch::autograd::Function<LayerNormFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, double eps) {
     const int64_t C = x.size(-1);
-    Tensor x2 = x.reshape({-1, C}).contiguous();
+    const Tensor x2 = packed(x.reshape({-1, C})), g = packed(weight), b = packed(bias);
     const int64_t rows = x2.size(0);
     Tensor y = at::empty_like(x2), stats = at::empty({2, rows}, x.options().dtype(at::kFloat));      // mean, 1 / std
     float* mean = stats.data_ptr<float>();
-    check(tmpi_layernorm_fwd(x2.data_ptr(), weight.data_ptr(), bias.data_ptr(), y.data_ptr(), mean, mean + rows, (int)rows, (int)C, (float)eps,
+    check(tmpi_layernorm_fwd(x2.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(), mean, mean + rows, (int)rows, (int)C, (float)eps,
                              dtype_code(x.scalar_type()), stream()));
     launched(LAYERNORM, 1);
-    ctx->save_for_backward({x2, weight, stats});
+    ctx->save_for_backward({x2, g, stats});
     ctx->saved_data["shape"] = x.sizes().vec();
     return y.view(x.sizes());
   }
@@ -172,7 +179,7 @@ struct LayerNormFn : public torch::autograd::Function<LayerNormFn> {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2 = saved[0], &weight = saved[1];
     const int64_t rows = x2.size(0), C = x2.size(1);
-    Tensor dy2 = grads[0].reshape({rows, C}).contiguous();
+    const Tensor dy2 = packed(grads[0].reshape({rows, C}));
     Tensor dx = at::empty_like(x2), dgamma = at::empty_like(weight), dbeta = at::empty_like(weight);
     Tensor scratch = at::empty({(int64_t)tmpi_layernorm_scratch_bytes((int)C)}, x2.options().dtype(at::kByte));
     const float* mean = saved[2].data_ptr<float>();

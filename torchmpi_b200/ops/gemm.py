@@ -204,8 +204,8 @@ def bias_grad(dy2: torch.Tensor, z: Optional[torch.Tensor] = None):
     rows, C = dy2.shape
     per_slab = 128 * (16 // dy2.element_size())
     if not (dy2.is_cuda and dy2.is_contiguous() and C % per_slab == 0 and has_symbol("tmpi_bias_grad")
-            and dy2.dtype in (torch.bfloat16, torch.float16, torch.float32)
-            and (z is None or (z.is_contiguous() and z.dtype == dy2.dtype))):
+            and dy2.dtype in (torch.bfloat16, torch.float16, torch.float32) and dy2.data_ptr() % 16 == 0
+            and (z is None or (z.is_contiguous() and z.dtype == dy2.dtype and z.data_ptr() % 16 == 0))):
         dz = torch.ops.aten.gelu_backward(dy2, z) if z is not None else dy2
         return dz, dz.sum(0)
     sp = stream_ptr()
