@@ -220,10 +220,13 @@ def test_gelu_forward_kernel():
     assert torch.allclose(gemm.gelu(edge), torch.nn.functional.gelu(edge), atol=1e-5)
 
 
-@pytest.mark.parametrize("M,N,K,bias", [(256, 256, 64, True), (300, 520, 136, True), (384, 264, 72, False), (3072, 1000, 200, True)])
+@pytest.mark.parametrize("M,N,K,bias", [(256, 256, 64, True), (300, 520, 136, True), (384, 264, 72, False), (3072, 1000, 200, True),
+                                        (8200, 4104, 136, True), (4104, 3000, 72, False), (2056, 2056, 136, True), (3592, 1032, 200, False)])
 def test_gelu_epilogue_equals_product_then_gelu(M, N, K, bias):
     """One kernel that writes z and gelu(z): the same bits as the product followed by the elementwise pass (GELU of the
-    rounded z), tiles of 256 and of 192 columns, ragged edges."""
+    rounded z), ragged edges.  On 74 clusters the first three shapes have a few tiles of 128 columns and the fourth 72 of 192, one
+    per cluster; the others several per cluster (accumulators and staging tiles used again): up to eight of 256 columns, three
+    of 256, two of 192, two of 128."""
     from torchmpi_b200.ops import gemm
     torch.manual_seed(M + N)
     a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
@@ -238,9 +241,10 @@ def test_gelu_epilogue_equals_product_then_gelu(M, N, K, bias):
     assert ((z.float() - ref).norm() / ref.norm()).item() < 4e-3          # one bf16 rounding: 2^-9 at most
 
 
-@pytest.mark.parametrize("M,N,K", [(3072, 1024, 200), (3072, 1000, 72), (8192, 384, 136)])
+@pytest.mark.parametrize("M,N,K", [(3072, 1024, 200), (3072, 1000, 72), (8192, 384, 136), (2056, 2056, 136), (3592, 1032, 200)])
 def test_pair_gemm_narrow_tiles(M, N, K):
-    """Shapes whose tiles are 192 columns wide (they fill the SMs better than 256), all operand layouts, a bias."""
+    """Shapes whose tiles are 192 columns wide (they fill the SMs better than 256), the last one 128, all operand layouts, a
+    bias; the last two with more tiles than clusters."""
     from torchmpi_b200.ops import gemm
     torch.manual_seed(M + N + K)
     a = torch.randn(M, K, device="cuda").to(torch.bfloat16)

@@ -374,10 +374,13 @@ def test_cross_entropy_infinities_and_bad_labels():
         xg = x.clone().requires_grad_(True)
         labels = torch.zeros(6, dtype=torch.int64, device="cuda")
         labels[1] = 1
-        loss = xent.cross_entropy(xg, labels)
+        bad = labels.clone()
+        bad[4], bad[5] = -1, cols                          # no class: nothing is taken off the gradient
+        loss = xent.cross_entropy(xg, bad)
         loss.backward()
         ref = x.clone().requires_grad_(True)
         torch.nn.functional.cross_entropy(ref, labels).backward()
+        ref.grad[4:, 0] += 1.0 / 6
         assert torch.isnan(loss)
         for r in (0, 1, 3, 4, 5):
             assert torch.allclose(xg.grad[r], ref.grad[r], rtol=1e-5, atol=1e-8), (cols, r)
@@ -625,3 +628,28 @@ def test_operands_between_16_byte_boundaries(dtype):
                 y = gemm.linear(*leaves, gelu=gelu)
                 out.append(torch.autograd.grad(y, leaves, place(dy)))
             assert all(torch.equal(a, c) for a, c in zip(*out))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [10, 1000, 5003, 60001])
+def test_cross_entropy_labels_outside_the_row(cols, dtype):
+    """A label that names no class counts as the largest logit in the loss and takes nothing off the gradient, in the kernel of
+    short rows, of rows in shared memory and of rows that are read three times."""
+    from torchmpi_b200.ops import xent
+    torch.manual_seed(cols)
+    x = torch.randn(6, cols, device="cuda").mul_(2.0).to(dtype).requires_grad_(True)
+    labels = torch.tensor([-100, cols, cols - 1, -1, 2 ** 31 - 1, 0], device="cuda")
+    loss = xent.cross_entropy(x, labels)
+    loss.backward()
+    xd = x.detach().double()
+    inside = (labels >= 0) & (labels < cols)
+    picked = torch.where(inside, xd.gather(1, labels.clamp(0, cols - 1)[:, None])[:, 0], xd.max(1).values)
+    want = (torch.logsumexp(xd, 1) - picked).mean()
+    assert abs(loss.item() - want.item()) <= 2e-6 * max(1.0, abs(want.item()))
+    p = torch.softmax(xd, 1)
+    p[inside, labels[inside]] -= 1.0
+    p /= 6
+    # exponentials from the special-function unit, fp16 between the passes of long 16-bit rows, one final rounding
+    unit = {torch.float32: 2e-6, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7.5}[dtype]
+    floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / 6
+    assert bool(((x.grad.double() - p).abs() <= unit * p.abs() + floor).all())
