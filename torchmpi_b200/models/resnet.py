@@ -5,7 +5,8 @@ The reference ships no model beyond a logistic regressor
 (He et al. 2015, stride on the 3x3 convolution) written for channels_last bf16
 training.  With ``fused_bn=True`` batch-norm + ReLU (+ residual add) run as the fused kernels of
 ``ops.bn_relu``, the max-pool as ``ops.pool`` and the stem convolution as an implicit tcgen05 GEMM
-(``ops.stem_conv``); the other convolutions run in cuDNN.
+(``ops.stem_conv``).  The 1x1 convolutions run on ``ops.conv``'s implicit GEMM, the 3x3 ones in cuDNN (on the former too
+with the tunable ``conv_own_3x3``).
 """
 from __future__ import annotations
 
