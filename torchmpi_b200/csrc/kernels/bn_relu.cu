@@ -26,21 +26,75 @@ namespace tmpi {
 constexpr int kBnThreads = 256;
 constexpr int kBnMaxGrid = 592;     // 148 SMs x 4 resident CTAs
 
-static int bn_grid(size_t nvec) {
-  size_t want = (nvec + kBnThreads - 1) / kBnThreads;
-  return (int)std::max<size_t>(1, std::min<size_t>(want, kBnMaxGrid));
+// Blocks of a streaming pass: `most`, or fewer where there are not U vectors for every thread of them.
+static int bn_grid(size_t nvec, int most, int U) {
+  const size_t want = (nvec + (size_t)kBnThreads * U - 1) / ((size_t)kBnThreads * U);
+  return (int)std::max<size_t>(1, std::min<size_t>(want, most));
 }
 
+// A pack of NW 32-bit words (8 or 16 bytes), elements taken out and put in by shifts and pair conversions (element-wise
+// structs cost a register per 16-bit element here and spilled).
+template <int NW> struct BpWords { uint32_t w[NW]; };
+template <int NW> __device__ __forceinline__ BpWords<NW> bp_ld(const void* p) {
+  if constexpr (NW == 4) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    return BpWords<NW>{{u.x, u.y, u.z, u.w}};
+  } else {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return BpWords<NW>{{u.x, u.y}};
+  }
+}
+template <int NW> __device__ __forceinline__ void bp_st(void* p, const BpWords<NW>& b) {
+  if constexpr (NW == 4) *reinterpret_cast<uint4*>(p) = make_uint4(b.w[0], b.w[1], b.w[2], b.w[3]);
+  else *reinterpret_cast<uint2*>(p) = make_uint2(b.w[0], b.w[1]);
+}
+template <typename T, int NW> __device__ __forceinline__ float bp_get(const BpWords<NW>& b, int c) {
+  if constexpr (sizeof(T) == 4) return __uint_as_float(b.w[c]);
+  else if constexpr (std::is_same<T, __nv_bfloat16>::value) return __uint_as_float((c & 1) ? b.w[c >> 1] & 0xffff0000u : b.w[c >> 1] << 16);
+  else return __half2float(__ushort_as_half((unsigned short)((c & 1) ? b.w[c >> 1] >> 16 : b.w[c >> 1])));
+}
+// from V floats
+template <typename T, int V> __device__ __forceinline__ BpWords<V * sizeof(T) / 4> bp_put(const float (&f)[V]) {
+  BpWords<V * sizeof(T) / 4> b;
+#pragma unroll
+  for (int k = 0; k < (int)(V * sizeof(T) / 4); ++k) {
+    if constexpr (sizeof(T) == 4) b.w[k] = __float_as_uint(f[k]);
+    else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+      b.w[k] = *reinterpret_cast<uint32_t*>(&h);
+    } else {
+      __half2 h = __floats2half2_rn(f[2 * k], f[2 * k + 1]);
+      b.w[k] = *reinterpret_cast<uint32_t*>(&h);
+    }
+  }
+  return b;
+}
+
+// The passes stream each tensor once and are bound by memory, so what counts is bytes in flight: each thread issues the loads
+// of U vectors before it uses the first, without branches between them (mask source, residual and its gradient are template
+// parameters), and past L1, where lines in flight would compete for space.  Fewer resident blocks with more registers hold
+// more bytes in flight than eight or four small ones.  Measured, 256 x 28 x 28, bf16, before and now: 512 channels, backward
+// sums under mask bits 93 -> 69 us (411 MB: 63 at the copy rate; 97 with the branches), forward apply with a residual
+// 120 -> 108 (96); 128 channels, backward sums 27 -> 20, backward apply 28 -> 22.
+template <typename T>
+__device__ __forceinline__ BpWords<4> bn_ld(const T* p) {
+  BpWords<4> u;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
+  return u;
+}
+constexpr int kBnReduceU = 4, kBnApplyU = 2;
+constexpr int kBnReduceBwdGrid = 296, kBnApplyGrid = 740, kBnApplyBwdGrid = 444;       // resident blocks: 2, 5, 3 per SM
+
 // partial[(block * 2 + which) * C + c]
-// MASKX (backward only): the ReLU mask comes from x, gamma and beta instead of y.  A template
-// parameter, not a run-time flag: the extra scale / shift registers would otherwise cost the other
-// path one resident block per SM.
-template <typename T, int V, bool BWD, bool MASKX>
-__global__ void __launch_bounds__(kBnThreads, 4) bn_reduce_kernel(
+// Where a backward pass takes the ReLU mask from (a template parameter: a choice at run time puts branches between the loads).
+enum { MASK_NONE = 0, MASK_X = 1 /* recomputed from x, gamma, beta */, MASK_BITS = 2, MASK_Y = 3 };
+
+template <typename T, int V, bool BWD, int MASK>
+__global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
     const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy,
     const float* __restrict__ mean, const float* __restrict__ invstd,
     const float* __restrict__ gamma, const float* __restrict__ beta, const unsigned char* __restrict__ bits,
-    size_t nvec, int C, int relu, int reverse, float* __restrict__ partial) {
+    size_t nvec, int C, int reverse, float* __restrict__ partial) {
   const int cvn = C / V;
   const size_t T0 = (size_t)blockIdx.x * kBnThreads + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * kBnThreads;
@@ -48,70 +102,59 @@ __global__ void __launch_bounds__(kBnThreads, 4) bn_reduce_kernel(
   // the lines the producer wrote last are still in L2; the apply pass that follows walks up from the
   // start, which this pass read last.  nvec and the stride are multiples of cvn: the group stays fixed.
   const int cv = reverse ? cvn - 1 - (int)(T0 % cvn) : (int)(T0 % cvn);
-  const T* xe = x + (nvec - 1) * V;
-  const T* ge = BWD ? dy + (nvec - 1) * V : nullptr;
-  const T* ye = (BWD && y) ? y + (nvec - 1) * V : nullptr;
-  constexpr bool mask_from_x = BWD && MASKX;
-  float a[V], b[V], mu[V], is[V], sc[V], sh[V];
+  float a[V], b[V], mu[V], sc[V], sh[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) { a[k] = 0.f; b[k] = 0.f; }
-  if (BWD) {
+  if constexpr (BWD) {
 #pragma unroll
-    for (int k = 0; k < V; ++k) { mu[k] = mean[cv * V + k]; is[k] = invstd[cv * V + k]; }
-    if (mask_from_x) {
-#pragma unroll
-      for (int k = 0; k < V; ++k) { sc[k] = is[k] * gamma[cv * V + k]; sh[k] = beta[cv * V + k] - mu[k] * sc[k]; }
+    for (int k = 0; k < V; ++k) {
+      mu[k] = mean[cv * V + k];
+      if constexpr (MASK == MASK_X) { sc[k] = invstd[cv * V + k] * gamma[cv * V + k]; sh[k] = beta[cv * V + k] - mu[k] * sc[k]; }
     }
   }
-  // U independent vectors per thread and iteration: the loads of all of them are issued before
-  // the first use, so a thread keeps U (forward) or up to 3U (backward) 16-byte loads in flight
-  constexpr int U = BWD ? 1 : 4;       // backward already has 2-3 loads per vector and no registers to spare
   // bits (backward, ReLU layers with a residual): one byte per vector written by the forward apply
   // pass, bit k set where the output was positive; replaces the read of y
-  auto accumulate = [&](const Pack<T, V>& xv, const Pack<T, V>& gv, const Pack<T, V>& yv, unsigned mb = 0) {
-    if (!BWD) {
+  auto accumulate = [&](const BpWords<4>& xv, const BpWords<4>& gv, const BpWords<4>& yv, unsigned mb) {
 #pragma unroll
-      for (int k = 0; k < V; ++k) { float f = (float)to_acc<T>(xv.v[k]); a[k] += f; b[k] += f * f; }
-    } else {
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        float g = (float)to_acc<T>(gv.v[k]);
-        if (mask_from_x) {
-          if (!((float)to_acc<T>(xv.v[k]) * sc[k] + sh[k] > 0.f)) g = 0.f;
-        } else if (relu) {
-          if (bits ? !((mb >> k) & 1u) : !((float)to_acc<T>(yv.v[k]) > 0.f)) g = 0.f;
-        }
+    for (int k = 0; k < V; ++k) {
+      const float f = bp_get<T>(xv, k);
+      if constexpr (!BWD) {
+        a[k] += f;
+        b[k] += f * f;
+      } else {
+        float g = bp_get<T>(gv, k);
+        if (MASK == MASK_X && !(f * sc[k] + sh[k] > 0.f)) g = 0.f;
+        if (MASK == MASK_BITS && !((mb >> k) & 1u)) g = 0.f;
+        if (MASK == MASK_Y && !(bp_get<T>(yv, k) > 0.f)) g = 0.f;
         a[k] += g;
-        b[k] += g * ((float)to_acc<T>(xv.v[k]) - mu[k]) * is[k];
+        b[k] += g * (f - mu[k]);             // times 1 / std at the end
       }
     }
   };
-  size_t v = T0;
-  if constexpr (U > 1)
-  for (; v + (U - 1) * stride < nvec; v += U * stride) {
-    Pack<T, V> xv[U], gv[U], yv[U];
+  auto pass = [&](size_t v, auto count) {
+    constexpr int U = decltype(count)::value;
+    BpWords<4> xv[U], gv[U], yv[U];
+    unsigned mb[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      xv[u] = ld_pack<T, V>(reverse ? xe - (v + u * stride) * V : x + (v + u * stride) * V);
-      if (BWD) {
-        gv[u] = ld_pack<T, V>(reverse ? ge - (v + u * stride) * V : dy + (v + u * stride) * V);
-        if (relu && !mask_from_x) yv[u] = ld_pack<T, V>(reverse ? ye - (v + u * stride) * V : y + (v + u * stride) * V);
+      const size_t at = reverse ? nvec - 1 - (v + u * stride) : v + u * stride;
+      xv[u] = bn_ld(x + at * V);
+      mb[u] = 0;
+      if constexpr (BWD) {
+        gv[u] = bn_ld(dy + at * V);
+        if constexpr (MASK == MASK_BITS) mb[u] = bits[at];
+        if constexpr (MASK == MASK_Y) yv[u] = bn_ld(y + at * V);
       }
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) accumulate(xv[u], gv[u], yv[u]);
-  }
-  for (; v < nvec; v += stride) {
-    Pack<T, V> xv = ld_pack<T, V>(reverse ? xe - v * V : x + v * V), gv, yv;
-    unsigned mb = 0;
-    if (BWD) {
-      gv = ld_pack<T, V>(reverse ? ge - v * V : dy + v * V);
-      if (relu && !mask_from_x) {
-        if (bits) mb = bits[reverse ? nvec - 1 - v : v];
-        else yv = ld_pack<T, V>(reverse ? ye - v * V : y + v * V);
-      }
-    }
-    accumulate(xv, gv, yv, mb);
+    for (int u = 0; u < U; ++u) accumulate(xv[u], gv[u], yv[u], mb[u]);
+  };
+  size_t v = T0;
+  for (; v + (kBnReduceU - 1) * stride < nvec; v += kBnReduceU * stride) pass(v, std::integral_constant<int, kBnReduceU>());
+  for (; v < nvec; v += stride) pass(v, std::integral_constant<int, 1>());
+  if constexpr (BWD) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) b[k] *= invstd[cv * V + k];
   }
   __shared__ float s[kBnThreads][2 * V + 1];
 #pragma unroll
@@ -188,10 +231,9 @@ __global__ void __launch_bounds__(1024) bn_finalize_bwd_kernel(const float* __re
   if (acc_gamma) acc_gamma[c] += s2;
 }
 
-// BITS: also write the ReLU mask byte of every vector (residual layers only; a template parameter so
-// that the other layers keep 32 registers and eight resident blocks)
-template <typename T, int V, bool BITS>
-__global__ void __launch_bounds__(kBnThreads) bn_apply_fwd_kernel(
+// RES: a residual is added.  BITS: also write the ReLU mask byte of every vector (residual layers only).
+template <typename T, int V, bool RES, bool BITS>
+__global__ void __launch_bounds__(kBnThreads, 5) bn_apply_fwd_kernel(
     const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y, const float* __restrict__ gamma,
     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ invstd,
     unsigned char* __restrict__ bits, size_t nvec, int C, int relu) {
@@ -206,66 +248,95 @@ __global__ void __launch_bounds__(kBnThreads) bn_apply_fwd_kernel(
     sc[k] = invstd[c] * gamma[c];
     sh[k] = beta[c] - mean[c] * sc[k];
   }
-  for (size_t v = T0; v < nvec; v += stride) {
-    Pack<T, V> xv = ld_pack<T, V>(x + v * V), rv, out;
-    unsigned mb = 0;
-    if (res) rv = ld_pack<T, V>(res + v * V);
+  auto pass = [&](size_t v, auto count) {
+    constexpr int U = decltype(count)::value;
+    BpWords<4> xv[U], rv[U];
 #pragma unroll
-    for (int k = 0; k < V; ++k) {
-      float z = (float)to_acc<T>(xv.v[k]) * sc[k] + sh[k];
-      if (res) z += (float)to_acc<T>(rv.v[k]);
-      if (relu) z = fmaxf(z, 0.f);
-      out.v[k] = from_acc<T>((typename AccOf<T>::type)z);
-      if (BITS && (float)to_acc<T>(out.v[k]) > 0.f) mb |= 1u << k;     // what `y > 0` would read back
+    for (int u = 0; u < U; ++u) {
+      xv[u] = bn_ld(x + (v + u * stride) * V);
+      if constexpr (RES) rv[u] = bn_ld(res + (v + u * stride) * V);
     }
-    st_pack<T, V>(y + v * V, out);
-    if (BITS) bits[v] = (unsigned char)mb;
-  }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float out[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        float z = bp_get<T>(xv[u], k) * sc[k] + sh[k];
+        if constexpr (RES) z += bp_get<T>(rv[u], k);
+        if (relu) z = fmaxf(z, 0.f);
+        out[k] = z;
+      }
+      const BpWords<4> o = bp_put<T, V>(out);
+      bp_st(y + (v + u * stride) * V, o);
+      if (BITS) {
+        unsigned mb = 0;
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+          if (bp_get<T>(o, k) > 0.f) mb |= 1u << k;        // what `y > 0` would read back
+        bits[v + u * stride] = (unsigned char)mb;
+      }
+    }
+  };
+  size_t v = T0;
+  for (; v + (kBnApplyU - 1) * stride < nvec; v += kBnApplyU * stride) pass(v, std::integral_constant<int, kBnApplyU>());
+  for (; v < nvec; v += stride) pass(v, std::integral_constant<int, 1>());
 }
 
-template <typename T, int V, bool MASKX>
-__global__ void __launch_bounds__(kBnThreads, 4) bn_apply_bwd_kernel(
+// DRES: the residual's gradient, the masked dy, is written too.
+template <typename T, int V, int MASK, bool DRES>
+__global__ void __launch_bounds__(kBnThreads, 3) bn_apply_bwd_kernel(
     const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx,
     T* __restrict__ dres, const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean,
     const float* __restrict__ invstd, const float* __restrict__ dgamma, const float* __restrict__ dbeta,
-    const unsigned char* __restrict__ bits, size_t nvec, int C, int relu, float inv_m) {
+    const unsigned char* __restrict__ bits, size_t nvec, int C, float inv_m) {
   const int cvn = C / V;
   const size_t T0 = (size_t)blockIdx.x * kBnThreads + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * kBnThreads;
   const int cv = (int)(T0 % cvn);
-  constexpr bool mask_from_x = MASKX;
-  float mu[V], is[V], k1[V], k2[V], k3[V], sh[V];
+  float mu[V], k1[V], k2[V], k3[V], sh[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     const int c = cv * V + k;
-    mu[k] = mean[c]; is[k] = invstd[c];
-    k1[k] = gamma[c] * is[k];            // dx = k1 * (dz - k2 - xhat * k3); also the forward scale
+    const float is = invstd[c];
+    mu[k] = mean[c];
+    k1[k] = gamma[c] * is;               // dx = k1 * (dz - k2 - (x - mean) * k3); also the forward scale
     k2[k] = dbeta[c] * inv_m;
-    k3[k] = dgamma[c] * inv_m;
-    sh[k] = mask_from_x ? beta[c] - mu[k] * k1[k] : 0.f;
+    k3[k] = is * dgamma[c] * inv_m;
+    sh[k] = MASK == MASK_X ? beta[c] - mu[k] * k1[k] : 0.f;
   }
-  for (size_t v = T0; v < nvec; v += stride) {
-    Pack<T, V> xv = ld_pack<T, V>(x + v * V), gv = ld_pack<T, V>(dy + v * V), yv, ox, orr;
-    unsigned mb = 0;
-    if (relu && !mask_from_x) {
-      if (bits) mb = bits[v];
-      else yv = ld_pack<T, V>(y + v * V);
+  auto pass = [&](size_t v, auto count) {
+    constexpr int U = decltype(count)::value;
+    BpWords<4> xv[U], gv[U], yv[U];
+    unsigned mb[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t at = v + u * stride;
+      xv[u] = bn_ld(x + at * V);
+      gv[u] = bn_ld(dy + at * V);
+      mb[u] = 0;
+      if constexpr (MASK == MASK_BITS) mb[u] = bits[at];
+      if constexpr (MASK == MASK_Y) yv[u] = bn_ld(y + at * V);
     }
 #pragma unroll
-    for (int k = 0; k < V; ++k) {
-      float g = (float)to_acc<T>(gv.v[k]);
-      if (mask_from_x) {
-        if (!((float)to_acc<T>(xv.v[k]) * k1[k] + sh[k] > 0.f)) g = 0.f;
-      } else if (relu) {
-        if (bits ? !((mb >> k) & 1u) : !((float)to_acc<T>(yv.v[k]) > 0.f)) g = 0.f;
+    for (int u = 0; u < U; ++u) {
+      float ox[V], og[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const float f = bp_get<T>(xv[u], k);
+        float g = bp_get<T>(gv[u], k);
+        if (MASK == MASK_X && !(f * k1[k] + sh[k] > 0.f)) g = 0.f;
+        if (MASK == MASK_BITS && !((mb[u] >> k) & 1u)) g = 0.f;
+        if (MASK == MASK_Y && !(bp_get<T>(yv[u], k) > 0.f)) g = 0.f;
+        ox[k] = k1[k] * (g - k2[k] - (f - mu[k]) * k3[k]);
+        og[k] = g;
       }
-      float xhat = ((float)to_acc<T>(xv.v[k]) - mu[k]) * is[k];
-      ox.v[k] = from_acc<T>((typename AccOf<T>::type)(k1[k] * (g - k2[k] - xhat * k3[k])));
-      orr.v[k] = from_acc<T>((typename AccOf<T>::type)g);
+      bp_st(dx + (v + u * stride) * V, bp_put<T, V>(ox));
+      if constexpr (DRES) bp_st(dres + (v + u * stride) * V, bp_put<T, V>(og));
     }
-    st_pack<T, V>(dx + v * V, ox);
-    if (dres) st_pack<T, V>(dres + v * V, orr);
-  }
+  };
+  size_t v = T0;
+  for (; v + (kBnApplyU - 1) * stride < nvec; v += kBnApplyU * stride) pass(v, std::integral_constant<int, kBnApplyU>());
+  for (; v < nvec; v += stride) pass(v, std::integral_constant<int, 1>());
 }
 
 static int bn_check(int64_t rows, int C, int V) {
@@ -283,27 +354,23 @@ static int bn_fwd_t(const void* x, const void* res, void* y, const float* gamma,
   int st = bn_check(rows, C, V);
   if (st) return st;
   size_t nvec = (size_t)rows * (C / V);
-  int grid = bn_grid(nvec);
+  int grid = bn_grid(nvec, kBnMaxGrid, kBnReduceU);
   const int reverse = tunable("bn_reverse_stats") != 0;
   if (training) {
     // given_rows > 0: the producer of x (a convolution epilogue) has left that many rows of partial sums in scratch
     if (given_rows > 0) grid = given_rows;
     else
-    bn_reduce_kernel<T, V, false, false><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                                     nullptr, nvec, C, 0, reverse, (float*)scratch);
+    bn_reduce_kernel<T, V, false, MASK_NONE><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                                     nullptr, nvec, C, reverse, (float*)scratch);
     float m = (float)rows;
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
                                                            rows > 1 ? m / (m - 1.f) : 1.f, eps, momentum, smean, sinv,
                                                            rmean, rvar);
   }
-  // the apply pass keeps no partials and needs 32 registers: eight blocks per SM
-  const int apply_grid = (int)std::max<size_t>(1, std::min<size_t>((nvec + kBnThreads - 1) / kBnThreads, 2 * kBnMaxGrid));
-  if (bits)
-    bn_apply_fwd_kernel<T, V, true><<<apply_grid, kBnThreads, 0, s>>>((const T*)x, (const T*)res, (T*)y, gamma, beta, smean, sinv,
-                                                                      (unsigned char*)bits, nvec, C, relu);
-  else
-    bn_apply_fwd_kernel<T, V, false><<<apply_grid, kBnThreads, 0, s>>>((const T*)x, (const T*)res, (T*)y, gamma, beta, smean, sinv,
-                                                                       nullptr, nvec, C, relu);
+  const int apply_grid = bn_grid(nvec, kBnApplyGrid, kBnApplyU);
+  const auto apply = bits ? (res ? bn_apply_fwd_kernel<T, V, true, true> : bn_apply_fwd_kernel<T, V, false, true>)
+                          : (res ? bn_apply_fwd_kernel<T, V, true, false> : bn_apply_fwd_kernel<T, V, false, false>);
+  apply<<<apply_grid, kBnThreads, 0, s>>>((const T*)x, (const T*)res, (T*)y, gamma, beta, smean, sinv, (unsigned char*)bits, nvec, C, relu);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn forward launch: %s", cudaGetErrorString(e));
 }
@@ -318,23 +385,22 @@ static int bn_bwd_t(const void* x, const void* y, const void* dy, void* dx, void
   if (relu && !y && !bits && (!beta || dres))
     return fail(TMPI_ERR_INVALID, "bn backward: without y or mask bits the layer needs beta and no residual");
   size_t nvec = (size_t)rows * (C / V);
-  int grid = bn_grid(nvec);
+  const int grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU), apply_grid = bn_grid(nvec, kBnApplyBwdGrid, kBnApplyU);
   const int reverse = tunable("bn_reverse_stats") != 0;
-  const bool maskx = relu && !y && !bits;
   const unsigned char* mb = (const unsigned char*)bits;
-  if (maskx)
-    bn_reduce_kernel<T, V, true, true><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, (const T*)dy, smean, sinv, gamma, beta, nullptr,
-                                                                   nvec, C, relu, reverse, (float*)scratch);
-  else
-    bn_reduce_kernel<T, V, true, false><<<grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, smean, sinv, gamma, beta, mb,
-                                                                    nvec, C, relu, reverse, (float*)scratch);
-  bn_finalize_bwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, dgamma, dbeta, acc_gamma, acc_beta);
-  if (maskx)
-    bn_apply_bwd_kernel<T, V, true><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, (const T*)dy, (T*)dx, (T*)dres, gamma, beta,
-                                                                smean, sinv, dgamma, dbeta, nullptr, nvec, C, relu, 1.f / (float)rows);
-  else
-    bn_apply_bwd_kernel<T, V, false><<<grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, (T*)dx, (T*)dres, gamma, beta,
-                                                                 smean, sinv, dgamma, dbeta, mb, nvec, C, relu, 1.f / (float)rows);
+  auto passes = [&](auto mode) {
+    constexpr int MASK = decltype(mode)::value;
+    bn_reduce_kernel<T, V, true, MASK><<<grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, smean, sinv, gamma, beta, mb, nvec,
+                                                                   C, reverse, (float*)scratch);
+    bn_finalize_bwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, dgamma, dbeta, acc_gamma, acc_beta);
+    const auto apply = dres ? bn_apply_bwd_kernel<T, V, MASK, true> : bn_apply_bwd_kernel<T, V, MASK, false>;
+    apply<<<apply_grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, (T*)dx, (T*)dres, gamma, beta, smean, sinv, dgamma,
+                                            dbeta, mb, nvec, C, 1.f / (float)rows);
+  };
+  if (!relu) passes(std::integral_constant<int, MASK_NONE>());
+  else if (bits) passes(std::integral_constant<int, MASK_BITS>());
+  else if (y) passes(std::integral_constant<int, MASK_Y>());
+  else passes(std::integral_constant<int, MASK_X>());
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn backward launch: %s", cudaGetErrorString(e));
 }
@@ -384,44 +450,6 @@ __device__ __forceinline__ void bp_item(long long t, int cvn, const BpDims& d, i
   *ow = (int)(r - q * d.OW);
   *n = (int)(q / strips);
   *strip = (int)(q - (long long)*n * strips);
-}
-
-// A pack of NW 32-bit words (8 or 16 bytes), elements taken out and put in by shifts and pair conversions (element-wise
-// structs cost a register per 16-bit element here and spilled).
-template <int NW> struct BpWords { uint32_t w[NW]; };
-template <int NW> __device__ __forceinline__ BpWords<NW> bp_ld(const void* p) {
-  if constexpr (NW == 4) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    return BpWords<NW>{{u.x, u.y, u.z, u.w}};
-  } else {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);
-    return BpWords<NW>{{u.x, u.y}};
-  }
-}
-template <int NW> __device__ __forceinline__ void bp_st(void* p, const BpWords<NW>& b) {
-  if constexpr (NW == 4) *reinterpret_cast<uint4*>(p) = make_uint4(b.w[0], b.w[1], b.w[2], b.w[3]);
-  else *reinterpret_cast<uint2*>(p) = make_uint2(b.w[0], b.w[1]);
-}
-template <typename T, int NW> __device__ __forceinline__ float bp_get(const BpWords<NW>& b, int c) {
-  if constexpr (sizeof(T) == 4) return __uint_as_float(b.w[c]);
-  else if constexpr (std::is_same<T, __nv_bfloat16>::value) return __uint_as_float((c & 1) ? b.w[c >> 1] & 0xffff0000u : b.w[c >> 1] << 16);
-  else return __half2float(__ushort_as_half((unsigned short)((c & 1) ? b.w[c >> 1] >> 16 : b.w[c >> 1])));
-}
-// from V floats
-template <typename T, int V> __device__ __forceinline__ BpWords<V * sizeof(T) / 4> bp_put(const float (&f)[V]) {
-  BpWords<V * sizeof(T) / 4> b;
-#pragma unroll
-  for (int k = 0; k < (int)(V * sizeof(T) / 4); ++k) {
-    if constexpr (sizeof(T) == 4) b.w[k] = __float_as_uint(f[k]);
-    else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
-      b.w[k] = *reinterpret_cast<uint32_t*>(&h);
-    } else {
-      __half2 h = __floats2half2_rn(f[2 * k], f[2 * k + 1]);
-      b.w[k] = *reinterpret_cast<uint32_t*>(&h);
-    }
-  }
-  return b;
 }
 
 // A window whose maximum is 0 passes no gradient (the ReLU under it is closed everywhere), so its index names no
@@ -739,9 +767,9 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, 
   if (st) return st;
   if (training) {
     size_t nvec = (size_t)rows * (C / V);
-    int grid = bn_grid(nvec);
-    bn_reduce_kernel<T, V, false, false><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                                     nullptr, nvec, C, 0, tunable("bn_reverse_stats") != 0, (float*)scratch);
+    const int grid = bn_grid(nvec, kBnMaxGrid, kBnReduceU);
+    bn_reduce_kernel<T, V, false, MASK_NONE><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                                                     nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
     float m = (float)rows;
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
                                                            rows > 1 ? m / (m - 1.f) : 1.f, eps, momentum, smean, sinv, rmean, rvar);
