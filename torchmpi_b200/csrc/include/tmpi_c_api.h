@@ -283,6 +283,8 @@ int tmpi_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, in
                   int pad, float* stats, int* stat_rows, void* stream);
 int tmpi_conv_dgrad(const void* dy, const void* w, void* dx, const void* add, int N, int H, int W, int Cin, int Cout, int R,
                     int S, int stride, int pad, void* stream);
+int tmpi_conv_dgrad_masked(const void* dy, const void* w, void* dx, const void* add, const void* add_bits, int N, int H, int W, int Cin,
+                           int Cout, int R, int S, int stride, int pad, void* stream);
 size_t tmpi_conv_wgrad_workspace_bytes(int N, int H, int W, int Cin, int Cout, int R, int S, int stride, int pad);
 int tmpi_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                     int stride, int pad, void* workspace, size_t workspace_bytes, int accumulate, void* stream);

@@ -19,8 +19,7 @@
 // stages, the weight is loaded once and stays resident while only the activation streams.  The
 // epilogue warps work independently (own staging tile, no barrier between warps), two tiles drain at a
 // time.  Epilogues:
-//   store    bf16 rows: each warp transposes its 32 x 64 slice through a swizzled staging tile and
-//            writes full 128-byte lines; optionally the per-channel sum and sum of squares of the
+//   store    bf16 rows: each warp converts its 32 x 64 slice into a swizzled staging tile for a TMA store; optionally the per-channel sum and sum of squares of the
 //            stored values (the batch statistics of the batch-norm that follows, accumulated per lane
 //            in registers over all tiles of the CTA and written as one partial row per CTA: no atomics,
 //            fixed order), and optionally
@@ -51,17 +50,18 @@ constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, MAX_STAGES = 12, TMEM_CO
 constexpr int EPI_WARPS = 8, THREADS = 32 * (2 + EPI_WARPS);
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int CHUNK_BYTES = 64 * BK * 2;                      // one 64 x 64 box of an MN-major operand
-constexpr int SLICE = 64, WARP_STAGING_BYTES = 32 * SLICE * 2, STAGING_BYTES = EPI_WARPS * WARP_STAGING_BYTES;
+constexpr int SLICE = 64, WARP_STAGING_BYTES = 32 * SLICE * 2;
+constexpr int RING = 2, STAGING_BYTES = EPI_WARPS * RING * WARP_STAGING_BYTES;      // staging tiles of each epilogue warp
 constexpr size_t SMEM_LIMIT = 232448;
 constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 512 /*barriers*/ + STAGING_BYTES;
 constexpr unsigned long long kWaitBudgetNs = 4000000000ull;
 
 enum { A_TILED = 0, A_IM2COL = 1, A_MN = 2 };
 enum { B_K = 0, B_MN = 2, B_MN_IM2COL = 3 };
-enum { EPI_STATS = 1, EPI_ADD = 2, EPI_SPLITK = 4 };
+enum { EPI_STATS = 1, EPI_ADD = 2, EPI_SPLITK = 4, EPI_ADD_BITS = 8 };
 
 struct Shared {
-  uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], b_full;
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], b_full, add_full[EPI_WARPS][RING];
   uint32_t tmem_base;
   int error;
 };
@@ -85,9 +85,8 @@ struct Problem {
   int b_block_bytes;           // bytes of one K block of B (mma_n * 128)
   int stat_bytes;              // shared-memory bytes of the statistics accumulators ([warp][2][BN] floats) or 0
   float* stats;                // EPI_STATS: [gridDim.x][2][N] partial sums
-  const __nv_bfloat16* add;    // EPI_ADD: [M, N] row-major tensor added to the product
+  const unsigned char* add_bits;   // EPI_ADD_BITS: one bit per element of add, eight columns to a byte; where it is 0, nothing is added
   float* workspace;            // EPI_SPLITK: [tile][slice][BM][mma_n] fp32
-  __nv_bfloat16* out;          // store epilogue: [M, N] row-major result
   int* status;
 };
 
@@ -227,16 +226,54 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
   for (int e = 0; e < 4; ++e) { f[2 * e] = __uint_as_float(w[e] << 16); f[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
 }
 
-// bf16 rows (+ statistics, + added tensor).  Every warp works on its own: it reads its 32 accumulator
-// rows 64 columns at a time, converts them into its staging tile (32 rows x 128 bytes, swizzled so that
-// both the row-wise writes and the line-wise reads are conflict free), reads the tile back line by line
-// - eight lanes per 128-byte row, four rows per instruction - and stores full lines.  The same read
-// feeds the column sums.  Group g (four warps, one per lane quarter) drains accumulator g, so two tiles
-// are in the epilogue at any time and no barrier between warps sits in the loop.
-template <bool do_stats, bool do_add>
-__device__ void epilogue_store(Shared* sh, unsigned char* stg, float* stats_all, const Problem& p, int ew, int quarter, int lane) {
+// Two half words, each the sign of one byte of a or b (selector digits 8 - 11 and 12 - 15) spread over 16 bits: the mask of a
+// pair of elements, under which a masked one is the +0 that an unmasked tensor would hold.
+__device__ __forceinline__ uint32_t sign_halves(uint32_t a, uint32_t b, uint32_t selector) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(selector));
+  return r;
+}
+
+// Slices (32 rows x 64 columns) of one epilogue warp, in the order in which it takes them; slices below the matrix are left out.
+struct SliceCursor {
+  int it, m_blk, n_blk, sl, slices;
+  bool live;
+  __device__ __forceinline__ void tile(const Problem& p, int quarter) {
+    int slice;
+    for (;; it += 2) {
+      live = item(p, it, &m_blk, &n_blk, &slice);
+      if (!live) return;
+      if (m_blk * BM + quarter * 32 < p.M) break;
+    }
+    sl = 0;
+    slices = (min(p.mma_n, p.N - n_blk * BN) + SLICE - 1) / SLICE;
+  }
+  __device__ __forceinline__ void next(const Problem& p, int quarter) {
+    if (++sl == slices) { it += 2; tile(p, quarter); }
+  }
+};
+
+// bf16 rows (+ statistics, + added tensor).  Every warp works on its own: it reads its 32 accumulator rows 64 columns at a
+// time, converts them into a staging tile (32 rows x 128 bytes, swizzled) and gives that to the TMA unit to store.  For the
+// column sums it reads the tile back line by line (eight lanes per row).  Group g (four warps, one per lane quarter) drains
+// accumulator g, so two tiles are in the epilogue at any time and no barrier between warps sits in the loop.
+//
+// A second gradient comes through the same staging tiles: a TMA load brings the next slice while one is being added to.  With add_bits it is the gradient
+// of a residual add followed by a ReLU, read as the incoming gradient and its mask in place of a tensor that batch-norm's
+// backward would write for this kernel alone.
+//
+// Bound by memory where the warps keep up: two per scheduler, so the instructions and waits of a slice count.  With lines
+// stored, and the second gradient loaded, from registers in the slice that used them, 256 x 28 x 28, 128 -> 512 channels took
+// 122 us with a second gradient, where the bytes take 71 at the copy rate; 76 now, 83 under mask bits (whose batch-norm pass
+// writes one tensor less: 135 -> 101), and 50 -> 48 without.  Four staging tiles per warp in place of two: no faster, and
+// slower where their shared memory is missing for operands in flight (256 x 7 x 7, 512 -> 2048: 46 against 36).
+template <bool do_stats, bool do_add, bool do_bits>
+__device__ void epilogue_store(Shared* sh, unsigned char* staging, float* stats_all, const Problem& p, const CUtensorMap* map_out,
+                               const CUtensorMap* map_add, int ew, int quarter, int lane) {
   const int group = ew >> 2;                      // ew: index of this warp among the epilogue warps
   const int chunk = lane & 7, rsub = lane >> 3;
+  unsigned char* ring = staging + (size_t)ew * RING * WARP_STAGING_BYTES;
+  uint64_t* add_full = sh->add_full[ew];
   // Running column sums of this lane (packed fp32 pairs) for the 8 columns of its chunk in each of the four
   // 64-column slices of a tile.  The CTA always visits the same n_blk (the grid is a multiple of tiles_n), so
   // the columns stay the same over all its tiles and the sums live in registers until the kernel ends.
@@ -245,63 +282,115 @@ __device__ void epilogue_store(Shared* sh, unsigned char* stg, float* stats_all,
   for (int sl = 0; sl < 4; ++sl)
 #pragma unroll
     for (int e = 0; e < 4; ++e) { cs2[sl][e] = 0ull; cq2[sl][e] = 0ull; }
-  int m_blk, n_blk, slice;
-  for (int it = group; item(p, it, &m_blk, &n_blk, &slice); it += 2) {
-    const uint32_t acc_phase = (it >> 1) & 1;
-    if (!sm100::mbar_wait(&sh->acc_full[group], acc_phase, kWaitBudgetNs) || sh->error) { fail(sh, p, 5); break; }
-    sm100::tc_fence_after();
-    const int row0 = m_blk * BM + quarter * 32;
-    const uint32_t t_base = sh->tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)group * BN;
+
+  SliceCursor ahead{};                            // the next slice of the second gradient to be loaded
+  int loads = 0, done = 0;                        // slices loaded and finished so far
+  auto load_add = [&]() {
+    if (!ahead.live) return;
+    if (lane == 0) {
+      uint64_t* bar = &add_full[loads % RING];
+      sm100::mbar_expect_tx(bar, WARP_STAGING_BYTES);
+      sm100::tma_load_2d(ring + (loads % RING) * WARP_STAGING_BYTES, map_add, ahead.n_blk * BN + ahead.sl * SLICE,
+                         ahead.m_blk * BM + quarter * 32, bar);
+    }
+    ++loads;
+    ahead.next(p, quarter);
+  };
+  // mask bits of row `lane` in a tile: eight bytes per slice, read one tile ahead (a slice of a row is a quarter of a sector)
+  uint2 bits[BN / SLICE];
+  auto load_bits = [&](int it) {
+    int m, n, unused;
+    const bool live = item(p, it, &m, &n, &unused);
+    const int row = m * BM + quarter * 32 + lane;
 #pragma unroll
     for (int sl = 0; sl < BN / SLICE; ++sl) {
-      const int c0 = sl * SLICE;
-      const int col0 = n_blk * BN + c0;
-      if (c0 < p.mma_n && col0 < p.N) {
-        // the second gradient, read line by line like the store (the eight loads fly while the accumulator is converted)
-        uint4 av[8];
-        if (do_add) {
-          const __nv_bfloat16* addp = p.add + (size_t)row0 * p.N + col0 + chunk * 8;
+      bits[sl] = make_uint2(0u, 0u);
+      if (live && row < p.M && n * BN + sl * SLICE < p.N)
+        bits[sl] = __ldg(reinterpret_cast<const uint2*>(p.add_bits + (((size_t)row * p.N + n * BN) >> 3)) + sl);
+    }
+  };
+  if (do_add) {
+    ahead.it = group;
+    ahead.tile(p, quarter);
+    load_add();
+    if (do_bits) load_bits(group);
+  }
+  int m_blk, n_blk, slice;
+  bool ok = true;
+  for (int it = group; ok && item(p, it, &m_blk, &n_blk, &slice); it += 2) {
+    const uint32_t acc_phase = (it >> 1) & 1;
+    ok = __all_sync(~0u, sm100::mbar_wait(&sh->acc_full[group], acc_phase, kWaitBudgetNs) && !sh->error);
+    if (!ok) { fail(sh, p, 5); break; }
+    sm100::tc_fence_after();
+    const int row0 = m_blk * BM + quarter * 32;
+    const int slices = row0 < p.M ? (min(p.mma_n, p.N - n_blk * BN) + SLICE - 1) / SLICE : 0;
+    const uint32_t t_base = sh->tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)group * BN;
+    uint2 tile_bits[BN / SLICE] = {};
+    if (do_bits) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rw = i * 4 + rsub;
-            av[i] = row0 + rw < p.M ? __ldg(reinterpret_cast<const uint4*>(addp + (size_t)rw * p.N)) : make_uint4(0, 0, 0, 0);
-          }
-        }
+      for (int sl = 0; sl < BN / SLICE; ++sl) tile_bits[sl] = bits[sl];
+      load_bits(it + 2);
+    }
+#pragma unroll
+    for (int sl = 0; sl < BN / SLICE; ++sl) {
+      if (ok && sl < slices) {
+        const int c0 = sl * SLICE;
+        unsigned char* stg = ring + (done % RING) * WARP_STAGING_BYTES;
         uint32_t r[2][32];
         sm100::tmem_ld_32x32(t_base + c0, r[0]);
         sm100::tmem_ld_32x32(t_base + c0 + 32, r[1]);
-        sm100::tmem_ld_wait();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            __nv_bfloat162 h0 = __floats2bfloat162_rn(__uint_as_float(r[h][j]), __uint_as_float(r[h][j + 1]));
-            __nv_bfloat162 h1 = __floats2bfloat162_rn(__uint_as_float(r[h][j + 2]), __uint_as_float(r[h][j + 3]));
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(r[h][j + 4]), __uint_as_float(r[h][j + 5]));
-            __nv_bfloat162 h3 = __floats2bfloat162_rn(__uint_as_float(r[h][j + 6]), __uint_as_float(r[h][j + 7]));
-            uint4 u;
-            u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
-            u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
-            const int ck = h * 4 + j / 8;
-            *reinterpret_cast<uint4*>(stg + (size_t)lane * 128 + ((ck ^ (lane & 7)) << 4)) = u;
-          }
+        // the staging tile that is written next has been stored: this slice's, or with a second gradient the next slice's
+        if (lane == 0) {
+          if (do_add) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        }
+        if (do_add) {
+          load_add();
+          ok = __all_sync(~0u, sm100::mbar_wait(&add_full[done % RING], (done / RING) & 1, kWaitBudgetNs) && !sh->error);
+          if (!ok) fail(sh, p, 8);
         }
         __syncwarp();
-        __nv_bfloat16* out = p.out + (size_t)row0 * p.N + col0 + chunk * 8;
+        sm100::tmem_ld_wait();
+        unsigned char* row = stg + (size_t)lane * 128;
+        uint32_t shift[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rw = i * 4 + rsub;
-          uint4 u = *reinterpret_cast<const uint4*>(stg + (size_t)rw * 128 + ((chunk ^ (rw & 7)) << 4));
-          if (row0 + rw < p.M) {
-            if (do_add) {                       // bf16(product) + it, as a separate accumulation kernel would compute
-              __nv_bfloat162* uu = reinterpret_cast<__nv_bfloat162*>(&u);
-              const __nv_bfloat162* aa = reinterpret_cast<const __nv_bfloat162*>(&av[i]);
+        for (int ck = 0; ck < 8; ++ck) {
+          if (do_bits && (ck & 3) == 0) {
+            // shift[s]: the bit of element 8 q + 7 - s of these 32 becomes the sign of byte q
+            const uint32_t half = ck ? tile_bits[sl].y : tile_bits[sl].x;
 #pragma unroll
-              for (int e = 0; e < 4; ++e) uu[e] = __hadd2(uu[e], aa[e]);
-            }
-            *reinterpret_cast<uint4*>(out + (size_t)rw * p.N) = u;
+            for (int s = 0; s < 8; ++s) shift[s] = half << s;
           }
-          if (do_stats) {                       // rows past M hold zeros
+          uint4* cell = reinterpret_cast<uint4*>(row + ((ck ^ (lane & 7)) << 4));
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[ck >> 2][(ck & 3) * 8 + 2 * e]), __uint_as_float(r[ck >> 2][(ck & 3) * 8 + 2 * e + 1]));
+            w[e] = *reinterpret_cast<uint32_t*>(&h);
+          }
+          if (do_add) {                           // bf16(product) + it, as a separate accumulation kernel would compute
+            const uint4 u = *cell;
+            uint32_t av[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (do_bits) av[e] &= sign_halves(shift[7 - 2 * e], shift[6 - 2 * e], (8 + (ck & 3)) * 0x11 | (12 + (ck & 3)) * 0x1100);
+              __nv_bfloat162 h = __hadd2(*reinterpret_cast<__nv_bfloat162*>(&w[e]), *reinterpret_cast<__nv_bfloat162*>(&av[e]));
+              w[e] = *reinterpret_cast<uint32_t*>(&h);
+            }
+          }
+          *cell = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        sm100::fence_proxy_async_smem();          // generic-proxy writes to shared memory -> visible to the TMA unit
+        __syncwarp();
+        if (lane == 0) {
+          if (ok) sm100::tma_store_2d(map_out, stg, n_blk * BN + c0, row0);        // rows beyond the matrix are clipped
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        if (do_stats) {                           // rows past M hold zeros
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rw = i * 4 + rsub;
+            const uint4 u = *reinterpret_cast<const uint4*>(stg + (size_t)rw * 128 + ((chunk ^ (rw & 7)) << 4));
             const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -311,14 +400,17 @@ __device__ void epilogue_store(Shared* sh, unsigned char* stg, float* stats_all,
               asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(cq2[sl][e]) : "l"(f2));
             }
           }
+          __syncwarp();                           // read by all before lane 0 lets the tile be written again
         }
-        __syncwarp();                           // the staging tile is rewritten by the next slice
+        ++done;
       }
     }
     sm100::tc_fence_before();
     __syncwarp();
     if (lane == 0) sm100::mbar_arrive(&sh->acc_empty[group]);
   }
+  // the tiles have been read before the CTA gives its shared memory back; the writes themselves complete with the kernel
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   if (do_stats) {
     // once per kernel: add the four row groups of the warp (lanes l, l + 8, l + 16, l + 24 hold the same
     // columns), park the warp's sums in shared memory, then add the eight warps in a fixed order
@@ -390,7 +482,8 @@ __device__ void epilogue_splitk(Shared* sh, const Problem& p, int group, int qua
 // EPI: the epilogue flags as a template parameter, so that each flavour carries only its own registers
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
-conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Problem p) {
+conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                 const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_add, const Problem p) {
   extern __shared__ unsigned char smem_raw[];
   const uintptr_t base = ((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023;
   unsigned char* tiles = (unsigned char*)base;
@@ -405,6 +498,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     for (int s = 0; s < p.stages; ++s) { sm100::mbar_init(&sh->full[s], 1); sm100::mbar_init(&sh->empty[s], 1); }
     for (int a = 0; a < 2; ++a) { sm100::mbar_init(&sh->acc_full[a], 1); sm100::mbar_init(&sh->acc_empty[a], 4); }
     sm100::mbar_init(&sh->b_full, 1);
+    for (int e = 0; e < EPI_WARPS * RING; ++e) sm100::mbar_init(&sh->add_full[0][0] + e, 1);
     sh->error = 0;
     sm100::fence_barrier_init();
   }
@@ -425,8 +519,8 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   } else if constexpr ((EPI & EPI_SPLITK) != 0) {
     epilogue_splitk(sh, p, (warp - 2) >> 2, warp & 3, lane);
   } else {
-    epilogue_store<(EPI & EPI_STATS) != 0, (EPI & EPI_ADD) != 0>(sh, staging + (size_t)(warp - 2) * WARP_STAGING_BYTES, stats, p,
-                                                              warp - 2, warp & 3, lane);
+    epilogue_store<(EPI & EPI_STATS) != 0, (EPI & EPI_ADD) != 0, (EPI & EPI_ADD_BITS) != 0>(
+        sh, staging, stats, p, &map_out, &map_add, warp - 2, warp & 3, lane);
   }
   __syncwarp();
   sm100::tc_fence_before();
@@ -562,17 +656,23 @@ static int* conv_status_word(int** host_out = nullptr) {
 }
 
 // Plans the shared memory (stages, resident weight) and launches.
-static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, conv::Problem& p, int* grid_out, cudaStream_t s) {
-  void (*kernel)(const CUtensorMap, const CUtensorMap, const conv::Problem) = nullptr;
+static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const void* out, const void* add, conv::Problem& p, int* grid_out,
+                       cudaStream_t s) {
+  void (*kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const conv::Problem) = nullptr;
   switch (p.epi) {
     case 0: kernel = conv::conv_gemm_kernel<0>; break;
     case conv::EPI_STATS: kernel = conv::conv_gemm_kernel<conv::EPI_STATS>; break;
     case conv::EPI_ADD: kernel = conv::conv_gemm_kernel<conv::EPI_ADD>; break;
+    case conv::EPI_ADD | conv::EPI_ADD_BITS: kernel = conv::conv_gemm_kernel<conv::EPI_ADD | conv::EPI_ADD_BITS>; break;
     case conv::EPI_SPLITK: kernel = conv::conv_gemm_kernel<conv::EPI_SPLITK>; break;
     default: return fail(TMPI_ERR_INVALID, "conv: unsupported epilogue combination %d", p.epi);
   }
   cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv::SMEM_LIMIT);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "conv: shared memory attribute: %s", cudaGetErrorString(ae));
+  CUtensorMap mo = ma, md = ma;                  // output and second gradient: slices of 32 rows x 64 columns
+  int st;
+  if (out && (st = make_tmap_bf16(&mo, out, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.N, 32))) return st;
+  if (add && (st = make_tmap_bf16(&md, add, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.N, 32))) return st;
   p.status = conv_status_word();
   p.b_block_bytes = p.mma_n * conv::BK * 2;
   p.stat_bytes = (p.epi & conv::EPI_STATS) ? conv::EPI_WARPS * 2 * conv::BN * (int)sizeof(float) : 0;
@@ -594,7 +694,7 @@ static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, conv::Probl
   // statistics: a CTA keeps sums for one window of 256 columns, so every tile it visits must have the same n_blk
   if ((p.epi & conv::EPI_STATS) && grid % p.tiles_n) grid -= grid % p.tiles_n;
   if (grid_out) *grid_out = grid;
-  kernel<<<grid, conv::THREADS, smem, s>>>(ma, mb, p);
+  kernel<<<grid, conv::THREADS, smem, s>>>(ma, mb, mo, md, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "conv launch: %s", cudaGetErrorString(e));
 }
@@ -659,7 +759,6 @@ int tmpi_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, in
   p.mma_n = std::min(conv::BN, (Cout + 15) / 16 * 16);
   if ((st = make_tmap_bf16(&mb, w, (uint64_t)Cout, (uint64_t)R * S * Cin, (uint64_t)R * S * Cin, (uint32_t)p.mma_n))) return st;
   if ((uintptr_t)y & 15) return fail(TMPI_ERR_INVALID, "conv: output must be 16-byte aligned");
-  p.out = (__nv_bfloat16*)y;
   p.tiles_m = (int)((M + conv::BM - 1) / conv::BM);
   p.tiles_n = (Cout + conv::BN - 1) / conv::BN;
   p.taps = R * S; p.S = S; p.cblocks = Cin / conv::BK; p.Cb = Cin;
@@ -668,13 +767,14 @@ int tmpi_conv_fwd(const void* x, const void* w, void* y, int N, int H, int W, in
   p.Ho = g.Ho; p.Wo = g.Wo; p.stride = stride; p.pad = pad;
   p.epi = stats ? conv::EPI_STATS : 0;
   p.stats = stats;
-  return conv_launch(ma, mb, p, stat_rows, (cudaStream_t)stream);
+  return conv_launch(ma, mb, y, nullptr, p, stat_rows, (cudaStream_t)stream);
 }
 
 // dx[N, H, W, Cin] = gradient of the stride-1 convolution above with respect to x, given dy[N, Ho, Wo, Cout];
-// add (nullable): a tensor shaped like dx that is added to the result (a second gradient into the same activation).
-int tmpi_conv_dgrad(const void* dy, const void* w, void* dx, const void* add, int N, int H, int W, int Cin, int Cout, int R,
-                    int S, int stride, int pad, void* stream) {
+// add (nullable): a tensor shaped like dx that is added to the result (a second gradient into the same activation);
+// add_bits (nullable): a mask for it, one byte per eight channels as tmpi_bn_relu_fwd writes it.
+int tmpi_conv_dgrad_masked(const void* dy, const void* w, void* dx, const void* add, const void* add_bits, int N, int H, int W, int Cin,
+                           int Cout, int R, int S, int stride, int pad, void* stream) {
   const Geom g = geom(N, H, W, Cin, Cout, R, S, stride, pad);
   int st = check_geom(g, "conv dgrad");
   if (st) return st;
@@ -691,16 +791,21 @@ int tmpi_conv_dgrad(const void* dy, const void* w, void* dx, const void* add, in
   p.mma_n = std::min(conv::BN, Cin);
   if ((st = make_tmap_bf16(&mb, w, (uint64_t)Cout, (uint64_t)R * S * Cin, (uint64_t)R * S * Cin, 64))) return st;
   if (((uintptr_t)dx | (uintptr_t)add) & 15) return fail(TMPI_ERR_INVALID, "conv: gradients must be 16-byte aligned");
-  p.out = (__nv_bfloat16*)dx;
   p.tiles_m = (int)((M + conv::BM - 1) / conv::BM);
   p.tiles_n = (Cin + conv::BN - 1) / conv::BN;
   p.taps = R * S; p.S = S; p.cblocks = Cout / conv::BK; p.Cb = Cin; p.flip = 1;
   p.k_blocks_total = p.taps * p.cblocks; p.k_per_slice = p.k_blocks_total; p.slices = 1;
   p.a_mode = plain ? conv::A_TILED : conv::A_IM2COL; p.b_mode = conv::B_MN;
   p.Ho = H; p.Wo = W; p.stride = 1; p.pad = bpad;    // the walk is over the pixels of dx
-  p.epi = add ? conv::EPI_ADD : 0;
-  p.add = (const __nv_bfloat16*)add;
-  return conv_launch(ma, mb, p, nullptr, (cudaStream_t)stream);
+  p.epi = add ? conv::EPI_ADD | (add_bits ? conv::EPI_ADD_BITS : 0) : 0;
+  p.add_bits = (const unsigned char*)add_bits;
+  if ((uintptr_t)add_bits & 7) return fail(TMPI_ERR_INVALID, "conv: mask bits must be 8-byte aligned");
+  return conv_launch(ma, mb, dx, add, p, nullptr, (cudaStream_t)stream);
+}
+
+int tmpi_conv_dgrad(const void* dy, const void* w, void* dx, const void* add, int N, int H, int W, int Cin, int Cout, int R,
+                    int S, int stride, int pad, void* stream) {
+  return tmpi_conv_dgrad_masked(dy, w, dx, add, nullptr, N, H, W, Cin, Cout, R, S, stride, pad, stream);
 }
 
 // Split of the K dimension (the pixels, for a weight gradient) of a [Mrows, Ncols] product over P rows of K.
@@ -755,7 +860,7 @@ int tmpi_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, int W
   p.Ho = g.Ho; p.Wo = g.Wo; p.stride = stride; p.pad = pad;
   p.epi = conv::EPI_SPLITK;
   p.workspace = (float*)workspace;
-  if ((st = conv_launch(ma, mb, p, nullptr, (cudaStream_t)stream))) return st;
+  if ((st = conv_launch(ma, mb, nullptr, nullptr, p, nullptr, (cudaStream_t)stream))) return st;
   return launch_splitk_reduce(p, workspace, dw, accumulate, (cudaStream_t)stream);
 }
 
@@ -788,7 +893,7 @@ int tmpi_gemm_bf16_tn_splitk(const void* A, const void* B, void* C, int M, int N
   p.Ho = p.Wo = 1; p.stride = 1;
   p.epi = conv::EPI_SPLITK;
   p.workspace = (float*)workspace;
-  if ((st = conv_launch(ma, mb, p, nullptr, (cudaStream_t)stream))) return st;
+  if ((st = conv_launch(ma, mb, nullptr, nullptr, p, nullptr, (cudaStream_t)stream))) return st;
   return launch_splitk_reduce(p, workspace, C, accumulate, (cudaStream_t)stream);
 }
 

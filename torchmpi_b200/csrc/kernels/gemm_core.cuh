@@ -194,10 +194,6 @@ __device__ __forceinline__ void epilogue(Shared* sh, const Problem& p, int quart
 // DestMap(m_blk, &map, &row0) picks the destination tensor map (box 64 columns x 128 rows) and the
 // first row inside it.  Rows and columns beyond the tensor are clipped by the TMA unit.
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(map), "r"(sm100::smem_u32(smem_src)), "r"(c0), "r"(c1) : "memory");
-}
 
 // Release(acc) is called by one lane of each of the four warps once the accumulator is drained.
 template <typename Sh, typename TileOrder, typename DestMap, typename Release>
@@ -265,7 +261,7 @@ __device__ __forceinline__ void epilogue_tma_impl(Sh* sh, unsigned char* staging
       sm100::fence_proxy_async();        // generic-proxy writes to shared memory -> visible to the TMA unit
       epi_bar_sync();
       if (leader && cmap) {
-        tma_store_2d(cmap, stg, col0, row0);
+        sm100::tma_store_2d(cmap, stg, col0, row0);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
     }

@@ -239,7 +239,7 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
           *reinterpret_cast<uint4*>(stg_row + ((u ^ (row & 7)) << 4)) = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
         sm100::fence_proxy_async_smem();       // generic-proxy writes to shared memory -> visible to the TMA unit
         group_sync(group);
-        if (store) gemm::tma_store_2d(map, stg, col0, row0);
+        if (store) sm100::tma_store_2d(map, stg, col0, row0);
         if (leader) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       };
       put(map_c, 0);

@@ -100,10 +100,12 @@ class _BnReluFn(torch.autograd.Function):
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
-        dres = torch.empty_like(x, memory_format=torch.channels_last) if ctx.has_res else None
+        # the first of several consumers of the residual parks its gradient for the last one's kernel: as dy and the mask bits
+        masked = ctx.has_res and bits is not None and ctx.res_fork is not None and ctx.res_fork.parks_first()
+        dres = torch.empty_like(x, memory_format=torch.channels_last) if ctx.has_res and not masked else None
         dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
         dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
-        from ..parallel.flat_buckets import direct_grad, grad_written
+        from ..parallel.flat_buckets import MaskedGrad, direct_grad, grad_written
         acc_g = acc_b = None
         if ctx.params is not None and has_symbol("tmpi_bn_relu_bwd_acc"):
             acc_g, acc_b = direct_grad(ctx.params[0]), direct_grad(ctx.params[1])
@@ -121,8 +123,10 @@ class _BnReluFn(torch.autograd.Function):
             grad_written(ctx.params[0])
             grad_written(ctx.params[1])
             dgamma = dbeta = None
-        if dres is not None and ctx.res_fork is not None:
-            dres = ctx.res_fork.offer(lambda add: dres if add is None else dres.add_(add))
+        if masked:
+            ctx.res_fork.offer(lambda add: MaskedGrad(dy, bits))
+        elif dres is not None and ctx.res_fork is not None:
+            dres = ctx.res_fork.offer(lambda add: dres if add is None else dres.add_(add.tensor() if isinstance(add, MaskedGrad) else add))
         return dx, dres, dgamma, dbeta, None, None, None, None, None, None, None, None, None
 
 

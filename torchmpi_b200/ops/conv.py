@@ -65,13 +65,15 @@ def conv_forward(x, w, stride, pad, stats: Optional[torch.Tensor] = None):
     return y, rows.value
 
 
-def conv_dgrad(dy, w, x_shape, stride, pad, add: Optional[torch.Tensor] = None):
+def conv_dgrad(dy, w, x_shape, stride, pad, add: Optional[torch.Tensor] = None, add_bits: Optional[torch.Tensor] = None):
+    """``add`` is added to the gradient; with ``add_bits`` (one bit per element, eight channels to a byte) where its bit is set."""
     global launch_count
     N, Cin, H, W = x_shape
     Cout, _, R, S = w.shape
     dx = torch.empty(x_shape, dtype=dy.dtype, device=dy.device, memory_format=torch.channels_last)
-    check(lib.tmpi_conv_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), add.data_ptr() if add is not None else None,
-                              N, H, W, Cin, Cout, R, S, stride, pad, stream_ptr()))
+    check(lib.tmpi_conv_dgrad_masked(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), add.data_ptr() if add is not None else None,
+                                     add_bits.data_ptr() if add_bits is not None else None,
+                                     N, H, W, Cin, Cout, R, S, stride, pad, stream_ptr()))
     launch_count += 1
     return dx
 
@@ -144,10 +146,14 @@ class _ConvFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
         dy = _cl(dy)
-        from ..parallel.flat_buckets import direct_grad, grad_written
+        from ..parallel.flat_buckets import MaskedGrad, direct_grad, grad_written
         dx = dw = None
         if ctx.needs_input_grad[0]:
             def make_dx(add):
+                if isinstance(add, MaskedGrad):
+                    if ctx.stride == 1 and add.grad.shape == x.shape and add.grad.dtype == x.dtype and add.grad.data_ptr() % 16 == 0:
+                        return conv_dgrad(dy, w, x.shape, 1, ctx.pad, add=add.grad, add_bits=add.bits)
+                    add = add.tensor()
                 if ctx.stride == 1:
                     return conv_dgrad(dy, w, x.shape, 1, ctx.pad, add=_cl(add) if add is not None else None)
                 # strided input gradients stay on the library

@@ -40,6 +40,21 @@ def _dense(p: torch.Tensor) -> bool:
         (p.dim() == 5 and p.is_contiguous(memory_format=torch.channels_last_3d))
 
 
+class MaskedGrad:
+    """A gradient of a residual that has not been written: the (channels-last) incoming gradient where the ReLU's mask bit is set.
+    The kernel that adds it reads both, which saves writing and reading a tensor of this size."""
+
+    def __init__(self, grad: torch.Tensor, bits: torch.Tensor):
+        self.grad, self.bits = grad, bits
+
+    def tensor(self) -> torch.Tensor:
+        N, C, H, W = self.grad.shape
+        per = N * C * H * W // self.bits.numel()                             # elements of a byte
+        shift = torch.arange(per, device=self.bits.device, dtype=torch.uint8)
+        on = (self.bits[:, None] >> shift & 1).view(N, H, W, C).permute(0, 3, 1, 2)
+        return torch.where(on.bool(), self.grad, torch.zeros((), dtype=self.grad.dtype, device=self.grad.device))
+
+
 class GradFork:
     """Sums the gradients that several consumers send into one activation without a separate add kernel.
 
@@ -52,8 +67,13 @@ class GradFork:
     def __init__(self, consumers: int):
         self.consumers, self.seen, self.parked = consumers, 0, None
 
+    def parks_first(self) -> bool:
+        """Whether the next offer is the first of several: it may then be a ``MaskedGrad``."""
+        return self.seen == 0 and self.consumers > 1
+
     def offer(self, make_grad):
-        """``make_grad(add)`` returns this consumer's gradient, plus ``add`` when ``add`` is not None."""
+        """``make_grad(add)`` returns this consumer's gradient, plus ``add`` (a tensor, or the ``MaskedGrad`` that the first
+        consumer parked) when ``add`` is not None."""
         self.seen += 1
         g = make_grad(self.parked)
         if self.seen < self.consumers:
