@@ -1,0 +1,58 @@
+"""Causal attention whose items are shared by the two teams of a CTA, against fp64."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape):
+    return torch.randn(*shape, device="cuda").to(torch.bfloat16)
+
+
+def _attention64(qkv, heads):
+    B, T, C3 = qkv.shape
+    q, k, v = (t.reshape(B, T, heads, 64).transpose(1, 2) for t in qkv.split(C3 // 3, dim=2))
+    s = (q @ k.transpose(-1, -2)) * 0.125
+    s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device=qkv.device).triu(1), -math.inf)
+    return (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B, T, C3 // 3)
+
+
+# one to sixteen key blocks per item; fewer items than CTAs, one to two and more rounds of items shared by two teams
+@pytest.mark.parametrize("B,T,H", [(1, 128, 1), (1, 256, 3), (1, 384, 1), (1, 640, 2), (1, 1920, 4), (1, 2048, 16), (3, 1024, 12), (2, 2048, 11)])
+def test_attention_items_shared_by_teams(B, T, H):
+    from torchmpi_b200.ops import attention
+    torch.manual_seed(T + H)
+    qkv = _rand(B, T, 3 * H * 64)
+    qkv[0, T // 3, : H * 64] *= 8.0                        # one query whose weights lie far apart
+    qkv.requires_grad_(True)
+    y = attention.causal_attention(qkv, H)
+    dy = _rand(B, T, H * 64)
+    y.backward(dy)
+    x = qkv.detach().double().requires_grad_(True)
+    ref = _attention64(x, H)
+    ref.backward(dy.double())
+    # probabilities in bf16: 2^-9 of sums of order one each way; the gradient's products twice
+    assert ((y.double() - ref).norm() / ref.norm()) < 5e-3
+    assert (y.double() - ref).abs().max() < 3e-2
+    assert ((qkv.grad.double() - x.grad).norm() / x.grad.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("T", [256, 1024])
+def test_attention_shared_items_non_finite(T):
+    """A key that scores -inf weighs nothing wherever the split lies; NaN and +inf reach the rows that see them, and no others."""
+    from torchmpi_b200.ops import attention
+    torch.manual_seed(1)
+    for value, at in ((-math.inf, T - 3), (math.nan, T // 2 + 5), (math.inf, 70)):
+        qkv = _rand(1, T, 192)
+        qkv[:, :, 0] = 1.0                                  # first query coordinate: the key's decides the score
+        qkv[0, at, 64] = value
+        with torch.no_grad():
+            y = attention.causal_attention(qkv, 1)
+        assert torch.isfinite(y[0, :at]).all()
+        if value == -math.inf:
+            ref = _attention64(torch.cat([qkv[..., :64], qkv[..., 64:128].nan_to_num(neginf=-1e30), qkv[..., 128:]], -1).double(), 1)
+            assert torch.isfinite(y).all() and (y.double() - ref)[0].abs().max() < 3e-2
+        else:
+            assert torch.isnan(y[0, at:]).all()

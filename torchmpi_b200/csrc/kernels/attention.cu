@@ -61,13 +61,15 @@ constexpr int TILE_BYTES = 128 * D * 2;                       // a 128 x 64 bf16
 constexpr int Q_OFF = 0, K_OFF = 2 * TILE_BYTES, V_OFF = 4 * TILE_BYTES, SMEM_TILES = 6 * TILE_BYTES;
 constexpr int SMEM_SHARED = 256;                              // the teams' barrier blocks follow their tiles
 constexpr int XCH_BYTES = 2 * 2 * BQ * 4;                     // two phases x two halves of the rows: values the halves exchange
-constexpr int SMEM_BYTES = TEAMS * (SMEM_TILES + SMEM_SHARED + XCH_BYTES);
+constexpr int MERGE_BYTES = 2 * BQ * 4;                       // team 1's row maxima and sums of an item that the teams share
+constexpr int SMEM_BYTES = TEAMS * (SMEM_TILES + SMEM_SHARED + XCH_BYTES) + MERGE_BYTES;
 constexpr int TMEM_COLS = 256, TMEM_P = 128, TMEM_O = 192;    // S: columns 0-127 of a team, P (bf16 pairs): 128-191, O: 192-255
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
   uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_full, pv_done, o_empty;
   uint64_t pair[4];            // the two warps that share 32 rows meet here (bounded, unlike a named barrier)
+  uint64_t merge_full, merge_empty;      // of team 1, where the teams share items: its row sums are there, have been read
   uint32_t tmem_base;
   int error;
 };
@@ -99,26 +101,42 @@ __device__ __forceinline__ void stamp(const Params& p, int round, int j, int ev)
   if (p.trace && blockIdx.x == 0 && round == 0 && team() == 0) p.trace[j * 16 + ev] = sm100::now_ns();
 }
 
-// The item of this team in a round: (batch, head) and query block, long ones (late query blocks) first, every other
-// round in reverse so that a team that got a long item gets a short one next.
-__device__ __forceinline__ bool item(const Params& p, int round, int* bh, int* qblk) {
-  const int g = TEAMS * (int)gridDim.x, i = (int)blockIdx.x + team() * (int)gridDim.x;
-  const long long t = (long long)round * g + ((round & 1) ? g - 1 - i : i);
-  if (t >= p.items) return false;
-  const int n = p.B * p.H;
-  *qblk = p.q_blocks - 1 - (int)(t / n);
-  *bh = (int)(t % n);
-  return true;
-}
+// The items of a team one after the other: (batch, head), query block and the key blocks [first, end) of it that are the
+// team's.  Long items (late query blocks) first, every other round in reverse so that a team that got a long item gets a short
+// one next.  SHARED: the CTA is the unit; team 0 takes the first half of an item's key blocks, team 1 the rest up to the
+// diagonal (nothing of an item of one block).
+template <bool SHARED> struct Items {
+  int round = -1, qblk, first, end;
+  __device__ __forceinline__ long long index(const Params& p) const {
+    const int g = SHARED ? (int)gridDim.x : TEAMS * (int)gridDim.x;
+    const int i = (int)blockIdx.x + (SHARED ? 0 : team() * (int)gridDim.x);
+    return (long long)round * g + ((round & 1) ? g - 1 - i : i);
+  }
+  __device__ __forceinline__ int bh(const Params& p) const { return (int)(index(p) % (p.B * p.H)); }
+  __device__ __forceinline__ bool next(const Params& p) {
+    do {
+      ++round;
+      const long long t = index(p);
+      if (t >= p.items) return false;
+      qblk = p.q_blocks - 1 - (int)(t / (p.B * p.H));
+      const int half = (qblk + 2) >> 1;
+      first = SHARED && team() ? half : 0;
+      end = SHARED && !team() ? half : qblk + 1;
+    } while (first == end);
+    return true;
+  }
+};
 
 #define ATTN_WAIT(bar, parity, where) \
   do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
 
+template <bool SHARED>
 __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
                          const CUtensorMap* mv) {
-  int kc = 0, vc = 0, bh, qblk;                            // K and V tiles loaded so far, over all items
-  for (int r = 0; item(p, r, &bh, &qblk); ++r) {
-    const int b = bh / p.H, h = bh - b * p.H, row0 = b * p.T;
+  int kc = 0, vc = 0;                                      // K and V tiles loaded so far, over all items
+  Items<SHARED> it;
+  for (int r = 0; it.next(p); ++r) {
+    const int bh = it.bh(p), b = bh / p.H, h = bh - b * p.H, row0 = b * p.T;
     auto load_k = [&](int j) -> bool {
       const int st = kc & 1;
       if (kc >= 2 && (!sm100::mbar_wait(&sh->k_empty[st], ((kc >> 1) - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
@@ -129,10 +147,10 @@ __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, cons
     };
     if (r >= 2) ATTN_WAIT(&sh->q_empty[r & 1], ((r >> 1) - 1) & 1, 12);
     sm100::mbar_expect_tx(&sh->q_full[r & 1], TILE_BYTES);
-    sm100::tma_load_2d(tiles + Q_OFF + (r & 1) * TILE_BYTES, mq, h * D, row0 + qblk * BQ, &sh->q_full[r & 1]);
-    if (!load_k(0)) { fail(sh, p, 1); return; }
-    for (int j = 0; j <= qblk; ++j) {
-      if (j < qblk && !load_k(j + 1)) { fail(sh, p, 1); return; }          // K runs one block ahead of V
+    sm100::tma_load_2d(tiles + Q_OFF + (r & 1) * TILE_BYTES, mq, h * D, row0 + it.qblk * BQ, &sh->q_full[r & 1]);
+    if (!load_k(it.first)) { fail(sh, p, 1); return; }
+    for (int j = it.first; j < it.end; ++j) {
+      if (j + 1 < it.end && !load_k(j + 1)) { fail(sh, p, 1); return; }          // K runs one block ahead of V
       const int st = vc & 1;
       if (vc >= 2) ATTN_WAIT(&sh->v_empty[st], ((vc >> 1) - 1) & 1, 13);
       sm100::mbar_expect_tx(&sh->v_full[st], TILE_BYTES);
@@ -142,6 +160,7 @@ __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, cons
   }
 }
 
+template <bool SHARED>
 __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
   const uint32_t tmem_s = sh->tmem_base, tmem_p = sh->tmem_base + TMEM_P, tmem_o = sh->tmem_base + TMEM_O;
   constexpr uint32_t idesc_s = sm100::make_idesc_f16(BQ, BKV, true);            // Q and K both K-major
@@ -152,10 +171,9 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
   // a slice further into shared memory only adds to the address field (bytes / 16 in the low 14 bits)
   auto at = [](uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); };
   int g = 0;                                               // key blocks whose S has been issued, over all items
-  int bh, qblk;
-  // S of key block j of round r (block number g): waits for the softmax warps to have read the previous S
-  auto issue_s = [&](int r, int j, int last) -> bool {
-    if (j == 0 && (!sm100::mbar_wait(&sh->q_full[r & 1], (r >> 1) & 1, kWaitBudgetNs) || sh->error)) return false;
+  // S of a key block of this team's r-th item (block number g): waits for the softmax warps to have read the previous S
+  auto issue_s = [&](int r, bool first, bool last) -> bool {
+    if (first && (!sm100::mbar_wait(&sh->q_full[r & 1], (r >> 1) & 1, kWaitBudgetNs) || sh->error)) return false;
     if (!sm100::mbar_wait(&sh->k_full[g & 1], (g >> 1) & 1, kWaitBudgetNs) || sh->error) return false;
     if (g >= 1 && (!sm100::mbar_wait(&sh->s_empty, (g - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
     sm100::tc_fence_after();
@@ -165,25 +183,26 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
       sm100::umma_f16(tmem_s, at(a, k * UMMA_K * 2), at(b, k * UMMA_K * 2), idesc_s, k > 0 ? 1u : 0u);
     sm100::umma_commit(&sh->s_full);
     sm100::umma_commit(&sh->k_empty[g & 1]);
-    if (j == last) sm100::umma_commit(&sh->q_empty[r & 1]);
+    if (last) sm100::umma_commit(&sh->q_empty[r & 1]);
     ++g;
     return true;
   };
-  bool more = item(p, 0, &bh, &qblk);
-  if (more && !issue_s(0, 0, qblk)) { fail(sh, p, 3); return; }
+  Items<SHARED> it;
+  bool more = it.next(p);
+  if (more && !issue_s(0, true, it.end - it.first == 1)) { fail(sh, p, 3); return; }
   int v = 0;                                               // P V products issued so far
   for (int r = 0; more; ++r) {
-    const int last = qblk;
-    more = item(p, r + 1, &bh, &qblk);                     // the next round's item: its first S runs before this one's last P V
-    for (int j = 0; j <= last; ++j) {
+    const int first = it.first, last = it.end - 1;
+    more = it.next(p);                                     // the next item: its first S runs before this one's last P V
+    for (int j = first; j <= last; ++j) {
       if (j < last) {
         stamp(p, r, j, 8);
-        if (!issue_s(r, j + 1, last)) { fail(sh, p, 4); return; }
+        if (!issue_s(r, false, j + 1 == last)) { fail(sh, p, 4); return; }
         stamp(p, r, j, 9);
       } else if (more) {
-        if (!issue_s(r + 1, 0, qblk)) { fail(sh, p, 5); return; }
+        if (!issue_s(r + 1, true, it.end - it.first == 1)) { fail(sh, p, 5); return; }
       }
-      if (j == 0 && r > 0) ATTN_WAIT(&sh->o_empty, (r - 1) & 1, 14);       // the previous item's output has been read
+      if (j == first && r > 0) ATTN_WAIT(&sh->o_empty, (r - 1) & 1, 14);       // the previous item's output has been read
       ATTN_WAIT(&sh->p_full, v & 1, 6);
       stamp(p, r, j, 10);
       ATTN_WAIT(&sh->v_full[v & 1], (v >> 1) & 1, 15);
@@ -192,7 +211,7 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
       const uint64_t b = at(dv, (v & 1) * TILE_BYTES);
 #pragma unroll
       for (int k = 0; k < BKV / UMMA_K; ++k)               // 16 keys: eight columns of packed P, 16 rows of V
-        sm100::umma_f16_tmem_a(tmem_o, tmem_p + k * (UMMA_K / 2), at(b, k * UMMA_K * 128), idesc_o, (j | k) ? 1u : 0u);
+        sm100::umma_f16_tmem_a(tmem_o, tmem_p + k * (UMMA_K / 2), at(b, k * UMMA_K * 128), idesc_o, (j > first || k) ? 1u : 0u);
       sm100::umma_commit(&sh->pv_done);
       sm100::umma_commit(&sh->v_empty[v & 1]);
       stamp(p, r, j, 12);
@@ -220,14 +239,15 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint32_t (&w)
 
 // Two threads per query row: `half` picks 64 of the 128 scores of a block and 32 of the 64 output columns.  The halves
 // exchange their maxima through shared memory, block by block, and their row sums at the end of an item.
-__device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarter, int half, int lane) {
+template <bool SHARED>
+__device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2* merge, const Params& p, int quarter, int half, int lane) {
   const int row = quarter * 32 + lane;                     // the row of the tile; its tensor-memory lane
   const uint32_t tmem = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
   const uint32_t tmem_s = tmem + half * 64, tmem_p = tmem + TMEM_P + half * 32, tmem_o = tmem + TMEM_O + half * 32;
   const float c2 = p.scale_log2;
   const unsigned long long c2x2 = pack2(__float_as_uint(c2), __float_as_uint(c2));
   const bool tracer = row == 0 && half == 0;
-  int g = 0, met = 0, bh, qblk;                            // key blocks done and exchanges made so far, over all items
+  int g = 0, met = 0, merged = 0;                          // key blocks done, exchanges made and items merged so far
   // this row's value of the other half
   auto exchange = [&](float v, float* other) -> bool {
     float* x = xch + (met & 1) * 2 * BQ;
@@ -239,11 +259,12 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
     ++met;
     return true;
   };
-  for (int r = 0; item(p, r, &bh, &qblk); ++r) {
+  Items<SHARED> it;
+  for (int r = 0; it.next(p); ++r) {
     float m = -INFINITY;                                   // the running maximum
     unsigned long long sum2[2] = {0ull, 0ull};
-    for (int j = 0; j <= qblk; ++j, ++g) {
-      const bool diag = j == qblk;
+    for (int j = it.first; j < it.end; ++j, ++g) {
+      const bool diag = j == it.qblk;
       uint32_t s[2][32];
       if (tracer) stamp(p, r, j, 0);
       ATTN_WAIT(&sh->s_full, g & 1, 7);
@@ -280,7 +301,7 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
       if (tracer) stamp(p, r, j, 2);
       // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
       const float next = max_nan(m, mx);
-      const bool grew = j > 0 && __any_sync(~0u, next > m);
+      const bool grew = j > it.first && __any_sync(~0u, next > m);
       const float alpha = ex2((m - next) * c2);
       const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
       m = next;
@@ -299,7 +320,7 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
         }
         if (c == 0 && g > 0) {     // the previous block's product has read its P and added to O
           ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 8);
-          if (tracer && j > 0) { stamp(p, r, j - 1, 5); stamp(p, r, j - 1, 6); }
+          if (tracer && j > it.first) { stamp(p, r, j - 1, 5); stamp(p, r, j - 1, 6); }
           sm100::tc_fence_after();
         }
         sm100::tmem_st_32x16(tmem_p + c * 16, w);
@@ -330,18 +351,56 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
     float l0, l1, l_other;
     unpack2(add2(sum2[0], sum2[1]), l0, l1);
     if (!exchange(l0 + l1, &l_other)) return;
-    const float l = half ? l_other + (l0 + l1) : (l0 + l1) + l_other, inv = 1.f / l;
+    float l = half ? l_other + (l0 + l1) : (l0 + l1) + l_other;
+    const bool merges = SHARED && it.qblk > 0;
+    if (merges && team()) {                                // hand over O (in tensor memory), maximum and sum; go on
+      if (merged > 0) ATTN_WAIT(&sh->merge_empty, (merged - 1) & 1, 16);
+      if (half == 0) merge[row] = make_float2(m, l);
+      ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
+      sm100::tc_fence_after();
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&sh->merge_full);
+      ++merged;
+      continue;
+    }
     ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
-    if (tracer) stamp(p, r, qblk, 5);
+    if (tracer) stamp(p, r, it.qblk, 5);
     sm100::tc_fence_after();
     uint32_t o[32];
     sm100::tmem_ld_32x32(tmem_o, o);
     sm100::tmem_ld_wait();
+    if (merges) {
+      ATTN_WAIT(&other_team->merge_full, merged & 1, 17);
+      ++merged;
+      sm100::tc_fence_after();
+      const float2 with = merge[row];
+      const float next = max_nan(m, with.x);
+      const float a0 = ex2((m - next) * c2);
+      // keys that are all -inf weigh nothing, as if they came after the others in one pass
+      const bool none = with.x == -INFINITY;
+      const float a1 = none ? 0.f : ex2((with.x - next) * c2);
+      l = l * a0 + (none ? 0.f : with.y * a1);
+      m = next;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t o1[16];
+        sm100::tmem_ld_32x16(tmem_o + TMEM_COLS + q * 16, o1);
+        sm100::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          o[q * 16 + i] = __float_as_uint(__uint_as_float(o[q * 16 + i]) * a0 + (none ? 0.f : __uint_as_float(o1[i]) * a1));
+      }
+    }
+    const float inv = 1.f / l;
     sm100::tc_fence_before();
     __syncwarp();
-    if (lane == 0) sm100::mbar_arrive(&sh->o_empty);
-    const int b = bh / p.H, h = bh - b * p.H;
-    const size_t t = (size_t)qblk * BQ + row;
+    if (lane == 0) {
+      sm100::mbar_arrive(&sh->o_empty);
+      if (merges) { sm100::mbar_arrive(&other_team->o_empty); sm100::mbar_arrive(&other_team->merge_empty); }
+    }
+    const int bh = it.bh(p), b = bh / p.H, h = bh - b * p.H;
+    const size_t t = (size_t)it.qblk * BQ + row;
     __nv_bfloat16* out = p.out + ((size_t)b * p.T + t) * p.ld_out + h * D + half * 32;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -352,10 +411,13 @@ __device__ void softmax_rows(Shared* sh, float* xch, const Params& p, int quarte
       *reinterpret_cast<uint4*>(out + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (p.lse && half == 0) p.lse[(size_t)bh * p.T + t] = m * c2 * 0.6931471805599453f + __logf(l);
-    if (tracer) stamp(p, r, qblk, 6);
+    if (tracer) stamp(p, r, it.qblk, 6);
   }
 }
 
+// SHARED: both teams of a CTA work on each of its items, half of the key blocks each (see attention_shares).  A template
+// parameter: as an argument it cost the other form registers (8 x 16 x 1024 forward and backward 170 -> 174 us).
+template <bool SHARED>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const Params p) {
@@ -378,6 +440,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     sm100::mbar_init(&sh->pv_done, 1);
     sm100::mbar_init(&sh->o_empty, SOFTMAX_WARPS);
     for (int q = 0; q < 4; ++q) sm100::mbar_init(&sh->pair[q], 2);
+    sm100::mbar_init(&sh->merge_full, SOFTMAX_WARPS);
+    sm100::mbar_init(&sh->merge_empty, SOFTMAX_WARPS);
     sh->error = 0;
     sm100::fence_barrier_init();
   }
@@ -400,14 +464,16 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   } else if (warp < 4) {                                   // registers per four warps: 56 + 4 * 104 of the launch's 5 * 96
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp < 2) {
-      if (sm100::elect_one()) producer(sh, tiles, p, &map_q, &map_k, &map_v);
+      if (sm100::elect_one()) producer<SHARED>(sh, tiles, p, &map_q, &map_k, &map_v);
     } else {
-      if (sm100::elect_one()) mma_issuer(sh, tiles, p);
+      if (sm100::elect_one()) mma_issuer<SHARED>(sh, tiles, p);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     float* xch = (float*)(smem_raw + TEAMS * (SMEM_TILES + SMEM_SHARED) + team() * XCH_BYTES);
-    softmax_rows(sh, xch, p, warp & 3, ((warp - 4) >> 2) & 1, lane);
+    float2* merge = (float2*)(smem_raw + TEAMS * (SMEM_TILES + SMEM_SHARED + XCH_BYTES));
+    Shared* other_team = (Shared*)(smem_raw + TEAMS * SMEM_TILES + (team() ^ 1) * SMEM_SHARED);
+    softmax_rows<SHARED>(sh, other_team, xch, merge, p, warp & 3, ((warp - 4) >> 2) & 1, lane);
   }
   __syncwarp();
   sm100::tc_fence_before();
@@ -426,6 +492,30 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 }  // namespace attn
 
 static unsigned long long* g_attn_trace = nullptr;
+
+// Whether the teams of a CTA share its items.  The launch takes as long as its busiest team: the key blocks of its items and a
+// fixed part per item, Q and the first S before, the output after (about 1.5 blocks; 2 with a merge, and both teams pay it).
+// Sharing halves the longest item where there are few, and costs the fixed part twice where there are many: 1 x 16 x 2048
+// (256 items on 148 CTAs) 31.0 -> 26.9 us; 8 x 16 x 1024 (1024 items) stays with a team per item.
+static bool attention_shares(int items, int per_block, int q_blocks, int grid) {
+  const int teams = attn::TEAMS * grid;
+  if (items > 8 * teams) return false;                       // many items each are balanced as they are
+  auto busiest = [&](int units, bool shared) {               // in half blocks
+    int most = 0;
+    for (int i = 0; i < units; ++i) {
+      int sum = 0;
+      for (int round = 0;; ++round) {
+        const long long t = (long long)round * units + ((round & 1) ? units - 1 - i : i);
+        if (t >= items) break;
+        const int blocks = q_blocks - (int)(t / per_block);
+        sum += shared ? (blocks + 1) / 2 * 2 + 4 : blocks * 2 + 3;
+      }
+      most = std::max(most, sum);
+    }
+    return most;
+  };
+  return busiest(grid, true) < busiest(teams, false);
+}
 
 static int* attn_status_word(int** host_out = nullptr) {
   static int* dev_ptr = nullptr;
@@ -457,8 +547,6 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   if ((st = make_tmap_bf16(&mq, q, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mk, k, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mv, v, rows, cols, (uint64_t)ld_qkv, 128))) return st;
-  cudaError_t ae = cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
-  if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
   attn::Params p;
   p.B = B; p.T = T; p.H = H; p.q_blocks = T / attn::BQ;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -468,15 +556,19 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.items = B * H * p.q_blocks;
   // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
   const int grid = std::min(p.items, gemm_sm_count());
-  cudaError_t e = launch_overlapped(attn::attention_fwd_kernel, grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream, mq, mk, mv, p);
+  const bool shared = !p.trace && attention_shares(p.items, B * H, p.q_blocks, grid);      // a trace follows one team through an item
+  const auto kernel = shared ? attn::attention_fwd_kernel<true> : attn::attention_fwd_kernel<false>;
+  cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
+  if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
+  cudaError_t e = launch_overlapped(kernel, grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream, mq, mk, mv, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));
 }
 
 // Resident CTAs of the attention kernel per SM (1: a CTA holds two teams that overlap each other).
 int tmpi_attention_ctas_per_sm(void) {
   int n = 0;
-  cudaFuncSetAttribute(attn::attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn::attention_fwd_kernel, attn::THREADS, attn::SMEM_BYTES) != cudaSuccess) return -1;
+  cudaFuncSetAttribute(attn::attention_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn::attention_fwd_kernel<false>, attn::THREADS, attn::SMEM_BYTES) != cudaSuccess) return -1;
   return n;
 }
 
