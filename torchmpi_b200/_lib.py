@@ -203,6 +203,7 @@ _CUDA_PROTOS = {
     "tmpi_maxpool_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "tmpi_maxpool_bwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "tmpi_gemm_bf16_any": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_gelu": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_ex": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp]),
     "tmpi_gemm_status": (_i, []),
@@ -220,6 +221,7 @@ _CUDA_PROTOS = {
     "tmpi_attention_ctas_per_sm": (_i, []),
     "tmpi_attention_set_trace": (None, [_vp]),
     "tmpi_attention_status": (_i, []),
+    "tmpi_gemm_tn_prefers_splitk": (_i, [_i, _i, _i64]),
     "tmpi_gemm_tn_splitk_workspace_bytes": (_sz, [_i, _i, _i64]),
     "tmpi_gemm_bf16_tn_splitk": (_i, [_vp, _vp, _vp, _i, _i, _i64, _i64, _i64, _vp, _sz, _i, _vp]),
 }

@@ -67,9 +67,13 @@ bool pair_enabled() {
 // ---------------------------------------------------------------- linear
 Tensor matmul_nt(const Tensor& a_, const Tensor& b_, const Tensor& bias) {
   const Tensor a = a_.contiguous(), b = b_.contiguous(), c = bias.defined() ? bias.contiguous() : bias;
-  Tensor out = at::empty({a.size(0), b.size(0)}, a.options());
-  check(tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), c.defined() ? c.data_ptr() : nullptr, (int)a.size(0), (int)b.size(0),
-                       (int)a.size(1), c.defined() ? EPI_BIAS : 0, stream()));
+  const int M = (int)a.size(0), N = (int)b.size(0), K = (int)a.size(1), epi = c.defined() ? EPI_BIAS : 0;
+  Tensor out = at::empty({M, N}, a.options());
+  // few rows or columns: the pair kernel's narrow tiles, over more SMs
+  if ((M < 256 || N < 256) && M >= 1 && N >= 1 && K >= 1 && N % 8 == 0 && K % 8 == 0 && pair_enabled())
+    check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, c.defined() ? c.data_ptr() : nullptr, M, N, K, epi, stream()));
+  else
+    check(tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), c.defined() ? c.data_ptr() : nullptr, M, N, K, epi, stream()));
   launched(LINEAR, 1);
   return out;
 }
@@ -85,14 +89,14 @@ Tensor gelu_pass(const Tensor& z) {
 // (z, gelu(z)); one kernel where the CTA-pair GEMM applies
 std::pair<Tensor, Tensor> matmul_nt_gelu(const Tensor& a_, const Tensor& b_, const Tensor& bias) {
   const int64_t M = a_.size(0), N = b_.size(0), K = a_.size(1);
-  if (!(M >= 256 && N >= 256 && N % 8 == 0 && K % 8 == 0 && pair_enabled())) {
+  if (!(M >= 1 && N >= 1 && K >= 1 && N % 8 == 0 && K % 8 == 0 && pair_enabled())) {
     Tensor z = matmul_nt(a_, b_, bias);
     return {z, gelu_pass(z)};
   }
   const Tensor a = a_.contiguous(), b = b_.contiguous(), c = bias.defined() ? bias.contiguous() : bias;
   Tensor z = at::empty({M, N}, a.options()), y = at::empty({M, N}, a.options());
-  check(tmpi_gemm_bf16_gelu(a.data_ptr(), b.data_ptr(), z.data_ptr(), y.data_ptr(), c.defined() ? c.data_ptr() : nullptr, (int)M, (int)N,
-                            (int)K, stream()));
+  check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), z.data_ptr(), y.data_ptr(), c.defined() ? c.data_ptr() : nullptr, (int)M, (int)N,
+                           (int)K, c.defined() ? EPI_BIAS : 0, stream()));
   launched(LINEAR, 1);
   return {z, y};
 }
@@ -100,9 +104,9 @@ std::pair<Tensor, Tensor> matmul_nt_gelu(const Tensor& a_, const Tensor& b_, con
 Tensor matmul_nn(const Tensor& a_, const Tensor& b_) {
   const Tensor a = a_.contiguous(), b = b_.contiguous();
   const int64_t M = a.size(0), K = a.size(1), N = b.size(1);
-  if (!(M >= 256 && N >= 256 && N % 8 == 0 && K % 8 == 0 && pair_enabled())) return matmul_nt(a, b.t().contiguous(), Tensor());
+  if (!(M >= 1 && N % 8 == 0 && K % 8 == 0 && K >= 1 && pair_enabled())) return matmul_nt(a, b.t().contiguous(), Tensor());
   Tensor out = at::empty({M, N}, a.options());
-  check(tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K, B_IS_KN, stream()));
+  check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, nullptr, (int)M, (int)N, (int)K, B_IS_KN, stream()));
   launched(LINEAR, 1);
   return out;
 }
@@ -110,9 +114,16 @@ Tensor matmul_nn(const Tensor& a_, const Tensor& b_) {
 Tensor matmul_tn(const Tensor& a_, const Tensor& b_) {
   const Tensor a = a_.contiguous(), b = b_.contiguous();
   const int64_t K = a.size(0), M = a.size(1), N = b.size(1);
-  if (!(M >= 256 && N >= 256 && M % 8 == 0 && N % 8 == 0 && pair_enabled())) return matmul_nt(a.t().contiguous(), b.t().contiguous(), Tensor());
+  if (!(K >= 1 && M % 8 == 0 && N % 8 == 0 && pair_enabled())) return matmul_nt(a.t().contiguous(), b.t().contiguous(), Tensor());
   Tensor out = at::empty({M, N}, a.options());
-  check(tmpi_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K, A_IS_KM | B_IS_KN, stream()));
+  if (tmpi_gemm_tn_prefers_splitk((int)M, (int)N, K)) {       // few tiles, many rows: K over the SMs, fp32 partial tiles
+    const size_t need = tmpi_gemm_tn_splitk_workspace_bytes((int)M, (int)N, K);
+    const Tensor ws = at::empty({(int64_t)need}, a.options().dtype(at::kByte));
+    check(tmpi_gemm_bf16_tn_splitk(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, K, 0, 0, ws.data_ptr(), need, 0, stream()));
+    launched(LINEAR, 2);
+    return out;
+  }
+  check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, nullptr, (int)M, (int)N, (int)K, A_IS_KM | B_IS_KN, stream()));
   launched(LINEAR, 1);
   return out;
 }

@@ -304,6 +304,7 @@ int tmpi_attention_ctas_per_sm(void);
 void tmpi_attention_set_trace(void* device_buffer);   // tuning aid: phase time stamps of one CTA
 int tmpi_attention_status(void);
 // C[M, N] (+)= A^T B for A [K, M], B [K, N] with a long K and a small output (split over K; same kernel family)
+int tmpi_gemm_tn_prefers_splitk(int M, int N, int64_t K);
 size_t tmpi_gemm_tn_splitk_workspace_bytes(int M, int N, int64_t K);
 int tmpi_gemm_bf16_tn_splitk(const void* A, const void* B, void* C, int M, int N, int64_t K, int64_t lda, int64_t ldb,
                              void* workspace, size_t workspace_bytes, int accumulate, void* stream);
@@ -340,6 +341,8 @@ int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, 
 int tmpi_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                    int epilogue, void* stream);
 // Z = A B^T + bias and Y = gelu(Z) of the rounded Z in one kernel; M, N >= 256, N and K multiples of 8
+int tmpi_gemm_bf16_any(const void* A, const void* B, void* C, void* gelu_out, const void* bias, int M, int N, int K, int epilogue,
+                       void* stream);   // operands as stored, any size
 int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream);
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
