@@ -106,19 +106,15 @@ __device__ __forceinline__ void stamp(const Params& p, int round, int j, int ev)
 // one next.  SHARED: the CTA is the unit; team 0 takes the first half of an item's key blocks, team 1 the rest up to the
 // diagonal (nothing of an item of one block).
 template <bool SHARED> struct Items {
-  int round = -1, qblk, first, end;
-  __device__ __forceinline__ long long index(const Params& p) const {
-    const int g = SHARED ? (int)gridDim.x : TEAMS * (int)gridDim.x;
-    const int i = (int)blockIdx.x + (SHARED ? 0 : team() * (int)gridDim.x);
-    return (long long)round * g + ((round & 1) ? g - 1 - i : i);
-  }
-  __device__ __forceinline__ int bh(const Params& p) const { return (int)(index(p) % (p.B * p.H)); }
+  int round = -1, bh, qblk, first, end;
   __device__ __forceinline__ bool next(const Params& p) {
+    const unsigned g = SHARED ? gridDim.x : TEAMS * gridDim.x, i = blockIdx.x + (SHARED ? 0u : team() * gridDim.x), n = p.B * p.H;
     do {
       ++round;
-      const long long t = index(p);
-      if (t >= p.items) return false;
-      qblk = p.q_blocks - 1 - (int)(t / (p.B * p.H));
+      const unsigned t = round * g + ((round & 1) ? g - 1 - i : i);        // below 2^31 and one round more
+      if (t >= (unsigned)p.items) return false;
+      qblk = p.q_blocks - 1 - (int)(t / n);
+      bh = (int)(t % n);
       const int half = (qblk + 2) >> 1;
       first = SHARED && team() ? half : 0;
       end = SHARED && !team() ? half : qblk + 1;
@@ -136,7 +132,7 @@ __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, cons
   int kc = 0, vc = 0;                                      // K and V tiles loaded so far, over all items
   Items<SHARED> it;
   for (int r = 0; it.next(p); ++r) {
-    const int bh = it.bh(p), b = bh / p.H, h = bh - b * p.H, row0 = b * p.T;
+    const int b = it.bh / p.H, h = it.bh - b * p.H, row0 = b * p.T;
     auto load_k = [&](int j) -> bool {
       const int st = kc & 1;
       if (kc >= 2 && (!sm100::mbar_wait(&sh->k_empty[st], ((kc >> 1) - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
@@ -399,7 +395,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       sm100::mbar_arrive(&sh->o_empty);
       if (merges) { sm100::mbar_arrive(&other_team->o_empty); sm100::mbar_arrive(&other_team->merge_empty); }
     }
-    const int bh = it.bh(p), b = bh / p.H, h = bh - b * p.H;
+    const int b = it.bh / p.H, h = it.bh - b * p.H;
     const size_t t = (size_t)it.qblk * BQ + row;
     __nv_bfloat16* out = p.out + ((size_t)b * p.T + t) * p.ld_out + h * D + half * 32;
 #pragma unroll
@@ -410,7 +406,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
         w[i] = pack_bf16(__float_as_uint(__uint_as_float(o[u * 8 + 2 * i]) * inv), __float_as_uint(__uint_as_float(o[u * 8 + 2 * i + 1]) * inv));
       *reinterpret_cast<uint4*>(out + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    if (p.lse && half == 0) p.lse[(size_t)bh * p.T + t] = m * c2 * 0.6931471805599453f + __logf(l);
+    if (p.lse && half == 0) p.lse[(size_t)it.bh * p.T + t] = m * c2 * 0.6931471805599453f + __logf(l);
     if (tracer) stamp(p, r, it.qblk, 6);
   }
 }
@@ -496,7 +492,7 @@ static unsigned long long* g_attn_trace = nullptr;
 // Whether the teams of a CTA share its items.  The launch takes as long as its busiest team: the key blocks of its items and a
 // fixed part per item, Q and the first S before, the output after (about 1.5 blocks; 2 with a merge, and both teams pay it).
 // Sharing halves the longest item where there are few, and costs the fixed part twice where there are many: 1 x 16 x 2048
-// (256 items on 148 CTAs) 31.0 -> 26.9 us; 8 x 16 x 1024 (1024 items) stays with a team per item.
+// (256 items on 148 CTAs) 31.0 -> 25.4 us; 8 x 16 x 1024 (1024 items) stays with a team per item.
 static bool attention_shares(int items, int per_block, int q_blocks, int grid) {
   const int teams = attn::TEAMS * grid;
   if (items > 8 * teams) return false;                       // many items each are balanced as they are
