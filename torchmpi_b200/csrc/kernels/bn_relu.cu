@@ -87,7 +87,8 @@ constexpr int kBnReduceBwdGrid = 296, kBnApplyGrid = 740, kBnApplyBwdGrid = 444;
 
 // partial[(block * 2 + which) * C + c]
 // Where a backward pass takes the ReLU mask from (a template parameter: a choice at run time puts branches between the loads).
-enum { MASK_NONE = 0, MASK_X = 1 /* recomputed from x, gamma, beta */, MASK_BITS = 2, MASK_Y = 3 };
+enum { MASK_NONE = 0, MASK_X = 1 /* recomputed from x, gamma, beta */, MASK_BITS = 2, MASK_Y = 3, MASK_X_ROUNDED = 4 /* MASK_X, of the value rounded to T */ };
+__host__ __device__ constexpr bool bn_mask_from_x(int mask) { return mask == MASK_X || mask == MASK_X_ROUNDED; }
 
 template <typename T, int V, bool BWD, int MASK>
 __global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       mu[k] = mean[cv * V + k];
-      if constexpr (MASK == MASK_X) { sc[k] = invstd[cv * V + k] * gamma[cv * V + k]; sh[k] = beta[cv * V + k] - mu[k] * sc[k]; }
+      if constexpr (bn_mask_from_x(MASK)) { sc[k] = invstd[cv * V + k] * gamma[cv * V + k]; sh[k] = beta[cv * V + k] - mu[k] * sc[k]; }
     }
   }
   // bits (backward, ReLU layers with a residual): one byte per vector written by the forward apply
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
       } else {
         float g = bp_get<T>(gv, k);
         if (MASK == MASK_X && !(f * sc[k] + sh[k] > 0.f)) g = 0.f;
+        if (MASK == MASK_X_ROUNDED && !((float)to_acc<T>(from_acc<T>((typename AccOf<T>::type)(f * sc[k] + sh[k]))) > 0.f)) g = 0.f;
         if (MASK == MASK_BITS && !((mb >> k) & 1u)) g = 0.f;
         if (MASK == MASK_Y && !(bp_get<T>(yv, k) > 0.f)) g = 0.f;
         a[k] += g;
@@ -250,7 +252,8 @@ __global__ void __launch_bounds__(kBnThreads, 5) bn_apply_fwd_kernel(
   }
   auto pass = [&](size_t v, auto count) {
     constexpr int U = decltype(count)::value;
-    BpWords<4> xv[U], rv[U];
+    BpWords<4> xv[U];
+    [[maybe_unused]] BpWords<4> rv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       xv[u] = bn_ld(x + (v + u * stride) * V);
@@ -456,68 +459,51 @@ __device__ __forceinline__ void bp_item(long long t, int cvn, const BpDims& d, i
 // position: backward needs no mask of its own.
 constexpr uint32_t kBpNowhere = 255;
 
-// Running maximum of a window row with the position of the first maximum.  16-bit types: the rectified values are not
-// negative, so their bit patterns order like the values and one unsigned key holds (value, code) with larger codes for
-// earlier positions: a step is a byte permute and an integer maximum.  0 is "no position" (codes start at 1).
-template <typename T, int V, bool KEYS = sizeof(T) == 2>
-struct BpBest {
-  using Words = BpWords<V * sizeof(T) / 4>;
-  uint32_t key[V];
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int k = 0; k < V; ++k) key[k] = 0u;
-  }
-  __device__ __forceinline__ void take(const Words& a, uint32_t code) {        // code: 3, 2, 1 for kw = 0, 1, 2
-#pragma unroll
-    for (int k = 0; k < V; k += 2) {
-      key[k] = umax(key[k], __byte_perm(a.w[k / 2], code, 0x1054));
-      key[k + 1] = umax(key[k + 1], __byte_perm(a.w[k / 2], code, 0x3254));
+// One 32-bit word of rectified values (two of a 16-bit type, or one float): batch-norm and ReLU, maximum, and the elements that
+// are equal as a mask.  The values are not negative (no -0 either) and not NaN.
+template <typename T> struct BpWord {
+  static __device__ __forceinline__ uint32_t rectified(uint32_t x, const float* sc, const float* sh) {
+    if constexpr (sizeof(T) == 4) {
+      return __float_as_uint(fmaxf(__uint_as_float(x) * sc[0] + sh[0], 0.f));
+    } else {
+      const BpWords<1> w{{x}};
+      const float f[2] = {fmaxf(bp_get<T>(w, 0) * sc[0] + sh[0], 0.f), fmaxf(bp_get<T>(w, 1) * sc[1] + sh[1], 0.f)};
+      return bp_put<T, 2>(f).w[0];
     }
   }
-  __device__ __forceinline__ void merge(const BpBest& row, uint32_t kh_code) {      // kh_code: 6, 3, 0 for kh = 0, 1, 2
-#pragma unroll
-    for (int k = 0; k < V; ++k) key[k] = umax(key[k], row.key[k] + (row.key[k] ? kh_code : 0u));
+  static __device__ __forceinline__ uint32_t larger(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (sizeof(T) == 4) r = __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+    else if constexpr (std::is_same<T, __nv_bfloat16>::value) asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
   }
-  __device__ __forceinline__ Words values() const {
-    Words b;
-#pragma unroll
-    for (int k = 0; k < V / 2; ++k) b.w[k] = __byte_perm(key[2 * k], key[2 * k + 1], 0x7632);
-    return b;
-  }
-  __device__ __forceinline__ unsigned char position(int k) const {
-    return (unsigned char)(key[k] < 0x10000u ? kBpNowhere : 9u - (key[k] & 0xffffu));
+  static __device__ __forceinline__ uint32_t equal(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (sizeof(T) == 4) r = __uint_as_float(a) == __uint_as_float(b) ? ~0u : 0u;
+    // bit patterns below 0x8000: 0x8000 minus their difference's bits keeps its top bit only where there is none
+    else asm("prmt.b32 %0, %1, %1, 0xbb99;" : "=r"(r) : "r"(0x80008000u - (a ^ b)));
+    return r;
   }
 };
-template <typename T, int V>
-struct BpBest<T, V, false> {
-  using Words = BpWords<V * sizeof(T) / 4>;
-  float val[V];
-  uint32_t code[V];
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int k = 0; k < V; ++k) { val[k] = -1.f; code[k] = 0u; }
-  }
-  __device__ __forceinline__ void take(const Words& a, uint32_t c) {
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-      if (bp_get<T>(a, k) > val[k]) { val[k] = bp_get<T>(a, k); code[k] = c; }
-  }
-  __device__ __forceinline__ void merge(const BpBest& row, uint32_t kh_code) {
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-      if (row.val[k] > val[k]) { val[k] = row.val[k]; code[k] = row.code[k] + kh_code; }
-  }
-  __device__ __forceinline__ Words values() const { return bp_put<T, V>(val); }
-  __device__ __forceinline__ unsigned char position(int k) const { return (unsigned char)(val[k] > 0.f ? 9u - code[k] : kBpNowhere); }
-};
+__device__ __forceinline__ uint32_t bp_select(uint32_t mask, uint32_t a, uint32_t b) { return (mask & a) | (~mask & b); }
 
 // forward: per pooled row two new input rows of three columns each (the third row is the previous pooled row's last one,
-// kept as its row maximum).  About 4.5 instructions per loaded element, 27 per pooled one, against some 80 of the
-// shared-memory version.  Measured, 256 x 112 x 112 x 64 bf16: 325 -> 134 us.
-template <typename T, int V>
-__global__ void __launch_bounds__(kBpThreads) bn_pool_fwd_kernel(
-    const T* __restrict__ x, T* __restrict__ y, unsigned char* __restrict__ idx, const float* __restrict__ gamma,
+// kept as its maximum).  Values are compared two at a time in their 16-bit type, and the first position that equals the
+// maximum is selected afterwards together with its input value (32-bit (value, position) keys took more instructions without
+// it).  The next pooled row's loads are issued before this one is computed.
+// xmax (nullable) receives the input at the maximum: all that the backward sums need of x, a quarter of its size.
+// Bound by memory and instruction issue, 565 MB and 103 MB of xmax at 256 x 112 x 112 x 64 bf16 (102 us at the copy rate).
+// Measured: 133 us before, without xmax; about 145 with it.
+constexpr int kBpV = 4;                                      // channels of a thread
+template <typename T>
+__global__ void __launch_bounds__(kBpThreads, sizeof(T) == 2 ? 4 : 2) bn_pool_fwd_kernel(
+    const T* __restrict__ x, T* __restrict__ y, unsigned char* __restrict__ idx, T* __restrict__ xmax, const float* __restrict__ gamma,
     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ invstd, BpDims d, BpWalk walk) {
+  constexpr int V = kBpV, NW = V * sizeof(T) / 4, E = 4 / sizeof(T);      // words of a pack, elements of a word
+  constexpr uint32_t ONES = E == 2 ? 0x00010001u : 1u;      // one per element of a word
+  using Words = BpWords<NW>;
+  using Word = BpWord<T>;
   const int cvn = d.C / V;
   const long long t = (long long)blockIdx.x * kBpThreads + threadIdx.x;
   if (t >= walk.items) return;
@@ -530,59 +516,85 @@ __global__ void __launch_bounds__(kBpThreads) bn_pool_fwd_kernel(
     sc[k] = invstd[c] * gamma[c];
     sh[k] = beta[c] - mean[c] * sc[k];
   }
+  const int oh0 = strip * walk.rows, oh1 = min(oh0 + walk.rows, d.OH);
   const size_t line = (size_t)d.W * d.C;
-  const T* col = x + (size_t)n * d.H * line + (size_t)(2 * ow) * d.C + cv * V;      // input column 2 ow
-  const bool left = ow > 0, right = 2 * ow + 1 < d.W;
-  // normalised, rectified and rounded to T, as the next layer would read it
-  using Words = BpWords<V * sizeof(T) / 4>;
-  constexpr int NW = V * sizeof(T) / 4;
-  auto rectified = [&](const Words& v) {
-    float f[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) f[k] = fmaxf(bp_get<T>(v, k) * sc[k] + sh[k], 0.f);
-    return bp_put<T, V>(f);
-  };
+  // A column outside the image counts as 0, which only a window whose maximum is 0 finds; its input is the middle one's,
+  // which then is not positive after batch-norm either.
+  const uint32_t left = ow > 0 ? ~0u : 0u, right = 2 * ow + 1 < d.W ? ~0u : 0u;
+  const T* pc = x + ((size_t)n * d.H + 2 * oh0) * line + (size_t)(2 * ow) * d.C + cv * V;      // input column 2 ow
+  const T *pl = left ? pc - d.C : pc, *pr = right ? pc + d.C : pc;
   struct Row { Words l, c, r; };
-  auto load = [&](int ih, Row& q) {
-    const T* p = col + (size_t)ih * line;
-    q.c = bp_ld<NW>(p);
-    if (left) q.l = bp_ld<NW>(p - d.C);
-    if (right) q.r = bp_ld<NW>(p + d.C);
-  };
+  auto load = [&](Row& q) { q.l = bp_ld<NW>(pl); q.c = bp_ld<NW>(pc); q.r = bp_ld<NW>(pr); };
+  auto down = [&]() { pl += line; pc += line; pr += line; };
+  struct Best { uint32_t max[NW], x[NW], at[NW]; };          // of a row or window; `at`: position in it, one per element
   auto row_best = [&](const Row& q) {
-    BpBest<T, V> b;
-    b.clear();
-    if (left) b.take(rectified(q.l), 3);
-    b.take(rectified(q.c), 2);
-    if (right) b.take(rectified(q.r), 1);
+    Best b;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const uint32_t l = Word::rectified(q.l.w[w], sc + w * E, sh + w * E) & left, c = Word::rectified(q.c.w[w], sc + w * E, sh + w * E),
+                     r = Word::rectified(q.r.w[w], sc + w * E, sh + w * E) & right;
+      b.max[w] = Word::larger(l, Word::larger(c, r));
+      const uint32_t is_c = Word::equal(c, b.max[w]), is_l = Word::equal(l, b.max[w]);
+      b.at[w] = bp_select(is_c, ONES, 2 * ONES) & ~is_l;
+      b.x[w] = bp_select(is_l, q.l.w[w], bp_select(is_c, q.c.w[w], q.r.w[w]));
+    }
     return b;
   };
-  const int oh0 = strip * walk.rows, oh1 = min(oh0 + walk.rows, d.OH);
-  BpBest<T, V> above;                                      // the row above the window's middle row
-  above.clear();
-  if (oh0 > 0) { Row q; load(2 * oh0 - 1, q); above = row_best(q); }
+  Best above;                                                // the row above the window's middle row
+  Row q0, q1;
+  if (oh0 > 0) {
+    pl -= line; pc -= line; pr -= line;
+    load(q0);
+    above = row_best(q0);
+    down();
+  }
+  load(q0);
+  down();
+  if (2 * oh0 + 1 < d.H) load(q1);
   size_t o = (((size_t)n * d.OH + oh0) * d.OW + ow) * d.C + cv * V;
 #pragma unroll 1
   for (int oh = oh0; oh < oh1; ++oh, o += (size_t)d.OW * d.C) {
-    const bool below = 2 * oh + 1 < d.H;
-    Row q0, q1;
-    load(2 * oh, q0);
-    if (below) load(2 * oh + 1, q1);
-    BpBest<T, V> best, last;
-    best.clear();
-    best.merge(above, 6);
-    best.merge(row_best(q0), 3);
-    last.clear();
-    if (below) last = row_best(q1);
-    best.merge(last, 0);
-    above = last;
-    uint32_t oi[V / 4];
+    const Row r0 = q0, r1 = q1;
+    if (oh + 1 < oh1) {
+      down();
+      load(q0);
+      down();
+      if (2 * oh + 3 < d.H) load(q1);
+    }
+    const Best mid = row_best(r0);
+    Best last;
+    if (2 * oh + 1 < d.H) {
+      last = row_best(r1);
+    } else {                                                 // rows outside the image, like columns
+      last = mid;
 #pragma unroll
-    for (int k = 0; k < V; k += 4)
-      oi[k / 4] = best.position(k) | best.position(k + 1) << 8 | best.position(k + 2) << 16 | (uint32_t)best.position(k + 3) << 24;
-    bp_st(y + o, best.values());
-    if constexpr (V == 8) *reinterpret_cast<uint2*>(idx + o) = make_uint2(oi[0], oi[V / 4 - 1]);
-    else *reinterpret_cast<uint32_t*>(idx + o) = oi[0];
+      for (int w = 0; w < NW; ++w) last.max[w] = 0u;
+    }
+    if (oh == 0) {
+      above = mid;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) above.max[w] = 0u;
+    }
+    Words ym, xm;
+    uint32_t at[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      ym.w[w] = Word::larger(above.max[w], Word::larger(mid.max[w], last.max[w]));
+      const uint32_t is_mid = Word::equal(mid.max[w], ym.w[w]), is_above = Word::equal(above.max[w], ym.w[w]);
+      xm.w[w] = bp_select(is_above, above.x[w], bp_select(is_mid, mid.x[w], last.x[w]));
+      at[w] = bp_select(is_above, above.at[w], bp_select(is_mid, mid.at[w] + 3 * ONES, last.at[w] + 6 * ONES));
+    }
+    above = last;
+    bp_st(y + o, ym);
+    uint32_t packed = E == 2 ? __byte_perm(at[0], at[1], 0x6420)
+                             : __byte_perm(__byte_perm(at[0], at[1], 0x0040), __byte_perm(at[NW - 2], at[NW - 1], 0x0040), 0x5410);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {                            // a window whose maximum is 0 names no position
+      const uint32_t bits = E == 2 ? (k & 1 ? ym.w[k / 2 % NW] >> 16 : ym.w[k / 2 % NW] & 0xffffu) : ym.w[k % NW];
+      if (bits == 0u) packed |= kBpNowhere << (8 * k);
+    }
+    *reinterpret_cast<uint32_t*>(idx + o) = packed;
+    if (xmax) bp_st(xmax + o, xm);
   }
 }
 
@@ -661,45 +673,6 @@ __device__ __forceinline__ void bp_walk_strips(const T* __restrict__ x, const T*
   }
 }
 
-// backward statistics: sums of dz and dz * (x - mean) per channel, one partial row per block
-// Measured, 256 x 112 x 112 x 64 bf16: 137 us (pool backward 318 and statistics 168 as separate passes).
-template <typename T, int V, int BLOCKS>
-__global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_reduce_kernel(
-    const T* __restrict__ x, const T* __restrict__ dy, const unsigned char* __restrict__ idx, const float* __restrict__ mean,
-    const float* __restrict__ invstd, BpDims d, BpWalk walk, float* __restrict__ partial) {
-  const int cvn = d.C / V, cv = threadIdx.x % cvn;                // kBpThreads is a multiple of cvn
-  float a[V], b[V], mu[V];
-#pragma unroll
-  for (int k = 0; k < V; ++k) { a[k] = 0.f; b[k] = 0.f; mu[k] = mean[cv * V + k]; }
-  bp_walk_strips<T, V>(x, dy, idx, d, walk, [&](const BpWords<V * sizeof(T) / 4> (&xv)[4], size_t, const int (&)[4], const BpWindow<T, V> (&w)[2][2], const bool (&in)[4]) {
-#pragma unroll
-    for (int c = 0; c < V; ++c) {
-      float g[4];
-      bp_route<T, V>(w, c, g);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (!in[q]) continue;
-        a[c] += g[q];
-        b[c] += g[q] * (bp_get<T>(xv[q], c) - mu[c]);
-      }
-    }
-  });
-  __shared__ float s[kBpThreads][2 * V + 1];
-#pragma unroll
-  for (int k = 0; k < V; ++k) {
-    s[threadIdx.x][k] = a[k];
-    s[threadIdx.x][V + k] = b[k] * invstd[cv * V + k];
-  }
-  __syncthreads();
-  for (int o = threadIdx.x; o < cvn * 2 * V; o += kBpThreads) {
-    const int c = o / (2 * V), k = o % (2 * V);
-    float t = 0.f;
-    for (int g = c; g < kBpThreads; g += cvn) t += s[g][k];
-    const int which = k / V, ch = c * V + (k % V);
-    partial[((size_t)blockIdx.x * 2 + which) * d.C + ch] = t;
-  }
-}
-
 // backward apply; measured, 256 x 112 x 112 x 64 bf16: 179 us (208 with the gradient that the pool had written, 411 MB, to read).
 template <typename T, int V, int BLOCKS>
 __global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_apply_kernel(
@@ -757,7 +730,7 @@ static int bn_pool_check(int64_t rows, const BpDims& d, int V) {
 }
 
 template <typename T>
-static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, const float* beta, float* rmean, float* rvar,
+static int bn_pool_fwd_t(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta, float* rmean, float* rvar,
                          float* smean, float* sinv, int N, int H, int W, int C, float eps, float momentum, int training,
                          void* scratch, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
@@ -774,30 +747,24 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, const float* gamma, 
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
                                                            rows > 1 ? m / (m - 1.f) : 1.f, eps, momentum, smean, sinv, rmean, rvar);
   }
-  const BpWalk walk = bp_walk<V>(d);
-  bn_pool_fwd_kernel<T, V><<<(unsigned)((walk.items + kBpThreads - 1) / kBpThreads), kBpThreads, 0, s>>>(
-      (const T*)x, (T*)y, (unsigned char*)idx, gamma, beta, smean, sinv, d, walk);
+  const BpWalk walk = bp_walk<kBpV>(d);
+  bn_pool_fwd_kernel<T><<<(unsigned)((walk.items + kBpThreads - 1) / kBpThreads), kBpThreads, 0, s>>>(
+      (const T*)x, (T*)y, (unsigned char*)idx, (T*)xmax, gamma, beta, smean, sinv, d, walk);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn+pool forward launch: %s", cudaGetErrorString(e));
 }
 
 template <typename T, int V, int BLOCKS>
-static void bn_pool_bwd_launch(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* smean,
-                               const float* sinv, float* dgamma, float* dbeta, const BpDims& d, void* scratch, cudaStream_t s) {
+static void bn_pool_bwd_apply(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* smean,
+                              const float* sinv, const float* dgamma, const float* dbeta, const BpDims& d, cudaStream_t s) {
   const BpWalk walk = bp_walk<V>(d);
-  const long long blocks = (walk.items + kBpThreads - 1) / kBpThreads;
-  const int grid = (int)std::min<long long>(blocks, 148 * BLOCKS);         // one resident wave; at most kBnMaxGrid partial rows
-  static_assert(148 * BLOCKS <= kBnMaxGrid, "partial rows in scratch");
-  bn_pool_bwd_reduce_kernel<T, V, BLOCKS><<<grid, kBpThreads, 0, s>>>((const T*)x, (const T*)dy, (const unsigned char*)idx, smean, sinv, d,
-                                                                      walk, (float*)scratch);
-  bn_finalize_bwd_kernel<<<(d.C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, d.C, dgamma, dbeta);
-  bn_pool_bwd_apply_kernel<T, V, BLOCKS><<<(unsigned)blocks, kBpThreads, 0, s>>>(
+  bn_pool_bwd_apply_kernel<T, V, BLOCKS><<<(unsigned)((walk.items + kBpThreads - 1) / kBpThreads), kBpThreads, 0, s>>>(
       (const T*)x, (const T*)dy, (const unsigned char*)idx, (T*)dx, gamma, smean, sinv, dgamma, dbeta, d, walk,
       1.f / (float)((int64_t)d.N * d.H * d.W));
 }
 
 template <typename T>
-static int bn_pool_bwd_t(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
+static int bn_pool_bwd_t(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
                          const float* smean, const float* sinv, float* dgamma, float* dbeta, int N, int H, int W, int C,
                          void* scratch, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
@@ -805,16 +772,21 @@ static int bn_pool_bwd_t(const void* x, const void* dy, const void* idx, void* d
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
   int st = bn_pool_check(rows, d, V);
   if (st) return st;
+  // The sums: dz is zero but at the maximum of each open window, so they run over the pooled positions, with the input that
+  // the forward kept for each and the ReLU mask that it implies.  256 x 112 x 112 x 64 bf16: 36 us (206 MB; 136 over
+  // all positions of x, 411 MB, with the gradient routed to each).
+  const size_t nvec = (size_t)N * d.OH * d.OW * (C / V);
+  const int grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU);
+  bn_reduce_kernel<T, V, true, MASK_X_ROUNDED><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
+                                                                           nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
+  bn_finalize_bwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, dgamma, dbeta);
   // 16-bit types: packs of four channels where their groups divide the block (up to 1024 channels).  They halve the
-  // per-channel state, so that three blocks fit on an SM instead of two (256 x 112 x 112 x 64: statistics 150 -> 137 us, apply 254 -> 179).
+  // per-channel state, so that three blocks fit on an SM instead of two (256 x 112 x 112 x 64: 254 -> 179 us).
   if constexpr (sizeof(T) == 2) {
-    if (kBpThreads % (C / 4) == 0) {
-      bn_pool_bwd_launch<T, 4, 3>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, scratch, s);
-    } else {
-      bn_pool_bwd_launch<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, scratch, s);
-    }
+    if (kBpThreads % (C / 4) == 0) bn_pool_bwd_apply<T, 4, 3>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
+    else bn_pool_bwd_apply<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
   } else {
-    bn_pool_bwd_launch<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, scratch, s);
+    bn_pool_bwd_apply<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn+pool backward launch: %s", cudaGetErrorString(e));
@@ -897,31 +869,32 @@ int tmpi_bn_relu_bwd_acc(const void* x, const void* y, const void* dy, void* dx,
 
 // Batch-norm + ReLU + max-pool (3x3, stride 2, pad 1) in one stage.  x: [N, H, W, C] channels-last;
 // y, idx: [N, OH, OW, C] with OH = (H - 1) / 2 + 1.  Other arguments as tmpi_bn_relu_fwd / _bwd.
-int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, const float* gamma, const float* beta, float* running_mean,
+// xmax (nullable): [N, OH, OW, C], the input at each window's maximum, which backward needs.
+int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta, float* running_mean,
                           float* running_var, float* save_mean, float* save_invstd, int N, int H, int W, int channels,
                           float eps, float momentum, int training, int dtype, void* scratch, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   switch (dtype) {
-    case TMPI_BF16: return bn_pool_fwd_t<__nv_bfloat16>(x, y, idx, gamma, beta, running_mean, running_var, save_mean, save_invstd,
+    case TMPI_BF16: return bn_pool_fwd_t<__nv_bfloat16>(x, y, idx, xmax, gamma, beta, running_mean, running_var, save_mean, save_invstd,
                                                         N, H, W, channels, eps, momentum, training, scratch, s);
-    case TMPI_F16: return bn_pool_fwd_t<__half>(x, y, idx, gamma, beta, running_mean, running_var, save_mean, save_invstd, N, H, W,
+    case TMPI_F16: return bn_pool_fwd_t<__half>(x, y, idx, xmax, gamma, beta, running_mean, running_var, save_mean, save_invstd, N, H, W,
                                                 channels, eps, momentum, training, scratch, s);
-    case TMPI_F32: return bn_pool_fwd_t<float>(x, y, idx, gamma, beta, running_mean, running_var, save_mean, save_invstd, N, H, W,
+    case TMPI_F32: return bn_pool_fwd_t<float>(x, y, idx, xmax, gamma, beta, running_mean, running_var, save_mean, save_invstd, N, H, W,
                                                channels, eps, momentum, training, scratch, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: dtype %d", dtype);
 }
 
-int tmpi_bn_relu_pool_bwd(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
+int tmpi_bn_relu_pool_bwd(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
                           const float* save_mean, const float* save_invstd, float* dgamma, float* dbeta, int N, int H, int W,
                           int channels, int dtype, void* scratch, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   switch (dtype) {
-    case TMPI_BF16: return bn_pool_bwd_t<__nv_bfloat16>(x, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W,
+    case TMPI_BF16: return bn_pool_bwd_t<__nv_bfloat16>(x, xmax, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W,
                                                         channels, scratch, s);
-    case TMPI_F16: return bn_pool_bwd_t<__half>(x, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W, channels,
+    case TMPI_F16: return bn_pool_bwd_t<__half>(x, xmax, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W, channels,
                                                 scratch, s);
-    case TMPI_F32: return bn_pool_bwd_t<float>(x, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W, channels,
+    case TMPI_F32: return bn_pool_bwd_t<float>(x, xmax, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W, channels,
                                                scratch, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: dtype %d", dtype);

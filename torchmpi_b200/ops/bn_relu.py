@@ -141,6 +141,8 @@ class _BnReluPoolFn(torch.autograd.Function):
         OH, OW = (H - 1) // 2 + 1, (W - 1) // 2 + 1
         y = torch.empty((N, C, OH, OW), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
         idx = torch.empty((N, OH, OW, C), dtype=torch.uint8, device=x.device)
+        # the input at each window's maximum, from which backward forms its sums
+        xmax = torch.empty_like(y) if any(ctx.needs_input_grad) and config.get("bn_pool_fused_bwd") else None
         if training:
             mean = torch.empty(C, dtype=torch.float32, device=x.device)
             invstd = torch.empty(C, dtype=torch.float32, device=x.device)
@@ -148,28 +150,29 @@ class _BnReluPoolFn(torch.autograd.Function):
             mean = running_mean.float()
             invstd = torch.rsqrt(running_var.float() + eps)
         check(lib.tmpi_bn_relu_pool_fwd(
-            x.data_ptr(), y.data_ptr(), idx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+            x.data_ptr(), y.data_ptr(), idx.data_ptr(), xmax.data_ptr() if xmax is not None else None, gamma.data_ptr(), beta.data_ptr(),
             running_mean.data_ptr() if (training and running_mean is not None) else None,
             running_var.data_ptr() if (training and running_var is not None) else None,
             mean.data_ptr(), invstd.data_ptr(), N, H, W, C, eps, momentum, int(training), dtype_code(x.dtype),
             _scratch_for(x.device, C).data_ptr(), stream_ptr()))
         launch_count += 3 if training else 1
-        ctx.save_for_backward(x, idx, gamma, beta, mean, invstd)
+        ctx.save_for_backward(x, xmax, idx, gamma, beta, mean, invstd)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         global launch_count
-        x, idx, gamma, beta, mean, invstd = ctx.saved_tensors
+        x, xmax, idx, gamma, beta, mean, invstd = ctx.saved_tensors
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
         dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
         dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
-        if config.get("bn_pool_fused_bwd"):
-            # one stage: both batch-norm passes rebuild the pool's gradient routing from dy and the index
+        if xmax is not None:
+            # one stage: the sums run over the pooled positions, the apply pass rebuilds the pool's gradient routing from dy and
+            # the index
             check(lib.tmpi_bn_relu_pool_bwd(
-                x.data_ptr(), dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+                x.data_ptr(), xmax.data_ptr(), dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
                 mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
                 _scratch_for(x.device, C).data_ptr(), stream_ptr()))
             launch_count += 3
