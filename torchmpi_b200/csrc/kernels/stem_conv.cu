@@ -7,8 +7,12 @@
 // layout of the tensor core: eight consecutive output pixels x 8 values are 128 contiguous bytes, the next tap pair is the
 // same 128 bytes moved by one unit.  Overlapping core matrices cost nothing, so nothing is copied per window.
 //
-//   forward          Y[ow, co] += X[ow, (pair, channel)] W[co, (pair, channel)] for each of the seven input rows of a window:
-//                    14 MMAs of 128 x 64 x 16 per output row (K = 7 rows x 4 pairs x 8 = 224 for 147 weights)
+//   forward          Y[ow, co] += X[ow, (pair, channel)] W[co, (pair, channel)] for each input row of a window, two output rows
+//                    at a time: input rows 2 - 6 of the nine that they cover meet kernel row r for the first and r - 2 for
+//                    the second, side by side in one operand of 128 columns: 19 MMAs of 128 x 128 (or 64) x 16 for two rows
+//                    (K = 7 rows x 4 pairs x 8 = 224 for 147 weights) in place of 28 narrow ones.  An MMA is paced by its
+//                    128-row operand, so a wide one costs little more: with the pooling stage, forward and backward,
+//                    770 -> 757 us at 256 x 224 x 224, of which this kernel takes about 125 (138 before).
 //   weight gradient  the output pixels are the K dimension.  Two output rows share an operand: M = 128 = dY rows (i, i + 1)
 //                    of 64 channels, N = 80 = ten input rows x 8 values of one tap pair (the rows are a constant stride
 //                    apart), four MMAs per 16 pixels; input row r meets kernel row r of dY row i and r - 2 of row i + 1.
@@ -18,7 +22,7 @@
 //                    that is not its own (tail units, the single row).
 //
 // What bounds it: forward the 411 MB of output (62 us at the copy rate, 256 images of 224 x 224) and, about as much, the
-// MMAs (448 cycles per output row); the weight gradient the reads of dY, the same bytes, and the MMAs (their 128-row dY
+// MMAs; the weight gradient the reads of dY, the same bytes, and the MMAs (their 128-row dY
 // operand comes out of shared memory once per tap pair).  The patch matrix that both products read before was 1.03 GB,
 // written once and read twice.  Measured, 256 x 224 x 224: forward 138 us
 // (patch matrix 354 + product 262 + weight layout 9), weight gradient 147 us (split-K product 221).
@@ -47,6 +51,7 @@ constexpr int MAX_OW = 128;
 constexpr int LOADERS = 256, THREADS = 512;        // warp 0 issues MMAs, warps 4-7 drain, warps 8-15 load x; wgrad: warp 1 loads dY
 constexpr int STAGING = 4096;                      // 32 pixels x 64 channels
 constexpr int W_BYTES = KROWS * TAPS * 8 * COUT * 2;
+constexpr int W_BLOCK = COUT * 16, W_TAP = KROWS * W_BLOCK;      // one kernel row of a tap pair, one tap pair
 constexpr int ACCS = 4, DY_STAGES = 3, WG_N = 80;
 constexpr int TAILS = 2;                           // tap pairs whose last 16 pixels are kept once more
 constexpr int SINGLE_N = 32, SINGLE_COL = TAPS * WG_N;      // accumulators of an odd height's last row: input rows 2..5 of each tap pair
@@ -172,23 +177,40 @@ __device__ __forceinline__ void teardown(Shared* sh, int warp) {
 }
 
 // ---------------------------------------------------------------- forward
+// Weights of a tap pair: a block of 64 output channels x 16 bytes per kernel row, in the order 6 4 2 0 5 3 1, so that the
+// block of row r is followed by that of row r - 2.
+__device__ __forceinline__ int weight_block(int kh) { return (kh & 1) ? 4 + (5 - kh) / 2 : (6 - kh) / 2; }
+
 __device__ void fwd_mma(Shared* sh, unsigned char* rows, unsigned char* weights, const Params& p) {
-  constexpr uint32_t idesc = sm100::make_idesc_f16(128, COUT, true);
+  constexpr uint32_t idesc_one = sm100::make_idesc_f16(128, COUT, true), idesc_two = sm100::make_idesc_f16(128, 2 * COUT, true);
   const uint32_t x0 = sm100::smem_u32(rows), w0 = sm100::smem_u32(weights);
   int n, oh0, count = 0;
   for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
     const int b = it & 1;
     STEM_WAIT(&sh->x_full[b], (it >> 1) & 1, 62);
     const int lines = min(R, p.OH - oh0);
-    for (int i = 0; i < lines; ++i, ++count) {
+    for (int i = 0; i < lines; i += 2, ++count) {
       const int acc = count % ACCS;
       if (count >= ACCS) STEM_WAIT(&sh->acc_empty[acc], (count / ACCS - 1) & 1, 63);
       sm100::tc_fence_after();
+      const bool two = i + 1 < lines;
+      const uint32_t d = sh->tmem_base + acc * 2 * COUT;
 #pragma unroll
-      for (int k = 0; k < 2 * KROWS; ++k) {                  // kernel row k / 2, tap pairs 2 (k % 2) and the next
-        const uint32_t a = x0 + (uint32_t)(b * IN_ROWS + 2 * i + (k >> 1)) * p.row_bytes + (k & 1) * 32;
-        sm100::umma_f16(sh->tmem_base + acc * COUT, desc_plain(a, 16, 128), desc_plain(w0 + k * 2 * COUT * 16, COUT * 16, 128), idesc,
-                        k > 0 ? 1u : 0u);
+      for (int r = 0; r < KROWS + 2; ++r) {                  // input row; tap pairs 2 h and the next
+        if (r >= KROWS && !two) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint64_t a = desc_plain(x0 + (uint32_t)(b * IN_ROWS + 2 * i + r) * p.row_bytes + h * 32, 16, 128);
+          const uint32_t w = w0 + h * 2 * W_TAP + weight_block(r < KROWS ? r : r - 2) * W_BLOCK;
+          // rows 0 and 1 are the first output row's alone, 7 and 8 the second one's, whose sums start at row 2
+          if (r == 2 && h == 0 && two) {
+            sm100::umma_f16(d, a, desc_plain(w, W_TAP, 128), idesc_one, 1u);
+            sm100::umma_f16(d + COUT, a, desc_plain(w + W_BLOCK, W_TAP, 128), idesc_one, 0u);
+          } else {
+            sm100::umma_f16(r < KROWS ? d : d + COUT, a, desc_plain(w, W_TAP, 128), two && r >= 2 && r < KROWS ? idesc_two : idesc_one,
+                            (r | h) ? 1u : 0u);
+          }
+        }
       }
       sm100::umma_commit(&sh->acc_full[acc]);
     }
@@ -220,7 +242,7 @@ __device__ __noinline__ void redo_pixel(const __nv_bfloat16* img, int H, int W, 
         if (iw0 + kw < 0 || iw0 + kw >= W) continue;
         for (int c = 0; c < 3; ++c)
           sum += __bfloat162float(img[((size_t)ih * W + iw0 + kw) * 3 + c]) *
-                 __bfloat162float(w[((kh * TAPS + (kw + 1) / 2) * COUT + co) * 8 + ((kw + 1) & 1) * 4 + c]);
+                 __bfloat162float(w[(((kw + 1) / 2 * KROWS + weight_block(kh)) * COUT + co) * 8 + ((kw + 1) & 1) * 4 + c]);
       }
     }
     *reinterpret_cast<__nv_bfloat16*>(out + (((co >> 3) ^ swizzle) << 4) + (co & 7) * 2) = __float2bfloat16(sum);
@@ -229,26 +251,30 @@ __device__ __noinline__ void redo_pixel(const __nv_bfloat16* img, int H, int W, 
 
 __device__ void fwd_drain(Shared* sh, unsigned char* staging, const unsigned char* weights, const Params& p, const CUtensorMap* my, int quarter, int lane) {
   const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
-  int n, oh0, count = 0;
+  int n, oh0, count = 0, row = 0;                             // accumulators and rows drained
   for (int it = 0; chunk(p, it, &n, &oh0); ++it) {
     const int lines = min(R, p.OH - oh0);
-    for (int i = 0; i < lines; ++i, ++count) {
+    for (int i = 0; i < lines; ++i, ++row) {
       const int acc = count % ACCS;
-      STEM_WAIT(&sh->acc_full[acc], (count / ACCS) & 1, 64);
-      sm100::tc_fence_after();
+      const bool second = i & 1, last = second || i + 1 == lines;            // of its accumulator
+      if (!second) {
+        STEM_WAIT(&sh->acc_full[acc], (count / ACCS) & 1, 64);
+        sm100::tc_fence_after();
+      }
       uint32_t r[2][32];
-      sm100::tmem_ld_32x32(tm + acc * COUT, r[0]);
-      sm100::tmem_ld_32x32(tm + acc * COUT + 32, r[1]);
+      const uint32_t at = tm + acc * 2 * COUT + (second ? COUT : 0);
+      sm100::tmem_ld_32x32(at, r[0]);
+      sm100::tmem_ld_32x32(at + 32, r[1]);
       sm100::tmem_ld_wait();
       sm100::tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        sm100::mbar_arrive(&sh->acc_empty[acc]);
+        if (last) sm100::mbar_arrive(&sh->acc_empty[acc]);
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the store two rows ago has read its tile
       }
       __syncwarp();
       if (quarter * 32 < p.OW) {
-        unsigned char* stg = staging + (quarter * 2 + (count & 1)) * STAGING;
+        unsigned char* stg = staging + (quarter * 2 + (row & 1)) * STAGING;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           uint32_t w[4];
@@ -267,6 +293,7 @@ __device__ void fwd_drain(Shared* sh, unsigned char* staging, const unsigned cha
         if (lane == 0) sm100::tma_store_4d(my, stg, 0, quarter * 32, oh0 + i, n);      // pixels beyond the row are clipped
       }
       if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      if (last) ++count;
     }
   }
   if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -281,7 +308,6 @@ __global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_const
   Shared* sh = (Shared*)(rows + 2 * IN_ROWS * p.row_bytes + (MAX_OW + 4) * 16);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   setup(sh, warp);
-  // weights: K chunk k (kernel row k / 2, tap pairs 2 (k % 2) ..), its halves, groups of eight output channels
   for (int t = threadIdx.x; t < KROWS * TAPS * COUT; t += THREADS) {
     const int co = t % COUT, unit = t / COUT, kh = unit / TAPS, tap = unit % TAPS;
     unsigned short v[8];
@@ -292,8 +318,8 @@ __global__ void __launch_bounds__(THREADS, 1) stem_fwd_kernel(const __grid_const
       if (kw >= 0 && kw < 7 && c < 3)
         v[e] = *reinterpret_cast<const unsigned short*>(p.w + co * p.ws_co + c * p.ws_c + kh * p.ws_h + kw * p.ws_w);
     }
-    *reinterpret_cast<uint4*>(weights + (size_t)t * 16) = make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16,
-                                                                     v[4] | (uint32_t)v[5] << 16, v[6] | (uint32_t)v[7] << 16);
+    *reinterpret_cast<uint4*>(weights + tap * W_TAP + weight_block(kh) * W_BLOCK + co * 16) =
+        make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16, v[4] | (uint32_t)v[5] << 16, v[6] | (uint32_t)v[7] << 16);
   }
   sm100::fence_proxy_async_smem();
   sm100::tc_fence_before();
