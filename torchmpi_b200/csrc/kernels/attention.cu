@@ -493,24 +493,11 @@ static unsigned long long* g_attn_trace = nullptr;
 // fixed part per item, Q and the first S before, the output after (about 1.5 blocks; 2 with a merge, and both teams pay it).
 // Sharing halves the longest item where there are few, and costs the fixed part twice where there are many: 1 x 16 x 2048
 // (256 items on 148 CTAs) 31.0 -> 25.4 us; 8 x 16 x 1024 (1024 items) stays with a team per item.
-static bool attention_shares(int items, int per_block, int q_blocks, int grid) {
-  const int teams = attn::TEAMS * grid;
-  if (items > 8 * teams) return false;                       // many items each are balanced as they are
-  auto busiest = [&](int units, bool shared) {               // in half blocks
-    int most = 0;
-    for (int i = 0; i < units; ++i) {
-      int sum = 0;
-      for (int round = 0;; ++round) {
-        const long long t = (long long)round * units + ((round & 1) ? units - 1 - i : i);
-        if (t >= items) break;
-        const int blocks = q_blocks - (int)(t / per_block);
-        sum += shared ? (blocks + 1) / 2 * 2 + 4 : blocks * 2 + 3;
-      }
-      most = std::max(most, sum);
-    }
-    return most;
-  };
-  return busiest(grid, true) < busiest(teams, false);
+static bool attention_shares(int per_block, int q_blocks, int grid) {      // per_block: items of each length, one to q_blocks
+  // in half blocks: the longest item, or the average of all where that is more
+  const double q = q_blocks, alone = per_block * (q * (q + 1) + 3 * q) / (attn::TEAMS * grid);
+  const double both = per_block * (q * (q + 1) / 2 + q / 2 + 4 * q) / grid;
+  return std::max(q + 5, both) < 0.95 * std::max(2 * q + 3, alone);
 }
 
 static int* attn_status_word(int** host_out = nullptr) {
@@ -552,7 +539,7 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.items = B * H * p.q_blocks;
   // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
   const int grid = std::min(p.items, gemm_sm_count());
-  const bool shared = !p.trace && attention_shares(p.items, B * H, p.q_blocks, grid);      // a trace follows one team through an item
+  const bool shared = !p.trace && attention_shares(B * H, p.q_blocks, grid);      // a trace follows one team through an item
   const auto kernel = shared ? attn::attention_fwd_kernel<true> : attn::attention_fwd_kernel<false>;
   cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
