@@ -293,6 +293,9 @@ int tmpi_conv_status(void);
 // blocks of a fused QKV projection), out [B * T, ld_out], lse [B, H, T] fp32 (optional); T a multiple of 128
 int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
                        int B, int T, int H, float scale, void* stream);
+int tmpi_attention_fwd_form(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
+                            int B, int T, int H, float scale, int shared, void* stream);
+int tmpi_attention_fwd_shares(int B, int T, int H);
 // gradients: o and dout [B * T, H * 64] with their own pitches, lse from the forward, delta [B, H, T] scratch, dq_acc a
 // fp32 [B * T, H * 64] buffer (cleared by the call) that receives dQ, dq (optional: dq_acc rounded) / dk / dv bf16 [B * T, ld_dkv]
 int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_qkv, const void* o, int64_t ld_o,

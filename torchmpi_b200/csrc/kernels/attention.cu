@@ -298,12 +298,14 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
       const float next = max_nan(m, mx);
       const bool grew = j > it.first && __any_sync(~0u, next > m);
-      const float alpha = ex2((m - next) * c2);
+      // While every key has scored -inf, scores are taken relative to 0: those keys weigh 0, wherever they lie.
+      const float base = next == -INFINITY ? 0.f : next;
+      const float alpha = ex2((m - base) * c2);
       const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
       m = next;
       if (grew) { sum2[0] = mul2(sum2[0], al2); sum2[1] = mul2(sum2[1], al2); }
-      // NaN where the maximum is NaN or infinite, and with it every P of the row: the polynomial's clamp alone would drop a NaN
-      const float nmc = fmaf(m, 0.f, -m * c2);
+      // NaN where the maximum is NaN or +inf, and with it every P of the row: the polynomial's clamp alone would drop a NaN
+      const float nmc = fmaf(base, 0.f, -base * c2);
       const unsigned long long nmc2 = pack2(__float_as_uint(nmc), __float_as_uint(nmc));
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -371,12 +373,9 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       ++merged;
       sm100::tc_fence_after();
       const float2 with = merge[row];
-      const float next = max_nan(m, with.x);
-      const float a0 = ex2((m - next) * c2);
-      // keys that are all -inf weigh nothing, as if they came after the others in one pass
-      const bool none = with.x == -INFINITY;
-      const float a1 = none ? 0.f : ex2((with.x - next) * c2);
-      l = l * a0 + (none ? 0.f : with.y * a1);
+      const float next = max_nan(m, with.x), base = next == -INFINITY ? 0.f : next;      // as in the blocks' loop
+      const float a0 = ex2((m - base) * c2), a1 = ex2((with.x - base) * c2);
+      l = l * a0 + with.y * a1;
       m = next;
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -385,7 +384,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
         sm100::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          o[q * 16 + i] = __float_as_uint(__uint_as_float(o[q * 16 + i]) * a0 + (none ? 0.f : __uint_as_float(o1[i]) * a1));
+          o[q * 16 + i] = __float_as_uint(__uint_as_float(o[q * 16 + i]) * a0 + __uint_as_float(o1[i]) * a1);
       }
     }
     const float inv = 1.f / l;
@@ -514,13 +513,9 @@ static int* attn_status_word(int** host_out = nullptr) {
   return dev_ptr;
 }
 
-extern "C" {
-
-// out[b, t, h, :] = sum_s softmax_s(scale * q[b, t, h, :] . k[b, s, h, :], s <= t) v[b, s, h, :] for bf16 q, k, v given
-// as [B * T, H * 64] matrices with a common row pitch of ld_qkv elements (for instance the three column blocks of a
-// fused QKV projection); out is [B * T, ld_out]; lse (optional) is [B, H, T] fp32.  T must be a multiple of 128.
-int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
-                       int B, int T, int H, float scale, void* stream) {
+// form: 0 a team per item, 1 the teams of a CTA share their items, -1 the rule's choice
+static int attention_fwd(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
+                         int B, int T, int H, float scale, int form, void* stream) {
   if (B < 1 || H < 1 || T < 128 || T % 128) return fail(TMPI_ERR_UNSUPPORTED, "attention: T=%d must be a positive multiple of 128", T);
   if (ld_out % 8 || ((uintptr_t)out & 15)) return fail(TMPI_ERR_INVALID, "attention: the output must be 16-byte aligned with a pitch that is a multiple of 8");
   if ((int64_t)B * H * (T / 128) > 0x7fffffffLL) return fail(TMPI_ERR_INVALID, "attention: too many blocks");
@@ -539,12 +534,34 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.items = B * H * p.q_blocks;
   // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
   const int grid = std::min(p.items, gemm_sm_count());
-  const bool shared = !p.trace && attention_shares(B * H, p.q_blocks, grid);      // a trace follows one team through an item
+  const bool shared = form < 0 ? !p.trace && attention_shares(B * H, p.q_blocks, grid)      // a trace follows one team through an item
+                               : form != 0;
   const auto kernel = shared ? attn::attention_fwd_kernel<true> : attn::attention_fwd_kernel<false>;
   cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
   cudaError_t e = launch_overlapped(kernel, grid, attn::THREADS, attn::SMEM_BYTES, (cudaStream_t)stream, mq, mk, mv, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention launch: %s", cudaGetErrorString(e));
+}
+
+extern "C" {
+
+// out[b, t, h, :] = sum_s softmax_s(scale * q[b, t, h, :] . k[b, s, h, :], s <= t) v[b, s, h, :] for bf16 q, k, v given
+// as [B * T, H * 64] matrices with a common row pitch of ld_qkv elements (for instance the three column blocks of a
+// fused QKV projection); out is [B * T, ld_out]; lse (optional) is [B, H, T] fp32.  T must be a multiple of 128.
+int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
+                       int B, int T, int H, float scale, void* stream) {
+  return attention_fwd(q, k, v, ld_qkv, out, ld_out, lse, B, T, H, scale, -1, stream);
+}
+
+// The same in a given form (for tests and timing), and the form that tmpi_attention_fwd takes.
+int tmpi_attention_fwd_form(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
+                            int B, int T, int H, float scale, int shared, void* stream) {
+  return attention_fwd(q, k, v, ld_qkv, out, ld_out, lse, B, T, H, scale, shared != 0, stream);
+}
+int tmpi_attention_fwd_shares(int B, int T, int H) {
+  const int64_t items = (int64_t)B * H * (T / attn::BQ);
+  if (B < 1 || H < 1 || T < attn::BQ || items > 0x7fffffffLL) return 0;
+  return attention_shares(B * H, T / attn::BQ, (int)std::min<int64_t>(items, gemm_sm_count()));
 }
 
 // Resident CTAs of the attention kernel per SM (1: a CTA holds two teams that overlap each other).
