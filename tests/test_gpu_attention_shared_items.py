@@ -33,7 +33,10 @@ def test_attention_items_shared_by_teams(B, T, H):
     x = qkv.detach().double().requires_grad_(True)
     ref = _attention64(x, H)
     ref.backward(dy.double())
+    shared, _ = _forward(qkv.detach(), H, True)            # whichever form the rule takes at this size
     # probabilities in bf16: 2^-9 of sums of order one each way; the gradient's products twice
+    assert ((shared.double() - ref).norm() / ref.norm()) < 5e-3
+    assert (shared.double() - ref).abs().max() < 3e-2
     assert ((y.double() - ref).norm() / ref.norm()) < 5e-3
     assert (y.double() - ref).abs().max() < 3e-2
     assert ((qkv.grad.double() - x.grad).norm() / x.grad.norm()) < 1e-2
@@ -42,6 +45,7 @@ def test_attention_items_shared_by_teams(B, T, H):
 @pytest.mark.parametrize("T", [256, 1024])
 def test_attention_shared_items_non_finite(T):
     """A key that scores -inf weighs nothing wherever the split lies; NaN and +inf reach the rows that see them, and no others."""
+    from torchmpi_b200._lib import lib
     from torchmpi_b200.ops import attention
     torch.manual_seed(1)
     for value, at in ((-math.inf, T - 3), (math.nan, T // 2 + 5), (math.inf, 70)):
@@ -50,6 +54,7 @@ def test_attention_shared_items_non_finite(T):
         qkv[0, at, 64] = value
         with torch.no_grad():
             y = attention.causal_attention(qkv, 1)
+        assert lib.tmpi_attention_fwd_shares(1, T, 1) and torch.equal(y.nan_to_num(9.0), _forward(qkv, 1, True)[0].nan_to_num(9.0))
         assert torch.isfinite(y[0, :at]).all()
         if value == -math.inf:
             ref = _attention64(torch.cat([qkv[..., :64], qkv[..., 64:128].nan_to_num(neginf=-1e30), qkv[..., 128:]], -1).double(), 1)

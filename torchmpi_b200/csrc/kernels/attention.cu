@@ -488,15 +488,35 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 static unsigned long long* g_attn_trace = nullptr;
 
-// Whether the teams of a CTA share its items.  The launch takes as long as its busiest team: the key blocks of its items and a
-// fixed part per item, Q and the first S before, the output after (about 1.5 blocks; 2 with a merge, and both teams pay it).
-// Sharing halves the longest item where there are few, and costs the fixed part twice where there are many: 1 x 16 x 2048
-// (256 items on 148 CTAs) 31.0 -> 25.4 us; 8 x 16 x 1024 (1024 items) stays with a team per item.
+// Half key blocks of the busiest unit (a team, or a CTA whose teams share) of a launch: its items in snake order, as Items deals
+// them, and 2.5 blocks for each (Q and the first S before, the output or the merge after; 1.5 where a shared item is one block and
+// has no merge).  One pass over the units per round, in runs of equal items.
+static int attention_busiest(int items, int per_block, int q_blocks, int units, bool shared) {
+  int load[1024] = {};
+  for (int round = 0, t = 0; t < items; ++round) {
+    const int end = std::min(items, t + units);
+    int at = 0, blocks = q_blocks - t / per_block, run = per_block - t % per_block;
+    for (; t < end; --blocks, run = per_block) {
+      const int n = std::min(run, end - t), cost = shared ? (blocks + 1) / 2 * 2 + (blocks > 1 ? 5 : 3) : 2 * blocks + 5;
+      int* l = load + ((round & 1) ? units - at - n : at);
+      for (int k = 0; k < n; ++k) l[k] += cost;
+      at += n;
+      t += n;
+    }
+  }
+  return *std::max_element(load, load + units);
+}
+
+// Whether the teams of a CTA share its items.  The launch takes as long as its busiest unit.  Sharing halves the longest item
+// where there are few, and costs the fixed part twice where there are many; between one and three items per CTA it turns on
+// how many of them the busiest one gets, which an average does not show.  Beyond that a team per item was faster throughout.
+// Measured over 1 - 256 items of each length, lengths of 1 - 32 blocks, on 148 SMs (a team per item, shared, in us): 16 x 16 (heads
+// x blocks) 31.4, 25.0; 37 x 8 19.0, 18.3; 64 x 3 10.3, 10.8; 52 x 4 11.9, 12.5; 27 x 13 27.9, 30.3; 20 x 20 40.6, 46.2; 128 x 8
+// 48.4, 60.0.  The form taken was the faster one of both, or within 3.1 % of it, at each of those sizes.
 static bool attention_shares(int per_block, int q_blocks, int grid) {      // per_block: items of each length, one to q_blocks
-  // in half blocks: the longest item, or the average of all where that is more
-  const double q = q_blocks, alone = per_block * (q * (q + 1) + 3 * q) / (attn::TEAMS * grid);
-  const double both = per_block * (q * (q + 1) / 2 + q / 2 + 4 * q) / grid;
-  return std::max(q + 5, both) < 0.95 * std::max(2 * q + 3, alone);
+  const long long items = (long long)per_block * q_blocks;
+  if (items > 4 * grid || attn::TEAMS * grid > 1024) return false;
+  return attention_busiest((int)items, per_block, q_blocks, grid, true) < attention_busiest((int)items, per_block, q_blocks, attn::TEAMS * grid, false);
 }
 
 static int* attn_status_word(int** host_out = nullptr) {
