@@ -53,12 +53,21 @@ constexpr int CHUNK_BYTES = 64 * BK * 2;                      // one 64 x 64 box
 constexpr int SLICE = 64, WARP_STAGING_BYTES = 32 * SLICE * 2;
 constexpr int RING = 2, STAGING_BYTES = EPI_WARPS * RING * WARP_STAGING_BYTES;      // staging tiles of each epilogue warp
 constexpr size_t SMEM_LIMIT = 232448;
-constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 512 /*barriers*/ + STAGING_BYTES;
+constexpr size_t SMEM_FIXED = 1024 /*alignment slack*/ + 512 /*barriers*/;
 constexpr unsigned long long kWaitBudgetNs = 4000000000ull;
 
 enum { A_TILED = 0, A_IM2COL = 1, A_MN = 2 };
 enum { B_K = 0, B_MN = 2, B_MN_IM2COL = 3 };
 enum { EPI_STATS = 1, EPI_ADD = 2, EPI_SPLITK = 4, EPI_ADD_BITS = 8 };
+
+// Partial tiles go from registers to memory: split-K kernels leave the staging tiles' shared memory to loads in flight.
+constexpr int staging_bytes(int epi) { return (epi & EPI_SPLITK) ? 0 : STAGING_BYTES; }
+static_assert((SMEM_LIMIT - SMEM_FIXED - staging_bytes(EPI_SPLITK)) / (A_BYTES + BN * BK * 2) >= 4, "stages of a split-K tile of 256 columns");
+// Ring of a split-K product of one or two output tiles.  It reads each operand once, out of DRAM, and every CTA's ring adds to the
+// streams open there; a product of more tiles reads them again, out of L2, whose latency wants all that fits.  Measured, weight
+// gradients of 1x1 convolutions, with 160 KB and with all (227) of it: 64 -> 256 channels of 256 x 56 x 56 86.9 us, 91.6; 256 -> 64
+// 95.8, 98.3; 512 -> 128 of 28 x 28 62.0, 62.6; but 1024 -> 256 of 14 x 14 (eight tiles) 55.5, 51.4; 512 -> 2048 of 7 x 7 41.3, 39.2.
+constexpr long SPLITK_STREAM_RING = 160 << 10;
 
 struct Shared {
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], b_full, add_full[EPI_WARPS][RING];
@@ -489,7 +498,7 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   unsigned char* tiles = (unsigned char*)base;
   unsigned char* b_res = tiles + (size_t)p.stages * p.stage_bytes;
   unsigned char* staging = b_res + (p.b_resident ? (size_t)p.k_blocks_total * p.b_block_bytes : 0);
-  float* stats = (float*)(staging + STAGING_BYTES);
+  float* stats = (float*)(staging + staging_bytes(EPI));
   Shared* sh = (Shared*)((unsigned char*)stats + p.stat_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && sm100::elect_one()) {
@@ -676,7 +685,9 @@ static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const void*
   p.status = conv_status_word();
   p.b_block_bytes = p.mma_n * conv::BK * 2;
   p.stat_bytes = (p.epi & conv::EPI_STATS) ? conv::EPI_WARPS * 2 * conv::BN * (int)sizeof(float) : 0;
-  const long budget = (long)conv::SMEM_LIMIT - (long)conv::SMEM_FIXED - p.stat_bytes;
+  const size_t fixed = conv::SMEM_FIXED + conv::staging_bytes(p.epi) + p.stat_bytes;
+  long budget = (long)conv::SMEM_LIMIT - (long)fixed;
+  if ((p.epi & conv::EPI_SPLITK) && p.tiles_m * p.tiles_n <= 2) budget = std::min(budget, conv::SPLITK_STREAM_RING);
   const long b_all = (long)p.k_blocks_total * p.b_block_bytes;
   p.b_resident = 0;
   if (p.tiles_n == 1 && p.slices == 1 && b_all < (1 << 20) && (budget - b_all) / conv::A_BYTES >= 5) {
@@ -688,7 +699,7 @@ static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const void*
     p.stages = (int)std::min<long>(conv::MAX_STAGES, budget / p.stage_bytes);
   }
   if (p.stages < 2) return fail(TMPI_ERR_UNSUPPORTED, "conv: shared memory plan leaves %d stages", p.stages);
-  const size_t smem = conv::SMEM_FIXED + p.stat_bytes + (size_t)p.stages * p.stage_bytes + (p.b_resident ? (size_t)b_all : 0);
+  const size_t smem = fixed + (size_t)p.stages * p.stage_bytes + (p.b_resident ? (size_t)b_all : 0);
   const int items = p.tiles_m * p.tiles_n * p.slices;
   int grid = std::min(items, gemm_sm_count());
   // statistics: a CTA keeps sums for one window of 256 columns, so every tile it visits must have the same n_blk
