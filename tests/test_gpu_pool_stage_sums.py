@@ -33,3 +33,38 @@ def test_pool_stage_keeps_inputs_and_positions(dtype, N, C, H, W):
     open_ = (ref > 0).double() * dy.double()
     assert (m.bias.grad.double() - open_.sum((0, 2, 3))).abs().max() <= 2e-6 * ref.numel() / C + 1e-5
     assert (m.weight.grad.double() - (open_ * kept.double() * (1 + m.eps) ** -0.5).sum((0, 2, 3))).abs().max() <= 1e-5 * ref.numel() / C + 1e-4
+
+
+# packs of four and eight channels, both element sizes; odd sizes, several strips
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("N,C,H,W", [(1, 8, 1, 1), (2, 64, 30, 31), (1, 2048, 5, 4)])
+def test_pool_stage_entries_without_kept_inputs(dtype, N, C, H, W):
+    """The C entries that take no kept inputs sum over all of x; they give what the ones with kept inputs give."""
+    from torchmpi_b200._lib import check, dtype_code, lib, stream_ptr
+    if 256 % (C // (16 // dtype.itemsize)):
+        pytest.skip("channels the kernel does not take")
+    torch.manual_seed(C + H)
+    x = (torch.randn(N, H, W, C, device="cuda") + 0.25).to(dtype)
+    gamma, beta = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda") * 0.1
+    out = (N, (H - 1) // 2 + 1, (W - 1) // 2 + 1, C)
+    dy = torch.randn(out, device="cuda").to(dtype)
+    got = []
+    for keep in (False, True):
+        y, idx, xmax = torch.empty_like(dy), torch.empty(out, dtype=torch.uint8, device="cuda"), torch.empty_like(dy)
+        mean, invstd, dgamma, dbeta = (torch.empty(C, device="cuda") for _ in range(4))
+        dx, scratch = torch.empty_like(x), torch.empty(lib.tmpi_bn_scratch_bytes(C), dtype=torch.uint8, device="cuda")
+        kept = [xmax.data_ptr()] if keep else []
+        fwd, bwd = ((lib.tmpi_bn_relu_pool_fwd_keep, lib.tmpi_bn_relu_pool_bwd_kept) if keep else
+                    (lib.tmpi_bn_relu_pool_fwd, lib.tmpi_bn_relu_pool_bwd))
+        check(fwd(x.data_ptr(), y.data_ptr(), idx.data_ptr(), *kept, gamma.data_ptr(), beta.data_ptr(), None, None, mean.data_ptr(),
+                  invstd.data_ptr(), N, H, W, C, 1e-5, 0.1, 1, dtype_code(dtype), scratch.data_ptr(), stream_ptr()))
+        check(bwd(x.data_ptr(), *kept, dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(), mean.data_ptr(),
+                  invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(dtype), scratch.data_ptr(), stream_ptr()))
+        got.append((y, idx, dx, dgamma, dbeta))
+    (y0, idx0, dx0, dg0, db0), (y1, idx1, dx1, dg1, db1) = got
+    assert torch.equal(y0, y1) and torch.equal(idx0, idx1)
+    # the same terms of order one in another order, in fp32; dx is rounded to its type after that
+    terms = N * out[1] * out[2]
+    assert (dg0 - dg1).abs().max() <= 2e-6 * terms + 1e-5 and (db0 - db1).abs().max() <= 2e-6 * terms + 1e-5
+    eps = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -9, torch.float32: 1e-5}[dtype]
+    assert (dx0.float() - dx1.float()).abs().max() <= eps * dx1.float().abs().max() + 1e-6

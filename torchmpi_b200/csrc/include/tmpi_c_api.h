@@ -312,14 +312,23 @@ size_t tmpi_gemm_tn_splitk_workspace_bytes(int M, int N, int64_t K);
 int tmpi_gemm_bf16_tn_splitk(const void* A, const void* B, void* C, int M, int N, int64_t K, int64_t lda, int64_t ldb,
                              void* workspace, size_t workspace_bytes, int accumulate, void* stream);
 // batch-norm + ReLU + max-pool (3x3, stride 2, pad 1) as one stage; y, idx: [N, (H-1)/2+1, (W-1)/2+1, C]
-int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta,
+int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, const float* gamma, const float* beta,
                           float* running_mean, float* running_var, float* save_mean, float* save_invstd,
                           int N, int H, int W, int channels, float eps, float momentum, int training,
                           int dtype, void* scratch, void* stream);
-int tmpi_bn_relu_pool_bwd(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma,
+int tmpi_bn_relu_pool_bwd(const void* x, const void* dy, const void* idx, void* dx, const float* gamma,
                           const float* beta, const float* save_mean, const float* save_invstd,
                           float* dgamma, float* dbeta, int N, int H, int W, int channels, int dtype,
                           void* scratch, void* stream);
+// the same with xmax (nullable), shaped like y: the input at each window's maximum, from which backward forms its sums
+int tmpi_bn_relu_pool_fwd_keep(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta,
+                               float* running_mean, float* running_var, float* save_mean, float* save_invstd,
+                               int N, int H, int W, int channels, float eps, float momentum, int training,
+                               int dtype, void* scratch, void* stream);
+int tmpi_bn_relu_pool_bwd_kept(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma,
+                               const float* beta, const float* save_mean, const float* save_invstd,
+                               float* dgamma, float* dbeta, int N, int H, int W, int channels, int dtype,
+                               void* scratch, void* stream);
 // channels-last max pooling; idx holds one byte per output element (position inside the window)
 int tmpi_maxpool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, int OH, int OW,
                      int k, int s, int p, int dtype, void* stream);

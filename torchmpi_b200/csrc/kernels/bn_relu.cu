@@ -673,6 +673,45 @@ __device__ __forceinline__ void bp_walk_strips(const T* __restrict__ x, const T*
   }
 }
 
+// backward statistics without the kept inputs: sums of dz and dz * (x - mean) per channel over all positions of x, one partial
+// row per block.  256 x 112 x 112 x 64 bf16: 137 us, against 36 over the kept inputs.
+template <typename T, int V, int BLOCKS>
+__global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_reduce_kernel(
+    const T* __restrict__ x, const T* __restrict__ dy, const unsigned char* __restrict__ idx, const float* __restrict__ mean,
+    const float* __restrict__ invstd, BpDims d, BpWalk walk, float* __restrict__ partial) {
+  const int cvn = d.C / V, cv = threadIdx.x % cvn;                // kBpThreads is a multiple of cvn
+  float a[V], b[V], mu[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) { a[k] = 0.f; b[k] = 0.f; mu[k] = mean[cv * V + k]; }
+  bp_walk_strips<T, V>(x, dy, idx, d, walk, [&](const BpWords<V * sizeof(T) / 4> (&xv)[4], size_t, const int (&)[4], const BpWindow<T, V> (&w)[2][2], const bool (&in)[4]) {
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      float g[4];
+      bp_route<T, V>(w, c, g);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!in[q]) continue;
+        a[c] += g[q];
+        b[c] += g[q] * (bp_get<T>(xv[q], c) - mu[c]);
+      }
+    }
+  });
+  __shared__ float s[kBpThreads][2 * V + 1];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    s[threadIdx.x][k] = a[k];
+    s[threadIdx.x][V + k] = b[k] * invstd[cv * V + k];
+  }
+  __syncthreads();
+  for (int o = threadIdx.x; o < cvn * 2 * V; o += kBpThreads) {
+    const int c = o / (2 * V), k = o % (2 * V);
+    float t = 0.f;
+    for (int g = c; g < kBpThreads; g += cvn) t += s[g][k];
+    const int which = k / V, ch = c * V + (k % V);
+    partial[((size_t)blockIdx.x * 2 + which) * d.C + ch] = t;
+  }
+}
+
 // backward apply; measured, 256 x 112 x 112 x 64 bf16: 179 us (208 with the gradient that the pool had written, 411 MB, to read).
 template <typename T, int V, int BLOCKS>
 __global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_apply_kernel(
@@ -754,6 +793,18 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, void* xmax, const fl
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn+pool forward launch: %s", cudaGetErrorString(e));
 }
 
+// returns the rows of partial sums: one resident wave of blocks
+template <typename T, int V, int BLOCKS>
+static int bn_pool_bwd_reduce(const void* x, const void* dy, const void* idx, const float* smean, const float* sinv, const BpDims& d,
+                              void* scratch, cudaStream_t s) {
+  static_assert(148 * BLOCKS <= kBnMaxGrid, "partial rows in scratch");
+  const BpWalk walk = bp_walk<V>(d);
+  const int grid = (int)std::min<long long>((walk.items + kBpThreads - 1) / kBpThreads, 148 * BLOCKS);
+  bn_pool_bwd_reduce_kernel<T, V, BLOCKS><<<grid, kBpThreads, 0, s>>>((const T*)x, (const T*)dy, (const unsigned char*)idx, smean, sinv, d,
+                                                                      walk, (float*)scratch);
+  return grid;
+}
+
 template <typename T, int V, int BLOCKS>
 static void bn_pool_bwd_apply(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* smean,
                               const float* sinv, const float* dgamma, const float* dbeta, const BpDims& d, cudaStream_t s) {
@@ -772,18 +823,26 @@ static int bn_pool_bwd_t(const void* x, const void* xmax, const void* dy, const 
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
   int st = bn_pool_check(rows, d, V);
   if (st) return st;
-  // The sums: dz is zero but at the maximum of each open window, so they run over the pooled positions, with the input that
-  // the forward kept for each and the ReLU mask that it implies.  256 x 112 x 112 x 64 bf16: 36 us (206 MB; 136 over
-  // all positions of x, 411 MB, with the gradient routed to each).
-  const size_t nvec = (size_t)N * d.OH * d.OW * (C / V);
-  const int grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU);
-  bn_reduce_kernel<T, V, true, MASK_X_ROUNDED><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
-                                                                           nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
+  const bool fours = sizeof(T) == 2 && kBpThreads % (C / 4) == 0;       // packs of four channels, see below
+  int grid;
+  if (xmax) {
+    // The sums: dz is zero but at the maximum of each open window, so they run over the pooled positions, with the input that
+    // the forward kept for each and the ReLU mask that it implies.  256 x 112 x 112 x 64 bf16: 36 us (206 MB; 136 over
+    // all positions of x, 411 MB, with the gradient routed to each).
+    const size_t nvec = (size_t)N * d.OH * d.OW * (C / V);
+    grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU);
+    bn_reduce_kernel<T, V, true, MASK_X_ROUNDED><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
+                                                                             nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
+  } else if (fours) {
+    grid = bn_pool_bwd_reduce<T, sizeof(T) == 2 ? 4 : V, sizeof(T) == 2 ? 3 : 2>(x, dy, idx, smean, sinv, d, scratch, s);
+  } else {
+    grid = bn_pool_bwd_reduce<T, V, 2>(x, dy, idx, smean, sinv, d, scratch, s);
+  }
   bn_finalize_bwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, dgamma, dbeta);
   // 16-bit types: packs of four channels where their groups divide the block (up to 1024 channels).  They halve the
   // per-channel state, so that three blocks fit on an SM instead of two (256 x 112 x 112 x 64: 254 -> 179 us).
   if constexpr (sizeof(T) == 2) {
-    if (kBpThreads % (C / 4) == 0) bn_pool_bwd_apply<T, 4, 3>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
+    if (fours) bn_pool_bwd_apply<T, 4, 3>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
     else bn_pool_bwd_apply<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
   } else {
     bn_pool_bwd_apply<T, V, 2>(x, dy, idx, dx, gamma, smean, sinv, dgamma, dbeta, d, s);
@@ -869,9 +928,9 @@ int tmpi_bn_relu_bwd_acc(const void* x, const void* y, const void* dy, void* dx,
 
 // Batch-norm + ReLU + max-pool (3x3, stride 2, pad 1) in one stage.  x: [N, H, W, C] channels-last;
 // y, idx: [N, OH, OW, C] with OH = (H - 1) / 2 + 1.  Other arguments as tmpi_bn_relu_fwd / _bwd.
-// xmax (nullable): [N, OH, OW, C], the input at each window's maximum, which backward needs.
-int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta, float* running_mean,
-                          float* running_var, float* save_mean, float* save_invstd, int N, int H, int W, int channels,
+// xmax (nullable): [N, OH, OW, C], the input at each window's maximum; backward forms its sums from it, or over x without it.
+int tmpi_bn_relu_pool_fwd_keep(const void* x, void* y, void* idx, void* xmax, const float* gamma, const float* beta, float* running_mean,
+                               float* running_var, float* save_mean, float* save_invstd, int N, int H, int W, int channels,
                           float eps, float momentum, int training, int dtype, void* scratch, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   switch (dtype) {
@@ -885,7 +944,7 @@ int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, void* xmax, const f
   return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: dtype %d", dtype);
 }
 
-int tmpi_bn_relu_pool_bwd(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
+int tmpi_bn_relu_pool_bwd_kept(const void* x, const void* xmax, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
                           const float* save_mean, const float* save_invstd, float* dgamma, float* dbeta, int N, int H, int W,
                           int channels, int dtype, void* scratch, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
@@ -898,6 +957,20 @@ int tmpi_bn_relu_pool_bwd(const void* x, const void* xmax, const void* dy, const
                                                scratch, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: dtype %d", dtype);
+}
+
+int tmpi_bn_relu_pool_fwd(const void* x, void* y, void* idx, const float* gamma, const float* beta, float* running_mean,
+                          float* running_var, float* save_mean, float* save_invstd, int N, int H, int W, int channels,
+                          float eps, float momentum, int training, int dtype, void* scratch, void* stream) {
+  return tmpi_bn_relu_pool_fwd_keep(x, y, idx, nullptr, gamma, beta, running_mean, running_var, save_mean, save_invstd, N, H, W, channels,
+                                    eps, momentum, training, dtype, scratch, stream);
+}
+
+int tmpi_bn_relu_pool_bwd(const void* x, const void* dy, const void* idx, void* dx, const float* gamma, const float* beta,
+                          const float* save_mean, const float* save_invstd, float* dgamma, float* dbeta, int N, int H, int W,
+                          int channels, int dtype, void* scratch, void* stream) {
+  return tmpi_bn_relu_pool_bwd_kept(x, nullptr, dy, idx, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, N, H, W, channels, dtype,
+                                    scratch, stream);
 }
 
 }  // extern "C"

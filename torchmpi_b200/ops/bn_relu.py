@@ -149,7 +149,7 @@ class _BnReluPoolFn(torch.autograd.Function):
         else:
             mean = running_mean.float()
             invstd = torch.rsqrt(running_var.float() + eps)
-        check(lib.tmpi_bn_relu_pool_fwd(
+        check(lib.tmpi_bn_relu_pool_fwd_keep(
             x.data_ptr(), y.data_ptr(), idx.data_ptr(), xmax.data_ptr() if xmax is not None else None, gamma.data_ptr(), beta.data_ptr(),
             running_mean.data_ptr() if (training and running_mean is not None) else None,
             running_var.data_ptr() if (training and running_var is not None) else None,
@@ -171,7 +171,7 @@ class _BnReluPoolFn(torch.autograd.Function):
         if xmax is not None:
             # one stage: the sums run over the pooled positions, the apply pass rebuilds the pool's gradient routing from dy and
             # the index
-            check(lib.tmpi_bn_relu_pool_bwd(
+            check(lib.tmpi_bn_relu_pool_bwd_kept(
                 x.data_ptr(), xmax.data_ptr(), dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
                 mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
                 _scratch_for(x.device, C).data_ptr(), stream_ptr()))
