@@ -68,3 +68,37 @@ def test_pool_stage_entries_without_kept_inputs(dtype, N, C, H, W):
     assert (dg0 - dg1).abs().max() <= 2e-6 * terms + 1e-5 and (db0 - db1).abs().max() <= 2e-6 * terms + 1e-5
     eps = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -9, torch.float32: 1e-5}[dtype]
     assert (dx0.float() - dx1.float()).abs().max() <= eps * dx1.float().abs().max() + 1e-6
+
+
+def test_pool_stage_keeps_nothing_without_gradients():
+    """Inference allocates the output and its index, not the inputs that only a backward reads; neither setting of the backward's
+    tunable has to be the one that held during forward."""
+    from torchmpi_b200 import config
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLUMaxPool
+    m = FusedBatchNormReLUMaxPool(64).cuda()
+    x = torch.randn(16, 112, 112, 64, device="cuda").to(torch.bfloat16).permute(0, 3, 1, 2)
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            m(x)
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            y = m(x)
+            out = y.numel()
+            assert torch.cuda.max_memory_allocated() - before <= 3 * out + (2 << 20)       # y, the index and what the allocator leaves unsplit
+    grads = []
+    for fwd, bwd in ((1, 1), (0, 1), (1, 0)):
+        try:
+            config.set("bn_pool_fused_bwd", fwd)
+            xs = x.detach().requires_grad_(True)
+            m.zero_grad(set_to_none=True)
+            y = m(xs)
+            config.set("bn_pool_fused_bwd", bwd)
+            y.backward(torch.ones_like(y))
+        finally:
+            config.set("bn_pool_fused_bwd", 1)
+        grads.append((xs.grad, m.weight.grad, m.bias.grad))
+    for dx, dg, db in grads[1:]:
+        # sums of 50176 terms of order one in fp32, in another order; bf16 gradients of positions under several windows
+        assert (dg - grads[0][1]).abs().max() < 0.1 and (db - grads[0][2]).abs().max() < 0.1
+        assert (dx.float() - grads[0][0].float()).norm() <= 1e-2 * grads[0][0].float().norm()

@@ -134,15 +134,16 @@ class _BnReluPoolFn(torch.autograd.Function):
     """``max_pool2d(relu(batch_norm(x)), 3, 2, 1)`` without materialising the full-resolution activation."""
 
     @staticmethod
-    def forward(ctx, x, gamma, beta, running_mean, running_var, eps, momentum, training):
+    def forward(ctx, x, gamma, beta, running_mean, running_var, eps, momentum, training, grad_mode):
         global launch_count
         x = x.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         OH, OW = (H - 1) // 2 + 1, (W - 1) // 2 + 1
         y = torch.empty((N, C, OH, OW), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
         idx = torch.empty((N, OH, OW, C), dtype=torch.uint8, device=x.device)
-        # the input at each window's maximum, from which backward forms its sums
-        xmax = torch.empty_like(y) if any(ctx.needs_input_grad) and config.get("bn_pool_fused_bwd") else None
+        # the input at each window's maximum, from which backward forms its sums (held until then: as large as y).  Where no
+        # backward can follow (needs_input_grad does not know of no_grad) it is not kept.
+        xmax = torch.empty_like(y) if grad_mode and any(ctx.needs_input_grad) else None
         if training:
             mean = torch.empty(C, dtype=torch.float32, device=x.device)
             invstd = torch.empty(C, dtype=torch.float32, device=x.device)
@@ -168,11 +169,11 @@ class _BnReluPoolFn(torch.autograd.Function):
         dx = torch.empty_like(x, memory_format=torch.channels_last)
         dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
         dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
-        if xmax is not None:
+        if config.get("bn_pool_fused_bwd"):
             # one stage: the sums run over the pooled positions, the apply pass rebuilds the pool's gradient routing from dy and
             # the index
             check(lib.tmpi_bn_relu_pool_bwd_kept(
-                x.data_ptr(), xmax.data_ptr(), dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+                x.data_ptr(), xmax.data_ptr() if xmax is not None else None, dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
                 mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
                 _scratch_for(x.device, C).data_ptr(), stream_ptr()))
             launch_count += 3
@@ -188,7 +189,7 @@ class _BnReluPoolFn(torch.autograd.Function):
                 mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N * H * W, C, 1,
                 dtype_code(x.dtype), None, _scratch_for(x.device, C).data_ptr(), stream_ptr()))
             launch_count += 4
-        return dx, dgamma, dbeta, None, None, None, None, None
+        return dx, dgamma, dbeta, None, None, None, None, None, None
 
 
 class FusedBatchNormReLUMaxPool(nn.BatchNorm2d):
@@ -201,7 +202,7 @@ class FusedBatchNormReLUMaxPool(nn.BatchNorm2d):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if supported(x) and self.weight.dtype == torch.float32 and has_symbol("tmpi_bn_relu_pool_fwd"):
             return _BnReluPoolFn.apply(x, self.weight, self.bias, self.running_mean, self.running_var, self.eps,
-                                       self.momentum, self.training)
+                                       self.momentum, self.training, torch.is_grad_enabled())
         out = torch.relu(F.batch_norm(x, self.running_mean, self.running_var, self.weight, self.bias, self.training,
                                       self.momentum, self.eps))
         return F.max_pool2d(out, 3, 2, 1)
