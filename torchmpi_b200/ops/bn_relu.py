@@ -21,12 +21,14 @@ launch_count = 0
 _scratch = {}
 
 
-def _scratch_for(dev: torch.device, C: int) -> torch.Tensor:
-    key = (dev.index, stream_ptr())
-    need = lib.tmpi_bn_scratch_bytes(C)
+def _scratch_for(dev: torch.device, C: int, stream: Optional[int] = None) -> torch.Tensor:
+    key = (dev.index, stream_ptr() if stream is None else stream)
     buf = _scratch.get(key)
+    if buf is not None and C <= 2048:                    # every buffer holds at least as much as 2048 channels need
+        return buf
+    need = lib.tmpi_bn_scratch_bytes(max(C, 2048))
     if buf is None or buf.numel() < need:
-        buf = _scratch[key] = torch.empty(max(need, lib.tmpi_bn_scratch_bytes(2048)), dtype=torch.uint8, device=dev)
+        buf = _scratch[key] = torch.empty(need, dtype=torch.uint8, device=dev)
     return buf
 
 
@@ -130,6 +132,11 @@ class _BnReluFn(torch.autograd.Function):
         return dx, dres, dgamma, dbeta, None, None, None, None, None, None, None, None, None
 
 
+def _invstd_ptr(mean: torch.Tensor, invstd: Optional[torch.Tensor]) -> int:
+    """Where 1 / std is: a tensor of its own, or the second half of ``mean``'s (one allocation per call fewer)."""
+    return invstd.data_ptr() if invstd is not None else mean.data_ptr() + 2 * mean.numel()
+
+
 class _BnReluPoolFn(torch.autograd.Function):
     """``max_pool2d(relu(batch_norm(x)), 3, 2, 1)`` without materialising the full-resolution activation."""
 
@@ -145,17 +152,17 @@ class _BnReluPoolFn(torch.autograd.Function):
         # backward can follow (needs_input_grad does not know of no_grad) it is not kept.
         xmax = torch.empty_like(y) if grad_mode and any(ctx.needs_input_grad) else None
         if training:
-            mean = torch.empty(C, dtype=torch.float32, device=x.device)
-            invstd = torch.empty(C, dtype=torch.float32, device=x.device)
+            mean, invstd = torch.empty(2 * C, dtype=torch.float32, device=x.device), None      # 1 / std behind the mean
         else:
             mean = running_mean.float()
             invstd = torch.rsqrt(running_var.float() + eps)
+        stream = stream_ptr()
         check(lib.tmpi_bn_relu_pool_fwd_keep(
             x.data_ptr(), y.data_ptr(), idx.data_ptr(), xmax.data_ptr() if xmax is not None else None, gamma.data_ptr(), beta.data_ptr(),
             running_mean.data_ptr() if (training and running_mean is not None) else None,
             running_var.data_ptr() if (training and running_var is not None) else None,
-            mean.data_ptr(), invstd.data_ptr(), N, H, W, C, eps, momentum, int(training), dtype_code(x.dtype),
-            _scratch_for(x.device, C).data_ptr(), stream_ptr()))
+            mean.data_ptr(), _invstd_ptr(mean, invstd), N, H, W, C, eps, momentum, int(training), dtype_code(x.dtype),
+            _scratch_for(x.device, C, stream).data_ptr(), stream))
         launch_count += 3 if training else 1
         ctx.save_for_backward(x, xmax, idx, gamma, beta, mean, invstd)
         return y
@@ -169,13 +176,14 @@ class _BnReluPoolFn(torch.autograd.Function):
         dx = torch.empty_like(x, memory_format=torch.channels_last)
         dgamma = torch.empty(C, dtype=torch.float32, device=x.device)
         dbeta = torch.empty(C, dtype=torch.float32, device=x.device)
+        stream = stream_ptr()
         if config.get("bn_pool_fused_bwd"):
             # one stage: the sums run over the pooled positions, the apply pass rebuilds the pool's gradient routing from dy and
             # the index
             check(lib.tmpi_bn_relu_pool_bwd_kept(
                 x.data_ptr(), xmax.data_ptr() if xmax is not None else None, dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-                mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
-                _scratch_for(x.device, C).data_ptr(), stream_ptr()))
+                mean.data_ptr(), _invstd_ptr(mean, invstd), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
+                _scratch_for(x.device, C, stream).data_ptr(), stream))
             launch_count += 3
         else:
             # in two stages: route the gradient through the pool, then the batch-norm backward with the ReLU mask
@@ -186,8 +194,8 @@ class _BnReluPoolFn(torch.autograd.Function):
                                        dtype_code(x.dtype), stream_ptr()))
             check(lib.tmpi_bn_relu_bwd(
                 x.data_ptr(), None, da.data_ptr(), dx.data_ptr(), None, gamma.data_ptr(), beta.data_ptr(),
-                mean.data_ptr(), invstd.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), N * H * W, C, 1,
-                dtype_code(x.dtype), None, _scratch_for(x.device, C).data_ptr(), stream_ptr()))
+                mean.data_ptr(), _invstd_ptr(mean, invstd), dgamma.data_ptr(), dbeta.data_ptr(), N * H * W, C, 1,
+                dtype_code(x.dtype), None, _scratch_for(x.device, C, stream).data_ptr(), stream))
             launch_count += 4
         return dx, dgamma, dbeta, None, None, None, None, None, None
 

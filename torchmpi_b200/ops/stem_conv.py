@@ -12,6 +12,7 @@ saved patch matrix.  Inputs that neither takes go to ``F.conv2d``.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 import torch.nn as nn
@@ -22,6 +23,12 @@ from . import gemm
 
 launch_count = 0
 PATCH = 147
+_Strides = ctypes.c_int64 * 4
+
+
+@functools.lru_cache(maxsize=None)
+def _wgrad_workspace_bytes() -> int:
+    return lib.tmpi_stem_conv_wgrad_workspace_bytes()            # of the chip, not of the call
 
 
 class _StemDirectFn(torch.autograd.Function):
@@ -34,7 +41,7 @@ class _StemDirectFn(torch.autograd.Function):
         y = torch.empty((N, w.shape[0], (H - 1) // 2 + 1, (W - 1) // 2 + 1), dtype=x.dtype, device=x.device,
                         memory_format=torch.channels_last)
         check(lib.tmpi_stem_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, w.shape[0],
-                                     (ctypes.c_int64 * 4)(*w.stride()), stream_ptr()))
+                                     _Strides(*w.stride()), stream_ptr()))
         launch_count += 1
         ctx.save_for_backward(x)
         ctx.wshape, ctx.wstride = tuple(w.shape), w.stride()
@@ -50,9 +57,9 @@ class _StemDirectFn(torch.autograd.Function):
             dy = dy.clone(memory_format=torch.channels_last)
         dw = torch.empty_strided(ctx.wshape, ctx.wstride, dtype=x.dtype, device=x.device)
         # partial sums of the CTAs (24 MB), from the allocator: calls on other streams, threads and in graphs have their own
-        ws = torch.empty(lib.tmpi_stem_conv_wgrad_workspace_bytes(), dtype=torch.uint8, device=x.device)
+        ws = torch.empty(_wgrad_workspace_bytes(), dtype=torch.uint8, device=x.device)
         check(lib.tmpi_stem_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, H, W, ctx.wshape[0],
-                                       (ctypes.c_int64 * 4)(*dw.stride()), ws.data_ptr(), ws.numel(), stream_ptr()))
+                                       _Strides(*ctx.wstride), ws.data_ptr(), _wgrad_workspace_bytes(), stream_ptr()))
         launch_count += 2
         return None, dw
 
