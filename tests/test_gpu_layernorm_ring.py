@@ -13,7 +13,7 @@ EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10, torch.float32: 2e-6
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows", [1, 7, 1184, 4737, 6000])
 def test_layer_norm_backward_ring(dtype, rows):
-    from torchmpi_b200.ops.layernorm import LayerNorm, supported
+    from torchmpi_b200.ops.layernorm import LayerNorm, check_status, supported
     unit = 128 if dtype == torch.float32 else 256
     for C in (unit, 3 * unit, 4 * unit, 8 * unit):
         torch.manual_seed(C)
@@ -24,6 +24,7 @@ def test_layer_norm_backward_ring(dtype, rows):
         assert supported(x, m.weight, m.bias)
         dy = torch.randn(rows, C, device="cuda").to(dtype)
         m(x).backward(dy)
+        check_status()
         xr, w, b = x.detach().double().requires_grad_(True), m.weight.detach().double().requires_grad_(True), m.bias.detach().double().requires_grad_(True)
         F.layer_norm(xr, (C,), w, b, m.eps).backward(dy.double())
         eps = EPS[dtype]

@@ -1,0 +1,15 @@
+"""A bounded wait that ran out is reported by the module whose function launched the kernel."""
+import types
+
+import pytest
+
+
+def test_layer_norm_reports_its_own_waits(monkeypatch):
+    from torchmpi_b200._lib import TorchMPIError
+    from torchmpi_b200.ops import gemm, layernorm
+    fake = types.SimpleNamespace(tmpi_layernorm_status=lambda: 4001, tmpi_gemm_status=lambda: 0, tmpi_conv_status=lambda: 0)
+    monkeypatch.setattr(layernorm, "lib", fake)
+    monkeypatch.setattr(gemm, "lib", fake)
+    with pytest.raises(TorchMPIError, match="layer norm.*4001"):
+        layernorm.check_status()
+    gemm.check_status()

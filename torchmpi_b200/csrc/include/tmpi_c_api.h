@@ -254,6 +254,7 @@ int tmpi_layernorm_fwd(const void* x, const void* gamma, const void* beta, void*
 int tmpi_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                        void* dx, void* dgamma, void* dbeta, int rows, int channels, int dtype, void* scratch,
                        void* stream);
+int tmpi_layernorm_status(void);
 int tmpi_bn_relu_fwd(const void* x, const void* residual, void* y, const float* gamma,
                      const float* beta, float* running_mean, float* running_var,
                      float* save_mean, float* save_invstd, int64_t rows, int channels,

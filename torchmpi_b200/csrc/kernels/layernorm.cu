@@ -17,7 +17,9 @@
 
 namespace tmpi {
 
-int* gemm_status_word();
+// Set where a backward gave up on a bounded wait.  On the device: nothing has to be allocated on a first call, which may be
+// inside a graph capture.
+static __device__ int g_ln_status;
 
 constexpr int kLnThreads = 256, kLnWarps = kLnThreads / 32;
 constexpr int kLnMaxGrid = 296;           // forward: two blocks per SM; backward (about 200 registers): half of it, one per SM
@@ -84,7 +86,7 @@ template <typename T, int V, int NP>
 __global__ void __launch_bounds__(kLnThreads) ln_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                             const T* __restrict__ gamma, const float* __restrict__ mean,
                                                             const float* __restrict__ rstd, T* __restrict__ dx,
-                                                            float* __restrict__ partial, int rows, int* status) {
+                                                            float* __restrict__ partial, int rows) {
   constexpr int C = 32 * NP * V, ROW = C * (int)sizeof(T), RING = ln_ring(NP);
   extern __shared__ __align__(128) unsigned char ln_smem[];
   __shared__ uint64_t full[kLnWarps][RING];
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_bwd_kernel(const T* __restrict_
     const float mu = mu_next, rs = rs_next;
     if (r + stride < rows) { mu_next = mean[r + stride]; rs_next = rstd[r + stride]; }
     if (!__all_sync(~0u, sm100::mbar_wait(&full[warp][k], phase, 2000000000ull))) {
-      if (status && lane == 0) atomicCAS(status, 0, 1090);
+      if (lane == 0) atomicCAS(&g_ln_status, 0, 4001);
       const unsigned long long t0 = sm100::now_ns();
       while (sm100::now_ns() - t0 < 200000000ull) { __nanosleep(1000); }   // copies in flight land within microseconds
       break;
@@ -218,7 +220,7 @@ static cudaError_t ln_launch(bool fwd, const void* x, const void* a, const void*
   cudaError_t e = cudaFuncSetAttribute(ln_bwd_kernel<T, V, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   e = launch_overlapped(ln_bwd_kernel<T, V, NP>, grid, kLnThreads, smem, s, (const T*)x, (const T*)a, (const T*)gamma, mean, rstd, (T*)out,
-                        partial, rows, gemm_status_word());
+                        partial, rows);
   if (e != cudaSuccess) return e;
   return launch_overlapped(ln_finalize_kernel<T>, 2 * C / 32, 32 * kLnFinGroups, 0, s, partial, grid, C, (T*)dgamma, (T*)dbeta);
 }
@@ -284,6 +286,16 @@ int tmpi_layernorm_bwd(const void* x, const void* dy, const void* gamma, const f
     case TMPI_F32: return ln_dispatch<float>(false, x, dy, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "layernorm: dtype %d", dtype);
+}
+
+// Non-zero after a layer-norm backward on the current device gave up on a bounded wait (rows of its dx are missing); clears it.
+// Waits for the device's work on the default stream.
+int tmpi_layernorm_status(void) {
+  int v = 0;
+  const int zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_ln_status, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return 0; }
+  if (v) cudaMemcpyToSymbol(g_ln_status, &zero, sizeof(zero));
+  return v;
 }
 
 }  // extern "C"

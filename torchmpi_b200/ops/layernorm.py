@@ -13,7 +13,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .. import _native
-from .._lib import lib, dtype_code, has_symbol
+from .._lib import lib, dtype_code, has_symbol, TorchMPIError
 
 
 def __getattr__(name: str):
@@ -26,6 +26,13 @@ def supported(x: torch.Tensor, weight, bias) -> bool:
     return (x.is_cuda and weight is not None and bias is not None and weight.dtype == x.dtype and bias.dtype == x.dtype
             and x.dtype in (torch.bfloat16, torch.float16, torch.float32) and has_symbol("tmpi_layernorm_fwd")
             and bool(lib.tmpi_layernorm_supported(x.shape[-1], dtype_code(x.dtype))))
+
+
+def check_status() -> None:
+    """Raises if a layer-norm backward on the current device gave up on one of its bounded waits since the last call."""
+    st = lib.tmpi_layernorm_status()
+    if st:
+        raise TorchMPIError(3, f"layer norm: a bounded wait ran out (code {st})")
 
 
 class LayerNorm(nn.LayerNorm):
