@@ -13,3 +13,11 @@ def test_layer_norm_reports_its_own_waits(monkeypatch):
     with pytest.raises(TorchMPIError, match="layer norm.*4001"):
         layernorm.check_status()
     gemm.check_status()
+
+
+def test_linear_reports_waits_of_its_split_weight_gradient(monkeypatch):
+    from torchmpi_b200._lib import TorchMPIError
+    from torchmpi_b200.ops import gemm
+    monkeypatch.setattr(gemm, "lib", types.SimpleNamespace(tmpi_gemm_status=lambda: 0, tmpi_conv_status=lambda: 2006))
+    with pytest.raises(TorchMPIError, match="2006"):
+        gemm.check_status()

@@ -100,8 +100,9 @@ def matmul_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
 
 
 def check_status() -> None:
-    """Raises if a GEMM CTA gave up on one of its bounded waits since the last call."""
-    st = lib.tmpi_gemm_status()
+    """Raises if a GEMM CTA gave up on one of its bounded waits since the last call.  Weight gradients of few tiles and many
+    rows run on the convolution's split-K kernels, which report to the convolution's word."""
+    st = lib.tmpi_gemm_status() or lib.tmpi_conv_status()
     if st:
         raise TorchMPIError(3, f"tcgen05 GEMM: a bounded wait ran out (code {st})")
 
