@@ -21,3 +21,11 @@ def test_linear_reports_waits_of_its_split_weight_gradient(monkeypatch):
     monkeypatch.setattr(gemm, "lib", types.SimpleNamespace(tmpi_gemm_status=lambda: 0, tmpi_conv_status=lambda: 2006))
     with pytest.raises(TorchMPIError, match="2006"):
         gemm.check_status()
+
+
+def test_attention_reports_its_waits(monkeypatch):
+    from torchmpi_b200._lib import TorchMPIError
+    from torchmpi_b200.ops import attention
+    monkeypatch.setattr(attention, "lib", types.SimpleNamespace(tmpi_attention_status=lambda: 3011))
+    with pytest.raises(TorchMPIError, match="3011"):
+        attention.check_status()

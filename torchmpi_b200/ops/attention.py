@@ -57,7 +57,7 @@ def check_status() -> None:
     """Raises if an attention CTA gave up on one of its bounded waits since the last call."""
     st = lib.tmpi_attention_status() or (lib.tmpi_attention_bwd_status() if has_symbol("tmpi_attention_bwd") else 0)
     if st:
-        raise TorchMPIError(f"attention kernel: a bounded wait ran out (code {st})")
+        raise TorchMPIError(3, f"attention kernel: a bounded wait ran out (code {st})")
 
 
 def attention_forward(qkv: torch.Tensor, n_head: int, need_lse: bool = True):
