@@ -75,15 +75,22 @@ __global__ void __launch_bounds__(kLnThreads) ln_fwd_kernel(const T* __restrict_
 // four rows (16 KB at 1024 bf16 columns) per warp are in flight whatever the registers hold; the sums, 64 per lane there,
 // leave no room for a second row in registers, and one row at a time left the memory idle while it was computed.  Measured,
 // 8192 x 1024 bf16, back to back: 19.7 -> 11.4 us (50 MB: 7.7 at the copy rate); 14.3 with nothing in L2, 32768 rows 41.7 (31).
-__host__ __device__ constexpr int ln_ring(int np) { return np <= 6 ? 4 : 3; }      // rows of a warp's ring; 192 KB at most
+__host__ __device__ constexpr int ln_ring(int np) { return np <= 6 ? 4 : 2; }      // rows of a warp's ring, 192 KB at most; of the widest rows
+                                                                                   // three took 61.9 us where two take 56.9 (8192 x 2048 bf16)
+// One block per SM, by a floor of shared memory and for the register allocation.  The grid is one block per SM, but under a launch
+// that overlaps the one before it blocks start as SMs become free, and where several of these fit into one (rows of 1 KB and
+// less: 32 to 64 KB each) the first free SMs got several and others none: 32768 x 256, forward and backward, bf16 47.3 us against
+// 30.6 with the floor, fp32 50.9 against 36.5; 8192 x 256 18.6 against 12.6 (16.5 when rows came into registers).
+constexpr int kLnOneBlock = 116 << 10;
 template <typename T, int NP> constexpr int ln_bwd_smem() {
   const int ring = kLnWarps * ln_ring(NP) * 2 * 32 * NP * 16, sums = kLnWarps * 2 * 32 * NP * 16 / (int)sizeof(T) * 4;
-  return ring > sums ? ring : sums;         // the warps' sums take the ring's place
+  const int need = ring > sums ? ring : sums;         // the warps' sums take the ring's place
+  return need > kLnOneBlock ? need : kLnOneBlock;
 }
 
 // partial[(block * 2 + which) * C + c], which: 0 = dbeta, 1 = dgamma
 template <typename T, int V, int NP>
-__global__ void __launch_bounds__(kLnThreads) ln_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
+__global__ void __launch_bounds__(kLnThreads, 1) ln_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
                                                             const T* __restrict__ gamma, const float* __restrict__ mean,
                                                             const float* __restrict__ rstd, T* __restrict__ dx,
                                                             float* __restrict__ partial, int rows) {
