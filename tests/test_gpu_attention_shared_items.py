@@ -63,7 +63,7 @@ def test_attention_shared_items_non_finite(T):
             assert torch.isnan(y[0, at:]).all()
 
 
-def _forward(qkv, heads, shared):
+def _forward(qkv, heads, shared, scale=0.125):
     """(out, lse) of one form of the kernel: a team per item, or items shared by the two teams of a CTA."""
     from torchmpi_b200._lib import check, lib, stream_ptr
     B, T, C3 = qkv.shape
@@ -71,7 +71,7 @@ def _forward(qkv, heads, shared):
     out = torch.empty((B, T, C), dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty((B, heads, T), dtype=torch.float32, device=qkv.device)
     base = qkv.data_ptr()
-    check(lib.tmpi_attention_fwd_form(base, base + 2 * C, base + 4 * C, C3, out.data_ptr(), C, lse.data_ptr(), B, T, heads, 0.125,
+    check(lib.tmpi_attention_fwd_form(base, base + 2 * C, base + 4 * C, C3, out.data_ptr(), C, lse.data_ptr(), B, T, heads, scale,
                                       int(shared), stream_ptr()))
     return out, lse
 
@@ -79,18 +79,19 @@ def _forward(qkv, heads, shared):
 # keys of whole blocks that score -inf: the middle one, where the second team of the last items starts; the first; the one on the
 # last diagonal, all but its last key; several, so that a team has none or only some of its keys left
 @pytest.mark.parametrize("shared", [False, True])
-@pytest.mark.parametrize("T,keys", [(1024, (512, 640)), (1024, (0, 128)), (1024, (896, 1023)), (1024, (512, 1023)), (1024, (128, 900)),
-                                    (1024, (0, 600)), (384, (256, 383)), (256, (128, 255)), (640, (384, 512))])
-def test_attention_blocks_of_minus_infinity(shared, T, keys):
+@pytest.mark.parametrize("T,keys,scale", [(1024, (512, 640), 0.125), (1024, (0, 128), 0.125), (1024, (896, 1023), 0.125),
+                                          (1024, (512, 1023), 0.125), (1024, (128, 900), 0.125), (1024, (0, 600), 0.125),
+                                          (1024, (0, 600), 0.69), (384, (256, 383), 0.125), (256, (128, 255), 0.125), (640, (384, 512), 0.125)])
+def test_attention_blocks_of_minus_infinity(shared, T, keys, scale):
     from torchmpi_b200.ops import attention
     torch.manual_seed(T + keys[0])
     qkv = _rand(2, T, 192)
     qkv[:, :, 0] = 1.0                                      # first query coordinate: the key's decides the score
     qkv[:, keys[0]:keys[1], 64] = -math.inf
-    y, lse = _forward(qkv, 1, shared)
+    y, lse = _forward(qkv, 1, shared, scale)
     attention.check_status()
     finite = torch.cat([qkv[..., :64], qkv[..., 64:128].nan_to_num(neginf=-1e30), qkv[..., 128:]], -1).double()
-    s = (finite[..., :64] @ finite[..., 64:128].transpose(1, 2)) * 0.125
+    s = (finite[..., :64] @ finite[..., 64:128].transpose(1, 2)) * scale
     s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), -math.inf)
     s = s.masked_fill(s < -1e20, -math.inf)
     ref = torch.softmax(s, -1) @ finite[..., 128:]          # NaN where every key of a row scores -inf

@@ -64,6 +64,7 @@ constexpr int XCH_BYTES = 2 * 2 * BQ * 4;                     // two phases x tw
 constexpr int MERGE_BYTES = 2 * BQ * 4;                       // team 1's row maxima and sums of an item that the teams share
 constexpr int SMEM_BYTES = TEAMS * (SMEM_TILES + SMEM_SHARED + XCH_BYTES) + MERGE_BYTES;
 constexpr int TMEM_COLS = 256, TMEM_P = 128, TMEM_O = 192;    // S: columns 0-127 of a team, P (bf16 pairs): 128-191, O: 192-255
+constexpr float LOWEST = -3.402823466e38f;
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
@@ -118,7 +119,7 @@ template <bool SHARED> struct Items {
       const int half = (qblk + 2) >> 1;
       first = SHARED && team() ? half : 0;
       end = SHARED && !team() ? half : qblk + 1;
-    } while (first == end);
+    } while (SHARED && first == end);
     return true;
   }
 };
@@ -298,8 +299,11 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
       const float next = max_nan(m, mx);
       const bool grew = j > it.first && __any_sync(~0u, next > m);
-      // While every key has scored -inf, scores are taken relative to 0: those keys weigh 0, wherever they lie.
-      const float base = next == -INFINITY ? 0.f : next;
+      // While every key has scored -inf, scores are taken relative to a finite value: those keys weigh 0, wherever they lie.  (One
+      // instruction with an immediate: a comparison and a selection, or a bound from the parameters, cost 8 x 16 x 1024 a
+      // microsecond of 49.4.  LOWEST * c2 is finite for scales up to ln 2; a steeper one is not given shared items, and keys that
+      // score -inf throughout the first block still make a row NaN there.)
+      const float base = max_nan(next, LOWEST);
       const float alpha = ex2((m - base) * c2);
       const unsigned long long al2 = pack2(__float_as_uint(alpha), __float_as_uint(alpha));
       m = next;
@@ -362,6 +366,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       ++merged;
       continue;
     }
+    float inv = 1.f / l;
     ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
     if (tracer) stamp(p, r, it.qblk, 5);
     sm100::tc_fence_after();
@@ -373,9 +378,10 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       ++merged;
       sm100::tc_fence_after();
       const float2 with = merge[row];
-      const float next = max_nan(m, with.x), base = next == -INFINITY ? 0.f : next;      // as in the blocks' loop
+      const float next = max_nan(m, with.x), base = max_nan(next, LOWEST);      // as in the blocks' loop
       const float a0 = ex2((m - base) * c2), a1 = ex2((with.x - base) * c2);
       l = l * a0 + with.y * a1;
+      inv = 1.f / l;
       m = next;
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -387,7 +393,6 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
           o[q * 16 + i] = __float_as_uint(__uint_as_float(o[q * 16 + i]) * a0 + __uint_as_float(o1[i]) * a1);
       }
     }
-    const float inv = 1.f / l;
     sm100::tc_fence_before();
     __syncwarp();
     if (lane == 0) {
@@ -488,16 +493,17 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 static unsigned long long* g_attn_trace = nullptr;
 
-// Half key blocks of the busiest unit (a team, or a CTA whose teams share) of a launch: its items in snake order, as Items deals
-// them, and 2.5 blocks for each (Q and the first S before, the output or the merge after; 1.5 where a shared item is one block and
-// has no merge).  One pass over the units per round, in runs of equal items.
+// Time of the busiest unit (a team, or a CTA whose teams share) of a launch, in twentieths of a key block: its items in snake order,
+// as Items deals them, and two blocks for each (Q and the first S before, the output or the merge after; one where a shared item is
+// one block and has no merge).  A block of an item that is a team's own takes nine tenths of one that is shared.  One pass over
+// the units per round, in runs of equal items.
 static int attention_busiest(int items, int per_block, int q_blocks, int units, bool shared) {
   int load[1024] = {};
   for (int round = 0, t = 0; t < items; ++round) {
     const int end = std::min(items, t + units);
     int at = 0, blocks = q_blocks - t / per_block, run = per_block - t % per_block;
     for (; t < end; --blocks, run = per_block) {
-      const int n = std::min(run, end - t), cost = shared ? (blocks + 1) / 2 * 2 + (blocks > 1 ? 5 : 3) : 2 * blocks + 5;
+      const int n = std::min(run, end - t), cost = shared ? (blocks + 1) / 2 * 20 + (blocks > 1 ? 40 : 20) : 18 * blocks + 40;
       int* l = load + ((round & 1) ? units - at - n : at);
       for (int k = 0; k < n; ++k) l[k] += cost;
       at += n;
@@ -511,11 +517,11 @@ static int attention_busiest(int items, int per_block, int q_blocks, int units, 
 // where there are few, and costs the fixed part twice where there are many; between one and three items per CTA it turns on
 // how many of them the busiest one gets, which an average does not show.  Beyond that a team per item was faster throughout.
 // Measured over 1 - 256 items of each length, lengths of 1 - 32 blocks, on 148 SMs (a team per item, shared, in us): 16 x 16 (heads
-// x blocks) 31.4, 25.0; 37 x 8 19.0, 18.3; 64 x 3 10.3, 10.8; 52 x 4 11.9, 12.5; 27 x 13 27.9, 30.3; 20 x 20 40.6, 46.2; 128 x 8
-// 48.4, 60.0.  The form taken was the faster one of both, or within 3.1 % of it, at each of those sizes.
+// x blocks) 30.4, 25.0; 37 x 8 18.7, 18.2; 64 x 3 10.2, 10.7; 52 x 4 11.7, 12.5; 27 x 13 27.4, 30.4; 20 x 20 39.9, 46.5; 128 x 8
+// 47.3, 60.4.  The form taken is the faster one of both, or within 1.7 % of it, at each of those sizes.
 static bool attention_shares(int per_block, int q_blocks, int grid) {      // per_block: items of each length, one to q_blocks
   const long long items = (long long)per_block * q_blocks;
-  if (items > 4 * grid || attn::TEAMS * grid > 1024) return false;
+  if (q_blocks < 2 || items > 4 * grid || attn::TEAMS * grid > 1024) return false;
   return attention_busiest((int)items, per_block, q_blocks, grid, true) < attention_busiest((int)items, per_block, q_blocks, attn::TEAMS * grid, false);
 }
 
@@ -554,8 +560,8 @@ static int attention_fwd(const void* q, const void* k, const void* v, int64_t ld
   p.items = B * H * p.q_blocks;
   // one CTA of two teams per SM, persistent; with fewer items than SMs each gets an SM of its own
   const int grid = std::min(p.items, gemm_sm_count());
-  const bool shared = form < 0 ? !p.trace && attention_shares(B * H, p.q_blocks, grid)      // a trace follows one team through an item
-                               : form != 0;
+  // a trace follows one team through an item; steep scales: see softmax_rows
+  const bool shared = form < 0 ? !p.trace && p.scale_log2 <= 1.f && attention_shares(B * H, p.q_blocks, grid) : form != 0;
   const auto kernel = shared ? attn::attention_fwd_kernel<true> : attn::attention_fwd_kernel<false>;
   cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn::SMEM_BYTES);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention: shared memory attribute: %s", cudaGetErrorString(ae));
@@ -573,7 +579,7 @@ int tmpi_attention_fwd(const void* q, const void* k, const void* v, int64_t ld_q
   return attention_fwd(q, k, v, ld_qkv, out, ld_out, lse, B, T, H, scale, -1, stream);
 }
 
-// The same in a given form (for tests and timing), and the form that tmpi_attention_fwd takes.
+// The same in a given form (for tests and timing), and the form that tmpi_attention_fwd takes for scales of up to ln 2.
 int tmpi_attention_fwd_form(const void* q, const void* k, const void* v, int64_t ld_qkv, void* out, int64_t ld_out, float* lse,
                             int B, int T, int H, float scale, int shared, void* stream) {
   return attention_fwd(q, k, v, ld_qkv, out, ld_out, lse, B, T, H, scale, shared != 0, stream);
