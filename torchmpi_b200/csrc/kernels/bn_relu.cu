@@ -26,10 +26,11 @@ namespace tmpi {
 constexpr int kBnThreads = 256;
 constexpr int kBnMaxGrid = 592;     // 148 SMs x 4 resident CTAs
 
-// Blocks of a streaming pass: `most`, or fewer where there are not U vectors for every thread of them.
+// Blocks of a streaming pass: `most`, or fewer where there are not U vectors for every thread of them; but a block per SM where
+// there is one vector each, so that the smallest tensors are not left to a few SMs.
 static int bn_grid(size_t nvec, int most, int U) {
-  const size_t want = (nvec + (size_t)kBnThreads * U - 1) / ((size_t)kBnThreads * U);
-  return (int)std::max<size_t>(1, std::min<size_t>(want, most));
+  const size_t one = (nvec + kBnThreads - 1) / kBnThreads;
+  return (int)std::max<size_t>(1, std::min<size_t>(std::max((one + U - 1) / U, std::min<size_t>(one, 148)), most));
 }
 
 // A pack of NW 32-bit words (8 or 16 bytes), elements taken out and put in by shifts and pair conversions (element-wise
@@ -72,14 +73,25 @@ template <typename T, int V> __device__ __forceinline__ BpWords<V * sizeof(T) / 
 
 // The passes stream each tensor once and are bound by memory, so what counts is bytes in flight: each thread issues the loads
 // of U vectors before it uses the first, without branches between them (mask source, residual and its gradient are template
-// parameters), and past L1, where lines in flight would compete for space.  Fewer resident blocks with more registers hold
-// more bytes in flight than eight or four small ones.  Measured, 256 x 28 x 28, bf16, before and now: 512 channels, backward
-// sums under mask bits 93 -> 69 us (411 MB: 63 at the copy rate; 97 with the branches), forward apply with a residual
-// 120 -> 108 (96); 128 channels, backward sums 27 -> 20, backward apply 28 -> 22.
-template <typename T>
+// parameters; the loads are volatile to stay in front).  Fewer resident blocks with more registers hold more bytes in flight
+// than eight or four small ones.
+// Measured, in us, one small vector at a time as it was first, and now: bf16, 256 x 28 x 28 x 512, sums under mask bits 92, 73 (411
+// MB: 63 at the copy rate), forward apply with a residual 109, 94 (96), backward apply with the residual's gradient 130, 128;
+// 256 x 28 x 28 x 128, sums 30, 23, forward apply 16.5, 14.7, backward apply 28.7, 22.1; fp32, 64 x 56 x 56 x 64, forward apply 12.6,
+// 12.1, backward apply 20.5, 19.1.
+//
+// PAST_L1: loads that allocate nothing in L1.  They are the faster ones where a pass is the first to read what a kernel before it
+// has written (the forward apply behind a convolution: inference through a bottleneck of 32 x 56 x 56, 113 us with them and 120
+// without, 96 x 28 x 28 220 and 231; the statistics of the stem's 411 MB: 702 and 715 for the stem), and the slower ones where it
+// reads again what another pass of the layer has just read (forward apply after the statistics 107 and 94, 20.0 and 14.7, 17.5
+// and 12.1 for the sizes above; backward apply after the sums 135 and 128, 27.1 and 22.1, 25.4 and 19.1).
+template <bool PAST_L1, typename T>
 __device__ __forceinline__ BpWords<4> bn_ld(const T* p) {
   BpWords<4> u;
-  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
+  if constexpr (PAST_L1)
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
+  else
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
   return u;
 }
 constexpr int kBnReduceU = 4, kBnApplyU = 2;
@@ -90,7 +102,7 @@ constexpr int kBnReduceBwdGrid = 296, kBnApplyGrid = 740, kBnApplyBwdGrid = 444;
 enum { MASK_NONE = 0, MASK_X = 1 /* recomputed from x, gamma, beta */, MASK_BITS = 2, MASK_Y = 3, MASK_X_ROUNDED = 4 /* MASK_X, of the value rounded to T */ };
 __host__ __device__ constexpr bool bn_mask_from_x(int mask) { return mask == MASK_X || mask == MASK_X_ROUNDED; }
 
-template <typename T, int V, bool BWD, int MASK>
+template <typename T, int V, bool BWD, int MASK, bool PAST_L1>
 __global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
     const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ dy,
     const float* __restrict__ mean, const float* __restrict__ invstd,
@@ -140,12 +152,12 @@ __global__ void __launch_bounds__(kBnThreads, BWD ? 2 : 4) bn_reduce_kernel(
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const size_t at = reverse ? nvec - 1 - (v + u * stride) : v + u * stride;
-      xv[u] = bn_ld(x + at * V);
+      xv[u] = bn_ld<PAST_L1>(x + at * V);
       mb[u] = 0;
       if constexpr (BWD) {
-        gv[u] = bn_ld(dy + at * V);
+        gv[u] = bn_ld<PAST_L1>(dy + at * V);
         if constexpr (MASK == MASK_BITS) mb[u] = bits[at];
-        if constexpr (MASK == MASK_Y) yv[u] = bn_ld(y + at * V);
+        if constexpr (MASK == MASK_Y) yv[u] = bn_ld<PAST_L1>(y + at * V);
       }
     }
 #pragma unroll
@@ -234,7 +246,7 @@ __global__ void __launch_bounds__(1024) bn_finalize_bwd_kernel(const float* __re
 }
 
 // RES: a residual is added.  BITS: also write the ReLU mask byte of every vector (residual layers only).
-template <typename T, int V, bool RES, bool BITS>
+template <typename T, int V, bool RES, bool BITS, bool PAST_L1>
 __global__ void __launch_bounds__(kBnThreads, 5) bn_apply_fwd_kernel(
     const T* __restrict__ x, const T* __restrict__ res, T* __restrict__ y, const float* __restrict__ gamma,
     const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ invstd,
@@ -256,8 +268,8 @@ __global__ void __launch_bounds__(kBnThreads, 5) bn_apply_fwd_kernel(
     [[maybe_unused]] BpWords<4> rv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      xv[u] = bn_ld(x + (v + u * stride) * V);
-      if constexpr (RES) rv[u] = bn_ld(res + (v + u * stride) * V);
+      xv[u] = bn_ld<PAST_L1>(x + (v + u * stride) * V);
+      if constexpr (RES) rv[u] = bn_ld<PAST_L1>(res + (v + u * stride) * V);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -314,11 +326,11 @@ __global__ void __launch_bounds__(kBnThreads, 3) bn_apply_bwd_kernel(
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const size_t at = v + u * stride;
-      xv[u] = bn_ld(x + at * V);
-      gv[u] = bn_ld(dy + at * V);
+      xv[u] = bn_ld<false>(x + at * V);
+      gv[u] = bn_ld<false>(dy + at * V);
       mb[u] = 0;
       if constexpr (MASK == MASK_BITS) mb[u] = bits[at];
-      if constexpr (MASK == MASK_Y) yv[u] = bn_ld(y + at * V);
+      if constexpr (MASK == MASK_Y) yv[u] = bn_ld<false>(y + at * V);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -363,7 +375,7 @@ static int bn_fwd_t(const void* x, const void* res, void* y, const float* gamma,
     // given_rows > 0: the producer of x (a convolution epilogue) has left that many rows of partial sums in scratch
     if (given_rows > 0) grid = given_rows;
     else
-    bn_reduce_kernel<T, V, false, MASK_NONE><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+    bn_reduce_kernel<T, V, false, MASK_NONE, false><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                                                                      nullptr, nvec, C, reverse, (float*)scratch);
     float m = (float)rows;
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
@@ -371,8 +383,13 @@ static int bn_fwd_t(const void* x, const void* res, void* y, const float* gamma,
                                                            rmean, rvar);
   }
   const int apply_grid = bn_grid(nvec, kBnApplyGrid, kBnApplyU);
-  const auto apply = bits ? (res ? bn_apply_fwd_kernel<T, V, true, true> : bn_apply_fwd_kernel<T, V, false, true>)
-                          : (res ? bn_apply_fwd_kernel<T, V, true, false> : bn_apply_fwd_kernel<T, V, false, false>);
+  auto pick = [&](auto past) {
+    constexpr bool P = decltype(past)::value;
+    return bits ? (res ? bn_apply_fwd_kernel<T, V, true, true, P> : bn_apply_fwd_kernel<T, V, false, true, P>)
+                : (res ? bn_apply_fwd_kernel<T, V, true, false, P> : bn_apply_fwd_kernel<T, V, false, false, P>);
+  };
+  const bool read_before = training && given_rows <= 0;        // by the statistics pass
+  const auto apply = read_before ? pick(std::false_type()) : pick(std::true_type());
   apply<<<apply_grid, kBnThreads, 0, s>>>((const T*)x, (const T*)res, (T*)y, gamma, beta, smean, sinv, (unsigned char*)bits, nvec, C, relu);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "bn forward launch: %s", cudaGetErrorString(e));
@@ -393,7 +410,7 @@ static int bn_bwd_t(const void* x, const void* y, const void* dy, void* dx, void
   const unsigned char* mb = (const unsigned char*)bits;
   auto passes = [&](auto mode) {
     constexpr int MASK = decltype(mode)::value;
-    bn_reduce_kernel<T, V, true, MASK><<<grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, smean, sinv, gamma, beta, mb, nvec,
+    bn_reduce_kernel<T, V, true, MASK, false><<<grid, kBnThreads, 0, s>>>((const T*)x, (const T*)y, (const T*)dy, smean, sinv, gamma, beta, mb, nvec,
                                                                    C, reverse, (float*)scratch);
     bn_finalize_bwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, dgamma, dbeta, acc_gamma, acc_beta);
     const auto apply = dres ? bn_apply_bwd_kernel<T, V, MASK, true> : bn_apply_bwd_kernel<T, V, MASK, false>;
@@ -780,7 +797,7 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, void* xmax, const fl
   if (training) {
     size_t nvec = (size_t)rows * (C / V);
     const int grid = bn_grid(nvec, kBnMaxGrid, kBnReduceU);
-    bn_reduce_kernel<T, V, false, MASK_NONE><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+    bn_reduce_kernel<T, V, false, MASK_NONE, true><<<grid, kBnThreads, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                                                                      nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
     float m = (float)rows;
     bn_finalize_fwd_kernel<<<(C + 31) / 32, dim3(32, 32), 0, s>>>((const float*)scratch, grid, C, 1.f / m,
@@ -831,7 +848,7 @@ static int bn_pool_bwd_t(const void* x, const void* xmax, const void* dy, const 
     // all positions of x, 411 MB, with the gradient routed to each).
     const size_t nvec = (size_t)N * d.OH * d.OW * (C / V);
     grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU);
-    bn_reduce_kernel<T, V, true, MASK_X_ROUNDED><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
+    bn_reduce_kernel<T, V, true, MASK_X_ROUNDED, false><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
                                                                              nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
   } else if (fours) {
     grid = bn_pool_bwd_reduce<T, sizeof(T) == 2 ? 4 : V, sizeof(T) == 2 ? 3 : 2>(x, dy, idx, smean, sinv, d, scratch, s);
