@@ -82,7 +82,8 @@ template <typename T, int V> __device__ __forceinline__ BpWords<V * sizeof(T) / 
 //
 // PAST_L1: loads that allocate nothing in L1.  They are the faster ones where a pass is the first to read what a kernel before it
 // has written (the forward apply behind a convolution: inference through a bottleneck of 32 x 56 x 56, 113 us with them and 120
-// without, 96 x 28 x 28 220 and 231; the statistics of the stem's 411 MB: 702 and 715 for the stem), and the slower ones where it
+// without, 96 x 28 x 28 220 and 231; the statistics of the stem's 411 MB: 702 and 715 for the stem;
+// its backward sums over the kept inputs 757 and 760), and the slower ones where it
 // reads again what another pass of the layer has just read (forward apply after the statistics 107 and 94, 20.0 and 14.7, 17.5
 // and 12.1 for the sizes above; backward apply after the sums 135 and 128, 27.1 and 22.1, 25.4 and 19.1).
 template <bool PAST_L1, typename T>
@@ -848,7 +849,7 @@ static int bn_pool_bwd_t(const void* x, const void* xmax, const void* dy, const 
     // all positions of x, 411 MB, with the gradient routed to each).
     const size_t nvec = (size_t)N * d.OH * d.OW * (C / V);
     grid = bn_grid(nvec, kBnReduceBwdGrid, kBnReduceU);
-    bn_reduce_kernel<T, V, true, MASK_X_ROUNDED, false><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
+    bn_reduce_kernel<T, V, true, MASK_X_ROUNDED, true><<<grid, kBnThreads, 0, s>>>((const T*)xmax, nullptr, (const T*)dy, smean, sinv, gamma, beta,
                                                                              nullptr, nvec, C, tunable("bn_reverse_stats") != 0, (float*)scratch);
   } else if (fours) {
     grid = bn_pool_bwd_reduce<T, sizeof(T) == 2 ? 4 : V, sizeof(T) == 2 ? 3 : 2>(x, dy, idx, smean, sinv, d, scratch, s);
