@@ -353,9 +353,9 @@ int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, 
 // C[M,N] = act(A[M,K] * B[N,K]^T (+ bias)), bf16 in, fp32 accumulate in TMEM.
 int tmpi_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                    int epilogue, void* stream);
-// Z = A B^T + bias and Y = gelu(Z) of the rounded Z in one kernel; M, N >= 256, N and K multiples of 8
 int tmpi_gemm_bf16_any(const void* A, const void* B, void* C, void* gelu_out, const void* bias, int M, int N, int K, int epilogue,
                        void* stream);   // operands as stored, any size
+// Z = A B^T + bias and Y = gelu(Z) of the rounded Z in one kernel; M, N >= 256, N and K multiples of 8
 int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream);
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,

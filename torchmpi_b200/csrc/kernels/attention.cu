@@ -22,13 +22,13 @@
 // no longer exactly 1, and its bf16 rounding showed in the output); one thread per row (63 us in place of 56); all
 // exponentials before the wait for the previous product (61); descriptors in uniform registers (no difference).
 //
-// A CTA (one per SM) runs two such teams, each with its own items, rings, barriers and 256 tensor-memory columns, so that
-// one exponentiates while the other waits.  Teams are persistent and take items longest-first in snake order (item
+// A CTA (one per SM) runs two such teams, each with its own rings, barriers and 256 tensor-memory columns, so that
+// one exponentiates while the other waits.  Each has items of its own, or, where there are few, both work on the same one, on half
+// of its key blocks each (attention_shares).  Teams are persistent and take items longest-first in snake order (item
 // r * G + i, then r * G + G - 1 - i), which leaves the key blocks per team within one of each other at 8 x 16 x 1024; the
 // next item's loads and first S run under the end of the current one.
 //
-// Measured on a B200, back to back: 8 x 16 heads x 1024 x 64 64.2 -> 55.7 us, 1 x 16 x 2048 36.5 -> 32.7; before, P went
-// through shared memory and O through registers for each block, and every thread read the whole row for its maximum.
+// Measured on a B200, launches in a row: 8 x 16 heads x 1024 x 64 49.7 us, 1 x 16 x 2048 26.8 (33.4 with a team per item).
 //
 // Q, K and V are read where the fused QKV projection left them ([B * T, 3 C], one tensor map per operand) and the
 // output is written as [B * T, C]: no transposes around the kernel.  Every wait is bounded; a CTA that gives up records

@@ -17,10 +17,10 @@
 // tensor cores, so the shared memory goes to loads in flight: the ring has as many stages as fit
 // (up to 12), and when one column tile covers the output and the whole weight fits beside five
 // stages, the weight is loaded once and stays resident while only the activation streams.  The
-// epilogue warps work independently (own staging tile, no barrier between warps), two tiles drain at a
+// epilogue warps work independently (own staging tiles, no barrier between warps), two tiles drain at a
 // time.  Epilogues:
-//   store    bf16 rows: each warp converts its 32 x 64 slice into a swizzled staging tile for a TMA store; optionally the per-channel sum and sum of squares of the
-//            stored values (the batch statistics of the batch-norm that follows, accumulated per lane
+//   store    bf16 rows: each warp converts its 32 x 64 slice into a swizzled staging tile for a TMA
+//            store; optionally the per-channel sum and sum of squares of the stored values (the batch statistics of the batch-norm that follows, accumulated per lane
 //            in registers over all tiles of the CTA and written as one partial row per CTA: no atomics,
 //            fixed order), and optionally
 //            "+ R" for a second gradient that flows into the same tensor (added to the rounded product,

@@ -211,7 +211,8 @@ int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, i
 }
 
 // Z = A B^T + bias and Y = gelu(Z) (of the rounded Z), both [M, N], in one kernel: the forward of a linear layer that is
-// followed by a GELU and keeps its pre-activation.  CTA-pair kernel only (M, N >= 256, N and K multiples of 8).
+// followed by a GELU and keeps its pre-activation.  M, N >= 256, N and K multiples of 8 (tmpi_gemm_bf16_any takes fewer rows
+// and columns).
 int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8) return fail(TMPI_ERR_INVALID, "gemm_gelu: needs a non-empty product with K a multiple of 8");
   if (!tunable("gemm_pair") || !gemm_pair_applicable(Z, M, N, K, 0) || ((uintptr_t)Y & 15))

@@ -8,7 +8,9 @@
 //
 // Used where a transformer block's kernels follow each other (linear, layer norm, attention, bias gradient): forward and
 // backward of a block of 8 x 1024 x 1024 in bf16 take 926 us, 950 without it; attention forward and backward at
-// 8 x 16 x 1024 x 64 take 170 us, 173 without; a prefill of 1 x 16 x 2048 x 64 31.1 us, 32.8 without.  Not for the
+// 8 x 16 x 1024 x 64 take 170 us, 173 without; a prefill of 1 x 16 x 2048 x 64 with a team per item 31.1 us, 32.8 without.  A launch whose
+// blocks do not all fit beside the one before it starts them as SMs become free: a grid of one block per SM has to take up an SM
+// alone to be spread over all of them (see layernorm.cu).  Not for the
 // batch-norm, convolution and pooling kernels, which fill the chip for longer than a launch takes: with it a bottleneck of
 // 256 x 28 x 28 took 1154 us instead of 1166 (runs differ by 1.9 %), the stem with its pooling stage 1037 instead of 850.
 #pragma once
