@@ -183,6 +183,7 @@ _CUDA_PROTOS = {
     "tmpi_bias_grad_scratch_bytes": (_sz, [_i]),
     "tmpi_bias_grad": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp]),
     "tmpi_gelu_fwd": (_i, [_vp, _vp, _sz, _i, _vp]),
+    "tmpi_gelu_bwd": (_i, [_vp, _vp, _vp, _sz, _i, _vp]),
     "tmpi_layernorm_supported": (_i, [_i, _i]),
     "tmpi_layernorm_scratch_bytes": (_sz, [_i]),
     "tmpi_layernorm_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp]),
@@ -208,6 +209,8 @@ _CUDA_PROTOS = {
     "tmpi_gemm_bf16_any": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_gelu": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_ex": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp]),
+    "tmpi_linear_bwd_plan": (_i, [_i, _i, _i, _i, _i, C.POINTER(_sz), _ip]),
+    "tmpi_linear_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp, _i, _vp]),
     "tmpi_gemm_status": (_i, []),
     "tmpi_conv_max_ctas": (_i, []),
     "tmpi_conv_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _ip, _vp]),

@@ -1,11 +1,10 @@
 // Autograd functions of the hot single-GPU layers, in C++: linear (with bias and GELU), layer norm, causal attention and
-// cross-entropy.  They call the same C entry points as the Python wrappers in torchmpi_b200/ops did, with the same
-// checks, operand layouts and saved tensors; only the host work around a launch is native.  A forward and backward of
+// cross-entropy.  They make the checks of the Python functions that they stand for, and save the same tensors; only the host work around a launch is native.  A forward and backward of
 // one layer took 100 - 160 us of Python (autograd.Function both ways, ctypes argument conversion, tensor bookkeeping)
 // around 10 - 50 us of kernels, and a transformer block about as long as its kernels.
 //
-// Scratch memory is allocated per call from PyTorch's caching allocator on the calling stream; the one buffer that is kept
-// (cross-entropy, see xent_scratch) belongs to one stream.  A non-zero status is raised through torchmpi_b200._lib.check, so callers see the usual exceptions.
+// Scratch memory is allocated per call from PyTorch's caching allocator on the calling stream; the buffers that are kept
+// (KeptZeros) belong to one stream each.  A non-zero status is raised through torchmpi_b200._lib.check, so callers see the usual exceptions.
 // The reference has no counterpart (its layers are Torch7's).
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -25,7 +24,7 @@ using torch::autograd::variable_list;
 
 enum { LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD, KINDS };
 std::atomic<long long> g_launches[KINDS];      // attention: calls, and those of the backward alone
-enum { EPI_BIAS = 1, B_IS_KN = 4, A_IS_KM = 8 };
+enum { EPI_BIAS = 1 };
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 void launched(int what, int n) { g_launches[what].fetch_add(n, std::memory_order_relaxed); }
@@ -57,6 +56,36 @@ Tensor packed(const Tensor& t) {
   const Tensor c = t.contiguous();
   return (uintptr_t)c.data_ptr() % 16 ? c.clone() : c;
 }
+
+// Buffers of arrival counters, which a kernel finds zero and leaves zero.  Two calls may share one only if one ends before the
+// other starts, so there is one per stream, grown to the next power of two.  A call that is being captured gets its own, cleared
+// inside the graph: the graph may be replayed on any stream, and has not run when the next eager call comes.  So does a call
+// that needs a large one.  Buffers go back to the allocator, which hands them out on the stream they were used on.
+struct KeptZeros {
+  static constexpr size_t KEEP_BYTES = size_t(1) << 20, KEEP_STREAMS = 64;
+  std::mutex lock;
+  std::map<std::pair<int, void*>, Tensor> kept;
+
+  Tensor get(const Tensor& like, size_t need) {
+    const auto bytes = like.options().dtype(at::kByte);
+    if (need > KEEP_BYTES || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+      return at::zeros({(int64_t)need}, bytes);
+    const std::pair<int, void*> key(like.get_device(), stream());
+    {
+      std::lock_guard<std::mutex> hold(lock);
+      const auto found = kept.find(key);
+      if (found != kept.end() && (size_t)found->second.numel() >= need) return found->second;
+    }
+    size_t size = 4096;
+    while (size < need) size *= 2;
+    const Tensor fresh = at::zeros({(int64_t)size}, bytes);
+    std::map<std::pair<int, void*>, Tensor> old;                           // released outside the lock
+    std::lock_guard<std::mutex> hold(lock);
+    if (kept.size() >= KEEP_STREAMS) old.swap(kept);
+    kept[key] = fresh;
+    return fresh;
+  }
+};
 
 bool pair_enabled() {
   int64_t v = 0;
@@ -101,32 +130,9 @@ std::pair<Tensor, Tensor> matmul_nt_gelu(const Tensor& a_, const Tensor& b_, con
   return {z, y};
 }
 
-Tensor matmul_nn(const Tensor& a_, const Tensor& b_) {
-  const Tensor a = a_.contiguous(), b = b_.contiguous();
-  const int64_t M = a.size(0), K = a.size(1), N = b.size(1);
-  if (!(M >= 1 && N % 8 == 0 && K % 8 == 0 && K >= 1 && pair_enabled())) return matmul_nt(a, b.t().contiguous(), Tensor());
-  Tensor out = at::empty({M, N}, a.options());
-  check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, nullptr, (int)M, (int)N, (int)K, B_IS_KN, stream()));
-  launched(LINEAR, 1);
-  return out;
-}
-
-Tensor matmul_tn(const Tensor& a_, const Tensor& b_) {
-  const Tensor a = a_.contiguous(), b = b_.contiguous();
-  const int64_t K = a.size(0), M = a.size(1), N = b.size(1);
-  if (!(K >= 1 && M % 8 == 0 && N % 8 == 0 && pair_enabled())) return matmul_nt(a.t().contiguous(), b.t().contiguous(), Tensor());
-  Tensor out = at::empty({M, N}, a.options());
-  if (tmpi_gemm_tn_prefers_splitk((int)M, (int)N, K)) {       // few tiles, many rows: K over the SMs, fp32 partial tiles
-    const size_t need = tmpi_gemm_tn_splitk_workspace_bytes((int)M, (int)N, K);
-    const Tensor ws = at::empty({(int64_t)need}, a.options().dtype(at::kByte));
-    check(tmpi_gemm_bf16_tn_splitk(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, K, 0, 0, ws.data_ptr(), need, 0, stream()));
-    launched(LINEAR, 2);
-    return out;
-  }
-  check(tmpi_gemm_bf16_any(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, nullptr, (int)M, (int)N, (int)K, A_IS_KM | B_IS_KN, stream()));
-  launched(LINEAR, 1);
-  return out;
-}
+// a b and a^T b without the CTA-pair kernel: through transposed copies
+Tensor matmul_nn(const Tensor& a, const Tensor& b) { return matmul_nt(a, b.t().contiguous(), Tensor()); }
+Tensor matmul_tn(const Tensor& a, const Tensor& b) { return matmul_nt(a.t().contiguous(), b.t().contiguous(), Tensor()); }
 
 // dz = dy * gelu'(z) (dy itself without z) and its column sum, in one pass where the kernel applies
 std::pair<Tensor, Tensor> bias_grad(const Tensor& dy, const Tensor& z) {
@@ -141,6 +147,36 @@ std::pair<Tensor, Tensor> bias_grad(const Tensor& dy, const Tensor& z) {
                        (int)C, dtype_code(dy.scalar_type()), scratch.data_ptr(), stream()));
   launched(LINEAR, 2);
   return {dz, db};
+}
+
+// dX = dY W, dW = dY^T X and db = column sums of dY, those that are wanted, in one launch
+void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor* dx, Tensor* dw, Tensor* db) {
+  const int rows = (int)x.size(0), in = (int)x.size(1), out = (int)w.size(0), want = (dx ? 1 : 0) | (dw ? 2 : 0) | (db ? 4 : 0);
+  size_t bytes = 0;
+  int counters = 0;
+  check(tmpi_linear_bwd_plan(rows, in, out, want, 0, &bytes, &counters));
+  Tensor ws, arrivals;
+  if (bytes) ws = at::empty({(int64_t)bytes}, dy.options().dtype(at::kByte));
+  if (counters) {
+    static auto& kept = *new KeptZeros;
+    arrivals = kept.get(dy, sizeof(unsigned) * (size_t)counters);
+  }
+  if (dx) *dx = at::empty({rows, in}, dy.options());
+  if (dw) *dw = at::empty({out, in}, dy.options());
+  if (db) *db = at::empty({out}, dy.options());
+  check(tmpi_linear_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), dx ? dx->data_ptr() : nullptr, dw ? dw->data_ptr() : nullptr,
+                        db ? db->data_ptr() : nullptr, rows, in, out, 0, bytes ? ws.data_ptr() : nullptr, bytes,
+                        counters ? arrivals.data_ptr() : nullptr, counters, stream()));
+  launched(LINEAR, 1);
+}
+
+// dy * gelu'(z)
+Tensor gelu_gradient(const Tensor& dy, const Tensor& z) {
+  if ((uintptr_t)z.data_ptr() % 16) return at::gelu_backward(dy, z);
+  Tensor dz = at::empty_like(dy);
+  check(tmpi_gelu_bwd(dy.data_ptr(), z.data_ptr(), dz.data_ptr(), (size_t)dy.numel(), dtype_code(dy.scalar_type()), stream()));
+  launched(LINEAR, 1);
+  return dz;
 }
 
 struct LinearFn : public torch::autograd::Function<LinearFn> {
@@ -163,10 +199,18 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     const Tensor &x2 = saved[0], &w = saved[1], &z = saved[2];
     const Tensor& dy = grads[0];
     Tensor dy2 = packed(dy.reshape({-1, dy.size(-1)})), db, dx, dw;
+    const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    if ((need_x || need_w) && dy2.size(1) % 8 == 0 && pair_enabled()) {
+      if (z.defined()) dy2 = gelu_gradient(dy2, z);
+      const bool need_b = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
+      linear_gradients(dy2, x2.contiguous(), w.contiguous(), need_x ? &dx : nullptr, need_w ? &dw : nullptr, need_b ? &db : nullptr);
+      if (need_x) dx = dx.view(ctx->saved_data["shape"].toIntVector());
+      return {dx, dw, db, Tensor()};
+    }
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) std::tie(dy2, db) = bias_grad(dy2, z);
     else if (z.defined()) dy2 = at::gelu_backward(dy2, z);
-    if (ctx->needs_input_grad(0)) dx = matmul_nn(dy2, w).reshape(ctx->saved_data["shape"].toIntVector());
-    if (ctx->needs_input_grad(1)) dw = matmul_tn(dy2, x2);
+    if (need_x) dx = matmul_nn(dy2, w).reshape(ctx->saved_data["shape"].toIntVector());
+    if (need_w) dw = matmul_tn(dy2, x2);
     return {dx, dw, db, Tensor()};
   }
 };
@@ -234,33 +278,11 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
 };
 
 // ---------------------------------------------------------------- cross-entropy
-// The arrival counter of the kernel's blocks (zero before and after every call) and the row losses.  Two calls may share a
-// buffer only if one ends before the other starts, so there is one per stream, grown to the next power of two.  A call that
-// is being captured gets its own, cleared inside the graph: the graph may be replayed on any stream, and has not run when the
-// next eager call comes.  So does a call of very many rows, where the clearing costs nothing beside the pass and the buffer
-// would be large to keep.  Buffers go back to the allocator, which hands them out on the stream they were used on.
+// The arrival counter of the kernel's blocks and the row losses.  A call of very many rows clears a buffer of its own: the clearing
+// costs nothing beside the pass and the buffer would be large to keep.
 Tensor xent_scratch(const Tensor& x, int64_t rows) {
-  constexpr size_t KEEP_BYTES = size_t(1) << 20, KEEP_STREAMS = 64;
-  static std::mutex lock;
-  static auto& kept = *new std::map<std::pair<int, void*>, Tensor>();      // outlives the CUDA context: never destroyed
-  size_t need = tmpi_xent_scratch_bytes((int)rows);
-  const auto bytes = x.options().dtype(at::kByte);
-  if (need > KEEP_BYTES || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-    return at::zeros({(int64_t)need}, bytes);
-  const std::pair<int, void*> key(x.get_device(), stream());
-  {
-    std::lock_guard<std::mutex> hold(lock);
-    const auto found = kept.find(key);
-    if (found != kept.end() && (size_t)found->second.numel() >= need) return found->second;
-  }
-  size_t size = 4096;
-  while (size < need) size *= 2;
-  const Tensor fresh = at::zeros({(int64_t)size}, bytes);
-  std::map<std::pair<int, void*>, Tensor> old;                             // released outside the lock
-  std::lock_guard<std::mutex> hold(lock);
-  if (kept.size() >= KEEP_STREAMS) old.swap(kept);
-  kept[key] = fresh;
-  return fresh;
+  static auto& kept = *new KeptZeros;                          // outlives the CUDA context: never destroyed
+  return kept.get(x, tmpi_xent_scratch_bytes((int)rows));
 }
 
 // The gradient is computed with the loss and scaled in place by the incoming gradient, so backward runs once.

@@ -244,6 +244,7 @@ size_t tmpi_bias_grad_scratch_bytes(int channels);
 int tmpi_bias_grad(const void* dy, const void* z, void* dz, void* db, int rows, int channels, int dtype,
                    void* scratch, void* stream);
 // y = gelu(z), erf form, n elements (a multiple of 16 bytes, pointers 16-byte aligned)
+int tmpi_gelu_bwd(const void* dy, const void* z, void* dz, size_t n, int dtype, void* stream);   // dz = dy * gelu'(z)
 int tmpi_gelu_fwd(const void* z, void* y, size_t n, int dtype, void* stream);
 // layer normalisation over the last dimension of [rows, channels]; x, y, gamma, beta share the dtype;
 // mean / rstd ([rows], fp32) are written by forward and read by backward
@@ -360,6 +361,11 @@ int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const vo
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                       int64_t lda, int64_t ldb, int64_t ldc, int epilogue, void* stream);
+// The gradients of a linear layer in one launch (linear_bwd.cu): dx [rows, in] = dy w, dw [out, in] = dy^T x, db [out] = column sums
+// of dy; in and out multiples of 8.  want: 1 dx, 2 dw, 4 db.  form: 0, or the tiles and slices (linear_bwd.cu, plan).
+int tmpi_linear_bwd_plan(int rows, int in, int out, int want, int form, size_t* workspace_bytes, int* counters);
+int tmpi_linear_bwd(const void* dy, const void* x, const void* w, void* dx, void* dw, void* db, int rows, int in, int out, int form,
+                    void* workspace, size_t workspace_bytes, void* counters, int ncounters, void* stream);
 
 // ---------------------------------------------------------------- tracing
 // ring buffer of (op, algo, bytes, microseconds) records per process

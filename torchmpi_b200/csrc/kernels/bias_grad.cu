@@ -66,6 +66,46 @@ static int gelu_fwd_t(const void* z, void* y, size_t n, cudaStream_t s) {
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "gelu_fwd launch: %s", cudaGetErrorString(e));
 }
 
+// dz = dy * gelu'(z), packs as above.
+template <typename T, int V>
+__global__ void __launch_bounds__(256, 4) gelu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __restrict__ dz, size_t npacks) {
+  wait_previous(dy, z);
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int U = 2;
+  auto one = [&](const Pack<T, V>& g, const Pack<T, V>& a, size_t at) {
+    Pack<T, V> o;
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+      float d[2];
+      gelu_grad2((float)to_acc<T>(a.v[k]), (float)to_acc<T>(a.v[k + 1]), &d[0], &d[1]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) o.v[k + e] = from_acc<T>((typename AccOf<T>::type)((float)to_acc<T>(g.v[k + e]) * d[e]));
+    }
+    st_pack<T, V>(dz + at * V, o);
+  };
+  for (; i + (U - 1) * stride < npacks; i += U * stride) {
+    Pack<T, V> g[U], a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) { g[u] = ld_pack<T, V>(dy + (i + u * stride) * V); a[u] = ld_pack<T, V>(z + (i + u * stride) * V); }
+#pragma unroll
+    for (int u = 0; u < U; ++u) one(g[u], a[u], i + u * stride);
+  }
+  for (; i < npacks; i += stride) one(ld_pack<T, V>(dy + i * V), ld_pack<T, V>(z + i * V), i);
+}
+
+template <typename T>
+static int gelu_bwd_t(const void* dy, const void* z, void* dz, size_t n, cudaStream_t s) {
+  constexpr int V = 16 / sizeof(T);
+  if (n % V || (((uintptr_t)dy | (uintptr_t)z | (uintptr_t)dz) & 15))
+    return fail(TMPI_ERR_UNSUPPORTED, "gelu_bwd: n=%zu must be a multiple of %d and the pointers 16-byte aligned", n, V);
+  const size_t npacks = n / V;
+  if (!npacks) return TMPI_OK;
+  const int blocks = (int)std::min<size_t>((npacks + 255) / 256, (size_t)148 * 4);
+  cudaError_t e = launch_overlapped(gelu_bwd_kernel<T, V>, blocks, 256, 0, s, (const T*)dy, (const T*)z, (T*)dz, npacks);
+  return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "gelu_bwd launch: %s", cudaGetErrorString(e));
+}
+
 // partial[blockIdx.y * C + c]
 template <typename T, int V, bool GELU>
 __global__ void __launch_bounds__(kBgThreads, 4)
@@ -196,6 +236,17 @@ int tmpi_bias_grad(const void* dy, const void* z, void* dz, void* db, int rows, 
     case TMPI_F32: return bias_grad_t<float>(dy, z, dz, db, rows, channels, scratch, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "bias_grad: dtype %d", dtype);
+}
+
+// dz = dy * gelu'(z) for n elements of `dtype`.
+int tmpi_gelu_bwd(const void* dy, const void* z, void* dz, size_t n, int dtype, void* stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (dtype) {
+    case TMPI_BF16: return gelu_bwd_t<__nv_bfloat16>(dy, z, dz, n, s);
+    case TMPI_F16: return gelu_bwd_t<__half>(dy, z, dz, n, s);
+    case TMPI_F32: return gelu_bwd_t<float>(dy, z, dz, n, s);
+  }
+  return fail(TMPI_ERR_UNSUPPORTED, "gelu_bwd: dtype %d", dtype);
 }
 
 // y = gelu(z) (erf form) for n elements of `dtype`; the forward companion of tmpi_bias_grad's derivative.

@@ -1,6 +1,5 @@
 // bf16 GEMM on CTA pairs: C[M,N] = act(A[M,K] * B[N,K]^T + bias) with 256 x 256 tiles computed by
-// two CTAs of a cluster (gemm_pair.cuh).  One cluster per TPC, persistent; tiles are visited in
-// bands of 8 tile-rows so that the clusters running at one time share B panels in L2.
+// two CTAs of a cluster (gemm_pair.cuh).  One cluster per TPC, persistent.
 #include "gemm_pair.cuh"
 #include "pdl.cuh"
 #include "../include/tmpi_c_api.h"
@@ -15,17 +14,6 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t c
 int gemm_sm_count();
 
 namespace gemm2 {
-
-constexpr int BAND = 8;   // 256-row tiles per band
-
-__device__ __forceinline__ void band_order(int t, int tiles_m, int tiles_n, int* m_tile, int* n_blk) {
-  const int per_band = BAND * tiles_n;
-  const int band = t / per_band;
-  const int rows = min(BAND, tiles_m - band * BAND);
-  const int r = t - band * per_band;
-  *m_tile = band * BAND + r % rows;
-  *n_blk = r / rows;
-}
 
 // p.tiles_m counts 256-row tiles here.  TWO: gelu(C) goes to map_y beside C.
 template <bool TWO>

@@ -34,6 +34,18 @@ constexpr unsigned long long kWaitBudgetNs = gemm::kWaitBudgetNs;
 static_assert(BN == gemm::BN && BM == gemm::BM, "the epilogue is shared with the single-CTA kernel");
 static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
 
+// Tiles are visited in bands of 8 tile-rows, so that the clusters running at one time share B panels in L2.
+constexpr int BAND = 8;   // 256-row tiles per band
+
+__device__ __forceinline__ void band_order(int t, int tiles_m, int tiles_n, int* m_tile, int* n_blk) {
+  const int per_band = BAND * tiles_n;
+  const int band = t / per_band;
+  const int rows = min(BAND, tiles_m - band * BAND);
+  const int r = t - band * per_band;
+  *m_tile = band * BAND + r % rows;
+  *n_blk = r / rows;
+}
+
 struct Shared {
   uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;

@@ -1,0 +1,526 @@
+// The gradients of a linear layer, dX = dY W, dW = dY^T X and db = column sums of dY, in one launch on CTA pairs
+// (gemm_pair.cuh): dY [rows, out], W [out, in] and X [rows, in] are read as they lie.
+//
+// Work units.  Each product is cut into tiles of 256 rows x bn columns, and a tile whose K is long beside what the other clusters
+// have to do into slices of K.  The units of all three products form one list, longest first, dealt to the persistent clusters in
+// turn.  Two launches of their own each end in a partly filled round (8192 x 1024 x 1024: 128 tiles of dX on 74 clusters, then 16
+// long ones of dW); in one list the short units fill what the long ones leave.
+//
+// A sliced tile's partial sums go to the workspace in fp32; the CTA that arrives last at its tile adds all slices in their
+// order (bit-reproducible, nobody waits) and writes the result.  The arrival counters wrap to zero by themselves.
+//
+// db is a product as well: dY^T times a column of ones that lies in shared memory, accumulated in fp32 like the others; a unit of
+// it loads A tiles only, which dW's units bring into L2.  A pass over dY of its own took two launches.
+#include "gemm_pair.cuh"
+#include "pdl.cuh"
+#include "../include/tmpi_c_api.h"
+#include "../runtime/common.h"
+#include <algorithm>
+#include <mutex>
+
+namespace tmpi {
+
+int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+int gemm_sm_count();
+int* gemm_status_word();
+
+namespace lbwd {
+
+using namespace gemm2;
+enum { DX = 0, DW = 1, DB = 2 };
+constexpr int ONES_N = 32, ONES_BYTES = 1024;        // N of the MMAs with the ones; each CTA stages 16 of its rows
+constexpr int EPI_THREADS = GROUPS * 128;
+constexpr size_t BWD_SMEM_BYTES = SMEM_BYTES + ONES_BYTES;
+static_assert(BWD_SMEM_BYTES <= 232448, "shared memory of one CTA");
+
+struct Part {
+  int what;
+  int M, N;                  // extents of the result
+  int tiles_m, tiles_n, bn;  // 256-row tiles, tiles of bn columns
+  int k_blocks, per, slices; // 64-wide blocks of K, those of one slice
+  int first;                 // its first unit in the list
+  int arrivals;              // its first arrival counter (two per tile)
+  long long ws;              // its first float of the workspace
+};
+
+struct Problem {
+  Part part[3];
+  int parts, total;
+  float* ws;
+  unsigned* arrivals;
+  __nv_bfloat16* db;
+  int* status;
+};
+
+struct Unit { int m_blk, n_blk, kb0, kb1, tile, slice; };
+
+// f(part, unit, number of the unit in this cluster's list) for each unit of this cluster until it returns false; m_blk counts
+// 128-row blocks (of this CTA).
+template <typename F>
+__device__ __forceinline__ void for_units(const Problem& p, uint32_t rank, F f) {
+  const int step = (int)(gridDim.x >> 1);
+  int at = (int)(blockIdx.x >> 1), it = 0;
+  for (int i = 0; i < p.parts; ++i) {
+    const Part& q = p.part[i];
+    const int tiles = q.tiles_m * q.tiles_n, end = q.first + tiles * q.slices;
+    for (; at < end; at += step, ++it) {
+      Unit u;
+      const int r = at - q.first;
+      u.slice = r / tiles;             // the tiles of one slice run together and share its operands in L2
+      u.tile = r - u.slice * tiles;
+      int m_tile;
+      band_order(u.tile, q.tiles_m, q.tiles_n, &m_tile, &u.n_blk);
+      u.m_blk = m_tile * 2 + (int)rank;
+      u.kb0 = u.slice * q.per;
+      u.kb1 = min(q.k_blocks, u.kb0 + q.per);
+      if (!f(q, u, it)) return;
+    }
+  }
+}
+
+struct Sh { Shared s; int last; };
+static_assert(sizeof(Sh) <= 256, "barriers");
+
+__device__ __forceinline__ void give_up(Shared* sh, const Problem& p, int where) {
+  atomicExch(&sh->error, where);
+  if (p.status) atomicCAS(p.status, 0, 1000 + where);
+}
+
+struct Ring { int stage; uint32_t phase; };
+__device__ __forceinline__ void advance(Ring* r) { if (++r->stage == STAGES) { r->stage = 0; r->phase ^= 1; } }
+
+// One thread in each CTA.
+template <int WHAT>
+__device__ __forceinline__ bool produce_unit(Shared* sh, unsigned char* tiles, const Problem& p, const CUtensorMap* ma, const CUtensorMap* mb,
+                                             uint32_t rank, int bn, const Unit& u, Ring* ring) {
+  const int half = bn / 2, m0 = u.m_blk * BM, n0 = u.n_blk * bn + (int)rank * half;
+  const bool two = half > 64;
+  // bytes of a stage in both CTAs: A, and one or two boxes of 64 columns of B, of which bn / 2 columns are used
+  const uint32_t tx = 2 * (A_BYTES + (WHAT == DB ? 0 : two ? B_BYTES : B_BYTES / 2));
+  for (int kb = u.kb0; kb < u.kb1; ++kb) {
+    const int stage = ring->stage;
+    if (!sm100::mbar_wait(&sh->empty[stage], ring->phase ^ 1, kWaitBudgetNs) || sh->error) { give_up(sh, p, 21); return false; }
+    unsigned char* dst = tiles + (size_t)stage * STAGE_BYTES;
+    const uint32_t full0 = sm100::map_to_cta(&sh->full[stage], 0);
+    if (rank == 0) sm100::mbar_expect_tx(&sh->full[stage], tx);
+    const int k0 = kb * BK;
+    if (WHAT == DX) {          // rows of dY: K contiguous
+      sm100::tma_load_2d_pair(dst, ma, k0, m0, full0);
+      sm100::tma_load_2d_pair(dst + A_BYTES / 2, ma, k0, m0 + 64, full0);
+    } else {                   // columns of dY: M contiguous
+      sm100::tma_load_2d_pair(dst, ma, m0, k0, full0);
+      sm100::tma_load_2d_pair(dst + A_BYTES / 2, ma, m0 + 64, k0, full0);
+    }
+    if (WHAT != DB) {
+      sm100::tma_load_2d_pair(dst + A_BYTES, mb, n0, k0, full0);
+      if (two) sm100::tma_load_2d_pair(dst + A_BYTES + B_BYTES / 2, mb, n0 + 64, k0, full0);
+    }
+    advance(ring);
+  }
+  return true;
+}
+
+// One thread of the even CTA.
+template <int WHAT>
+__device__ __forceinline__ bool issue_unit(Shared* sh, unsigned char* tiles, uint64_t ones, const Problem& p, int bn, const Unit& u, int it, Ring* ring) {
+  const uint32_t idesc = WHAT == DB ? sm100::make_idesc_f16(2 * BM, ONES_N, true, false, true) : sm100::make_idesc_f16(2 * BM, bn, true, true, WHAT == DW);
+  const int acc = it & 1;
+  if (!sm100::mbar_wait(&sh->acc_empty[acc], ((it >> 1) & 1) ^ 1, kWaitBudgetNs) || sh->error) { give_up(sh, p, 22); return false; }
+  sm100::tc_fence_after();
+  const uint32_t d = sh->tmem_base + (uint32_t)acc * BN;
+  for (int kb = u.kb0; kb < u.kb1; ++kb) {
+    const int stage = ring->stage;
+    if (!sm100::mbar_wait(&sh->full[stage], ring->phase, kWaitBudgetNs) || sh->error) { give_up(sh, p, 23); return false; }
+    sm100::tc_fence_after();
+    const uint32_t a = sm100::smem_u32(tiles + (size_t)stage * STAGE_BYTES), b = a + A_BYTES;
+#pragma unroll
+    for (int k = 0; k < BK / UMMA_K; ++k) {
+      const uint64_t da = WHAT == DX ? sm100::make_desc_sw128(a + k * UMMA_K * 2) : sm100::make_desc_sw128_mn(a + k * UMMA_K * 128, A_BYTES / 2, 1024);
+      const uint64_t db = WHAT == DB ? ones : sm100::make_desc_sw128_mn(b + k * UMMA_K * 128, B_BYTES / 2, 1024);
+      sm100::umma_f16_pair(d, da, db, idesc, (uint32_t)(kb > u.kb0) | (uint32_t)k);
+    }
+    sm100::umma_commit_pair(sm100::map_to_cta(&sh->empty[stage], 0));
+    sm100::umma_commit_pair(sm100::map_to_cta(&sh->empty[stage], 1));
+    advance(ring);
+  }
+  sm100::umma_commit_pair(sm100::map_to_cta(&sh->acc_full[acc], 0));
+  sm100::umma_commit_pair(sm100::map_to_cta(&sh->acc_full[acc], 1));
+  return true;
+}
+
+__device__ __forceinline__ void all_sync() { asm volatile("bar.sync 3, %0;" ::"n"(EPI_THREADS) : "memory"); }
+
+// The eight epilogue warps of each CTA: two groups of four, which take the 64-column slices of a tile in turn.
+__device__ __forceinline__ void finish(Sh* shl, unsigned char* staging, const Problem& p, const CUtensorMap* mdx, const CUtensorMap* mdw,
+                                       uint32_t rank, int group, int quarter, int lane) {
+  Shared* sh = &shl->s;
+  constexpr int SLICE = 64, SLICE_BYTES = BM * SLICE * 2;
+  const int row = quarter * 32 + lane;
+  const bool leader = quarter == 0 && lane == 0;
+  unsigned char* stg = staging + group * SLICE_BYTES;
+  unsigned char* stg_row = stg + row * 128;
+  for_units(p, rank, [&](const Part& q, const Unit& u, int it) -> bool {
+    const int acc = it & 1, S = q.slices, M = q.M, N = q.N, bn = q.bn;
+    const uint32_t ok = sm100::mbar_wait(&sh->acc_full[acc], (it >> 1) & 1, kWaitBudgetNs) && !sh->error;
+    uint32_t all_ok;                    // the warps meet below: they go on, or leave, together
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.and.pred q, 3, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(all_ok) : "r"(ok), "n"(EPI_THREADS) : "memory");
+    if (!all_ok) { give_up(sh, p, 24); return false; }
+    sm100::tc_fence_after();
+    const int row0 = u.m_blk * BM;
+    const uint32_t t_base = sh->tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+    auto release = [&] {                // the accumulator has been read
+      sm100::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive_cluster(sm100::map_to_cta(&sh->acc_empty[acc], 0));
+    };
+    // Whether this CTA is the last of the tile's slices; their partial sums are then visible to all its epilogue threads.
+    auto arrive = [&]() -> bool {
+      __threadfence();
+      all_sync();
+      if (group == 0 && leader)
+        shl->last = atomicInc(&p.arrivals[q.arrivals + 2 * u.tile + (int)rank], (unsigned)(S - 1)) == (unsigned)(S - 1);
+      all_sync();
+      const bool last = shl->last != 0;
+      if (last) __threadfence();
+      return last;
+    };
+    // slot of a slice: 128 rows x bn columns as [column / 4][row][4] (db: [row])
+    const long long slot = (long long)(q.what == DB ? 1 : bn) * BM;
+    float* ws = p.ws + q.ws + ((long long)u.tile * S * 2 + (int)rank) * slot;      // of slice 0; the next one 2 * slot further
+    if (q.what == DB) {
+      float sum = 0.f;
+      if (group == 0) {
+        uint32_t r[16];
+        sm100::tmem_ld_32x16(t_base, r);
+        sm100::tmem_ld_wait();
+        sum = __uint_as_float(r[0]);
+      }
+      release();
+      bool write = true;
+      if (S > 1) {
+        if (group == 0) __stcg(ws + 2 * slot * u.slice + row, sum);
+        write = arrive();
+        if (write && group == 0) {
+          sum = 0.f;
+          for (int s = 0; s < S; ++s) sum += __ldcg(ws + 2 * slot * s + row);
+        }
+      }
+      if (write && group == 0 && row0 + row < M) p.db[row0 + row] = __float2bfloat16_rn(sum);
+      return true;
+    }
+    const CUtensorMap* map = q.what == DX ? mdx : mdw;
+    auto put = [&](const uint32_t (&r)[2][32], int col0) {
+      if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      group_sync(group);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 8 * j + 2 * e;
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c >> 5][c & 31]), __uint_as_float(r[c >> 5][(c & 31) + 1]));
+          w[e] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(stg_row + ((j ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      sm100::fence_proxy_async_smem();
+      group_sync(group);
+      if (leader) {
+        if (row0 < M) sm100::tma_store_2d(map, stg, col0, row0);
+        if (row0 + 64 < M) sm100::tma_store_2d(map, stg + SLICE_BYTES / 2, col0, row0 + 64);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+    };
+#pragma unroll 1
+    for (int c0 = group * SLICE; c0 < bn && u.n_blk * bn + c0 < N; c0 += GROUPS * SLICE) {
+      uint32_t r[2][32];
+      sm100::tmem_ld_32x32(t_base + c0, r[0]);
+      sm100::tmem_ld_32x32(t_base + c0 + 32, r[1]);
+      sm100::tmem_ld_wait();
+      if (S == 1) {
+        put(r, u.n_blk * bn + c0);
+      } else {
+        float4* to = reinterpret_cast<float4*>(ws + 2 * slot * u.slice) + (c0 / 4) * BM + row;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const uint32_t* v = &r[j >> 3][(j & 7) * 4];
+          __stcg(to + j * BM, make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3])));
+        }
+      }
+    }
+    release();
+    if (S > 1 && arrive()) {
+#pragma unroll 1
+      for (int c0 = group * SLICE; c0 < bn && u.n_blk * bn + c0 < N; c0 += GROUPS * SLICE) {
+        uint32_t r[2][32];
+#pragma unroll
+        for (int j = 0; j < 64; ++j) r[j >> 5][j & 31] = 0u;
+#pragma unroll 1
+        for (int s = 0; s < S; ++s) {
+          const float4* from = reinterpret_cast<const float4*>(ws + 2 * slot * s) + (c0 / 4) * BM + row;
+          float4 v[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = __ldcg(from + j * BM);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            uint32_t* a = &r[j >> 3][(j & 7) * 4];
+            a[0] = __float_as_uint(__uint_as_float(a[0]) + v[j].x);
+            a[1] = __float_as_uint(__uint_as_float(a[1]) + v[j].y);
+            a[2] = __float_as_uint(__uint_as_float(a[2]) + v[j].z);
+            a[3] = __float_as_uint(__uint_as_float(a[3]) + v[j].w);
+          }
+        }
+        put(r, u.n_blk * bn + c0);
+      }
+    }
+    return true;
+  });
+  if (leader) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(GROUP_THREADS, 1)
+linear_bwd_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                  const __grid_constant__ CUtensorMap map_dx, const __grid_constant__ CUtensorMap map_dw, const __grid_constant__ Problem p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *tiles, *staging;
+  Shared* sh;
+  carve(smem_raw, &tiles, &sh, &staging);
+  unsigned char* ones = (unsigned char*)sh + 256;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = sm100::cluster_ctarank();
+  for (int i = threadIdx.x; i < ONES_BYTES / 4; i += GROUP_THREADS) reinterpret_cast<uint32_t*>(ones)[i] = 0x3F803F80u;
+  sm100::fence_proxy_async_smem();
+  setup(sh, warp, &map_dy, &map_x, 4 * GROUPS);
+  wait_previous();
+  if (warp == 0) {
+    if (sm100::elect_one()) {
+      Ring ring{0, 0};
+      for_units(p, rank, [&](const Part& q, const Unit& u, int) -> bool {
+        if (q.what == DX) return produce_unit<DX>(sh, tiles, p, &map_dy, &map_w, rank, q.bn, u, &ring);
+        if (q.what == DW) return produce_unit<DW>(sh, tiles, p, &map_dy, &map_x, rank, q.bn, u, &ring);
+        return produce_unit<DB>(sh, tiles, p, &map_dy, nullptr, rank, q.bn, u, &ring);
+      });
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && sm100::elect_one()) {
+      // the ones as unswizzled core matrices of 8 rows x 16 bytes: 512 bytes apart along K, 128 along N
+      const uint64_t d_ones = (uint64_t)((sm100::smem_u32(ones) & 0x3FFFF) >> 4) | (uint64_t)(512 >> 4) << 16 | (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
+      Ring ring{0, 0};
+      for_units(p, 0, [&](const Part& q, const Unit& u, int it) -> bool {
+        if (q.what == DX) return issue_unit<DX>(sh, tiles, 0, p, q.bn, u, it, &ring);
+        if (q.what == DW) return issue_unit<DW>(sh, tiles, 0, p, q.bn, u, it, &ring);
+        return issue_unit<DB>(sh, tiles, d_ones, p, q.bn, u, it, &ring);
+      });
+    }
+  } else {
+    finish((Sh*)sh, staging, p, &map_dx, &map_dw, rank, (warp - 2) >> 2, warp & 3, lane);
+  }
+  __syncwarp();
+  teardown(sh, warp);
+}
+
+static int max_clusters() {
+  static int n = 0;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaFuncSetAttribute(linear_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BWD_SMEM_BYTES);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2 * (gemm_sm_count() / 2)); cfg.blockDim = dim3(GROUP_THREADS);
+    cfg.dynamicSmemBytes = BWD_SMEM_BYTES; cfg.attrs = at; cfg.numAttrs = 1;
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, (void*)linear_bwd_kernel, &cfg) == cudaSuccess && c > 0) n = c;
+    else { cudaGetLastError(); n = gemm_sm_count() / 2; }
+  });
+  return n;
+}
+
+// ---------------------------------------------------------------- the work list
+struct Choice { int bn, slices; };
+
+static void set_part(Part* q, int what, int rows, int in, int out, Choice c) {
+  q->what = what;
+  q->M = what == DX ? rows : out;
+  q->N = what == DB ? 1 : in;
+  q->bn = what == DB ? BN : c.bn;
+  q->tiles_m = (q->M + 2 * BM - 1) / (2 * BM);
+  q->tiles_n = what == DB ? 1 : (in + c.bn - 1) / c.bn;
+  q->k_blocks = ((what == DX ? out : rows) + BK - 1) / BK;
+  q->per = (q->k_blocks + c.slices - 1) / c.slices;
+  q->slices = (q->k_blocks + q->per - 1) / q->per;
+}
+
+// Cycles of a unit: those of its K blocks (the MMAs of 256 columns, the operands' way out of L2 for fewer) and its epilogue's
+// share, with the partial tile's way to the workspace and back where there are slices.  Fitted to 41 shapes (8 - 8192 rows, 128 - 4096
+// inputs and outputs) in up to 1500 forms each: the form that these numbers choose takes 0.7 % longer than the best of them on
+// average, 7 % at most.
+static int unit_cycles(const Part& q) {
+  if (q.what == DB) return q.per * 301 + 303 + (q.slices > 1 ? 76 * q.slices : 0);
+  return q.per * (q.bn == 256 ? 512 : q.bn == 192 ? 403 : 342) + (q.slices > 1 ? 53 * q.bn + 11 * q.bn * q.slices / 2 : 35 * q.bn / 2);
+}
+
+struct Candidate { Choice c; int cycles, units; };
+
+static int candidates(int what, int rows, int in, int out, int clusters, Candidate* list) {
+  int n = 0;
+  for (int bn = 256; bn >= (what == DB ? 256 : 128); bn -= 64)
+    for (int s : {1, 2, 3, 4, 6, 8}) {
+      Part q;
+      set_part(&q, what, rows, in, out, {bn, s});
+      const int units = q.tiles_m * q.tiles_n * q.slices;
+      // slices of eight K blocks or more, and of an output that leaves clusters idle or deals out badly
+      if (s == 1 || (q.slices == s && q.per >= 8 && (what == DB || units <= 4 * clusters))) list[n++] = {{bn, s}, unit_cycles(q), units};
+    }
+  return n;
+}
+
+// The time of the first cluster, which has the longest unit of every round.
+static long long span(const Candidate* const (&c)[3], int parts, int clusters) {
+  const Candidate* o[3];
+  for (int i = 0; i < parts; ++i) {          // longest first
+    int j = i;
+    for (; j > 0 && o[j - 1]->cycles < c[i]->cycles; --j) o[j] = o[j - 1];
+    o[j] = c[i];
+  }
+  long long t = 0, at = 0, end = 0;
+  for (int i = 0; i < parts; ++i) {
+    end += o[i]->units;
+    if (at < end) {
+      const long long rounds = (end - at + clusters - 1) / clusters;
+      t += rounds * o[i]->cycles;
+      at += rounds * clusters;
+    }
+  }
+  return t;
+}
+
+// Tiles and slices of the products in `want`; kept per thread for the sizes last asked for (about 1 - 10 us to find).
+static void choose(int rows, int in, int out, int want, int clusters, Choice (&best)[3]) {
+  struct Kept { int key[5]; Choice c[3]; };
+  static thread_local Kept kept[32];
+  const int key[5] = {rows, in, out, want, clusters};
+  Kept& k = kept[((unsigned)rows * 31 + (unsigned)in * 7 + (unsigned)out * 3 + (unsigned)want) / 8 % 32];
+  if (!std::equal(key, key + 5, k.key)) {
+    Candidate x[18], w[18], b[6];
+    const int nx = want >> DX & 1 ? candidates(DX, rows, in, out, clusters, x) : 0, nw = want >> DW & 1 ? candidates(DW, rows, in, out, clusters, w) : 0;
+    const int nb = want >> DB & 1 ? candidates(DB, rows, in, out, clusters, b) : 0;
+    long long least = -1;
+    for (int i = 0; i < std::max(1, nx); ++i)
+      for (int j = 0; j < std::max(1, nw); ++j) {
+        const Candidate* c[3] = {};
+        int parts = 0, l = 0;
+        if (nx) c[parts++] = &x[i];
+        if (nw) c[parts++] = &w[j];
+        if (nb) {                              // db's units no longer than dW's, with which they run
+          while (l + 1 < nb && b[l].cycles > (nw ? w[j].cycles : x[i].cycles)) ++l;
+          c[parts++] = &b[l];
+        }
+        const long long t = span(c, parts, clusters);
+        if (least < 0 || t < least) {
+          least = t;
+          k.c[DX] = nx ? x[i].c : Choice{BN, 1};
+          k.c[DW] = nw ? w[j].c : Choice{BN, 1};
+          k.c[DB] = nb ? b[l].c : Choice{BN, 1};
+        }
+      }
+    std::copy(key, key + 5, k.key);
+  }
+  std::copy(k.c, k.c + 3, best);
+}
+
+// form (0: chosen): columns / 64 and slices of dX, of dW, slices of db, four bits each from the lowest.
+static int plan(int rows, int in, int out, int want, int form, int clusters, Problem* p, size_t* ws_floats, int* counters) {
+  Choice c[3];
+  if (form) {
+    for (int what = DX; what <= DW; ++what) {
+      c[what] = {64 * (form >> (8 * what) & 15), form >> (8 * what + 4) & 15};
+      if (c[what].bn < 128 || c[what].bn > 256) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
+    }
+    c[DB] = {BN, form >> 16 & 15};
+    for (const Choice& x : c) if (x.slices < 1) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
+  } else {
+    choose(rows, in, out, want, clusters, c);
+  }
+  p->parts = 0;
+  for (int what = DX; what <= DB; ++what)
+    if (want >> what & 1) set_part(&p->part[p->parts++], what, rows, in, out, c[what]);
+  std::sort(p->part, p->part + p->parts, [](const Part& a, const Part& b) { return unit_cycles(a) > unit_cycles(b); });
+  long long first = 0, ws = 0;
+  *counters = 0;
+  for (int i = 0; i < p->parts; ++i) {
+    Part& q = p->part[i];
+    const int tiles = q.tiles_m * q.tiles_n;
+    q.first = (int)first;
+    q.ws = ws;
+    q.arrivals = *counters;
+    first += (long long)tiles * q.slices;
+    if (q.slices > 1) {
+      ws += 2LL * tiles * q.slices * BM * (q.what == DB ? 1 : q.bn);
+      *counters += 2 * tiles;
+    }
+  }
+  p->total = (int)first;
+  *ws_floats = (size_t)ws;
+  return TMPI_OK;
+}
+
+}  // namespace lbwd
+}  // namespace tmpi
+
+using namespace tmpi;
+
+extern "C" {
+
+// What a call needs: bytes of workspace and arrival counters (unsigned, zero before the first call that uses them; every call leaves
+// them zero).  want: 1 dX, 2 dW, 4 db, of which at least one of the first two.
+int tmpi_linear_bwd_plan(int rows, int in, int out, int want, int form, size_t* workspace_bytes, int* counters) {
+  if (rows < 1 || in < 1 || out < 1 || in % 8 || out % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
+  if (!(want & 3) || want & ~7) return fail(TMPI_ERR_INVALID, "linear_bwd: nothing to compute");
+  lbwd::Problem p{};
+  size_t ws = 0;
+  const int st = lbwd::plan(rows, in, out, want, form, lbwd::max_clusters(), &p, &ws, counters);
+  *workspace_bytes = ws * sizeof(float);
+  return st;
+}
+
+// dx [rows, in] = dy w, dw [out, in] = dy^T x, db [out] = column sums of dy, for dy [rows, out], x [rows, in], w [out, in], all dense
+// bf16 with fp32 accumulation; dx, dw, db may be null.  Calls that share workspace or counters must not overlap.
+int tmpi_linear_bwd(const void* dy, const void* x, const void* w, void* dx, void* dw, void* db, int rows, int in, int out, int form,
+                    void* workspace, size_t workspace_bytes, void* counters, int ncounters, void* stream) {
+  const int want = (dx ? 1 : 0) | (dw ? 2 : 0) | (db ? 4 : 0);
+  if (rows < 1 || in < 1 || out < 1 || in % 8 || out % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
+  if (!(want & 3)) return fail(TMPI_ERR_INVALID, "linear_bwd: nothing to compute");
+  const int clusters = lbwd::max_clusters();
+  lbwd::Problem p{};
+  size_t ws = 0;
+  int need = 0, st;
+  if ((st = lbwd::plan(rows, in, out, want, form, clusters, &p, &ws, &need))) return st;
+  if ((ws && (!workspace || ((uintptr_t)workspace & 15))) || workspace_bytes < ws * sizeof(float) || ncounters < need || (need && !counters))
+    return fail(TMPI_ERR_INVALID, "linear_bwd: workspace of %zu bytes (16-byte aligned) and %d counters needed", ws * sizeof(float), need);
+  p.ws = (float*)workspace;
+  p.arrivals = (unsigned*)counters;
+  p.db = (__nv_bfloat16*)db;
+  p.status = gemm_status_word();
+  CUtensorMap mdy, mx, mw, mdx, mdw;
+  if ((st = make_tmap_bf16(&mdy, dy, (uint64_t)rows, (uint64_t)out, (uint64_t)out, 64))) return st;
+  mx = mw = mdx = mdw = mdy;
+  if (dw && (st = make_tmap_bf16(&mx, x, (uint64_t)rows, (uint64_t)in, (uint64_t)in, 64))) return st;
+  if (dx && (st = make_tmap_bf16(&mw, w, (uint64_t)out, (uint64_t)in, (uint64_t)in, 64))) return st;
+  if (dx && (st = make_tmap_bf16(&mdx, dx, (uint64_t)rows, (uint64_t)in, (uint64_t)in, 64))) return st;
+  if (dw && (st = make_tmap_bf16(&mdw, dw, (uint64_t)out, (uint64_t)in, (uint64_t)in, 64))) return st;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see pdl.cuh
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(2 * std::min(p.total, clusters)); cfg.blockDim = dim3(gemm2::GROUP_THREADS);
+  cfg.dynamicSmemBytes = lbwd::BWD_SMEM_BYTES; cfg.stream = (cudaStream_t)stream; cfg.attrs = at; cfg.numAttrs = 2;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, lbwd::linear_bwd_kernel, mdy, mx, mw, mdx, mdw, p);
+  return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "linear_bwd launch: %s", cudaGetErrorString(e));
+}
+
+}  // extern "C"

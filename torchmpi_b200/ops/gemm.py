@@ -2,8 +2,8 @@
 
 ``matmul_nt(a, b)`` computes ``a @ b.T`` for row-major ``a [M, K]`` and ``b [N, K]`` (K contiguous,
 bf16), optionally with bias and GELU in the epilogue.  ``linear(x, w, bias, gelu)`` is the autograd
-version (csrc/bindings/autograd.cpp): ``dX = dY @ W`` (as ``matmul_nn``) and ``dW = dY.T @ X`` (as ``matmul_tn``) read
-their operands as they lie, through MN-major shared-memory descriptors, so backward makes no transposed copies.
+version (csrc/bindings/autograd.cpp): ``dX = dY @ W``, ``dW = dY.T @ X`` and the bias gradient are one launch
+(csrc/kernels/linear_bwd.cu) that reads its operands as they lie, so backward makes no transposed copies.
 """
 from __future__ import annotations
 
@@ -100,8 +100,8 @@ def matmul_tn(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = No
 
 
 def check_status() -> None:
-    """Raises if a GEMM CTA gave up on one of its bounded waits since the last call.  Weight gradients of few tiles and many
-    rows run on the convolution's split-K kernels, which report to the convolution's word."""
+    """Raises if a GEMM CTA gave up on one of its bounded waits since the last call.  ``conv.matmul_tn_splitk`` runs on
+    the convolution's kernels, which report to the convolution's word."""
     st = lib.tmpi_gemm_status() or lib.tmpi_conv_status()
     if st:
         raise TorchMPIError(3, f"tcgen05 GEMM: a bounded wait ran out (code {st})")
