@@ -15,12 +15,13 @@
 //
 // What bounds it: neither the special-function unit (16 exp2 per cycle and SM, 1024 cycles per 128 x 128 block; a quarter of
 // them run as a cubic on the FMA pipe) nor the MMAs (512 cycles per block), but the latency of a team's chain S -> maximum
-// -> P -> P V, about 1.9 us per key block.  Everything that is not needed per score is therefore kept off the softmax
+// -> P -> P V, about 1.6 us per key block.  Everything that is not needed per score is therefore kept off the softmax
 // warps: P goes to tensor memory (no shared-memory stores, swizzle arithmetic or proxy fence), and O stays in tensor
 // memory: only where a row's maximum grew do its threads scale O there by exp2(old max - new max), instead of reading every
 // O_j back.  Tried and taken back: moving the maximum only when it grows by more than 2^8 (the largest P of a row is then
 // no longer exactly 1, and its bf16 rounding showed in the output); one thread per row (63 us in place of 56); all
-// exponentials before the wait for the previous product (61); descriptors in uniform registers (no difference).
+// exponentials before the wait for the previous product (61); descriptors in uniform registers (no difference); an item's output
+// written inside the next one's first block (no faster, 34 in place of 22 us where the teams share items: registers).
 //
 // A CTA (one per SM) runs two such teams, each with its own rings, barriers and 256 tensor-memory columns, so that
 // one exponentiates while the other waits.  Each has items of its own, or, where there are few, both work on the same one, on half
@@ -28,7 +29,8 @@
 // r * G + i, then r * G + G - 1 - i), which leaves the key blocks per team within one of each other at 8 x 16 x 1024; the
 // next item's loads and first S run under the end of the current one.
 //
-// Measured on a B200, launches in a row: 8 x 16 heads x 1024 x 64 49.7 us, 1 x 16 x 2048 26.8 (33.4 with a team per item).
+// Measured on a B200, launches in a row: 8 x 16 heads x 1024 x 64 40.6 us, 1 x 16 x 2048 21.0 (47.7 and 25.5 before waiting warps
+// slept, waits looked at the error word only when they do not succeed, and the halves met at named barriers).
 //
 // Q, K and V are read where the fused QKV projection left them ([B * T, 3 C], one tensor map per operand) and the
 // output is written as [B * T, C]: no transposes around the kernel.  Every wait is bounded; a CTA that gives up records
@@ -69,7 +71,6 @@ constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
   uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_full, pv_done, o_empty;
-  uint64_t pair[4];            // the two warps that share 32 rows meet here (bounded, unlike a named barrier)
   uint64_t merge_full, merge_empty;      // of team 1, where the teams share items: its row sums are there, have been read
   uint32_t tmem_base;
   int error;
@@ -125,7 +126,7 @@ template <bool SHARED> struct Items {
 };
 
 #define ATTN_WAIT(bar, parity, where) \
-  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
+  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); return; } } while (0)
 
 template <bool SHARED>
 __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
@@ -136,7 +137,7 @@ __device__ void producer(Shared* sh, unsigned char* tiles, const Params& p, cons
     const int b = it.bh / p.H, h = it.bh - b * p.H, row0 = b * p.T;
     auto load_k = [&](int j) -> bool {
       const int st = kc & 1;
-      if (kc >= 2 && (!sm100::mbar_wait(&sh->k_empty[st], ((kc >> 1) - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
+      if (kc >= 2 && (!sm100::mbar_wait(&sh->k_empty[st], ((kc >> 1) - 1) & 1, kWaitBudgetNs, &sh->error))) return false;
       sm100::mbar_expect_tx(&sh->k_full[st], TILE_BYTES);
       sm100::tma_load_2d(tiles + K_OFF + st * TILE_BYTES, mk, h * D, row0 + j * BKV, &sh->k_full[st]);
       ++kc;
@@ -170,9 +171,9 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, const Params& p) {
   int g = 0;                                               // key blocks whose S has been issued, over all items
   // S of a key block of this team's r-th item (block number g): waits for the softmax warps to have read the previous S
   auto issue_s = [&](int r, bool first, bool last) -> bool {
-    if (first && (!sm100::mbar_wait(&sh->q_full[r & 1], (r >> 1) & 1, kWaitBudgetNs) || sh->error)) return false;
-    if (!sm100::mbar_wait(&sh->k_full[g & 1], (g >> 1) & 1, kWaitBudgetNs) || sh->error) return false;
-    if (g >= 1 && (!sm100::mbar_wait(&sh->s_empty, (g - 1) & 1, kWaitBudgetNs) || sh->error)) return false;
+    if (first && (!sm100::mbar_wait(&sh->q_full[r & 1], (r >> 1) & 1, kWaitBudgetNs, &sh->error))) return false;
+    if (!sm100::mbar_wait(&sh->k_full[g & 1], (g >> 1) & 1, kWaitBudgetNs, &sh->error)) return false;
+    if (g >= 1 && (!sm100::mbar_wait(&sh->s_empty, (g - 1) & 1, kWaitBudgetNs, &sh->error))) return false;
     sm100::tc_fence_after();
     const uint64_t a = at(dq, (r & 1) * TILE_BYTES), b = at(dk, (g & 1) * TILE_BYTES);
 #pragma unroll
@@ -234,6 +235,15 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint32_t (&w)
   }
 }
 
+// The two warps that share 32 rows meet at a named barrier (an mbarrier between them: 42.3 us in place of 40.8 at 8 x 16 x 1024, 22.1 in
+// place of 20.9 for 1 x 16 x 2048).  A warp that gives up sets the error word and arrives there once more, so that its partner is
+// not left waiting.  The partner then ends at its next s_full or pv_done, which need all warps; only at the end of an item does it come
+// here twice without such a wait, and looks at the word in between.
+__device__ __forceinline__ void pair_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(1 + team() * 4 + quarter) : "memory"); }
+__device__ __forceinline__ void pair_leave(int quarter) { asm volatile("bar.arrive %0, 64;" ::"r"(1 + team() * 4 + quarter) : "memory"); }
+#define ROWS_WAIT(bar, parity, where) \
+  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); __syncwarp(); pair_leave(quarter); return; } } while (0)
+
 // Two threads per query row: `half` picks 64 of the 128 scores of a block and 32 of the 64 output columns.  The halves
 // exchange their maxima through shared memory, block by block, and their row sums at the end of an item.
 template <bool SHARED>
@@ -246,15 +256,12 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
   const bool tracer = row == 0 && half == 0;
   int g = 0, met = 0, merged = 0;                          // key blocks done, exchanges made and items merged so far
   // this row's value of the other half
-  auto exchange = [&](float v, float* other) -> bool {
+  auto exchange = [&](float v, float* other) {
     float* x = xch + (met & 1) * 2 * BQ;
     x[half * BQ + row] = v;
-    __syncwarp();
-    if (lane == 0) sm100::mbar_arrive(&sh->pair[quarter]);
-    if (!sm100::mbar_wait(&sh->pair[quarter], met & 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 11); return false; }
+    pair_sync(quarter);
     *other = x[(half ^ 1) * BQ + row];
     ++met;
-    return true;
   };
   Items<SHARED> it;
   for (int r = 0; it.next(p); ++r) {
@@ -264,7 +271,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       const bool diag = j == it.qblk;
       uint32_t s[2][32];
       if (tracer) stamp(p, r, j, 0);
-      ATTN_WAIT(&sh->s_full, g & 1, 7);
+      ROWS_WAIT(&sh->s_full, g & 1, 7);
       if (tracer) stamp(p, r, j, 1);
       sm100::tc_fence_after();
 #pragma unroll
@@ -293,7 +300,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
         mx3 = max3_nan(mx3, __uint_as_float(s[1][i + 2]), __uint_as_float(s[1][i + 3]));
       }
       float mx = max_nan(max3_nan(mx0, mx1, mx2), mx3), mx_other;
-      if (!exchange(mx, &mx_other)) return;
+      exchange(mx, &mx_other);
       mx = max_nan(mx, mx_other);
       if (tracer) stamp(p, r, j, 2);
       // the running maximum; where it grew, O and l so far are scaled by alpha (1 for rows where it did not)
@@ -321,7 +328,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
           exp_chunk(s[c], w, c2x2, nmc2, sum2[c]);
         }
         if (c == 0 && g > 0) {     // the previous block's product has read its P and added to O
-          ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 8);
+          ROWS_WAIT(&sh->pv_done, (g - 1) & 1, 8);
           if (tracer && j > it.first) { stamp(p, r, j - 1, 5); stamp(p, r, j - 1, 6); }
           sm100::tc_fence_after();
         }
@@ -352,13 +359,14 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
     // the item's output: O / l
     float l0, l1, l_other;
     unpack2(add2(sum2[0], sum2[1]), l0, l1);
-    if (!exchange(l0 + l1, &l_other)) return;
+    if (*(volatile int*)&sh->error) { pair_leave(quarter); return; }     // the partner may have left at the last exchange
+    exchange(l0 + l1, &l_other);
     float l = half ? l_other + (l0 + l1) : (l0 + l1) + l_other;
     const bool merges = SHARED && it.qblk > 0;
     if (merges && team()) {                                // hand over O (in tensor memory), maximum and sum; go on
-      if (merged > 0) ATTN_WAIT(&sh->merge_empty, (merged - 1) & 1, 16);
+      if (merged > 0) ROWS_WAIT(&sh->merge_empty, (merged - 1) & 1, 16);
       if (half == 0) merge[row] = make_float2(m, l);
-      ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
+      ROWS_WAIT(&sh->pv_done, (g - 1) & 1, 10);
       sm100::tc_fence_after();
       sm100::tc_fence_before();
       __syncwarp();
@@ -367,14 +375,14 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
       continue;
     }
     float inv = 1.f / l;
-    ATTN_WAIT(&sh->pv_done, (g - 1) & 1, 10);
+    ROWS_WAIT(&sh->pv_done, (g - 1) & 1, 10);
     if (tracer) stamp(p, r, it.qblk, 5);
     sm100::tc_fence_after();
     uint32_t o[32];
     sm100::tmem_ld_32x32(tmem_o, o);
     sm100::tmem_ld_wait();
     if (merges) {
-      ATTN_WAIT(&other_team->merge_full, merged & 1, 17);
+      ROWS_WAIT(&other_team->merge_full, merged & 1, 17);
       ++merged;
       sm100::tc_fence_after();
       const float2 with = merge[row];
@@ -439,7 +447,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     sm100::mbar_init(&sh->p_full, SOFTMAX_WARPS);
     sm100::mbar_init(&sh->pv_done, 1);
     sm100::mbar_init(&sh->o_empty, SOFTMAX_WARPS);
-    for (int q = 0; q < 4; ++q) sm100::mbar_init(&sh->pair[q], 2);
     sm100::mbar_init(&sh->merge_full, SOFTMAX_WARPS);
     sm100::mbar_init(&sh->merge_empty, SOFTMAX_WARPS);
     sh->error = 0;

@@ -2,32 +2,34 @@
 // log-sum-exp and delta = rowsum(dO * O).
 //
 // A work item is one block of 128 keys of one (batch, head); a persistent CTA per SM walks the query blocks of an item
-// from its diagonal to the end of the sequence.  Scores are computed transposed, [key][query], so that P and dS are born
-// in the layout in which the tensor core takes its first operand out of tensor memory.  Per pair (query block i, key
+// from its diagonal to the end of the sequence.  Scores are computed transposed, [key][query], so that P is born in
+// the layout in which the tensor core takes its first operand out of tensor memory.  Per pair (query block i, key
 // block j), five MMAs with fp32 accumulators in tensor memory:
 //
 //   S^T  = K_j Q_i^T          dP^T = V_j dO_i^T                     (128 keys x 128 queries each)
-//   dV  += P^T dO_i           dK  += dS^T Q_i                       (P^T, dS^T read from tensor memory; 128 x 64)
-//   dQ_ij = dS K_j                                                  (dS^T read MN-major out of shared memory; 128 x 64)
+//   dV  += P^T dO_i                                                 (P^T read from tensor memory; 128 x 64)
+//   dK  += dS^T Q_i           dQ_ij = dS K_j                        (dS^T read out of shared memory, K-major and MN-major; 128 x 64)
 //
 // with P = exp(scale S - lse) and dS = P (dP - delta); the softmax scale is applied to dK and dQ at the end.
 //
 //   warp 0      TMA producer: K_j and V_j through two buffers (the next item's arrive under the current one), Q_i, dO_i
 //               and the block's 128 lse / delta values through a three-stage ring
-//   warp 1      MMA issuer; order per pair n: S(n+1), dV(n), dK(n), dQ(n), dP(n+1), so that the exponentials of pair
+//   warp 1      MMA issuer; order per pair n: S(n+1), dV(n), dP(n+1), dK(n), dQ(n), so that the exponentials of pair
 //               n + 1 run under the products of pair n
 //   warps 4-7   drain dQ_ij (every pair) and dK, dV (every item): one thread per row; dQ goes through a swizzled staging
-//               tile and is added to the fp32 buffer by the TMA unit (cp.reduce, whole 128-byte rows)
-//   warps 8-23  four threads per key row: P^T as bf16 into its own tensor-memory columns, then dS^T over the dP^T columns
-//               that the thread itself has read, and into shared memory for dQ
+//               tile and is added to the fp32 buffer by the TMA unit (cp.reduce, whole 128-byte rows), dK and dV are stored
+//               through the same tiles (as 16-byte stores of 32 different rows they held up the next item for 2.5 us)
+//   warps 8-23  four threads per key row: P^T as bf16 into its own tensor-memory columns, dS^T into shared memory, where both
+//               dK and dQ read it: dP of the next pair need not wait until dK has read dS out of dP's columns
 //
-// What bounds it: not the MMAs (1280 cycles per pair, about 1700 with their shared-memory operands) nor the 16384
-// exponentials (1024 cycles), but the chain dP -> dS -> dK, dQ -> dP of a pair, about 4000 cycles: tensor-memory and
-// shared-memory latencies of warps that work on the same pair.  So nothing but two packed operations per pair of scores, the
-// rounding and the stores lies on it, and sixteen softmax warps share it (eight: 105 us in place of 97).  The version before
-// kept P and dS in shared memory (2400 cycles of operand traffic per pair), was not persistent, and added dQ with
-// red.global.v4 from the accumulator layout (32 different lines per instruction).  Measured on a B200, 8 x 16 heads x
-// 1024 x 64, this kernel: 122 -> 97 us.
+// What bounds it: neither the MMAs (about 1500 cycles per pair with their shared-memory operands) nor the 16384
+// exponentials (1024 cycles), but the softmax warps' instructions and latencies, which fill the pair's 3500 cycles without a wait for
+// the MMAs.  So nothing but two packed operations per pair of scores, the rounding and the stores lies there; masks are
+// applied in the diagonal pair's own branch; a wait that succeeds does not look at the error word; waiting warps sleep.  Sixteen softmax
+// warps share the work (eight: 105 us in place of 97).  Tried and taken back: half of the softmax warps offset by half a pair, so
+// that the exponentials of some run beside the stores of the others (116 in place of 109); the statistics scaled by a warp of their
+// own (100 in place of 96).  Measured on a B200, 8 x 16 heads x 1024 x 64, the three launches of a backward in a row: 113.5
+// -> 93.8 us, of which this kernel 70; 1 x 16 x 2048 46.8 -> 40.1.
 //
 // The order in which CTAs add to dQ is not fixed, so its low bits vary; dK and dV are bit-reproducible.  Every wait is
 // bounded; a CTA that gives up records where and frees its tensor memory.
@@ -70,7 +72,7 @@ constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
 
 struct alignas(128) Shared {
   uint64_t kv_full[2], kv_empty[2], qd_full[QD_STAGES], qd_empty[QD_STAGES], s_full, s_empty, p_full, dv_done, dp_full, ds_full,
-      dk_done, dq_full, dq_empty, acc_full, acc_empty;
+      dq_full, dq_empty, acc_full, acc_empty;
   uint32_t tmem_base;
   int error;
 };
@@ -81,9 +83,6 @@ struct Params {
   float scale, scale_log2;
   const float* lse;            // [B, H, T], natural log
   const float* delta;          // [B, H, T]
-  __nv_bfloat16* dk;           // [B * T, ld_dkv], head h at columns h * 64
-  __nv_bfloat16* dv;
-  int ld_dkv;
   int* status;
   unsigned long long* trace;   // optional: time stamps of the phases of CTA 0 (see tmpi_attention_bwd_set_trace)
 };
@@ -118,7 +117,7 @@ struct Ring {
 };
 
 #define ATTNB_WAIT(bar, parity, where) \
-  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs) || sh->error) { fail(sh, p, (where)); return; } } while (0)
+  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); return; } } while (0)
 
 __device__ void producer(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
                          const CUtensorMap* mv, const CUtensorMap* mdo) {
@@ -158,8 +157,9 @@ __device__ void mma_issuer(Shared* sh, unsigned char* smem, const Params& p) {
   const uint64_t q_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + Q_OFF), TILE, 1024);
   const uint64_t do_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + DO_OFF), TILE, 1024);
   const uint64_t ds_mn = sm100::make_desc_sw128_mn(sm100::smem_u32(smem + DS_OFF), TILE, 1024);
+  const uint64_t ds_k = sm100::make_desc_sw128(sm100::smem_u32(smem + DS_OFF));
   auto ready = [&](uint64_t* bar, int parity, int where) -> bool {
-    if (sm100::mbar_wait(bar, parity & 1, kWaitBudgetNs) && !sh->error) return true;
+    if (sm100::mbar_wait(bar, parity & 1, kWaitBudgetNs, &sh->error)) return true;
     fail(sh, p, where);
     return false;
   };
@@ -206,12 +206,15 @@ __device__ void mma_issuer(Shared* sh, unsigned char* smem, const Params& p) {
       if (!ready(&sh->ds_full, g, 8)) return;
       stamp(p, r, n, 10);
       sm100::tc_fence_after();
+      if (next) {                                          // dP of the next pair: this pair's has been read
+        product_128(T_DP, at(v_k, kvn * TILE), at(do_k, qn.stage * TILE));
+        sm100::umma_commit(&sh->dp_full);
+      }
 #pragma unroll
-      for (int k = 0; k < BLK / UMMA_K; ++k)               // dK += dS^T Q: dS^T sits in the first half of each 32 columns of dP^T
-        sm100::umma_f16_tmem_a(tm + T_DK, tm + T_DP + (k >> 1) * 32 + (k & 1) * 8, at(q_mn, q.stage * TILE + k * UMMA_K * 128), idesc_a,
-                               (n | k) ? 1u : 0u);
-      sm100::umma_commit(&sh->dk_done);
-      sm100::umma_commit(&sh->qd_empty[q.stage]);          // both products that read this stage are done
+      for (int k = 0; k < BLK / UMMA_K; ++k)               // dK += dS^T Q: 16 queries = 32 bytes of the rows of dS^T, 16 rows of Q
+        sm100::umma_f16(tm + T_DK, at(ds_k, (k >> 2) * TILE + (k & 3) * UMMA_K * 2), at(q_mn, q.stage * TILE + k * UMMA_K * 128), idesc_a,
+                        (n | k) ? 1u : 0u);
+      sm100::umma_commit(&sh->qd_empty[q.stage]);          // every product that reads this stage is done
       if (last) sm100::umma_commit(&sh->acc_full);
       if (g > 0 && !ready(&sh->dq_empty, g - 1, 9)) return;
       sm100::tc_fence_after();
@@ -221,12 +224,6 @@ __device__ void mma_issuer(Shared* sh, unsigned char* smem, const Params& p) {
       sm100::umma_commit(&sh->dq_full);                    // also: dS in shared memory is free again
       if (last) sm100::umma_commit(&sh->kv_empty[kv]);
       stamp(p, r, n, 12);
-      if (next) {                                          // dP of the next pair, once dK has read dS out of these columns
-        if (!ready(&sh->dk_done, g, 10)) return;
-        sm100::tc_fence_after();
-        product_128(T_DP, at(v_k, kvn * TILE), at(do_k, qn.stage * TILE));
-        sm100::umma_commit(&sh->dp_full);
-      }
       q = qn;
     }
   }
@@ -237,8 +234,8 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
   const int row = quarter * 32 + lane;                     // key inside the block; tensor-memory lane
   const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
   const uint32_t t_s = tm + T_S + part * 32, t_dp = tm + T_DP + part * 32, t_p = tm + T_P + part * 16;
-  unsigned char* ds_row = smem + DS_OFF + (part >> 1) * TILE + row * 128;
-  const int unit0 = (part & 1) * 4;                        // first 16-byte unit of this thread's queries in the row
+  // this thread's first 16-byte unit in the swizzled row of dS; the other three differ from it in two bits of the address
+  const uint32_t ds_unit = sm100::smem_u32(smem + DS_OFF + (part >> 1) * TILE + row * 128) + ((((part & 1) * 4) ^ (row & 7)) << 4);
   const unsigned long long c2x2 = pack2(__float_as_uint(p.scale_log2), __float_as_uint(p.scale_log2));
   const unsigned long long nl2e = pack2(__float_as_uint(-1.4426950408889634f), __float_as_uint(-1.4426950408889634f));
   const bool tracer = row == 0 && part == 0;
@@ -251,7 +248,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       const float4* delta = lse + STAT_BYTES / 16;
       const bool diag = n == 0, masked = diag && part < quarter;               // masked: every query of the thread is before its key
       if (tracer) stamp(p, r, n, 0);
-      ATTNB_WAIT(&sh->qd_full[q.stage], q.use & 1, 11);    // lse and delta (the MMA waits for the tiles itself)
+      ATTNB_WAIT(&sh->qd_full[q.stage], q.use & 1, 11);
       ATTNB_WAIT(&sh->s_full, g & 1, 12);
       if (tracer) stamp(p, r, n, 1);
       sm100::tc_fence_after();
@@ -261,12 +258,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       sm100::tc_fence_before();
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&sh->s_empty);     // S is in registers: the next pair's may overwrite it
-      if (masked) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) s[e] = 0u;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) w[e] = 0u;
-      } else {
+      if (!masked) {
 #pragma unroll
         for (int u = 0; u < 8; ++u) {                      // P = exp2(S * scale * log2(e) - lse * log2(e)) over S in place
           const float4 l = lse[u];                         // the same four values for all lanes
@@ -276,15 +268,16 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
           unpack2(fma2(pack2(s[4 * u], s[4 * u + 1]), c2x2, l01), a[0], a[1]);
           unpack2(fma2(pack2(s[4 * u + 2], s[4 * u + 3]), c2x2, l23), a[2], a[3]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float v = ex2(a[e]);
-            if (diag && part * 32 + 4 * u + e < row) v = 0.f;                  // the diagonal block: a query before the key
-            s[4 * u + e] = __float_as_uint(v);
-          }
-          w[2 * u] = pack_bf16(s[4 * u], s[4 * u + 1]);
-          w[2 * u + 1] = pack_bf16(s[4 * u + 2], s[4 * u + 3]);
+          for (int e = 0; e < 4; ++e) s[4 * u + e] = __float_as_uint(ex2(a[e]));
         }
       }
+      if (diag) {                                          // the diagonal block: queries before the key
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (part * 32 + e < row) s[e] = 0u;
+      }
+#pragma unroll
+      for (int e = 0; e < 16; ++e) w[e] = pack_bf16(s[2 * e], s[2 * e + 1]);
       if (g > 0) {                                         // dV of the previous pair has read P
         ATTNB_WAIT(&sh->dv_done, (g - 1) & 1, 13);
         sm100::tc_fence_after();
@@ -294,8 +287,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       sm100::tc_fence_before();
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&sh->p_full);
-      if (g > 0) ATTNB_WAIT(&sh->dq_full, (g - 1) & 1, 14);                    // dQ of the previous pair has read dS
-      ATTNB_WAIT(&sh->dp_full, g & 1, 15);
+      ATTNB_WAIT(&sh->dp_full, g & 1, 14);
       sm100::tc_fence_after();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {                        // dS = P (dP - delta), 16 queries at a time
@@ -314,22 +306,25 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             __nv_bfloat162 hh = __floats2bfloat162_rn(a[2 * e], a[2 * e + 1]);
-            v[2 * u + e] = masked ? 0u : *reinterpret_cast<uint32_t*>(&hh);
+            v[2 * u + e] = *reinterpret_cast<uint32_t*>(&hh);
           }
         }
-        sm100::tmem_st_32x8(t_dp + c * 8, v);              // columns that this thread has read already
+        if (masked) {                                      // dP - delta may be no number there
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = 0u;
+        }
+        if (c == 0 && g > 0) ATTNB_WAIT(&sh->dq_full, (g - 1) & 1, 15);          // dK and dQ of the previous pair have read dS
 #pragma unroll
         for (int u = 0; u < 2; ++u)                        // eight queries = one 16-byte unit of the swizzled row
-          *reinterpret_cast<uint4*>(ds_row + (((unit0 + c * 2 + u) ^ (row & 7)) << 4)) =
-              make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                       ::"r"(ds_unit ^ ((c * 2 + u) << 4)), "r"(v[4 * u]), "r"(v[4 * u + 1]), "r"(v[4 * u + 2]), "r"(v[4 * u + 3]) : "memory");
       }
-      sm100::tmem_st_wait();
       sm100::fence_proxy_async_smem();                     // the MMA reads dS through the async proxy
       sm100::tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         sm100::mbar_arrive(&sh->ds_full);
-        sm100::mbar_arrive(&sh->qd_empty[q.stage]);        // lse and delta have been read
+        sm100::mbar_arrive(&sh->qd_empty[q.stage]);        // the statistics have been read
       }
       if (tracer) stamp(p, r, n, 2);
     }
@@ -337,7 +332,8 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
 }
 
 // Reads dQ of every pair and dK, dV of every item; one thread per row of the tile.
-__device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mdq, int quarter, int lane) {
+__device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mdq, const CUtensorMap* mdk, const CUtensorMap* mdv,
+                      int quarter, int lane) {
   const uint32_t tm = sh->tmem_base + ((uint32_t)(quarter * 32) << 16);
   unsigned char* staging = smem + DQ_OFF + quarter * (TILE / DRAIN_WARPS);      // 32 rows of 128 bytes
   const unsigned long long scale2 = pack2(__float_as_uint(p.scale), __float_as_uint(p.scale));
@@ -385,24 +381,27 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
     }
     ATTNB_WAIT(&sh->acc_full, r & 1, 17);
     sm100::tc_fence_after();
-    const size_t at = ((size_t)b * p.T + (size_t)jblk * BLK + quarter * 32 + lane) * p.ld_dkv + h * D;
-    auto store = [&](__nv_bfloat16* o) {
+    auto store = [&](const CUtensorMap* map) {             // 32 rows of 64 bf16 through the staging tile
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      __syncwarp();
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         uint32_t w[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = (u & 3) * 8 + 2 * e;
-          __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(v[u >> 2][i]), __uint_as_float(v[u >> 2][i + 1]));
-          w[e] = *reinterpret_cast<uint32_t*>(&hh);
-        }
-        *reinterpret_cast<uint4*>(o + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int e = 0; e < 4; ++e) w[e] = pack_bf16(v[u >> 2][(u & 3) * 8 + 2 * e], v[u >> 2][(u & 3) * 8 + 2 * e + 1]);
+        *reinterpret_cast<uint4*>(staging + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      sm100::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        sm100::tma_store_2d(map, staging, h * D, b * p.T + jblk * BLK + quarter * 32);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
     };
     sm100::tmem_ld_32x32(tm + T_DV, v[0]);
     sm100::tmem_ld_32x32(tm + T_DV + 32, v[1]);
     sm100::tmem_ld_wait();
-    store(p.dv + at);
+    store(mdv);
     sm100::tmem_ld_32x32(tm + T_DK, v[0]);
     sm100::tmem_ld_32x32(tm + T_DK + 32, v[1]);
     sm100::tmem_ld_wait();
@@ -411,7 +410,7 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
     if (lane == 0) sm100::mbar_arrive(&sh->acc_empty);
     scaled(v[0]);
     scaled(v[1]);
-    store(p.dk + at);
+    store(mdk);
   }
   if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");     // every addition is done before the kernel ends
 }
@@ -419,7 +418,8 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
 __global__ void __launch_bounds__(THREADS, 1)
 attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
-                     const __grid_constant__ CUtensorMap map_dq, const Params p) {
+                     const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dk,
+                     const __grid_constant__ CUtensorMap map_dv, const Params p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   Shared* sh = (Shared*)(smem_raw + SHARED_OFF);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -437,7 +437,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     sm100::mbar_init(&sh->dv_done, 1);
     sm100::mbar_init(&sh->dp_full, 1);
     sm100::mbar_init(&sh->ds_full, SOFTMAX_WARPS);
-    sm100::mbar_init(&sh->dk_done, 1);
     sm100::mbar_init(&sh->dq_full, 1);
     sm100::mbar_init(&sh->dq_empty, DRAIN_WARPS);
     sm100::mbar_init(&sh->acc_full, 1);
@@ -466,7 +465,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
   } else if (warp < 4 + DRAIN_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    drain(sh, smem_raw, p, &map_dq, warp & 3, lane);
+    drain(sh, smem_raw, p, &map_dq, &map_dk, &map_dv, warp & 3, lane);
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
     softmax_rows(sh, smem_raw, p, warp & 3, (warp - 4 - DRAIN_WARPS) >> 2, lane);
@@ -579,7 +578,7 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   cudaError_t e = launch_overlapped(attnb::attention_delta_kernel, dgrid, 256, 0, s, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                     ld_o, ld_do, delta, dq_acc, B, T, H);
   if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention backward launch: %s", cudaGetErrorString(e));
-  CUtensorMap mq, mk, mv, mdo, mdq;
+  CUtensorMap mq, mk, mv, mdo, mdq, mdk, mdv;
   int st;
   const uint64_t rows = (uint64_t)B * T, cols = (uint64_t)H * attnb::D;
   if ((st = make_tmap_bf16(&mq, q, rows, cols, (uint64_t)ld_qkv, 128))) return st;
@@ -587,6 +586,8 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   if ((st = make_tmap_bf16(&mv, v, rows, cols, (uint64_t)ld_qkv, 128))) return st;
   if ((st = make_tmap_bf16(&mdo, dout, rows, cols, (uint64_t)ld_do, 128))) return st;
   if ((st = make_tmap_f32(&mdq, dq_acc, rows, cols, cols, 32))) return st;
+  if ((st = make_tmap_bf16(&mdk, dk, rows, cols, (uint64_t)ld_dkv, 32))) return st;
+  if ((st = make_tmap_bf16(&mdv, dv, rows, cols, (uint64_t)ld_dkv, 32))) return st;
   const int smem = attnb::SMEM_BYTES;
   cudaError_t ae = cudaFuncSetAttribute(attnb::attention_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ae != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention backward: shared memory attribute: %s", cudaGetErrorString(ae));
@@ -594,11 +595,10 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   p.B = B; p.T = T; p.H = H; p.blocks = T / attnb::BLK;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse = lse; p.delta = delta;
-  p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.ld_dkv = (int)ld_dkv;
   p.status = attnb_status_word();
   p.trace = g_attnb_trace;
   p.items = B * H * p.blocks;
-  e = launch_overlapped(attnb::attention_bwd_kernel, std::min(p.items, gemm_sm_count()), attnb::THREADS, smem, s, mq, mk, mv, mdo, mdq, p);
+  e = launch_overlapped(attnb::attention_bwd_kernel, std::min(p.items, gemm_sm_count()), attnb::THREADS, smem, s, mq, mk, mv, mdo, mdq, mdk, mdv, p);
   if (dq && e == cudaSuccess) {
     if ((uintptr_t)dq & 15) return fail(TMPI_ERR_INVALID, "attention backward: dq must be 16-byte aligned");
     const long long groups = (long long)rows * (cols / 8);

@@ -70,19 +70,17 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
 // 2^(a - n) on [-0.5, 0.5] (relative error 7.5e-5, far below the bf16 rounding of P), and times 2^n.  Like ex2 it flushes
 // subnormals: the last product does, so that an argument of -inf (a masked score, clamped to -126) gives exactly 0.
 __device__ __forceinline__ unsigned long long ex2_fma2(float a, float b) {
-  const float x[2] = {fmaxf(a, -126.f), fmaxf(b, -126.f)};
-  uint32_t q[2], p[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float t = x[i] + 12582912.f;
-    const float f = x[i] - (t - 12582912.f);
-    float c = fmaf(0.05517157167196274f, f, 0.2426111102104187f);
-    c = fmaf(c, f, 0.6932610273361206f);
-    q[i] = __float_as_uint(fmaf(c, f, 0.9999280571937561f));
-    p[i] = (__float_as_uint(t) << 23) + 0x3f800000u;
-  }
+  auto both = [](float v) { return pack2(__float_as_uint(v), __float_as_uint(v)); };
+  const unsigned long long x = pack2(__float_as_uint(fmaxf(a, -126.f)), __float_as_uint(fmaxf(b, -126.f)));
+  const unsigned long long t = add2(x, both(12582912.f)), f = sub2(x, add2(t, both(-12582912.f)));
+  unsigned long long c = fma2(both(0.05517157167196274f), f, both(0.2426111102104187f));
+  c = fma2(c, f, both(0.6932610273361206f));
+  c = fma2(c, f, both(0.9999280571937561f));
+  float t0, t1;
+  unpack2(t, t0, t1);
   unsigned long long r;
-  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(q[0], q[1])), "l"(pack2(p[0], p[1])));
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;"
+      : "=l"(r) : "l"(c), "l"(pack2((__float_as_uint(t0) << 23) + 0x3f800000u, (__float_as_uint(t1) << 23) + 0x3f800000u)));
   return r;
 }
 

@@ -28,10 +28,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The thread may be suspended for up to 20 us (it goes on as soon as the phase is complete): without the hint a waiting warp comes
+// back soon and polls, and the polls of all roles that wait take issue slots from those that work.  Attention forward of
+// 8 x 16 heads x 1024 x 64: 47.2 -> 43.8 us, backward 95.6 -> 93.5.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
@@ -49,6 +52,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     for (int i = 0; i < 256; ++i)
       if (mbar_try_wait(bar, parity)) return true;
     if (now_ns() - t0 > budget_ns) return false;
+  }
+}
+
+// The same for the roles of a CTA that share an error word: a wait that does not succeed soon also ends (returns false) once another role
+// has given up.  A wait that succeeds does not look at the word: it costs a shared-memory load and a branch on the critical path of
+// every pipeline step, and a role that has given up leaves the others waiting here sooner or later.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long budget_ns, const int* error) {
+  for (int i = 0; i < 1024; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = now_ns();
+  for (;;) {
+    for (int i = 0; i < 256; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    if (*(const volatile int*)error || now_ns() - t0 > budget_ns) return false;
   }
 }
 
