@@ -29,7 +29,7 @@
 // warps share the work (eight: 105 us in place of 97).  Tried and taken back: half of the softmax warps offset by half a pair, so
 // that the exponentials of some run beside the stores of the others (116 in place of 109); the statistics scaled by a warp of their
 // own (100 in place of 96).  Measured on a B200, 8 x 16 heads x 1024 x 64, the three launches of a backward in a row: 113.5
-// -> 93.8 us, of which this kernel 70; 1 x 16 x 2048 46.8 -> 40.1.
+// -> 90.2 us, of which this kernel 70; 1 x 16 x 2048 46.8 -> 39.5.
 //
 // The order in which CTAs add to dQ is not fixed, so its low bits vary; dK and dV are bit-reproducible.  Every wait is
 // bounded; a CTA that gives up records where and frees its tensor memory.
@@ -484,6 +484,12 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   }
 }
 
+// The two passes around the main kernel are bound by the latency of their few dependent loads per thread.  Their indices are divided
+// in 32 bits (there are below 2^32 of them: the fp32 dQ buffer alone would have 137 GB), which is a fraction of the
+// instructions of a 64-bit division, and there are two rounds of blocks.  8 x 16 heads x 1024 x 64, the whole backward: 93.5 us with
+// 64-bit divisions and half the blocks, 92.0 and 90.2 without.
+constexpr int kPassBlocks = 148 * 16;
+
 // delta[b, h, t] = sum_d dO[b, t, h, d] * O[b, t, h, d]: eight threads per (row, head), one 16-byte load of O and of
 // dO each (a warp reads four whole 128-byte lines of each tensor per instruction), three shuffles; the same threads
 // clear their 64 entries of the fp32 dQ buffer, so the caller need not.
@@ -495,10 +501,10 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
   const int sub = threadIdx.x & 7;
   for (long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; idx < total;
        idx += ((long long)gridDim.x * blockDim.x) >> 3) {
-    const int h = (int)(idx % H);
-    const long long r = idx / H;                                 // b * T + t
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(o + r * ld_o + h * D) + sub);
-    const uint4 g = __ldg(reinterpret_cast<const uint4*>(dout + r * ld_do + h * D) + sub);
+    const unsigned r = (unsigned)idx / (unsigned)H;              // b * T + t
+    const int h = (int)((unsigned)idx - r * (unsigned)H);
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(o + (size_t)r * ld_o + h * D) + sub);
+    const uint4 g = __ldg(reinterpret_cast<const uint4*>(dout + (size_t)r * ld_do + h * D) + sub);
     const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wg[4] = {g.x, g.y, g.z, g.w};
     float acc = 0.f;
 #pragma unroll
@@ -511,7 +517,7 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
     acc += __shfl_xor_sync(group, acc, 2);
     acc += __shfl_xor_sync(group, acc, 4);
     if (sub == 0) {
-      const int b = (int)(r / T), t = (int)(r - (long long)b * T);
+      const int b = (int)(r / (unsigned)T), t = (int)(r - (unsigned)b * (unsigned)T);
       delta[((size_t)b * H + h) * T + t] = acc;
     }
     float4* z = reinterpret_cast<float4*>(dq_acc + (size_t)r * (H * D) + h * D) + sub * 2;
@@ -527,8 +533,8 @@ attention_dq_round_kernel(const float* __restrict__ acc, __nv_bfloat16* __restri
   const int groups = cols / 8;
   const long long total = rows * groups;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-    const long long r = idx / groups;
-    const int c = (int)(idx - r * groups) * 8;
+    const long long r = (unsigned)idx / (unsigned)groups;
+    const int c = (int)((unsigned)idx - (unsigned)r * (unsigned)groups) * 8;
     const float4 a = *reinterpret_cast<const float4*>(acc + r * cols + c), b = *reinterpret_cast<const float4*>(acc + r * cols + c + 4);
     __nv_bfloat162 h0 = __floats2bfloat162_rn(a.x, a.y), h1 = __floats2bfloat162_rn(a.z, a.w);
     __nv_bfloat162 h2 = __floats2bfloat162_rn(b.x, b.y), h3 = __floats2bfloat162_rn(b.z, b.w);
@@ -574,7 +580,7 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   if ((int64_t)B * H * (T / 128) > 0x7fffffffLL) return fail(TMPI_ERR_INVALID, "attention backward: too many blocks");
   cudaStream_t s = (cudaStream_t)stream;
   const long long rows_heads = (long long)B * T * H;
-  const int dgrid = (int)std::min<long long>((rows_heads * 8 + 255) / 256, 148 * 8);
+  const int dgrid = (int)std::min<long long>((rows_heads * 8 + 255) / 256, attnb::kPassBlocks);
   cudaError_t e = launch_overlapped(attnb::attention_delta_kernel, dgrid, 256, 0, s, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
                                     ld_o, ld_do, delta, dq_acc, B, T, H);
   if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "attention backward launch: %s", cudaGetErrorString(e));
@@ -602,7 +608,7 @@ int tmpi_attention_bwd(const void* q, const void* k, const void* v, int64_t ld_q
   if (dq && e == cudaSuccess) {
     if ((uintptr_t)dq & 15) return fail(TMPI_ERR_INVALID, "attention backward: dq must be 16-byte aligned");
     const long long groups = (long long)rows * (cols / 8);
-    const int cgrid = (int)std::min<long long>((groups + 255) / 256, 148 * 8);
+    const int cgrid = (int)std::min<long long>((groups + 255) / 256, attnb::kPassBlocks);
     e = launch_overlapped(attnb::attention_dq_round_kernel, cgrid, 256, 0, s, dq_acc, (__nv_bfloat16*)dq, ld_dkv, (long long)rows, (int)cols);
   }
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "attention backward launch: %s", cudaGetErrorString(e));
