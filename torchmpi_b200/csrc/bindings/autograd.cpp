@@ -107,6 +107,16 @@ Tensor matmul_nt(const Tensor& a_, const Tensor& b_, const Tensor& bias) {
   return out;
 }
 
+// a b^T + bias + residual, rounded once (linear_add of ops/gemm.py has made the checks)
+Tensor matmul_nt_residual(const Tensor& a_, const Tensor& b_, const Tensor& bias, const Tensor& residual_) {
+  const Tensor a = a_.contiguous(), b = b_.contiguous(), c = bias.defined() ? bias.contiguous() : bias, residual = packed(residual_);
+  Tensor out = at::empty({a.size(0), b.size(0)}, a.options());
+  check(tmpi_gemm_bf16_residual(a.data_ptr(), b.data_ptr(), out.data_ptr(), c.defined() ? c.data_ptr() : nullptr, residual.data_ptr(), (int)a.size(0),
+                                (int)b.size(0), (int)a.size(1), stream()));
+  launched(LINEAR, 1);
+  return out;
+}
+
 Tensor gelu_pass(const Tensor& z) {
   if ((z.numel() * z.element_size()) % 16 || (uintptr_t)z.data_ptr() % 16) return at::gelu(z);
   Tensor y = at::empty_like(z);
@@ -180,15 +190,18 @@ Tensor gelu_gradient(const Tensor& dy, const Tensor& z) {
 }
 
 struct LinearFn : public torch::autograd::Function<LinearFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias_, bool with_gelu) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias_, bool with_gelu,
+                        const c10::optional<Tensor>& residual) {
     const Tensor bias = bias_.has_value() ? *bias_ : Tensor();
     Tensor x2 = x.reshape({-1, x.size(-1)}), y, z;
     if (!(w.dim() == 2 && w.is_cuda() && w.size(1) == x2.size(1)))
       throw std::invalid_argument("matmul_nt expects bf16 CUDA matrices [M, K] and [N, K] with K a multiple of 8");
     if (with_gelu) std::tie(z, y) = matmul_nt_gelu(x2, w, bias);          // the pre-activation is needed by backward
+    else if (residual.has_value()) y = matmul_nt_residual(x2, w, bias, residual->reshape({-1, w.size(0)}));
     else y = matmul_nt(x2, w, bias);
     ctx->save_for_backward({x2, w, z});
     ctx->saved_data["bias"] = bias.defined();
+    ctx->saved_data["residual"] = residual.has_value();
     std::vector<int64_t> shape = x.sizes().vec();
     ctx->saved_data["shape"] = shape;
     shape.back() = w.size(0);
@@ -200,48 +213,70 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     const Tensor& dy = grads[0];
     Tensor dy2 = packed(dy.reshape({-1, dy.size(-1)})), db, dx, dw;
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    const Tensor dres = ctx->saved_data["residual"].toBool() ? dy : Tensor();               // the sum hands its gradient on as it is
     if ((need_x || need_w) && dy2.size(1) % 8 == 0 && pair_enabled()) {
       if (z.defined()) dy2 = gelu_gradient(dy2, z);
       const bool need_b = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
       linear_gradients(dy2, x2.contiguous(), w.contiguous(), need_x ? &dx : nullptr, need_w ? &dw : nullptr, need_b ? &db : nullptr);
       if (need_x) dx = dx.view(ctx->saved_data["shape"].toIntVector());
-      return {dx, dw, db, Tensor()};
+      return {dx, dw, db, Tensor(), dres};
     }
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) std::tie(dy2, db) = bias_grad(dy2, z);
     else if (z.defined()) dy2 = at::gelu_backward(dy2, z);
     if (need_x) dx = matmul_nn(dy2, w).reshape(ctx->saved_data["shape"].toIntVector());
     if (need_w) dw = matmul_tn(dy2, x2);
-    return {dx, dw, db, Tensor()};
+    return {dx, dw, db, Tensor(), dres};
   }
 };
 
 // ---------------------------------------------------------------- layer norm
+Tensor layer_norm_forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, double eps) {
+  const int64_t C = x.size(-1);
+  const Tensor x2 = packed(x.reshape({-1, C})), g = packed(weight), b = packed(bias);
+  const int64_t rows = x2.size(0);
+  Tensor y = at::empty_like(x2), stats = at::empty({2, rows}, x.options().dtype(at::kFloat));      // mean, 1 / std
+  float* mean = stats.data_ptr<float>();
+  check(tmpi_layernorm_fwd(x2.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(), mean, mean + rows, (int)rows, (int)C, (float)eps,
+                           dtype_code(x.scalar_type()), stream()));
+  launched(LAYERNORM, 1);
+  ctx->save_for_backward({x2, g, stats});
+  ctx->saved_data["shape"] = x.sizes().vec();
+  return y.view(x.sizes());
+}
+
+// `add` (may be undefined): a gradient of x from elsewhere, added to dx
+variable_list layer_norm_backward(AutogradContext* ctx, const Tensor& dy, const Tensor& add) {
+  const auto saved = ctx->get_saved_variables();
+  const Tensor &x2 = saved[0], &weight = saved[1];
+  const int64_t rows = x2.size(0), C = x2.size(1);
+  const Tensor dy2 = packed(dy.reshape({rows, C})), add2 = add.defined() ? packed(add.reshape({rows, C})) : add;
+  Tensor dx = at::empty_like(x2), dgamma = at::empty_like(weight), dbeta = at::empty_like(weight);
+  Tensor scratch = at::empty({(int64_t)tmpi_layernorm_scratch_bytes((int)C)}, x2.options().dtype(at::kByte));
+  const float* mean = saved[2].data_ptr<float>();
+  check(tmpi_layernorm_bwd_add(x2.data_ptr(), dy2.data_ptr(), add2.defined() ? add2.data_ptr() : nullptr, weight.data_ptr(), mean, mean + rows,
+                               dx.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), (int)rows, (int)C, dtype_code(x2.scalar_type()),
+                               scratch.data_ptr(), stream()));
+  launched(LAYERNORM, 2);
+  return {dx.view(ctx->saved_data["shape"].toIntVector()), dgamma, dbeta, Tensor()};
+}
+
 struct LayerNormFn : public torch::autograd::Function<LayerNormFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, double eps) {
-    const int64_t C = x.size(-1);
-    const Tensor x2 = packed(x.reshape({-1, C})), g = packed(weight), b = packed(bias);
-    const int64_t rows = x2.size(0);
-    Tensor y = at::empty_like(x2), stats = at::empty({2, rows}, x.options().dtype(at::kFloat));      // mean, 1 / std
-    float* mean = stats.data_ptr<float>();
-    check(tmpi_layernorm_fwd(x2.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(), mean, mean + rows, (int)rows, (int)C, (float)eps,
-                             dtype_code(x.scalar_type()), stream()));
-    launched(LAYERNORM, 1);
-    ctx->save_for_backward({x2, g, stats});
-    ctx->saved_data["shape"] = x.sizes().vec();
-    return y.view(x.sizes());
+    return layer_norm_forward(ctx, x, weight, bias, eps);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) { return layer_norm_backward(ctx, grads[0], Tensor()); }
+};
+
+// The layer norm of x and x itself, for a residual block whose identity takes the second output: the two gradients that reach x are
+// added by the layer norm's kernel.
+struct LayerNormForkFn : public torch::autograd::Function<LayerNormForkFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias, double eps) {
+    ctx->set_materialize_grads(false);
+    return {layer_norm_forward(ctx, x, weight, bias, eps), x};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &x2 = saved[0], &weight = saved[1];
-    const int64_t rows = x2.size(0), C = x2.size(1);
-    const Tensor dy2 = packed(grads[0].reshape({rows, C}));
-    Tensor dx = at::empty_like(x2), dgamma = at::empty_like(weight), dbeta = at::empty_like(weight);
-    Tensor scratch = at::empty({(int64_t)tmpi_layernorm_scratch_bytes((int)C)}, x2.options().dtype(at::kByte));
-    const float* mean = saved[2].data_ptr<float>();
-    check(tmpi_layernorm_bwd(x2.data_ptr(), dy2.data_ptr(), weight.data_ptr(), mean, mean + rows, dx.data_ptr(), dgamma.data_ptr(),
-                             dbeta.data_ptr(), (int)rows, (int)C, dtype_code(x2.scalar_type()), scratch.data_ptr(), stream()));
-    launched(LAYERNORM, 2);
-    return {dx.view(ctx->saved_data["shape"].toIntVector()), dgamma, dbeta, Tensor()};
+    if (!grads[0].defined()) return {grads[1], Tensor(), Tensor(), Tensor()};
+    return layer_norm_backward(ctx, grads[0], grads[1]);
   }
 };
 
@@ -321,8 +356,12 @@ struct XentFn : public torch::autograd::Function<XentFn> {
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, bool gelu) {
-    return LinearFn::apply(x, w, bias, gelu);      // an input without a tensor has to be a nullopt: apply asks every Tensor for its device
+    return LinearFn::apply(x, w, bias, gelu, c10::optional<Tensor>());      // an input without a tensor has to be a nullopt: apply asks every Tensor for its device
   });
+  m.def("linear_add", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, const Tensor& residual) {
+    return LinearFn::apply(x, w, bias, false, c10::optional<Tensor>(residual));
+  });
+  m.def("layer_norm_fork", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormForkFn::apply(x, w, b, eps); });
   m.def("layer_norm", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormFn::apply(x, w, b, eps); });
   m.def("causal_attention", [](const Tensor& qkv, int64_t heads) { return AttentionFn::apply(qkv, heads); });
   m.def("cross_entropy", [](const Tensor& logits, const Tensor& labels, bool unit_grad) {

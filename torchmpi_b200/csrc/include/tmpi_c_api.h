@@ -255,6 +255,9 @@ int tmpi_layernorm_fwd(const void* x, const void* gamma, const void* beta, void*
 int tmpi_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd,
                        void* dx, void* dgamma, void* dbeta, int rows, int channels, int dtype, void* scratch,
                        void* stream);
+// the same with `add` added to dx (null: nothing)
+int tmpi_layernorm_bwd_add(const void* x, const void* dy, const void* add, const void* gamma, const float* mean, const float* rstd, void* dx,
+                           void* dgamma, void* dbeta, int rows, int channels, int dtype, void* scratch, void* stream);
 int tmpi_layernorm_status(void);
 int tmpi_bn_relu_fwd(const void* x, const void* residual, void* y, const float* gamma,
                      const float* beta, float* running_mean, float* running_var,
@@ -358,6 +361,8 @@ int tmpi_gemm_bf16_any(const void* A, const void* B, void* C, void* gelu_out, co
                        void* stream);   // operands as stored, any size
 // Z = A B^T + bias and Y = gelu(Z) of the rounded Z in one kernel; M, N >= 256, N and K multiples of 8
 int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const void* bias, int M, int N, int K, void* stream);
+// C = A B^T (+ bias) + residual, any size; N and K multiples of 8
+int tmpi_gemm_bf16_residual(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K, void* stream);
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                       int64_t lda, int64_t ldb, int64_t ldc, int epilogue, void* stream);

@@ -43,6 +43,7 @@ struct Problem {
   int tiles_m, tiles_n, k_blocks;
   int epilogue;
   const __nv_bfloat16* bias;   // [N] or nullptr
+  const __nv_bfloat16* residual;   // plain CTA-pair GEMM: [M, N], dense, added to the result
   int tma_store;               // epilogue writes through TMA (needs 16-byte aligned rows of C)
   int b_mn;                    // B is given as [K, N] with N contiguous (CTA-pair kernels only)
   int a_mn;                    // A is given as [K, M] with M contiguous (plain CTA-pair GEMM only)

@@ -15,15 +15,15 @@ int gemm_sm_count();
 
 namespace gemm2 {
 
-// p.tiles_m counts 256-row tiles here.  TWO: gelu(C) goes to map_y beside C.
-template <bool TWO>
+// p.tiles_m counts 256-row tiles here.  WITH_GELU: gelu(C) goes to map_y beside C.
+template <int MODE>
 __global__ void __launch_bounds__(GROUP_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_y, const Problem p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char *tiles, *staging;
   Shared* sh;
-  constexpr int NST = TWO ? STAGES - 1 : STAGES;
+  constexpr int NST = MODE == WITH_GELU ? STAGES - 1 : STAGES;
   carve<NST>(smem_raw, &tiles, &sh, &staging);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = sm100::cluster_ctarank();
@@ -45,7 +45,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else if (warp == 1) {
     if (rank == 0 && sm100::elect_one()) mma_issuer<NST>(sh, tiles, p, order);
   } else {
-    epilogue_groups<TWO>(sh, staging, p, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
+    epilogue_groups<MODE>(sh, staging, p, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
   }
   __syncwarp();
   teardown(sh, warp);
@@ -56,8 +56,9 @@ static int max_clusters() {
   static int n = 0;
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-    cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(gemm_bf16_pair_kernel<PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(gemm_bf16_pair_kernel<WITH_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    cudaFuncSetAttribute(gemm_bf16_pair_kernel<RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -65,7 +66,7 @@ static int max_clusters() {
     cfg.gridDim = dim3(2 * (gemm_sm_count() / 2)); cfg.blockDim = dim3(GROUP_THREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES; cfg.attrs = at; cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, (void*)gemm_bf16_pair_kernel<false>, &cfg) == cudaSuccess && c > 0) n = c;
+    if (cudaOccupancyMaxActiveClusters(&c, (void*)gemm_bf16_pair_kernel<PLAIN>, &cfg) == cudaSuccess && c > 0) n = c;
     else { cudaGetLastError(); n = gemm_sm_count() / 2; }
   });
   return n;
@@ -97,9 +98,10 @@ bool gemm_pair_applicable(const void* C, int M, int N, int K, int flags) {
 
 // lda / ldb / ldc: row pitch of A, B, C as stored, in elements (0: dense).  With explicit pitches the
 // extents themselves need not be multiples of 8 (a [T, 50257] matrix held in rows of 50264).
-// gelu_out (optional): a second [M, N] matrix with C's pitch that receives gelu(C).
+// gelu_out (optional): a second [M, N] matrix with C's pitch that receives gelu(C); residual (optional, not both): a dense [M, N]
+// matrix that is added to C.
 int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int epilogue,
-                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out) {
+                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out, const void* residual) {
   CUtensorMap ma, mb, mc, my;
   int st;
   const int clusters = gemm2::max_clusters();
@@ -129,6 +131,7 @@ int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, in
   p.b_mn = b_kn ? 1 : 0;
   p.a_mn = a_km ? 1 : 0;
   p.bias = (const __nv_bfloat16*)bias;
+  p.residual = (const __nv_bfloat16*)residual;
   p.tma_store = 1;
   p.status = status_word;
   const int nclusters = std::min(p.tiles_m * p.tiles_n, clusters);
@@ -140,8 +143,9 @@ int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, in
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(2 * nclusters); cfg.blockDim = dim3(gemm2::GROUP_THREADS);
   cfg.dynamicSmemBytes = gemm2::SMEM_BYTES; cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = 2;
-  cudaError_t e = gelu_out ? cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<true>, ma, mb, mc, my, p)
-                           : cudaLaunchKernelEx(&cfg, gemm2::gemm_bf16_pair_kernel<false>, ma, mb, mc, my, p);
+  const auto kernel = gelu_out ? gemm2::gemm_bf16_pair_kernel<gemm2::WITH_GELU> : residual ? gemm2::gemm_bf16_pair_kernel<gemm2::RESIDUAL>
+                                                                                           : gemm2::gemm_bf16_pair_kernel<gemm2::PLAIN>;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, mc, my, p);
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "pair gemm launch: %s", cudaGetErrorString(e));
 }
 

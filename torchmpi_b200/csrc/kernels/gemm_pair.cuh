@@ -175,13 +175,17 @@ __device__ __forceinline__ void epilogue(Shared* sh, unsigned char* staging, con
 // without that pass's launch and its read of C.  It has staging tiles of its own (the operand ring gives up a stage for
 // them), so a group never waits for the store it has just issued.  8192 x 4096 x 1024: product 83 and pass 36 us before, one
 // kernel of 69 now (82 with one staging tile per group).
+// RESIDUAL: p.residual is added before the rounding.  A thread reads its row's 128 bytes of the next slice while it works on this one.
+// (A pass that adds after the product reads both and writes the sum: 8 us at 8192 x 1024.)
+enum { PLAIN = 0, WITH_GELU = 1, RESIDUAL = 2 };
 constexpr int GROUPS = 2, GROUP_THREADS = 64 + GROUPS * 128;
 
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
-template <bool TWO, typename TileOrder>
+template <int MODE, typename TileOrder>
 __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* staging, const Problem& p, int group, int quarter,
                                                 int lane, TileOrder order, const CUtensorMap* map_c, const CUtensorMap* map2) {
+  constexpr bool TWO = MODE == WITH_GELU;
   constexpr int SLICE = 64, SLICE_BYTES = BM * SLICE * 2;
   static_assert(GROUPS * SLICE_BYTES <= gemm::EPI_STAGING_BYTES && GROUPS * SLICE_BYTES <= STAGE_BYTES, "a staging tile per group and output");
   const int row = quarter * 32 + lane;
@@ -190,8 +194,17 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
   unsigned char* stg0 = staging + group * SLICE_BYTES;
   const bool bias_vec = ((uintptr_t)p.bias & 15) == 0;
   int m_blk, n_blk;
+  uint4 res[8], res_next[8];
+  auto read_residual = [&](uint4 (&v)[8], int col0) {
+    const long long at = (long long)(m_blk * BM + row) * p.N + col0;
+    const bool inside = m_blk * BM + row < p.M;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)          // N is a multiple of 8
+      v[j] = inside && col0 + 8 * j < p.N ? __ldg(reinterpret_cast<const uint4*>(p.residual + at) + j) : make_uint4(0u, 0u, 0u, 0u);
+  };
   for (int it = 0; order(it, &m_blk, &n_blk); ++it) {
     const int acc = it & 1;
+    if (MODE == RESIDUAL) read_residual(res_next, n_blk * bn + group * SLICE);
     const uint32_t ok = sm100::mbar_wait(&sh->acc_full[acc], (it >> 1) & 1, kWaitBudgetNs) && !sh->error;
     uint32_t all_ok;                    // the group meets at named barriers below: it goes on, or leaves, together
     asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, 128, p;\n selp.u32 %0, 1, 0, q;\n}\n"
@@ -208,6 +221,11 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
       uint32_t r[2][32], w[32];
       sm100::tmem_ld_32x32(t_base + c0, r[0]);
       sm100::tmem_ld_32x32(t_base + c0 + 32, r[1]);
+      if (MODE == RESIDUAL) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) res[j] = res_next[j];
+        if (c0 + GROUPS * SLICE < bn) read_residual(res_next, col0 + GROUPS * SLICE);
+      }
       sm100::tmem_ld_wait();
       if (p.epilogue & gemm::EPI_BIAS) {
         if (bias_vec && col0 + SLICE <= p.N) {
@@ -226,6 +244,18 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
 #pragma unroll
           for (int j = 0; j < 64; ++j)
             if (col0 + j < p.N) r[j >> 5][j & 31] = __float_as_uint(__uint_as_float(r[j >> 5][j & 31]) + __bfloat162float(p.bias[col0 + j]));
+        }
+      }
+      if (MODE == RESIDUAL) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t b[4] = {res[j].x, res[j].y, res[j].z, res[j].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint32_t* v = &r[j >> 2][(j & 3) * 8 + 2 * q];
+            v[0] = __float_as_uint(__uint_as_float(v[0]) + __uint_as_float(b[q] << 16));
+            v[1] = __float_as_uint(__uint_as_float(v[1]) + __uint_as_float(b[q] & 0xffff0000u));
+          }
         }
       }
       if (p.epilogue & gemm::EPI_GELU) {

@@ -136,7 +136,7 @@ int gemm_sm_count() {
 
 bool gemm_pair_applicable(const void* C, int M, int N, int K, int flags);
 int launch_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int epilogue,
-                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out);
+                     int* status_word, cudaStream_t stream, int64_t lda, int64_t ldb, int64_t ldc, void* gelu_out, const void* residual);
 
 int* gemm_status_word() {
   static int* dev_ptr = nullptr;
@@ -164,7 +164,7 @@ int tmpi_gemm_bf16(const void* A, const void* B, void* C, const void* bias, int 
   if (k_rows && K % 8) return fail(TMPI_ERR_INVALID, "gemm: K must be a multiple of 8 (16-byte rows for TMA)");
   if ((epilogue & gemm::EPI_BIAS) && !bias) return fail(TMPI_ERR_INVALID, "gemm: bias epilogue without bias");
   if (tunable("gemm_pair") && gemm_pair_applicable(C, M, N, K, epilogue))
-    return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, nullptr);
+    return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, nullptr, nullptr);
   if (epilogue & (gemm::B_IS_KN | gemm::A_IS_KM))
     return fail(TMPI_ERR_UNSUPPORTED, "gemm: operands given as [K, M] / [K, N] need the CTA-pair kernel (M, N >= 256, M, N %% 8 == 0)");
   CUtensorMap ma, mb;
@@ -207,7 +207,7 @@ int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, i
   if ((lda | ldb | ldc) % 8 || lda <= 0 || ldb <= 0 || ldc <= 0)
     return fail(TMPI_ERR_INVALID, "gemm_ex: row pitches must be positive multiples of 8 elements");
   if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return fail(TMPI_ERR_INVALID, "gemm_ex: operands must be 16-byte aligned");
-  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, lda, ldb, ldc, nullptr);
+  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, lda, ldb, ldc, nullptr, nullptr);
 }
 
 // Z = A B^T + bias and Y = gelu(Z) (of the rounded Z), both [M, N], in one kernel: the forward of a linear layer that is
@@ -217,7 +217,7 @@ int tmpi_gemm_bf16_gelu(const void* A, const void* B, void* Z, void* Y, const vo
   if (M < 1 || N < 1 || K < 1 || K % 8) return fail(TMPI_ERR_INVALID, "gemm_gelu: needs a non-empty product with K a multiple of 8");
   if (!tunable("gemm_pair") || !gemm_pair_applicable(Z, M, N, K, 0) || ((uintptr_t)Y & 15))
     return fail(TMPI_ERR_UNSUPPORTED, "gemm_gelu: needs the CTA-pair kernel (M, N >= 256, N %% 8 == 0, 16-byte aligned outputs)");
-  return launch_gemm_pair(A, B, Z, bias, M, N, K, bias ? gemm::EPI_BIAS : 0, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, Y);
+  return launch_gemm_pair(A, B, Z, bias, M, N, K, bias ? gemm::EPI_BIAS : 0, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, Y, nullptr);
 }
 
 // C = op(A) op(B) (+ bias) with operands as they are stored (epilogue: EPI_BIAS, B_IS_KN, A_IS_KM), and gelu(C) in gelu_out when
@@ -231,7 +231,15 @@ int tmpi_gemm_bf16_any(const void* A, const void* B, void* C, void* gelu_out, co
   const bool a_km = (epilogue & gemm::A_IS_KM) != 0, b_kn = (epilogue & gemm::B_IS_KN) != 0;
   if (N % 8 || (a_km ? M : K) % 8 || (!b_kn && K % 8)) return fail(TMPI_ERR_INVALID, "gemm: stored rows must be multiples of 16 bytes (TMA)");
   if ((epilogue & gemm::EPI_BIAS) && !bias) return fail(TMPI_ERR_INVALID, "gemm: bias epilogue without bias");
-  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, gelu_out);
+  return launch_gemm_pair(A, B, C, bias, M, N, K, epilogue, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, gelu_out, nullptr);
+}
+
+// C = A B^T (+ bias) + residual, rounded once; residual and C dense [M, N] and 16-byte aligned, any size, N and K multiples of 8.
+int tmpi_gemm_bf16_residual(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K, void* stream) {
+  if (M < 1 || N < 1 || K < 1) return fail(TMPI_ERR_INVALID, "gemm: empty problem");
+  if (N % 8 || K % 8) return fail(TMPI_ERR_INVALID, "gemm: stored rows must be multiples of 16 bytes (TMA)");
+  if (!residual || ((uintptr_t)residual & 15)) return fail(TMPI_ERR_INVALID, "gemm: the residual must be 16-byte aligned");
+  return launch_gemm_pair(A, B, C, bias, M, N, K, bias ? gemm::EPI_BIAS : 0, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, nullptr, residual);
 }
 
 // Non-zero after a GEMM CTA gave up on a bounded wait (1000 + the point where it happened); clears it.

@@ -75,42 +75,45 @@ __global__ void __launch_bounds__(kLnThreads) ln_fwd_kernel(const T* __restrict_
 // four rows (16 KB at 1024 bf16 columns) per warp are in flight whatever the registers hold; the sums, 64 per lane there,
 // leave no room for a second row in registers, and one row at a time left the memory idle while it was computed.  Measured,
 // 8192 x 1024 bf16, back to back: 19.7 -> 11.4 us (50 MB: 7.7 at the copy rate); 14.3 with nothing in L2, 32768 rows 41.7 (31).
-__host__ __device__ constexpr int ln_ring(int np) { return np <= 6 ? 4 : 2; }      // rows of a warp's ring, 192 KB at most; of the widest rows
-                                                                                   // three took 61.9 us where two take 56.9 (8192 x 2048 bf16)
+// Rows of a warp's ring, 192 KB at most (216 with a third tensor); of the widest rows three took 61.9 us where two take 56.9 (8192 x
+// 2048 bf16).  ADD: a third tensor is added to dx, the gradient that reaches x beside the layer norm (of a residual block's
+// identity), which an elementwise pass would read and write once more.
+__host__ __device__ constexpr int ln_ring(int np, bool add) { return add ? (np <= 4 ? 4 : np <= 6 ? 3 : 2) : np <= 6 ? 4 : 2; }
 // One block per SM, by a floor of shared memory and for the register allocation.  The grid is one block per SM, but under a launch
 // that overlaps the one before it blocks start as SMs become free, and where several of these fit into one (rows of 1 KB and
 // less: 32 to 64 KB each) the first free SMs got several and others none: 32768 x 256, forward and backward, bf16 47.3 us against
 // 30.6 with the floor, fp32 50.9 against 36.5; 8192 x 256 18.6 against 12.6 (16.5 when rows came into registers).
 constexpr int kLnOneBlock = 116 << 10;
-template <typename T, int NP> constexpr int ln_bwd_smem() {
-  const int ring = kLnWarps * ln_ring(NP) * 2 * 32 * NP * 16, sums = kLnWarps * 2 * 32 * NP * 16 / (int)sizeof(T) * 4;
+template <typename T, int NP, bool ADD> constexpr int ln_bwd_smem() {
+  const int ring = kLnWarps * ln_ring(NP, ADD) * (ADD ? 3 : 2) * 32 * NP * 16, sums = kLnWarps * 2 * 32 * NP * 16 / (int)sizeof(T) * 4;
   const int need = ring > sums ? ring : sums;         // the warps' sums take the ring's place
   return need > kLnOneBlock ? need : kLnOneBlock;
 }
 
 // partial[(block * 2 + which) * C + c], which: 0 = dbeta, 1 = dgamma
-template <typename T, int V, int NP>
-__global__ void __launch_bounds__(kLnThreads, 1) ln_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy,
+template <typename T, int V, int NP, bool ADD>
+__global__ void __launch_bounds__(kLnThreads, 1) ln_bwd_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ add,
                                                             const T* __restrict__ gamma, const float* __restrict__ mean,
                                                             const float* __restrict__ rstd, T* __restrict__ dx,
                                                             float* __restrict__ partial, int rows) {
-  constexpr int C = 32 * NP * V, ROW = C * (int)sizeof(T), RING = ln_ring(NP);
+  constexpr int C = 32 * NP * V, ROW = C * (int)sizeof(T), RING = ln_ring(NP, ADD), SET = (ADD ? 3 : 2) * ROW;
   extern __shared__ __align__(128) unsigned char ln_smem[];
   __shared__ uint64_t full[kLnWarps][RING];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char* ring = ln_smem + warp * RING * 2 * ROW;
+  unsigned char* ring = ln_smem + warp * RING * SET;
   if (lane == 0) {
     for (int k = 0; k < RING; ++k) sm100::mbar_init(&full[warp][k], 1);
     sm100::fence_barrier_init();
   }
   __syncwarp();
-  wait_previous(x, dy, gamma, mean, rstd);
+  wait_previous(x, dy, add, gamma, mean, rstd);
   const int first = blockIdx.x * kLnWarps + warp, stride = gridDim.x * kLnWarps;
   auto fetch = [&](long long r, int k) {
     if (r >= rows || lane) return;
-    sm100::mbar_expect_tx(&full[warp][k], 2 * ROW);
-    sm100::bulk_load(ring + k * 2 * ROW, x + (size_t)r * C, ROW, &full[warp][k]);
-    sm100::bulk_load(ring + k * 2 * ROW + ROW, dy + (size_t)r * C, ROW, &full[warp][k]);
+    sm100::mbar_expect_tx(&full[warp][k], SET);
+    sm100::bulk_load(ring + k * SET, x + (size_t)r * C, ROW, &full[warp][k]);
+    sm100::bulk_load(ring + k * SET + ROW, dy + (size_t)r * C, ROW, &full[warp][k]);
+    if (ADD) sm100::bulk_load(ring + k * SET + 2 * ROW, add + (size_t)r * C, ROW, &full[warp][k]);
   };
 #pragma unroll
   for (int k = 0; k < RING; ++k) fetch((long long)first + (long long)k * stride, k);
@@ -133,10 +136,14 @@ __global__ void __launch_bounds__(kLnThreads, 1) ln_bwd_kernel(const T* __restri
       while (sm100::now_ns() - t0 < 200000000ull) { __nanosleep(1000); }   // copies in flight land within microseconds
       break;
     }
-    const T* row = reinterpret_cast<const T*>(ring + k * 2 * ROW);
-    Pack<T, V> xv[NP], yv[NP];
+    const T* row = reinterpret_cast<const T*>(ring + k * SET);
+    Pack<T, V> xv[NP], yv[NP], av[ADD ? NP : 1];
 #pragma unroll
-    for (int p = 0; p < NP; ++p) { xv[p] = ld_pack<T, V>(row + (p * 32 + lane) * V); yv[p] = ld_pack<T, V>(row + C + (p * 32 + lane) * V); }
+    for (int p = 0; p < NP; ++p) {
+      xv[p] = ld_pack<T, V>(row + (p * 32 + lane) * V);
+      yv[p] = ld_pack<T, V>(row + C + (p * 32 + lane) * V);
+      if (ADD) av[p] = ld_pack<T, V>(row + 2 * C + (p * 32 + lane) * V);
+    }
     __syncwarp();                           // the row is in registers
     fetch((long long)r + (long long)RING * stride, k);
     if (++k == RING) { k = 0; phase ^= 1; }
@@ -162,7 +169,9 @@ __global__ void __launch_bounds__(kLnThreads, 1) ln_bwd_kernel(const T* __restri
       for (int e = 0; e < V; ++e) {
         const float d = (float)to_acc<T>(yv[p].v[e]);
         const float xh = ((float)to_acc<T>(xv[p].v[e]) - mu) * rs;
-        o.v[e] = from_acc<T>((typename AccOf<T>::type)(rs * (d * g[p][e] - s1 - xh * s2)));
+        float dxv = rs * (d * g[p][e] - s1 - xh * s2);
+        if (ADD) dxv += (float)to_acc<T>(av[p].v[e]);
+        o.v[e] = from_acc<T>((typename AccOf<T>::type)dxv);
       }
       st_pack<T, V>(dr + (p * 32 + lane) * V, o);
     }
@@ -215,7 +224,7 @@ __global__ void __launch_bounds__(32 * kLnFinGroups) ln_finalize_kernel(const fl
 static int ln_grid(int rows) { return std::max(1, std::min((rows + kLnWarps - 1) / kLnWarps, kLnMaxGrid)); }
 
 template <typename T, int NP>
-static cudaError_t ln_launch(bool fwd, const void* x, const void* a, const void* gamma, const void* beta, void* out, float* mean,
+static cudaError_t ln_launch(bool fwd, const void* x, const void* a, const void* add, const void* gamma, const void* beta, void* out, float* mean,
                              float* rstd, float* partial, void* dgamma, void* dbeta, int rows, float eps, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   constexpr int C = 32 * NP * V;
@@ -223,29 +232,32 @@ static cudaError_t ln_launch(bool fwd, const void* x, const void* a, const void*
   if (fwd)
     return launch_overlapped(ln_fwd_kernel<T, V, NP>, grid, kLnThreads, 0, s, (const T*)x, (const T*)gamma, (const T*)beta, (T*)out, mean,
                              rstd, rows, eps);
-  constexpr int smem = ln_bwd_smem<T, NP>();
-  cudaError_t e = cudaFuncSetAttribute(ln_bwd_kernel<T, V, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  e = launch_overlapped(ln_bwd_kernel<T, V, NP>, grid, kLnThreads, smem, s, (const T*)x, (const T*)a, (const T*)gamma, mean, rstd, (T*)out,
-                        partial, rows);
+  const auto backward = [&](auto kernel, int smem) -> cudaError_t {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    return launch_overlapped(kernel, grid, kLnThreads, smem, s, (const T*)x, (const T*)a, (const T*)add, (const T*)gamma, mean, rstd, (T*)out,
+                             partial, rows);
+  };
+  const cudaError_t e = add ? backward(ln_bwd_kernel<T, V, NP, true>, ln_bwd_smem<T, NP, true>())
+                            : backward(ln_bwd_kernel<T, V, NP, false>, ln_bwd_smem<T, NP, false>());
   if (e != cudaSuccess) return e;
   return launch_overlapped(ln_finalize_kernel<T>, 2 * C / 32, 32 * kLnFinGroups, 0, s, partial, grid, C, (T*)dgamma, (T*)dbeta);
 }
 
 template <typename T>
-static int ln_dispatch(bool fwd, const void* x, const void* a, const void* gamma, const void* beta, void* out, float* mean,
+static int ln_dispatch(bool fwd, const void* x, const void* a, const void* add, const void* gamma, const void* beta, void* out, float* mean,
                        float* rstd, float* partial, void* dgamma, void* dbeta, int rows, int C, float eps, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   if (rows < 1 || C % (32 * V)) return fail(TMPI_ERR_UNSUPPORTED, "layernorm: C=%d must be a multiple of %d", C, 32 * V);
   cudaError_t e;
   switch (C / (32 * V)) {
-    case 1: e = ln_launch<T, 1>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 2: e = ln_launch<T, 2>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 3: e = ln_launch<T, 3>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 4: e = ln_launch<T, 4>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 5: e = ln_launch<T, 5>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 6: e = ln_launch<T, 6>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
-    case 8: e = ln_launch<T, 8>(fwd, x, a, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 1: e = ln_launch<T, 1>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 2: e = ln_launch<T, 2>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 3: e = ln_launch<T, 3>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 4: e = ln_launch<T, 4>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 5: e = ln_launch<T, 5>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 6: e = ln_launch<T, 6>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
+    case 8: e = ln_launch<T, 8>(fwd, x, a, add, gamma, beta, out, mean, rstd, partial, dgamma, dbeta, rows, eps, s); break;
     default: return fail(TMPI_ERR_UNSUPPORTED, "layernorm: C=%d is not covered (%d elements per lane)", C, C / 32);
   }
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "layernorm launch: %s", cudaGetErrorString(e));
@@ -274,9 +286,9 @@ int tmpi_layernorm_fwd(const void* x, const void* gamma, const void* beta, void*
                        int channels, float eps, int dtype, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   switch (dtype) {
-    case TMPI_BF16: return ln_dispatch<__nv_bfloat16>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
-    case TMPI_F16: return ln_dispatch<__half>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
-    case TMPI_F32: return ln_dispatch<float>(true, x, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
+    case TMPI_BF16: return ln_dispatch<__nv_bfloat16>(true, x, nullptr, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
+    case TMPI_F16: return ln_dispatch<__half>(true, x, nullptr, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
+    case TMPI_F32: return ln_dispatch<float>(true, x, nullptr, nullptr, gamma, beta, y, mean, rstd, nullptr, nullptr, nullptr, rows, channels, eps, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "layernorm: dtype %d", dtype);
 }
@@ -284,13 +296,19 @@ int tmpi_layernorm_fwd(const void* x, const void* gamma, const void* beta, void*
 // dx, dgamma, dbeta from dy in one pass over (x, dy); scratch: tmpi_layernorm_scratch_bytes(channels).
 int tmpi_layernorm_bwd(const void* x, const void* dy, const void* gamma, const float* mean, const float* rstd, void* dx,
                        void* dgamma, void* dbeta, int rows, int channels, int dtype, void* scratch, void* stream) {
+  return tmpi_layernorm_bwd_add(x, dy, nullptr, gamma, mean, rstd, dx, dgamma, dbeta, rows, channels, dtype, scratch, stream);
+}
+
+// The same with `add`, of x's shape and type, added to dx (null: nothing).
+int tmpi_layernorm_bwd_add(const void* x, const void* dy, const void* add, const void* gamma, const float* mean, const float* rstd, void* dx,
+                           void* dgamma, void* dbeta, int rows, int channels, int dtype, void* scratch, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   float* m = const_cast<float*>(mean);
   float* r = const_cast<float*>(rstd);
   switch (dtype) {
-    case TMPI_BF16: return ln_dispatch<__nv_bfloat16>(false, x, dy, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
-    case TMPI_F16: return ln_dispatch<__half>(false, x, dy, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
-    case TMPI_F32: return ln_dispatch<float>(false, x, dy, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
+    case TMPI_BF16: return ln_dispatch<__nv_bfloat16>(false, x, dy, add, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
+    case TMPI_F16: return ln_dispatch<__half>(false, x, dy, add, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
+    case TMPI_F32: return ln_dispatch<float>(false, x, dy, add, gamma, nullptr, dx, m, r, (float*)scratch, dgamma, dbeta, rows, channels, 0.f, s);
   }
   return fail(TMPI_ERR_UNSUPPORTED, "layernorm: dtype %d", dtype);
 }

@@ -241,6 +241,17 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     return torch.nn.functional.gelu(y) if gelu else y
 
 
+def linear_add(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], residual: torch.Tensor) -> torch.Tensor:
+    """``residual + linear(x, w, bias)``; where the kernel applies the sum is formed in its epilogue, in fp32, and rounded once."""
+    rows = x.numel() // max(1, x.shape[-1])
+    if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 \
+            and w.shape[0] % 8 == 0 and rows % 8 == 0 and rows > 0 and has_symbol("tmpi_gemm_bf16_residual") \
+            and residual.is_cuda and residual.dtype == torch.bfloat16 and w.dim() == 2 \
+            and residual.shape == x.shape[:-1] + w.shape[:1] and config_get("gemm_pair"):
+        return _native.ext().linear_add(x, w, bias, residual)
+    return residual + linear(x, w, bias)
+
+
 class Linear(torch.nn.Linear):
     """``nn.Linear`` whose matrix products run on the hand-written tcgen05 kernel."""
 

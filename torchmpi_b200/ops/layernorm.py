@@ -35,6 +35,12 @@ def check_status() -> None:
         raise TorchMPIError(3, f"layer norm: a bounded wait ran out (code {st})")
 
 
+def layer_norm_fork(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float):
+    """``(layer_norm(x), x)`` for the two branches of a residual block: in backward the gradients of both outputs are summed by
+    the layer norm's kernel.  ``x`` must be ``supported``."""
+    return _native.ext().layer_norm_fork(x, weight, bias, eps)
+
+
 class LayerNorm(nn.LayerNorm):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if len(self.normalized_shape) == 1 and supported(x, self.weight, self.bias):
