@@ -11,6 +11,13 @@ def _form(bx, sx, bw, sw, sb):
     return bx // 64 | sx << 4 | bw // 64 << 8 | sw << 12 | sb << 16
 
 
+def _rand(*shape):
+    """Rows that are not whole 16-byte units sit in a pitched buffer, whose padding is NaN."""
+    t = torch.full(shape[:-1] + ((shape[-1] + 7) // 8 * 8,), float("nan"), device="cuda", dtype=torch.bfloat16)
+    t[:, :shape[-1]] = torch.randn(*shape, device="cuda")
+    return t[:, :shape[-1]]
+
+
 def _run(dy, x, w, want, form):
     from torchmpi_b200._lib import check, lib, stream_ptr
     rows, out = dy.shape
@@ -21,19 +28,19 @@ def _run(dy, x, w, want, form):
     counters = torch.zeros(max(1, n.value), device="cuda", dtype=torch.int32)
     res = [torch.full(s, float("nan"), device="cuda", dtype=torch.bfloat16) for s in ((rows, inp), (out, inp), (out,))]
     for _ in range(2):                                                                          # the second on the counters of the first
-        check(lib.tmpi_linear_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), *(t.data_ptr() if want >> k & 1 else None for k, t in enumerate(res)),
+        check(lib.tmpi_linear_bwd(dy.data_ptr(), dy.stride(0), x.data_ptr(), w.data_ptr(), *(t.data_ptr() if want >> k & 1 else None for k, t in enumerate(res)),
                                   rows, inp, out, form, ws.data_ptr(), size.value, counters.data_ptr(), n.value, stream_ptr()))
         assert not counters.any()
     return res
 
 
 # one pack, a row more and a row less than a tile, remainders in every dimension, several rounds of units, long K
-@pytest.mark.parametrize("rows,inp,out", [(1, 8, 8), (255, 264, 72), (257, 136, 520), (1000, 768, 1000), (2056, 200, 8), (72, 2056, 264), (4096, 1024, 1536)])
-@pytest.mark.parametrize("form", [0, _form(256, 1, 256, 1, 1), _form(192, 2, 128, 3, 2), _form(128, 3, 192, 8, 4), _form(256, 5, 256, 15, 15)])
+@pytest.mark.parametrize("rows,inp,out", [(1, 8, 8), (255, 264, 72), (257, 136, 520), (1000, 768, 1000), (2056, 200, 8), (72, 2056, 264), (4096, 1024, 1536), (520, 256, 1003)])
+@pytest.mark.parametrize("form", [0, _form(256, 1, 256, 1, 1), _form(192, 2, 128, 3, 2), _form(128, 3, 192, 8, 4), _form(256, 5, 256, 15, 15), 1 << 20 | _form(128, 2, 192, 3, 4)])
 def test_forms_of_the_work_list(rows, inp, out, form):
     from torchmpi_b200.ops import gemm
     torch.manual_seed(rows)
-    dy, x, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((rows, out), (rows, inp), (out, inp)))
+    dy, x, w = (_rand(*s) for s in ((rows, out), (rows, inp), (out, inp)))
     d = dy.double()
     refs = (d @ w.double(), d.t() @ x.double(), d.sum(0))
     # absolute sums of the products: an fp32 sum of K terms is off by K / 16 roundings of a partial sum at most (an MMA adds 16
@@ -55,7 +62,7 @@ def test_refused_sizes_and_scratch():
     from torchmpi_b200._lib import TorchMPIError, check, lib
     size, n = ctypes.c_size_t(0), ctypes.c_int(0)
     t = torch.zeros(8192, 8, device="cuda", dtype=torch.bfloat16)
-    for rows, inp, out, want, form in ((0, 8, 8, 7, 0), (8, 12, 8, 7, 0), (8, 8, 12, 7, 0), (8, 8, 8, 4, 0), (8, 8, 8, 8, 0), (8, 8, 8, 7, 1)):
+    for rows, inp, out, want, form in ((0, 8, 8, 7, 0), (8, 12, 8, 7, 0), (8, 8, 8, 4, 0), (8, 8, 8, 8, 0), (8, 8, 8, 7, 1)):
         with pytest.raises(TorchMPIError):
             check(lib.tmpi_linear_bwd_plan(rows, inp, out, want, form, ctypes.byref(size), ctypes.byref(n)))
     form = _form(128, 1, 128, 4, 1)
@@ -63,7 +70,7 @@ def test_refused_sizes_and_scratch():
     ws, counters, dw = torch.empty(size.value, device="cuda", dtype=torch.uint8), torch.zeros(n.value, device="cuda", dtype=torch.int32), torch.empty_like(t[:8])
     for got in ((size.value - 4, n.value), (size.value, n.value - 1)):
         with pytest.raises(TorchMPIError):
-            check(lib.tmpi_linear_bwd(t.data_ptr(), t.data_ptr(), None, None, dw.data_ptr(), None, 8192, 8, 8, form, ws.data_ptr(), got[0],
+            check(lib.tmpi_linear_bwd(t.data_ptr(), 0, t.data_ptr(), None, None, dw.data_ptr(), None, 8192, 8, 8, form, ws.data_ptr(), got[0],
                                       counters.data_ptr(), got[1], None))
 
 

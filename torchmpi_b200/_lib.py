@@ -212,7 +212,7 @@ _CUDA_PROTOS = {
     "tmpi_gemm_bf16_residual": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "tmpi_gemm_bf16_ex": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i64, _i, _vp]),
     "tmpi_linear_bwd_plan": (_i, [_i, _i, _i, _i, _i, C.POINTER(_sz), _ip]),
-    "tmpi_linear_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp, _i, _vp]),
+    "tmpi_linear_bwd": (_i, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp, _i, _vp]),
     "tmpi_gemm_status": (_i, []),
     "tmpi_conv_max_ctas": (_i, []),
     "tmpi_conv_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _ip, _vp]),

@@ -159,7 +159,7 @@ std::pair<Tensor, Tensor> bias_grad(const Tensor& dy, const Tensor& z) {
   return {dz, db};
 }
 
-// dX = dY W, dW = dY^T X and db = column sums of dY, those that are wanted, in one launch
+// dX = dY W, dW = dY^T X and db = column sums of dY, those that are wanted, in one launch; dY may have a row pitch
 void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor* dx, Tensor* dw, Tensor* db) {
   const int rows = (int)x.size(0), in = (int)x.size(1), out = (int)w.size(0), want = (dx ? 1 : 0) | (dw ? 2 : 0) | (db ? 4 : 0);
   size_t bytes = 0;
@@ -174,7 +174,7 @@ void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor
   if (dx) *dx = at::empty({rows, in}, dy.options());
   if (dw) *dw = at::empty({out, in}, dy.options());
   if (db) *db = at::empty({out}, dy.options());
-  check(tmpi_linear_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), dx ? dx->data_ptr() : nullptr, dw ? dw->data_ptr() : nullptr,
+  check(tmpi_linear_bwd(dy.data_ptr(), rows > 1 ? dy.stride(0) : 0, x.data_ptr(), w.data_ptr(), dx ? dx->data_ptr() : nullptr, dw ? dw->data_ptr() : nullptr,
                         db ? db->data_ptr() : nullptr, rows, in, out, 0, bytes ? ws.data_ptr() : nullptr, bytes,
                         counters ? arrivals.data_ptr() : nullptr, counters, stream()));
   launched(LINEAR, 1);
@@ -226,6 +226,31 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     if (need_x) dx = matmul_nn(dy2, w).reshape(ctx->saved_data["shape"].toIntVector());
     if (need_w) dw = matmul_tn(dy2, x2);
     return {dx, dw, db, Tensor(), dres};
+  }
+};
+
+// The head of ops/gemm.py (wide_head): x w^T for any number of outputs, in a buffer whose row pitch is the next multiple of 8, so that all
+// three products run on the CTA-pair kernels with explicit pitches and no padding copies.
+struct WideHeadFn : public torch::autograd::Function<WideHeadFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
+    const int64_t T = x.size(0), d = x.size(1), V = w.size(0), pitch = (V + 7) / 8 * 8;
+    Tensor buf = at::empty({T, pitch}, x.options());
+    check(tmpi_gemm_bf16_ex(x.data_ptr(), w.data_ptr(), buf.data_ptr(), nullptr, (int)T, (int)V, (int)d, d, d, pitch, 0, stream()));
+    launched(LINEAR, 1);
+    ctx->save_for_backward({x, w});
+    return buf.narrow(1, 0, V);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    Tensor dl = grads[0], dx, dw;
+    if (!(dl.stride(1) == 1 && dl.stride(0) % 8 == 0 && dl.stride(0) >= dl.size(1) && (uintptr_t)dl.data_ptr() % 16 == 0)) {
+      Tensor padded = at::zeros({dl.size(0), (dl.size(1) + 7) / 8 * 8}, dl.options());
+      dl = padded.narrow(1, 0, dl.size(1)).copy_(dl);
+    }
+    const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    if (need_x || need_w) linear_gradients(dl, x, w, need_x ? &dx : nullptr, need_w ? &dw : nullptr, nullptr);
+    return {dx, dw};
   }
 };
 
@@ -361,6 +386,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_add", [](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, const Tensor& residual) {
     return LinearFn::apply(x, w, bias, false, c10::optional<Tensor>(residual));
   });
+  m.def("wide_head", [](const Tensor& x, const Tensor& w) { return WideHeadFn::apply(x, w); });
   m.def("layer_norm_fork", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormForkFn::apply(x, w, b, eps); });
   m.def("layer_norm", [](const Tensor& x, const Tensor& w, const Tensor& b, double eps) { return LayerNormFn::apply(x, w, b, eps); });
   m.def("causal_attention", [](const Tensor& qkv, int64_t heads) { return AttentionFn::apply(qkv, heads); });

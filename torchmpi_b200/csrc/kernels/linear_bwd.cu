@@ -340,6 +340,7 @@ static int max_clusters() {
 
 // ---------------------------------------------------------------- the work list
 struct Choice { int bn, slices; };
+constexpr int LAUNCH_CYCLES = 14000;          // what a second launch costs, the first one's tail and the second one's first loads
 
 static void set_part(Part* q, int what, int rows, int in, int out, Choice c) {
   q->what = what;
@@ -371,8 +372,9 @@ static int candidates(int what, int rows, int in, int out, int clusters, Candida
       Part q;
       set_part(&q, what, rows, in, out, {bn, s});
       const int units = q.tiles_m * q.tiles_n * q.slices;
-      // slices of eight K blocks or more, and of an output that leaves clusters idle or deals out badly
-      if (s == 1 || (q.slices == s && q.per >= 8 && (what == DB || units <= 4 * clusters))) list[n++] = {{bn, s}, unit_cycles(q), units};
+      // slices of eight K blocks or more, and of an output that leaves clusters idle or deals out badly; long slices (the K of a
+      // vocabulary) also of more tiles: 8192 x 50257 x 1024 1484 us whole, 1407 with dX in four slices
+      if (s == 1 || (q.slices == s && q.per >= 8 && (what == DB || units <= (q.per >= 32 ? 8 : 4) * clusters))) list[n++] = {{bn, s}, unit_cycles(q), units};
     }
   return n;
 }
@@ -397,74 +399,102 @@ static long long span(const Candidate* const (&c)[3], int parts, int clusters) {
   return t;
 }
 
-// Tiles and slices of the products in `want`; kept per thread for the sizes last asked for (about 1 - 10 us to find).
-static void choose(int rows, int in, int out, int want, int clusters, Choice (&best)[3]) {
-  struct Kept { int key[5]; Choice c[3]; };
+struct Plan { Choice c[3]; bool apart; };      // apart: dX in a launch of its own, before the one of dW and db
+
+// The best tiles and slices of the products in `want` as one list, and that list's time.
+static long long best_list(int rows, int in, int out, int want, int clusters, Choice* best) {
+  Candidate x[18], w[18], b[6];
+  const int nx = want >> DX & 1 ? candidates(DX, rows, in, out, clusters, x) : 0, nw = want >> DW & 1 ? candidates(DW, rows, in, out, clusters, w) : 0;
+  const int nb = want >> DB & 1 ? candidates(DB, rows, in, out, clusters, b) : 0;
+  long long least = -1;
+  for (int i = 0; i < std::max(1, nx); ++i)
+    for (int j = 0; j < std::max(1, nw); ++j) {
+      const Candidate* c[3] = {};
+      int parts = 0, l = 0;
+      if (nx) c[parts++] = &x[i];
+      if (nw) c[parts++] = &w[j];
+      if (nb) {                                // db's units no longer than dW's, with which they run
+        while (l + 1 < nb && b[l].cycles > (nw ? w[j].cycles : x[i].cycles)) ++l;
+        c[parts++] = &b[l];
+      }
+      const long long t = span(c, parts, clusters);
+      if (least < 0 || t < least) {
+        least = t;
+        if (nx) best[DX] = x[i].c;
+        if (nw) best[DW] = w[j].c;
+        if (nb) best[DB] = b[l].c;
+      }
+    }
+  return least;
+}
+
+// The plan of a call; kept per thread for the sizes last asked for (1 - 10 us to find).
+// One list has to be a twentieth shorter than two, for units of both products that run together share less of dY in L2, which a
+// list of many rounds does not win back.  Single calls on a cool chip, us, two launches and one: 8192 x 1024 x 50257 (a head) 1221, 1315;
+// 4096 x 1024 x 50257 598, 604; 8192 x 2048 x 3072 187, 172; 8192 x 1024 x 4096 140, 121; 2048 x 1024 x 3072 79, 73.
+static Plan choose(int rows, int in, int out, int want, int clusters) {
+  struct Kept { int key[5]; Plan plan; };
   static thread_local Kept kept[32];
   const int key[5] = {rows, in, out, want, clusters};
   Kept& k = kept[((unsigned)rows * 31 + (unsigned)in * 7 + (unsigned)out * 3 + (unsigned)want) / 8 % 32];
   if (!std::equal(key, key + 5, k.key)) {
-    Candidate x[18], w[18], b[6];
-    const int nx = want >> DX & 1 ? candidates(DX, rows, in, out, clusters, x) : 0, nw = want >> DW & 1 ? candidates(DW, rows, in, out, clusters, w) : 0;
-    const int nb = want >> DB & 1 ? candidates(DB, rows, in, out, clusters, b) : 0;
-    long long least = -1;
-    for (int i = 0; i < std::max(1, nx); ++i)
-      for (int j = 0; j < std::max(1, nw); ++j) {
-        const Candidate* c[3] = {};
-        int parts = 0, l = 0;
-        if (nx) c[parts++] = &x[i];
-        if (nw) c[parts++] = &w[j];
-        if (nb) {                              // db's units no longer than dW's, with which they run
-          while (l + 1 < nb && b[l].cycles > (nw ? w[j].cycles : x[i].cycles)) ++l;
-          c[parts++] = &b[l];
-        }
-        const long long t = span(c, parts, clusters);
-        if (least < 0 || t < least) {
-          least = t;
-          k.c[DX] = nx ? x[i].c : Choice{BN, 1};
-          k.c[DW] = nw ? w[j].c : Choice{BN, 1};
-          k.c[DB] = nb ? b[l].c : Choice{BN, 1};
-        }
-      }
+    Plan together{{{BN, 1}, {BN, 1}, {BN, 1}}, false}, apart{{{BN, 1}, {BN, 1}, {BN, 1}}, true};
+    const long long one = best_list(rows, in, out, want, clusters, together.c);
+    k.plan = together;
+    if ((want & 3) == 3) {
+      const long long two = best_list(rows, in, out, 1 << DX, clusters, apart.c) + best_list(rows, in, out, want & ~(1 << DX), clusters, apart.c);
+      if (20 * one > 19 * (two + LAUNCH_CYCLES)) k.plan = apart;
+    }
     std::copy(key, key + 5, k.key);
   }
-  std::copy(k.c, k.c + 3, best);
+  return k.plan;
 }
 
-// form (0: chosen): columns / 64 and slices of dX, of dW, slices of db, four bits each from the lowest.
-static int plan(int rows, int in, int out, int want, int form, int clusters, Problem* p, size_t* ws_floats, int* counters) {
-  Choice c[3];
-  if (form) {
-    for (int what = DX; what <= DW; ++what) {
-      c[what] = {64 * (form >> (8 * what) & 15), form >> (8 * what + 4) & 15};
-      if (c[what].bn < 128 || c[what].bn > 256) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
-    }
-    c[DB] = {BN, form >> 16 & 15};
-    for (const Choice& x : c) if (x.slices < 1) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
-  } else {
-    choose(rows, in, out, want, clusters, c);
-  }
+static int make_problem(int rows, int in, int out, int want, const Choice* c, Problem* p, size_t* ws_floats, int* counters) {
   p->parts = 0;
   for (int what = DX; what <= DB; ++what)
     if (want >> what & 1) set_part(&p->part[p->parts++], what, rows, in, out, c[what]);
   std::sort(p->part, p->part + p->parts, [](const Part& a, const Part& b) { return unit_cycles(a) > unit_cycles(b); });
   long long first = 0, ws = 0;
-  *counters = 0;
+  int arrivals = 0;
   for (int i = 0; i < p->parts; ++i) {
     Part& q = p->part[i];
     const int tiles = q.tiles_m * q.tiles_n;
     q.first = (int)first;
     q.ws = ws;
-    q.arrivals = *counters;
+    q.arrivals = arrivals;
     first += (long long)tiles * q.slices;
     if (q.slices > 1) {
       ws += 2LL * tiles * q.slices * BM * (q.what == DB ? 1 : q.bn);
-      *counters += 2 * tiles;
+      arrivals += 2 * tiles;
     }
   }
   p->total = (int)first;
-  *ws_floats = (size_t)ws;
+  *ws_floats = std::max(*ws_floats, (size_t)ws);       // launches that follow each other share it
+  *counters = std::max(*counters, arrivals);
   return TMPI_OK;
+}
+
+// The launches of a call: one or two.  form (0: chosen): columns / 64 and slices of dX, of dW, slices of db, four bits each from the
+// lowest, then one bit for dX apart.
+static int plan(int rows, int in, int out, int want, int form, int clusters, Problem* p, int* launches, size_t* ws_floats, int* counters) {
+  Plan c;
+  if (form) {
+    for (int what = DX; what <= DW; ++what) {
+      c.c[what] = {64 * (form >> (8 * what) & 15), form >> (8 * what + 4) & 15};
+      if (c.c[what].bn < 128 || c.c[what].bn > 256) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
+    }
+    c.c[DB] = {BN, form >> 16 & 15};
+    for (const Choice& x : c.c) if (x.slices < 1) return fail(TMPI_ERR_INVALID, "linear_bwd: form %#x", form);
+    c.apart = (form >> 20 & 1) && (want & 3) == 3;
+  } else {
+    c = choose(rows, in, out, want, clusters);
+  }
+  *ws_floats = 0;
+  *counters = 0;
+  *launches = 0;
+  if (c.apart) make_problem(rows, in, out, 1 << DX, c.c, &p[(*launches)++], ws_floats, counters);
+  return make_problem(rows, in, out, c.apart ? want & ~(1 << DX) : want, c.c, &p[(*launches)++], ws_floats, counters);
 }
 
 }  // namespace lbwd
@@ -477,35 +507,34 @@ extern "C" {
 // What a call needs: bytes of workspace and arrival counters (unsigned, zero before the first call that uses them; every call leaves
 // them zero).  want: 1 dX, 2 dW, 4 db, of which at least one of the first two.
 int tmpi_linear_bwd_plan(int rows, int in, int out, int want, int form, size_t* workspace_bytes, int* counters) {
-  if (rows < 1 || in < 1 || out < 1 || in % 8 || out % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
+  if (rows < 1 || in < 1 || out < 1 || in % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
   if (!(want & 3) || want & ~7) return fail(TMPI_ERR_INVALID, "linear_bwd: nothing to compute");
-  lbwd::Problem p{};
+  lbwd::Problem p[2] = {};
   size_t ws = 0;
-  const int st = lbwd::plan(rows, in, out, want, form, lbwd::max_clusters(), &p, &ws, counters);
+  int launches;
+  const int st = lbwd::plan(rows, in, out, want, form, lbwd::max_clusters(), p, &launches, &ws, counters);
   *workspace_bytes = ws * sizeof(float);
   return st;
 }
 
-// dx [rows, in] = dy w, dw [out, in] = dy^T x, db [out] = column sums of dy, for dy [rows, out], x [rows, in], w [out, in], all dense
-// bf16 with fp32 accumulation; dx, dw, db may be null.  Calls that share workspace or counters must not overlap.
-int tmpi_linear_bwd(const void* dy, const void* x, const void* w, void* dx, void* dw, void* db, int rows, int in, int out, int form,
+// dx [rows, in] = dy w, dw [out, in] = dy^T x, db [out] = column sums of dy, for dy [rows, out] with rows ld_dy elements apart (0: dense;
+// a multiple of 8, which out need not be), x [rows, in], w [out, in], all bf16 with fp32 accumulation; dx, dw, db may be null.
+// Calls that share workspace or counters must not overlap.
+int tmpi_linear_bwd(const void* dy, int64_t ld_dy, const void* x, const void* w, void* dx, void* dw, void* db, int rows, int in, int out, int form,
                     void* workspace, size_t workspace_bytes, void* counters, int ncounters, void* stream) {
   const int want = (dx ? 1 : 0) | (dw ? 2 : 0) | (db ? 4 : 0);
-  if (rows < 1 || in < 1 || out < 1 || in % 8 || out % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
+  if (!ld_dy) ld_dy = out;
+  if (rows < 1 || in < 1 || out < 1 || in % 8 || ld_dy % 8 || ld_dy < out) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
   if (!(want & 3)) return fail(TMPI_ERR_INVALID, "linear_bwd: nothing to compute");
   const int clusters = lbwd::max_clusters();
-  lbwd::Problem p{};
+  lbwd::Problem p[2] = {};
   size_t ws = 0;
-  int need = 0, st;
-  if ((st = lbwd::plan(rows, in, out, want, form, clusters, &p, &ws, &need))) return st;
+  int launches, need, st;
+  if ((st = lbwd::plan(rows, in, out, want, form, clusters, p, &launches, &ws, &need))) return st;
   if ((ws && (!workspace || ((uintptr_t)workspace & 15))) || workspace_bytes < ws * sizeof(float) || ncounters < need || (need && !counters))
     return fail(TMPI_ERR_INVALID, "linear_bwd: workspace of %zu bytes (16-byte aligned) and %d counters needed", ws * sizeof(float), need);
-  p.ws = (float*)workspace;
-  p.arrivals = (unsigned*)counters;
-  p.db = (__nv_bfloat16*)db;
-  p.status = gemm_status_word();
   CUtensorMap mdy, mx, mw, mdx, mdw;
-  if ((st = make_tmap_bf16(&mdy, dy, (uint64_t)rows, (uint64_t)out, (uint64_t)out, 64))) return st;
+  if ((st = make_tmap_bf16(&mdy, dy, (uint64_t)rows, (uint64_t)out, (uint64_t)ld_dy, 64))) return st;
   mx = mw = mdx = mdw = mdy;
   if (dw && (st = make_tmap_bf16(&mx, x, (uint64_t)rows, (uint64_t)in, (uint64_t)in, 64))) return st;
   if (dx && (st = make_tmap_bf16(&mw, w, (uint64_t)out, (uint64_t)in, (uint64_t)in, 64))) return st;
@@ -517,10 +546,18 @@ int tmpi_linear_bwd(const void* dy, const void* x, const void* w, void* dx, void
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see pdl.cuh
   at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(2 * std::min(p.total, clusters)); cfg.blockDim = dim3(gemm2::GROUP_THREADS);
+  cfg.blockDim = dim3(gemm2::GROUP_THREADS);
   cfg.dynamicSmemBytes = lbwd::BWD_SMEM_BYTES; cfg.stream = (cudaStream_t)stream; cfg.attrs = at; cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, lbwd::linear_bwd_kernel, mdy, mx, mw, mdx, mdw, p);
-  return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "linear_bwd launch: %s", cudaGetErrorString(e));
+  for (int i = 0; i < launches; ++i) {
+    p[i].ws = (float*)workspace;
+    p[i].arrivals = (unsigned*)counters;
+    p[i].db = (__nv_bfloat16*)db;
+    p[i].status = gemm_status_word();
+    cfg.gridDim = dim3(2 * std::min(p[i].total, clusters));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, lbwd::linear_bwd_kernel, mdy, mx, mw, mdx, mdw, p[i]);
+    if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "linear_bwd launch: %s", cudaGetErrorString(e));
+  }
+  return TMPI_OK;
 }
 
 }  // extern "C"
