@@ -10,7 +10,7 @@ import importlib.util
 
 from . import _lib, build  # noqa: F401  (_lib loads the native library first)
 
-LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD = range(5)      # counters of ``launches``; attention counts calls
+LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD, BATCHNORM, CONV, STEM = range(8)      # counters of ``launches``; attention counts calls
 _ext = None
 
 
@@ -31,3 +31,12 @@ def launches(what: int) -> int:
     """Kernels (for attention: calls, both ways or backward alone) that the C++ functions of one kind have launched in this
     process; 0 before the first use."""
     return _ext.launches(what) if _ext is not None else 0
+
+
+def takes(*params) -> bool:
+    """Whether the C++ functions take a layer with these parameters: they return every gradient to autograd, so not where a flat
+    bucket wants it added in place (``parallel.flat_buckets.direct_grad``)."""
+    for p in params:
+        if getattr(p, "_tmpi_grad_sink", None) is not None:
+            return False
+    return True

@@ -22,7 +22,7 @@ using at::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-enum { LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD, KINDS };
+enum { LINEAR, LAYERNORM, ATTENTION, XENT, ATTENTION_BACKWARD, BATCHNORM, CONV, STEM, KINDS };
 std::atomic<long long> g_launches[KINDS];      // attention: calls, and those of the backward alone
 enum { EPI_BIAS = 1 };
 
@@ -377,6 +377,210 @@ struct XentFn : public torch::autograd::Function<XentFn> {
   }
 };
 
+// ---------------------------------------------------------------- batch norm and convolution of channels-last activations
+// Sums the gradients that several consumers send into one activation inside their kernels: every consumer but the last parks its
+// gradient here and returns none to autograd, the last one's kernel adds the parked sum.  A residual's gradient may be parked unwritten,
+// as the incoming gradient and the ReLU's mask bits.  (GradFork of parallel/flat_buckets.py, for the functions below.)
+struct Fork : torch::CustomClassHolder {
+  int64_t consumers, seen = 0;
+  Tensor parked, bits;
+  explicit Fork(int64_t n) : consumers(n) {}
+  bool parks_first() const { return seen == 0 && consumers > 1; }
+  // make(add, bits): this consumer's gradient plus `add` (where its bit is set, if there are bits), when that is defined
+  template <typename F> Tensor offer(F make) {
+    ++seen;
+    Tensor g = make(parked, bits);
+    if (seen < consumers) {
+      parked = g;
+      bits = Tensor();
+      return Tensor();
+    }
+    seen = 0;
+    parked = bits = Tensor();
+    return g;
+  }
+  void park_masked(const Tensor& grad, const Tensor& mask) {
+    ++seen;
+    parked = grad;
+    bits = mask;
+  }
+};
+using ForkPtr = c10::intrusive_ptr<Fork>;
+
+c10::IValue keep_fork(const ForkPtr& f) { return f ? c10::IValue::make_capsule(f) : c10::IValue(); }
+ForkPtr kept_fork(AutogradContext* ctx, const char* name) {
+  const c10::IValue& v = ctx->saved_data[name];
+  return v.isCapsule() ? c10::static_intrusive_pointer_cast<Fork>(v.toCapsule()) : ForkPtr();
+}
+
+Tensor channels_last(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
+Tensor empty_channels_last(at::IntArrayRef sizes, const Tensor& like) {
+  return at::empty(sizes, like.options(), at::MemoryFormat::ChannelsLast);
+}
+const void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+float* floats(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
+// the gradient where its mask bit is set
+Tensor masked_tensor(const Tensor& grad, const Tensor& bits) {
+  const int64_t per = grad.numel() / bits.numel(), N = grad.size(0), C = grad.size(1), H = grad.size(2), W = grad.size(3);      // elements of a byte
+  const Tensor on = at::bitwise_and(at::bitwise_right_shift(bits.unsqueeze(1), at::arange(per, bits.options())), 1);
+  return at::where(on.view({N, H, W, C}).permute({0, 3, 1, 2}).to(at::kBool), grad, at::zeros({}, grad.options()));
+}
+
+struct BnArgs { double eps, momentum; bool relu, training, keeps; int partial_rows; Tensor scratch; ForkPtr res_fork; };
+
+struct BnFn : public torch::autograd::Function<BnFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const c10::optional<Tensor>& residual_, const Tensor& gamma, const Tensor& beta,
+                        const c10::optional<Tensor>& running_mean, const c10::optional<Tensor>& running_var, const BnArgs& a) {
+    const Tensor x = channels_last(x_), residual = residual_.has_value() ? channels_last(*residual_) : Tensor();
+    const int64_t C = x.size(1), rows = x.size(0) * x.size(2) * x.size(3);
+    Tensor y = empty_channels_last(x.sizes(), x), mean, invstd, bits;
+    if (a.training) {
+      mean = at::empty({2, C}, gamma.options());                       // and 1 / std behind it
+      invstd = mean[1];
+    } else {
+      mean = running_mean->to(at::kFloat);
+      invstd = at::rsqrt(running_var->to(at::kFloat) + a.eps);
+    }
+    // a ReLU layer with a residual keeps one mask bit per element for its backward (a sixteenth of y)
+    if (a.relu && residual.defined() && a.keeps) bits = at::empty({rows * C / (16 / x.element_size())}, x.options().dtype(at::kByte));
+    float *m = mean.data_ptr<float>(), *v = invstd.data_ptr<float>();
+    const int type = dtype_code(x.scalar_type());
+    float *rm = a.training && running_mean.has_value() ? floats(*running_mean) : nullptr, *rv = a.training && running_var.has_value() ? floats(*running_var) : nullptr;
+    if (a.training && a.partial_rows > 0)
+      check(tmpi_bn_relu_fwd_partials(x.data_ptr(), ptr(residual), y.data_ptr(), floats(gamma), floats(beta), rm, rv, m, v, rows, (int)C, (float)a.eps,
+                                      (float)a.momentum, a.relu, type, (void*)ptr(bits), a.scratch.data_ptr(), a.partial_rows, stream()));
+    else
+      check(tmpi_bn_relu_fwd(x.data_ptr(), ptr(residual), y.data_ptr(), floats(gamma), floats(beta), rm, rv, m, v, rows, (int)C, (float)a.eps,
+                             (float)a.momentum, a.relu, a.training, type, (void*)ptr(bits), a.scratch.data_ptr(), stream()));
+    launched(BATCHNORM, !a.training ? 1 : a.partial_rows > 0 ? 2 : 3);
+    // a ReLU layer without a residual rebuilds its mask from x in backward; neither kind reads y again
+    const bool keep_y = a.relu && residual.defined() && !bits.defined();
+    ctx->save_for_backward({x, keep_y ? y : Tensor(), gamma, beta, mean, a.training ? Tensor() : invstd, bits});
+    ctx->saved_data["relu"] = a.relu;
+    ctx->saved_data["residual"] = residual.defined();
+    ctx->saved_data["fork"] = keep_fork(a.res_fork);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &y = saved[1], &gamma = saved[2], &beta = saved[3], &mean = saved[4], &invstd = saved[5], &bits = saved[6];
+    const Tensor dy = channels_last(grads[0]);
+    const int64_t C = x.size(1), rows = x.size(0) * x.size(2) * x.size(3);
+    const bool has_res = ctx->saved_data["residual"].toBool();
+    const ForkPtr fork = kept_fork(ctx, "fork");
+    // the first of several consumers of the residual parks its gradient for the last one's kernel: as dy and the mask bits
+    const bool masked = has_res && bits.defined() && fork && fork->parks_first();
+    Tensor dx = empty_channels_last(x.sizes(), x), dres = has_res && !masked ? empty_channels_last(x.sizes(), x) : Tensor();
+    Tensor dgamma = at::empty({C}, gamma.options()), dbeta = at::empty({C}, gamma.options());
+    const Tensor scratch = at::empty({(int64_t)tmpi_bn_scratch_bytes((int)C)}, x.options().dtype(at::kByte));
+    check(tmpi_bn_relu_bwd_acc(x.data_ptr(), ptr(y), dy.data_ptr(), dx.data_ptr(), (void*)ptr(dres), floats(gamma), floats(beta), floats(mean),
+                               invstd.defined() ? floats(invstd) : floats(mean) + C, floats(dgamma), floats(dbeta), rows, (int)C,
+                               ctx->saved_data["relu"].toBool(), dtype_code(x.scalar_type()), ptr(bits), scratch.data_ptr(), nullptr, nullptr, stream()));
+    launched(BATCHNORM, 3);
+    if (masked) fork->park_masked(dy, bits);
+    else if (dres.defined() && fork)
+      dres = fork->offer([&](const Tensor& add, const Tensor& mask) { return add.defined() ? dres.add_(mask.defined() ? masked_tensor(add, mask) : add) : dres; });
+    return {dx, dres, dgamma, dbeta, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+struct ConvArgs { int stride, pad; float* stats; int* rows; ForkPtr fork; };
+
+struct ConvFn : public torch::autograd::Function<ConvFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_, const ConvArgs& a) {
+    const Tensor x = channels_last(x_), w = channels_last(w_);
+    const int64_t N = x.size(0), Cin = x.size(1), H = x.size(2), W = x.size(3), Cout = w.size(0), R = w.size(2), S = w.size(3);
+    Tensor y = empty_channels_last({N, Cout, (H + 2 * a.pad - R) / a.stride + 1, (W + 2 * a.pad - S) / a.stride + 1}, x);
+    int rows = 0;
+    check(tmpi_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int)N, (int)H, (int)W, (int)Cin, (int)Cout, (int)R, (int)S, a.stride, a.pad, a.stats,
+                        &rows, stream()));
+    launched(CONV, 1);
+    if (a.rows) *a.rows = rows;
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["stride"] = (int64_t)a.stride;
+    ctx->saved_data["pad"] = (int64_t)a.pad;
+    ctx->saved_data["fork"] = keep_fork(a.fork);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor dy = channels_last(grads[0]);
+    const int N = (int)x.size(0), Cin = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), Cout = (int)w.size(0), R = (int)w.size(2), S = (int)w.size(3);
+    const int stride = (int)ctx->saved_data["stride"].toInt(), pad = (int)ctx->saved_data["pad"].toInt();
+    Tensor dx, dw;
+    if (ctx->needs_input_grad(0)) {
+      auto make = [&](Tensor add, Tensor bits) {
+        if (bits.defined() && !(stride == 1 && add.sizes() == x.sizes() && add.scalar_type() == x.scalar_type() && (uintptr_t)add.data_ptr() % 16 == 0)) {
+          add = masked_tensor(add, bits);
+          bits = Tensor();
+        }
+        if (stride == 1) {
+          if (add.defined()) add = channels_last(add);
+          Tensor g = empty_channels_last(x.sizes(), dy);
+          check(tmpi_conv_dgrad_masked(dy.data_ptr(), w.data_ptr(), g.data_ptr(), ptr(add), ptr(bits), N, H, W, Cin, Cout, R, S, 1, pad, stream()));
+          launched(CONV, 1);
+          return g;
+        }
+        Tensor g = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1, {true, false, false}));
+        return add.defined() ? g.add_(add) : g;                     // strided input gradients stay on the library
+      };
+      const ForkPtr fork = kept_fork(ctx, "fork");
+      dx = fork ? fork->offer(make) : make(Tensor(), Tensor());
+    }
+    if (ctx->needs_input_grad(1)) {
+      const size_t need = tmpi_conv_wgrad_workspace_bytes(N, H, W, Cin, Cout, R, S, stride, pad);
+      const Tensor ws = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
+      dw = channels_last(at::empty(w.sizes(), x.options()));
+      check(tmpi_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, H, W, Cin, Cout, R, S, stride, pad, ws.data_ptr(), need, 0, stream()));
+      launched(CONV, 2);
+    }
+    return {dx, dw, Tensor()};
+  }
+};
+
+Tensor bn_relu(const Tensor& x, const c10::optional<Tensor>& residual, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& running_mean,
+               const c10::optional<Tensor>& running_var, double eps, double momentum, bool relu, bool training, const ForkPtr& res_fork, int partial_rows,
+               Tensor scratch) {
+  auto wants = [](const Tensor& t) { return t.requires_grad(); };
+  const bool keeps = at::GradMode::is_enabled() && (wants(x) || wants(gamma) || wants(beta) || (residual.has_value() && wants(*residual)));
+  if (!scratch.defined()) scratch = at::empty({(int64_t)tmpi_bn_scratch_bytes((int)x.size(1))}, x.options().dtype(at::kByte));
+  if (!training && !(running_mean.has_value() && running_var.has_value()))
+    throw std::invalid_argument("batch norm: evaluation needs running statistics");
+  return BnFn::apply(x, residual, gamma, beta, running_mean, running_var,
+                     BnArgs{eps, momentum, relu, training, keeps, partial_rows, scratch, res_fork});
+}
+
+// ---------------------------------------------------------------- the ResNet stem's convolution
+struct StemFn : public torch::autograd::Function<StemFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
+    const int64_t N = x.size(0), H = x.size(2), W = x.size(3);
+    Tensor y = empty_channels_last({N, w.size(0), (H - 1) / 2 + 1, (W - 1) / 2 + 1}, x);
+    check(tmpi_stem_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int)N, (int)H, (int)W, (int)w.size(0), w.strides().data(), stream()));
+    launched(STEM, 1);
+    ctx->save_for_backward({x});                                 // nothing but the image is kept
+    ctx->saved_data["shape"] = w.sizes().vec();
+    ctx->saved_data["strides"] = w.strides().vec();
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor& x = saved[0];
+    Tensor dy = channels_last(grads[0]);
+    if ((uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);          // a view into a larger buffer
+    const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector(), strides = ctx->saved_data["strides"].toIntVector();
+    Tensor dw = at::empty_strided(shape, strides, x.options());
+    // partial sums of the CTAs (24 MB), from the allocator: calls on other streams, threads and in graphs have their own
+    const size_t need = tmpi_stem_conv_wgrad_workspace_bytes();
+    const Tensor ws = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
+    check(tmpi_stem_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), (int)x.size(0), (int)x.size(2), (int)x.size(3), (int)shape[0], strides.data(),
+                               ws.data_ptr(), need, stream()));
+    launched(STEM, 2);
+    return {Tensor(), dw};
+  }
+};
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -392,6 +596,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("causal_attention", [](const Tensor& qkv, int64_t heads) { return AttentionFn::apply(qkv, heads); });
   m.def("cross_entropy", [](const Tensor& logits, const Tensor& labels, bool unit_grad) {
     return XentFn::apply(logits, labels, unit_grad);
+  });
+  pybind11::class_<Fork, ForkPtr>(m, "Fork").def(pybind11::init([](int64_t n) { return c10::make_intrusive<Fork>(n); })).def_readwrite("consumers", &Fork::consumers);
+  m.def("bn_relu", [](const Tensor& x, const c10::optional<Tensor>& residual, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& rm,
+                      const c10::optional<Tensor>& rv, double eps, double momentum, bool relu, bool training, const ForkPtr& res_fork) {
+    return bn_relu(x, residual, gamma, beta, rm, rv, eps, momentum, relu, training, res_fork, 0, Tensor());
+  });
+  m.def("stem_conv", [](const Tensor& x, const Tensor& w) { return StemFn::apply(x, w); });
+  m.def("conv2d", [](const Tensor& x, const Tensor& w, int stride, int pad, const ForkPtr& fork) {
+    return ConvFn::apply(x, w, ConvArgs{stride, pad, nullptr, nullptr, fork});
+  });
+  // bn(conv(x), residual) in training: the convolution's epilogue leaves the partial sums of its output's statistics
+  m.def("conv_bn", [](const Tensor& x, const Tensor& w, int stride, int pad, const c10::optional<Tensor>& residual, const Tensor& gamma, const Tensor& beta,
+                      const c10::optional<Tensor>& rm, const c10::optional<Tensor>& rv, double eps, double momentum, bool relu, const ForkPtr& fork,
+                      const ForkPtr& res_fork) {
+    const Tensor scratch = at::empty({(int64_t)tmpi_bn_scratch_bytes((int)w.size(0))}, x.options().dtype(at::kByte));
+    int rows = 0;
+    const Tensor y = ConvFn::apply(x, w, ConvArgs{stride, pad, (float*)scratch.data_ptr(), &rows, fork});
+    return bn_relu(y, residual, gamma, beta, rm, rv, eps, momentum, relu, true, res_fork, rows, scratch);
   });
   m.def("cross_entropy_scratch", xent_scratch);
   m.def("launches", [](int what) { return g_launches[what].load(std::memory_order_relaxed); });

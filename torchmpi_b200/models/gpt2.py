@@ -58,15 +58,6 @@ def _layer_norm(c: "GPT2Config") -> nn.LayerNorm:
     return nn.LayerNorm(c.n_embd)
 
 
-def _bare(m: nn.Module) -> bool:
-    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__)
-
-
-def _global_hooks() -> bool:
-    from torch.nn.modules import module as M
-    return bool(M._global_forward_hooks or M._global_forward_pre_hooks or M._global_backward_hooks or M._global_backward_pre_hooks)
-
-
 class Block(nn.Module):
     def __init__(self, c: GPT2Config):
         super().__init__()
@@ -89,11 +80,12 @@ class Block(nn.Module):
         if not (self.own_attention and x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3):
             return False
         from ..ops import layernorm
+        from ..ops.conv import bare
         mods = self._modules
-        if not all(type(mods[n]) is layernorm.LayerNorm and _bare(mods[n]) and mods[n].normalized_shape == x.shape[-1:]
+        if not all(type(mods[n]) is layernorm.LayerNorm and bare(mods[n]) and mods[n].normalized_shape == x.shape[-1:]
                    and layernorm.supported(x, mods[n].weight, mods[n].bias) for n in ("ln1", "ln2")):
             return False
-        return all(type(mods[n]) is _Linear and mods[n].tc and not mods[n].gelu and _bare(mods[n]) for n in ("proj", "out")) and not _global_hooks()
+        return all(type(mods[n]) is _Linear and mods[n].tc and not mods[n].gelu and bare(mods[n]) for n in ("proj", "out"))
 
     def forward(self, x):
         if self._sums_in_kernels(x):

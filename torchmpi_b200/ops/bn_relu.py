@@ -14,10 +14,10 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .. import config
+from .. import _native, config
 from .._lib import lib, check, dtype_code, has_symbol, stream_ptr
 
-launch_count = 0
+_launches = 0
 _scratch = {}
 
 
@@ -32,13 +32,22 @@ def _scratch_for(dev: torch.device, C: int, stream: Optional[int] = None) -> tor
     return buf
 
 
+def __getattr__(name: str):
+    if name == "launch_count":               # kernels launched by this module, the C++ functions' included
+        return _launches + _native.launches(_native.BATCHNORM)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 def supported(x: torch.Tensor) -> bool:
     if not (x.is_cuda and x.dim() == 4 and has_symbol("tmpi_bn_relu_fwd")):
         return False
     if x.dtype not in (torch.bfloat16, torch.float16, torch.float32):
         return False
-    V = 16 // x.element_size()
-    C = x.shape[1]
+    return width_supported(x.shape[1], x.element_size())
+
+
+def width_supported(C: int, element_size: int) -> bool:
+    V = 16 // element_size
     return C % V == 0 and 256 % (C // V) == 0
 
 
@@ -50,7 +59,7 @@ class _BnReluFn(torch.autograd.Function):
         rows of partial sums in this stream's scratch buffer, so the statistics pass is skipped.  ``params``: the
         (weight, bias) Parameters, whose gradients are added in place when a flat bucket owns their buffers;
         ``res_fork``: a ``GradFork`` shared by the consumers of ``residual``."""
-        global launch_count
+        global _launches
         x = x.contiguous(memory_format=torch.channels_last)
         if residual is not None:
             residual = residual.contiguous(memory_format=torch.channels_last)
@@ -76,7 +85,7 @@ class _BnReluFn(torch.autograd.Function):
                 mean.data_ptr(), invstd.data_ptr(), rows, C, eps, momentum, int(relu),
                 dtype_code(x.dtype), bits.data_ptr() if bits is not None else None,
                 _scratch_for(x.device, C).data_ptr(), int(partial_rows), stream_ptr()))
-            launch_count += 2
+            _launches += 2
         else:
             check(lib.tmpi_bn_relu_fwd(
                 x.data_ptr(), residual.data_ptr() if residual is not None else None, y.data_ptr(),
@@ -86,7 +95,7 @@ class _BnReluFn(torch.autograd.Function):
                 mean.data_ptr(), invstd.data_ptr(), rows, C, eps, momentum, int(relu), int(training),
                 dtype_code(x.dtype), bits.data_ptr() if bits is not None else None,
                 _scratch_for(x.device, C).data_ptr(), stream_ptr()))
-            launch_count += 3 if training else 1
+            _launches += 3 if training else 1
         # a ReLU layer without a residual rebuilds its mask from x in backward; neither kind reads y again
         ctx.mask_from_x = relu and residual is None
         keep_y = relu and not ctx.mask_from_x and bits is None
@@ -97,7 +106,7 @@ class _BnReluFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        global launch_count
+        global _launches
         x, y, gamma, beta, mean, invstd, bits = ctx.saved_tensors
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
@@ -120,7 +129,7 @@ class _BnReluFn(torch.autograd.Function):
             N * H * W, C, int(ctx.relu), dtype_code(x.dtype), bits.data_ptr() if bits is not None else None,
             _scratch_for(x.device, C).data_ptr(), acc_g.data_ptr() if acc_g is not None else None,
             acc_b.data_ptr() if acc_b is not None else None, stream_ptr()))
-        launch_count += 3
+        _launches += 3
         if acc_g is not None:                  # the parameter gradients were added in place by the finalize kernel
             grad_written(ctx.params[0])
             grad_written(ctx.params[1])
@@ -142,7 +151,7 @@ class _BnReluPoolFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, gamma, beta, running_mean, running_var, eps, momentum, training, grad_mode):
-        global launch_count
+        global _launches
         x = x.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         OH, OW = (H - 1) // 2 + 1, (W - 1) // 2 + 1
@@ -163,13 +172,13 @@ class _BnReluPoolFn(torch.autograd.Function):
             running_var.data_ptr() if (training and running_var is not None) else None,
             mean.data_ptr(), _invstd_ptr(mean, invstd), N, H, W, C, eps, momentum, int(training), dtype_code(x.dtype),
             _scratch_for(x.device, C, stream).data_ptr(), stream))
-        launch_count += 3 if training else 1
+        _launches += 3 if training else 1
         ctx.save_for_backward(x, xmax, idx, gamma, beta, mean, invstd)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        global launch_count
+        global _launches
         x, xmax, idx, gamma, beta, mean, invstd = ctx.saved_tensors
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
@@ -184,7 +193,7 @@ class _BnReluPoolFn(torch.autograd.Function):
                 x.data_ptr(), xmax.data_ptr() if xmax is not None else None, dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
                 mean.data_ptr(), _invstd_ptr(mean, invstd), dgamma.data_ptr(), dbeta.data_ptr(), N, H, W, C, dtype_code(x.dtype),
                 _scratch_for(x.device, C, stream).data_ptr(), stream))
-            launch_count += 3
+            _launches += 3
         else:
             # in two stages: route the gradient through the pool, then the batch-norm backward with the ReLU mask
             # rebuilt from x (the rectified activation itself was never stored)
@@ -196,7 +205,7 @@ class _BnReluPoolFn(torch.autograd.Function):
                 x.data_ptr(), None, da.data_ptr(), dx.data_ptr(), None, gamma.data_ptr(), beta.data_ptr(),
                 mean.data_ptr(), _invstd_ptr(mean, invstd), dgamma.data_ptr(), dbeta.data_ptr(), N * H * W, C, 1,
                 dtype_code(x.dtype), None, _scratch_for(x.device, C, stream).data_ptr(), stream))
-            launch_count += 4
+            _launches += 4
         return dx, dgamma, dbeta, None, None, None, None, None, None
 
 
@@ -225,6 +234,10 @@ class FusedBatchNormReLU(nn.BatchNorm2d):
 
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, partial_rows: int = 0, res_fork=None) -> torch.Tensor:
         if supported(x) and self.weight.dtype == torch.float32:
+            w, b = self.weight, self.bias
+            if partial_rows == 0 and _native.takes(w, b) and (res_fork is None or isinstance(res_fork, _native.ext().Fork)):
+                return _native.ext().bn_relu(x, residual, w, b, self.running_mean, self.running_var, self.eps, self.momentum, self.relu,
+                                             self.training, res_fork)
             # num_batches_tracked is only needed for momentum=None (cumulative average), not supported here
             return _BnReluFn.apply(x, residual, self.weight, self.bias, self.running_mean, self.running_var,
                                    self.eps, self.momentum, self.relu, self.training, partial_rows,

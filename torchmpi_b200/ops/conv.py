@@ -19,10 +19,17 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _native
 from .._lib import lib, check, has_symbol, stream_ptr, TorchMPIError
 
-launch_count = 0
+_launches = 0
 _ws = {}
+
+
+def __getattr__(name: str):
+    if name == "launch_count":               # kernels launched by this module, the C++ functions' included
+        return _launches + _native.launches(_native.CONV)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _workspace(dev: torch.device, need: int) -> torch.Tensor:
@@ -53,7 +60,7 @@ def _out_hw(H, W, R, S, stride, pad):
 def conv_forward(x, w, stride, pad, stats: Optional[torch.Tensor] = None):
     """Raw forward launch: returns ``(y, stat_rows)``; ``stats`` (fp32, at least ``max_ctas * 2 * Cout``) receives
     the partial sums when given."""
-    global launch_count
+    global _launches
     N, Cin, H, W = x.shape
     Cout, _, R, S = w.shape
     Ho, Wo = _out_hw(H, W, R, S, stride, pad)
@@ -61,27 +68,27 @@ def conv_forward(x, w, stride, pad, stats: Optional[torch.Tensor] = None):
     rows = C.c_int(0)
     check(lib.tmpi_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, Cin, Cout, R, S, stride, pad,
                             stats.data_ptr() if stats is not None else None, C.byref(rows), stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return y, rows.value
 
 
 def conv_dgrad(dy, w, x_shape, stride, pad, add: Optional[torch.Tensor] = None, add_bits: Optional[torch.Tensor] = None):
     """``add`` is added to the gradient; with ``add_bits`` (one bit per element, eight channels to a byte) where its bit is set."""
-    global launch_count
+    global _launches
     N, Cin, H, W = x_shape
     Cout, _, R, S = w.shape
     dx = torch.empty(x_shape, dtype=dy.dtype, device=dy.device, memory_format=torch.channels_last)
     check(lib.tmpi_conv_dgrad_masked(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), add.data_ptr() if add is not None else None,
                                      add_bits.data_ptr() if add_bits is not None else None,
                                      N, H, W, Cin, Cout, R, S, stride, pad, stream_ptr()))
-    launch_count += 1
+    _launches += 1
     return dx
 
 
 def conv_wgrad(dy, x, w_shape, stride, pad, out: Optional[torch.Tensor] = None, accumulate: bool = False):
     """``dW`` in the channels-last layout of the weight; ``out`` (a channels-last weight-shaped tensor, e.g. the
     parameter's gradient view) is written or accumulated in place when given."""
-    global launch_count
+    global _launches
     N, Cin, H, W = x.shape
     Cout, _, R, S = w_shape
     need = lib.tmpi_conv_wgrad_workspace_bytes(N, H, W, Cin, Cout, R, S, stride, pad)
@@ -91,14 +98,14 @@ def conv_wgrad(dy, x, w_shape, stride, pad, out: Optional[torch.Tensor] = None, 
         accumulate = False
     check(lib.tmpi_conv_wgrad(dy.data_ptr(), x.data_ptr(), out.data_ptr(), N, H, W, Cin, Cout, R, S, stride, pad,
                               ws.data_ptr(), ws.numel(), int(accumulate), stream_ptr()))
-    launch_count += 2
+    _launches += 2
     return out
 
 
 def matmul_tn_splitk(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False) -> torch.Tensor:
     """``a.T @ b`` for row-major ``a [K, M]`` and ``b [K, N]`` with a long ``K`` and a small output (a weight
     gradient over many rows): ``K`` is split over the SMs.  Rows of ``a`` / ``b`` may be pitched views."""
-    global launch_count
+    global _launches
     K, M = a.shape
     N = b.shape[1]
     ok = (has_symbol("tmpi_gemm_bf16_tn_splitk") and a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -116,7 +123,7 @@ def matmul_tn_splitk(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tenso
         accumulate = False
     check(lib.tmpi_gemm_bf16_tn_splitk(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
                                        ws.data_ptr(), ws.numel(), int(accumulate), stream_ptr()))
-    launch_count += 2
+    _launches += 2
     return out
 
 
@@ -173,7 +180,7 @@ class _ConvFn(torch.autograd.Function):
 
 def conv2d(x: torch.Tensor, w: torch.Tensor, stride: int = 1, padding: int = 0) -> torch.Tensor:
     if supported(x, w, stride, padding) and own_kernel_enabled(w.shape[2]):
-        return _ConvFn.apply(x, w, stride, padding, None)
+        return _native.ext().conv2d(x, w, stride, padding, None)
     return F.conv2d(x, w, None, stride, padding)
 
 
@@ -192,16 +199,31 @@ def conv_bn(conv: nn.Conv2d, bn, x: torch.Tensor, residual: Optional[torch.Tenso
         if fork is not None:
             fork.consumers -= 1       # a library convolution: autograd itself adds its gradient into x
         return bn(F.conv2d(x, w, None, conv.stride, conv.padding), residual, **bn_kw)
+    ext = _native.ext()
+    native = _native.takes(w) and (fork is None or isinstance(fork, ext.Fork))
     fn_state = {"param": w, "fork": fork}
     fuse = (bn.training and x.dtype == torch.bfloat16 and bn.weight.dtype == torch.float32
             and has_symbol("tmpi_bn_relu_fwd_partials") and fused_bn)
     if not fuse:
-        return bn(_ConvFn.apply(x, w, stride, pad, None, fn_state), residual, **bn_kw)
+        return bn(ext.conv2d(x, w, stride, pad, fork) if native else _ConvFn.apply(x, w, stride, pad, None, fn_state), residual, **bn_kw)
+    if native and type(bn) is bn_relu.FusedBatchNormReLU and _native.takes(bn.weight, bn.bias) and bn_relu.width_supported(w.shape[0], x.element_size()) \
+            and (res_fork is None or isinstance(res_fork, ext.Fork)) and bare(bn):
+        return ext.conv_bn(x, w, stride, pad, residual, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps, bn.momentum, bn.relu,
+                           fork, res_fork)
+    if native and (fork is not None or isinstance(res_fork, ext.Fork)):      # the C++ functions' fork, and a batch norm called as a module
+        return bn(ext.conv2d(x, w, stride, pad, fork), residual, **bn_kw)
     stats = bn_relu._scratch_for(x.device, w.shape[0]).view(torch.float32)
     y = _ConvFn.apply(x, w, stride, pad, stats, fn_state)
     if not bn_relu.supported(y):
         return bn(y, residual, **bn_kw)
     return bn(y, residual, partial_rows=fn_state["rows"], **bn_kw)
+
+
+def bare(m: nn.Module) -> bool:
+    """No hooks that a call of the module would run, its own or global ones."""
+    from torch.nn.modules import module as M
+    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+                or M._global_forward_hooks or M._global_forward_pre_hooks or M._global_backward_hooks or M._global_backward_pre_hooks)
 
 
 def own_kernel_enabled(kernel_size: int) -> bool:

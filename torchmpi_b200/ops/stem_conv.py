@@ -11,57 +11,30 @@ saved patch matrix.  Inputs that neither takes go to ``F.conv2d``.
 """
 from __future__ import annotations
 
-import ctypes
-import functools
-
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _native
 from .._lib import lib, check, dtype_code, has_symbol, stream_ptr
 from . import gemm
 
-launch_count = 0
+_launches = 0
 PATCH = 147
-_Strides = ctypes.c_int64 * 4
 
 
-@functools.lru_cache(maxsize=None)
-def _wgrad_workspace_bytes() -> int:
-    return lib.tmpi_stem_conv_wgrad_workspace_bytes()            # of the chip, not of the call
+def __getattr__(name: str):
+    if name == "launch_count":               # kernels launched by this module, the C++ functions' included
+        return _launches + _native.launches(_native.STEM)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
-class _StemDirectFn(torch.autograd.Function):
-    """The implicit GEMMs: nothing but the image is kept for backward."""
-
-    @staticmethod
-    def forward(ctx, x, w):
-        global launch_count
-        N, _, H, W = x.shape
-        y = torch.empty((N, w.shape[0], (H - 1) // 2 + 1, (W - 1) // 2 + 1), dtype=x.dtype, device=x.device,
-                        memory_format=torch.channels_last)
-        check(lib.tmpi_stem_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), N, H, W, w.shape[0],
-                                     _Strides(*w.stride()), stream_ptr()))
-        launch_count += 1
-        ctx.save_for_backward(x)
-        ctx.wshape, ctx.wstride = tuple(w.shape), w.stride()
-        return y
+class _StemDirectFn:
+    """The implicit GEMMs (csrc/bindings/autograd.cpp): nothing but the image is kept for backward."""
 
     @staticmethod
-    def backward(ctx, dy):
-        global launch_count
-        (x,) = ctx.saved_tensors
-        N, _, H, W = x.shape
-        dy = dy.contiguous(memory_format=torch.channels_last)
-        if dy.data_ptr() % 16:                                               # a view into a larger buffer
-            dy = dy.clone(memory_format=torch.channels_last)
-        dw = torch.empty_strided(ctx.wshape, ctx.wstride, dtype=x.dtype, device=x.device)
-        # partial sums of the CTAs (24 MB), from the allocator: calls on other streams, threads and in graphs have their own
-        ws = torch.empty(_wgrad_workspace_bytes(), dtype=torch.uint8, device=x.device)
-        check(lib.tmpi_stem_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, H, W, ctx.wshape[0],
-                                       _Strides(*ctx.wstride), ws.data_ptr(), _wgrad_workspace_bytes(), stream_ptr()))
-        launch_count += 2
-        return None, dw
+    def apply(x, w):
+        return _native.ext().stem_conv(x, w)
 
 
 def direct(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -80,7 +53,7 @@ def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 class _StemConvFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w):
-        global launch_count
+        global _launches
         N, _, H, W = x.shape
         OH, OW = (H + 6 - 7) // 2 + 1, (W + 6 - 7) // 2 + 1
         M, Cout = N * OH * OW, w.shape[0]
@@ -91,7 +64,7 @@ class _StemConvFn(torch.autograd.Function):
         w2d[:, :PATCH] = w.permute(0, 2, 3, 1).reshape(Cout, PATCH)          # (kh, kw, c) order of the patch rows
         y = torch.empty((N, Cout, OH, OW), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
         gemm.matmul_nt(col, w2d, out=y.permute(0, 2, 3, 1).reshape(M, Cout))
-        launch_count += 2
+        _launches += 2
         ctx.save_for_backward(col)
         ctx.wshape = tuple(w.shape)
         return y
