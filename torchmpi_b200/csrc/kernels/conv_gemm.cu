@@ -171,7 +171,7 @@ __device__ void producer(Shared* sh, unsigned char* tiles, unsigned char* b_res,
     const uint32_t tx = A_BYTES + (p.b_resident ? 0u : p.b_mode == B_K ? (uint32_t)p.b_block_bytes : (uint32_t)chunks * CHUNK_BYTES);
     const int kb0 = slice * p.k_per_slice, kb1 = min(kb0 + p.k_per_slice, p.k_blocks_total);
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!sm100::mbar_wait(&sh->empty[stage], phase ^ 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 2); return; }
+      if (!sm100::mbar_wait<true>(&sh->empty[stage], phase ^ 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 2); return; }
       unsigned char* a_dst = tiles + (size_t)stage * p.stage_bytes;
       uint64_t* bar = &sh->full[stage];
       sm100::mbar_expect_tx(bar, tx);
@@ -195,7 +195,7 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, unsigned char* b_re
   const bool a_mn = p.a_mode == A_MN, b_mn = p.b_mode != B_K;
   const uint32_t idesc = sm100::make_idesc_f16(BM, p.mma_n, true, b_mn, a_mn);
   if (p.b_resident) {
-    if (!sm100::mbar_wait(&sh->b_full, 0, kWaitBudgetNs) || sh->error) { fail(sh, p, 7); return; }
+    if (!sm100::mbar_wait<true>(&sh->b_full, 0, kWaitBudgetNs) || sh->error) { fail(sh, p, 7); return; }
     sm100::tc_fence_after();
   }
   const uint32_t b_res_addr = sm100::smem_u32(b_res);
@@ -205,12 +205,12 @@ __device__ void mma_issuer(Shared* sh, unsigned char* tiles, unsigned char* b_re
   for (int it = 0; item(p, it, &m_blk, &n_blk, &slice); ++it) {
     const int acc = it & 1;
     const uint32_t acc_phase = (it >> 1) & 1;
-    if (!sm100::mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 3); return; }
+    if (!sm100::mbar_wait<true>(&sh->acc_empty[acc], acc_phase ^ 1, kWaitBudgetNs) || sh->error) { fail(sh, p, 3); return; }
     sm100::tc_fence_after();
     const uint32_t d_tmem = sh->tmem_base + (uint32_t)acc * BN;
     const int kb0 = slice * p.k_per_slice, kb1 = min(kb0 + p.k_per_slice, p.k_blocks_total);
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!sm100::mbar_wait(&sh->full[stage], phase, kWaitBudgetNs) || sh->error) { fail(sh, p, 4); return; }
+      if (!sm100::mbar_wait<true>(&sh->full[stage], phase, kWaitBudgetNs) || sh->error) { fail(sh, p, 4); return; }
       sm100::tc_fence_after();
       const uint32_t a_addr = sm100::smem_u32(tiles + (size_t)stage * p.stage_bytes);
       const uint32_t b_addr = p.b_resident ? b_res_addr + (uint32_t)kb * (uint32_t)p.b_block_bytes : a_addr + A_BYTES;
@@ -328,7 +328,7 @@ __device__ void epilogue_store(Shared* sh, unsigned char* staging, float* stats_
   bool ok = true;
   for (int it = group; ok && item(p, it, &m_blk, &n_blk, &slice); it += 2) {
     const uint32_t acc_phase = (it >> 1) & 1;
-    ok = __all_sync(~0u, sm100::mbar_wait(&sh->acc_full[group], acc_phase, kWaitBudgetNs) && !sh->error);
+    ok = __all_sync(~0u, sm100::mbar_wait<true>(&sh->acc_full[group], acc_phase, kWaitBudgetNs) && !sh->error);
     if (!ok) { fail(sh, p, 5); break; }
     sm100::tc_fence_after();
     const int row0 = m_blk * BM + quarter * 32;
@@ -355,7 +355,7 @@ __device__ void epilogue_store(Shared* sh, unsigned char* staging, float* stats_
         }
         if (do_add) {
           load_add();
-          ok = __all_sync(~0u, sm100::mbar_wait(&add_full[done % RING], (done / RING) & 1, kWaitBudgetNs) && !sh->error);
+          ok = __all_sync(~0u, sm100::mbar_wait<true>(&add_full[done % RING], (done / RING) & 1, kWaitBudgetNs) && !sh->error);
           if (!ok) fail(sh, p, 8);
         }
         __syncwarp();
@@ -467,7 +467,7 @@ __device__ void epilogue_splitk(Shared* sh, const Problem& p, int group, int qua
   int m_blk, n_blk, slice;
   for (int it = group; item(p, it, &m_blk, &n_blk, &slice); it += 2) {
     const uint32_t acc_phase = (it >> 1) & 1;
-    if (!sm100::mbar_wait(&sh->acc_full[group], acc_phase, kWaitBudgetNs) || sh->error) { fail(sh, p, 6); break; }
+    if (!sm100::mbar_wait<true>(&sh->acc_full[group], acc_phase, kWaitBudgetNs) || sh->error) { fail(sh, p, 6); break; }
     sm100::tc_fence_after();
     const int tile = n_blk * p.tiles_m + m_blk;
     const int ncols = min(p.mma_n, p.N - n_blk * BN);

@@ -30,12 +30,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // The thread may be suspended for up to 20 us (it goes on as soon as the phase is complete): without the hint a waiting warp comes
 // back soon and polls, and the polls of all roles that wait take issue slots from those that work.  Attention forward of
-// 8 x 16 heads x 1024 x 64: 47.2 -> 43.8 us, backward 95.6 -> 93.5.
+// 8 x 16 heads x 1024 x 64: 47.2 -> 43.8 us, backward 95.6 -> 93.5; linear layer of 1024 x 1024 x 1024, both ways, 22.7 -> 20.7; stem 706 ->
+// 702.  POLL: without it, for the convolution kernel, whose short waits it made longer (a block of 64 x 1024 x 14 x 14 495.7 in place of
+// 491.0).
+template <bool POLL = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  if (POLL)
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -44,13 +52,14 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 // Waits for the phase with the given parity; gives up after `budget_ns` (returns false).
+template <bool POLL = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long budget_ns) {
   for (int i = 0; i < 1024; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<POLL>(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
   for (;;) {
     for (int i = 0; i < 256; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<POLL>(bar, parity)) return true;
     if (now_ns() - t0 > budget_ns) return false;
   }
 }
