@@ -66,7 +66,9 @@ static int gelu_fwd_t(const void* z, void* y, size_t n, cudaStream_t s) {
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "gelu_fwd launch: %s", cudaGetErrorString(e));
 }
 
-// dz = dy * gelu'(z), packs as above.
+// dz = dy * gelu'(z), packs as above.  Bound by memory: 8192 x 4096 bf16 33.1 us, 0.93 of the copy rate, with two packs of each operand in
+// flight and four blocks per SM; 50.2 with four packs and the registers that they take.  The pass below, with the column sums,
+// takes 42.4.
 template <typename T, int V>
 __global__ void __launch_bounds__(256, 4) gelu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __restrict__ dz, size_t npacks) {
   wait_previous(dy, z);

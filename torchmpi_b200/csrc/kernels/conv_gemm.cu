@@ -884,7 +884,7 @@ size_t tmpi_gemm_tn_splitk_workspace_bytes(int M, int N, int64_t K) {
   return (size_t)tm * tn * sl * conv::BM * mn * sizeof(float);
 }
 
-// Whether that beats the CTA-pair kernel: where whole tiles leave most SMs idle over a long K, against a second kernel and the
+// (The linear layers' weight gradients come from linear_bwd.cu.)  Whether that beats the CTA-pair kernel: where whole tiles leave most SMs idle over a long K, against a second kernel and the
 // partial tiles' way to memory and back.  An output of more than half as many tiles as SMs is not split at all: it would only
 // take that way, in several rounds.  Measured, back to back, in us (pair, split): 8192 x 1024 x 1024 37, 29; 8192 x 512 x 512
 // 37, 22; 8192 x 128 x 256 36, 14; 8192 x 1536 x 1536 39, 41; 4096 x 512 x 512 20, 20; 4096 x 1024 x 1024 21, 22; 2048 x 512 x 512
