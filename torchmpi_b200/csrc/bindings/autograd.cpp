@@ -65,21 +65,27 @@ struct KeptZeros {
   static constexpr size_t KEEP_BYTES = size_t(1) << 20, KEEP_STREAMS = 64;
   std::mutex lock;
   std::map<std::pair<int, void*>, Tensor> kept;
+  int kept_at = 0;
 
-  Tensor get(const Tensor& like, size_t need) {
+  // failures: a number that grows when a kernel may have left a buffer behind that is not zero; all are dropped then
+  Tensor get(const Tensor& like, size_t need, int failures = 0) {
     const auto bytes = like.options().dtype(at::kByte);
     if (need > KEEP_BYTES || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
       return at::zeros({(int64_t)need}, bytes);
     const std::pair<int, void*> key(like.get_device(), stream());
+    std::map<std::pair<int, void*>, Tensor> old;                           // released outside the lock
     {
       std::lock_guard<std::mutex> hold(lock);
+      if (failures != kept_at) {
+        old.swap(kept);
+        kept_at = failures;
+      }
       const auto found = kept.find(key);
       if (found != kept.end() && (size_t)found->second.numel() >= need) return found->second;
     }
     size_t size = 4096;
     while (size < need) size *= 2;
     const Tensor fresh = at::zeros({(int64_t)size}, bytes);
-    std::map<std::pair<int, void*>, Tensor> old;                           // released outside the lock
     std::lock_guard<std::mutex> hold(lock);
     if (kept.size() >= KEEP_STREAMS) old.swap(kept);
     kept[key] = fresh;
@@ -169,7 +175,7 @@ void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor
   if (bytes) ws = at::empty({(int64_t)bytes}, dy.options().dtype(at::kByte));
   if (counters) {
     static auto& kept = *new KeptZeros;
-    arrivals = kept.get(dy, sizeof(unsigned) * (size_t)counters);
+    arrivals = kept.get(dy, sizeof(unsigned) * (size_t)counters, tmpi_gemm_failures());
   }
   if (dx) *dx = at::empty({rows, in}, dy.options());
   if (dw) *dw = at::empty({out, in}, dy.options());

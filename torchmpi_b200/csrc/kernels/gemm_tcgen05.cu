@@ -10,6 +10,7 @@
 #include "tmap_encode.h"
 #include "../include/tmpi_c_api.h"
 #include "../runtime/common.h"
+#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -242,20 +243,30 @@ int tmpi_gemm_bf16_residual(const void* A, const void* B, void* C, const void* b
   return launch_gemm_pair(A, B, C, bias, M, N, K, bias ? gemm::EPI_BIAS : 0, gemm_status_word(), (cudaStream_t)stream, 0, 0, 0, nullptr, residual);
 }
 
+static int* gemm_status_host() {
+  static int* const host = [] {
+    int* d = gemm_status_word();
+    cudaPointerAttributes at;             // the mapped host pointer of the same word
+    return d && cudaPointerGetAttributes(&at, d) == cudaSuccess ? (int*)at.hostPointer : (int*)nullptr;
+  }();
+  return host;
+}
+static std::atomic<int> g_gemm_failures{0};          // non-zero words that have been read and cleared
+
 // Non-zero after a GEMM CTA gave up on a bounded wait (1000 + the point where it happened); clears it.
 int tmpi_gemm_status(void) {
-  int* d = gemm_status_word();
-  (void)d;
-  static int* host = nullptr;
-  if (!host && d) {
-    // the mapped host pointer of the same word
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, d) == cudaSuccess) host = (int*)at.hostPointer;
-  }
+  int* host = gemm_status_host();
   if (!host) return 0;
-  int v = *(volatile int*)host;
-  if (v) *(volatile int*)host = 0;
+  const int v = __atomic_exchange_n(host, 0, __ATOMIC_RELAXED);
+  if (v) g_gemm_failures.fetch_add(1);
   return v;
+}
+
+// Grows with every such report: whoever keeps something that a kernel leaves in order (arrival counters) starts afresh when it has
+// changed.
+int tmpi_gemm_failures(void) {
+  int* host = gemm_status_host();
+  return g_gemm_failures.load() + (host && __atomic_load_n(host, __ATOMIC_RELAXED) ? 1 : 0);
 }
 
 }  // extern "C"
