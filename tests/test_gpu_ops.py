@@ -653,3 +653,24 @@ def test_cross_entropy_labels_outside_the_row(cols, dtype):
     unit = {torch.float32: 2e-6, torch.float16: 2 ** -9, torch.bfloat16: 2 ** -7.5}[dtype]
     floor = (2 ** -24 if dtype == torch.float16 else 0.0) + 1e-6 / 6
     assert bool(((x.grad.double() - p).abs() <= unit * p.abs() + floor).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 10), (336, 10), (17, 5003), (5, 60001)])
+def test_cross_entropy_gradient_scaled_by_the_incoming_one(rows, cols, dtype):
+    """The bits of a multiplication by the incoming gradient in the logits' type; packs and remainders."""
+    from torchmpi_b200.ops import xent
+    torch.manual_seed(cols)
+    x = torch.randn(rows, cols, device="cuda").to(dtype)
+    labels = torch.randint(0, cols, (rows,), device="cuda")
+    grads = []
+    for unit in (True, False):
+        leaf = x.clone().requires_grad_(True)
+        loss = xent.cross_entropy(leaf, labels, unit)
+        (loss if unit else loss * 0.3).backward()
+        grads.append(leaf.grad)
+    assert torch.equal(grads[1], grads[0] * torch.tensor(0.3, device="cuda").to(dtype))
+    for bad in (float("inf"), float("nan")):
+        leaf = x.clone().requires_grad_(True)
+        (xent.cross_entropy(leaf, labels) * bad).backward()
+        assert torch.equal(leaf.grad.isnan(), (grads[0] * bad).isnan())

@@ -179,6 +179,7 @@ _CUDA_PROTOS = {
     "tmpi_absmean_var": (_i, [_vp, _i, _sz, _vp, _vp, _vp]),
     "tmpi_absmean_var_scratch_bytes": (_sz, []),
     "tmpi_easgd_elastic": (_i, [_vp, _vp, _vp, _sz, _i, _f, _vp]),
+    "tmpi_scale": (_i, [_vp, _sz, _i, _vp, _vp]),
     "tmpi_downpour_accum": (_i, [_vp, _vp, _sz, _i, _f, _i, _vp]),
     "tmpi_bias_grad_scratch_bytes": (_sz, [_i]),
     "tmpi_bias_grad": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp]),

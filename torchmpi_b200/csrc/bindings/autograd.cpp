@@ -378,7 +378,10 @@ struct XentFn : public torch::autograd::Function<XentFn> {
     TORCH_CHECK(kept.isTensor(), "cross_entropy: the gradient of this loss has been handed out already (backward runs once)");
     Tensor buf = kept.toTensor();
     kept = c10::IValue();
-    if (!ctx->saved_data["unit"].toBool()) buf.mul_(grads[0].to(buf.scalar_type()));
+    if (!ctx->saved_data["unit"].toBool()) {
+      check(tmpi_scale(buf.data_ptr(), (size_t)buf.numel(), dtype_code(buf.scalar_type()), grads[0].data_ptr<float>(), stream()));
+      launched(XENT, 1);
+    }
     return {buf.narrow(1, 0, ctx->saved_data["cols"].toInt()), Tensor(), Tensor()};
   }
 };

@@ -236,6 +236,7 @@ int tmpi_absmean_var(const void* x, int dtype, size_t n, double* out2, void* scr
 size_t tmpi_absmean_var_scratch_bytes(void);
 int tmpi_easgd_elastic(void* local, const void* center, void* delta, size_t n, int dtype,
                        float alpha, void* stream);
+int tmpi_scale(void* x, size_t n, int dtype, const float* scale, void* stream);   // x *= *scale
 int tmpi_downpour_accum(void* accum, const void* grad, size_t n, int dtype, float scale,
                         int zero_first, void* stream);
 // bias gradient of a linear layer: db[c] = sum_r dz[r, c]; with z given, dz = dy * gelu'(z) is computed and
