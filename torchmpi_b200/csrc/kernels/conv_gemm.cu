@@ -545,68 +545,50 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 }
 
-// out[row, n0 + c] (+)= sum over slices of the partial tiles.  L lanes (a power of two up to 32) share one group of
-// 8 columns: lane j adds slices j, j + L, ... and the L partial sums are combined by a fixed butterfly, so the
-// result does not depend on timing.
-__global__ void __launch_bounds__(256)
-conv_splitk_reduce_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int M, int N, int tiles_m, int tiles_n,
-                          int slices, int mma_n, int accumulate, int L) {
-  const int groups = N / 8;                                    // N is a multiple of 8
-  const long long total = (long long)M * groups;
-  const int sub = threadIdx.x & (L - 1);
-  const long long per_block = blockDim.x / L;
-  for (long long i0 = (long long)blockIdx.x * per_block; i0 < total; i0 += (long long)gridDim.x * per_block) {
-    const long long i = i0 + threadIdx.x / L;
-    const bool live = i < total;
-    float a[8];
+// out[row, col] (+)= sum over slices of the partial tiles.  A warp reads 128 columns of a row (512 contiguous bytes) of every W-th slice,
+// U slices in flight; the W warps of a row add their sums in order, so the result does not depend on timing.  Bound by the loads'
+// latency.  Lanes that shared 8 columns and took a slice each read 32-byte pieces of 32 slices per instruction; before and now, images x
+// inputs x outputs x size, us: 256 x 512 x 128 x 28 9.3, 4.8; 256 x 128 x 512 x 28 7.0, 4.0; 32 x 1024 x 256 x 14 14.2, 6.8; 64 x 256 x 64 x 56
+// 5.2, 5.0; 8 x 512 x 2048 x 7, two slices, 2.8, 4.0.
+constexpr int RED_WARPS = 8;
+template <int U>
+__global__ void __launch_bounds__(32 * RED_WARPS)
+conv_splitk_reduce_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int M, int N, int tiles_m, int slices, int mma_n,
+                          int accumulate, int W, int col_blocks) {
+  __shared__ float4 part[RED_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % W;
+  const int row = (int)(blockIdx.x / (unsigned)col_blocks) * (RED_WARPS / W) + warp / W;
+  const int col = (int)(blockIdx.x % (unsigned)col_blocks) * 128 + lane * 4;
+  const bool live = row < M && col < N;                        // N is a multiple of 8
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [&](const float4& x) { a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w; };
+  if (live) {
+    const int m_blk = row / BM, n_blk = col / BN;
+    const size_t pitch = (size_t)BM * mma_n;
+    const float* src = ws + (size_t)(n_blk * tiles_m + m_blk) * slices * pitch + (size_t)(row - m_blk * BM) * mma_n + (col - n_blk * BN);
+    int s = sub;
+    for (; s < slices; s += U * W) {                           // an absent slice adds nothing
+      float4 x[U];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = 0.f;
-    int row = 0, col = 0;
-    if (live) {
-      row = (int)(i / groups); col = (int)(i - (long long)row * groups) * 8;
-      const int m_blk = row / BM, n_blk = col / BN;
-      const int tile = n_blk * tiles_m + m_blk;
-      const float* src = ws + (((size_t)tile * slices) * BM + (row - m_blk * BM)) * mma_n + (col - n_blk * BN);
-      int s = sub;
-      for (; s + 3 * L < slices; s += 4 * L) {                 // four slices of loads in flight
-        float4 x[4][2];
+      for (int u = 0; u < U; ++u)
+        x[u] = s + u * W < slices ? __ldcs(reinterpret_cast<const float4*>(src + (size_t)(s + u * W) * pitch)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4* q = reinterpret_cast<const float4*>(src + (size_t)(s + u * L) * BM * mma_n);
-          x[u][0] = __ldcs(q); x[u][1] = __ldcs(q + 1);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          a[0] += x[u][0].x; a[1] += x[u][0].y; a[2] += x[u][0].z; a[3] += x[u][0].w;
-          a[4] += x[u][1].x; a[5] += x[u][1].y; a[6] += x[u][1].z; a[7] += x[u][1].w;
-        }
-      }
-      for (; s < slices; s += L) {
-        const float4* q = reinterpret_cast<const float4*>(src + (size_t)s * BM * mma_n);
-        const float4 x0 = __ldcs(q), x1 = __ldcs(q + 1);
-        a[0] += x0.x; a[1] += x0.y; a[2] += x0.z; a[3] += x0.w; a[4] += x1.x; a[5] += x1.y; a[6] += x1.z; a[7] += x1.w;
-      }
-    }
-    for (int d = 1; d < L; d <<= 1) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] += __shfl_xor_sync(0xffffffffu, a[e], d);
-    }
-    if (live && sub == 0) {
-      __nv_bfloat16* dst = out + (size_t)row * N + col;
-      if (accumulate) {
-        float f[8];
-        unpack8(*reinterpret_cast<const uint4*>(dst), f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] += f[e];
-      }
-      __nv_bfloat162 h0 = __floats2bfloat162_rn(a[0], a[1]), h1 = __floats2bfloat162_rn(a[2], a[3]);
-      __nv_bfloat162 h2 = __floats2bfloat162_rn(a[4], a[5]), h3 = __floats2bfloat162_rn(a[6], a[7]);
-      uint4 u;
-      u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
-      u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
-      *reinterpret_cast<uint4*>(dst) = u;
+      for (int u = 0; u < U; ++u) add(x[u]);
     }
   }
+  if (W > 1) {
+    part[warp][lane] = a;
+    __syncthreads();
+  }
+  if (!live || sub) return;
+  for (int w = 1; w < W; ++w) add(part[warp + w][lane]);
+  __nv_bfloat16* dst = out + (size_t)row * N + col;
+  if (accumulate) {
+    const uint2 o = *reinterpret_cast<const uint2*>(dst);
+    add(make_float4(__uint_as_float(o.x << 16), __uint_as_float(o.x & 0xffff0000u), __uint_as_float(o.y << 16), __uint_as_float(o.y & 0xffff0000u)));
+  }
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+  *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 }  // namespace conv
@@ -711,13 +693,14 @@ static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const void*
 }
 
 static int launch_splitk_reduce(const conv::Problem& p, const void* workspace, void* out, int accumulate, cudaStream_t s) {
-  int L = 1;
-  while (L < 32 && L < p.slices) L <<= 1;                       // lanes per group of 8 columns
-  const long long groups = (long long)p.M * (p.N / 8);
-  const long long per_block = 256 / L;
-  const int grid = (int)std::min<long long>((groups + per_block - 1) / per_block, (long long)gemm_sm_count() * 8);
-  conv::conv_splitk_reduce_kernel<<<grid, 256, 0, s>>>((const float*)workspace, (__nv_bfloat16*)out, p.M, p.N, p.tiles_m, p.tiles_n,
-                                                     p.slices, p.mma_n, accumulate, L);
+  int W = 1;                                                    // warps of a row, two slices each or more
+  while (W < conv::RED_WARPS && 2 * W < p.slices) W <<= 1;
+  const int per_block = conv::RED_WARPS / W, col_blocks = (p.N + 127) / 128;
+  const long long blocks = (long long)((p.M + per_block - 1) / per_block) * col_blocks;
+  if (blocks > 0x7fffffffLL) return fail(TMPI_ERR_UNSUPPORTED, "split-K reduce: output too large");
+  const auto kernel = p.slices <= 2 * W ? conv::conv_splitk_reduce_kernel<2> : p.slices <= 5 * W ? conv::conv_splitk_reduce_kernel<5> : conv::conv_splitk_reduce_kernel<10>;
+  kernel<<<(unsigned)blocks, 32 * conv::RED_WARPS, 0, s>>>((const float*)workspace, (__nv_bfloat16*)out, p.M, p.N, p.tiles_m, p.slices, p.mma_n,
+                                                           accumulate, W, col_blocks);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "split-K reduce launch: %s", cudaGetErrorString(e));
 }
