@@ -473,31 +473,39 @@ __global__ void __launch_bounds__(THREADS, 1) stem_wgrad_kernel(const __grid_con
   teardown(sh, warp);
 }
 
-// One block per output channel: ten groups of threads add the partial rows of a contiguous range of CTAs (dY row i and, ten
-// input rows being shared by two dY rows, row i + 1 two input rows further on), the groups' sums are added in order.
-constexpr int RED_COLS = TAPS * WG_N / 4, RED_GROUPS = 10;
+// One block per output channel and tap pair: 32 groups of threads add the partial rows of a contiguous range of CTAs (dY row i and,
+// ten input rows being shared by two dY rows, row i + 1 two input rows further on), all loads of a thread in flight; the groups' sums are
+// added in order.  Bound by the 24 MB of partial sums.  A block per channel, with ten groups, 7.7 us; now 6.0.
+constexpr int RED_COLS = WG_N / 4, RED_GROUPS = 32, RED_ROWS = 5;
 __global__ void __launch_bounds__(RED_COLS * RED_GROUPS)
 stem_wgrad_reduce_kernel(const float* __restrict__ partial, int ctas, __nv_bfloat16* __restrict__ dw, int64_t s_co, int64_t s_c, int64_t s_h,
                          int64_t s_w) {
   __shared__ float4 sum[RED_GROUPS][2][RED_COLS];
-  const int col = threadIdx.x % RED_COLS, grp = threadIdx.x / RED_COLS, co = blockIdx.x;
-  const int per = (ctas + RED_GROUPS - 1) / RED_GROUPS;
+  const int col = threadIdx.x % RED_COLS, grp = threadIdx.x / RED_COLS, co = blockIdx.x, tap = blockIdx.y;
+  const int per = (ctas + RED_GROUPS - 1) / RED_GROUPS, end = min(ctas, (grp + 1) * per);
   float4 a[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll 4
-  for (int c = grp * per; c < min(ctas, (grp + 1) * per); ++c)
+  for (int c0 = grp * per; c0 < end; c0 += RED_ROWS) {
+    float4 v[RED_ROWS][2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(partial + ((size_t)c * 128 + h * 64 + co) * (TAPS * WG_N)) + col);
-      a[h].x += v.x; a[h].y += v.y; a[h].z += v.z; a[h].w += v.w;
-    }
+    for (int r = 0; r < RED_ROWS; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        v[r][h] = c0 + r < end ? __ldg(reinterpret_cast<const float4*>(partial + ((size_t)(c0 + r) * 128 + h * 64 + co) * (TAPS * WG_N) + tap * WG_N) + col)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RED_ROWS; ++r)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) { a[h].x += v[r][h].x; a[h].y += v[r][h].y; a[h].z += v[r][h].z; a[h].w += v[r][h].w; }
+  }
   sum[grp][0][col] = a[0];
   sum[grp][1][col] = a[1];
   __syncthreads();
   for (int o = threadIdx.x; o < 147; o += blockDim.x) {
-    const int kh = o / 21, kw = o % 21 / 3, c = o % 3;
-    const int tap = (kw + 1) >> 1, e = (kw + 1) & 1;
-    const int at0 = tap * WG_N + kh * 8 + e * 4 + c, at1 = at0 + 16;
+    const int kh = o / 21, kw = o % 21 / 3, c = o % 3, e = (kw + 1) & 1;
+    if (((kw + 1) >> 1) != tap) continue;
+    const int at0 = kh * 8 + e * 4 + c, at1 = at0 + 16;
     float t = 0.f;
+#pragma unroll
     for (int g = 0; g < RED_GROUPS; ++g)
       t += reinterpret_cast<const float*>(sum[g][0])[at0] + reinterpret_cast<const float*>(sum[g][1])[at1];
     dw[co * s_co + c * s_c + kh * s_h + kw * s_w] = __float2bfloat16_rn(t);
@@ -570,7 +578,7 @@ int tmpi_stem_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, 
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return fail(TMPI_ERR_CUDA, "stem weight gradient: shared memory attribute: %s", cudaGetErrorString(e));
   kernel<<<grid, stem::THREADS, smem, (cudaStream_t)stream>>>(mdy, p);
-  stem::stem_wgrad_reduce_kernel<<<stem::COUT, stem::RED_COLS * stem::RED_GROUPS, 0, (cudaStream_t)stream>>>(
+  stem::stem_wgrad_reduce_kernel<<<dim3(stem::COUT, stem::TAPS), stem::RED_COLS * stem::RED_GROUPS, 0, (cudaStream_t)stream>>>(
       (const float*)workspace, grid, (__nv_bfloat16*)dw, p.ws_co, p.ws_c, p.ws_h, p.ws_w);
   e = cudaGetLastError();
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "stem weight gradient launch: %s", cudaGetErrorString(e));
