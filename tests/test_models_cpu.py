@@ -45,3 +45,28 @@ def test_backward_route_order_from_environment(monkeypatch):
         monkeypatch.delenv("TORCHMPI_ATTENTION_BACKWARD")
         importlib.reload(attention)
     assert attention._BACKWARDS[0] == "own"
+
+
+def test_fused_bottleneck_trains_without_the_cuda_functions(monkeypatch):
+    """On the CPU every layer of a fused block takes PyTorch's functions, so the block runs where the CUDA extension is not there."""
+    from torchmpi_b200 import _native
+    from torchmpi_b200.models.resnet import Bottleneck, _bn
+
+    def missing():
+        raise ImportError("no CUDA extension")
+    monkeypatch.setattr(_native, "ext", missing)
+    for first in (False, True):
+        torch.manual_seed(0)
+        down = torch.nn.Sequential(torch.nn.Conv2d(64, 256, 1, bias=False), _bn(256, True, relu=False)) if first else None
+        m = Bottleneck(64 if first else 256, 64, 1, down, fused_bn=True)
+        x = torch.randn(2, 64 if first else 256, 6, 6, requires_grad=True)
+        y = m(x)
+        dy = torch.randn_like(y)
+        y.backward(dy)
+        plain = Bottleneck(64 if first else 256, 64, 1, None, fused_bn=False)
+        plain.downsample = torch.nn.Sequential(torch.nn.Conv2d(64, 256, 1, bias=False), torch.nn.BatchNorm2d(256)) if first else None
+        plain.load_state_dict({k: v for k, v in m.state_dict().items() if "running" not in k and "tracked" not in k}, strict=False)
+        leaf = x.detach().clone().requires_grad_(True)
+        ref = plain(leaf)
+        ref.backward(dy)
+        assert torch.allclose(y, ref, rtol=1e-4, atol=1e-5) and torch.allclose(x.grad, leaf.grad, rtol=1e-3, atol=1e-5)

@@ -42,13 +42,13 @@ class Bottleneck(nn.Module):
         self.bn3 = _bn(planes * 4, fused_bn, relu=True, zero_init=True)   # relu after the residual add
         self.downsample = downsample
 
-    def _fork(self):
-        """The C++ functions' fork where they take every layer of the block, the Python functions' otherwise."""
+    def _fork(self, x):
+        """The C++ functions' fork where they take every layer of the block, the Python functions' otherwise (and on the CPU)."""
         from .. import _native
         layers = [self.conv1, self.bn1, self.conv2, self.bn2, self.conv3, self.bn3]
         if self.downsample is not None:
             layers += list(self.downsample)
-        if _native.takes(*(p for m in layers for p in m._parameters.values())):
+        if x.is_cuda and _native.takes(*(p for m in layers for p in m._parameters.values())):
             return _native.ext().Fork(2)
         from ..parallel.flat_buckets import GradFork
         return GradFork(2)
@@ -60,7 +60,7 @@ class Bottleneck(nn.Module):
             # x has two consumers (the first convolution and the identity branch): their gradients are summed
             # inside the kernel of whichever runs last in backward instead of by a separate add
             from .. import config
-            fork = self._fork() if (torch.is_grad_enabled() and x.requires_grad and config.get("grad_fork")) else None
+            fork = self._fork(x) if (torch.is_grad_enabled() and x.requires_grad and config.get("grad_fork")) else None
             res_fork = None
             if self.downsample is not None:
                 identity = conv_bn(self.downsample[0], self.downsample[1], x, fork=fork)
