@@ -102,3 +102,33 @@ def test_gradients_on_several_streams_and_in_a_graph():
         eager = grads()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for g in (captured, eager) for a, b in zip(g, want))
+
+
+def test_counters_after_waits_that_ran_out():
+    """A kernel that gave up may leave its counters half way: none that was in use before or during a report is handed out after it."""
+    from torchmpi_b200 import _native
+    from torchmpi_b200._lib import TorchMPIError, check, lib
+    from torchmpi_b200.ops import gemm
+    like = torch.empty(1, device="cuda", dtype=torch.bfloat16)
+    take = _native.ext().arrival_counters
+    gemm.check_status()
+    first = take(like, 64)
+    assert take(like, 64).data_ptr() == first.data_ptr()                      # kept for the stream
+    held = [first]                                                            # alive, so that no new one lies where an old one was
+    try:
+        for again in (False, True):                                           # the second report while the first is unread
+            check(lib.tmpi_gemm_report(1024))
+            for _ in range(2):
+                fresh = take(like, 64)
+                assert not fresh.any() and all(fresh.data_ptr() != t.data_ptr() for t in held)
+                fresh.fill_(1)                                                # as the next kernel that gives up
+                held.append(fresh)
+            if again:
+                check(lib.tmpi_gemm_report(1025))
+    finally:
+        with pytest.raises(TorchMPIError, match="1024"):
+            gemm.check_status()
+    fresh = take(like, 64)
+    assert not fresh.any() and all(fresh.data_ptr() != t.data_ptr() for t in held)
+    assert take(like, 64).data_ptr() == fresh.data_ptr()
+    gemm.check_status()

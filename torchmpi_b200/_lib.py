@@ -216,6 +216,7 @@ _CUDA_PROTOS = {
     "tmpi_linear_bwd": (_i, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp, _i, _vp]),
     "tmpi_gemm_status": (_i, []),
     "tmpi_gemm_failures": (_i, []),
+    "tmpi_gemm_report": (_i, [_i]),
     "tmpi_conv_max_ctas": (_i, []),
     "tmpi_conv_fwd": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _ip, _vp]),
     "tmpi_conv_dgrad_masked": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),

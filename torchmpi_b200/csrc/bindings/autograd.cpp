@@ -67,10 +67,11 @@ struct KeptZeros {
   std::map<std::pair<int, void*>, Tensor> kept;
   int kept_at = 0;
 
-  // failures: a number that grows when a kernel may have left a buffer behind that is not zero; all are dropped then
+  // failures: a number that grows when a kernel may have left a buffer behind that is not zero; all are dropped then.  It is odd as long as
+  // a report of that waits to be read: further kernels may give up meanwhile without another change, so nothing is kept until then.
   Tensor get(const Tensor& like, size_t need, int failures = 0) {
     const auto bytes = like.options().dtype(at::kByte);
-    if (need > KEEP_BYTES || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    if (need > KEEP_BYTES || failures % 2 || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
       return at::zeros({(int64_t)need}, bytes);
     const std::pair<int, void*> key(like.get_device(), stream());
     std::map<std::pair<int, void*>, Tensor> old;                           // released outside the lock
@@ -165,6 +166,12 @@ std::pair<Tensor, Tensor> bias_grad(const Tensor& dy, const Tensor& z) {
   return {dz, db};
 }
 
+// Arrival counters for linear_bwd.cu
+Tensor arrival_counters(const Tensor& like, int64_t counters) {
+  static auto& kept = *new KeptZeros;
+  return kept.get(like, sizeof(unsigned) * (size_t)counters, tmpi_gemm_failures());
+}
+
 // dX = dY W, dW = dY^T X and db = column sums of dY, those that are wanted, in one launch; dY may have a row pitch
 void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor* dx, Tensor* dw, Tensor* db) {
   const int rows = (int)x.size(0), in = (int)x.size(1), out = (int)w.size(0), want = (dx ? 1 : 0) | (dw ? 2 : 0) | (db ? 4 : 0);
@@ -173,10 +180,7 @@ void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor
   check(tmpi_linear_bwd_plan(rows, in, out, want, 0, &bytes, &counters));
   Tensor ws, arrivals;
   if (bytes) ws = at::empty({(int64_t)bytes}, dy.options().dtype(at::kByte));
-  if (counters) {
-    static auto& kept = *new KeptZeros;
-    arrivals = kept.get(dy, sizeof(unsigned) * (size_t)counters, tmpi_gemm_failures());
-  }
+  if (counters) arrivals = arrival_counters(dy, counters);
   if (dx) *dx = at::empty({rows, in}, dy.options());
   if (dw) *dw = at::empty({out, in}, dy.options());
   if (db) *db = at::empty({out}, dy.options());
@@ -625,5 +629,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return bn_relu(y, residual, gamma, beta, rm, rv, eps, momentum, relu, true, res_fork, rows, scratch);
   });
   m.def("cross_entropy_scratch", xent_scratch);
+  m.def("arrival_counters", arrival_counters);
   m.def("launches", [](int what) { return g_launches[what].load(std::memory_order_relaxed); });
 }

@@ -367,7 +367,8 @@ int tmpi_gemm_bf16_residual(const void* A, const void* B, void* C, const void* b
 // explicit row pitches (elements, multiples of 8) of A, B, C as stored; M, N >= 256
 int tmpi_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                       int64_t lda, int64_t ldb, int64_t ldc, int epilogue, void* stream);
-int tmpi_gemm_failures(void);     // grows when a GEMM CTA has given up on a wait; tmpi_gemm_status does not set it back
+int tmpi_gemm_report(int code);   // sets the word that tmpi_gemm_status reads, as a CTA does that gives up (for tests)
+int tmpi_gemm_failures(void);     // twice the reports that tmpi_gemm_status has returned, odd while one waits to be read
 // The gradients of a linear layer in one launch (linear_bwd.cu): dx [rows, in] = dy w, dw [out, in] = dy^T x, db [out] = column sums
 // of dy (rows ld_dy elements apart, 0: dense); in and ld_dy multiples of 8.  want: 1 dx, 2 dw, 4 db.  form: 0, or the tiles and slices (linear_bwd.cu, plan).
 int tmpi_linear_bwd_plan(int rows, int in, int out, int want, int form, size_t* workspace_bytes, int* counters);

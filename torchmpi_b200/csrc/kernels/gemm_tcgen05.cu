@@ -251,22 +251,34 @@ static int* gemm_status_host() {
   }();
   return host;
 }
-static std::atomic<int> g_gemm_failures{0};          // non-zero words that have been read and cleared
+static std::atomic<int> g_gemm_failures{0};          // reports that have been read
 
 // Non-zero after a GEMM CTA gave up on a bounded wait (1000 + the point where it happened); clears it.
 int tmpi_gemm_status(void) {
   int* host = gemm_status_host();
   if (!host) return 0;
-  const int v = __atomic_exchange_n(host, 0, __ATOMIC_RELAXED);
-  if (v) g_gemm_failures.fetch_add(1);
-  return v;
+  if (!__atomic_load_n(host, __ATOMIC_SEQ_CST)) return 0;
+  g_gemm_failures.fetch_add(1);                      // before the word is cleared: it is never back at what it was before the report
+  return __atomic_exchange_n(host, 0, __ATOMIC_SEQ_CST);
 }
 
-// Grows with every such report: whoever keeps something that a kernel leaves in order (arrival counters) starts afresh when it has
-// changed.
+// Twice the reports that have been read, and one more while another waits to be read.  Whoever keeps something that a kernel leaves in order
+// (arrival counters) starts afresh when the number has changed, and keeps nothing while it is odd: the word holds the first report
+// only, so those that follow before it is read do not show.
 int tmpi_gemm_failures(void) {
   int* host = gemm_status_host();
-  return g_gemm_failures.load() + (host && __atomic_load_n(host, __ATOMIC_RELAXED) ? 1 : 0);
+  const int pending = host && __atomic_load_n(host, __ATOMIC_SEQ_CST) ? 1 : 0;
+  return 2 * g_gemm_failures.load() + pending;
+}
+
+// Reports on the host what a CTA reports that gives up on a wait: the code stays until tmpi_gemm_status reads it.  For tests of what
+// follows such a report, which no kernel has to be made to run into.
+int tmpi_gemm_report(int code) {
+  int* host = gemm_status_host();
+  if (!host) return fail(TMPI_ERR_CUDA, "gemm_report: no status word");
+  int none = 0;
+  __atomic_compare_exchange_n(host, &none, code, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
+  return TMPI_OK;
 }
 
 }  // extern "C"
