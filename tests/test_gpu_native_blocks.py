@@ -86,3 +86,70 @@ def test_block_on_a_side_stream_and_in_a_graph():
     torch.cuda.synchronize()
     for a, b, c in zip(want, got, captured):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+def _layers():
+    """(module, input, whether its gradient is wanted)"""
+    from torchmpi_b200.models import to_bf16_mixed
+    from torchmpi_b200.ops import attention, gemm, layernorm
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLUMaxPool
+    from torchmpi_b200.ops.stem_conv import StemConv7x7
+    bf16 = {"device": "cuda", "dtype": torch.bfloat16}
+
+    class Head(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.weight = torch.nn.Parameter(torch.randn(1003, 256, **bf16))
+
+        def forward(self, x):
+            return gemm.wide_head(x, self.weight)
+
+    class Attention(torch.nn.Module):
+        def forward(self, x):
+            return attention.causal_attention(x, 2)
+    image = torch.randn(2, 32, 64, 3, **bf16).permute(0, 3, 1, 2)
+    stem = to_bf16_mixed(torch.nn.Sequential(StemConv7x7(64), FusedBatchNormReLUMaxPool(64)).cuda()).to(memory_format=torch.channels_last)
+    with torch.device("cuda"):
+        up, wide, down = (gemm.Linear(128, n, gelu=g, dtype=torch.bfloat16) for n, g in ((384, True), (1024, True), (384, False)))
+    x = torch.randn(256, 128, **bf16)
+    sinks = _block(False)[1]
+    for p in sinks.parameters():
+        p._tmpi_grad_sink = lambda *a, **k: None
+    yield from ((up, x, True), (up, x, False), (wide, x, True), (down, x, True), (Head(), torch.randn(256, 256, **bf16), True),
+                (layernorm.LayerNorm(256, **bf16), torch.randn(40, 256, **bf16), True), (Attention(), torch.randn(2, 128, 384, **bf16), True), (stem, image, False))
+    for first in (False, True):
+        inp, m = _block(first)
+        yield m, torch.randn(3, 12, 10, inp, **bf16).permute(0, 3, 1, 2), True
+    yield sinks, torch.randn(3, 12, 10, 256, **bf16).permute(0, 3, 1, 2), True
+
+
+def test_saved_tensors_in_another_layout():
+    """Hooks on saved tensors may hand back the same values in another order in memory (save_on_cpu with pinned memory does)."""
+    torch.manual_seed(5)
+    for at, (m, x, grad) in enumerate(_layers()):
+        out, state = [], {k: v.clone() for k, v in m.state_dict().items()}
+        for relayout in (lambda t: t, lambda t: t.clone(memory_format=torch.contiguous_format), lambda t: t.transpose(0, 1).contiguous().transpose(0, 1) if t.dim() > 1 else t):
+            m.load_state_dict(state)
+            m.zero_grad(set_to_none=True)
+            leaf = x.clone().requires_grad_(grad)
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t, relayout):
+                y = m(leaf)
+            y.backward(torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(y.dtype))
+            out.append([leaf.grad] + [p.grad for p in m.parameters()])
+        for other in out[1:]:
+            for a, b in zip(out[0], other):
+                # the sums of attention's dQ have no fixed order, and the library's 3 x 3 convolutions go by the layout: some roundings to bf16
+                # (2^-8) differ; values in the wrong places differ by more than their norm
+                same = a is None and b is None or (torch.equal(a, b) if at < 6 or at == 7 else (a.float() - b.float()).norm() <= 2e-2 * a.float().norm())
+                assert same, (at, m)
+    # a bias alone
+    m, x, _ = next(_layers())
+    m.weight.requires_grad_(False)
+    out = []
+    for relayout in (lambda t: t, lambda t: t.t().contiguous().t() if t.dim() > 1 else t):
+        m.bias.grad = None
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, relayout):
+            y = m(x)
+        y.backward(torch.ones_like(y))
+        out.append(m.bias.grad)
+    assert torch.equal(*out)

@@ -57,6 +57,9 @@ Tensor packed(const Tensor& t) {
   return (uintptr_t)c.data_ptr() % 16 ? c.clone() : c;
 }
 
+// A saved tensor as it was saved: hooks (torch.autograd.graph.save_on_cpu, say) may hand it back in another layout.
+Tensor as_saved(const Tensor& t, at::MemoryFormat format = at::MemoryFormat::Contiguous) { return t.defined() ? t.contiguous(format) : t; }
+
 // Buffers of arrival counters, which a kernel finds zero and leaves zero.  Two calls may share one only if one ends before the
 // other starts, so there is one per stream, grown to the next power of two.  A call that is being captured gets its own, cleared
 // inside the graph: the graph may be replayed on any stream, and has not run when the next eager call comes.  So does a call
@@ -192,7 +195,6 @@ void linear_gradients(const Tensor& dy, const Tensor& x, const Tensor& w, Tensor
 
 // dy * gelu'(z)
 Tensor gelu_gradient(const Tensor& dy, const Tensor& z) {
-  if ((uintptr_t)z.data_ptr() % 16) return at::gelu_backward(dy, z);
   Tensor dz = at::empty_like(dy);
   check(tmpi_gelu_bwd(dy.data_ptr(), z.data_ptr(), dz.data_ptr(), (size_t)dy.numel(), dtype_code(dy.scalar_type()), stream()));
   launched(LINEAR, 1);
@@ -219,7 +221,7 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x2 = saved[0], &w = saved[1], &z = saved[2];
+    const Tensor x2 = as_saved(saved[0]), w = as_saved(saved[1]), z = as_saved(saved[2]);
     const Tensor& dy = grads[0];
     Tensor dy2 = packed(dy.reshape({-1, dy.size(-1)})), db, dx, dw;
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
@@ -227,7 +229,7 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     if ((need_x || need_w) && dy2.size(1) % 8 == 0 && pair_enabled()) {
       if (z.defined()) dy2 = gelu_gradient(dy2, z);
       const bool need_b = ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2);
-      linear_gradients(dy2, x2.contiguous(), w.contiguous(), need_x ? &dx : nullptr, need_w ? &dw : nullptr, need_b ? &db : nullptr);
+      linear_gradients(dy2, x2, w, need_x ? &dx : nullptr, need_w ? &dw : nullptr, need_b ? &db : nullptr);
       if (need_x) dx = dx.view(ctx->saved_data["shape"].toIntVector());
       return {dx, dw, db, Tensor(), dres};
     }
@@ -252,7 +254,7 @@ struct WideHeadFn : public torch::autograd::Function<WideHeadFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor x = as_saved(saved[0]), w = as_saved(saved[1]);
     Tensor dl = grads[0], dx, dw;
     if (!(dl.stride(1) == 1 && dl.stride(0) % 8 == 0 && dl.stride(0) >= dl.size(1) && (uintptr_t)dl.data_ptr() % 16 == 0)) {
       Tensor padded = at::zeros({dl.size(0), (dl.size(1) + 7) / 8 * 8}, dl.options());
@@ -282,12 +284,12 @@ Tensor layer_norm_forward(AutogradContext* ctx, const Tensor& x, const Tensor& w
 // `add` (may be undefined): a gradient of x from elsewhere, added to dx
 variable_list layer_norm_backward(AutogradContext* ctx, const Tensor& dy, const Tensor& add) {
   const auto saved = ctx->get_saved_variables();
-  const Tensor &x2 = saved[0], &weight = saved[1];
+  const Tensor x2 = as_saved(saved[0]), weight = as_saved(saved[1]), stats = as_saved(saved[2]);
   const int64_t rows = x2.size(0), C = x2.size(1);
   const Tensor dy2 = packed(dy.reshape({rows, C})), add2 = add.defined() ? packed(add.reshape({rows, C})) : add;
   Tensor dx = at::empty_like(x2), dgamma = at::empty_like(weight), dbeta = at::empty_like(weight);
   Tensor scratch = at::empty({(int64_t)tmpi_layernorm_scratch_bytes((int)C)}, x2.options().dtype(at::kByte));
-  const float* mean = saved[2].data_ptr<float>();
+  const float* mean = stats.data_ptr<float>();
   check(tmpi_layernorm_bwd_add(x2.data_ptr(), dy2.data_ptr(), add2.defined() ? add2.data_ptr() : nullptr, weight.data_ptr(), mean, mean + rows,
                                dx.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), (int)rows, (int)C, dtype_code(x2.scalar_type()),
                                scratch.data_ptr(), stream()));
@@ -332,7 +334,7 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &qkv = saved[0], &out = saved[1], &lse = saved[2];
+    const Tensor qkv = as_saved(saved[0]), out = as_saved(saved[1]), lse = as_saved(saved[2]);
     const int64_t heads = ctx->saved_data["heads"].toInt(), B = qkv.size(0), T = qkv.size(1), C3 = qkv.size(2), C = C3 / 3;
     const Tensor dout = grads[0].contiguous();
     Tensor dqkv = at::empty_like(qkv);
@@ -477,7 +479,9 @@ struct BnFn : public torch::autograd::Function<BnFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &y = saved[1], &gamma = saved[2], &beta = saved[3], &mean = saved[4], &invstd = saved[5], &bits = saved[6];
+    const auto cl = at::MemoryFormat::ChannelsLast;
+    const Tensor x = as_saved(saved[0], cl), y = as_saved(saved[1], cl), mean = as_saved(saved[4]);
+    const Tensor &gamma = saved[2], &beta = saved[3], &invstd = saved[5], &bits = saved[6];
     const Tensor dy = channels_last(grads[0]);
     const int64_t C = x.size(1), rows = x.size(0) * x.size(2) * x.size(3);
     const bool has_res = ctx->saved_data["residual"].toBool();
@@ -518,7 +522,7 @@ struct ConvFn : public torch::autograd::Function<ConvFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor x = channels_last(saved[0]), w = channels_last(saved[1]);
     const Tensor dy = channels_last(grads[0]);
     const int N = (int)x.size(0), Cin = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), Cout = (int)w.size(0), R = (int)w.size(2), S = (int)w.size(3);
     const int stride = (int)ctx->saved_data["stride"].toInt(), pad = (int)ctx->saved_data["pad"].toInt();
@@ -579,7 +583,7 @@ struct StemFn : public torch::autograd::Function<StemFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor& x = saved[0];
+    const Tensor x = channels_last(saved[0]);
     Tensor dy = channels_last(grads[0]);
     if ((uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);          // a view into a larger buffer
     const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector(), strides = ctx->saved_data["strides"].toIntVector();

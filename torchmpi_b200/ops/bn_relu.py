@@ -51,6 +51,11 @@ def width_supported(C: int, element_size: int) -> bool:
     return C % V == 0 and 256 % (C // V) == 0
 
 
+def _as_saved(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """A saved activation channels-last again: saved-tensor hooks may hand it back in another layout."""
+    return t.contiguous(memory_format=torch.channels_last) if t is not None else None
+
+
 class _BnReluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, gamma, beta, running_mean, running_var, eps, momentum, relu, training, partial_rows=0,
@@ -108,6 +113,7 @@ class _BnReluFn(torch.autograd.Function):
     def backward(ctx, dy):
         global _launches
         x, y, gamma, beta, mean, invstd, bits = ctx.saved_tensors
+        x, y = _as_saved(x), _as_saved(y)
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
@@ -180,6 +186,7 @@ class _BnReluPoolFn(torch.autograd.Function):
     def backward(ctx, dy):
         global _launches
         x, xmax, idx, gamma, beta, mean, invstd = ctx.saved_tensors
+        x, xmax, idx = _as_saved(x), _as_saved(xmax), idx.contiguous()
         dy = dy.contiguous(memory_format=torch.channels_last)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)

@@ -151,7 +151,7 @@ class _ConvFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, w = ctx.saved_tensors
+        x, w = map(_cl, ctx.saved_tensors)             # hooks may hand them back in another layout
         dy = _cl(dy)
         from ..parallel.flat_buckets import MaskedGrad, direct_grad, grad_written
         dx = dw = None
