@@ -242,7 +242,7 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint32_t (&w)
 __device__ __forceinline__ void pair_sync(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(1 + team() * 4 + quarter) : "memory"); }
 __device__ __forceinline__ void pair_leave(int quarter) { asm volatile("bar.arrive %0, 64;" ::"r"(1 + team() * 4 + quarter) : "memory"); }
 #define ROWS_WAIT(bar, parity, where) \
-  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); __syncwarp(); pair_leave(quarter); return; } } while (0)
+  do { if (!sm100::mbar_wait_warp((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); __syncwarp(); pair_leave(quarter); return; } } while (0)
 
 // Two threads per query row: `half` picks 64 of the 128 scores of a block and 32 of the 64 output columns.  The halves
 // exchange their maxima through shared memory, block by block, and their row sums at the end of an item.
@@ -359,7 +359,7 @@ __device__ void softmax_rows(Shared* sh, Shared* other_team, float* xch, float2*
     // the item's output: O / l
     float l0, l1, l_other;
     unpack2(add2(sum2[0], sum2[1]), l0, l1);
-    if (*(volatile int*)&sh->error) { pair_leave(quarter); return; }     // the partner may have left at the last exchange
+    if (__any_sync(~0u, *(volatile int*)&sh->error)) { pair_leave(quarter); return; }     // the partner may have left at the last exchange
     exchange(l0 + l1, &l_other);
     float l = half ? l_other + (l0 + l1) : (l0 + l1) + l_other;
     const bool merges = SHARED && it.qblk > 0;

@@ -118,6 +118,11 @@ struct Ring {
 
 #define ATTNB_WAIT(bar, parity, where) \
   do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); return; } } while (0)
+// In a whole warp the lanes go on, or leave, together: a wait may succeed for some of them and have run out for others, who would then be missing
+// at the warp's next barrier.  A wait that has run out is noted, the lane goes on, with values that no longer matter, and the warp
+// votes where its lanes meet anyway.
+#define ATTNB_WARP_WAIT(bar, parity, where) \
+  do { if (!sm100::mbar_wait((bar), (parity), kWaitBudgetNs, &sh->error)) { fail(sh, p, (where)); ok = false; } } while (0)
 
 __device__ void producer(Shared* sh, unsigned char* smem, const Params& p, const CUtensorMap* mq, const CUtensorMap* mk,
                          const CUtensorMap* mv, const CUtensorMap* mdo) {
@@ -239,6 +244,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
   const unsigned long long c2x2 = pack2(__float_as_uint(p.scale_log2), __float_as_uint(p.scale_log2));
   const unsigned long long nl2e = pack2(__float_as_uint(-1.4426950408889634f), __float_as_uint(-1.4426950408889634f));
   const bool tracer = row == 0 && part == 0;
+  bool ok = true;
   Ring<QD_STAGES> q;
   int g = 0, bh, jblk;
   for (int r = 0; item(p, r, &bh, &jblk); ++r) {
@@ -248,8 +254,8 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       const float4* delta = lse + STAT_BYTES / 16;
       const bool diag = n == 0, masked = diag && part < quarter;               // masked: every query of the thread is before its key
       if (tracer) stamp(p, r, n, 0);
-      ATTNB_WAIT(&sh->qd_full[q.stage], q.use & 1, 11);
-      ATTNB_WAIT(&sh->s_full, g & 1, 12);
+      ATTNB_WARP_WAIT(&sh->qd_full[q.stage], q.use & 1, 11);
+      ATTNB_WARP_WAIT(&sh->s_full, g & 1, 12);
       if (tracer) stamp(p, r, n, 1);
       sm100::tc_fence_after();
       uint32_t s[32], w[16];
@@ -279,7 +285,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
 #pragma unroll
       for (int e = 0; e < 16; ++e) w[e] = pack_bf16(s[2 * e], s[2 * e + 1]);
       if (g > 0) {                                         // dV of the previous pair has read P
-        ATTNB_WAIT(&sh->dv_done, (g - 1) & 1, 13);
+        ATTNB_WARP_WAIT(&sh->dv_done, (g - 1) & 1, 13);
         sm100::tc_fence_after();
       }
       sm100::tmem_st_32x16(t_p, w);
@@ -287,7 +293,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       sm100::tc_fence_before();
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&sh->p_full);
-      ATTNB_WAIT(&sh->dp_full, g & 1, 14);
+      ATTNB_WARP_WAIT(&sh->dp_full, g & 1, 14);
       sm100::tc_fence_after();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {                        // dS = P (dP - delta), 16 queries at a time
@@ -313,7 +319,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] = 0u;
         }
-        if (c == 0 && g > 0) ATTNB_WAIT(&sh->dq_full, (g - 1) & 1, 15);          // dK and dQ of the previous pair have read dS
+        if (c == 0 && g > 0) ATTNB_WARP_WAIT(&sh->dq_full, (g - 1) & 1, 15);          // dK and dQ of the previous pair have read dS
 #pragma unroll
         for (int u = 0; u < 2; ++u)                        // eight queries = one 16-byte unit of the swizzled row
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
@@ -321,7 +327,7 @@ __device__ void softmax_rows(Shared* sh, unsigned char* smem, const Params& p, i
       }
       sm100::fence_proxy_async_smem();                     // the MMA reads dS through the async proxy
       sm100::tc_fence_before();
-      __syncwarp();
+      if (!__all_sync(~0u, ok)) return;
       if (lane == 0) {
         sm100::mbar_arrive(&sh->ds_full);
         sm100::mbar_arrive(&sh->qd_empty[q.stage]);        // the statistics have been read
@@ -338,6 +344,7 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
   unsigned char* staging = smem + DQ_OFF + quarter * (TILE / DRAIN_WARPS);      // 32 rows of 128 bytes
   const unsigned long long scale2 = pack2(__float_as_uint(p.scale), __float_as_uint(p.scale));
   const bool tracer = quarter == 0 && lane == 0;
+  bool ok = true;
   auto scaled = [&](uint32_t (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
@@ -352,14 +359,14 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
     uint32_t v[2][32];
     for (int n = 0; n < pairs; ++n, ++g) {
       if (tracer) stamp(p, r, n, 3);
-      ATTNB_WAIT(&sh->dq_full, g & 1, 16);
+      ATTNB_WARP_WAIT(&sh->dq_full, g & 1, 16);
       if (tracer) stamp(p, r, n, 4);
       sm100::tc_fence_after();
       sm100::tmem_ld_32x32(tm + T_DQ, v[0]);
       sm100::tmem_ld_32x32(tm + T_DQ + 32, v[1]);
       sm100::tmem_ld_wait();
       sm100::tc_fence_before();
-      __syncwarp();
+      if (!__all_sync(~0u, ok)) return;
       if (lane == 0) sm100::mbar_arrive(&sh->dq_empty);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -379,7 +386,8 @@ __device__ void drain(Shared* sh, unsigned char* smem, const Params& p, const CU
       }
       if (tracer) stamp(p, r, n, 5);
     }
-    ATTNB_WAIT(&sh->acc_full, r & 1, 17);
+    ATTNB_WARP_WAIT(&sh->acc_full, r & 1, 17);
+    if (!__all_sync(~0u, ok)) return;
     sm100::tc_fence_after();
     auto store = [&](const CUtensorMap* map) {             // 32 rows of 64 bf16 through the staging tile
       if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");

@@ -78,6 +78,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   }
 }
 
+// The same for a whole warp, whose lanes go on, or give up, together: a wait may succeed for some lanes and have run out for others, which
+// would then be missing at the warp's next barrier.  Only the first look at the barrier is inlined: with the loops in its place the votes
+// took 4 % of the attention forward (1 x 16 x 2048 21.4 us in place of 20.5), like this nothing.
+static __device__ __noinline__ bool mbar_wait_on(uint64_t* bar, uint32_t parity, unsigned long long budget_ns, const int* error) {
+  return mbar_wait(bar, parity, budget_ns, error);
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long budget_ns, const int* error) {
+  return __all_sync(~0u, mbar_try_wait(bar, parity)) || __all_sync(~0u, mbar_wait_on(bar, parity, budget_ns, error));
+}
+
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
