@@ -84,3 +84,25 @@ def test_block_with_and_without_hooks(batch, seq, heads):
     assert len(seen) == 1 and float((seen[0].float() - x.float()).norm() / x.float().norm()) > 0.5       # not the sum
     for a, c in zip(*out):
         assert float((a.float() - c.float()).norm() / c.float().norm()) < 2e-2
+
+
+@pytest.mark.parametrize("rows,width", [(256, 256), (1024, 1024)])
+def test_residual_and_bias_of_the_kernel_in_front(rows, width):
+    """The product starts before the layer norm that writes its residual (and a row of which is its bias) has ended."""
+    from torchmpi_b200 import _native
+    from torchmpi_b200.ops import gemm
+    torch.manual_seed(rows)
+    x, w, one, zero = _rand(rows, width), _rand(width, width, scale=width ** -0.5), _rand(width), _rand(width)
+    outs = []
+    for sync in (torch.cuda.synchronize, lambda: None):
+        out = []
+        for k in range(8):                                                   # each norm's output lies where the one before lay
+            t = x + k
+            sync()
+            r = _native.ext().layer_norm(t * (k + 1.0), one, zero, 1e-5 * (k + 1))
+            sync()
+            out.append(gemm.linear_add(x, w, r[k], r * 1.0 if k % 2 else r))
+            sync()
+            del r
+        outs.append(out)
+    assert all(torch.equal(a, b) for a, b in zip(*outs))

@@ -28,7 +28,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = sm100::cluster_ctarank();
   setup(sh, warp, &map_a, &map_b, 4 * GROUPS);
-  wait_previous();
+  const __nv_bfloat16 *bias = p.bias, *residual = p.residual;      // read through the read-only path: not before the wait (pdl.cuh)
+  wait_previous(bias, residual);
 
   const int total = p.tiles_m * p.tiles_n;
   const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
@@ -45,7 +46,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   } else if (warp == 1) {
     if (rank == 0 && sm100::elect_one()) mma_issuer<NST>(sh, tiles, p, order);
   } else {
-    epilogue_groups<MODE>(sh, staging, p, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
+    epilogue_groups<MODE>(sh, staging, p, bias, residual, (warp - 2) >> 2, warp & 3, lane, order, &map_c, &map_y);
   }
   __syncwarp();
   teardown(sh, warp);

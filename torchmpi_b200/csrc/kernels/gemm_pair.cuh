@@ -175,7 +175,7 @@ __device__ __forceinline__ void epilogue(Shared* sh, unsigned char* staging, con
 // without that pass's launch and its read of C.  It has staging tiles of its own (the operand ring gives up a stage for
 // them), so a group never waits for the store it has just issued.  8192 x 4096 x 1024: product 83 and pass 36 us before, one
 // kernel of 69 now (82 with one staging tile per group).
-// RESIDUAL: p.residual is added before the rounding.  A thread reads its row's 128 bytes of the next slice while it works on this one.
+// RESIDUAL: the residual is added before the rounding.  A thread reads its row's 128 bytes of the next slice while it works on this one.
 // (A pass that adds after the product reads both and writes the sum: 8 us at 8192 x 1024.)
 enum { PLAIN = 0, WITH_GELU = 1, RESIDUAL = 2 };
 constexpr int GROUPS = 2, GROUP_THREADS = 64 + GROUPS * 128;
@@ -183,8 +183,8 @@ constexpr int GROUPS = 2, GROUP_THREADS = 64 + GROUPS * 128;
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
 template <int MODE, typename TileOrder>
-__device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* staging, const Problem& p, int group, int quarter,
-                                                int lane, TileOrder order, const CUtensorMap* map_c, const CUtensorMap* map2) {
+__device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* staging, const Problem& p, const __nv_bfloat16* bias,
+                                                const __nv_bfloat16* residual, int group, int quarter, int lane, TileOrder order, const CUtensorMap* map_c, const CUtensorMap* map2) {
   constexpr bool TWO = MODE == WITH_GELU;
   constexpr int SLICE = 64, SLICE_BYTES = BM * SLICE * 2;
   static_assert(GROUPS * SLICE_BYTES <= gemm::EPI_STAGING_BYTES && GROUPS * SLICE_BYTES <= STAGE_BYTES, "a staging tile per group and output");
@@ -192,7 +192,7 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
   const bool leader = quarter == 0 && lane == 0;
   const int bn = p.pair_n ? p.pair_n : BN;
   unsigned char* stg0 = staging + group * SLICE_BYTES;
-  const bool bias_vec = ((uintptr_t)p.bias & 15) == 0;
+  const bool bias_vec = ((uintptr_t)bias & 15) == 0;
   int m_blk, n_blk;
   uint4 res[8], res_next[8];
   auto read_residual = [&](uint4 (&v)[8], int col0) {
@@ -200,7 +200,7 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
     const bool inside = m_blk * BM + row < p.M;
 #pragma unroll
     for (int j = 0; j < 8; ++j)          // N is a multiple of 8
-      v[j] = inside && col0 + 8 * j < p.N ? __ldg(reinterpret_cast<const uint4*>(p.residual + at) + j) : make_uint4(0u, 0u, 0u, 0u);
+      v[j] = inside && col0 + 8 * j < p.N ? __ldg(reinterpret_cast<const uint4*>(residual + at) + j) : make_uint4(0u, 0u, 0u, 0u);
   };
   for (int it = 0; order(it, &m_blk, &n_blk); ++it) {
     const int acc = it & 1;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
         if (bias_vec && col0 + SLICE <= p.N) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + j);
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(bias + col0) + j);
             const uint32_t b[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -243,7 +243,7 @@ __device__ __forceinline__ void epilogue_groups(Shared* sh, unsigned char* stagi
         } else {
 #pragma unroll
           for (int j = 0; j < 64; ++j)
-            if (col0 + j < p.N) r[j >> 5][j & 31] = __float_as_uint(__uint_as_float(r[j >> 5][j & 31]) + __bfloat162float(p.bias[col0 + j]));
+            if (col0 + j < p.N) r[j >> 5][j & 31] = __float_as_uint(__uint_as_float(r[j >> 5][j & 31]) + __bfloat162float(bias[col0 + j]));
         }
       }
       if (MODE == RESIDUAL) {
