@@ -132,3 +132,32 @@ def test_counters_after_waits_that_ran_out():
     assert not fresh.any() and all(fresh.data_ptr() != t.data_ptr() for t in held)
     assert take(like, 64).data_ptr() == fresh.data_ptr()
     gemm.check_status()
+
+
+def _absorbing(rows, cols):
+    """Two large values that cancel, and small ones between them that a sum in one chain loses one by one."""
+    t = torch.full((rows, cols), 2.0 ** -14, device="cuda")
+    t[0], t[-1] = 2.0 ** 15, -2.0 ** 15
+    return t
+
+
+def _cancelling(rows, cols):
+    t = torch.randn(rows, cols, device="cuda") + 1.0
+    t[-64:] -= t.sum(0) / 64
+    return t
+
+
+@pytest.mark.parametrize("values", [_absorbing, _cancelling])
+@pytest.mark.parametrize("form", [0, 1 << 21 | _form(256, 1, 256, 1, 5)])                  # 21 slices of the sums
+@pytest.mark.parametrize("rows,out", [(512, 1024), (640, 20480), (2048, 520), (8192, 1024), (8192, 4096), (24576, 1000)])
+def test_bias_gradient_is_a_sum_of_short_chains(rows, out, form, values):
+    """Column sums that cancel show the error of the fp32 sum, and not the rounding of the result."""
+    torch.manual_seed(rows)
+    dy = values(rows, out).to(torch.bfloat16)
+    x, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((rows, 64), (out, 64)))
+    db = _run(dy, x, w, 7, form)[2].double()
+    ref, total = dy.double().sum(0), dy.double().abs().sum(0)
+    # a value passes the batches of 128 rows of its thread, at most 48 of a slice, three levels inside its batch, four over the threads, and
+    # the slices in fours, of which there are eight at most: so many roundings by half a unit, each of at most the sum of the absolute values
+    bound = (min(rows / 128, 48) + 3 + 4 + 2 + 8) * 2.0 ** -24 * total
+    assert bool(((db - ref).abs() <= 2.0 ** -9 * ref.abs() + bound).all())
