@@ -122,6 +122,26 @@ def test_matmul_tn_splitk_long_k_small_output():
     conv.check_status()
 
 
+# slices of four K blocks: one to three, ten and eleven; outputs with remainders of a tile, of a group of columns and of a warp's columns
+@pytest.mark.parametrize("M,N", [(1024, 256), (1032, 264), (136, 264), (8, 8)])
+@pytest.mark.parametrize("K", [8, 256, 512, 600, 768, 2560, 2816])
+def test_split_products_by_number_of_slices(K, M, N):
+    from torchmpi_b200.ops import conv
+    torch.manual_seed(K)
+    a, b = (torch.randn(K, n, device="cuda").to(torch.bfloat16) for n in (M, N))
+    want, sums = a.double().t() @ b.double(), a.double().abs().t() @ b.double().abs()
+    # K / 16 MMA steps and the slices in fp32 (2^-23 of a partial sum each), one rounding to bf16, and of the accumulated ones another
+    fp32 = (K / 16 + 16) * 2.0 ** -23 * sums
+    got = conv.matmul_tn_splitk(a, b)
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + fp32).all())
+    assert torch.equal(got, conv.matmul_tn_splitk(a, b))
+    acc = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    total = acc.double() + want
+    conv.matmul_tn_splitk(a, b, out=acc, accumulate=True)
+    assert bool(((acc.double() - total).abs() <= 2.0 ** -8 * total.abs() + 2.0 ** -23 * total.abs() + fp32).all())
+    conv.check_status()
+
+
 def test_conv_bn_fused_statistics_match_separate_pass():
     """conv -> batch-norm with the statistics from the convolution's epilogue equals conv -> batch-norm with its own pass."""
     from torchmpi_b200.ops import conv

@@ -32,6 +32,7 @@
 // Every mbarrier wait is bounded; a CTA that gives up records a status word, drains and returns.
 #include <cuda_bf16.h>
 #include <algorithm>
+#include <utility>
 #include <cstring>
 #include <mutex>
 #include "sm100_ptx.cuh"
@@ -545,11 +546,51 @@ conv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 }
 
+// out[row, col] (+)= sum over S slices of the partial tiles, all loads of eight columns in flight in one thread: for few slices of an output that
+// fills the chip with such threads, where sharing a row among warps only makes them short.  us with the kernel below and with this one:
+// one slice of 512 x 2048 4.0, 2.4, of 512 x 4608 6.7, 3.4; two 6.9, 4.5; three of 512 x 2048 6.5, 3.5; five of 256 x 1024 4.2, 3.0; ten 6.4, 3.6;
+// but five of 128 x 512 2.5, 2.8, ten 3.2, 3.4 (8192 threads).
+constexpr int FEW_SLICES = 10;
+constexpr long long FEW_THREADS = 16384;
+template <int S>
+__global__ void __launch_bounds__(256)
+conv_splitk_reduce_few_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int N, int tiles_m, int mma_n, int accumulate, unsigned total) {
+  const unsigned groups = (unsigned)N / 8;                     // N is a multiple of 8
+  const size_t pitch = (size_t)BM * mma_n;
+  for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    const int row = (int)(i / groups), col = (int)(i % groups) * 8, m_blk = row / BM, n_blk = col / BN;
+    const float* src = ws + (size_t)(n_blk * tiles_m + m_blk) * S * pitch + (size_t)(row - m_blk * BM) * mma_n + (col - n_blk * BN);
+    float4 x[S][2];
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) x[s][h] = __ldcs(reinterpret_cast<const float4*>(src + s * pitch) + h);
+    float a[8] = {x[0][0].x, x[0][0].y, x[0][0].z, x[0][0].w, x[0][1].x, x[0][1].y, x[0][1].z, x[0][1].w};
+#pragma unroll
+    for (int s = 1; s < S; ++s) {
+      const float b[8] = {x[s][0].x, x[s][0].y, x[s][0].z, x[s][0].w, x[s][1].x, x[s][1].y, x[s][1].z, x[s][1].w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] += b[e];
+    }
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * N + col);
+    if (accumulate) {
+      float f[8];
+      unpack8(*dst, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] += f[e];
+    }
+    const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a[0], a[1]), __floats2bfloat162_rn(a[2], a[3]), __floats2bfloat162_rn(a[4], a[5]),
+                                 __floats2bfloat162_rn(a[6], a[7])};
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(h);
+    *dst = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
 // out[row, col] (+)= sum over slices of the partial tiles.  A warp reads 128 columns of a row (512 contiguous bytes) of every W-th slice,
 // U slices in flight; the W warps of a row add their sums in order, so the result does not depend on timing.  Bound by the loads'
 // latency.  Lanes that shared 8 columns and took a slice each read 32-byte pieces of 32 slices per instruction; before and now, images x
 // inputs x outputs x size, us: 256 x 512 x 128 x 28 9.3, 4.8; 256 x 128 x 512 x 28 7.0, 4.0; 32 x 1024 x 256 x 14 14.2, 6.8; 64 x 256 x 64 x 56
-// 5.2, 5.0; 8 x 512 x 2048 x 7, two slices, 2.8, 4.0.
+// 5.2, 5.0.
 constexpr int RED_WARPS = 8;
 template <int U>
 __global__ void __launch_bounds__(32 * RED_WARPS)
@@ -692,8 +733,22 @@ static int conv_launch(const CUtensorMap& ma, const CUtensorMap& mb, const void*
   return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "conv launch: %s", cudaGetErrorString(e));
 }
 
+template <int... S>
+static decltype(&conv::conv_splitk_reduce_few_kernel<1>) few_kernel(int slices, std::integer_sequence<int, S...>) {
+  static constexpr decltype(&conv::conv_splitk_reduce_few_kernel<1>) kernels[] = {conv::conv_splitk_reduce_few_kernel<S + 1>...};
+  return kernels[slices - 1];
+}
+
 static int launch_splitk_reduce(const conv::Problem& p, const void* workspace, void* out, int accumulate, cudaStream_t s) {
-  int W = 1;                                                    // warps of a row, two slices each or more
+  const long long groups = (long long)p.M * (p.N / 8);
+  if (p.slices <= conv::FEW_SLICES && (p.slices <= 2 || groups >= conv::FEW_THREADS) && groups < 0x7fffffffLL) {
+    const int grid = (int)std::min<long long>((groups + 255) / 256, (long long)gemm_sm_count() * 8);
+    const auto kernel = few_kernel(p.slices, std::make_integer_sequence<int, conv::FEW_SLICES>());
+    kernel<<<grid, 256, 0, s>>>((const float*)workspace, (__nv_bfloat16*)out, p.N, p.tiles_m, p.mma_n, accumulate, (unsigned)groups);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? TMPI_OK : fail(TMPI_ERR_CUDA, "split-K reduce launch: %s", cudaGetErrorString(e));
+  }
+  int W = 1;                                                    // warps of a row, with at most two slices each up to sixteen slices
   while (W < conv::RED_WARPS && 2 * W < p.slices) W <<= 1;
   const int per_block = conv::RED_WARPS / W, col_blocks = (p.N + 127) / 128;
   const long long blocks = (long long)((p.M + per_block - 1) / per_block) * col_blocks;
