@@ -234,7 +234,6 @@ _CUDA_PROTOS = {
     "tmpi_attention_set_trace": (None, [_vp]),
     "tmpi_attention_status": (_i, []),
     "tmpi_layernorm_status": (_i, []),
-    "tmpi_gemm_tn_prefers_splitk": (_i, [_i, _i, _i64]),
     "tmpi_gemm_tn_splitk_workspace_bytes": (_sz, [_i, _i, _i64]),
     "tmpi_gemm_bf16_tn_splitk": (_i, [_vp, _vp, _vp, _i, _i, _i64, _i64, _i64, _vp, _sz, _i, _vp]),
 }

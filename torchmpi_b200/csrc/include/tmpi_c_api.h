@@ -313,7 +313,6 @@ int tmpi_attention_ctas_per_sm(void);
 void tmpi_attention_set_trace(void* device_buffer);   // tuning aid: phase time stamps of one CTA
 int tmpi_attention_status(void);
 // C[M, N] (+)= A^T B for A [K, M], B [K, N] with a long K and a small output (split over K; same kernel family)
-int tmpi_gemm_tn_prefers_splitk(int M, int N, int64_t K);
 size_t tmpi_gemm_tn_splitk_workspace_bytes(int M, int N, int64_t K);
 int tmpi_gemm_bf16_tn_splitk(const void* A, const void* B, void* C, int M, int N, int64_t K, int64_t lda, int64_t ldb,
                              void* workspace, size_t workspace_bytes, int accumulate, void* stream);

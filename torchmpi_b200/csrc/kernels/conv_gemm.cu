@@ -915,29 +915,12 @@ int tmpi_conv_wgrad(const void* dy, const void* x, void* dw, int N, int H, int W
 
 // C[M, N] (+)= A^T B for row-major A [K, M] and B [K, N] (both read as they lie) with a long K and a small
 // output: K is split over the SMs, fp32 partial tiles go to the workspace and a second kernel adds them in
-// slice order.  M, N multiples of 8; lda / ldb / ldc: row pitches in elements (0: dense).
+// slice order.  M, N multiples of 8; lda / ldb / ldc: row pitches in elements (0: dense).  (The linear layers' weight gradients come from
+// linear_bwd.cu.)
 size_t tmpi_gemm_tn_splitk_workspace_bytes(int M, int N, int64_t K) {
   int tm, tn, mn, kbt, per, sl;
   splitk_plan(M, N, K, &tm, &tn, &mn, &kbt, &per, &sl);
   return (size_t)tm * tn * sl * conv::BM * mn * sizeof(float);
-}
-
-// (The linear layers' weight gradients come from linear_bwd.cu.)  Whether that beats the CTA-pair kernel: where whole tiles leave most SMs idle over a long K, against a second kernel and the
-// partial tiles' way to memory and back.  An output of more than half as many tiles as SMs is not split at all: it would only
-// take that way, in several rounds.  Measured, back to back, in us (pair, split): 8192 x 1024 x 1024 37, 29; 8192 x 512 x 512
-// 37, 22; 8192 x 128 x 256 36, 14; 8192 x 1536 x 1536 39, 41; 4096 x 512 x 512 20, 20; 4096 x 1024 x 1024 21, 22; 2048 x 512 x 512
-// 12, 16; not split, 8192 x 3072 x 2048 84, 126; 8192 x 4096 x 4096 189, 293.  A round of the pair kernel takes about 4.5 + 0.25 per
-// 64-wide K block, the split kernels, one round, 11 + 0.25 per K block of a slice and the partial tiles at 3.3 TB/s.
-int tmpi_gemm_tn_prefers_splitk(int M, int N, int64_t K) {
-  if (M < 1 || N < 1 || K < 1 || M % 8 || N % 8) return 0;
-  int tm, tn, mn, kbt, per, sl;
-  splitk_plan(M, N, K, &tm, &tn, &mn, &kbt, &per, &sl);
-  if (sl < 2) return 0;
-  const int clusters = gemm_sm_count() / 2;
-  const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
-  const double pair = 4.5 + 0.25 * kbt * (double)((tiles + clusters - 1) / clusters);
-  const double split = 11 + 0.25 * per + 2.0 * tm * tn * sl * conv::BM * mn * sizeof(float) / 3.3e6;
-  return split < 0.9 * pair;
 }
 
 int tmpi_gemm_bf16_tn_splitk(const void* A, const void* B, void* C, int M, int N, int64_t K, int64_t lda, int64_t ldb,
