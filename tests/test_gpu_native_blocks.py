@@ -64,6 +64,43 @@ def test_bottleneck_takes_either_path(first, mode):
             assert torch.equal(a, b)
 
 
+def _odd(t):
+    """The values of a channels-last tensor, in a buffer in which they start two bytes behind a 16-byte boundary."""
+    rows = t.permute(0, 2, 3, 1)
+    buf = torch.empty(t.numel() + 8, device=t.device, dtype=t.dtype)[1:1 + t.numel()].view(rows.shape).copy_(rows).permute(0, 3, 1, 2)
+    assert buf.data_ptr() % 16 == t.element_size() and buf.is_contiguous(memory_format=torch.channels_last)
+    return buf
+
+
+@pytest.mark.parametrize("layer", ["block", "block in flat buckets", "pool", "stem"])
+def test_inputs_and_gradients_at_odd_addresses(layer):
+    """Views into larger buffers are read through a copy: the kernels' loads need 16-byte boundaries."""
+    from torchmpi_b200.models import to_bf16_mixed
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLUMaxPool
+    from torchmpi_b200.ops.pool import MaxPool2d
+    from torchmpi_b200.ops.stem_conv import StemConv7x7
+    torch.manual_seed(3)
+    if layer == "pool":
+        m, shape = MaxPool2d(3, 2, 1), (2, 64, 12, 10)
+    elif layer == "stem":
+        m, shape = to_bf16_mixed(torch.nn.Sequential(StemConv7x7(64), FusedBatchNormReLUMaxPool(64)).cuda()).to(memory_format=torch.channels_last), (2, 3, 32, 64)
+    else:
+        inp, m = _block(False)
+        shape = (3, inp, 12, 10)
+        if layer == "block in flat buckets":
+            for p in m.parameters():
+                p._tmpi_grad_sink = lambda *a, **k: None
+    x = torch.randn(shape, device="cuda").to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    state, out = {k: v.clone() for k, v in m.state_dict().items()}, []
+    for place in (lambda t: t, _odd):
+        m.load_state_dict(state)
+        leaf = place(x).detach().requires_grad_(layer != "stem")
+        y = m(leaf)
+        dy = torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(y.dtype).contiguous(memory_format=torch.channels_last)
+        out.append([y] + list(torch.autograd.grad(y, ([leaf] if layer != "stem" else []) + list(m.parameters()), place(dy))))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
 def test_block_on_a_side_stream_and_in_a_graph():
     """The functions' scratch is of the stream and the call."""
     inp, m = _block(False)

@@ -52,13 +52,13 @@ int dtype_code(at::ScalarType t) {
 
 // Contiguous and on a 16-byte boundary, which the elementwise kernels' loads need: a view into a larger buffer may start
 // anywhere.
-Tensor packed(const Tensor& t) {
-  const Tensor c = t.contiguous();
-  return (uintptr_t)c.data_ptr() % 16 ? c.clone() : c;
+Tensor packed(const Tensor& t, at::MemoryFormat format = at::MemoryFormat::Contiguous) {
+  const Tensor c = t.contiguous(format);
+  return (uintptr_t)c.data_ptr() % 16 ? c.clone(format) : c;
 }
 
 // A saved tensor as it was saved: hooks (torch.autograd.graph.save_on_cpu, say) may hand it back in another layout.
-Tensor as_saved(const Tensor& t, at::MemoryFormat format = at::MemoryFormat::Contiguous) { return t.defined() ? t.contiguous(format) : t; }
+Tensor as_saved(const Tensor& t, at::MemoryFormat format = at::MemoryFormat::Contiguous) { return t.defined() ? packed(t, format) : t; }
 
 // Buffers of arrival counters, which a kernel finds zero and leaves zero.  Two calls may share one only if one ends before the
 // other starts, so there is one per stream, grown to the next power of two.  A call that is being captured gets its own, cleared
@@ -428,7 +428,7 @@ ForkPtr kept_fork(AutogradContext* ctx, const char* name) {
   return v.isCapsule() ? c10::static_intrusive_pointer_cast<Fork>(v.toCapsule()) : ForkPtr();
 }
 
-Tensor channels_last(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
+Tensor channels_last(const Tensor& t) { return packed(t, at::MemoryFormat::ChannelsLast); }
 Tensor empty_channels_last(at::IntArrayRef sizes, const Tensor& like) {
   return at::empty(sizes, like.options(), at::MemoryFormat::ChannelsLast);
 }
@@ -584,8 +584,7 @@ struct StemFn : public torch::autograd::Function<StemFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor x = channels_last(saved[0]);
-    Tensor dy = channels_last(grads[0]);
-    if ((uintptr_t)dy.data_ptr() % 16) dy = dy.clone(at::MemoryFormat::ChannelsLast);          // a view into a larger buffer
+    const Tensor dy = channels_last(grads[0]);
     const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector(), strides = ctx->saved_data["strides"].toIntVector();
     Tensor dw = at::empty_strided(shape, strides, x.options());
     // partial sums of the CTAs (24 MB), from the allocator: calls on other streams, threads and in graphs have their own

@@ -204,6 +204,7 @@ bias_grad_finalize_kernel(const float* __restrict__ partial, int nblocks, int C,
 template <typename T>
 static int bias_grad_t(const void* dy, const void* z, void* dz, void* db, int rows, int C, void* scratch, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
+  if (!all_aligned16({dy, z, dz})) return fail(TMPI_ERR_INVALID, "bias_grad: tensors must be 16-byte aligned");
   if (rows < 1 || C % (kBgCols * V)) return fail(TMPI_ERR_UNSUPPORTED, "bias_grad: C=%d must be a multiple of %d", C, kBgCols * V);
   if (z && !dz) return fail(TMPI_ERR_INVALID, "bias_grad: z given without an output for dz");
   const int slabs = C / (kBgCols * V);

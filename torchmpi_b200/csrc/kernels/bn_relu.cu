@@ -365,7 +365,8 @@ __global__ void __launch_bounds__(kBnThreads, 3) bn_apply_bwd_kernel(
   for (; v < nvec; v += stride) pass(v, std::integral_constant<int, 1>());
 }
 
-static int bn_check(int64_t rows, int C, int V) {
+static int bn_check(int64_t rows, int C, int V, std::initializer_list<const void*> tensors) {
+  if (!all_aligned16(tensors)) return fail(TMPI_ERR_INVALID, "bn: tensors must be 16-byte aligned");
   if (rows < 1 || C < V || C % V) return fail(TMPI_ERR_INVALID, "bn: C=%d must be a multiple of %d", C, V);
   int cvn = C / V;
   if (kBnThreads % cvn) return fail(TMPI_ERR_UNSUPPORTED, "bn: C/%d = %d must divide %d", V, cvn, kBnThreads);
@@ -377,7 +378,7 @@ static int bn_fwd_t(const void* x, const void* res, void* y, const float* gamma,
                     float* rvar, float* smean, float* sinv, int64_t rows, int C, float eps, float momentum, int relu,
                     int training, void* bits, void* scratch, cudaStream_t s, int given_rows = 0) {
   constexpr int V = 16 / sizeof(T);
-  int st = bn_check(rows, C, V);
+  int st = bn_check(rows, C, V, {x, res, y});
   if (st) return st;
   size_t nvec = (size_t)rows * (C / V);
   int grid = bn_grid(nvec, kBnMaxGrid, kBnReduceU);
@@ -411,7 +412,7 @@ static int bn_bwd_t(const void* x, const void* y, const void* dy, void* dx, void
                     const float* beta, const float* smean, const float* sinv, float* dgamma, float* dbeta, int64_t rows, int C, int relu,
                     const void* bits, void* scratch, cudaStream_t s, float* acc_gamma = nullptr, float* acc_beta = nullptr) {
   constexpr int V = 16 / sizeof(T);
-  int st = bn_check(rows, C, V);
+  int st = bn_check(rows, C, V, {x, y, dy, dx, dres});
   if (st) return st;
   if (relu && !y && !bits && (!beta || dres))
     return fail(TMPI_ERR_INVALID, "bn backward: without y or mask bits the layer needs beta and no residual");
@@ -789,9 +790,10 @@ __global__ void __launch_bounds__(kBpThreads, BLOCKS) bn_pool_bwd_apply_kernel(
 
 // What both directions take, checked before anything is launched: the kernels stage nothing, so a row of any length that an
 // int can index.
-static int bn_pool_check(int64_t rows, const BpDims& d, int V) {
-  int st = bn_check(rows, d.C, V);
+static int bn_pool_check(int64_t rows, const BpDims& d, int V, const void* idx, std::initializer_list<const void*> tensors) {
+  int st = bn_check(rows, d.C, V, tensors);
   if (st) return st;
+  if ((uintptr_t)idx % V) return fail(TMPI_ERR_INVALID, "bn+pool: the index must be %d-byte aligned", V);
   if ((int64_t)(d.W + 1) * d.C > 0x7fffffffLL) return fail(TMPI_ERR_UNSUPPORTED, "bn+pool: rows of %d x %d are too long", d.W, d.C);
   return TMPI_OK;
 }
@@ -803,7 +805,7 @@ static int bn_pool_fwd_t(const void* x, void* y, void* idx, void* xmax, const fl
   constexpr int V = 16 / sizeof(T);
   const int64_t rows = (int64_t)N * H * W;
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
-  int st = bn_pool_check(rows, d, V);
+  int st = bn_pool_check(rows, d, V, idx, {x, y, xmax});
   if (st) return st;
   if (training) {
     size_t nvec = (size_t)rows * (C / V);
@@ -849,7 +851,7 @@ static int bn_pool_bwd_t(const void* x, const void* xmax, const void* dy, const 
   constexpr int V = 16 / sizeof(T);
   const int64_t rows = (int64_t)N * H * W;
   BpDims d{N, H, W, C, (H - 1) / 2 + 1, (W - 1) / 2 + 1};
-  int st = bn_pool_check(rows, d, V);
+  int st = bn_pool_check(rows, d, V, idx, {x, xmax, dy, dx});
   if (st) return st;
   const bool fours = sizeof(T) == 2 && kBpThreads % (C / 4) == 0;       // packs of four channels, see below
   int grid;

@@ -248,6 +248,8 @@ template <typename T>
 static int ln_dispatch(bool fwd, const void* x, const void* a, const void* add, const void* gamma, const void* beta, void* out, float* mean,
                        float* rstd, float* partial, void* dgamma, void* dbeta, int rows, int C, float eps, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
+  if (!all_aligned16({x, a, add, gamma, beta, out}))
+    return fail(TMPI_ERR_INVALID, "layernorm: tensors must be 16-byte aligned");
   if (rows < 1 || C % (32 * V)) return fail(TMPI_ERR_UNSUPPORTED, "layernorm: C=%d must be a multiple of %d", C, 32 * V);
   cudaError_t e;
   switch (C / (32 * V)) {

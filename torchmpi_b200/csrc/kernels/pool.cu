@@ -171,6 +171,8 @@ template <typename T>
 static int pool_launch(bool fwd, const void* a, void* b, void* idx, PoolDims d, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   if (d.C % V) return fail(TMPI_ERR_INVALID, "maxpool: C=%d must be a multiple of %d", d.C, V);
+  if (!all_aligned16({a, b})) return fail(TMPI_ERR_INVALID, "maxpool: tensors must be 16-byte aligned");
+  if ((uintptr_t)idx % V) return fail(TMPI_ERR_INVALID, "maxpool: the index must be %d-byte aligned", V);
   if (d.k * d.k > 255) return fail(TMPI_ERR_INVALID, "maxpool: window too large");
   const long long rows = (long long)d.N * (fwd ? d.OH : d.H);
   if (rows < 1 || rows > 0x7fffffffLL) return fail(TMPI_ERR_INVALID, "maxpool: %lld rows", rows);

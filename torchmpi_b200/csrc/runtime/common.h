@@ -5,6 +5,7 @@
 #include <string>
 #include <functional>
 #include <future>
+#include <initializer_list>
 #include "../include/tmpi_c_api.h"
 
 namespace tmpi {
@@ -12,6 +13,12 @@ namespace tmpi {
 // Records a message for tmpi_last_error() (thread local) and returns `code`.
 int fail(int code, const char* fmt, ...);
 void set_error(const char* fmt, va_list ap);
+// Whether all start on a 16-byte boundary (null does): what kernels with 16-byte loads and stores need, which fault otherwise.
+inline bool all_aligned16(std::initializer_list<const void*> pointers) {
+  for (const void* p : pointers)
+    if ((uintptr_t)p & 15) return false;
+  return true;
+}
 
 // Tunables are read through this accessor everywhere in the runtime.
 int64_t tunable(const char* name);

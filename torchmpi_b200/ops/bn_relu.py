@@ -51,9 +51,15 @@ def width_supported(C: int, element_size: int) -> bool:
     return C % V == 0 and 256 % (C // V) == 0
 
 
+def channels_last(t: torch.Tensor) -> torch.Tensor:
+    """``t`` channels-last and on a 16-byte boundary, which the kernels' loads need: a view into a larger buffer may start anywhere."""
+    t = t.contiguous(memory_format=torch.channels_last)
+    return t.clone(memory_format=torch.channels_last) if t.data_ptr() % 16 else t
+
+
 def _as_saved(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """A saved activation channels-last again: saved-tensor hooks may hand it back in another layout."""
-    return t.contiguous(memory_format=torch.channels_last) if t is not None else None
+    return channels_last(t) if t is not None else None
 
 
 class _BnReluFn(torch.autograd.Function):
@@ -65,9 +71,9 @@ class _BnReluFn(torch.autograd.Function):
         (weight, bias) Parameters, whose gradients are added in place when a flat bucket owns their buffers;
         ``res_fork``: a ``GradFork`` shared by the consumers of ``residual``."""
         global _launches
-        x = x.contiguous(memory_format=torch.channels_last)
+        x = channels_last(x)
         if residual is not None:
-            residual = residual.contiguous(memory_format=torch.channels_last)
+            residual = channels_last(residual)
         N, C, H, W = x.shape
         rows = N * H * W
         y = torch.empty_like(x, memory_format=torch.channels_last)
@@ -114,7 +120,7 @@ class _BnReluFn(torch.autograd.Function):
         global _launches
         x, y, gamma, beta, mean, invstd, bits = ctx.saved_tensors
         x, y = _as_saved(x), _as_saved(y)
-        dy = dy.contiguous(memory_format=torch.channels_last)
+        dy = channels_last(dy)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
         # the first of several consumers of the residual parks its gradient for the last one's kernel: as dy and the mask bits
@@ -158,7 +164,7 @@ class _BnReluPoolFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gamma, beta, running_mean, running_var, eps, momentum, training, grad_mode):
         global _launches
-        x = x.contiguous(memory_format=torch.channels_last)
+        x = channels_last(x)
         N, C, H, W = x.shape
         OH, OW = (H - 1) // 2 + 1, (W - 1) // 2 + 1
         y = torch.empty((N, C, OH, OW), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
@@ -187,7 +193,7 @@ class _BnReluPoolFn(torch.autograd.Function):
         global _launches
         x, xmax, idx, gamma, beta, mean, invstd = ctx.saved_tensors
         x, xmax, idx = _as_saved(x), _as_saved(xmax), idx.contiguous()
-        dy = dy.contiguous(memory_format=torch.channels_last)
+        dy = channels_last(dy)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
         dgamma = torch.empty(C, dtype=torch.float32, device=x.device)

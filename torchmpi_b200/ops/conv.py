@@ -21,6 +21,7 @@ import torch.nn.functional as F
 
 from .. import _native
 from .._lib import lib, check, has_symbol, stream_ptr, TorchMPIError
+from .bn_relu import channels_last as _cl
 
 _launches = 0
 _ws = {}
@@ -47,10 +48,6 @@ def supported(x: torch.Tensor, w: torch.Tensor, stride: int, padding: int) -> bo
     Cout, Cin, R, S = w.shape
     return (Cin % 64 == 0 and Cout % 64 == 0 and R == S and padding <= R - 1 and x.shape[1] == Cin
             and x.shape[0] * x.shape[2] * x.shape[3] < 2 ** 31)
-
-
-def _cl(t: torch.Tensor) -> torch.Tensor:
-    return t if t.is_contiguous(memory_format=torch.channels_last) else t.contiguous(memory_format=torch.channels_last)
 
 
 def _out_hw(H, W, R, S, stride, pad):

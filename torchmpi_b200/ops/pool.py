@@ -11,6 +11,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .._lib import lib, check, dtype_code, has_symbol, stream_ptr
+from .bn_relu import channels_last
 
 launch_count = 0
 
@@ -27,7 +28,7 @@ class _MaxPoolFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, k, s, p):
         global launch_count
-        x = x.contiguous(memory_format=torch.channels_last)
+        x = channels_last(x)
         N, C, H, W = x.shape
         OH, OW = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
         y = torch.empty((N, C, OH, OW), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
@@ -44,7 +45,7 @@ class _MaxPoolFn(torch.autograd.Function):
         global launch_count
         (idx,) = ctx.saved_tensors
         N, H, W, C, OH, OW, k, s, p = ctx.dims
-        dy = dy.contiguous(memory_format=torch.channels_last)
+        dy = channels_last(dy)
         dx = torch.empty((N, C, H, W), dtype=dy.dtype, device=dy.device, memory_format=torch.channels_last)
         check(lib.tmpi_maxpool_bwd(dy.data_ptr(), idx.data_ptr(), dx.data_ptr(), N, H, W, C, OH, OW, k, s, p,
                                    dtype_code(dy.dtype), stream_ptr()))

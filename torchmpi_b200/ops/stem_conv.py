@@ -86,6 +86,8 @@ class StemConv7x7(nn.Conv2d):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if supported(x, self.weight):
+            if x.data_ptr() % 16:
+                x = x.clone(memory_format=torch.channels_last)          # a view into a larger buffer
             if direct(x, self.weight):
                 return _StemDirectFn.apply(x, self.weight)
             return _StemConvFn.apply(x, self.weight)
