@@ -24,8 +24,11 @@ def _block(first, planes=64):
 @pytest.mark.parametrize("mode", ["train", "eval", "frozen input", "hooked", "no fork"])
 @pytest.mark.parametrize("first", [False, True])
 def test_bottleneck_takes_either_path(first, mode):
-    from torchmpi_b200 import config
+    from torchmpi_b200 import _native, config
     from torchmpi_b200.ops import bn_relu, conv
+
+    def launched():                              # by the C++ functions, by the Python ones
+        return [_native.launches(_native.CONV), _native.launches(_native.BATCHNORM)], [conv._launches, bn_relu._launches]
     inp, m = _block(first)
     m.train(mode != "eval")
     x = torch.randn(3, 12, 10, inp, device="cuda").to(torch.bfloat16).permute(0, 3, 1, 2)
@@ -36,16 +39,16 @@ def test_bottleneck_takes_either_path(first, mode):
             m.load_state_dict(state)
             m.zero_grad(set_to_none=True)
             if not native:
-                m.conv1.weight._tmpi_grad_sink = lambda *a, **k: None        # a gradient buffer that is not there yet: returned to autograd
-                for b in (m.bn1, m.bn2, m.bn3):
-                    b.weight._tmpi_grad_sink = lambda *a, **k: None
+                for p in m.parameters():
+                    p._tmpi_grad_sink = lambda *a, **k: None                 # a gradient buffer that is not there yet: returned to autograd
             hook = m.bn3.register_forward_hook(lambda mod, args, y: None) if mode == "hooked" else None
             leaf = x.clone().requires_grad_(mode != "frozen input")
-            before = conv.launch_count, bn_relu.launch_count
+            before = launched()
             y = m(leaf)
             dy = torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(y.dtype).contiguous(memory_format=torch.channels_last)
             y.backward(dy)
-            assert conv.launch_count > before[0] and bn_relu.launch_count > before[1]
+            cpp, py = ([n - o for n, o in zip(a, b)] for a, b in zip(launched(), before))
+            assert all(cpp) and (mode == "hooked" or not any(py)) if native else all(py) and not any(cpp)      # (the hooked layer is Python's)
             conv.check_status()
             if hook is not None:
                 hook.remove()
@@ -99,6 +102,28 @@ def test_inputs_and_gradients_at_odd_addresses(layer):
         dy = torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).to(y.dtype).contiguous(memory_format=torch.channels_last)
         out.append([y] + list(torch.autograd.grad(y, ([leaf] if layer != "stem" else []) + list(m.parameters()), place(dy))))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+def test_masked_gradient_without_a_kernel_that_takes_it():
+    """A residual's gradient that is parked as the incoming gradient and mask bits, and whose last consumer is another residual, or a
+    strided convolution, which leave the mask to tensor operations."""
+    from torchmpi_b200 import _native
+    from torchmpi_b200.ops.bn_relu import FusedBatchNormReLU
+    torch.manual_seed(4)
+    new = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16).to(memory_format=torch.channels_last)
+    first, second = FusedBatchNormReLU(64).cuda(), FusedBatchNormReLU(64).cuda()
+    w = new(64, 64, 1, 1).requires_grad_(True)
+    a, b, r, dy, dz = (new(2, 64, 6, 6) for _ in range(5))
+    for strided in (False, True):
+        grads = []
+        for fork in (_native.ext().Fork(2), None):
+            leaf = r.clone().requires_grad_(True)
+            # of the two consumers the one that ran last in forward is first in backward
+            z = _native.ext().conv2d(leaf, w, 2, 0, fork) if strided else second(b, leaf, res_fork=fork)
+            y = first(a, leaf, res_fork=fork)
+            grads.append(torch.autograd.grad((z, y), leaf, (dz[:, :, ::2, ::2].contiguous(memory_format=torch.channels_last) if strided else dz, dy))[0].float())
+        # one rounding of the sum to bf16, where autograd's own sum rounds the same terms
+        assert bool(((grads[0] - grads[1]).abs() <= 2.0 ** -7 * grads[1].abs() + 1e-6).all()), strided
 
 
 def test_block_on_a_side_stream_and_in_a_graph():
