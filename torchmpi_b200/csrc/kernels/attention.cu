@@ -29,7 +29,7 @@
 // r * G + i, then r * G + G - 1 - i), which leaves the key blocks per team within one of each other at 8 x 16 x 1024; the
 // next item's loads and first S run under the end of the current one.
 //
-// Measured on a B200, launches in a row: 8 x 16 heads x 1024 x 64 40.6 us, 1 x 16 x 2048 21.0 (47.7 and 25.5 before waiting warps
+// Measured on a B200, launches in a row: 8 x 16 heads x 1024 x 64 39.6 us, 1 x 16 x 2048 20.8 (47.7 and 25.5 before waiting warps
 // slept, waits looked at the error word only when they do not succeed, and the halves met at named barriers).
 //
 // Q, K and V are read where the fused QKV projection left them ([B * T, 3 C], one tensor map per operand) and the

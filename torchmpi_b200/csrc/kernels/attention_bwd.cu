@@ -29,7 +29,7 @@
 // warps share the work (eight: 105 us in place of 97).  Tried and taken back: half of the softmax warps offset by half a pair, so
 // that the exponentials of some run beside the stores of the others (116 in place of 109); the statistics scaled by a warp of their
 // own (100 in place of 96).  Measured on a B200, 8 x 16 heads x 1024 x 64, the three launches of a backward in a row: 113.5
-// -> 90.2 us, of which this kernel 70; 1 x 16 x 2048 46.8 -> 39.5.
+// -> 90.5 us, of which this kernel 70; 1 x 16 x 2048 46.8 -> 39.5.
 //
 // The order in which CTAs add to dQ is not fixed, so its low bits vary; dK and dV are bit-reproducible.  Every wait is
 // bounded; a CTA that gives up records where and frees its tensor memory.

@@ -442,7 +442,7 @@ static int candidates(int what, int rows, int in, int out, int clusters, Candida
       set_part(&q, what, rows, in, out, {bn, s});
       const int units = q.tiles_m * q.tiles_n * q.slices;
       // slices of eight K blocks or more, and of an output that leaves clusters idle or deals out badly; long slices (the K of a
-      // vocabulary) also of more tiles: 8192 x 50257 x 1024 1484 us whole, 1407 with dX in four slices
+      // vocabulary) also of more tiles: both gradients of a head of 1600 x 4096 x 32000 606 us with dX whole, 590 in three slices
       if (s == 1 || (q.slices == s && q.per >= 8 && units <= (q.per >= 32 ? 8 : 4) * clusters)) list[n++] = {{bn, s}, unit_cycles(q), units};
     }
   return n;
@@ -608,7 +608,8 @@ using namespace tmpi;
 extern "C" {
 
 // What a call needs: bytes of workspace and arrival counters (unsigned, zero before the first call that uses them; every call leaves
-// them zero).  want: 1 dX, 2 dW, 4 db, of which at least one of the first two.
+// them zero).  want: 1 dX, 2 dW, 4 db, of which at least one of the first two.  Up to eight tiles of 256 KB for each cluster and product:
+// none to 20 MB for most layers, 157 MB for 65536 x 256 x 50257.
 int tmpi_linear_bwd_plan(int rows, int in, int out, int want, int form, size_t* workspace_bytes, int* counters) {
   if (rows < 1 || in < 1 || out < 1 || in % 8) return fail(TMPI_ERR_INVALID, "linear_bwd: stored rows must be multiples of 16 bytes (TMA)");
   if (!(want & 3) || want & ~7) return fail(TMPI_ERR_INVALID, "linear_bwd: nothing to compute");
