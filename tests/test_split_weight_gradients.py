@@ -1,6 +1,7 @@
 """Which weight gradients of linear layers are cut into slices of their rows (csrc/kernels/linear_bwd.cu), as the plan of a call shows by
 its arrival counters and its workspace of fp32 partial tiles."""
 import ctypes
+import time
 
 import pytest
 
@@ -40,3 +41,24 @@ def test_workspace_is_bounded():
             for inp in (64, 768, 1024, 4096):
                 for want in (1, 2, 3, 7):
                     assert _plan(rows, inp, out, want)[0] <= 2 * 8 * 74 * 256 * 256 * 4 + 2 * 32 * 256 * 4 * -(-out // 256), (rows, out, inp, want)
+
+
+@pytest.mark.parametrize("rows,width", [(2048, 512), (8192, 1024), (128, 512)])
+def test_plans_of_a_model_are_kept(rows, width):
+    """The plans of a block's four layers, asked for in turn, are found again rather than made anew, which takes twice as long or longer."""
+    layers = [(rows, width, 3 * width), (rows, width, width), (rows, width, 4 * width), (rows, 4 * width, width)]
+    size, n = ctypes.c_size_t(0), ctypes.c_int(0)
+
+    def took(sizes):
+        best = float("inf")
+        for _ in range(20):
+            start = time.perf_counter()
+            for s in sizes * 50:
+                lib.tmpi_linear_bwd_plan(*s, 7, 0, ctypes.byref(size), ctypes.byref(n))
+            best = min(best, (time.perf_counter() - start) / len(sizes))
+        return best
+    for _ in range(10):                                      # a busy machine: once is enough
+        alone, turns = sum(took([s]) for s in layers) / 4, took(layers)
+        if turns < 1.3 * alone:
+            return
+    assert turns < 1.3 * alone, (alone, turns)
