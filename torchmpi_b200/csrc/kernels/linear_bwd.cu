@@ -519,7 +519,7 @@ static long long best_list(int rows, int in, int out, int want, int clusters, Ch
         least = t;
         if (nx) best[DX] = x[i].c;
         if (nw) best[DW] = w[j].c;
-        best[DB] = {BN, slices};
+        if (want >> DB & 1) best[DB] = {BN, slices};
       }
     }
   return least;
