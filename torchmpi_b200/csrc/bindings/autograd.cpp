@@ -54,8 +54,10 @@ int dtype_code(at::ScalarType t) {
 // Contiguous and on a 16-byte boundary, which the elementwise kernels' loads need: a view into a larger buffer may start
 // anywhere.
 Tensor packed(const Tensor& t, at::MemoryFormat format = at::MemoryFormat::Contiguous) {
-  const Tensor c = t.contiguous(format);
-  return (uintptr_t)c.data_ptr() % 16 ? c.clone(format) : c;
+  if (t.is_contiguous(format) && (uintptr_t)t.data_ptr() % 16 == 0) return t;
+  Tensor c = t.contiguous(format);
+  if ((uintptr_t)c.data_ptr() % 16) c = c.clone(format);
+  return c;
 }
 
 // A saved tensor as it was saved: hooks (torch.autograd.graph.save_on_cpu, say) may hand it back in another layout.
