@@ -51,15 +51,12 @@ def width_supported(C: int, element_size: int) -> bool:
     return C % V == 0 and 256 % (C // V) == 0
 
 
-def channels_last(t: torch.Tensor) -> torch.Tensor:
-    """``t`` channels-last and on a 16-byte boundary, which the kernels' loads need: a view into a larger buffer may start anywhere."""
-    t = t.contiguous(memory_format=torch.channels_last)
-    return t.clone(memory_format=torch.channels_last) if t.data_ptr() % 16 else t
-
-
-def _as_saved(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """A saved activation channels-last again: saved-tensor hooks may hand it back in another layout."""
-    return channels_last(t) if t is not None else None
+def channels_last(t: torch.Tensor, order=torch.channels_last) -> torch.Tensor:
+    """``t`` channels-last and on a 16-byte boundary, which the kernels' loads need: a view into a larger buffer may start anywhere.
+    (Saved tensors are asked for their order too: saved-tensor hooks may hand them back in another.)"""
+    if not t.is_contiguous(memory_format=order):
+        t = t.contiguous(memory_format=order)
+    return t.clone(memory_format=order) if t.data_ptr() & 15 else t
 
 
 class _BnReluFn(torch.autograd.Function):
@@ -119,7 +116,10 @@ class _BnReluFn(torch.autograd.Function):
     def backward(ctx, dy):
         global _launches
         x, y, gamma, beta, mean, invstd, bits = ctx.saved_tensors
-        x, y = _as_saved(x), _as_saved(y)
+        if not x.is_contiguous(memory_format=torch.channels_last):
+            x = channels_last(x)
+        if y is not None:
+            y = channels_last(y)
         dy = channels_last(dy)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)
@@ -192,7 +192,7 @@ class _BnReluPoolFn(torch.autograd.Function):
     def backward(ctx, dy):
         global _launches
         x, xmax, idx, gamma, beta, mean, invstd = ctx.saved_tensors
-        x, xmax, idx = _as_saved(x), _as_saved(xmax), idx.contiguous()
+        x, xmax, idx = channels_last(x), channels_last(xmax) if xmax is not None else None, idx.contiguous()
         dy = channels_last(dy)
         N, C, H, W = x.shape
         dx = torch.empty_like(x, memory_format=torch.channels_last)

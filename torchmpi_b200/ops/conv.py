@@ -148,7 +148,9 @@ class _ConvFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, w = map(_cl, ctx.saved_tensors)             # hooks may hand them back in another layout
+        x, w = ctx.saved_tensors
+        if not (x.is_contiguous(memory_format=torch.channels_last) and w.is_contiguous(memory_format=torch.channels_last)):
+            x, w = _cl(x), _cl(w)                      # hooks may hand them back in another layout
         dy = _cl(dy)
         from ..parallel.flat_buckets import MaskedGrad, direct_grad, grad_written
         dx = dw = None
