@@ -157,7 +157,7 @@ def test_bias_gradient_is_a_sum_of_short_chains(rows, out, form, values):
     x, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((rows, 64), (out, 64)))
     db = _run(dy, x, w, 7, form)[2].double()
     ref, total = dy.double().sum(0), dy.double().abs().sum(0)
-    # a value passes the batches of 128 rows of its thread, at most 48 of a slice, three levels inside its batch, four over the threads, and
+    # a value passes the batches of 256 rows of its thread, at most 24 of a slice, four levels inside its batch, four over the threads, and
     # the slices in fours, of which there are eight at most: so many roundings by half a unit, each of at most the sum of the absolute values
-    bound = (min(rows / 128, 48) + 3 + 4 + 2 + 8) * 2.0 ** -24 * total
+    bound = (min(rows / 256, 24) + 4 + 4 + 2 + 8) * 2.0 ** -24 * total
     assert bool(((db - ref).abs() <= 2.0 ** -9 * ref.abs() + bound).all())

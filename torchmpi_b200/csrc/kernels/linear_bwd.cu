@@ -161,8 +161,8 @@ __device__ __forceinline__ bool issue_unit(Shared* sh, unsigned char* tiles, con
 __device__ __forceinline__ void all_sync() { asm volatile("bar.sync 3, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
 // The sums of 128 columns of dY from col0 over the rows [r0, r1), by all epilogue threads; thread `row` of group 0 has column col0 + row.
-// Sixteen threads share eight columns, each with 16-byte loads of every 16th row, of which 8 to 16 are in flight; the values of a batch of
-// eight are added as a tree, and so are the threads' sums: a value passes 7 additions and one per 128 rows.  part: 8 KB of group 0's staging.
+// Sixteen threads share eight columns, each with 16-byte loads of every 16th row, of which 8 to 16 are in flight; the values of two batches
+// of eight are added as a tree, and so are the threads' sums: a value passes 8 additions and one per 256 rows.  part: 8 KB of group 0's staging.
 __device__ __forceinline__ float column_sums(const Problem& p, const __nv_bfloat16* dy, float* part, int col0, int r0, int r1, int group, int row) {
   constexpr int U = 8, STEP = DB_GROUPS;
   const int e = threadIdx.x - 64, col = col0 + (e % (BM / 8)) * 8, mine = e / (BM / 8);
@@ -175,7 +175,7 @@ __device__ __forceinline__ float column_sums(const Problem& p, const __nv_bfloat
     for (int i = 0; i < U; ++i)
       v[i] = r + i * STEP < (unsigned)end ? __ldcg(reinterpret_cast<const uint4*>(dy + (r + i * STEP) * p.ld_dy + col)) : make_uint4(0u, 0u, 0u, 0u);
   };
-  auto add = [&](const uint4 (&v)[U]) {
+  auto sum = [&](const uint4 (&v)[U], unsigned long long (&to)[4]) {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       unsigned long long t[U];
@@ -188,16 +188,19 @@ __device__ __forceinline__ float column_sums(const Problem& p, const __nv_bfloat
       for (int n = U / 2; n; n /= 2)
 #pragma unroll
         for (int i = 0; i < n; ++i) t[i] = attn_util::add2(t[i], t[i + n]);
-      acc[w] = attn_util::add2(acc[w], t[0]);
+      to[w] = t[0];
     }
   };
   uint4 a[U], b[U];
   load(a, r0 + mine);
   for (unsigned r = r0 + mine; r < (unsigned)end; r += 2 * U * STEP) {
+    unsigned long long first[4], second[4];
     load(b, r + U * STEP);
-    add(a);
+    sum(a, first);
     load(a, r + 2 * U * STEP);
-    add(b);
+    sum(b, second);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) acc[w] = attn_util::add2(acc[w], attn_util::add2(first[w], second[w]));
   }
   float s[8];
 #pragma unroll
@@ -473,7 +476,7 @@ static long long span(const Candidate* const (&c)[2], int parts, int clusters) {
 // Clusters that the list leaves idle sum it for nothing, if they are enough (at 430 cycles a K block of 256 columns: 330 on an idle chip, 650 beside
 // products that are bound by their loads).  Otherwise the epilogues of some of the others sum it under their first tile,
 // in a multiple of dW's slices, which then bring the same rows into L2.  In a list of one round all wait for those units, above all
-// where they are slices, so there every cluster takes a part.  A thread adds 48 times in the longest slice, of 96 K blocks (of
+// where they are slices, so there every cluster takes a part.  A thread adds 24 times in the longest slice, of 96 K blocks (of
 // very many rows, an eighth of them).
 // us without db and with 1, 2, 4, 8, 16 slices: 1024 x 1024 x 1024 8.6, 8.7, 8.7, 9.2; 8192 x 1024 x 1024 30.3, 36.6, 29.9, 30.0, 30.5, 30.6;
 // of that dW and db alone (64 units) 20.5, 27.7, 20.5, 22.3, 21.8, 21.5; 8192 x 1024 x 4096 95.5, 97.1, 97.3, 97.7, 98.7, 98.7; 65536 x 512 x 512
