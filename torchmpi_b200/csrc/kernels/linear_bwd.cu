@@ -477,14 +477,14 @@ static long long span(const Candidate* const (&c)[2], int parts, int clusters) {
 // products that are bound by their loads).  Otherwise the epilogues of some of the others sum it under their first tile,
 // in a multiple of dW's slices, which then bring the same rows into L2.  In a list of one round all wait for those units, above all
 // where they are slices, so there every cluster takes a part.  A thread adds 24 times in the longest slice, of 96 K blocks (of
-// very many rows, an eighth of them).
+// very many rows, an eighth of them); up to 1024 rows are one slice, whose call needs no arrival counters (a microsecond of the host).
 // us without db and with 1, 2, 4, 8, 16 slices: 1024 x 1024 x 1024 8.6, 8.7, 8.7, 9.2; 8192 x 1024 x 1024 30.3, 36.6, 29.9, 30.0, 30.5, 30.6;
 // of that dW and db alone (64 units) 20.5, 27.7, 20.5, 22.3, 21.8, 21.5; 8192 x 1024 x 4096 95.5, 97.1, 97.3, 97.7, 98.7, 98.7; 65536 x 512 x 512
 // (eight slices of dW) 80, 308, 179, 104, 80, 86, with nine 95; dW and db of 16384 x 1024 x 1024 (72 units, three slices) 35.9 and with 3, 6, 18 39.9, 37.8,
 // 37.5.
 static int sums_slices(int rows, int out, int units, long long time, int longest, int dw_slices, int clusters, int* added) {
   const int tiles = (out + 2 * BM - 1) / (2 * BM), k_blocks = (rows + BK - 1) / BK;
-  auto slices = [&](long long per) { return (int)std::min(32LL, (k_blocks - 1) / std::max(4LL, std::min((long long)std::max(96, k_blocks / 8), per)) + 1); };
+  auto slices = [&](long long per) { return (int)std::min(32LL, (k_blocks - 1) / std::max(16LL, std::min((long long)std::max(96, k_blocks / 8), per)) + 1); };
   *added = 0;
   int s = slices(longest / 430);
   if (units < clusters) {
